@@ -1,6 +1,7 @@
 // Chunked v2x2ssd scan on the 5th-generation tensor cores (tcgen05 + TMEM + TMA).
 //
-// Supported: P = 64, N = 64 (D = 2N = 128), bf16 or fp16 operands, float32 state.
+// Supported: P = 64, N <= 128 in multiples of 4, bf16 or fp16 operands, float32 state.  The kernels hold
+// blocks of 64 oscillators (128 real columns); the columns beyond N are zeros that the TMA loads fill in.
 // Everything else takes the exact SIMT path.
 //
 // Formulation (per (batch, head); chunk of L = 64 tokens, local index t, s).  The two
@@ -15,21 +16,20 @@
 //     K'_s  = conj(phi_s) g_s b_s                   (in place over B, stored conjugated)
 //     S     = mask_{s<t}( (Q K'^T) * exp(l_t - l_s) ),  S_tt = Re(conj(c_t) kc_t b_t)
 //     Y     = S U + exp(l_t) * (Q Zv^T)             (Zv = conj of the chunk-start state)
-//     Zv'   = conj(Pi_end) Zv + U^T K''             (K''_s = exp(l_end - l_s) phi_end K'_s)
+//     Zv'   = conj(phi_end) (exp(l_end) Zv + (exp(l_end - l_s) U)^T K')
 // Magnitudes only ever enter as exp(non-positive), exactly like the reference's
 // chunk_scan policy (slinoss/ops/v2x2ssd/reference.py:498-523, 1224-1261); phases are
 // applied to the 16-bit operands, decays to float32 accumulators.
 //
-// One CTA of 18 warps walks the chunks of one (batch, head) in order: 16 worker warps (4 TMEM
-// lane quadrants x 4 column groups: rotation passes and every epilogue), one warp that computes
-// the per-chunk scalars one chunk ahead, and one warp whose lane 0 issues every TMA load / store
-// and every tcgen05.mma.  U/B/C tiles arrive by TMA (128B swizzle, one chunk ahead), the state
-// lives in the workers' registers (float32), the MMAs have M = 64 (rows in lanes 0..15 of every
-// TMEM lane quadrant); scan_tc_fwd.cuh and scan_tc_bwd.cuh describe the thread-to-data mappings.
+// A stream is walked chunk by chunk by one CTA; streams that do not fill the chip are split into segments of
+// chunks: a cheap pre-pass over the segments (states only) and a combine kernel give every segment its start
+// state, and the segments then run side by side.  scan_tc_fwd.cuh and scan_tc_bwd.cuh describe the kernels and
+// the thread-to-data mappings; plan_segments() below holds the rule for the split.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -42,33 +42,8 @@ using namespace tc;
 
 constexpr int L = 64;
 constexpr uint32_t TILE = 8192;           // one [64][128 B] tile
-constexpr uint32_t STAGE = 7 * TILE;      // U | B0 | Zv0 | B1 | Zv1 | C0 | C1  (Zv written by the CTA)
-constexpr uint32_t OFF_KPP = 2 * STAGE;   // K'' (2 tiles)
-constexpr uint32_t OFF_S = OFF_KPP + 2 * TILE;
-constexpr uint32_t OFF_Y = OFF_S + TILE;  // 16-bit Y tile staged for its TMA store
-constexpr uint32_t OFF_SCAL = OFF_Y + TILE;
-constexpr int NSCAL = 12;                 // per-token float arrays
-constexpr uint32_t SMEM_BYTES = OFF_SCAL + 2 * NSCAL * 64 * 4 + 64 + 1024;
-// TMEM columns: [S | Yoff] 0..127 and 128..255 (chunk parity) | Ydiag 256..319 and 320..383 | Inc 384..511
-constexpr uint32_t TMEM_COLS = 512;
 
 __device__ int g_tc_status = 0;
-
-struct alignas(64) TcFwdParams {
-  CUtensorMap tmU, tmB, tmC;
-  CUtensorMap tmY, tmS;   // 16-bit output and chunk-state tensors (TMA stores); unused ones stay zero
-  const float* M;
-  const float* K;
-  const float* z0;
-  const void* Bprev;
-  const void* Uprev;
-  void* Y;
-  const float* Yadd;    // optional float32 (batch*heads, T, 64): added to the output before it is rounded
-  float* zfinal;
-  void* states16;       // optional (batch*heads, nchunks, 64, 128) 16-bit: conjugated start state of every chunk
-  int heads, groups, T, nchunks;
-  long long wait_limit;  // SM clocks a wait of the main loop may take before the kernel gives up
-};
 
 template <typename T> struct Pack2;
 template <> struct Pack2<__nv_bfloat16> {
@@ -79,6 +54,19 @@ template <> struct Pack2<__nv_bfloat16> {
     __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
   }
+  // two words (re, im), (re, im) -> the pair of real parts and the pair of imaginary parts, and back
+  static __device__ __forceinline__ void split(uint32_t w0, uint32_t w1, f2& re, f2& im) {
+    re = mk2(__uint_as_float(w0 << 16), __uint_as_float(w1 << 16));
+    im = mk2(__uint_as_float(w0 & 0xffff0000u), __uint_as_float(w1 & 0xffff0000u));
+  }
+  static __device__ __forceinline__ void join(f2 re, f2 im, uint32_t& w0, uint32_t& w1) {
+    const float2 a = un2(re), b = un2(im);
+    w0 = pack(a.x, b.x); w1 = pack(a.y, b.y);
+  }
+  static __device__ __forceinline__ f2 natural(uint32_t w) {
+    return mk2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+  }
+  static __device__ __forceinline__ uint32_t pack2(f2 v) { const float2 a = un2(v); return pack(a.x, a.y); }
   static constexpr int fmt = 1;
 };
 template <> struct Pack2<__half> {
@@ -89,6 +77,16 @@ template <> struct Pack2<__half> {
     __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
   }
+  static __device__ __forceinline__ void split(uint32_t w0, uint32_t w1, f2& re, f2& im) {
+    const float2 a = unpack(w0), b = unpack(w1);
+    re = mk2(a.x, b.x); im = mk2(a.y, b.y);
+  }
+  static __device__ __forceinline__ void join(f2 re, f2 im, uint32_t& w0, uint32_t& w1) {
+    const float2 a = un2(re), b = un2(im);
+    w0 = pack(a.x, b.x); w1 = pack(a.y, b.y);
+  }
+  static __device__ __forceinline__ f2 natural(uint32_t w) { const float2 a = unpack(w); return mk2(a.x, a.y); }
+  static __device__ __forceinline__ uint32_t pack2(f2 v) { const float2 a = un2(v); return pack(a.x, a.y); }
   static constexpr int fmt = 0;
 };
 
@@ -105,33 +103,55 @@ static long long wait_limit_clocks() {
   return tc::WAIT_CLOCKS_DEFAULT;
 }
 
-// Per-chunk scalars, computed by warp 0 (two tokens per lane) with shuffle scans.
-//  sc[0] l_t        sc[1] exp(l_t)     sc[2],sc[3] phi_t
-//  sc[4],sc[5] w_t = conj(phi_t) g_t                (K'  = w b)
-//  sc[6],sc[7] v_t = exp(l_end - l_t) phi_end w_t   (K'' = v b)
-//  sc[8],sc[9] kc_t                                 (diagonal)
-//  chunk-level: sc[10][0..1] = Pi_end, sc[10][2..3] = its unit phase
-__device__ void chunk_scalars(float* sc, const float* __restrict__ Mb, const float* __restrict__ Kb,
-                              int t0, int T, int lane) {
+// A wait that did not succeed at once: true when the barrier flips within ``limit`` SM clocks, false as soon as
+// another wait of the CTA has expired (``abort_flag``) or when this one does (recorded).
+__device__ __noinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, long long limit, int* abort_flag, int code) {
+  const long long t_begin = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    if (*reinterpret_cast<volatile int*>(abort_flag)) return false;
+    if (clock64() - t_begin > limit) {
+      report_timeout(code);
+      *reinterpret_cast<volatile int*>(abort_flag) = 1;
+      return false;
+    }
+  }
+  return true;
+}
+
+// coefficient of the pending prev-tap of the token before the sequence: kp_0 / m_0
+__device__ __forceinline__ void pending_tap(const float* Mb, const float* Kb, float& xr, float& xi) {
+  const float mr = Mb[0], mi = Mb[1], kr = Kb[0], ki = Kb[1];
+  const float den = mr * mr + mi * mi;
+  xr = (kr * mr + ki * mi) / den;
+  xi = (ki * mr - kr * mi) / den;
+}
+
+// Per-chunk scalars, computed by one warp (two tokens per lane) with shuffle scans.  Layout of a table (floats):
+//  [0, 256)    per token: phi_t (re, im), w_t = conj(phi_t) g_t (re, im)
+//  [256, 512)  per token: kc_t (re, im), exp(l_t), exp(l_end - l_t)
+//  [512, 576)  per token: l_t in units of log 2
+//  [576, 579)  exp(l_end), unit phase of Pi_end (re, im)
+constexpr int SC_KCL = 256, SC_L2 = 512, SC_TAIL = 576, SCW = 592;
+__device__ __noinline__ void chunk_scalars(float* sc, const float* __restrict__ Mb, const float* __restrict__ Kb,
+                                           int t0, int T, int lane) {
   float mr[3], mi[3], kpr[3], kpi[3], kcr[2], kci[2];
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     const int t = t0 + 2 * lane + q;
     mr[q] = 1.f; mi[q] = 0.f; kpr[q] = 0.f; kpi[q] = 0.f;
+    if (q < 2) { kcr[q] = 0.f; kci[q] = 0.f; }
     if (t < T) {
       const float2 m = *reinterpret_cast<const float2*>(Mb + 2 * (size_t)t);
       const float4 k = *reinterpret_cast<const float4*>(Kb + 4 * (size_t)t);
       mr[q] = m.x; mi[q] = m.y; kpr[q] = k.x; kpi[q] = k.y;
       if (q < 2) { kcr[q] = k.z; kci[q] = k.w; }
-    } else if (q < 2) {
-      kcr[q] = 0.f; kci[q] = 0.f;
     }
   }
   // local prefixes over the lane's two tokens
-  const float mag0 = sqrtf(mr[0] * mr[0] + mi[0] * mi[0]);
-  const float mag1 = sqrtf(mr[1] * mr[1] + mi[1] * mi[1]);
-  const float a0 = __logf(mag0), a1 = __logf(mag1);
-  const float u0r = mr[0] / mag0, u0i = mi[0] / mag0, u1r = mr[1] / mag1, u1i = mi[1] / mag1;
+  const float q0 = mr[0] * mr[0] + mi[0] * mi[0], q1 = mr[1] * mr[1] + mi[1] * mi[1];
+  const float i0 = rsqrtf(q0), i1 = rsqrtf(q1);
+  const float a0 = 0.5f * lg2f(q0), a1 = 0.5f * lg2f(q1);
+  const float u0r = mr[0] * i0, u0i = mi[0] * i0, u1r = mr[1] * i1, u1i = mi[1] * i1;
   float lsum = a0 + a1;                       // inclusive scan of log-magnitudes
   float pr = u0r * u1r - u0i * u1i, pi = u0r * u1i + u0i * u1r;  // and of unit phases
 #pragma unroll
@@ -148,8 +168,6 @@ __device__ void chunk_scalars(float* sc, const float* __restrict__ Mb, const flo
   float epr = __shfl_up_sync(0xffffffffu, pr, 1), epi = __shfl_up_sync(0xffffffffu, pi, 1);
   if (lane == 0) { el = 0.f; epr = 1.f; epi = 0.f; }
   const float l_end = __shfl_sync(0xffffffffu, lsum, 31);
-  float per = __shfl_sync(0xffffffffu, pr, 31), pei = __shfl_sync(0xffffffffu, pi, 31);
-  { const float n = rsqrtf(per * per + pei * pei); per *= n; pei *= n; }
   float lt[2], phr[2], phi[2];
   lt[0] = el + a0; lt[1] = el + a0 + a1;
   phr[0] = epr * u0r - epi * u0i; phi[0] = epr * u0i + epi * u0r;
@@ -162,21 +180,15 @@ __device__ void chunk_scalars(float* sc, const float* __restrict__ Mb, const flo
     const float den = mr[q + 1] * mr[q + 1] + mi[q + 1] * mi[q + 1];
     const float gr = kcr[q] + (kpr[q + 1] * mr[q + 1] + kpi[q + 1] * mi[q + 1]) / den;
     const float gi = kci[q] + (kpi[q + 1] * mr[q + 1] - kpr[q + 1] * mi[q + 1]) / den;
-    const float wr = phr[q] * gr + phi[q] * gi, wi = phr[q] * gi - phi[q] * gr;  // conj(phi) g
-    const float e = __expf(l_end - lt[q]);
-    const float vr = e * (per * wr - pei * wi), vi = e * (per * wi + pei * wr);
     const int i = 2 * lane + q;
-    sc[0 * 64 + i] = lt[q];
-    sc[1 * 64 + i] = __expf(lt[q]);
-    sc[2 * 64 + i] = phr[q]; sc[3 * 64 + i] = phi[q];
-    sc[4 * 64 + i] = wr; sc[5 * 64 + i] = wi;
-    sc[6 * 64 + i] = vr; sc[7 * 64 + i] = vi;
-    sc[8 * 64 + i] = kcr[q]; sc[9 * 64 + i] = kci[q];
+    reinterpret_cast<float4*>(sc)[i] =
+        make_float4(phr[q], phi[q], phr[q] * gr + phi[q] * gi, phr[q] * gi - phi[q] * gr);   // phi, conj(phi) g
+    reinterpret_cast<float4*>(sc + SC_KCL)[i] = make_float4(kcr[q], kci[q], ex2f(lt[q]), ex2f(l_end - lt[q]));
+    sc[SC_L2 + i] = lt[q];
   }
-  if (lane == 0) {
-    const float e = __expf(l_end);
-    sc[10 * 64 + 0] = e * per; sc[10 * 64 + 1] = e * pei;
-    sc[10 * 64 + 2] = per; sc[10 * 64 + 3] = pei;   // unit phase of Pi_end
+  if (lane == 31) {
+    sc[SC_TAIL] = ex2f(l_end);
+    sc[SC_TAIL + 1] = phr[1]; sc[SC_TAIL + 2] = phi[1];
   }
 }
 
@@ -185,264 +197,236 @@ __device__ void chunk_scalars(float* sc, const float* __restrict__ Mb, const flo
 
 }  // namespace
 
-// The kernels hold 64 complex state columns per (batch, head).  The recurrence does not couple state
-// columns (z[:, n] sees b[n] only, and y sums c[n] z[:, n] over n), so N = 128 runs as two passes over the
-// column blocks 0..63 and 64..127 of B and C, addressed in place through tensor maps with the full row
-// pitch; the passes' Y, dU, dM, dK and dU_prev add, everything else is per column block.
 bool scan_tc_supported(const ScanDims& d, int io_dtype) {
-  return d.P == 64 && (d.N == 64 || d.N == 128) && (io_dtype == SL_BF16 || io_dtype == SL_F16) && d.T >= 1 &&
+  return d.P == 64 && d.N <= 128 && d.N % 4 == 0 && (io_dtype == SL_BF16 || io_dtype == SL_F16) && d.T >= 1 &&
          tc::encode_tiled_fn() != nullptr;
 }
+
 namespace {
-inline ScanDims one_block(const ScanDims& d) { ScanDims o = d; o.N = 64; return o; }
-// forward workspace of the two-pass form: start state, final state and B_prev of one column block (dense),
-// and the float32 output of the first pass
-struct TcFwdSplitLayout { size_t z0, zf, bprev, ypart, total; };
-TcFwdSplitLayout tc_fwd_split_layout(const ScanDims& d) {
-  const size_t BH = (size_t)d.batch * d.heads, BG = (size_t)d.batch * d.groups;
-  TcFwdSplitLayout o{};
-  size_t off = 0;
-  auto take = [&](size_t bytes) { size_t r = off; off += round_up(bytes, 256); return r; };
-  o.z0 = take(BH * 64 * 128 * 4);
-  o.zf = take(BH * 64 * 128 * 4);
-  o.bprev = take(BG * 128 * 2);
-  o.ypart = take(BH * (size_t)d.T * 64 * 4);
-  o.total = off;
-  return o;
-}
-}  // namespace
-size_t scan_tc_fwd_workspace(const ScanDims& d) { return d.N == 128 ? tc_fwd_split_layout(d).total : 0; }
-namespace {
-struct TcBwdLayout {
-  size_t states, zfinal, dg, sterm, dkcd, anchor, dbh, dch, dstart, dgb, total;
-};
-// (the carried-tap regions are always reserved: the workspace query does not know whether the call
-// will carry B_prev / U_prev)
-TcBwdLayout tc_bwd_layout(const ScanDims& d) {
-  const size_t BH = (size_t)d.batch * d.heads, nC = (d.T + L - 1) / L;
-  TcBwdLayout o{};
-  size_t off = 0;
-  auto take = [&](size_t bytes) { size_t r = off; off += round_up(bytes, 256); return r; };
-  o.states = take(BH * nC * 64 * 128 * 2);
-  o.zfinal = take(BH * 64 * 128 * 4);
-  o.dg = take(BH * d.T * 8);
-  o.sterm = take(BH * d.T * 8);
-  o.dkcd = take(BH * d.T * 8);
-  o.anchor = take(BH * nC * 8);
-  if (d.groups != d.heads) {   // per-head dB / dC (16-bit) before the reduction over the heads of a group
-    o.dbh = take(BH * d.T * 128 * 2);
-    o.dch = take(BH * d.T * 128 * 2);
-  }
-  o.dstart = take(BH * 64 * 128 * 4);   // adjoint of the start state when the caller wants no d_initial
-  o.dgb = take(BH * 8);                 // gradient of the pending tap's coefficient
-  o.total = off;
-  return o;
-}
-}  // namespace
 
-// backward workspace of the two-pass form: the one-block workspace (reused by both passes), dense copies
-// of the per-block inputs, dense per-block outputs, and the second pass' summands
-struct TcBwdSplitLayout {
-  size_t inner, z0, zf, dfin, dinit, bprev, dbprev, du, dm, dk, duprev, total;
-};
-TcBwdSplitLayout tc_bwd_split_layout(const ScanDims& d) {
-  const size_t BH = (size_t)d.batch * d.heads, BG = (size_t)d.batch * d.groups;
-  TcBwdSplitLayout o{};
-  size_t off = 0;
-  auto take = [&](size_t bytes) { size_t r = off; off += round_up(bytes, 256); return r; };
-  o.inner = take(tc_bwd_layout(one_block(d)).total);
-  o.z0 = take(BH * 64 * 128 * 4);
-  o.zf = take(BH * 64 * 128 * 4);
-  o.dfin = take(BH * 64 * 128 * 4);
-  o.dinit = take(BH * 64 * 128 * 4);
-  o.bprev = take(BG * 128 * 2);
-  o.dbprev = take(BG * 128 * 2);
-  o.du = take(BH * (size_t)d.T * 64 * 2);
-  o.dm = take(BH * (size_t)d.T * 2 * 4);
-  o.dk = take(BH * (size_t)d.T * 4 * 4);
-  o.duprev = take(BH * 64 * 2);
-  o.total = off;
-  return o;
-}
+inline int blocks_of(const ScanDims& d) { return d.N <= 64 ? 1 : 2; }
+inline int chunks_of(const ScanDims& d) { return (d.T + L - 1) / L; }
 
-size_t scan_tc_bwd_workspace(const ScanDims& d) {
-  const size_t tcw = d.N == 128 ? tc_bwd_split_layout(d).total : tc_bwd_layout(d).total;
-  return std::max(scan_simt_bwd_workspace(d), tcw);
-}
-
-constexpr int NW = 4;   // worker warps per TMEM lane quadrant
-
-template <typename TIn, typename TY, bool STATES_ONLY>
-static int launch_tc_fwd(const TcFwdParams& p, int grid, cudaStream_t st) {
-  auto k = scan_tc_fwd_kernel<TIn, TY, STATES_ONLY, NW>;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES) != cudaSuccess)
+// Kernel attributes stick to a device: set once per (kernel, device) instead of on every launch.
+template <typename F>
+int ensure_smem(F k, size_t bytes, std::atomic<unsigned long long>& done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return SL_ERR_LAUNCH_FAILED;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (done.load(std::memory_order_relaxed) & bit) return SL_OK;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
     return SL_ERR_LAUNCH_FAILED;
-  k<<<grid, 128 * NW + 64, SMEM_BYTES, st>>>(p);
+  done.fetch_or(bit, std::memory_order_relaxed);
+  return SL_OK;
+}
+
+// Encoding a tensor map is a driver call and needs a current context, which a thread that has only been told its
+// device (an autograd worker, say) may not have yet: the runtime makes one current on the first cudaSetDevice.
+void ensure_context() {
+  static thread_local int ready = -1;
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev != ready && cudaSetDevice(dev) == cudaSuccess) ready = dev;
+}
+
+// Splitting in time.  ``streams`` CTAs of ``nchunks`` serial chunks each leave most of the chip idle when there
+// are few of them.  With S segments the main kernel runs S * streams CTAs of ceil(nchunks / S) chunks, at the
+// price of the pre-pass over the segments (``pre`` of a main chunk per chunk) and of two more launches
+// (``fixed`` chunk times).  The model below counts the chunk times of the most loaded SM: an SM with one
+// resident CTA takes 1 per chunk, one with two takes ``pair`` (2 when only one fits).
+constexpr int FOLD_SEGS = 8;
+struct SegPlan { int nseg, cps; };
+struct SegCost { double pair, pre, fixed; };
+constexpr int SMS = 148;
+inline double load_time(long long ctas, double chunks, double pair) {
+  const long long per_sm = (ctas + SMS - 1) / SMS;
+  return chunks * ((per_sm / 2) * pair + (per_sm & 1));
+}
+inline SegPlan plan_segments(long long streams, int nchunks, const SegCost& c) {
+  SegPlan best{1, nchunks};
+  double t_best = load_time(streams, nchunks, c.pair);
+  for (int s = 2; s <= nchunks && s * streams <= 4 * SMS; ++s) {
+    const int cps = (nchunks + s - 1) / s, ns = (nchunks + cps - 1) / cps;
+    if (ns != s) continue;
+    const double t = load_time(streams * s, cps, c.pair) + c.pre * load_time(streams * (s - 1), cps, c.pair) + c.fixed;
+    if (t < 0.97 * t_best) { t_best = t; best = {s, cps}; }
+  }
+  return best;
+}
+inline SegPlan fwd_plan(const ScanDims& d) {
+  return plan_segments((long long)d.batch * d.heads, chunks_of(d),
+                       blocks_of(d) == 1 ? SegCost{1.5, 0.45, 3.0} : SegCost{2.0, 0.35, 2.5});
+}
+inline SegPlan bwd_plan(const ScanDims& d) {
+  return plan_segments((long long)d.batch * d.heads * blocks_of(d), chunks_of(d), SegCost{2.0, 0.25, 2.0});
+}
+struct SegLayout { size_t seg, pi, total; };
+inline SegLayout seg_layout(const ScanDims& d, int nseg) {
+  const size_t BH = (size_t)d.batch * d.heads;
+  SegLayout o{};
+  if (nseg == 1) return o;
+  o.pi = round_up(BH * nseg * 64 * 128 * blocks_of(d) * 4, 256);
+  o.total = o.pi + round_up(BH * nseg * 8, 256);
+  return o;
+}
+
+template <typename TIn, typename TY, int MODE, int NB>
+int launch_fwd_kernel(const TcFwdParams& p, dim3 grid, cudaStream_t st) {
+  auto k = scan_tc_fwd_kernel<TIn, TY, MODE, NB>;
+  constexpr size_t bytes = FwdSmem<NB, MODE == 0>::BYTES;
+  static std::atomic<unsigned long long> done{0};
+  if (int e = ensure_smem(k, bytes, done)) return e;
+  k<<<grid, 256 * NB + 64, bytes, st>>>(p);
   note_launches(1);
   return launch_status();
 }
 
-// Y == nullptr runs the state pre-sweep only (chunk-start states + final state).
-// ``bc_pitch`` = elements per row of B and C (128, or 256 when B / C point at one column block of
-// N = 128 rows); everything else is dense with 64 state columns.  ``Yadd`` (float32, or null) is added to
-// the output before it is rounded: the first pass' output in the two-pass form.
-int scan_tc_fwd_impl(const void* U, const float* M, const float* K, const void* B, const void* C,
-                     const float* z0, const void* Bprev, const void* Uprev, void* Y, float* zfinal,
-                     void* states16, const ScanDims& d, int io_dtype, int y_dtype,
-                     cudaStream_t st, int bc_pitch = 128, const float* Yadd = nullptr) {
-  TcFwdParams p{};
-  const bool bf = io_dtype == SL_BF16;
-  const uint64_t BH = (uint64_t)d.batch * d.heads, BG = (uint64_t)d.batch * d.groups;
-  if (!tc::make_tmap_3d(&p.tmU, U, 64, d.T, BH, 64, bf) ||
-      !tc::make_tmap_3d(&p.tmB, B, 128, d.T, BG, 64, bf, bc_pitch) ||
-      !tc::make_tmap_3d(&p.tmC, C ? C : B, 128, d.T, BG, 64, bf, bc_pitch))
-    return SL_ERR_LAUNCH_FAILED;
-  p.M = M; p.K = K; p.z0 = z0; p.Bprev = Bprev; p.Uprev = Uprev; p.Y = Y; p.zfinal = zfinal; p.Yadd = Yadd;
-  p.states16 = states16;
-  p.heads = d.heads; p.groups = d.groups; p.T = d.T; p.nchunks = (d.T + L - 1) / L;
-  p.wait_limit = wait_limit_clocks();
-  if (Y && y_dtype != SL_F32 && !tc::make_tmap_3d(&p.tmY, Y, 64, d.T, BH, 64, y_dtype == SL_BF16))
-    return SL_ERR_LAUNCH_FAILED;
-  if (states16 && !tc::make_tmap_3d(&p.tmS, states16, 128, (uint64_t)p.nchunks * 64, BH, 64, bf))
-    return SL_ERR_LAUNCH_FAILED;
-  const int grid = (int)BH;
-  int rc = SL_ERR_UNSUPPORTED;
-  if (!Y) {
-    rc = bf ? launch_tc_fwd<__nv_bfloat16, float, true>(p, grid, st)
-            : launch_tc_fwd<__half, float, true>(p, grid, st);
-  } else if (bf) {
-    SL_DISPATCH_DTYPE(y_dtype, TY, { rc = launch_tc_fwd<__nv_bfloat16, TY, false>(p, grid, st); });
-  } else {
-    SL_DISPATCH_DTYPE(y_dtype, TY, { rc = launch_tc_fwd<__half, TY, false>(p, grid, st); });
+// pre-pass over the segments: MODE 1 forward in time over (U, B), MODE 2 backwards over (dY, C)
+template <typename TIn, int MODE>
+int launch_prepass(TcFwdParams p, int BH, int nb, cudaStream_t st) {
+  p.to_seg = 1; p.from_seg = 0;
+  p.states16 = nullptr; p.zfinal = nullptr; p.z0 = nullptr; p.Bprev = nullptr; p.Uprev = nullptr;
+  p.seg0 = MODE == 2 ? 1 : 0;   // the segment that ends the walk contributes to no other
+  const dim3 grid((unsigned)BH, (unsigned)(p.nseg - 1));
+  return nb == 1 ? launch_fwd_kernel<TIn, float, MODE, 1>(p, grid, st) : launch_fwd_kernel<TIn, float, MODE, 2>(p, grid, st);
+}
+
+// Forward (Y given) or chunk-start / final states only (Y null).
+template <typename TIn>
+int run_fwd(TcFwdParams& p, const ScanDims& d, int y_dtype, cudaStream_t st) {
+  const int BH = d.batch * d.heads, nb = blocks_of(d);
+  if (p.nseg > 1) {
+    if (int e = launch_prepass<TIn, 1>(p, BH, nb, st)) return e;
+    p.from_seg = p.nseg > FOLD_SEGS ? 1 : 2;
   }
+  if (p.from_seg == 1) {
+    scan_tc_combine_kernel<TIn, false><<<dim3((unsigned)BH, 16u * nb), 256, 0, st>>>(
+        p.seg, p.seg_pi, p.z0, reinterpret_cast<const TIn*>(p.Bprev), reinterpret_cast<const TIn*>(p.Uprev), p.M, p.K,
+        d.heads, d.groups, d.T, d.N, nb, p.nseg);
+    note_launches(1);
+  }
+  const dim3 grid((unsigned)BH, (unsigned)p.nseg);
+  if (!p.Y)
+    return nb == 1 ? launch_fwd_kernel<TIn, float, 1, 1>(p, grid, st) : launch_fwd_kernel<TIn, float, 1, 2>(p, grid, st);
+  int rc = SL_ERR_UNSUPPORTED;
+  SL_DISPATCH_DTYPE(y_dtype, TY, {
+    rc = nb == 1 ? launch_fwd_kernel<TIn, TY, 0, 1>(p, grid, st) : launch_fwd_kernel<TIn, TY, 0, 2>(p, grid, st);
+  });
   return rc;
 }
 
-size_t scan_tc_states_bytes(const ScanDims& d) {   // N = 128: the two column blocks one after the other
-  return (size_t)d.batch * d.heads * ((d.T + L - 1) / L) * 64 * 128 * 2 * (d.N / 64);
-}
-
-namespace {
-// column block ``blk`` (128 values of 256) of a (rows, 256) tensor <-> a dense (rows, 128) one
-inline bool copy_block_in(void* dense, const void* wide, int blk, size_t rows, size_t esize, cudaStream_t st) {
-  return cudaMemcpy2DAsync(dense, 128 * esize, reinterpret_cast<const uint8_t*>(wide) + blk * 128 * esize,
-                           256 * esize, 128 * esize, rows, cudaMemcpyDeviceToDevice, st) == cudaSuccess;
-}
-inline bool copy_block_out(void* wide, const void* dense, int blk, size_t rows, size_t esize, cudaStream_t st) {
-  return cudaMemcpy2DAsync(reinterpret_cast<uint8_t*>(wide) + blk * 128 * esize, 256 * esize, dense,
-                           128 * esize, 128 * esize, rows, cudaMemcpyDeviceToDevice, st) == cudaSuccess;
-}
-inline const void* block_of(const void* wide, int blk) {   // 16-bit rows of 256: start of a column block
-  return wide ? reinterpret_cast<const uint8_t*>(wide) + blk * 256 : nullptr;
-}
-
-// a += b over n 16-bit values (summed in float32) or float32 values; 16 bytes per thread, the last
-// thread takes what is left of a length that is no multiple of that
-template <typename T>
-__global__ void __launch_bounds__(256) add_into_kernel(T* __restrict__ a, const T* __restrict__ b, size_t n) {
-  constexpr int V = Vec16<T>::N;
-  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
-  if (i >= n) return;
-  if (i + V <= n) {
-    float x[V], y[V];
-    load16<T>(a + i, x);
-    load16<T>(b + i, y);
-#pragma unroll
-    for (int k = 0; k < V; ++k) x[k] += y[k];
-    store16<T>(a + i, x);
-  } else {
-    for (size_t j = i; j < n; ++j) a[j] = from_f32<T>(to_f32(a[j]) + to_f32(b[j]));
+int scan_tc_fwd_impl(const void* U, const float* M, const float* K, const void* B, const void* C, const float* z0,
+                     const void* Bprev, const void* Uprev, void* Y, float* zfinal, void* states16,
+                     const ScanDims& d, const SegPlan& plan, uint8_t* seg_ws, int io_dtype, int y_dtype,
+                     cudaStream_t st) {
+  TcFwdParams p{};
+  ensure_context();
+  const bool bf = io_dtype == SL_BF16;
+  const uint64_t BH = (uint64_t)d.batch * d.heads, BG = (uint64_t)d.batch * d.groups, W = 2 * (uint64_t)d.N;
+  if (!tc::make_tmap_3d(&p.tmU, U, 64, d.T, BH, 64, bf) || !tc::make_tmap_3d(&p.tmB, B, W, d.T, BG, 64, bf) ||
+      (C && !tc::make_tmap_3d(&p.tmC, C, W, d.T, BG, 64, bf)))
+    return SL_ERR_LAUNCH_FAILED;
+  p.M = M; p.K = K; p.z0 = z0; p.Bprev = Bprev; p.Uprev = Uprev; p.Y = Y; p.zfinal = zfinal;
+  p.states16 = states16;
+  p.heads = d.heads; p.groups = d.groups; p.T = d.T; p.N = d.N; p.nchunks = chunks_of(d);
+  p.nseg = plan.nseg; p.cps = plan.cps;
+  if (plan.nseg > 1) {
+    const SegLayout lay = seg_layout(d, plan.nseg);
+    p.seg = reinterpret_cast<float*>(seg_ws + lay.seg);
+    p.seg_pi = reinterpret_cast<float2*>(seg_ws + lay.pi);
   }
+  p.wait_limit = wait_limit_clocks();
+  if (Y && y_dtype != SL_F32 && !tc::make_tmap_3d(&p.tmY, Y, 64, d.T, BH, 64, y_dtype == SL_BF16))
+    return SL_ERR_LAUNCH_FAILED;
+  if (states16 && !tc::make_tmap_3d(&p.tmS, states16, 128, (uint64_t)p.nchunks * 64, BH * blocks_of(d), 64, bf))
+    return SL_ERR_LAUNCH_FAILED;
+  return bf ? run_fwd<__nv_bfloat16>(p, d, y_dtype, st) : run_fwd<__half>(p, d, y_dtype, st);
 }
-template <typename T>
-void add_into(void* a, const void* b, size_t n, cudaStream_t st) {
-  const size_t pieces = (n + Vec16<T>::N - 1) / Vec16<T>::N;
-  add_into_kernel<T><<<(unsigned)((pieces + 255) / 256), 256, 0, st>>>(reinterpret_cast<T*>(a),
-                                                                      reinterpret_cast<const T*>(b), n);
-  note_launches(1);
+
+// backward workspace (the carried-tap regions are always reserved: the workspace query does not know whether the
+// call will carry B_prev / U_prev)
+struct TcBwdLayout {
+  size_t states, zfinal, dg, sterm, dkcd, anchor, dbh, dch, dstart, dgb, du2, segs, total;
+};
+TcBwdLayout tc_bwd_layout(const ScanDims& d) {
+  const size_t BH = (size_t)d.batch * d.heads, nC = chunks_of(d), NB = blocks_of(d), W = 2 * (size_t)d.N;
+  TcBwdLayout o{};
+  size_t off = 0;
+  auto take = [&](size_t bytes) { size_t r = off; off += round_up(bytes, 256); return r; };
+  o.states = take(BH * nC * 64 * 128 * NB * 2);
+  o.zfinal = take(BH * 64 * W * 4);
+  o.dg = take(NB * BH * d.T * 8);
+  o.sterm = take(NB * BH * d.T * 8);
+  o.dkcd = take(NB * BH * d.T * 8);
+  o.anchor = take(NB * BH * nC * 8);
+  if (d.groups != d.heads) {   // per-head dB / dC (16-bit) before the reduction over the heads of a group
+    o.dbh = take(BH * d.T * W * 2);
+    o.dch = take(BH * d.T * W * 2);
+  }
+  o.dstart = take(BH * 64 * W * 4);   // adjoint of the start state when the caller wants no d_initial
+  o.dgb = take(BH * 8);               // gradient of the pending tap's coefficient
+  if (NB == 2) o.du2 = take(BH * d.T * 64 * 2);   // dU of the second column block
+  o.segs = take(std::max(seg_layout(d, fwd_plan(d).nseg).total, seg_layout(d, bwd_plan(d).nseg).total));
+  o.total = off;
+  return o;
 }
+
 }  // namespace
+
+size_t scan_tc_fwd_workspace(const ScanDims& d) {   // (two column blocks: never zero, callers test for that)
+  return std::max<size_t>(seg_layout(d, fwd_plan(d).nseg).total, blocks_of(d) == 2 ? 256 : 0);
+}
+size_t scan_tc_bwd_workspace(const ScanDims& d) {
+  return std::max(scan_simt_bwd_workspace(d), tc_bwd_layout(d).total);
+}
+size_t scan_tc_states_bytes(const ScanDims& d) {   // two column blocks: one after the other
+  return (size_t)d.batch * d.heads * chunks_of(d) * 64 * 128 * 2 * blocks_of(d);
+}
 
 int scan_tc_fwd(const void* U, const float* M, const float* K, const void* B, const void* C,
                 const float* z0, const void* Bprev, const void* Uprev, void* Y, float* zfinal,
                 void* states_out, const ScanDims& d, int io_dtype, int y_dtype, void* ws, size_t ws_bytes,
                 cudaStream_t st) {
-  if (d.N == 64)
-    return scan_tc_fwd_impl(U, M, K, B, C, z0, Bprev, Uprev, Y, zfinal, states_out, d, io_dtype, y_dtype, st);
-  // N = 128: two passes over the column blocks; the second adds the first's float32 output
-  const TcFwdSplitLayout lay = tc_fwd_split_layout(d);
-  if (!ws || ws_bytes < lay.total) return SL_ERR_WORKSPACE_TOO_SMALL;
-  uint8_t* w = reinterpret_cast<uint8_t*>(ws);
-  const ScanDims d1 = one_block(d);
-  const size_t BH = (size_t)d.batch * d.heads, BG = (size_t)d.batch * d.groups;
-  const size_t st_bytes = scan_tc_states_bytes(d1);
-  float* ypart = reinterpret_cast<float*>(w + lay.ypart);
-  for (int blk = 0; blk < 2; ++blk) {
-    float* z0b = z0 ? reinterpret_cast<float*>(w + lay.z0) : nullptr;
-    float* zfb = zfinal ? reinterpret_cast<float*>(w + lay.zf) : nullptr;
-    void* bpb = Bprev ? (void*)(w + lay.bprev) : nullptr;
-    if (z0 && !copy_block_in(z0b, z0, blk, BH * 64, 4, st)) return SL_ERR_LAUNCH_FAILED;
-    if (Bprev && !copy_block_in(bpb, Bprev, blk, BG, 2, st)) return SL_ERR_LAUNCH_FAILED;
-    void* st_out = states_out ? reinterpret_cast<uint8_t*>(states_out) + blk * st_bytes : nullptr;
-    const int rc = scan_tc_fwd_impl(U, M, K, block_of(B, blk), block_of(C, blk), z0b, bpb, Uprev,
-                                    blk == 0 ? (void*)ypart : Y, zfb, st_out, d1, io_dtype,
-                                    blk == 0 ? (int)SL_F32 : y_dtype, st, 256, blk == 0 ? nullptr : ypart);
-    if (rc != SL_OK) return rc;
-    if (zfinal && !copy_block_out(zfinal, zfb, blk, BH * 64, 4, st)) return SL_ERR_LAUNCH_FAILED;
-  }
-  return launch_status();
+  const SegPlan plan = fwd_plan(d);
+  if (plan.nseg > 1 && (!ws || ws_bytes < seg_layout(d, plan.nseg).total)) return SL_ERR_WORKSPACE_TOO_SMALL;
+  return scan_tc_fwd_impl(U, M, K, B, C, z0, Bprev, Uprev, Y, zfinal, states_out, d, plan,
+                          reinterpret_cast<uint8_t*>(ws), io_dtype, y_dtype, st);
 }
 
+namespace {
+
+// Tensor-core backward: state pre-sweep (unless the forward saved its chunk states), adjoint pre-pass when the
+// sweep is split in time, reverse sweep, the boundary terms of carried B_prev / U_prev, scalar finish, the sum of
+// the column blocks' dU (N > 64) and, for grouped B/C, the reduction of dB / dC over the heads of a group.
 template <typename TIn>
-static int launch_tc_bwd(const TcBwdParams& p, int grid, cudaStream_t st) {
-  auto k = scan_tc_bwd_kernel<TIn, NW>;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B_SMEM_BYTES) != cudaSuccess)
-    return SL_ERR_LAUNCH_FAILED;
-  k<<<grid, 128 * NW + 64, B_SMEM_BYTES, st>>>(p);
-  return launch_status();
-}
-
-// Tensor-core backward: state pre-sweep (unless the forward saved its chunk states), reverse sweep,
-// the boundary terms of carried B_prev / U_prev, scalar finish and, for grouped B/C, the reduction of
-// dB / dC over the heads of a group.  A dY of another dtype (or none) takes the exact float32 sweeps.
-//
-// One block of 64 state columns: ``d.N`` is 64; B, C, dB, dC have ``bc_pitch`` elements per row (128, or 256
-// when they point at one column block of N = 128 rows); every other tensor is dense.
-static int scan_tc_bwd_block(const void* U, const float* M, const float* K, const void* B, const void* C,
-                             const float* z0, const void* Bprev, const void* Uprev, const void* states_in,
-                             const float* zfinal_in, const void* dY, const float* dfinal, void* dU, float* dM,
-                             float* dK, void* dB, void* dC, float* dinit, void* dBprev, void* dUprev,
-                             const ScanDims& d, int io_dtype, void* ws, size_t ws_bytes, cudaStream_t st,
-                             int bc_pitch) {
+int run_bwd(const void* U, const float* M, const float* K, const void* B, const void* C, const float* z0,
+            const void* Bprev, const void* Uprev, const void* states_in, const float* zfinal_in, const void* dY,
+            const float* dfinal, void* dU, float* dM, float* dK, void* dB, void* dC, float* dinit, void* dBprev,
+            void* dUprev, const ScanDims& d, int io_dtype, uint8_t* w, cudaStream_t st) {
+  ensure_context();
   const TcBwdLayout lay = tc_bwd_layout(d);
-  if (!ws || ws_bytes < lay.total) return SL_ERR_WORKSPACE_TOO_SMALL;
-  uint8_t* w = reinterpret_cast<uint8_t*>(ws);
-  const bool bf = io_dtype == SL_BF16;
-  const uint64_t BH = (uint64_t)d.batch * d.heads, BG = (uint64_t)d.batch * d.groups;
-  const bool grouped = d.groups != d.heads;
+  const bool bf = io_dtype == SL_BF16, grouped = d.groups != d.heads;
+  const uint64_t BH = (uint64_t)d.batch * d.heads, BG = (uint64_t)d.batch * d.groups, W = 2 * (uint64_t)d.N;
+  const int nC = chunks_of(d), nb = blocks_of(d);
   void* dBh = grouped ? (void*)(w + lay.dbh) : dB;   // where the sweep stores dB / dC (per head)
   void* dCh = grouped ? (void*)(w + lay.dch) : dC;
-  const int nC = (d.T + L - 1) / L;
   const float* zfinal = zfinal_in;
   const void* states = states_in;
   if (!states || !zfinal) {   // nothing saved by the forward: recompute with the state pre-sweep
     float* zf = reinterpret_cast<float*>(w + lay.zfinal);
-    if (int e = scan_tc_fwd_impl(U, M, K, B, nullptr, z0, Bprev, Uprev, nullptr, zf, w + lay.states, d,
-                                 io_dtype, SL_F32, st, bc_pitch))
+    if (int e = scan_tc_fwd_impl(U, M, K, B, nullptr, z0, Bprev, Uprev, nullptr, zf, w + lay.states, d, fwd_plan(d),
+                                 w + lay.segs, io_dtype, SL_F32, st))
       return e;
     zfinal = zf;
     states = w + lay.states;
   }
+  const SegPlan plan = bwd_plan(d);
   TcBwdParams p{};
-  const uint64_t out_pitch = grouped ? 128 : bc_pitch;   // the per-head workspace is dense
-  if (!tc::make_tmap_3d(&p.tmU, U, 64, d.T, BH, 64, bf) ||
-      !tc::make_tmap_3d(&p.tmB, B, 128, d.T, BG, 64, bf, bc_pitch) ||
-      !tc::make_tmap_3d(&p.tmC, C, 128, d.T, BG, 64, bf, bc_pitch) ||
-      !tc::make_tmap_3d(&p.tmdY, dY, 64, d.T, BH, 64, bf) ||
-      !tc::make_tmap_3d(&p.tmZ, states, 128, (uint64_t)nC * 64, BH, 64, bf) ||
-      !tc::make_tmap_3d(&p.tmdU, dU, 64, d.T, BH, 64, bf) ||
-      !tc::make_tmap_3d(&p.tmdB, dBh, 128, d.T, BH, 64, bf, out_pitch) ||
-      !tc::make_tmap_3d(&p.tmdC, dCh, 128, d.T, BH, 64, bf, out_pitch))
+  if (!tc::make_tmap_3d(&p.tmU, U, 64, d.T, BH, 64, bf) || !tc::make_tmap_3d(&p.tmB, B, W, d.T, BG, 64, bf) ||
+      !tc::make_tmap_3d(&p.tmC, C, W, d.T, BG, 64, bf) || !tc::make_tmap_3d(&p.tmdY, dY, 64, d.T, BH, 64, bf) ||
+      !tc::make_tmap_3d(&p.tmZ, states, 128, (uint64_t)nC * 64, BH * nb, 64, bf) ||
+      !tc::make_tmap_3d(&p.tmdU[0], dU, 64, d.T, BH, 64, bf) ||
+      (nb == 2 && !tc::make_tmap_3d(&p.tmdU[1], w + lay.du2, 64, d.T, BH, 64, bf)) ||
+      !tc::make_tmap_3d(&p.tmdB, dBh, W, d.T, BH, 64, bf) || !tc::make_tmap_3d(&p.tmdC, dCh, W, d.T, BH, 64, bf))
     return SL_ERR_LAUNCH_FAILED;
   p.M = M; p.K = K; p.dfinal = dfinal; p.zfinal = zfinal;
   p.dg = reinterpret_cast<float2*>(w + lay.dg); p.sterm = reinterpret_cast<float2*>(w + lay.sterm);
@@ -450,41 +434,59 @@ static int scan_tc_bwd_block(const void* U, const float* M, const float* K, cons
   // with carried taps the adjoint of the start state is needed even when the caller asks for no d_initial
   float* dstart = dinit ? dinit : (Bprev ? reinterpret_cast<float*>(w + lay.dstart) : nullptr);
   float2* dgb = Bprev ? reinterpret_cast<float2*>(w + lay.dgb) : nullptr;
-  p.dinit = dstart; p.T = d.T; p.nchunks = nC; p.heads = d.heads; p.groups = d.groups;
+  p.dinit = dstart; p.T = d.T; p.N = d.N; p.nchunks = nC; p.cps = plan.cps; p.nseg = plan.nseg;
+  p.heads = d.heads; p.groups = d.groups;
   p.wait_limit = wait_limit_clocks();
-  int rc = SL_ERR_UNSUPPORTED;
-  rc = bf ? launch_tc_bwd<__nv_bfloat16>(p, (int)BH, st) : launch_tc_bwd<__half>(p, (int)BH, st);
-  if (rc != SL_OK) return rc;
+  if (plan.nseg > 1) {   // the adjoint at the end of every segment
+    const SegLayout sl = seg_layout(d, plan.nseg);
+    TcFwdParams q{};
+    q.tmU = p.tmdY; q.tmB = p.tmC;
+    q.M = M; q.K = K; q.heads = d.heads; q.groups = d.groups; q.T = d.T; q.N = d.N;
+    q.nchunks = nC; q.cps = plan.cps; q.nseg = plan.nseg; q.wait_limit = p.wait_limit;
+    q.seg = reinterpret_cast<float*>(w + lay.segs + sl.seg);
+    q.seg_pi = reinterpret_cast<float2*>(w + lay.segs + sl.pi);
+    if (int e = launch_prepass<TIn, 2>(q, (int)BH, nb, st)) return e;
+    p.fold = plan.nseg <= FOLD_SEGS;
+    if (!p.fold) {
+      scan_tc_combine_kernel<TIn, true><<<dim3((unsigned)BH, 16u * nb), 256, 0, st>>>(
+          q.seg, q.seg_pi, dfinal, nullptr, nullptr, M, K, d.heads, d.groups, d.T, d.N, nb, plan.nseg);
+      note_launches(1);
+    }
+    p.seg = q.seg; p.seg_pi = q.seg_pi;
+  }
+  {
+    auto k = scan_tc_bwd_kernel<TIn, 4>;
+    static std::atomic<unsigned long long> done{0};
+    if (int e = ensure_smem(k, B_SMEM_BYTES, done)) return e;
+    k<<<dim3((unsigned)BH, (unsigned)plan.nseg, (unsigned)nb), 576, B_SMEM_BYTES, st>>>(p);
+    note_launches(1);
+    if (int e = launch_status()) return e;
+  }
+  const TIn* bp = reinterpret_cast<const TIn*>(Bprev);
   if (Bprev) {
-    if (bf)
-      scan_tc_bwd_boundary_kernel<__nv_bfloat16><<<(unsigned)BG, 128, 0, st>>>(
-          dstart, (const __nv_bfloat16*)Bprev, (const __nv_bfloat16*)Uprev, M, K, (__nv_bfloat16*)dBprev,
-          (__nv_bfloat16*)dUprev, dgb, d.heads, d.groups, d.T);
-    else
-      scan_tc_bwd_boundary_kernel<__half><<<(unsigned)BG, 128, 0, st>>>(dstart, (const __half*)Bprev,
-                                                                       (const __half*)Uprev, M, K, (__half*)dBprev,
-                                                                       (__half*)dUprev, dgb, d.heads, d.groups, d.T);
+    scan_tc_bwd_boundary_kernel<TIn><<<(unsigned)BG, 256, 0, st>>>(
+        dstart, bp, reinterpret_cast<const TIn*>(Uprev), M, K, reinterpret_cast<TIn*>(dBprev),
+        reinterpret_cast<TIn*>(dUprev), dgb, d.heads, d.groups, d.T, d.N);
     note_launches(1);
   }
-  scan_tc_bwd_finish_kernel<<<dim3((unsigned)BH, (unsigned)((nC + 3) / 4)), 128, 0, st>>>(M, K, p.dg, p.sterm, p.dkcd, p.anchor, dgb, dM, dK, d.T, nC);
-  note_launches(2);
-  if (grouped) {
-    const size_t pieces = BG * (size_t)d.T * 16;
-    const unsigned blocks = (unsigned)((pieces + 255) / 256);
-    if (bf)
-      scan_tc_group_reduce_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(
-          (const __nv_bfloat16*)dBh, (const __nv_bfloat16*)dCh, (__nv_bfloat16*)dB, (__nv_bfloat16*)dC, d.heads,
-          d.groups, d.T, pieces, bc_pitch);
-    else
-      scan_tc_group_reduce_kernel<__half><<<blocks, 256, 0, st>>>((const __half*)dBh, (const __half*)dCh, (__half*)dB,
-                                                                 (__half*)dC, d.heads, d.groups, d.T, pieces,
-                                                                 bc_pitch);
-    note_launches(1);
-  }
+  TcPostParams q{};
+  q.M = M; q.K = K; q.dg = p.dg; q.sterm = p.sterm; q.dkcd = p.dkcd; q.anchor = p.anchor; q.dg_boundary = dgb;
+  q.dM = dM; q.dK = dK; q.dB = dB; q.dC = dC; q.dU = dU; q.dU2 = w + lay.du2;
+  q.per_head_b = dBh; q.per_head_c = dCh;
+  q.BH = (int)BH; q.heads = d.heads; q.groups = d.groups; q.T = d.T; q.nC = nC; q.D = (int)W;
+  q.fin_blocks = (unsigned)(BH * ((nC + 3) / 4));
+  q.red_blocks = grouped ? (unsigned)((BG * (size_t)d.T * (W / 8) + 127) / 128) : 0u;
+  const unsigned add_blocks = nb == 2 ? (unsigned)((BH * (size_t)d.T * 8 + 127) / 128) : 0u;
+  const unsigned blocks = q.fin_blocks + q.red_blocks + add_blocks;
+  if (nb == 1) scan_tc_bwd_post_kernel<TIn, 1><<<blocks, 128, 0, st>>>(q);
+  else scan_tc_bwd_post_kernel<TIn, 2><<<blocks, 128, 0, st>>>(q);
+  note_launches(1);
   return launch_status();
 }
 
+}  // namespace
 
+// A dY of another dtype than the operands (or none) takes the exact float32 sweeps.
 int scan_tc_bwd(const void* U, const float* M, const float* K, const void* B, const void* C,
                 const float* z0, const void* Bprev, const void* Uprev, const void* states_in,
                 const float* zfinal_in, const void* dY,
@@ -494,52 +496,13 @@ int scan_tc_bwd(const void* U, const float* M, const float* K, const void* B, co
   if (!dY || dy_dtype != io_dtype)
     return scan_simt_bwd(U, M, K, B, C, z0, Bprev, Uprev, dY, dfinal, dU, dM, dK, dB, dC, dinit, dBprev,
                          dUprev, d, io_dtype, dy_dtype, ws, ws_bytes, st);
-  if (d.N == 64)
-    return scan_tc_bwd_block(U, M, K, B, C, z0, Bprev, Uprev, states_in, zfinal_in, dY, dfinal, dU, dM, dK, dB,
-                             dC, dinit, dBprev, dUprev, d, io_dtype, ws, ws_bytes, st, 128);
-  // N = 128: one pass per column block.  dB, dC, d_initial and dB_prev are per block; dU, dM, dK and
-  // dU_prev are the sums of the passes (the second pass writes into the workspace and is added).
-  const TcBwdSplitLayout lay = tc_bwd_split_layout(d);
-  if (!ws || ws_bytes < lay.total) return SL_ERR_WORKSPACE_TOO_SMALL;
+  if (!ws || ws_bytes < tc_bwd_layout(d).total) return SL_ERR_WORKSPACE_TOO_SMALL;
   uint8_t* w = reinterpret_cast<uint8_t*>(ws);
-  const ScanDims d1 = one_block(d);
-  const size_t BH = (size_t)d.batch * d.heads, BG = (size_t)d.batch * d.groups;
-  const size_t st_bytes = scan_tc_states_bytes(d1), inner_bytes = tc_bwd_layout(d1).total;
-  const bool saved = states_in && zfinal_in;
-  for (int blk = 0; blk < 2; ++blk) {
-    float* z0b = z0 ? reinterpret_cast<float*>(w + lay.z0) : nullptr;
-    float* zfb = saved ? reinterpret_cast<float*>(w + lay.zf) : nullptr;
-    float* dfb = dfinal ? reinterpret_cast<float*>(w + lay.dfin) : nullptr;
-    float* dib = dinit ? reinterpret_cast<float*>(w + lay.dinit) : nullptr;
-    void* bpb = Bprev ? (void*)(w + lay.bprev) : nullptr;
-    void* dbpb = Bprev ? (void*)(w + lay.dbprev) : nullptr;
-    if (z0 && !copy_block_in(z0b, z0, blk, BH * 64, 4, st)) return SL_ERR_LAUNCH_FAILED;
-    if (saved && !copy_block_in(zfb, zfinal_in, blk, BH * 64, 4, st)) return SL_ERR_LAUNCH_FAILED;
-    if (dfinal && !copy_block_in(dfb, dfinal, blk, BH * 64, 4, st)) return SL_ERR_LAUNCH_FAILED;
-    if (Bprev && !copy_block_in(bpb, Bprev, blk, BG, 2, st)) return SL_ERR_LAUNCH_FAILED;
-    const void* stb = saved ? reinterpret_cast<const uint8_t*>(states_in) + blk * st_bytes : nullptr;
-    void* dUb = blk == 0 ? dU : (void*)(w + lay.du);
-    float* dMb = blk == 0 ? dM : reinterpret_cast<float*>(w + lay.dm);
-    float* dKb = blk == 0 ? dK : reinterpret_cast<float*>(w + lay.dk);
-    void* dUpb = !Uprev ? nullptr : (blk == 0 ? dUprev : (void*)(w + lay.duprev));
-    const int rc = scan_tc_bwd_block(U, M, K, block_of(B, blk), block_of(C, blk), z0b, bpb, Uprev, stb, zfb, dY, dfb,
-                                     dUb, dMb, dKb, const_cast<void*>(block_of(dB, blk)),
-                                     const_cast<void*>(block_of(dC, blk)), dib, dbpb, dUpb, d1, io_dtype,
-                                     w + lay.inner, inner_bytes, st, 256);
-    if (rc != SL_OK) return rc;
-    if (dinit && !copy_block_out(dinit, dib, blk, BH * 64, 4, st)) return SL_ERR_LAUNCH_FAILED;
-    if (Bprev && dBprev && !copy_block_out(dBprev, dbpb, blk, BG, 2, st)) return SL_ERR_LAUNCH_FAILED;
-  }
-  const bool bf = io_dtype == SL_BF16;
-  if (bf) add_into<__nv_bfloat16>(dU, w + lay.du, BH * (size_t)d.T * 64, st);
-  else add_into<__half>(dU, w + lay.du, BH * (size_t)d.T * 64, st);
-  add_into<float>(dM, w + lay.dm, BH * (size_t)d.T * 2, st);
-  add_into<float>(dK, w + lay.dk, BH * (size_t)d.T * 4, st);
-  if (Uprev && dUprev) {
-    if (bf) add_into<__nv_bfloat16>(dUprev, w + lay.duprev, BH * 64, st);
-    else add_into<__half>(dUprev, w + lay.duprev, BH * 64, st);
-  }
-  return launch_status();
+  return io_dtype == SL_BF16
+             ? run_bwd<__nv_bfloat16>(U, M, K, B, C, z0, Bprev, Uprev, states_in, zfinal_in, dY, dfinal, dU, dM, dK, dB, dC,
+                                      dinit, dBprev, dUprev, d, io_dtype, w, st)
+             : run_bwd<__half>(U, M, K, B, C, z0, Bprev, Uprev, states_in, zfinal_in, dY, dfinal, dU, dM, dK, dB, dC, dinit,
+                               dBprev, dUprev, d, io_dtype, w, st);
 }
 
 // The site code of the first expired wait on the current device since the last reset (0 = none).

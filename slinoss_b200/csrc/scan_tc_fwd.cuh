@@ -1,472 +1,603 @@
 // Forward kernel of the chunked scan on tcgen05 (included by scan_tc.cu inside its namespaces).
 //
-// NW = warps per TMEM lane quadrant (2 or 4).  The CTA has 4*NW worker warps; warp w reads TMEM
-// lanes 32*(w & 3) .. +31 (a hardware rule) and, inside every accumulator, the column group
-// (w >> 2) of NW.  All MMAs have M = 64, whose rows live in lanes 0..15 of every quadrant.  The
-// epilogues read them with the 16x256b shape of tcgen05.ld, which spreads those 16 lanes over all
-// 32 threads of the warp: thread t owns rows 16*quad + t/4 and + 8 and, in every block of 8
-// columns, the column pair 2*(t%4), 2*(t%4)+1 - a complex pair stays inside one thread.  Every
-// tcgen05.mma costs the tensor pipe >= 44 cycles whatever its N, so operands are laid out for few,
-// wide instructions: [K' ; Zv] is one 128-row B operand (scores and off-term in one MMA per
-// k-step) and K'' is one 128-column MN-major operand.
+// One CTA walks the chunks of one segment of one (batch, head) stream.  NB = 64-column blocks of the state
+// dimension held by the CTA (1: N <= 64, 2: N <= 128).  The CTA has 8 NB worker warps (4 TMEM lane quadrants x
+// 2 NB column groups), one scalar warp and one issue warp.
 //
-// STATES_ONLY: the state pre-sweep of the backward pass (no C, no scores, no Y).
-template <typename TIn, typename TY, bool STATES_ONLY, int NW>
-__global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_fwd_kernel(const __grid_constant__ TcFwdParams p) {
-  constexpr int NT = 128 * NW;  // worker threads; two more warps: per-chunk scalars, TMA + MMA issue
-  constexpr int ZC = 128 / NW;  // state columns per warp
-  constexpr int SC = 64 / NW;   // score / output columns per warp
-  constexpr int SB = SC / 8;    // 8-column blocks of a score / output group
-  constexpr int ZB = ZC / 8;    // 8-column blocks of a state group: 2 ZB state values per thread and row
-  constexpr int RSTEP = NT / 16;
+// MODE 0  full forward: Y, final state, optional 16-bit chunk-start states
+//      1  states only: chunk-start states / the end state of the segment (no C, no scores, no Y)
+//      2  adjoint states: the same walk backwards in time over C and dY, giving the adjoint of the segment's
+//         start state from a zero end adjoint (the pre-pass of a backward sweep that is split in time)
+//
+// What bounds it: the phases of a chunk (rotation, score product, masking, second product, state update) form
+// one dependent chain of about 5 k clocks, most of it latency; neither DRAM, the tensor pipe nor the issue
+// slots are full.  Hence two CTAs per SM for NB = 1 (80 KB of tiles, 256 TMEM columns, 96 registers): the
+// chain of one stream fills the waits of the other.  To fit twice, B and C are rotated in place in a single
+// stage that is refilled while the scores are masked, Y is staged over the score tile, and the second product
+// accumulates over the TMEM columns of the scores.
+//
+// Columns: inside every group of 16 real columns the 8 real parts precede the 8 imaginary parts (tiles K', Q,
+// Zv and the saved states), so that two neighbouring columns are the same part of two oscillators: all the
+// complex arithmetic of the passes and epilogues then runs on packed float32 pairs (fma.rn.f32x2).
+//
+// MMAs have M = 64 (rows in lanes 0..15 of every TMEM quadrant); the epilogues read them with the 16x256b shape
+// (thread t: rows t/4 and t/4 + 8 of the quadrant, column pair 2 (t%4) of every 8-column block).
+template <int NB, bool FULL>
+struct FwdSmem {
+  static constexpr uint32_t U = 0;                                   // two stages of U
+  static constexpr uint32_t KZ = 2 * TILE;                           // 2 NB x [K' ; Zv]
+  static constexpr uint32_t C = KZ + 4 * NB * TILE;                  // 2 NB x Q
+  static constexpr uint32_t UE = C + (FULL ? 2 * NB * TILE : 0);     // e^{l_end - l_s} U
+  static constexpr uint32_t S = UE + TILE;                           // scores, then Y
+  static constexpr uint32_t SCAL = S + (FULL ? TILE : 0);
+  static constexpr uint32_t BYTES = SCAL + 2 * SCW * 4 + NB * 64 * 4 + 1024;
+};
+
+struct alignas(64) TcFwdParams {
+  CUtensorMap tmU, tmB, tmC;   // MODE 2: dY, C, unused
+  CUtensorMap tmY, tmS;        // 16-bit output and chunk-state tensors (TMA stores); unused ones stay zero
+  const float* M;
+  const float* K;
+  const float* z0;      // (BH, 64, 2N) or null: start state of segment 0 (unless from_seg)
+  const void* Bprev;
+  const void* Uprev;
+  void* Y;
+  float* zfinal;        // (BH, 64, 2N) or null
+  void* states16;       // optional (NB, BH, nchunks, 64, 128) 16-bit: conjugated start state of every chunk
+  float* seg;           // (BH, nseg, 64, 128 NB) float32: start states (from_seg) or, MODE 1 / 2 pre-pass, results
+  float2* seg_pi;       // (BH, nseg): transition product of the segment (pre-pass)
+  int heads, groups, T, N, nchunks, cps, nseg, seg0;   // cps: chunks per segment; seg0: segment of blockIdx.y = 0
+  int from_seg;   // start states: 1 given in seg, 2 to be folded from the segments' contributions in seg
+  int to_seg;     // pre-pass: leave this segment's contribution in seg
+  long long wait_limit;  // SM clocks a wait of the main loop may take before the kernel gives up
+};
+
+template <typename TIn, typename TY, int MODE, int NB>
+__global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
+    scan_tc_fwd_kernel(const __grid_constant__ TcFwdParams p) {
+  constexpr bool FULL = MODE == 0, ADJ = MODE == 2;
+  using SM = FwdSmem<NB, FULL>;
+  constexpr int NWQ = 2 * NB;        // warps per TMEM lane quadrant
+  constexpr int NT = 128 * NWQ;      // worker threads
+  constexpr int SC = 64 / NWQ;       // score / output columns per warp
+  constexpr int SB = SC / 8;
+  constexpr uint32_t TM_COLS = FULL ? (NB == 1 ? 256 : 512) : 128 * NB;
+  constexpr uint32_t TM_INC = FULL ? 128 : 0;   // TMEM: [S, then Ydiag | Yoff] 0..127, Inc 128 NB columns
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  __shared__ uint64_t bar_tma[2], bar_mma[3], bar_drain;   // bar_mma: [S|Yoff] | Inc | Ydiag
-  __shared__ uint64_t bar_st;                  // Y tile staged in shared memory (16-bit outputs)
-  constexpr bool Y_TMA = !STATES_ONLY && sizeof(TY) == 2;
+  __shared__ uint64_t bar_u[2], bar_bc, bar_mma[3], bar_st, bar_sc, bar_drain;   // bar_mma: [S|Yoff] | Inc | Ydiag
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
-  float* sc_tab = reinterpret_cast<float*>(smem + OFF_SCAL);   // two tables: chunk parity
+  constexpr bool Y_TMA = FULL && sizeof(TY) == 2;
+  float* sc_tab = reinterpret_cast<float*>(smem + SM::SCAL);
+  float* s_diag = sc_tab + 2 * SCW;   // [NB][64] partial diagonal scores
   using PK = Pack2<TIn>;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool worker = warp < 4 * NW;     // warp 4 NW runs chunk_scalars one chunk ahead, warp 4 NW + 1 issues
+  const bool worker = warp < 4 * NWQ;
   const int quad = warp & 3, cg = worker ? (warp >> 2) : 0;
-  const int rowA = 16 * quad + (lane >> 2), rowB = rowA + 8;  // epilogue identity: two rows ...
-  const int cq = lane & 3;                                    // ... and one column pair per 8-column block
-  const int rcol = tid & 15, rrow0 = tid >> 4;               // rotation identity
+  const int rowA = 16 * quad + (lane >> 2), rowB = rowA + 8, cq = lane & 3;   // epilogue identity
+  const int rrow = (tid >> 2) & 63, rk = tid & 3, rgrp = (tid >> 8) & (NB - 1);   // rotation identity
   const uint32_t lane_base = (uint32_t)(32 * quad) << 16;
   const int bh = blockIdx.x, b = bh / p.heads, h = bh % p.heads;
   const int bg = b * p.groups + h / (p.heads / p.groups);
-  const int T = p.T;
+  const int seg = p.seg0 + blockIdx.y;
+  const int c0 = seg * p.cps, n = min(p.cps, p.nchunks - c0);   // this CTA's chunks: c0 .. c0 + n - 1
+  const int T = p.T, D = 2 * p.N;
   const float* Mb = p.M + (size_t)bh * T * 2;
   const float* Kb = p.K + (size_t)bh * T * 4;
-  const long long wl = p.wait_limit;   // limit of the main loop's waits (the drain waits keep the default)
+  const long long wl = p.wait_limit;
+  auto chunk_of = [&](int i) { return ADJ ? c0 + n - 1 - i : c0 + i; };
 
   if (tid == 0) {
-    mbar_init(&bar_tma[0], 1); mbar_init(&bar_tma[1], 1);
+    mbar_init(&bar_u[0], 1); mbar_init(&bar_u[1], 1); mbar_init(&bar_bc, 1);
     for (int i = 0; i < 3; ++i) mbar_init(&bar_mma[i], 1);
-    mbar_init(&bar_st, 4 * NW);   // one arrival per worker warp
+    mbar_init(&bar_st, 4 * NWQ);   // one arrival per worker warp
+    mbar_init(&bar_sc, 1);
     mbar_init(&bar_drain, 1);
     fence_barrier_init();
     s_abort = 0;
-    tma_prefetch_desc(&p.tmU); tma_prefetch_desc(&p.tmB); tma_prefetch_desc(&p.tmC);
-    if (Y_TMA) tma_prefetch_desc(&p.tmY);
-    if (p.states16) tma_prefetch_desc(&p.tmS);
   }
-  if (warp == 0) tmem_alloc(&tmem_slot, TMEM_COLS);
+  auto issue_u = [&](int i) {   // one thread
+    mbar_expect_tx(&bar_u[i & 1], TILE);
+    tma_load_3d(smem + SM::U + (i & 1) * TILE, &p.tmU, &bar_u[i & 1], 0, chunk_of(i) * L, bh);
+  };
+  auto issue_bc = [&](int i) {   // one thread
+    const int t0 = chunk_of(i) * L;
+    mbar_expect_tx(&bar_bc, (FULL ? 4 : 2) * NB * TILE);
+#pragma unroll
+    for (int q = 0; q < 2 * NB; ++q) {
+      tma_load_3d(smem + SM::KZ + 2 * q * TILE, &p.tmB, &bar_bc, 64 * q, t0, bg);
+      if (FULL) tma_load_3d(smem + SM::C + q * TILE, &p.tmC, &bar_bc, 64 * q, t0, bg);
+    }
+  };
+  if (warp == 0) {
+    tmem_alloc(&tmem_slot, TM_COLS);
+  } else if (warp == 4 * NWQ) {
+    chunk_scalars(sc_tab, Mb, Kb, chunk_of(0) * L, T, lane);
+  }
+  if (tid == 0) {   // (after the barriers were initialised by this same thread)
+    issue_bc(0);
+    issue_u(0);
+    if (n > 1) issue_u(1);
+  }
+
+  // ---- carried state, conjugated.  zz[2 j + hh]: 8-column block j of this warp's 64 columns, row (hh ? rowB :
+  // rowA), as a pair of neighbouring columns; even blocks hold real parts, odd blocks minus the imaginary parts
+  f2 zz[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) zz[j] = 0ull;
+  auto n_of = [&](int m) { return 32 * cg + 8 * m + 2 * cq; };   // oscillators n, n + 1 of block pair m
+  if (worker && !ADJ && !p.to_seg && p.from_seg != 1 && (p.z0 || p.Bprev)) {   // start state of the sequence
+    const TIn* Bp = reinterpret_cast<const TIn*>(p.Bprev);
+    const TIn* Up = reinterpret_cast<const TIn*>(p.Uprev);
+    float xr = 0.f, xi = 0.f, up[2] = {0.f, 0.f};
+    if (Bp) {  // pending prev-tap of the token before the sequence: u_prev (x) (kp_0 / m_0) b_prev
+      pending_tap(Mb, Kb, xr, xi);
+      up[0] = to_f32(Up[(size_t)bh * 64 + rowA]);
+      up[1] = to_f32(Up[(size_t)bh * 64 + rowB]);
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int nn = n_of(m);
+      if (nn >= p.N) continue;
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p.z0) z = *reinterpret_cast<const float4*>(p.z0 + ((size_t)bh * 64 + (hh ? rowB : rowA)) * D + 2 * nn);
+        if (Bp) {
+          const TIn* bp = Bp + (size_t)bg * D + 2 * nn;
+          const float b0r = to_f32(bp[0]), b0i = to_f32(bp[1]), b1r = to_f32(bp[2]), b1i = to_f32(bp[3]);
+          z.x += up[hh] * (xr * b0r - xi * b0i); z.y += up[hh] * (xr * b0i + xi * b0r);
+          z.z += up[hh] * (xr * b1r - xi * b1i); z.w += up[hh] * (xr * b1i + xi * b1r);
+        }
+        zz[4 * m + hh] = mk2(z.x, z.z);
+        zz[4 * m + 2 + hh] = mk2(-z.y, -z.w);
+      }
+    }
+  }
+  // start state of a later segment: given, or folded from the earlier segments' contributions
+  if (worker && p.from_seg) {
+    const size_t stride = (size_t)64 * 128 * NB;
+    const float* src = p.seg + (size_t)bh * p.nseg * stride + 64 * cg + 2 * cq;
+    const bool fold = p.from_seg == 2;
+    for (int s = fold ? 0 : seg; s < (fold ? seg : seg + 1); ++s) {
+      const float2 pi = fold ? p.seg_pi[(size_t)bh * p.nseg + s] : make_float2(0.f, 0.f);
+      const f2 pr = dup2(pi.x), pim = dup2(pi.y), npim = dup2(-pi.y);
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          const float* f = src + s * stride + (size_t)(hh ? rowB : rowA) * 128 * NB + 16 * m;
+          const float2 fr = *reinterpret_cast<const float2*>(f), fi = *reinterpret_cast<const float2*>(f + 8);
+          const f2 a = zz[4 * m + hh], c = zz[4 * m + 2 + hh];   // conj(Pi_s) z + F_s
+          zz[4 * m + hh] = fma2(pim, c, fma2(pr, a, mk2(fr.x, fr.y)));
+          zz[4 * m + 2 + hh] = fma2(npim, a, fma2(pr, c, mk2(fi.x, fi.y)));
+        }
+    }
+  }
+  // 16-bit copy of the state: rows p, K-major along d, directly below the K' rows of the same 64 columns, so that
+  // [K' ; Zv] is one 128-row operand
+  const bool keep_zv = FULL || p.states16 != nullptr;
+  auto store_zv_tile = [&]() {
+    uint8_t* tile = smem + SM::KZ + (2 * cg + 1) * TILE + 4 * cq;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      *reinterpret_cast<uint32_t*>(tile + sw128(rowA, j)) = PK::pack2(zz[2 * j]);
+      *reinterpret_cast<uint32_t*>(tile + sw128(rowB, j)) = PK::pack2(zz[2 * j + 1]);
+    }
+  };
+  auto store_states = [&](int i) {   // issue lane: the state tile of chunk i is exactly what the backward wants
+    const int c = chunk_of(i);
+#pragma unroll
+    for (int q = 0; q < 2 * NB; ++q)
+      tma_store_3d(&p.tmS, smem + SM::KZ + (2 * q + 1) * TILE, 64 * (q & 1), c * 64, (q >> 1) * (int)gridDim.x + bh);
+    tma_store_commit();
+  };
+  if (worker && keep_zv) { store_zv_tile(); fence_async_smem(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;
 
-  auto issue_loads = [&](int c) {   // one thread
-    uint8_t* st = smem + (c & 1) * STAGE;
-    uint64_t* bar = &bar_tma[c & 1];
-    mbar_expect_tx(bar, (STATES_ONLY ? 3 : 5) * TILE);
-    tma_load_3d(st, &p.tmU, bar, 0, c * L, bh);
-    tma_load_3d(st + TILE, &p.tmB, bar, 0, c * L, bg);
-    tma_load_3d(st + 3 * TILE, &p.tmB, bar, 64, c * L, bg);
-    if (!STATES_ONLY) {
-      tma_load_3d(st + 5 * TILE, &p.tmC, bar, 0, c * L, bg);
-      tma_load_3d(st + 6 * TILE, &p.tmC, bar, 64, c * L, bg);
-    }
+  // Bounded waits.  After the first expired one every warp keeps walking the chunk loop without working (named
+  // barriers have no time-out, so nobody may leave early); the other waits give up as soon as they see the flag.
+  auto wait_one = [&](uint64_t* bar, uint32_t parity, int code) {   // one thread
+    return mbar_try_wait(bar, parity) || wait_or_abort(bar, parity, wl, &s_abort, code);
   };
-  if (tid == 0) issue_loads(0);
-
-  // ---- carried state, conjugated: zv[2j], zv[2j+1] = (re, -im) of column pair j of this thread ----
-  const int d0 = cg * ZC;             // first state column (0..127) of this warp
-  // zv[4 i + 2 h + k]: block i, row (h ? rowB : rowA), k = 0 real part, 1 minus the imaginary part
-  float zv[4 * ZB];
-#pragma unroll
-  for (int j = 0; j < 4 * ZB; ++j) zv[j] = 0.f;
-  if (worker) {
-    const TIn* Bp = reinterpret_cast<const TIn*>(p.Bprev);
-    const TIn* Up = reinterpret_cast<const TIn*>(p.Uprev);
-    float cr = 0.f, ci = 0.f, up[2] = {0.f, 0.f};
-    if (Bp) {  // pending prev-tap of the token before the sequence: u_prev (x) (kp_0 / m_0) b_prev
-      const float mr = Mb[0], mi = Mb[1], kr = Kb[0], ki = Kb[1];
-      const float den = mr * mr + mi * mi;
-      cr = (kr * mr + ki * mi) / den; ci = (ki * mr - kr * mi) / den;
-      up[0] = to_f32(Up[(size_t)bh * 64 + rowA]);
-      up[1] = to_f32(Up[(size_t)bh * 64 + rowB]);
-    }
-#pragma unroll
-    for (int i = 0; i < ZB; ++i) {
-      const int d = d0 + 8 * i + 2 * cq;
-      float br = 0.f, bi = 0.f;
-      if (Bp) { br = to_f32(Bp[(size_t)bg * 128 + d]); bi = to_f32(Bp[(size_t)bg * 128 + d + 1]); }
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        float re = 0.f, im = 0.f;
-        if (p.z0) {
-          const float2 z = *reinterpret_cast<const float2*>(p.z0 + ((size_t)bh * 64 + (hh ? rowB : rowA)) * 128 + d);
-          re = z.x; im = z.y;
-        }
-        re += up[hh] * (cr * br - ci * bi);
-        im += up[hh] * (cr * bi + ci * br);
-        zv[4 * i + 2 * hh] = re; zv[4 * i + 2 * hh + 1] = -im;
-      }
-    }
-  }
-  // 16-bit copy of the state for chunk c: rows p, K-major along d, in the Zv slots of stage c & 1
-  // (directly below the K' rows, so that [K' ; Zv] is one 128-row operand)
-  auto store_zv_tile = [&](int c) {
-    uint8_t* stg = smem + (c & 1) * STAGE;
-#pragma unroll
-    for (int i = 0; i < ZB; ++i) {
-      const int ci = d0 / 8 + i;   // 16-byte chunk index along d (0..15)
-      uint8_t* tile = stg + (2 + 2 * (ci >> 3)) * TILE + 4 * cq;
-      *reinterpret_cast<uint32_t*>(tile + sw128(rowA, ci & 7)) = PK::pack(zv[4 * i], zv[4 * i + 1]);
-      *reinterpret_cast<uint32_t*>(tile + sw128(rowB, ci & 7)) = PK::pack(zv[4 * i + 2], zv[4 * i + 3]);
-    }
-  };
-  if (worker) store_zv_tile(0);
-  if (warp == 4 * NW) chunk_scalars(sc_tab, Mb, Kb, 0, T, lane);
-  __syncthreads();
-
-  constexpr uint32_t ID_S = make_idesc(64, 128, PK::fmt, 0, 0);    // K-major x K-major   [S | Yoff]
-  constexpr uint32_t ID_Y = make_idesc(64, 64, PK::fmt, 0, 1);     // K-major x MN-major  Ydiag
-  constexpr uint32_t ID_Z = make_idesc(64, 128, PK::fmt, 1, 1);    // MN-major x MN-major Inc
-  const uint32_t aKPP = smem_u32(smem + OFF_KPP), aS = smem_u32(smem + OFF_S);
-  bool ok = true;
-  int issued_hi = 0;   // issue lane: the last chunk whose loads were requested (chunk 0 by thread 0 above)
-
-  // ---- output epilogue of chunk cp: y = Y_diag + exp(l_t) Y_off.  It runs one iteration late, in the gap
-  // while the [S | Yoff] MMAs of the next chunk execute (their accumulators alternate by chunk parity).
-  float et_keep[2] = {0.f, 0.f};   // exp(l_t) of this thread's two rows in the chunk whose output is pending
-  auto output_epilogue = [&](int cp, bool live) {
-    float yadd[4 * SB];   // the summand of this thread's outputs, requested ahead of the wait
-#pragma unroll
-    for (int j = 0; j < 4 * SB; ++j) yadd[j] = 0.f;
-    if (!STATES_ONLY && p.Yadd != nullptr && live) {
-#pragma unroll
-      for (int i = 0; i < SB; ++i)
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const int t = cp * L + (hh ? rowB : rowA);
-          if (t < T) {
-            const float2 a = __ldg(reinterpret_cast<const float2*>(
-                p.Yadd + ((size_t)bh * T + t) * 64 + cg * SC + 8 * i + 2 * cq));
-            yadd[4 * i + 2 * hh] = a.x; yadd[4 * i + 2 * hh + 1] = a.y;
-          }
-        }
-    }
-    if (live && !mbar_wait(&bar_mma[2], cp & 1, wl)) { report_timeout(4); s_abort = 1; live = false; }
-    tc_fence_after_sync();
-    if (live) {
-      const int t0p = cp * L;
-      uint32_t yd[4 * SB], yo[4 * SB];
-      tmem_ld_16x256<SB>(tmem + lane_base + 256 + 64 * (cp & 1) + cg * SC, yd);
-      tmem_ld_16x256<SB>(tmem + lane_base + 128 * (cp & 1) + 64 + cg * SC, yo);
-      tmem_ld_wait();
-#pragma unroll
-      for (int i = 0; i < SB; ++i) {
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const int R = hh ? rowB : rowA;
-          const float et = hh ? et_keep[1] : et_keep[0];
-          const float y0 = __uint_as_float(yd[4 * i + 2 * hh]) + et * __uint_as_float(yo[4 * i + 2 * hh]) +
-                           yadd[4 * i + 2 * hh];
-          const float y1 = __uint_as_float(yd[4 * i + 2 * hh + 1]) + et * __uint_as_float(yo[4 * i + 2 * hh + 1]) +
-                           yadd[4 * i + 2 * hh + 1];
-          if constexpr (sizeof(TY) == 2) {   // into the staging tile; rows beyond T are clipped by the store
-            *reinterpret_cast<uint32_t*>(smem + OFF_Y + sw128(R, cg * SB + i) + 4 * cq) = Pack2<TY>::pack(y0, y1);
-          } else if (t0p + R < T) {
-            float* dst = reinterpret_cast<float*>(p.Y) + ((size_t)bh * T + t0p + R) * 64 + cg * SC + 8 * i + 2 * cq;
-            *reinterpret_cast<float2*>(dst) = make_float2(y0, y1);
-          }
-        }
-      }
-    }
-    if (Y_TMA) {   // the Y tile is complete once every worker warp has arrived
-      fence_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_st);
-    }
+  auto wait_warp = [&](uint64_t* bar, uint32_t parity, int code) {  // a converged warp
+    return __all_sync(0xffffffffu, wait_one(bar, parity, code)) != 0;
   };
 
-  for (int c = 0; c < p.nchunks && ok; ++c) {
-    const int t0 = c * L;
-    uint8_t* st = smem + (c & 1) * STAGE;
-    float* sc = sc_tab + (c & 1) * (NSCAL * 64);
-    float* s_diag = sc + 11 * 64;
-    if (warp == 4 * NW) {
-      // scalars of the NEXT chunk, started once the workers are through the rotation pass (global
-      // loads issued during the workers' shared-memory burst at the top of the iteration stalled
-      // the whole SM for about a DRAM round trip)
-      bar_sync(2, NT + 64);   // the workers only arrive here (bar_arrive): they never wait for this warp
-      if (c + 1 < p.nchunks) chunk_scalars(sc_tab + ((c + 1) & 1) * (NSCAL * 64), Mb, Kb, t0 + L, T, lane);
-    } else if (!worker) {
-      // Issue warp (one lane): the MMAs of this chunk, the TMA loads of the NEXT one and the TMA
-      // stores.  The workers never wait for this warp, only for the commit barriers of the products
-      // they read: they arrive on named barriers 2 ("rotation done") and 4 ("S tile written") without
-      // waiting and move on.
-      const uint64_t bU = make_desc(smem_u32(st), 8192, 1024);
-      const uint32_t tSY = tmem + 128 * (c & 1), tYD = tmem + 256 + 64 * (c & 1), tINC = tmem + 384;
-      // scores and off-term: [S | Yoff] = Q [K' ; Zv]^T, accumulated over the state dimension
-      const uint64_t bB = make_desc(smem_u32(st + TILE), 16, 1024);       // [K'_h ; Zv_h], h = k >> 2
-      const uint64_t bC = make_desc(smem_u32(st + 5 * TILE), 16, 1024);   // Q
-      if (lane == 0 && s_abort == 0 && c + 1 < p.nchunks) {
-        // Next chunk's tiles, a whole iteration ahead (half an iteration was not always enough for the data
-        // to arrive).  The stage being refilled held chunk c-1, whose last reader is its Y_diag MMA.
-        if (!STATES_ONLY && c > 0 && !mbar_wait(&bar_mma[2], (c - 1) & 1, wl)) { report_timeout(8); s_abort = 1; }
-        else { issue_loads(c + 1); issued_hi = c + 1; }
+  if (warp == 4 * NWQ) {
+    // ---- scalar warp: the per-chunk tables, one chunk ahead ------------------------------------------------
+    float pr = 1.f, pi = 0.f;   // transition product of the segment
+    for (int i = 0; i < n; ++i) {
+      if (p.to_seg) {
+        const float* tail = sc_tab + (i & 1) * SCW + SC_TAIL;
+        const float mr = tail[0] * tail[1], mi = tail[0] * tail[2];
+        const float nr = pr * mr - pi * mi;
+        pi = pr * mi + pi * mr; pr = nr;
       }
-      __syncwarp();
-      bar_sync(5, NT + 32);   // first column halves of Q and K' rotated (the Zv tile is the previous chunk's)
-      if (!STATES_ONLY && lane == 0 && s_abort == 0) {
-        tc_fence_after_sync();
+      bar_sync(2, NT + 64);   // the workers are through the previous chunk, whose table is overwritten now
+      if (i + 1 < n) {
+        chunk_scalars(sc_tab + ((i + 1) & 1) * SCW, Mb, Kb, chunk_of(i + 1) * L, T, lane);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_sc);
+      }
+    }
+    if (p.to_seg && lane == 0) p.seg_pi[(size_t)bh * p.nseg + seg] = make_float2(pr, pi);
+  } else if (!worker) {
+    // ---- issue warp (one lane): every TMA load and store and every MMA.  The workers never wait for it, only for
+    // the commit barriers of the products they read.
+    constexpr uint32_t ID_S = make_idesc(64, 128, PK::fmt, 0, 0);        // K-major x K-major   [S | Yoff]
+    constexpr uint32_t ID_Y = make_idesc(64, 64, PK::fmt, 0, 1);         // K-major x MN-major  Ydiag
+    constexpr uint32_t ID_Z = make_idesc(64, 128 * NB, PK::fmt, 1, 1);   // MN-major x MN-major Inc
+    const uint64_t dKZ = make_desc(smem_u32(smem + SM::KZ), 16, 1024);
+    const uint64_t dQ = make_desc(smem_u32(smem + SM::C), 16, 1024);
+    const uint64_t dKm = make_desc(smem_u32(smem + SM::KZ), 2 * TILE, 1024);   // 64-column blocks two tiles apart
+    const uint64_t dUE = make_desc(smem_u32(smem + SM::UE), TILE, 1024);
+    const uint64_t dS = make_desc(smem_u32(smem + SM::S), 16, 1024);
+    int req_u = min(n, 2), req_bc = 1;   // loads requested so far
+    auto scores = [&](int half) {        // [S | Yoff] = Q [K' ; Zv]^T over the even / odd 64-column tiles
+#pragma unroll
+      for (int q = half; q < 2 * NB; q += 2)
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          umma(tSY, desc_adv(bC, k * 32), desc_adv(bB, k * 32), ID_S, k > 0);
+          umma(tmem, desc_adv(dQ, q * TILE + 32 * k), desc_adv(dKZ, 2 * q * TILE + 32 * k), ID_S, q + k > 0);
+    };
+    if (lane == 0 && p.states16) store_states(0);
+    for (int i = 0; i < n; ++i) {
+      const bool lead = lane == 0;
+      if (FULL) {
+        bar_sync(5, NT + 32);   // even tiles of Q and K' rotated
+        if (lead && !s_abort) { tc_fence_after_sync(); scores(0); }
+        __syncwarp();
       }
-      __syncwarp();
-      bar_sync(2, NT + 64);   // rotation done: Q, K', K'' written; U landed; Zv tile stored by the previous chunk
-      const bool go = lane == 0 && s_abort == 0;
-      if (go) {
+      bar_sync(2, NT + 64);     // rotation done
+      if (lead && !s_abort) {
         tc_fence_after_sync();
-        if (!STATES_ONLY) {
-#pragma unroll
-          for (int k = 4; k < 8; ++k)
-            umma(tSY, desc_adv(bC, TILE + (k & 3) * 32), desc_adv(bB, 2 * TILE + (k & 3) * 32), ID_S, 1);
+        if (FULL) {
+          scores(1);
+          tma_store_wait_read();   // the score tile still holds the previous Y, the Zv tiles the saved state
           umma_commit(&bar_mma[0]);
         }
-        // Inc = U^T K''
-        const uint64_t bK = make_desc(aKPP, 8192, 1024);
+        // Inc = (e^{l_end - l_s} U)^T K'
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          umma(tINC, desc_adv(bU, 2048 * k), desc_adv(bK, 2048 * k), ID_Z, k > 0);
+        for (int k = 0; k < 4; ++k) umma(tmem + TM_INC, desc_adv(dUE, 2048 * k), desc_adv(dKm, 2048 * k), ID_Z, k > 0);
+        if (!FULL) tma_store_wait_read();
         umma_commit(&bar_mma[1]);
-        if (p.states16) {   // the 16-bit state tile of this chunk is exactly what the backward wants
-          tma_store_3d(&p.tmS, st + 2 * TILE, 0, c * 64, bh);
-          tma_store_3d(&p.tmS, st + 4 * TILE, 64, c * 64, bh);
-          tma_store_commit();
-        }
-        if (Y_TMA && c > 0) {   // the workers stage the Y tile of the PREVIOUS chunk while the MMAs above run
-          if (mbar_wait(&bar_st, (c - 1) & 1, wl)) {
-            tma_store_3d(&p.tmY, smem + OFF_Y, 0, t0 - L, bh);
-            tma_store_commit();
-          } else { report_timeout(5); s_abort = 1; }
+        // refill B and C as soon as their last products are done: what is left of the iteration hides the load
+        if (i + 1 < n && wait_one(&bar_mma[1], i & 1, 8)) {
+          issue_bc(i + 1); ++req_bc;
+          if (!FULL && i + 2 < n) { issue_u(i + 2); ++req_u; }
         }
       }
       __syncwarp();
-      if (!STATES_ONLY) bar_sync(4, NT + 32);   // S tile written
-      if (go && s_abort == 0) {
-        if (!STATES_ONLY) {
+      if (FULL) {
+        bar_sync(4, NT + 32);   // S tile written
+        if (lead && !s_abort) {
           tc_fence_after_sync();
-          const uint64_t bS = make_desc(aS, 16, 1024);
+          const uint64_t dU = make_desc(smem_u32(smem + SM::U + (i & 1) * TILE), TILE, 1024);
 #pragma unroll
-          for (int k = 0; k < 4; ++k)   // Y_diag = S U
-            umma(tYD, desc_adv(bS, 32 * k), desc_adv(bU, 2048 * k), ID_Y, k > 0);
+          for (int k = 0; k < 4; ++k) umma(tmem, desc_adv(dS, 32 * k), desc_adv(dU, 2048 * k), ID_Y, k > 0);   // S U
           umma_commit(&bar_mma[2]);
         }
-        // the state tiles and the Y tile stored in this iteration are overwritten by the workers in
-        // the next one: their stores must have read them by then (they were issued long ago)
-        tma_store_wait_read();
+      }
+      if (lead && !s_abort && (FULL || p.states16) && wait_one(&bar_st, i & 1, 5)) {
+        if (Y_TMA) {
+          tma_store_3d(&p.tmY, smem + SM::S, 0, chunk_of(i) * L, bh);
+          tma_store_commit();
+        }
+        if (p.states16 && i + 1 < n) store_states(i + 1);
+        if (FULL && i + 2 < n) { issue_u(i + 2); ++req_u; }
       }
       __syncwarp();
-    } else {
-    bool live = true;   // cleared when a bounded wait expired: the rest of the chunk is skipped
-    if (!mbar_wait(&bar_tma[c & 1], (c >> 1) & 1, wl)) { report_timeout(1); s_abort = 1; live = false; }
+    }
+    if (lane == 0) {
+      // Unwind: nothing of this CTA may still be in flight when shared memory and TMEM are released.
+      if (s_abort) {
+        mbar_wait(&bar_bc, (req_bc - 1) & 1);
+        for (int i = max(0, req_u - 2); i < req_u; ++i) mbar_wait(&bar_u[i & 1], (i >> 1) & 1);
+      }
+      umma_commit(&bar_drain);
+      mbar_wait(&bar_drain, 0);
+      tma_store_wait_all();
+    }
+    __syncwarp();
+  } else {
+    // ---- worker warps ---------------------------------------------------------------------------------------
+    bool live = true;   // warp-uniform; cleared when a wait expired
+    for (int i = 0; i < n; ++i) {
+      const float* sc = sc_tab + (i & 1) * SCW;
+      const float4* rot = reinterpret_cast<const float4*>(sc);
+      const float4* kcl = reinterpret_cast<const float4*>(sc + SC_KCL);
+      if (i > 0) live = live && wait_warp(&bar_sc, (i - 1) & 1, 9);
+      live = live && wait_warp(&bar_bc, i & 1, 1);
 
-    // ---- rotation: C -> Q, B -> K' (both in place), K'' ; diagonal scores --------------------
-    // Two phases, one per 64-column half of the state dimension: the score products accumulate over
-    // that dimension, so the issue warp starts their first four k-steps (named barrier 5) while the
-    // workers still rotate the second half.  A thread keeps its rows in both phases (8 threads per
-    // row, one 16-byte piece each), so the diagonal sums stay in registers until the end.
-    {
-      constexpr int IPT = 512 / NT;   // (row, piece) items per thread and phase
-      float dgk[IPT];
+      // ---- rotation: C -> Q, B -> K' (in place), diagonal scores.  A thread owns 32 bytes (8 oscillators) of a
+      // row in each of two tiles; the score products of the first tile start while the second is rotated.
+      {
+        const uint32_t o0 = sw128(rrow, 2 * rk), o1 = sw128(rrow, 2 * rk + 1);
+        const float4 rt = rot[rrow];   // phi, w
+        f2 dr = 0ull, di0 = 0ull, di1 = 0ull;   // sums of Re conj(c) b and of the two parts of Im conj(c) b
 #pragma unroll
-      for (int j = 0; j < IPT; ++j) dgk[j] = 0.f;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        if (live) {
-          uint8_t* tB = st + (1 + 2 * half) * TILE;
-          uint8_t* tC = st + (5 + half) * TILE;
-          uint8_t* tK = smem + OFF_KPP + half * TILE;
-          uint4 cvk[IPT], bvk[IPT];
-#pragma unroll
-          for (int j = 0; j < IPT; ++j) {   // all loads first: the stores below are in place
-            const int item = tid + NT * j;
-            const uint32_t off = sw128(item >> 3, item & 7);
-            cvk[j] = make_uint4(0u, 0u, 0u, 0u);
-            if (!STATES_ONLY) cvk[j] = *reinterpret_cast<const uint4*>(tC + off);
-            bvk[j] = *reinterpret_cast<const uint4*>(tB + off);
-          }
-#pragma unroll
-          for (int j = 0; j < IPT; ++j) {
-            const int item = tid + NT * j, r = item >> 3;
-            const uint32_t off = sw128(r, item & 7);
-            const float phr = sc[2 * 64 + r], phi = sc[3 * 64 + r];
-            const float wr = sc[4 * 64 + r], wi = sc[5 * 64 + r];
-            const float vr = sc[6 * 64 + r], vi = sc[7 * 64 + r];
-            const float kr = sc[8 * 64 + r], ki = sc[9 * 64 + r];
-            const uint4 cv = cvk[j], bv = bvk[j];
-            const uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w}, bw[4] = {bv.x, bv.y, bv.z, bv.w};
-            uint32_t qo[4], ko[4], vo[4];
-            float dg = 0.f;
+        for (int half = 0; half < 2; ++half) {
+          if (live) {
+            uint8_t* tB = smem + SM::KZ + 2 * (2 * rgrp + half) * TILE;
+            uint8_t* tC = smem + SM::C + (2 * rgrp + half) * TILE;
+            const uint4 b0 = *reinterpret_cast<const uint4*>(tB + o0), b1 = *reinterpret_cast<const uint4*>(tB + o1);
+            uint4 x0 = make_uint4(0u, 0u, 0u, 0u), x1 = x0;
+            if (FULL) { x0 = *reinterpret_cast<const uint4*>(tC + o0); x1 = *reinterpret_cast<const uint4*>(tC + o1); }
+            const uint32_t bw[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+            const uint32_t cw[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+            uint32_t kr[4], ki[4], qr[4], qi[4];
+            const f2 phr = dup2(rt.x), phi = dup2(rt.y), nphr = dup2(-rt.x);
+            const f2 wr = dup2(rt.z), nwr = dup2(-rt.z), nwi = dup2(-rt.w);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              const float2 cc = PK::unpack(cw[e]), bb = PK::unpack(bw[e]);
-              qo[e] = PK::pack(cc.x * phr + cc.y * phi, cc.x * phi - cc.y * phr);     // conj(c) phi
-              ko[e] = PK::pack(wr * bb.x - wi * bb.y, -(wr * bb.y + wi * bb.x));      // conj(w b)
-              vo[e] = PK::pack(vr * bb.x - vi * bb.y, -(vr * bb.y + vi * bb.x));      // conj(v b)
-              const float xr = kr * bb.x - ki * bb.y, xi = kr * bb.y + ki * bb.x;     // kc b
-              dg += cc.x * xr + cc.y * xi;                                            // Re(conj(c) kc b)
+              f2 br, bi;
+              PK::split(bw[2 * e], bw[2 * e + 1], br, bi);
+              if (ADJ) {   // B is the C operand here: q = conj(c) phi
+                kr[e] = PK::pack2(fma2(bi, phi, mul2(br, phr)));
+                ki[e] = PK::pack2(fma2(bi, nphr, mul2(br, phi)));
+              } else {     // k' = conj(w b)
+                kr[e] = PK::pack2(fma2(bi, nwi, mul2(br, wr)));
+                ki[e] = PK::pack2(fma2(bi, nwr, mul2(br, nwi)));
+              }
+              if (FULL) {
+                f2 cr, ci;
+                PK::split(cw[2 * e], cw[2 * e + 1], cr, ci);
+                qr[e] = PK::pack2(fma2(ci, phi, mul2(cr, phr)));    // q = conj(c) phi
+                qi[e] = PK::pack2(fma2(ci, nphr, mul2(cr, phi)));
+                dr = fma2(cr, br, dr); dr = fma2(ci, bi, dr);
+                di0 = fma2(cr, bi, di0); di1 = fma2(ci, br, di1);
+              }
             }
-            dgk[j] += dg;
-            *reinterpret_cast<uint4*>(tK + off) = make_uint4(vo[0], vo[1], vo[2], vo[3]);
-            if (!STATES_ONLY) {
-              *reinterpret_cast<uint4*>(tC + off) = make_uint4(qo[0], qo[1], qo[2], qo[3]);
-              *reinterpret_cast<uint4*>(tB + off) = make_uint4(ko[0], ko[1], ko[2], ko[3]);
+            *reinterpret_cast<uint4*>(tB + o0) = make_uint4(kr[0], kr[1], kr[2], kr[3]);
+            *reinterpret_cast<uint4*>(tB + o1) = make_uint4(ki[0], ki[1], ki[2], ki[3]);
+            if (FULL) {
+              *reinterpret_cast<uint4*>(tC + o0) = make_uint4(qr[0], qr[1], qr[2], qr[3]);
+              *reinterpret_cast<uint4*>(tC + o1) = make_uint4(qi[0], qi[1], qi[2], qi[3]);
             }
           }
-        }
-        if (half == 0) {   // first halves of Q and K' are complete: the score products may start
-          fence_async_smem();
-          tc_fence_before_sync();
-          bar_arrive(5, NT + 32);
-        }
-      }
-      if (live && !STATES_ONLY) {
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) {
-#pragma unroll
-          for (int j = 0; j < IPT; ++j) dgk[j] += __shfl_xor_sync(0xffffffffu, dgk[j], o);
-        }
-        if ((tid & 7) == 0) {
-#pragma unroll
-          for (int j = 0; j < IPT; ++j) s_diag[(tid + NT * j) >> 3] = dgk[j];
-        }
-      }
-    }
-    fence_async_smem();
-    tc_fence_before_sync();
-    // no barrier among the workers here: what a warp does next (the previous chunk's output, its decay
-    // factors) touches nothing the rotation of another warp reads or writes; the diagonal values of
-    // other warps are read after the score products' barrier, which all rotations precede
-    bar_arrive(2, NT + 64);      // the scalar and issue warps are told without being waited for
-    live = s_abort == 0;
-
-    if (!STATES_ONLY) {
-      // ---- [S | Yoff] and Inc MMAs are issued by the issue warp; meanwhile the output of the previous
-      // chunk is finished ---------------------------------------------------------------------------------
-      if (c > 0) output_epilogue(c - 1, live);
-      live = live && s_abort == 0;
-      // The wait and the TMEM load below are compiler barriers: what the scores epilogue reads from
-      // shared memory (and the exponentials of it) is computed BEFORE the wait it would otherwise
-      // queue behind.
-      float dfac[4 * SB], dg2[2];   // decay factors of this thread's cells [hh][i][q]; diagonal values
-      {
-        float ls[2 * SB];
-#pragma unroll
-        for (int i = 0; i < SB; ++i) {
-          const float2 l2 = *reinterpret_cast<const float2*>(sc + cg * SC + 8 * i + 2 * cq);
-          ls[2 * i] = l2.x; ls[2 * i + 1] = l2.y;
-        }
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const int R = hh ? rowB : rowA;
-          const float lt = sc[R];
-#pragma unroll
-          for (int k = 0; k < 2 * SB; ++k) dfac[hh * 2 * SB + k] = __expf(fminf(lt - ls[k], 0.f));
-        }
-      }
-      const float et_next[2] = {sc[1 * 64 + rowA], sc[1 * 64 + rowB]};
-      if (live && !mbar_wait(&bar_mma[0], c & 1, wl)) { report_timeout(2); s_abort = 1; live = false; }
-      tc_fence_after_sync();
-
-      // ---- scores epilogue: decay, causal mask, diagonal -> 16-bit S tile ------------------------
-      if (live) {
-        uint32_t r[4 * SB];
-        tmem_ld_16x256<SB>(tmem + lane_base + 128 * (c & 1) + cg * SC, r);
-        tmem_ld_wait();
-        et_keep[0] = et_next[0]; et_keep[1] = et_next[1];
-        dg2[0] = s_diag[rowA]; dg2[1] = s_diag[rowB];
-        uint8_t* tS = smem + OFF_S + 4 * cq;
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const int R = hh ? rowB : rowA;
-          const float dgv = dg2[hh];
-#pragma unroll
-          for (int i = 0; i < SB; ++i) {
-            float v2[2];
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const int s = cg * SC + 8 * i + 2 * cq + q;
-              float v = __uint_as_float(r[4 * i + 2 * hh + q]) * dfac[hh * 2 * SB + 2 * i + q];
-              v = s < R ? v : (s == R ? dgv : 0.f);
-              v2[q] = v;
-            }
-            *reinterpret_cast<uint32_t*>(tS + sw128(R, cg * SB + i)) = PK::pack(v2[0], v2[1]);
+          if (FULL && half == 0) {
+            fence_async_smem();
+            tc_fence_before_sync();
+            bar_arrive(5, NT + 32);
           }
+        }
+        live = live && wait_warp(&bar_u[i & 1], (i >> 1) & 1, 10);
+        if (live) {   // Ue = e^{l_end - l_s} U   (MODE 2: e^{l_t} dY)
+          const uint8_t* tU = smem + SM::U + (i & 1) * TILE;
+#pragma unroll
+          for (int j = 0; j < 512 / NT; ++j) {
+            const int item = tid + NT * j, r = item >> 3;
+            const uint32_t off = sw128(r, item & 7);
+            const uint4 uv = *reinterpret_cast<const uint4*>(tU + off);
+            const f2 ee = dup2(ADJ ? kcl[r].z : kcl[r].w);
+            *reinterpret_cast<uint4*>(smem + SM::UE + off) =
+                make_uint4(PK::pack2(mul2(PK::natural(uv.x), ee)), PK::pack2(mul2(PK::natural(uv.y), ee)),
+                           PK::pack2(mul2(PK::natural(uv.z), ee)), PK::pack2(mul2(PK::natural(uv.w), ee)));
+          }
+        }
+        if (FULL && live) {   // Re(conj(c) kc b) = kc_r Re(conj(c) b) - kc_i Im(conj(c) b), summed over the row
+          const float4 kc = kcl[rrow];
+          const float2 a = un2(dr), c = un2(di0), d = un2(di1);
+          float dg = kc.x * (a.x + a.y) - kc.y * ((c.x + c.y) - (d.x + d.y));
+          dg += __shfl_xor_sync(0xffffffffu, dg, 1);
+          dg += __shfl_xor_sync(0xffffffffu, dg, 2);
+          if (rk == 0) s_diag[rgrp * 64 + rrow] = dg;
         }
       }
       fence_async_smem();
       tc_fence_before_sync();
-      bar_arrive(4, NT + 32);   // the issue warp now issues Y_diag = S U (no barrier among the workers)
-      live = s_abort == 0;
-    }
+      bar_arrive(2, NT + 64);
 
-    // ---- state update (hides the Y_diag MMAs; the output epilogue follows in the next iteration) ---------
-    if (live && !mbar_wait(&bar_mma[1], c & 1, wl)) { report_timeout(3); s_abort = 1; live = false; }
-    tc_fence_after_sync();
-    // ---- state update: zv = conj(Pi_end) zv + Inc ---------------------------------------------------
-    if (live) {
-      const float pr = sc[10 * 64 + 0], pi = sc[10 * 64 + 1];
+      if (FULL) {
+        // ---- scores epilogue: decay, causal mask, diagonal -> 16-bit S tile.  The decay factors are computed ahead
+        // of the wait (waits and TMEM loads are compiler barriers); a warp whose cells all lie above the diagonal
+        // only writes zeros.
+        const bool empty = SC * cg > 16 * quad + 15;
+        float dfac[4 * SB];   // [hh][i][q]
+        if (!empty) {
+          float ls[2 * SB];
 #pragma unroll
-      for (int part = 0; part < ZB / 4; ++part) {
-        uint32_t inc[16];
-        tmem_ld_16x256<4>(tmem + lane_base + 384 + d0 + 32 * part, inc);
-        tmem_ld_wait();
+          for (int k = 0; k < SB; ++k) {
+            const float2 l2 = *reinterpret_cast<const float2*>(sc + SC_L2 + cg * SC + 8 * k + 2 * cq);
+            ls[2 * k] = l2.x; ls[2 * k + 1] = l2.y;
+          }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {   // 8 complex values: 4 blocks x 2 rows
-          const float a = zv[16 * part + 2 * j], bq = zv[16 * part + 2 * j + 1];
-          zv[16 * part + 2 * j] = pr * a + pi * bq + __uint_as_float(inc[2 * j]);
-          zv[16 * part + 2 * j + 1] = pr * bq - pi * a + __uint_as_float(inc[2 * j + 1]);
+          for (int hh = 0; hh < 2; ++hh) {
+            const float lt = sc[SC_L2 + (hh ? rowB : rowA)];
+#pragma unroll
+            for (int k = 0; k < 2 * SB; ++k) dfac[hh * 2 * SB + k] = ex2f(fminf(lt - ls[k], 0.f));
+          }
+        }
+        live = live && wait_warp(&bar_mma[0], i & 1, 2);
+        tc_fence_after_sync();
+        if (live) {
+          uint32_t r[4 * SB];
+          float dg2[2] = {0.f, 0.f};
+          if (!empty) {
+            tmem_ld_16x256<SB>(tmem + lane_base + cg * SC, r);
+            tmem_ld_wait();
+            dg2[0] = s_diag[rowA]; dg2[1] = s_diag[rowB];
+            if (NB == 2) { dg2[0] += s_diag[64 + rowA]; dg2[1] += s_diag[64 + rowB]; }
+          }
+          uint8_t* tS = smem + SM::S + 4 * cq;
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            const int R = hh ? rowB : rowA;
+#pragma unroll
+            for (int k = 0; k < SB; ++k) {
+              uint32_t word = 0u;
+              if (!empty) {
+                float v2[2];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                  const int s = cg * SC + 8 * k + 2 * cq + q;
+                  const float v = __uint_as_float(r[4 * k + 2 * hh + q]) * dfac[hh * 2 * SB + 2 * k + q];
+                  v2[q] = s < R ? v : (s == R ? dg2[hh] : 0.f);
+                }
+                word = PK::pack(v2[0], v2[1]);
+              }
+              *reinterpret_cast<uint32_t*>(tS + sw128(R, cg * SB + k)) = word;
+            }
+          }
+        }
+        fence_async_smem();
+        tc_fence_before_sync();
+        bar_arrive(4, NT + 32);
+      }
+
+      // ---- state update: zv = conj(u_end) (e^{l_end} zv + Inc);  MODE 2: dz = e^{l_end} (u_end dz) + Inc -----------
+      live = live && wait_warp(&bar_mma[1], i & 1, 3);
+      tc_fence_after_sync();
+      if (live) {
+        const float e_end = sc[SC_TAIL], ur = sc[SC_TAIL + 1], ui = sc[SC_TAIL + 2];
+        const f2 E = dup2(e_end), R = dup2(ADJ ? e_end * ur : ur), I = dup2(ADJ ? e_end * ui : ui);
+        const f2 NI = dup2(ADJ ? -e_end * ui : -ui);
+#pragma unroll
+        for (int part = 0; part < 2; ++part) {
+          uint32_t inc[16];
+          tmem_ld_16x256<4>(tmem + lane_base + TM_INC + 64 * cg + 32 * part, inc);
+          tmem_ld_wait();
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+              const int j = 8 * part + 4 * m + hh;   // zz[j]: real parts, zz[j + 2]: imaginary parts
+              const f2 ir = mk2(__uint_as_float(inc[8 * m + 2 * hh]), __uint_as_float(inc[8 * m + 2 * hh + 1]));
+              const f2 ii = mk2(__uint_as_float(inc[8 * m + 4 + 2 * hh]), __uint_as_float(inc[8 * m + 4 + 2 * hh + 1]));
+              if (ADJ) {
+                const f2 a = zz[j], c = zz[j + 2];
+                zz[j] = fma2(c, NI, fma2(a, R, ir));
+                zz[j + 2] = fma2(c, R, fma2(a, I, ii));
+              } else {
+                const f2 a = fma2(zz[j], E, ir), c = fma2(zz[j + 2], E, ii);
+                zz[j] = fma2(c, I, mul2(a, R));
+                zz[j + 2] = fma2(a, NI, mul2(c, R));
+              }
+            }
+        }
+        if (keep_zv) store_zv_tile();
+      }
+
+      if (FULL) {
+        // ---- output: y = Y_diag + e^{l_t} Y_off ---------------------------------------------------------------
+        const float et[2] = {kcl[rowA].z, kcl[rowB].z};
+        live = live && wait_warp(&bar_mma[2], i & 1, 4);
+        tc_fence_after_sync();
+        if (live) {
+          uint32_t yd[4 * SB], yo[4 * SB];
+          tmem_ld_16x256<SB>(tmem + lane_base + cg * SC, yd);
+          tmem_ld_16x256<SB>(tmem + lane_base + 64 + cg * SC, yo);
+          tmem_ld_wait();
+          const int t0 = (c0 + i) * L;
+#pragma unroll
+          for (int k = 0; k < SB; ++k)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+              const int R = hh ? rowB : rowA;
+              const float y0 = __uint_as_float(yd[4 * k + 2 * hh]) + et[hh] * __uint_as_float(yo[4 * k + 2 * hh]);
+              const float y1 = __uint_as_float(yd[4 * k + 2 * hh + 1]) + et[hh] * __uint_as_float(yo[4 * k + 2 * hh + 1]);
+              if constexpr (sizeof(TY) == 2) {   // over the score tile; rows beyond T are clipped by the store
+                *reinterpret_cast<uint32_t*>(smem + SM::S + sw128(R, cg * SB + k) + 4 * cq) = Pack2<TY>::pack(y0, y1);
+              } else if (t0 + R < T) {
+                float* dst = reinterpret_cast<float*>(p.Y) + ((size_t)bh * T + t0 + R) * 64 + cg * SC + 8 * k + 2 * cq;
+                *reinterpret_cast<float2*>(dst) = make_float2(y0, y1);
+              }
+            }
         }
       }
-      store_zv_tile(c + 1);
+      fence_async_smem();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_st);   // this warp's part of the Y and Zv tiles is complete
     }
-    fence_async_smem();
-    tc_fence_before_sync();
-    }  // worker
-    __syncthreads();
-    if (s_abort) { ok = false; break; }
-  }
-
-  if (!STATES_ONLY && ok) {
-    if (worker) {
-      output_epilogue(p.nchunks - 1, true);
-    } else if (Y_TMA && warp == 4 * NW + 1 && lane == 0) {
-      if (mbar_wait(&bar_st, (p.nchunks - 1) & 1, wl)) {
-        tma_store_3d(&p.tmY, smem + OFF_Y, 0, (p.nchunks - 1) * L, bh);
-        tma_store_commit();
-      } else { report_timeout(5); s_abort = 1; }
-    }
-  }
-  if (ok && p.zfinal && worker) {
+    if (live && p.to_seg) {
+      float* dst = p.seg + ((size_t)bh * p.nseg + seg) * 64 * 128 * NB + 64 * cg + 2 * cq;
 #pragma unroll
-    for (int i = 0; i < ZB; ++i) {
-      const int d = d0 + 8 * i + 2 * cq;
-      *reinterpret_cast<float2*>(p.zfinal + ((size_t)bh * 64 + rowA) * 128 + d) = make_float2(zv[4 * i], -zv[4 * i + 1]);
-      *reinterpret_cast<float2*>(p.zfinal + ((size_t)bh * 64 + rowB) * 128 + d) = make_float2(zv[4 * i + 2], -zv[4 * i + 3]);
+      for (int j = 0; j < 8; ++j) {
+        *reinterpret_cast<float2*>(dst + (size_t)rowA * 128 * NB + 8 * j) = un2(zz[2 * j]);
+        *reinterpret_cast<float2*>(dst + (size_t)rowB * 128 * NB + 8 * j) = un2(zz[2 * j + 1]);
+      }
+    } else if (live && p.zfinal && seg == p.nseg - 1) {
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const int nn = n_of(m);
+        if (nn >= p.N) continue;
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          const float2 re = un2(zz[4 * m + hh]), im = un2(zz[4 * m + 2 + hh]);
+          *reinterpret_cast<float4*>(p.zfinal + ((size_t)bh * 64 + (hh ? rowB : rowA)) * D + 2 * nn) =
+              make_float4(re.x, -im.x, re.y, -im.y);
+        }
+      }
     }
-  }
-  // Unwind: nothing of this CTA may still be in flight when shared memory and TMEM are released.  Every
-  // asynchronous operation was started by the issue lane (but for the loads of chunk 0), so it drains them:
-  // after an expired wait the loads of the last two requested chunks (their barriers, default long limit),
-  // every tcgen05.mma issued so far (one more commit) and, always, its TMA stores.
-  if (warp == 4 * NW + 1 && lane == 0) {
-    if (s_abort)
-      for (int cc = issued_hi > 0 ? issued_hi - 1 : 0; cc <= issued_hi; ++cc) mbar_wait(&bar_tma[cc & 1], (cc >> 1) & 1);
-    umma_commit(&bar_drain);
-    mbar_wait(&bar_drain, 0);
-    tma_store_wait_all();
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
+  if (warp == 0) tmem_dealloc(tmem, TM_COLS);
+}
+
+// Start state of every segment from the segments' own contributions: seg[s] <- Z_s, Z_{s+1} = Pi_s Z_s + F_s (conj
+// pairs, so conj(Pi_s)), or, for adjoints, backwards in time: seg[s] <- Z_s (at the segment's END), Z_{s-1} = Pi_s Z_s + F_s.
+// ``init`` = (BH, 64, 2N) start state / end adjoint or null; Bprev / Uprev add the pending tap to it.  One thread per
+// (row, oscillator); the serial chain is nseg multiply-adds long and its loads are requested eight at a time.
+// Used when there are more than FOLD_SEGS segments: up to there the sweeps fold the contributions of the segments
+// before theirs themselves (32 KB per segment and CTA from L2), which costs less than a launch.
+template <typename TIn, bool REVERSE>
+__global__ void __launch_bounds__(256) scan_tc_combine_kernel(float* __restrict__ seg, const float2* __restrict__ seg_pi,
+                                                              const float* __restrict__ init,
+                                                              const TIn* __restrict__ Bprev,
+                                                              const TIn* __restrict__ Uprev,
+                                                              const float* __restrict__ M, const float* __restrict__ K,
+                                                              int heads, int groups, int T, int N, int nb, int nseg) {
+  const int e = blockIdx.y * 256 + threadIdx.x, bh = blockIdx.x;
+  const int width = 64 * nb, row = e / width, n = e % width;
+  if (row >= 64) return;
+  float zr = 0.f, zi = 0.f;
+  if (n < N) {
+    if (init) {
+      const float2 z = *reinterpret_cast<const float2*>(init + ((size_t)bh * 64 + row) * 2 * N + 2 * n);
+      zr = z.x; zi = z.y;
+    }
+    if (Bprev) {
+      const int bg = (bh / heads) * groups + (bh % heads) / (heads / groups);
+      float xr, xi;
+      pending_tap(M + (size_t)bh * T * 2, K + (size_t)bh * T * 4, xr, xi);
+      const float br = to_f32(Bprev[(size_t)bg * 2 * N + 2 * n]), bi = to_f32(Bprev[(size_t)bg * 2 * N + 2 * n + 1]);
+      const float u = to_f32(Uprev[(size_t)bh * 64 + row]);
+      zr += u * (xr * br - xi * bi);
+      zi += u * (xr * bi + xi * br);
+    }
+  }
+  zi = -zi;
+  const size_t stride = (size_t)64 * 2 * width;
+  float* base = seg + (size_t)bh * nseg * stride + (size_t)row * 2 * width + (n >> 3) * 16 + (n & 7);
+  const float2* pis = seg_pi + (size_t)bh * nseg;
+  for (int k0 = 0; k0 < nseg; k0 += 8) {
+    float fr[8], fi[8];
+    float2 pi[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      fr[k] = fi[k] = 0.f; pi[k] = make_float2(0.f, 0.f);
+      if (k0 + k < nseg - 1) {   // (the contribution of the last segment of the walk is not needed)
+        const int s = REVERSE ? nseg - 1 - (k0 + k) : k0 + k;
+        fr[k] = base[s * stride]; fi[k] = base[s * stride + 8]; pi[k] = pis[s];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (k0 + k >= nseg) break;
+      const int s = REVERSE ? nseg - 1 - (k0 + k) : k0 + k;
+      base[s * stride] = zr; base[s * stride + 8] = zi;
+      const float pim = REVERSE ? pi[k].y : -pi[k].y;
+      const float nr = pi[k].x * zr - pim * zi + fr[k];
+      zi = pi[k].x * zi + pim * zr + fi[k];
+      zr = nr;
+    }
+  }
 }

@@ -1,0 +1,43 @@
+"""The tensor-core scan where it is split in time and where N is padded to the kernels' column blocks, against the
+oracle: segments of one and of several chunks, a last segment that is shorter, ragged last chunks, carried state
+and taps, grouped B/C, widths at the edges of the 64-column tiles."""
+
+import pytest
+import torch
+
+from oracle import scan_np
+from slinoss_b200 import _C
+from slinoss_b200.ops.v2x2ssd import v2x2ssd
+from slinoss_b200.synthetic import make_scan_case
+from tests.util import n64, rel
+
+pytestmark = pytest.mark.gpu
+NAMES = ("U", "M", "K", "B", "C", "initial_states", "B_prev", "U_prev")
+
+
+# (batch, heads, groups, T, N, carried state and taps, gradient of the final state)
+@pytest.mark.parametrize("shape", [
+    (1, 1, 1, 128, 64, False, False), (1, 2, 1, 129, 64, True, True), (1, 1, 1, 1221, 64, True, True),
+    (1, 3, 3, 640, 128, True, True), (2, 2, 1, 577, 128, False, True), (1, 2, 2, 200, 4, True, True),
+    (1, 2, 2, 333, 32, True, True), (2, 2, 1, 321, 36, False, False), (1, 2, 1, 450, 48, True, True),
+    (1, 2, 2, 300, 68, True, True), (1, 2, 2, 260, 96, True, False), (1, 1, 1, 64, 100, False, True),
+    (3, 16, 4, 260, 64, True, True), (1, 90, 90, 130, 64, False, True)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_split_and_padded_scan_matches_the_oracle(shape, dtype):
+    b, h, g, T, N, carried, with_dfinal = shape
+    case = make_scan_case(b, h, T, 64, N, groups=g, dtype=dtype, seed=T + N, streaming=carried, with_init=carried)
+    c = case.to("cuda")
+    leaves = {k: getattr(c, k).clone().requires_grad_(True) for k in NAMES if getattr(c, k) is not None}
+    Y, fin, _, _ = v2x2ssd(*[leaves[k] for k in "UMKBC"], chunk_size=64, initial_states=leaves.get("initial_states"),
+                           B_prev=leaves.get("B_prev"), U_prev=leaves.get("U_prev"))
+    d_final = torch.randn(fin.shape, generator=torch.Generator().manual_seed(5)).to(dtype) if with_dfinal else None
+    outs, cots = ([Y, fin], [c.dY, d_final.cuda()]) if with_dfinal else ([Y], [c.dY])
+    grads = torch.autograd.grad(outs, list(leaves.values()), cots)
+    assert _C.device_status() == 0
+    args = [n64(t) for t in case.tensors()]
+    kw = dict(initial_states=n64(case.initial_states), B_prev=n64(case.B_prev), U_prev=n64(case.U_prev))
+    wY, wfin, _, _ = scan_np.v2x2ssm(*args, **kw)
+    assert rel(Y, wY) <= 2e-2 and rel(fin, wfin) <= 2e-2
+    want = scan_np.v2x2ssd_bwd(*args, n64(case.dY), d_final_state=None if d_final is None else n64(d_final), **kw)
+    for name, grad in zip(leaves, grads):
+        assert rel(grad, want[name]) <= 2e-2, (name, rel(grad, want[name]))
