@@ -131,22 +131,35 @@ __device__ __forceinline__ void pending_tap(const float* Mb, const float* Kb, fl
 //  [256, 512)  per token: kc_t (re, im), exp(l_t), exp(l_end - l_t)
 //  [512, 576)  per token: l_t in units of log 2
 //  [576, 579)  exp(l_end), unit phase of Pi_end (re, im)
-constexpr int SC_KCL = 256, SC_L2 = 512, SC_TAIL = 576, SCW = 592;
-__device__ __noinline__ void chunk_scalars(float* sc, const float* __restrict__ Mb, const float* __restrict__ Kb,
-                                           int t0, int T, int lane) {
-  float mr[3], mi[3], kpr[3], kpi[3], kcr[2], kci[2];
+//  forward only:
+//  [592, 848)  per block q of 16 tokens and token s < 16 q: exp(l_{16 q} - l_s)
+//  [848, 912)  per token: exp(l_t - l_{16 (t / 16)})
+// A decay factor exp(l_t - l_s), s < t, is a product of the last two outside the 16 x 16 blocks on the diagonal
+// (both factors are <= 1, so nothing can overflow): the masking epilogue needs one multiplication per cell there
+// instead of an exponential.  (The backward's masking epilogue runs in the shadow of its MMAs: there the plain
+// exponentials measured 4 % faster than the branch on the block's place.)
+constexpr int SC_KCL = 256, SC_L2 = 512, SC_TAIL = 576, SC_COL = 592, SC_ROW = 848, SCW = 912, SCW_B = 592;
+struct ScalarRaw { float2 m[3]; float4 k[3]; };   // a lane's two tokens and the one after them
+__device__ __forceinline__ ScalarRaw load_scalars(const float* __restrict__ Mb, const float* __restrict__ Kb, int t0,
+                                                  int T, int lane) {
+  ScalarRaw r;
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     const int t = t0 + 2 * lane + q;
-    mr[q] = 1.f; mi[q] = 0.f; kpr[q] = 0.f; kpi[q] = 0.f;
-    if (q < 2) { kcr[q] = 0.f; kci[q] = 0.f; }
+    r.m[q] = make_float2(1.f, 0.f);
+    r.k[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (t < T) {
-      const float2 m = *reinterpret_cast<const float2*>(Mb + 2 * (size_t)t);
-      const float4 k = *reinterpret_cast<const float4*>(Kb + 4 * (size_t)t);
-      mr[q] = m.x; mi[q] = m.y; kpr[q] = k.x; kpi[q] = k.y;
-      if (q < 2) { kcr[q] = k.z; kci[q] = k.w; }
+      r.m[q] = *reinterpret_cast<const float2*>(Mb + 2 * (size_t)t);
+      r.k[q] = *reinterpret_cast<const float4*>(Kb + 4 * (size_t)t);
     }
   }
+  return r;
+}
+template <bool FACTORS>
+__device__ __forceinline__ void chunk_scalars(float* sc, const ScalarRaw& raw, int lane) {
+  const float mr[3] = {raw.m[0].x, raw.m[1].x, raw.m[2].x}, mi[3] = {raw.m[0].y, raw.m[1].y, raw.m[2].y};
+  const float kpr[3] = {raw.k[0].x, raw.k[1].x, raw.k[2].x}, kpi[3] = {raw.k[0].y, raw.k[1].y, raw.k[2].y};
+  const float kcr[2] = {raw.k[0].z, raw.k[1].z}, kci[2] = {raw.k[0].w, raw.k[1].w};
   // local prefixes over the lane's two tokens
   const float q0 = mr[0] * mr[0] + mi[0] * mi[0], q1 = mr[1] * mr[1] + mi[1] * mi[1];
   const float i0 = rsqrtf(q0), i1 = rsqrtf(q1);
@@ -186,10 +199,27 @@ __device__ __noinline__ void chunk_scalars(float* sc, const float* __restrict__ 
     reinterpret_cast<float4*>(sc + SC_KCL)[i] = make_float4(kcr[q], kci[q], ex2f(lt[q]), ex2f(l_end - lt[q]));
     sc[SC_L2 + i] = lt[q];
   }
+  if constexpr (FACTORS) {
+    float lref[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      lref[q] = __shfl_sync(0xffffffffu, lt[0], 8 * q);
+      *reinterpret_cast<float2*>(sc + SC_COL + 64 * q + 2 * lane) =
+          make_float2(ex2f(fminf(lref[q] - lt[0], 0.f)), ex2f(fminf(lref[q] - lt[1], 0.f)));
+    }
+    const float lr = lane < 8 ? lref[0] : lane < 16 ? lref[1] : lane < 24 ? lref[2] : lref[3];
+    *reinterpret_cast<float2*>(sc + SC_ROW + 2 * lane) = make_float2(ex2f(fminf(lt[0] - lr, 0.f)), ex2f(fminf(lt[1] - lr, 0.f)));
+  }
   if (lane == 31) {
     sc[SC_TAIL] = ex2f(l_end);
     sc[SC_TAIL + 1] = phr[1]; sc[SC_TAIL + 2] = phi[1];
   }
+}
+
+// Loads and table in one out-of-line call (the backward: its code is long enough for the instruction cache to matter).
+__device__ __noinline__ void chunk_scalars_at(float* sc, const float* __restrict__ Mb, const float* __restrict__ Kb,
+                                              int t0, int T, int lane) {
+  chunk_scalars<false>(sc, load_scalars(Mb, Kb, t0, T, lane), lane);
 }
 
 #include "scan_tc_fwd.cuh"
@@ -254,7 +284,7 @@ inline SegPlan plan_segments(long long streams, int nchunks, const SegCost& c) {
 }
 inline SegPlan fwd_plan(const ScanDims& d) {
   return plan_segments((long long)d.batch * d.heads, chunks_of(d),
-                       blocks_of(d) == 1 ? SegCost{1.5, 0.45, 3.0} : SegCost{2.0, 0.35, 2.5});
+                       blocks_of(d) == 1 ? SegCost{1.6, 0.5, 4.5} : SegCost{2.0, 0.4, 3.0});
 }
 inline SegPlan bwd_plan(const ScanDims& d) {
   return plan_segments((long long)d.batch * d.heads * blocks_of(d), chunks_of(d), SegCost{2.0, 0.25, 2.0});
@@ -269,15 +299,22 @@ inline SegLayout seg_layout(const ScanDims& d, int nseg) {
   return o;
 }
 
-template <typename TIn, typename TY, int MODE, int NB>
-int launch_fwd_kernel(const TcFwdParams& p, dim3 grid, cudaStream_t st) {
-  auto k = scan_tc_fwd_kernel<TIn, TY, MODE, NB>;
-  constexpr size_t bytes = FwdSmem<NB, MODE == 0>::BYTES;
+template <typename TIn, typename TY, int MODE, int NB, int NWQ>
+int launch_fwd_variant(const TcFwdParams& p, dim3 grid, cudaStream_t st) {
+  auto k = scan_tc_fwd_kernel<TIn, TY, MODE, NB, NWQ>;
+  constexpr size_t bytes = FwdSmem<NB, MODE == 0, NWQ>::BYTES;
   static std::atomic<unsigned long long> done{0};
   if (int e = ensure_smem(k, bytes, done)) return e;
-  k<<<grid, 256 * NB + 64, bytes, st>>>(p);
+  k<<<grid, 128 * NWQ + 64, bytes, st>>>(p);
   note_launches(1);
   return launch_status();
+}
+// NB = 1: 16 worker warps shorten the chain of a chunk when no SM gets two CTAs, 8 let two CTAs share an SM
+template <typename TIn, typename TY, int MODE>
+int launch_fwd_kernel(const TcFwdParams& p, dim3 grid, int nb, cudaStream_t st) {
+  if (nb == 2) return launch_fwd_variant<TIn, TY, MODE, 2, 4>(p, grid, st);
+  if ((long long)grid.x * grid.y <= SMS) return launch_fwd_variant<TIn, TY, MODE, 1, 4>(p, grid, st);
+  return launch_fwd_variant<TIn, TY, MODE, 1, 2>(p, grid, st);
 }
 
 // pre-pass over the segments: MODE 1 forward in time over (U, B), MODE 2 backwards over (dY, C)
@@ -287,7 +324,7 @@ int launch_prepass(TcFwdParams p, int BH, int nb, cudaStream_t st) {
   p.states16 = nullptr; p.zfinal = nullptr; p.z0 = nullptr; p.Bprev = nullptr; p.Uprev = nullptr;
   p.seg0 = MODE == 2 ? 1 : 0;   // the segment that ends the walk contributes to no other
   const dim3 grid((unsigned)BH, (unsigned)(p.nseg - 1));
-  return nb == 1 ? launch_fwd_kernel<TIn, float, MODE, 1>(p, grid, st) : launch_fwd_kernel<TIn, float, MODE, 2>(p, grid, st);
+  return launch_fwd_kernel<TIn, float, MODE>(p, grid, nb, st);
 }
 
 // Forward (Y given) or chunk-start / final states only (Y null).
@@ -306,11 +343,9 @@ int run_fwd(TcFwdParams& p, const ScanDims& d, int y_dtype, cudaStream_t st) {
   }
   const dim3 grid((unsigned)BH, (unsigned)p.nseg);
   if (!p.Y)
-    return nb == 1 ? launch_fwd_kernel<TIn, float, 1, 1>(p, grid, st) : launch_fwd_kernel<TIn, float, 1, 2>(p, grid, st);
+    return launch_fwd_kernel<TIn, float, 1>(p, grid, nb, st);
   int rc = SL_ERR_UNSUPPORTED;
-  SL_DISPATCH_DTYPE(y_dtype, TY, {
-    rc = nb == 1 ? launch_fwd_kernel<TIn, TY, 0, 1>(p, grid, st) : launch_fwd_kernel<TIn, TY, 0, 2>(p, grid, st);
-  });
+  SL_DISPATCH_DTYPE(y_dtype, TY, { rc = launch_fwd_kernel<TIn, TY, 0>(p, grid, nb, st); });
   return rc;
 }
 

@@ -28,7 +28,7 @@ constexpr uint32_t B_OFF_DP = B_OFF_PD + TILE;         // dP (1)
 constexpr uint32_t B_OFF_DW = B_OFF_DP + TILE;         // dWv (2)
 constexpr uint32_t B_OFF_UE = B_OFF_DW + 2 * TILE;     // e^{l_end-l_s} U (1)
 constexpr uint32_t B_OFF_SCAL = B_OFF_UE + TILE;
-constexpr int B_SCAL_FLOATS = 2 * SCW + 64 + 4 * 64 + 32 * 64;   // tables, sigma, [2][64] c conj(b), 4 x 8 partial sums
+constexpr int B_SCAL_FLOATS = 2 * SCW_B + 64 + 4 * 64 + 32 * 64;   // tables, sigma, [2][64] c conj(b), 4 x 8 partial sums
 constexpr uint32_t B_SMEM_BYTES = B_OFF_SCAL + B_SCAL_FLOATS * 4 + 1024;
 // TMEM columns: P~ then dUa 0 | dS then dUb 64 | dQ 128..255 | dX 256..383 | dZ 384..511.  All products have
 // M = 64 (rows in lanes 0..15 of a quadrant).  P~, dS, dUa and dUb are N = 64 and read with the 16x256b load
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __g
   __shared__ int s_abort;
   __shared__ float s_red[8 * NW + 2];
   float* sc_tab = reinterpret_cast<float*>(smem + B_OFF_SCAL);   // two tables (chunk parity)
-  float* s_sig = sc_tab + 2 * SCW;                               // sigma_t = <dy_t, u_t>
+  float* s_sig = sc_tab + 2 * SCW_B;                               // sigma_t = <dy_t, u_t>
   float2* s_cb = reinterpret_cast<float2*>(s_sig + 64);          // [2 halves][64]: sum_n c conj(b)
   float* s_acc = s_sig + 64 + 4 * 64;   // [4 quantities][8 = column group x half][64 rows]: re/im of <q,dq>, of R
   using PK = Pack2<TIn>;
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __g
   if (warp == 0) {
     tmem_alloc(&tmem_slot, B_TMEM_COLS);
   } else if (warp == 4 * NW) {
-    chunk_scalars(sc_tab, Mb, Kb, (c_lo + n - 1) * L, T, lane);
+    chunk_scalars_at(sc_tab, Mb, Kb, (c_lo + n - 1) * L, T, lane);
   }
   if (tid == 0) issue_loads(0);   // (after the barriers were initialised by this same thread)
 
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __g
     const int t0 = (c_lo + n - 1 - it) * L;
     uint8_t* st = smem + (it & 1) * B_STAGE;
     uint8_t *tU = st, *tB = st + TILE, *tC = st + 3 * TILE, *tDY = st + 5 * TILE, *tZ = st + 6 * TILE;
-    const float* sc = sc_tab + (it & 1) * SCW;
+    const float* sc = sc_tab + (it & 1) * SCW_B;
     const float4* rot = reinterpret_cast<const float4*>(sc);
     const float4* kcl = reinterpret_cast<const float4*>(sc + SC_KCL);
     if (warp == 4 * NW) {
@@ -271,9 +271,10 @@ __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __g
       // ends the iteration
       // (it starts after the workers' first passes: global loads issued while every worker warp
       // bursts shared-memory traffic at the top of the iteration stalled the whole SM for about a
-      // DRAM round trip)
+      // DRAM round trip; computing the table at the top from inputs requested an iteration ahead measured 10 %
+      // slower for the same reason)
       bar_sync(2, NT + 64);   // the workers only arrive here (bar_arrive): they never wait for this warp
-      if (it + 1 < n) chunk_scalars(sc_tab + ((it + 1) & 1) * SCW, Mb, Kb, t0 - L, T, lane);
+      if (it + 1 < n) chunk_scalars_at(sc_tab + ((it + 1) & 1) * SCW_B, Mb, Kb, t0 - L, T, lane);
       // the anchor of the previous chunk: a global store by a worker thread here would make that
       // thread's next proxy fence (epilogue 1) wait for the store, and every worker for that thread
       bar_sync(7, NT + 32);
@@ -294,7 +295,7 @@ __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __g
       const uint64_t mPD = make_desc(aPD, 8192, 1024), mDYO = make_desc(aDYO, 8192, 1024), kDYO = make_desc(aDYO, 16, 1024);
       const uint64_t kDW = make_desc(aDW, 16, 1024), mDW = make_desc(aDW, 8192, 1024);
       const uint64_t kUE = make_desc(aUE, 16, 1024);
-      bool go = lane == 0 && s_abort == 0;
+      bool go = elect_one() && s_abort == 0;
       if (go) do {
         // (1) products of raw tiles, as soon as the stage has landed
         if (!mbar_wait(&bar_tma[it & 1], (it >> 1) & 1, wl)) { report_timeout(20); s_abort = 1; go = false; break; }
@@ -514,9 +515,14 @@ __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __g
     // ---- epilogue 1: decayed, strictly causal Pdec and dP as 16-bit tiles -------------------------------
     if (live) {
       uint32_t pr[4 * WB], ds[4 * WB];
-      tmem_ld_16x256<WB>(tmem + lane_base + 0 + cg * WC, pr);
-      tmem_ld_16x256<WB>(tmem + lane_base + 64 + cg * WC, ds);
-      tmem_ld_wait();
+      if (cg <= quad) {
+        tmem_ld_16x256<WB>(tmem + lane_base + 0 + cg * WC, pr);
+        tmem_ld_16x256<WB>(tmem + lane_base + 64 + cg * WC, ds);
+        tmem_ld_wait();
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4 * WB; ++k) pr[k] = ds[k] = 0u;
+      }
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         const int R = hh ? rowB : rowA;

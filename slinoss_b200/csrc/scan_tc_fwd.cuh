@@ -1,8 +1,8 @@
 // Forward kernel of the chunked scan on tcgen05 (included by scan_tc.cu inside its namespaces).
 //
 // One CTA walks the chunks of one segment of one (batch, head) stream.  NB = 64-column blocks of the state
-// dimension held by the CTA (1: N <= 64, 2: N <= 128).  The CTA has 8 NB worker warps (4 TMEM lane quadrants x
-// 2 NB column groups), one scalar warp and one issue warp.
+// dimension held by the CTA (1: N <= 64, 2: N <= 128); NWQ = warps per TMEM lane quadrant.  The CTA has 4 NWQ worker
+// warps (4 lane quadrants x NWQ column groups), one scalar warp and one issue warp.
 //
 // MODE 0  full forward: Y, final state, optional 16-bit chunk-start states
 //      1  states only: chunk-start states / the end state of the segment (no C, no scores, no Y)
@@ -11,8 +11,8 @@
 //
 // What bounds it: the phases of a chunk (rotation, score product, masking, second product, state update) form
 // one dependent chain of about 5 k clocks, most of it latency; neither DRAM, the tensor pipe nor the issue
-// slots are full.  Hence two CTAs per SM for NB = 1 (80 KB of tiles, 256 TMEM columns, 96 registers): the
-// chain of one stream fills the waits of the other.  To fit twice, B and C are rotated in place in a single
+// slots are full.  Hence, when there are streams enough, two CTAs per SM for NB = 1 (NWQ = 2: 80 KB of tiles, 256 TMEM
+// columns, 96 registers): the chain of one stream fills the waits of the other.  To fit twice, B and C are rotated in place in a single
 // stage that is refilled while the scores are masked, Y is staged over the score tile, and the second product
 // accumulates over the TMEM columns of the scores.
 //
@@ -22,7 +22,7 @@
 //
 // MMAs have M = 64 (rows in lanes 0..15 of every TMEM quadrant); the epilogues read them with the 16x256b shape
 // (thread t: rows t/4 and t/4 + 8 of the quadrant, column pair 2 (t%4) of every 8-column block).
-template <int NB, bool FULL>
+template <int NB, bool FULL, int NWQ>
 struct FwdSmem {
   static constexpr uint32_t U = 0;                                   // two stages of U
   static constexpr uint32_t KZ = 2 * TILE;                           // 2 NB x [K' ; Zv]
@@ -30,7 +30,7 @@ struct FwdSmem {
   static constexpr uint32_t UE = C + (FULL ? 2 * NB * TILE : 0);     // e^{l_end - l_s} U
   static constexpr uint32_t S = UE + TILE;                           // scores, then Y
   static constexpr uint32_t SCAL = S + (FULL ? TILE : 0);
-  static constexpr uint32_t BYTES = SCAL + 2 * SCW * 4 + NB * 64 * 4 + 1024;
+  static constexpr uint32_t BYTES = SCAL + 3 * SCW * 4 + (NWQ / 2) * 64 * 4 + 1024;
 };
 
 struct alignas(64) TcFwdParams {
@@ -52,32 +52,34 @@ struct alignas(64) TcFwdParams {
   long long wait_limit;  // SM clocks a wait of the main loop may take before the kernel gives up
 };
 
-template <typename TIn, typename TY, int MODE, int NB>
-__global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
+template <typename TIn, typename TY, int MODE, int NB, int NWQ>
+__global__ void __launch_bounds__(128 * NWQ + 64, NWQ == 2 ? 2 : 1)
     scan_tc_fwd_kernel(const __grid_constant__ TcFwdParams p) {
   constexpr bool FULL = MODE == 0, ADJ = MODE == 2;
-  using SM = FwdSmem<NB, FULL>;
-  constexpr int NWQ = 2 * NB;        // warps per TMEM lane quadrant
+  using SM = FwdSmem<NB, FULL, NWQ>;
   constexpr int NT = 128 * NWQ;      // worker threads
   constexpr int SC = 64 / NWQ;       // score / output columns per warp
   constexpr int SB = SC / 8;
+  constexpr int ZC = 128 * NB / NWQ; // state columns per warp
+  constexpr int ZB = ZC / 8;
+  constexpr int TPT = 512 * NB / NT; // tiles of B (and C) a thread rotates
   constexpr uint32_t TM_COLS = FULL ? (NB == 1 ? 256 : 512) : 128 * NB;
   constexpr uint32_t TM_INC = FULL ? 128 : 0;   // TMEM: [S, then Ydiag | Yoff] 0..127, Inc 128 NB columns
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  __shared__ uint64_t bar_u[2], bar_bc, bar_mma[3], bar_st, bar_sc, bar_drain;   // bar_mma: [S|Yoff] | Inc | Ydiag
+  __shared__ uint64_t bar_u[2], bar_bc[2], bar_mma[3], bar_st, bar_sc[2], bar_drain;   // bar_mma: [S|Yoff] | Inc | Ydiag
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
   constexpr bool Y_TMA = FULL && sizeof(TY) == 2;
   float* sc_tab = reinterpret_cast<float*>(smem + SM::SCAL);
-  float* s_diag = sc_tab + 2 * SCW;   // [NB][64] partial diagonal scores
+  float* s_diag = sc_tab + 3 * SCW;   // [NWQ / 2][64] partial diagonal scores
   using PK = Pack2<TIn>;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool worker = warp < 4 * NWQ;
   const int quad = warp & 3, cg = worker ? (warp >> 2) : 0;
   const int rowA = 16 * quad + (lane >> 2), rowB = rowA + 8, cq = lane & 3;   // epilogue identity
-  const int rrow = (tid >> 2) & 63, rk = tid & 3, rgrp = (tid >> 8) & (NB - 1);   // rotation identity
+  const int rrow = (tid >> 2) & 63, rk = tid & 3, rgrp = tid >> 8;   // rotation identity
   const uint32_t lane_base = (uint32_t)(32 * quad) << 16;
   const int bh = blockIdx.x, b = bh / p.heads, h = bh % p.heads;
   const int bg = b * p.groups + h / (p.heads / p.groups);
@@ -90,10 +92,10 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
   auto chunk_of = [&](int i) { return ADJ ? c0 + n - 1 - i : c0 + i; };
 
   if (tid == 0) {
-    mbar_init(&bar_u[0], 1); mbar_init(&bar_u[1], 1); mbar_init(&bar_bc, 1);
+    mbar_init(&bar_u[0], 1); mbar_init(&bar_u[1], 1); mbar_init(&bar_bc[0], 1); mbar_init(&bar_bc[1], 1);
     for (int i = 0; i < 3; ++i) mbar_init(&bar_mma[i], 1);
     mbar_init(&bar_st, 4 * NWQ);   // one arrival per worker warp
-    mbar_init(&bar_sc, 1);
+    mbar_init(&bar_sc[0], 1); mbar_init(&bar_sc[1], 1);
     mbar_init(&bar_drain, 1);
     fence_barrier_init();
     s_abort = 0;
@@ -102,32 +104,46 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
     mbar_expect_tx(&bar_u[i & 1], TILE);
     tma_load_3d(smem + SM::U + (i & 1) * TILE, &p.tmU, &bar_u[i & 1], 0, chunk_of(i) * L, bh);
   };
+  // B is single-buffered where the other half of the KZ tiles holds the state, double-buffered in the pre-passes,
+  // which keep no state tile: there the load would otherwise be longer than the rest of a chunk's chain
+  const bool keep_zv = FULL || p.states16 != nullptr;
+  auto buf_of = [&](int i) { return keep_zv ? 0 : i & 1; };
+  auto phase_of = [&](int i) { return (uint32_t)(keep_zv ? i & 1 : (i >> 1) & 1); };
   auto issue_bc = [&](int i) {   // one thread
     const int t0 = chunk_of(i) * L;
-    mbar_expect_tx(&bar_bc, (FULL ? 4 : 2) * NB * TILE);
+    uint64_t* bar = &bar_bc[buf_of(i)];
+    mbar_expect_tx(bar, (FULL ? 4 : 2) * NB * TILE);
 #pragma unroll
     for (int q = 0; q < 2 * NB; ++q) {
-      tma_load_3d(smem + SM::KZ + 2 * q * TILE, &p.tmB, &bar_bc, 64 * q, t0, bg);
-      if (FULL) tma_load_3d(smem + SM::C + q * TILE, &p.tmC, &bar_bc, 64 * q, t0, bg);
+      tma_load_3d(smem + SM::KZ + (2 * q + buf_of(i)) * TILE, &p.tmB, bar, 64 * q, t0, bg);
+      if (FULL) tma_load_3d(smem + SM::C + q * TILE, &p.tmC, bar, 64 * q, t0, bg);
+    }
+  };
+  auto prefetch_bc = [&](int i) {   // one thread
+    const int t0 = chunk_of(i) * L;
+#pragma unroll
+    for (int q = 0; q < 2 * NB; ++q) {
+      tma_prefetch_3d(&p.tmB, 64 * q, t0, bg);
+      if (FULL) tma_prefetch_3d(&p.tmC, 64 * q, t0, bg);
     }
   };
   if (warp == 0) {
     tmem_alloc(&tmem_slot, TM_COLS);
   } else if (warp == 4 * NWQ) {
-    chunk_scalars(sc_tab, Mb, Kb, chunk_of(0) * L, T, lane);
+    chunk_scalars<FULL>(sc_tab, load_scalars(Mb, Kb, chunk_of(0) * L, T, lane), lane);
   }
   if (tid == 0) {   // (after the barriers were initialised by this same thread)
     issue_bc(0);
     issue_u(0);
-    if (n > 1) issue_u(1);
+    if (n > 1) { issue_u(1); if (keep_zv) prefetch_bc(1); else issue_bc(1); }
   }
 
-  // ---- carried state, conjugated.  zz[2 j + hh]: 8-column block j of this warp's 64 columns, row (hh ? rowB :
+  // ---- carried state, conjugated.  zz[2 j + hh]: 8-column block j of this warp's ZC columns, row (hh ? rowB :
   // rowA), as a pair of neighbouring columns; even blocks hold real parts, odd blocks minus the imaginary parts
-  f2 zz[16];
+  f2 zz[2 * ZB];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) zz[j] = 0ull;
-  auto n_of = [&](int m) { return 32 * cg + 8 * m + 2 * cq; };   // oscillators n, n + 1 of block pair m
+  for (int j = 0; j < 2 * ZB; ++j) zz[j] = 0ull;
+  auto n_of = [&](int m) { return ZC / 2 * cg + 8 * m + 2 * cq; };   // oscillators n, n + 1 of block pair m
   if (worker && !ADJ && !p.to_seg && p.from_seg != 1 && (p.z0 || p.Bprev)) {   // start state of the sequence
     const TIn* Bp = reinterpret_cast<const TIn*>(p.Bprev);
     const TIn* Up = reinterpret_cast<const TIn*>(p.Uprev);
@@ -138,7 +154,7 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
       up[1] = to_f32(Up[(size_t)bh * 64 + rowB]);
     }
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
+    for (int m = 0; m < ZB / 2; ++m) {
       const int nn = n_of(m);
       if (nn >= p.N) continue;
 #pragma unroll
@@ -159,13 +175,13 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
   // start state of a later segment: given, or folded from the earlier segments' contributions
   if (worker && p.from_seg) {
     const size_t stride = (size_t)64 * 128 * NB;
-    const float* src = p.seg + (size_t)bh * p.nseg * stride + 64 * cg + 2 * cq;
+    const float* src = p.seg + (size_t)bh * p.nseg * stride + ZC * cg + 2 * cq;
     const bool fold = p.from_seg == 2;
     for (int s = fold ? 0 : seg; s < (fold ? seg : seg + 1); ++s) {
       const float2 pi = fold ? p.seg_pi[(size_t)bh * p.nseg + s] : make_float2(0.f, 0.f);
       const f2 pr = dup2(pi.x), pim = dup2(pi.y), npim = dup2(-pi.y);
 #pragma unroll
-      for (int m = 0; m < 4; ++m)
+      for (int m = 0; m < ZB / 2; ++m)
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           const float* f = src + s * stride + (size_t)(hh ? rowB : rowA) * 128 * NB + 16 * m;
@@ -178,13 +194,14 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
   }
   // 16-bit copy of the state: rows p, K-major along d, directly below the K' rows of the same 64 columns, so that
   // [K' ; Zv] is one 128-row operand
-  const bool keep_zv = FULL || p.states16 != nullptr;
   auto store_zv_tile = [&]() {
-    uint8_t* tile = smem + SM::KZ + (2 * cg + 1) * TILE + 4 * cq;
+    uint8_t* tile = smem + SM::KZ + (2 * (cg * ZC / 64) + 1) * TILE + 4 * cq;
+    constexpr int CH = 64 / ZC;   // warps that share a tile
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      *reinterpret_cast<uint32_t*>(tile + sw128(rowA, j)) = PK::pack2(zz[2 * j]);
-      *reinterpret_cast<uint32_t*>(tile + sw128(rowB, j)) = PK::pack2(zz[2 * j + 1]);
+    for (int j = 0; j < ZB; ++j) {
+      const int ch = (cg % CH) * ZB + j;
+      *reinterpret_cast<uint32_t*>(tile + sw128(rowA, ch)) = PK::pack2(zz[2 * j]);
+      *reinterpret_cast<uint32_t*>(tile + sw128(rowB, ch)) = PK::pack2(zz[2 * j + 1]);
     }
   };
   auto store_states = [&](int i) {   // issue lane: the state tile of chunk i is exactly what the backward wants
@@ -210,20 +227,27 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
   };
 
   if (warp == 4 * NWQ) {
-    // ---- scalar warp: the per-chunk tables, one chunk ahead ------------------------------------------------
+    // ---- scalar warp: three tables, two chunks ahead, their inputs one more (the shuffle scans and the way to memory
+    // are longer than a chunk of a pre-pass) -----------------------------------------------------------------
     float pr = 1.f, pi = 0.f;   // transition product of the segment
-    for (int i = 0; i < n; ++i) {
-      if (p.to_seg) {
-        const float* tail = sc_tab + (i & 1) * SCW + SC_TAIL;
-        const float mr = tail[0] * tail[1], mi = tail[0] * tail[2];
-        const float nr = pr * mr - pi * mi;
-        pi = pr * mi + pi * mr; pr = nr;
+    ScalarRaw raw = load_scalars(Mb, Kb, chunk_of(min(1, n - 1)) * L, T, lane);
+    for (int i = -1; i < n; ++i) {
+      if (i >= 0) {
+        if (p.to_seg) {
+          const float* tail = sc_tab + (i % 3) * SCW + SC_TAIL;
+          const float mr = tail[0] * tail[1], mi = tail[0] * tail[2];
+          const float nr = pr * mr - pi * mi;
+          pi = pr * mi + pi * mr; pr = nr;
+        }
+        bar_sync(2, NT + 64);   // the workers are through chunk i - 1, whose table is overwritten now
       }
-      bar_sync(2, NT + 64);   // the workers are through the previous chunk, whose table is overwritten now
-      if (i + 1 < n) {
-        chunk_scalars(sc_tab + ((i + 1) & 1) * SCW, Mb, Kb, chunk_of(i + 1) * L, T, lane);
+      const int j = i + 2;
+      if (j < n) {
+        const ScalarRaw cur = raw;
+        if (j + 1 < n) raw = load_scalars(Mb, Kb, chunk_of(j + 1) * L, T, lane);
+        chunk_scalars<FULL>(sc_tab + (j % 3) * SCW, cur, lane);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bar_sc);
+        if (lane == 0) mbar_arrive(&bar_sc[j & 1]);
       }
     }
     if (p.to_seg && lane == 0) p.seg_pi[(size_t)bh * p.nseg + seg] = make_float2(pr, pi);
@@ -238,19 +262,21 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
     const uint64_t dKm = make_desc(smem_u32(smem + SM::KZ), 2 * TILE, 1024);   // 64-column blocks two tiles apart
     const uint64_t dUE = make_desc(smem_u32(smem + SM::UE), TILE, 1024);
     const uint64_t dS = make_desc(smem_u32(smem + SM::S), 16, 1024);
-    int req_u = min(n, 2), req_bc = 1;   // loads requested so far
-    auto scores = [&](int half) {        // [S | Yoff] = Q [K' ; Zv]^T over the even / odd 64-column tiles
+    int req_u = min(n, 2), req_bc = keep_zv ? 1 : min(n, 2);   // loads requested so far
+    // [S | Yoff] = Q [K' ; Zv]^T over the tiles of the first / second rotation step
+    auto scores = [&](int step) {
 #pragma unroll
-      for (int q = half; q < 2 * NB; q += 2)
+      for (int q = step; q < 2 * NB; q += TPT)
 #pragma unroll
         for (int k = 0; k < 4; ++k)
           umma(tmem, desc_adv(dQ, q * TILE + 32 * k), desc_adv(dKZ, 2 * q * TILE + 32 * k), ID_S, q + k > 0);
     };
     if (lane == 0 && p.states16) store_states(0);
+    __syncwarp();
     for (int i = 0; i < n; ++i) {
-      const bool lead = lane == 0;
+      const bool lead = elect_one();
       if (FULL) {
-        bar_sync(5, NT + 32);   // even tiles of Q and K' rotated
+        bar_sync(5, NT + 32);   // the first (TPT = 1: all) tiles of Q and K' rotated
         if (lead && !s_abort) { tc_fence_after_sync(); scores(0); }
         __syncwarp();
       }
@@ -258,19 +284,23 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
       if (lead && !s_abort) {
         tc_fence_after_sync();
         if (FULL) {
-          scores(1);
+          if (TPT == 2) scores(1);
           tma_store_wait_read();   // the score tile still holds the previous Y, the Zv tiles the saved state
           umma_commit(&bar_mma[0]);
         }
         // Inc = (e^{l_end - l_s} U)^T K'
 #pragma unroll
-        for (int k = 0; k < 4; ++k) umma(tmem + TM_INC, desc_adv(dUE, 2048 * k), desc_adv(dKm, 2048 * k), ID_Z, k > 0);
+        for (int k = 0; k < 4; ++k) umma(tmem + TM_INC, desc_adv(dUE, 2048 * k), desc_adv(dKm, buf_of(i) * TILE + 2048 * k), ID_Z, k > 0);
         if (!FULL) tma_store_wait_read();
         umma_commit(&bar_mma[1]);
         // refill B and C as soon as their last products are done: what is left of the iteration hides the load
-        if (i + 1 < n && wait_one(&bar_mma[1], i & 1, 8)) {
-          issue_bc(i + 1); ++req_bc;
-          if (!FULL && i + 2 < n) { issue_u(i + 2); ++req_u; }
+        const int nxt = i + (keep_zv ? 1 : 2);
+        if (nxt < n && wait_one(&bar_mma[1], i & 1, 8)) {
+          issue_bc(nxt); ++req_bc;
+          if (i + 2 < n) {
+            if (keep_zv) prefetch_bc(i + 2);   // on their way to L2 for a whole iteration
+            if (!FULL) { issue_u(i + 2); ++req_u; }
+          }
         }
       }
       __syncwarp();
@@ -297,7 +327,7 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
     if (lane == 0) {
       // Unwind: nothing of this CTA may still be in flight when shared memory and TMEM are released.
       if (s_abort) {
-        mbar_wait(&bar_bc, (req_bc - 1) & 1);
+        for (int i = max(0, req_bc - 2); i < req_bc; ++i) mbar_wait(&bar_bc[buf_of(i)], phase_of(i));
         for (int i = max(0, req_u - 2); i < req_u; ++i) mbar_wait(&bar_u[i & 1], (i >> 1) & 1);
       }
       umma_commit(&bar_drain);
@@ -309,23 +339,23 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
     // ---- worker warps ---------------------------------------------------------------------------------------
     bool live = true;   // warp-uniform; cleared when a wait expired
     for (int i = 0; i < n; ++i) {
-      const float* sc = sc_tab + (i & 1) * SCW;
+      const float* sc = sc_tab + (i % 3) * SCW;
       const float4* rot = reinterpret_cast<const float4*>(sc);
       const float4* kcl = reinterpret_cast<const float4*>(sc + SC_KCL);
-      if (i > 0) live = live && wait_warp(&bar_sc, (i - 1) & 1, 9);
-      live = live && wait_warp(&bar_bc, i & 1, 1);
+      if (i > 0) live = live && wait_warp(&bar_sc[i & 1], ((i - 1) >> 1) & 1, 9);
+      live = live && wait_warp(&bar_bc[buf_of(i)], phase_of(i), 1);
 
       // ---- rotation: C -> Q, B -> K' (in place), diagonal scores.  A thread owns 32 bytes (8 oscillators) of a
-      // row in each of two tiles; the score products of the first tile start while the second is rotated.
+      // row in each of TPT tiles; the score products of the first tile start while the second is rotated.
       {
         const uint32_t o0 = sw128(rrow, 2 * rk), o1 = sw128(rrow, 2 * rk + 1);
         const float4 rt = rot[rrow];   // phi, w
         f2 dr = 0ull, di0 = 0ull, di1 = 0ull;   // sums of Re conj(c) b and of the two parts of Im conj(c) b
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
+        for (int half = 0; half < TPT; ++half) {
           if (live) {
-            uint8_t* tB = smem + SM::KZ + 2 * (2 * rgrp + half) * TILE;
-            uint8_t* tC = smem + SM::C + (2 * rgrp + half) * TILE;
+            uint8_t* tB = smem + SM::KZ + (2 * (TPT * rgrp + half) + buf_of(i)) * TILE;
+            uint8_t* tC = smem + SM::C + (TPT * rgrp + half) * TILE;
             const uint4 b0 = *reinterpret_cast<const uint4*>(tB + o0), b1 = *reinterpret_cast<const uint4*>(tB + o1);
             uint4 x0 = make_uint4(0u, 0u, 0u, 0u), x1 = x0;
             if (FULL) { x0 = *reinterpret_cast<const uint4*>(tC + o0); x1 = *reinterpret_cast<const uint4*>(tC + o1); }
@@ -395,52 +425,61 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
       bar_arrive(2, NT + 64);
 
       if (FULL) {
-        // ---- scores epilogue: decay, causal mask, diagonal -> 16-bit S tile.  The decay factors are computed ahead
-        // of the wait (waits and TMEM loads are compiler barriers); a warp whose cells all lie above the diagonal
-        // only writes zeros.
-        const bool empty = SC * cg > 16 * quad + 15;
-        float dfac[4 * SB];   // [hh][i][q]
-        if (!empty) {
-          float ls[2 * SB];
+        // ---- scores epilogue: decay, causal mask, diagonal -> 16-bit S tile.  The 16 rows of a warp meet SB / 2 blocks
+        // of 16 columns: left of the diagonal block (factored decays), on it, or right of it (zeros).  What does not
+        // depend on the scores is fetched ahead of the wait, which is a compiler barrier.
+        float fac[4 * SB];   // [k][q][hh]: factors of this thread's cells
+        float dg2[2] = {0.f, 0.f};
+        {
+          const float rf[2] = {sc[SC_ROW + rowA], sc[SC_ROW + rowB]};
 #pragma unroll
           for (int k = 0; k < SB; ++k) {
-            const float2 l2 = *reinterpret_cast<const float2*>(sc + SC_L2 + cg * SC + 8 * k + 2 * cq);
-            ls[2 * k] = l2.x; ls[2 * k + 1] = l2.y;
-          }
+            const int blk16 = (cg * SB + k) >> 1, s0 = cg * SC + 8 * k + 2 * cq;
+            if (blk16 < quad) {
+              const float2 cf = *reinterpret_cast<const float2*>(sc + SC_COL + 64 * quad + s0);
+              fac[4 * k] = cf.x * rf[0]; fac[4 * k + 1] = cf.x * rf[1];
+              fac[4 * k + 2] = cf.y * rf[0]; fac[4 * k + 3] = cf.y * rf[1];
+            } else if (blk16 == quad) {
+              const float2 ls = *reinterpret_cast<const float2*>(sc + SC_L2 + s0);
 #pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const float lt = sc[SC_L2 + (hh ? rowB : rowA)];
-#pragma unroll
-            for (int k = 0; k < 2 * SB; ++k) dfac[hh * 2 * SB + k] = ex2f(fminf(lt - ls[k], 0.f));
+              for (int hh = 0; hh < 2; ++hh) {
+                const int R = hh ? rowB : rowA;
+                const float lt = sc[SC_L2 + R];
+                fac[4 * k + hh] = s0 < R ? ex2f(fminf(lt - ls.x, 0.f)) : 0.f;
+                fac[4 * k + 2 + hh] = s0 + 1 < R ? ex2f(fminf(lt - ls.y, 0.f)) : 0.f;
+              }
+            } else {
+              fac[4 * k] = fac[4 * k + 1] = fac[4 * k + 2] = fac[4 * k + 3] = 0.f;
+            }
           }
         }
+        const bool has_diag = (quad * 2) / SB == cg, empty = cg * SB > 2 * quad + 1;
         live = live && wait_warp(&bar_mma[0], i & 1, 2);
         tc_fence_after_sync();
         if (live) {
           uint32_t r[4 * SB];
-          float dg2[2] = {0.f, 0.f};
-          if (!empty) {
-            tmem_ld_16x256<SB>(tmem + lane_base + cg * SC, r);
-            tmem_ld_wait();
+          if (!empty) tmem_ld_16x256<SB>(tmem + lane_base + cg * SC, r);
+          if (has_diag) {
             dg2[0] = s_diag[rowA]; dg2[1] = s_diag[rowB];
-            if (NB == 2) { dg2[0] += s_diag[64 + rowA]; dg2[1] += s_diag[64 + rowB]; }
+            if (NWQ == 4) { dg2[0] += s_diag[64 + rowA]; dg2[1] += s_diag[64 + rowB]; }
           }
+          tmem_ld_wait();
           uint8_t* tS = smem + SM::S + 4 * cq;
 #pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const int R = hh ? rowB : rowA;
+          for (int k = 0; k < SB; ++k) {
+            const int blk16 = (cg * SB + k) >> 1, s0 = cg * SC + 8 * k + 2 * cq;
 #pragma unroll
-            for (int k = 0; k < SB; ++k) {
+            for (int hh = 0; hh < 2; ++hh) {
+              const int R = hh ? rowB : rowA;
               uint32_t word = 0u;
-              if (!empty) {
-                float v2[2];
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                  const int s = cg * SC + 8 * k + 2 * cq + q;
-                  const float v = __uint_as_float(r[4 * k + 2 * hh + q]) * dfac[hh * 2 * SB + 2 * k + q];
-                  v2[q] = s < R ? v : (s == R ? dg2[hh] : 0.f);
+              if (blk16 <= quad) {
+                float v0 = __uint_as_float(r[4 * k + 2 * hh]) * fac[4 * k + hh];
+                float v1 = __uint_as_float(r[4 * k + 2 * hh + 1]) * fac[4 * k + 2 + hh];
+                if (blk16 == quad) {
+                  v0 = s0 == R ? dg2[hh] : v0;
+                  v1 = s0 + 1 == R ? dg2[hh] : v1;
                 }
-                word = PK::pack(v2[0], v2[1]);
+                word = PK::pack(v0, v1);
               }
               *reinterpret_cast<uint32_t*>(tS + sw128(R, cg * SB + k)) = word;
             }
@@ -459,9 +498,9 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
         const f2 E = dup2(e_end), R = dup2(ADJ ? e_end * ur : ur), I = dup2(ADJ ? e_end * ui : ui);
         const f2 NI = dup2(ADJ ? -e_end * ui : -ui);
 #pragma unroll
-        for (int part = 0; part < 2; ++part) {
+        for (int part = 0; part < ZC / 32; ++part) {
           uint32_t inc[16];
-          tmem_ld_16x256<4>(tmem + lane_base + TM_INC + 64 * cg + 32 * part, inc);
+          tmem_ld_16x256<4>(tmem + lane_base + TM_INC + ZC * cg + 32 * part, inc);
           tmem_ld_wait();
 #pragma unroll
           for (int m = 0; m < 2; ++m)
@@ -517,15 +556,15 @@ __global__ void __launch_bounds__(256 * NB + 64, NB == 1 ? 2 : 1)
       if (lane == 0) mbar_arrive(&bar_st);   // this warp's part of the Y and Zv tiles is complete
     }
     if (live && p.to_seg) {
-      float* dst = p.seg + ((size_t)bh * p.nseg + seg) * 64 * 128 * NB + 64 * cg + 2 * cq;
+      float* dst = p.seg + ((size_t)bh * p.nseg + seg) * 64 * 128 * NB + ZC * cg + 2 * cq;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < ZB; ++j) {
         *reinterpret_cast<float2*>(dst + (size_t)rowA * 128 * NB + 8 * j) = un2(zz[2 * j]);
         *reinterpret_cast<float2*>(dst + (size_t)rowB * 128 * NB + 8 * j) = un2(zz[2 * j + 1]);
       }
     } else if (live && p.zfinal && seg == p.nseg - 1) {
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
+      for (int m = 0; m < ZB / 2; ++m) {
         const int nn = n_of(m);
         if (nn >= p.N) continue;
 #pragma unroll

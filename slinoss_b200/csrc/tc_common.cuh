@@ -86,6 +86,12 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* m, uin
       : "memory");
 }
 
+// the same tile into L2 only
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* m, int x, int y, int z) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(m)),
+               "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
 // 3-D tiled store shared -> global (bulk async-group completion); rows beyond the tensor's
 // extent are clipped by the hardware.  The shared tile must have been made visible to the
 // async proxy (fence_async_smem by its writers, then a barrier) before this is issued.
@@ -165,6 +171,14 @@ __device__ __forceinline__ void bar_arrive(int id, int nthreads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// One lane of a converged warp.  The compiler knows that a single lane is active behind elect.sync and keeps the
+// descriptors of the MMAs issued there in uniform registers; behind ``lane == 0`` it moved them for every
+// instruction (60 - 90 clocks per MMA).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
 // D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.
 __device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                      uint32_t accumulate) {
