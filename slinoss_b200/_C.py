@@ -6,15 +6,16 @@ Two layers live here:
   declares the prototypes of every ``sl_*`` symbol of ``include/slinoss_b200.h``.
   There is no fallback: if the library is missing, ``lib()`` raises.
 * tensor-level launchers (``scan_fwd``, ``scan_bwd``, ``scan_decode``,
-  ``scanprep_conv_fwd`` ...) that allocate outputs and scratch with torch, pass raw
-  device pointers and torch's *current stream* to the C functions and turn
-  non-zero status codes into exceptions.  The ops in ``slinoss_b200.ops`` only
-  talk to these launchers.
+  ``scanprep_conv_fwd`` ...): names and defaults for the functions of the native host
+  module (``csrc/host.cpp``), which allocate outputs and scratch with torch, launch on
+  torch's *current stream* and turn non-zero status codes into exceptions.  The ops in
+  ``slinoss_b200.ops`` only talk to these launchers.
 """
 
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_float, c_int, c_int64, c_size_t, c_void_p
 from pathlib import Path
 
@@ -94,6 +95,52 @@ def lib():
     return _lib
 
 
+_HOST_PATH = _LIB_PATH.parent / "_host.so"
+_host_module = None
+
+
+def host():
+    """The native host module (the launchers for torch tensors).  Raises if it has not been built."""
+    global _host_module
+    if _host_module is None:
+        lib()
+        if not _HOST_PATH.exists():
+            raise RuntimeError(
+                f"slinoss_b200: host module {_HOST_PATH} is missing. Build it with "
+                "`python -m slinoss_b200.build`; there is no fallback path.")
+        import importlib.util
+        spec = importlib.util.spec_from_file_location("_host", _HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _host_module = module
+    return _host_module
+
+
+def opaque(fn):
+    """Keep ``fn`` out of ``torch.compile`` graphs.  ``torch.compiler.disable`` alone costs 3 us on every eager call;
+    here the eager call goes straight through and only a trace meets the disabled function."""
+    disabled = torch.compiler.disable(fn)
+
+    @functools.wraps(fn)
+    def call(*args, **kwargs):
+        return disabled(*args, **kwargs) if torch.compiler.is_compiling() else fn(*args, **kwargs)
+    return call
+
+
+def grad_needed(*tensors) -> bool:
+    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
+
+
+def as_f32(t: torch.Tensor) -> torch.Tensor:
+    """``t`` itself when it is dense float32 already, else a float32 copy."""
+    return t if t.dtype is torch.float32 and t.is_contiguous() else t.detach().to(torch.float32).contiguous()
+
+
+def as_type(t, dtype):
+    """``t`` itself when it is dense and of ``dtype`` already (or None), else a copy."""
+    return t if t is None or (t.dtype is dtype and t.is_contiguous()) else t.detach().to(dtype).contiguous()
+
+
 def kernel_launches() -> int:
     """Kernels launched by the library in this process so far."""
     return int(lib().sl_kernel_launches())
@@ -148,13 +195,6 @@ def _stream(dev) -> int:
     return torch.cuda.current_stream(dev).cuda_stream
 
 
-def _workspace(kind, dev, batch, heads, groups, T, P, N, chunk, io, path):
-    nbytes = lib().sl_workspace_bytes(kind, batch, heads, groups, T, P, N, chunk, io, path)
-    if nbytes == 0:
-        return None, 0
-    return torch.empty(nbytes, dtype=torch.uint8, device=dev), nbytes
-
-
 def workspace_bytes(kind, batch, heads, groups, T, P, N, chunk, io_dtype, path="auto") -> int:
     return int(lib().sl_workspace_bytes(kind, batch, heads, groups, T, P, N, chunk,
                                         dtype_code(io_dtype), _PATHS[path]))
@@ -168,28 +208,9 @@ def scan_fwd(U, M, K, B, C, z0, B_prev, U_prev, *, chunk_size, y_dtype, want_fin
     """Launch ``sl_v2x2ssd_fwd``.  ``U,B,C,B_prev,U_prev`` share one dtype; ``M,K,z0``
     are float32.  Returns ``(Y, final_state or None)``; with ``save_states`` a third item:
     the chunk-state buffer for ``scan_bwd`` (None when the chosen path keeps none)."""
-    dev = require_cuda(U, M, K, B, C, z0, B_prev, U_prev)
-    batch, heads, T, P = U.shape
-    groups, N = B.shape[1], B.shape[3] // 2
-    io, pcode = dtype_code(U.dtype), _PATHS[path]
-    Y = torch.empty((batch, heads, T, P), dtype=y_dtype, device=dev)
-    states = None
-    with torch.cuda.device(dev):
-        if save_states:
-            sbytes = lib().sl_workspace_bytes(WS_SCAN_STATES, batch, heads, groups, T, P, N,
-                                              chunk_size, io, pcode)
-            if sbytes:
-                states = torch.empty(sbytes, dtype=torch.uint8, device=dev)
-        final = torch.empty((batch, heads, P, 2 * N), dtype=torch.float32, device=dev) \
-            if (want_final or states is not None) else None
-        ws, nbytes = _workspace(WS_SCAN_FWD, dev, batch, heads, groups, T, P, N, chunk_size, io, pcode)
-        check(lib().sl_v2x2ssd_fwd(
-            _ptr(U), _ptr(M), _ptr(K), _ptr(B), _ptr(C), _ptr(z0), _ptr(B_prev), _ptr(U_prev),
-            _ptr(Y), _ptr(final), _ptr(states), batch, heads, groups, T, P, N, chunk_size, io,
-            dtype_code(y_dtype), pcode, _ptr(ws), nbytes, _stream(dev)), "sl_v2x2ssd_fwd")
-    if save_states:
-        return Y, final, states
-    return Y, final
+    out = host().scan_fwd(U, M, K, B, C, z0, B_prev, U_prev, chunk_size, dtype_code(y_dtype), want_final,
+                          _PATHS[path], save_states)
+    return out if save_states else out[:2]
 
 
 def scan_bwd(U, M, K, B, C, z0, B_prev, U_prev, dY, d_final, *, chunk_size, path="auto",
@@ -197,30 +218,8 @@ def scan_bwd(U, M, K, B, C, z0, B_prev, U_prev, dY, d_final, *, chunk_size, path
     """Launch ``sl_v2x2ssd_bwd``.  Returns ``(dU, dM, dK, dB, dC, d_initial, dB_prev,
     dU_prev)``; the last three are None when the matching input is absent.  ``saved`` is
     ``(chunk_states, final_state)`` from ``scan_fwd(..., save_states=True)`` or None."""
-    dev = require_cuda(U, M, K, B, C, z0, B_prev, U_prev, dY, d_final)
     states, zfinal = saved if (saved is not None and saved[0] is not None) else (None, None)
-    batch, heads, T, P = U.shape
-    groups, N = B.shape[1], B.shape[3] // 2
-    io, pcode = dtype_code(U.dtype), _PATHS[path]
-    dU = torch.empty_like(U)
-    dM = torch.empty((batch, heads, T, 2), dtype=torch.float32, device=dev)
-    dK = torch.empty((batch, heads, T, 2, 2), dtype=torch.float32, device=dev)
-    dB = torch.empty_like(B)
-    dC = torch.empty_like(C)
-    d_init = torch.empty((batch, heads, P, 2 * N), dtype=torch.float32, device=dev) \
-        if z0 is not None else None
-    dB_prev = torch.empty_like(B_prev) if B_prev is not None else None
-    dU_prev = torch.empty_like(U_prev) if U_prev is not None else None
-    dy_code = dtype_code(dY.dtype) if dY is not None else io
-    with torch.cuda.device(dev):
-        ws, nbytes = _workspace(WS_SCAN_BWD, dev, batch, heads, groups, T, P, N, chunk_size, io, pcode)
-        check(lib().sl_v2x2ssd_bwd(
-            _ptr(U), _ptr(M), _ptr(K), _ptr(B), _ptr(C), _ptr(z0), _ptr(B_prev), _ptr(U_prev),
-            _ptr(states), _ptr(zfinal), _ptr(dY), _ptr(d_final), _ptr(dU), _ptr(dM), _ptr(dK),
-            _ptr(dB), _ptr(dC), _ptr(d_init), _ptr(dB_prev), _ptr(dU_prev), batch, heads, groups,
-            T, P, N, chunk_size, io, dy_code, pcode, _ptr(ws), nbytes, _stream(dev)),
-            "sl_v2x2ssd_bwd")
-    return dU, dM, dK, dB, dC, d_init, dB_prev, dU_prev
+    return host().scan_bwd(U, M, K, B, C, z0, B_prev, U_prev, states, zfinal, dY, d_final, chunk_size, _PATHS[path])
 
 
 def scan_bwd_static(U, M, K, B, C, z0, B_prev, U_prev, dY, d_final, outs):
@@ -245,18 +244,7 @@ def scan_bwd_static(U, M, K, B, C, z0, B_prev, U_prev, dY, d_final, outs):
 def scan_decode(U, M, K, B, C, state, B_prev, U_prev, *, y_dtype, state_out=None):
     """Launch ``sl_v2x2ssd_decode``: one token over the carried float32 state.
     ``state_out`` defaults to a fresh tensor; pass ``state`` itself to update in place."""
-    dev = require_cuda(U, M, K, B, C, state, B_prev, U_prev)
-    batch, heads, P = U.shape
-    groups, N = B.shape[1], B.shape[2] // 2
-    Y = torch.empty((batch, heads, P), dtype=y_dtype, device=dev)
-    if state_out is None:
-        state_out = torch.empty_like(state)
-    with torch.cuda.device(dev):
-        check(lib().sl_v2x2ssd_decode(
-            _ptr(U), _ptr(M), _ptr(K), _ptr(B), _ptr(C), _ptr(state), _ptr(B_prev), _ptr(U_prev),
-            _ptr(Y), _ptr(state_out), batch, heads, groups, P, N, dtype_code(U.dtype),
-            dtype_code(y_dtype), _stream(dev)), "sl_v2x2ssd_decode")
-    return Y, state_out
+    return host().scan_decode(U, M, K, B, C, state, B_prev, U_prev, dtype_code(y_dtype), state_out)
 
 
 # ---------------------------------------------------------------------------------
@@ -266,6 +254,13 @@ def make_config(owner) -> ScanPrepConfig:
     return ScanPrepConfig(owner.dt_min, owner.dt_max, owner.alpha_min, owner.alpha_max,
                           owner.theta_init_min, owner.theta_init_max, owner.theta_mod_scale,
                           owner.r_min, owner.r_max, owner.eps)
+
+
+CONFIG_FIELDS = tuple(n for n, _ in ScanPrepConfig._fields_)
+
+
+def _config_values(cfg):
+    return None if cfg is None else [getattr(cfg, n) for n in CONFIG_FIELDS]
 
 
 def _row_stride(x: torch.Tensor) -> int:
@@ -292,44 +287,8 @@ def scanprep_conv_fwd(value, conv_weight, conv_bias, conv_state, params, bc, bia
     ``bc`` (batch,T,groups,4,N) or None; ``biases`` = (dt_bias, alpha_bias, theta_mod_bias,
     theta_bias, theta_sign).  Returns ``(U, M, K, B, C, next_conv_state)`` with None for
     skipped parts.  ``u_layout`` "bhtp" gives (batch,heads,T,P), "btc" (batch,T,heads*P)."""
-    ref = value if value is not None else (params if params is not None else bc)
-    dev = require_cuda(value, conv_weight, conv_bias, conv_state, params, bc, *(biases or ()))
-    batch, T = ref.shape[0], ref.shape[1]
-    io = dtype_code(ref.dtype)
-    U = M = K = Bo = Co = nstate = None
-    usb = ush = ust = 0
-    vstride = 0
-    d_conv = 1
-    if value is not None:
-        value = as_rows(value)
-        vstride = _row_stride(value)
-        if u_layout == "bhtp":
-            U = torch.empty((batch, heads, T, P), dtype=value.dtype, device=dev)
-            usb, ush, ust = heads * T * P, T * P, P
-        else:
-            U = torch.empty((batch, T, heads * P), dtype=value.dtype, device=dev)
-            usb, ush, ust = T * heads * P, P, heads * P
-        if conv_weight is not None:
-            d_conv = int(conv_weight.shape[1])
-            if want_state:
-                nstate = torch.empty((batch, heads * P, d_conv - 1), dtype=value.dtype, device=dev)
-    groups = N = 1
-    if bc is not None:
-        groups, N = int(bc.shape[2]), int(bc.shape[4])
-        Bo = torch.empty((batch, groups, T, 2 * N), dtype=bc.dtype, device=dev)
-        Co = torch.empty_like(Bo)
-    if params is not None:
-        M = torch.empty((batch, heads, T, 2), dtype=torch.float32, device=dev)
-        K = torch.empty((batch, heads, T, 2, 2), dtype=torch.float32, device=dev)
-    b5 = list(biases) if biases is not None else [None] * 5
-    with torch.cuda.device(dev):
-        check(lib().sl_scanprep_conv_fwd(
-            _ptr(value), vstride, _ptr(conv_weight), _ptr(conv_bias), _ptr(conv_state),
-            _ptr(nstate), d_conv, _ptr(params), _ptr(bc), *[_ptr(b) for b in b5],
-            ctypes.byref(cfg) if cfg is not None else None, _ptr(U), usb, ush, ust, _ptr(M),
-            _ptr(K), _ptr(Bo), _ptr(Co), batch, heads, groups, T, P, N, io, _stream(dev)),
-            "sl_scanprep_conv_fwd")
-    return U, M, K, Bo, Co, nstate
+    return host().scanprep_fwd(value, conv_weight, conv_bias, conv_state, params, bc, biases or (),
+                               _config_values(cfg), heads, P, u_layout == "bhtp", want_state)
 
 
 def scanprep_conv_bwd(value, conv_weight, conv_bias, conv_state, params, bc, biases, cfg, dU, dM,
@@ -338,54 +297,10 @@ def scanprep_conv_bwd(value, conv_weight, conv_bias, conv_state, params, bc, bia
     d_conv_bias, d_conv_state, d_params, d_bc, d_dt_bias, d_alpha_bias,
     d_theta_mod_bias, d_theta_bias (None for skipped parts; bias / weight gradients
     are float32 accumulators)."""
-    ref = value if value is not None else (params if params is not None else bc)
-    dev = require_cuda(value, conv_weight, conv_bias, conv_state, params, bc, dU, dM, dK, dBo, dCo)
-    batch, T = ref.shape[0], ref.shape[1]
-    io = dtype_code(ref.dtype)
-    out = dict.fromkeys(("d_value", "d_conv_weight", "d_conv_bias", "d_conv_state", "d_params",
-                         "d_bc", "d_dt_bias", "d_alpha_bias", "d_theta_mod_bias", "d_theta_bias"))
-    usb = ush = ust = 0
-    vstride = 0
-    d_conv = 1
-    f32 = dict(dtype=torch.float32, device=dev)
-    if dU is not None:
-        value = as_rows(value)
-        vstride = _row_stride(value)
-        dU = dU.contiguous()
-        if u_layout == "bhtp":
-            usb, ush, ust = heads * T * P, T * P, P
-        else:
-            usb, ush, ust = T * heads * P, P, heads * P
-        out["d_value"] = torch.empty((batch, T, heads * P), dtype=value.dtype, device=dev)
-        if conv_weight is not None:
-            d_conv = int(conv_weight.shape[1])
-            out["d_conv_weight"] = torch.zeros((heads * P, d_conv), **f32)
-            out["d_conv_bias"] = torch.zeros((heads * P,), **f32)
-            if want_dstate and d_conv > 1:
-                out["d_conv_state"] = torch.zeros((batch, heads * P, d_conv - 1),
-                                                  dtype=value.dtype, device=dev)
-    groups = N = 1
-    if dBo is not None:
-        groups, N = int(bc.shape[2]), int(bc.shape[4])
-        dBo, dCo = dBo.contiguous(), dCo.contiguous()
-        out["d_bc"] = torch.empty(bc.shape, dtype=bc.dtype, device=dev)
-    if dM is not None:
-        dM, dK = dM.contiguous(), dK.contiguous()
-        out["d_params"] = torch.empty(params.shape, dtype=params.dtype, device=dev)
-        for k in ("d_dt_bias", "d_alpha_bias", "d_theta_mod_bias", "d_theta_bias"):
-            out[k] = torch.zeros((heads,), **f32)
-    b5 = list(biases) if biases is not None else [None] * 5
-    with torch.cuda.device(dev):
-        check(lib().sl_scanprep_conv_bwd(
-            _ptr(value), vstride, _ptr(conv_weight), _ptr(conv_bias), _ptr(conv_state), d_conv,
-            _ptr(params), _ptr(bc), *[_ptr(b) for b in b5],
-            ctypes.byref(cfg) if cfg is not None else None, _ptr(dU), usb, ush, ust, _ptr(dM),
-            _ptr(dK), _ptr(dBo), _ptr(dCo), _ptr(out["d_value"]), _ptr(out["d_conv_weight"]),
-            _ptr(out["d_conv_bias"]), _ptr(out["d_conv_state"]), _ptr(out["d_params"]),
-            _ptr(out["d_bc"]), _ptr(out["d_dt_bias"]), _ptr(out["d_alpha_bias"]),
-            _ptr(out["d_theta_mod_bias"]), _ptr(out["d_theta_bias"]), batch, heads, groups, T, P,
-            N, io, _stream(dev)), "sl_scanprep_conv_bwd")
-    return out
+    out = host().scanprep_bwd(value, conv_weight, conv_bias, conv_state, params, bc, biases or (),
+                              _config_values(cfg), dU, dM, dK, dBo, dCo, heads, P, u_layout == "bhtp", want_dstate)
+    return dict(zip(("d_value", "d_conv_weight", "d_conv_bias", "d_conv_state", "d_params", "d_bc", "d_dt_bias",
+                     "d_alpha_bias", "d_theta_mod_bias", "d_theta_bias"), out))
 
 
 # ---------------------------------------------------------------------------------
@@ -393,36 +308,13 @@ def scanprep_conv_bwd(value, conv_weight, conv_bias, conv_state, params, bc, bia
 # ---------------------------------------------------------------------------------
 def mixer_tail_fwd(Y, gate, skip, d_skip, norm_weight, eps):
     """Launch ``sl_mixer_tail_fwd``.  Returns normed (batch,T,heads*P)."""
-    dev = require_cuda(Y, gate, skip, d_skip, norm_weight)
-    batch, heads, T, P = Y.shape
-    gate = as_rows(gate)
-    normed = torch.empty((batch, T, heads * P), dtype=Y.dtype, device=dev)
-    with torch.cuda.device(dev):
-        check(lib().sl_mixer_tail_fwd(
-            _ptr(Y), _ptr(gate), _row_stride(gate), _ptr(skip), _ptr(d_skip), _ptr(norm_weight),
-            float(eps), _ptr(normed), batch, heads, T, P, dtype_code(Y.dtype), _stream(dev)),
-            "sl_mixer_tail_fwd")
-    return normed
+    return host().tail_fwd(Y, gate, skip, d_skip, norm_weight, eps)
 
 
 def mixer_tail_bwd(Y, gate, skip, d_skip, norm_weight, eps, d_normed):
     """Launch ``sl_mixer_tail_bwd``.  Returns ``(dY, d_gate, d_skip_input, d_d_skip,
     d_norm_weight)``; the last two are float32 accumulators."""
-    dev = require_cuda(Y, gate, skip, d_skip, norm_weight, d_normed)
-    batch, heads, T, P = Y.shape
-    gate = as_rows(gate)
-    d_normed = d_normed.contiguous()
-    dY = torch.empty_like(Y)
-    d_gate = torch.empty((batch, T, heads * P), dtype=Y.dtype, device=dev)
-    d_skip_in = torch.empty_like(Y) if skip is not None else None
-    d_d_skip = torch.zeros((heads,), dtype=torch.float32, device=dev) if skip is not None else None
-    d_w = torch.zeros((heads * P,), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        check(lib().sl_mixer_tail_bwd(
-            _ptr(Y), _ptr(gate), _row_stride(gate), _ptr(skip), _ptr(d_skip), _ptr(norm_weight),
-            float(eps), _ptr(d_normed), _ptr(dY), _ptr(d_gate), _ptr(d_skip_in), _ptr(d_d_skip),
-            _ptr(d_w), batch, heads, T, P, dtype_code(Y.dtype), _stream(dev)), "sl_mixer_tail_bwd")
-    return dY, d_gate, d_skip_in, d_d_skip, d_w
+    return host().tail_bwd(Y, gate, skip, d_skip, norm_weight, eps, d_normed)
 
 
 # ---------------------------------------------------------------------------------
@@ -472,47 +364,18 @@ def rmsnorm_supported(C: int, dtype: torch.dtype) -> bool:
 
 def rmsnorm_fwd(x, weight, eps):
     """``x (..., C)`` dense -> same shape; launches ``sl_rmsnorm_fwd``."""
-    dev = require_cuda(x, weight)
-    C = int(x.shape[-1])
-    out = torch.empty_like(x)
-    with torch.cuda.device(dev):
-        check(lib().sl_rmsnorm_fwd(_ptr(x), _ptr(weight), float(eps), _ptr(out), x.numel() // C, C,
-                                   dtype_code(x.dtype), _stream(dev)), "sl_rmsnorm_fwd")
-    return out
+    return host().rmsnorm_fwd(x, weight, eps)
 
 
 def rmsnorm_bwd(x, weight, eps, d_out):
     """Returns ``(d_x, d_weight float32)``."""
-    dev = require_cuda(x, weight, d_out)
-    C = int(x.shape[-1])
-    d_x = torch.empty_like(x)
-    d_w = torch.zeros(C, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        check(lib().sl_rmsnorm_bwd(_ptr(x), _ptr(weight), float(eps), _ptr(d_out), _ptr(d_x), _ptr(d_w),
-                                   x.numel() // C, C, dtype_code(x.dtype), _stream(dev)), "sl_rmsnorm_bwd")
-    return d_x, d_w
+    return host().rmsnorm_bwd(x, weight, eps, d_out)
 
 
 def ffn_activation_fwd(projected, kind: str):
     """``projected (..., W)`` dense, W = hidden (gelu) or 2*hidden (swiglu) -> ``hidden (..., hidden)``."""
-    dev = require_cuda(projected)
-    W = int(projected.shape[-1])
-    H = W // 2 if kind == "swiglu" else W
-    hidden = torch.empty(projected.shape[:-1] + (H,), dtype=projected.dtype, device=dev)
-    with torch.cuda.device(dev):
-        check(lib().sl_ffn_activation_fwd(_ptr(projected), _ptr(hidden), projected.numel() // W, H,
-                                          FFN_KINDS[kind], dtype_code(projected.dtype), _stream(dev)),
-              "sl_ffn_activation_fwd")
-    return hidden
+    return host().ffn_act_fwd(projected, FFN_KINDS[kind])
 
 
 def ffn_activation_bwd(projected, d_hidden, kind: str):
-    dev = require_cuda(projected, d_hidden)
-    W = int(projected.shape[-1])
-    H = W // 2 if kind == "swiglu" else W
-    d_proj = torch.empty_like(projected)
-    with torch.cuda.device(dev):
-        check(lib().sl_ffn_activation_bwd(_ptr(projected), _ptr(d_hidden), _ptr(d_proj), projected.numel() // W, H,
-                                          FFN_KINDS[kind], dtype_code(projected.dtype), _stream(dev)),
-              "sl_ffn_activation_bwd")
-    return d_proj
+    return host().ffn_act_bwd(projected, d_hidden, FFN_KINDS[kind])

@@ -12,7 +12,9 @@ import torch
 import torch.nn.functional as F
 from torch import nn
 
+from .. import _C
 from ..layers import RMSNorm, SLinOSSMixer
+from ..layers.mixer import _norm_eps
 from ..layers.mlp import SLinOSSMLP
 from ..ops.block import ffn_residual, ffn_residual_supported, residual_add
 from .config import SLinOSSBlockConfig
@@ -28,6 +30,29 @@ def make_norm(kind, d_model, *, eps, device=None, dtype=None) -> nn.Module:
 def apply_norm(norm: nn.Module, x: torch.Tensor) -> torch.Tensor:
     w = getattr(norm, "weight", None)
     return norm(x.to(dtype=w.dtype)) if isinstance(w, torch.Tensor) else norm(x)
+
+
+def _plain_rmsnorm(norm, x) -> bool:
+    if type(norm) is not RMSNorm or norm._forward_hooks or norm._forward_pre_hooks:
+        return False
+    w = norm._parameters["weight"]
+    return (w is not None and w.dtype == x.dtype and w.device == x.device and w.shape == x.shape[-1:]
+            and x.dtype in (torch.bfloat16, torch.float16) and _C.rmsnorm_supported(int(x.shape[-1]), x.dtype))
+
+
+def _plain_linear(layer, x) -> bool:
+    w, b = layer._parameters["weight"], layer._parameters["bias"]
+    return (type(layer) is nn.Linear and not layer._forward_hooks and not layer._forward_pre_hooks
+            and w.dtype == x.dtype and w.device == x.device and w.is_contiguous()
+            and (b is None or b.dtype == x.dtype))
+
+
+@_C.opaque
+def _ffn_token(x, norm, ffn):
+    """``x + ffn(norm(x))`` for the rows of one token: two launches for small batches."""
+    w1, w2 = ffn.in_proj._parameters, ffn.out_proj._parameters
+    return _C.host().ffn_token(x, norm.weight, _norm_eps(norm), w1["weight"], w1["bias"], w2["weight"], w2["bias"],
+                               _C.FFN_KINDS[ffn.kind])
 
 
 class SLinOSSBlock(nn.Module):
@@ -85,6 +110,27 @@ class SLinOSSBlock(nn.Module):
             out = self._ffn_residual(out)
         return (out, nxt) if return_state else out
 
+    def _native_step(self, token, state, inplace):
+        """The whole step in five launches (see ``SLinOSSMixer.decode_native``), or None when something asks for the
+        composed path: gradients, another norm, dropout, autocast, hooks, an injected backend, a partial state."""
+        mixer = self.mixer
+        if torch.is_grad_enabled() or state is None or not token.is_cuda or (inplace is not None and not inplace) or \
+                (self.residual_dropout > 0.0 and self.training) or type(mixer) is not SLinOSSMixer:
+            return None
+        norm, ms = self.mixer_norm, state.mixer
+        if not (_plain_rmsnorm(norm, token) and mixer._fused_decode_ready(ms, token)
+                and mixer._native_decode_ready(token)) or mixer._forward_hooks or mixer._forward_pre_hooks:
+            return None
+        ffn = self.ffn
+        if ffn is not None and not (_plain_rmsnorm(self.ffn_norm, token) and type(ffn) is SLinOSSMLP
+                                    and not ffn._forward_hooks and not ffn._forward_pre_hooks
+                                    and _plain_linear(ffn.in_proj, token) and _plain_linear(ffn.out_proj, token)):
+            return None
+        out = mixer.decode_native(token, ms, pre_norm=norm, residual=token)
+        if ffn is not None:
+            out = _ffn_token(out, self.ffn_norm, ffn)
+        return out, SLinOSSBlockState(mixer=ms)
+
     def step(self, x, state: SLinOSSBlockState | None = None, *, inplace=None, context=None):
         token = x
         if token.ndim == 3:
@@ -94,6 +140,9 @@ class SLinOSSBlock(nn.Module):
         if token.ndim != 2 or token.shape[-1] != self.d_model:
             raise ValueError(f"Expected x shape (batch, {self.d_model}) or "
                              f"(batch, 1, {self.d_model}), got {tuple(x.shape)}.")
+        done = self._native_step(token, state, inplace)
+        if done is not None:
+            return done if x.ndim == 2 else (done[0].unsqueeze(1), done[1])
         mixed, mixer_state = self.mixer.step(apply_norm(self.mixer_norm, token),
                                              None if state is None else state.mixer, inplace=inplace)
         out = self._add(token, self._drop(mixed.to(dtype=token.dtype)))

@@ -27,6 +27,7 @@ int scan_tc_bwd(const void* U, const float* M, const float* K, const void* B, co
                 int dy_dtype, void* ws, size_t ws_bytes, cudaStream_t st);
 
 int scan_tc_device_status(bool reset);
+int mixer_step_device_status(bool reset);   // mixer_step.cu
 
 namespace {
 
@@ -63,10 +64,13 @@ extern "C" unsigned long long sl_kernel_launches(void) {
 }
 
 extern "C" int sl_device_status(void) {
-  return sl::scan_tc_device_status(false) != 0 ? SL_ERR_DEVICE_TIMEOUT : SL_OK;
+  return sl::scan_tc_device_status(false) != 0 || sl::mixer_step_device_status(false) != 0 ? SL_ERR_DEVICE_TIMEOUT : SL_OK;
 }
 
-extern "C" int sl_device_status_reset(void) { return sl::scan_tc_device_status(true); }
+extern "C" int sl_device_status_reset(void) {
+  const int scan = sl::scan_tc_device_status(true), step = sl::mixer_step_device_status(true);
+  return scan ? scan : step;
+}
 
 extern "C" const char* sl_last_cuda_error(void) {
   return cudaGetErrorString((cudaError_t)sl::g_cuda_error.load(std::memory_order_relaxed));

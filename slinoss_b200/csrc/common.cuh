@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/slinoss_b200.h"
 
 namespace sl {
@@ -102,6 +104,21 @@ __device__ __forceinline__ float warp_sum(float v) {
 __device__ __forceinline__ float silu_f(float x) { return __fdividef(x, 1.f + __expf(-x)); }
 __device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 
+// 16-bit rows take the one-instruction tanh (relative error 2^-11, below the rounding of the output);
+// float32 rows the precise one.
+template <bool FAST> __device__ __forceinline__ float tanh_io(float x) {
+  if (FAST) {
+    float y;
+    asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+  }
+  return tanhf(x);
+}
+template <bool FAST> __device__ __forceinline__ float gelu_tanh_f(float x) {
+  const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
+  return 0.5f * x * (1.f + tanh_io<FAST>(u));
+}
+
 // ---- host side -----------------------------------------------------------------
 inline size_t dtype_size(int dt) { return dt == SL_F32 ? 4 : 2; }
 inline bool dtype_ok(int dt) { return dt == SL_F32 || dt == SL_BF16 || dt == SL_F16; }
@@ -119,6 +136,19 @@ inline int launch_status() {
   if (e == cudaSuccess) return SL_OK;
   note_cuda_error((int)e);
   return SL_ERR_LAUNCH_FAILED;
+}
+
+// Kernel attributes stick to a device: set once per (kernel, device) instead of on every launch.
+template <typename F>
+inline int ensure_smem(F k, size_t bytes, std::atomic<unsigned long long>& done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return SL_ERR_LAUNCH_FAILED;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (done.load(std::memory_order_relaxed) & bit) return SL_OK;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+    return SL_ERR_LAUNCH_FAILED;
+  done.fetch_or(bit, std::memory_order_relaxed);
+  return SL_OK;
 }
 
 // Dispatch a callable templated on the io element type.

@@ -124,20 +124,6 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_kernel(const T* __restrict
   }
 }
 
-// 16-bit rows take the one-instruction tanh (relative error 2^-11, below the rounding of the output);
-// float32 rows the precise one.
-template <bool FAST> __device__ __forceinline__ float tanh_io(float x) {
-  if (FAST) {
-    float y;
-    asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-  }
-  return tanhf(x);
-}
-template <bool FAST> __device__ __forceinline__ float gelu_tanh_f(float x) {
-  const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-  return 0.5f * x * (1.f + tanh_io<FAST>(u));
-}
 template <bool FAST> __device__ __forceinline__ float dgelu_tanh_f(float x) {
   const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
   const float t = tanh_io<FAST>(u);

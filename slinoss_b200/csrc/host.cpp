@@ -1,0 +1,389 @@
+// Host module of the package: the launchers of the C ABI for torch tensors, in native code.
+//
+// A launch from Python cost 15 to 30 us of interpreter time (argument conversion of up to 40 ctypes arguments, device
+// guard, stream lookup, output allocation); the same work takes 2 to 4 us here.  Every function allocates its outputs
+// and scratch with torch, launches on torch's current stream and turns status codes into exceptions.
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include "../../include/slinoss_b200.h"
+#include "host_abi.h"
+
+namespace {
+
+using at::Tensor;
+using OptT = c10::optional<Tensor>;
+
+int code_of(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return SL_F32;
+    case at::kBFloat16: return SL_BF16;
+    case at::kHalf: return SL_F16;
+    default: throw pybind11::value_error("unsupported dtype; expected float32, bfloat16 or float16");
+  }
+}
+at::ScalarType type_of(int code) { return code == SL_F32 ? at::kFloat : code == SL_BF16 ? at::kBFloat16 : at::kHalf; }
+
+void check(int status, const char* what) {
+  if (status == SL_OK) return;
+  std::string text = std::string("slinoss_b200.") + what + " failed with status " + std::to_string(status) + ": " +
+                     sl_status_string(status);
+  if (status == SL_ERR_LAUNCH_FAILED) text += std::string(" (") + sl_last_cuda_error() + ")";
+  throw std::runtime_error(text);
+}
+
+// Device guard and stream of a call; every tensor handed to it must live on one CUDA device.
+struct Call {
+  c10::cuda::OptionalCUDAGuard guard;
+  c10::Device dev{c10::kCPU};
+  bool any = false;
+  void need(const Tensor& t) {
+    if (!t.is_cuda()) throw pybind11::value_error("slinoss_b200 kernels require CUDA tensors.");
+    if (!any) { dev = t.device(); any = true; }
+    else if (t.device() != dev) throw pybind11::value_error("All tensors must be on the same device.");
+  }
+  void need(const OptT& t) { if (t) need(*t); }
+  template <typename... Ts> explicit Call(const Ts&... ts) { (need(ts), ...); guard.set_device(dev); }
+  void* stream() const { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
+  Tensor empty(at::IntArrayRef shape, at::ScalarType t) const { return at::empty(shape, at::TensorOptions().dtype(t).device(dev)); }
+  Tensor zeros(at::IntArrayRef shape, at::ScalarType t) const { return at::zeros(shape, at::TensorOptions().dtype(t).device(dev)); }
+  Tensor bytes(size_t n) const { return empty({(int64_t)n}, at::kByte); }
+};
+
+const void* ptr(const Tensor& t) { return t.data_ptr(); }
+const void* ptr(const OptT& t) { return t ? t->data_ptr() : nullptr; }
+void* mptr(const Tensor& t) { return t.data_ptr(); }
+void* mptr(const OptT& t) { return t ? t->data_ptr() : nullptr; }
+const float* fptr(const Tensor& t) { return static_cast<const float*>(t.data_ptr()); }
+const float* fptr(const OptT& t) { return t ? static_cast<const float*>(t->data_ptr()) : nullptr; }
+float* mfptr(const Tensor& t) { return static_cast<float*>(t.data_ptr()); }
+float* mfptr(const OptT& t) { return t ? static_cast<float*>(t->data_ptr()) : nullptr; }
+
+using Config = std::array<float, 10>;
+sl_scanprep_config config_of(const Config& c) {
+  return sl_scanprep_config{c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], c[8], c[9]};
+}
+
+// ---- scan ---------------------------------------------------------------------------------------------------------
+std::tuple<Tensor, OptT, OptT> scan_fwd(const Tensor& U, const Tensor& M, const Tensor& K, const Tensor& B, const Tensor& C,
+                                        const OptT& z0, const OptT& Bp, const OptT& Up, int chunk, int y_code,
+                                        bool want_final, int path, bool save_states) {
+  Call call(U, M, K, B, C, z0, Bp, Up);
+  const int batch = U.size(0), heads = U.size(1), T = U.size(2), P = U.size(3), groups = B.size(1), N = B.size(3) / 2;
+  const int io = code_of(U.scalar_type());
+  Tensor Y = call.empty({batch, heads, T, P}, type_of(y_code));
+  OptT final_state, states, ws;
+  if (save_states) {
+    const size_t n = sl_workspace_bytes(SL_WS_SCAN_STATES, batch, heads, groups, T, P, N, chunk, io, path);
+    if (n) states = call.bytes(n);
+  }
+  if (want_final || states) final_state = call.empty({batch, heads, P, 2 * N}, at::kFloat);
+  const size_t n = sl_workspace_bytes(SL_WS_SCAN_FWD, batch, heads, groups, T, P, N, chunk, io, path);
+  if (n) ws = call.bytes(n);
+  check(sl_v2x2ssd_fwd(ptr(U), fptr(M), fptr(K), ptr(B), ptr(C), fptr(z0), ptr(Bp), ptr(Up), mptr(Y), mfptr(final_state),
+                       mptr(states), batch, heads, groups, T, P, N, chunk, io, y_code, path, mptr(ws), n, call.stream()),
+        "sl_v2x2ssd_fwd");
+  return {Y, final_state, states};
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, OptT, OptT, OptT> scan_bwd(
+    const Tensor& U, const Tensor& M, const Tensor& K, const Tensor& B, const Tensor& C, const OptT& z0, const OptT& Bp,
+    const OptT& Up, const OptT& states, const OptT& final_state, const OptT& dY, const OptT& dfinal, int chunk, int path) {
+  Call call(U, M, K, B, C, z0, Bp, Up, dY, dfinal);
+  const int batch = U.size(0), heads = U.size(1), T = U.size(2), P = U.size(3), groups = B.size(1), N = B.size(3) / 2;
+  const int io = code_of(U.scalar_type()), dy = dY ? code_of(dY->scalar_type()) : io;
+  Tensor dU = at::empty_like(U), dM = call.empty({batch, heads, T, 2}, at::kFloat);
+  Tensor dK = call.empty({batch, heads, T, 2, 2}, at::kFloat), dB = at::empty_like(B), dC = at::empty_like(C);
+  OptT dinit, dBp, dUp, ws;
+  if (z0) dinit = call.empty({batch, heads, P, 2 * N}, at::kFloat);
+  if (Bp) dBp = at::empty_like(*Bp);
+  if (Up) dUp = at::empty_like(*Up);
+  const size_t n = sl_workspace_bytes(SL_WS_SCAN_BWD, batch, heads, groups, T, P, N, chunk, io, path);
+  if (n) ws = call.bytes(n);
+  check(sl_v2x2ssd_bwd(ptr(U), fptr(M), fptr(K), ptr(B), ptr(C), fptr(z0), ptr(Bp), ptr(Up), ptr(states), fptr(final_state),
+                       ptr(dY), fptr(dfinal), mptr(dU), mfptr(dM), mfptr(dK), mptr(dB), mptr(dC), mfptr(dinit), mptr(dBp),
+                       mptr(dUp), batch, heads, groups, T, P, N, chunk, io, dy, path, mptr(ws), n, call.stream()),
+        "sl_v2x2ssd_bwd");
+  return {dU, dM, dK, dB, dC, dinit, dBp, dUp};
+}
+
+std::tuple<Tensor, Tensor> scan_decode(const Tensor& U, const Tensor& M, const Tensor& K, const Tensor& B, const Tensor& C,
+                                       const Tensor& state, const OptT& Bp, const OptT& Up, int y_code, const OptT& state_out) {
+  Call call(U, M, K, B, C, state, Bp, Up);
+  const int batch = U.size(0), heads = U.size(1), P = U.size(2), groups = B.size(1), N = B.size(2) / 2;
+  Tensor Y = call.empty({batch, heads, P}, type_of(y_code));
+  Tensor out = state_out ? *state_out : at::empty_like(state);
+  check(sl_v2x2ssd_decode(ptr(U), fptr(M), fptr(K), ptr(B), ptr(C), fptr(state), ptr(Bp), ptr(Up), mptr(Y), mfptr(out), batch,
+                          heads, groups, P, N, code_of(U.scalar_type()), y_code, call.stream()),
+        "sl_v2x2ssd_decode");
+  return {Y, out};
+}
+
+// ---- scan preparation (+ causal conv) -------------------------------------------------------------------------------
+// (batch, T, C) rows in a layout with dense channels and batch stride T * row stride, copied only if needed
+Tensor as_rows(const Tensor& x) {
+  if (x.stride(2) == 1 && (x.size(0) == 1 || x.stride(0) == x.size(1) * x.stride(1)) &&
+      (x.size(1) > 1 || x.stride(1) >= x.size(2)))
+    return x;
+  return x.contiguous();
+}
+int64_t row_stride(const Tensor& x) { return x.size(1) > 1 ? x.stride(1) : std::max<int64_t>(x.stride(1), x.size(2)); }
+
+struct ULayout { int64_t b = 0, h = 0, t = 0; };
+ULayout u_layout(bool bhtp, int64_t heads, int64_t T, int64_t P) {
+  return bhtp ? ULayout{heads * T * P, T * P, P} : ULayout{T * heads * P, P, heads * P};
+}
+struct Biases { const float* p[5] = {nullptr, nullptr, nullptr, nullptr, nullptr}; };
+Biases biases_of(const std::vector<Tensor>& v) {
+  Biases b;
+  for (size_t i = 0; i < v.size() && i < 5; ++i) b.p[i] = fptr(v[i]);
+  return b;
+}
+
+std::tuple<OptT, OptT, OptT, OptT, OptT, OptT> scanprep_fwd(const OptT& value, const OptT& w, const OptT& bias, const OptT& st,
+                                                            const OptT& params, const OptT& bc,
+                                                            const std::vector<Tensor>& biases, const c10::optional<Config>& cfg,
+                                                            int heads, int P, bool bhtp, bool want_state) {
+  const Tensor& ref = value ? *value : params ? *params : *bc;
+  Call call(value, w, bias, st, params, bc);
+  for (const auto& t : biases) call.need(t);
+  const int64_t batch = ref.size(0), T = ref.size(1);
+  OptT U, M, K, Bo, Co, nstate, rows;
+  ULayout lay;
+  int64_t vstride = 0;
+  int d_conv = 1, groups = 1, N = 1;
+  if (value) {
+    rows = as_rows(*value);
+    vstride = row_stride(*rows);
+    lay = u_layout(bhtp, heads, T, P);
+    U = bhtp ? call.empty({batch, heads, T, P}, value->scalar_type()) : call.empty({batch, T, (int64_t)heads * P}, value->scalar_type());
+    if (w) {
+      d_conv = w->size(1);
+      if (want_state) nstate = call.empty({batch, (int64_t)heads * P, d_conv - 1}, value->scalar_type());
+    }
+  }
+  if (bc) {
+    groups = bc->size(2); N = bc->size(4);
+    Bo = call.empty({batch, groups, T, 2 * N}, bc->scalar_type());
+    Co = call.empty({batch, groups, T, 2 * N}, bc->scalar_type());
+  }
+  if (params) {
+    M = call.empty({batch, heads, T, 2}, at::kFloat);
+    K = call.empty({batch, heads, T, 2, 2}, at::kFloat);
+  }
+  const Biases bs = biases_of(biases);
+  sl_scanprep_config c{};
+  if (cfg) c = config_of(*cfg);
+  check(sl_scanprep_conv_fwd(ptr(rows), vstride, ptr(w), ptr(bias), ptr(st), mptr(nstate), d_conv, ptr(params), ptr(bc), bs.p[0],
+                             bs.p[1], bs.p[2], bs.p[3], bs.p[4], cfg ? &c : nullptr, mptr(U), lay.b, lay.h, lay.t, mfptr(M),
+                             mfptr(K), mptr(Bo), mptr(Co), batch, heads, groups, T, P, N, code_of(ref.scalar_type()),
+                             call.stream()),
+        "sl_scanprep_conv_fwd");
+  return {U, M, K, Bo, Co, nstate};
+}
+
+// d_value | d_conv_weight | d_conv_bias | d_conv_state | d_params | d_bc | d_dt_bias | d_alpha_bias | d_theta_mod_bias |
+// d_theta_bias.  The float32 accumulators are slices of one zeroed buffer.
+std::vector<OptT> scanprep_bwd(const OptT& value, const OptT& w, const OptT& bias, const OptT& st, const OptT& params,
+                               const OptT& bc, const std::vector<Tensor>& biases, const c10::optional<Config>& cfg,
+                               const OptT& dU, const OptT& dM, const OptT& dK, const OptT& dBo, const OptT& dCo, int heads,
+                               int P, bool bhtp, bool want_dstate) {
+  const Tensor& ref = value ? *value : params ? *params : *bc;
+  Call call(value, w, bias, st, params, bc, dU, dM, dK, dBo, dCo);
+  const int64_t batch = ref.size(0), T = ref.size(1), C = (int64_t)heads * P;
+  std::vector<OptT> out(10);
+  ULayout lay;
+  int64_t vstride = 0;
+  int d_conv = w ? w->size(1) : 1, groups = 1, N = 1;
+  OptT rows, gU, gM, gK, gB, gC;
+  const int64_t nw = dU && w ? C * d_conv : 0, nb = dU && w ? C : 0, nh = dM ? 4 * heads : 0;
+  Tensor acc;
+  if (nw + nb + nh) acc = call.zeros({nw + nb + nh}, at::kFloat);
+  if (dU) {
+    rows = as_rows(*value);
+    vstride = row_stride(*rows);
+    gU = dU->contiguous();
+    lay = u_layout(bhtp, heads, T, P);
+    out[0] = call.empty({batch, T, C}, value->scalar_type());
+    if (w) {
+      out[1] = acc.narrow(0, 0, nw).view({C, d_conv});
+      out[2] = acc.narrow(0, nw, nb);
+      if (want_dstate && d_conv > 1) out[3] = call.zeros({batch, C, d_conv - 1}, value->scalar_type());
+    }
+  }
+  if (dBo) {
+    groups = bc->size(2); N = bc->size(4);
+    gB = dBo->contiguous(); gC = dCo->contiguous();
+    out[5] = call.empty(bc->sizes(), bc->scalar_type());
+  }
+  if (dM) {
+    gM = dM->contiguous(); gK = dK->contiguous();
+    out[4] = call.empty(params->sizes(), params->scalar_type());
+    for (int i = 0; i < 4; ++i) out[6 + i] = acc.narrow(0, nw + nb + i * heads, heads);
+  }
+  const Biases bs = biases_of(biases);
+  sl_scanprep_config c{};
+  if (cfg) c = config_of(*cfg);
+  check(sl_scanprep_conv_bwd(ptr(rows), vstride, ptr(w), ptr(bias), ptr(st), d_conv, ptr(params), ptr(bc), bs.p[0], bs.p[1],
+                             bs.p[2], bs.p[3], bs.p[4], cfg ? &c : nullptr, ptr(gU), lay.b, lay.h, lay.t, fptr(gM), fptr(gK),
+                             ptr(gB), ptr(gC), mptr(out[0]), mfptr(out[1]), mfptr(out[2]), mptr(out[3]), mptr(out[4]),
+                             mptr(out[5]), mfptr(out[6]), mfptr(out[7]), mfptr(out[8]), mfptr(out[9]), batch, heads, groups, T,
+                             P, N, code_of(ref.scalar_type()), call.stream()),
+        "sl_scanprep_conv_bwd");
+  return out;
+}
+
+// ---- mixer tail, RMSNorm, FFN activation --------------------------------------------------------------------------------
+Tensor tail_fwd(const Tensor& Y, const Tensor& gate_in, const OptT& skip, const OptT& d_skip, const Tensor& w, float eps) {
+  Call call(Y, gate_in, skip, d_skip, w);
+  const Tensor gate = as_rows(gate_in);
+  const int64_t batch = Y.size(0), heads = Y.size(1), T = Y.size(2), P = Y.size(3);
+  Tensor normed = call.empty({batch, T, heads * P}, Y.scalar_type());
+  check(sl_mixer_tail_fwd(ptr(Y), ptr(gate), row_stride(gate), ptr(skip), fptr(d_skip), ptr(w), eps, mptr(normed), batch, heads,
+                          T, P, code_of(Y.scalar_type()), call.stream()),
+        "sl_mixer_tail_fwd");
+  return normed;
+}
+
+std::tuple<Tensor, Tensor, OptT, OptT, Tensor> tail_bwd(const Tensor& Y, const Tensor& gate_in, const OptT& skip,
+                                                        const OptT& d_skip, const Tensor& w, float eps, const Tensor& dn_in) {
+  Call call(Y, gate_in, skip, d_skip, w, dn_in);
+  const Tensor gate = as_rows(gate_in), dn = dn_in.contiguous();
+  const int64_t batch = Y.size(0), heads = Y.size(1), T = Y.size(2), P = Y.size(3), nh = skip ? heads : 0;
+  Tensor dY = at::empty_like(Y), dgate = call.empty({batch, T, heads * P}, Y.scalar_type());
+  Tensor acc = call.zeros({heads * P + nh}, at::kFloat), dw = acc.narrow(0, 0, heads * P);
+  OptT dskip_in, dd;
+  if (skip) { dskip_in = at::empty_like(Y); dd = acc.narrow(0, heads * P, nh); }
+  check(sl_mixer_tail_bwd(ptr(Y), ptr(gate), row_stride(gate), ptr(skip), fptr(d_skip), ptr(w), eps, ptr(dn), mptr(dY), mptr(dgate),
+                          mptr(dskip_in), mfptr(dd), mfptr(dw), batch, heads, T, P, code_of(Y.scalar_type()), call.stream()),
+        "sl_mixer_tail_bwd");
+  return {dY, dgate, dskip_in, dd, dw};
+}
+
+Tensor rmsnorm_fwd(const Tensor& x, const Tensor& w, float eps) {
+  Call call(x, w);
+  const int64_t C = x.size(-1);
+  Tensor out = at::empty_like(x);
+  check(sl_rmsnorm_fwd(ptr(x), ptr(w), eps, mptr(out), x.numel() / C, C, code_of(x.scalar_type()), call.stream()), "sl_rmsnorm_fwd");
+  return out;
+}
+std::tuple<Tensor, Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, float eps, const Tensor& dy) {
+  Call call(x, w, dy);
+  const int64_t C = x.size(-1);
+  Tensor dx = at::empty_like(x), dw = call.zeros({C}, at::kFloat);
+  check(sl_rmsnorm_bwd(ptr(x), ptr(w), eps, ptr(dy), mptr(dx), mfptr(dw), x.numel() / C, C, code_of(x.scalar_type()), call.stream()),
+        "sl_rmsnorm_bwd");
+  return {dx, dw};
+}
+Tensor ffn_act_fwd(const Tensor& proj, int kind) {
+  Call call(proj);
+  const int64_t W = proj.size(-1), H = kind == 1 ? W / 2 : W;
+  auto shape = proj.sizes().vec();
+  shape.back() = H;
+  Tensor hidden = call.empty(shape, proj.scalar_type());
+  check(sl_ffn_activation_fwd(ptr(proj), mptr(hidden), proj.numel() / W, H, kind, code_of(proj.scalar_type()), call.stream()),
+        "sl_ffn_activation_fwd");
+  return hidden;
+}
+Tensor ffn_act_bwd(const Tensor& proj, const Tensor& dhid, int kind) {
+  Call call(proj, dhid);
+  const int64_t W = proj.size(-1), H = kind == 1 ? W / 2 : W;
+  Tensor dproj = at::empty_like(proj);
+  check(sl_ffn_activation_bwd(ptr(proj), ptr(dhid), mptr(dproj), proj.numel() / W, H, kind, code_of(proj.scalar_type()), call.stream()),
+        "sl_ffn_activation_bwd");
+  return dproj;
+}
+
+// ---- decode: one token of a mixer, and of an FFN branch ---------------------------------------------------------------
+// y = W x' (+ residual), x' = x or its RMSNorm: the small-batch kernel where it applies, else the library GEMM behind the
+// row kernel of the norm.
+struct Norm { OptT weight; float eps = 0.f; };
+
+Tensor linear_rows(const Call& call, const Tensor& x, const Norm& norm, const Tensor& W, const OptT& bias, int act,
+                   const OptT& residual, const OptT& out_in) {
+  const int64_t M = x.size(0), K = x.size(1), O = act == sl::LINEAR_SWIGLU ? W.size(0) / 2 : W.size(0);
+  const int io = code_of(x.scalar_type());
+  if (M <= 64 && K % 8 == 0 && K <= 4096 && io != SL_F32 && W.is_contiguous() && x.stride(1) == 1 && x.stride(0) % 8 == 0) {
+    Tensor out = out_in ? *out_in : call.empty({M, O}, x.scalar_type());
+    const sl::SkinnyArgs a{ptr(x), x.stride(0), ptr(norm.weight), norm.eps, nullptr, 0, ptr(W), ptr(bias), ptr(residual),
+                           mptr(out), (int)M, (int)K, (int)O, act, io};
+    check(sl::skinny_linear(a, static_cast<cudaStream_t>(call.stream())), "skinny_linear");
+    return out;
+  }
+  const Tensor in = norm.weight ? rmsnorm_fwd(x.contiguous(), *norm.weight, norm.eps) : x;
+  Tensor y;
+  if (bias) y = at::linear(in, W, *bias);
+  else if (out_in && act == sl::LINEAR_NONE && !residual) { y = *out_in; at::mm_out(y, in, W.t()); return y; }
+  else y = at::mm(in, W.t());
+  if (act != sl::LINEAR_NONE) y = ffn_act_fwd(y, act == sl::LINEAR_SWIGLU ? 1 : 0);
+  if (residual) y = *residual + y;
+  if (out_in) { out_in->copy_(y); return *out_in; }
+  return y;
+}
+
+// One token between the residual stream and itself: x (batch, d_model) -> (residual +) mixer(norm(x)).  conv, state and
+// u_prev are updated in place; the new b_prev goes to b_prev itself when every head has its own group, else to a tensor of
+// its own (the heads of a group read the old one at different times).
+std::tuple<Tensor, Tensor, Tensor> mixer_token(const Tensor& x, const OptT& pre_norm, float pre_eps, const Tensor& in_w,
+                                               const Tensor& dw_w, const Tensor& dw_b, const std::vector<Tensor>& biases,
+                                               const Config& cfg, const Tensor& d_skip, const Tensor& norm_w, float norm_eps,
+                                               const Tensor& out_w, const OptT& out_b, const Tensor& conv, const Tensor& state,
+                                               const Tensor& b_prev, const Tensor& u_prev, const OptT& workspace, int heads,
+                                               int groups, int P, int N, const OptT& residual, const OptT& out) {
+  Call call(x, pre_norm, in_w, dw_w, dw_b, d_skip, norm_w, out_w, out_b, conv, state, b_prev, u_prev, workspace, residual, out);
+  for (const auto& t : biases) call.need(t);
+  const int64_t batch = x.size(0), C = (int64_t)heads * P, O = in_w.size(0);
+  const int io = code_of(x.scalar_type());
+  const Tensor proj = linear_rows(call, x, Norm{pre_norm, pre_eps}, in_w, {}, sl::LINEAR_NONE, {}, {});
+  const size_t ws_bytes = sl_mixer_decode_step_workspace_bytes(batch, heads, P);
+  Tensor ws = workspace && (size_t)workspace->numel() >= ws_bytes ? *workspace : call.bytes(ws_bytes);
+  Tensor b_next = groups == heads ? b_prev : at::empty_like(b_prev);
+  const Biases bs = biases_of(biases);
+  const sl_scanprep_config c = config_of(cfg);
+  const auto* base = static_cast<const uint8_t*>(proj.data_ptr());
+  const int64_t e = proj.element_size();
+  const sl::MixerStepArgs a{base, base + C * e, base + 2 * C * e, base + (2 * C + 3 * heads) * e, O, O, O, O, ptr(dw_w), ptr(dw_b),
+                            mptr(conv), (int)dw_w.size(1), bs.p[0], bs.p[1], bs.p[2], bs.p[3], bs.p[4], &c, fptr(d_skip),
+                            mfptr(state), ptr(b_prev), mptr(b_next), mptr(u_prev), mptr(ws), (size_t)ws.numel(), (int)batch, heads,
+                            groups, P, N, io};
+  const auto st = static_cast<cudaStream_t>(call.stream());
+  check(sl::mixer_step_launch(a, st), "mixer_step");
+  const int64_t K = C, OO = out_w.size(0);
+  if (batch <= 64 && K % 8 == 0 && K <= 4096 && io != SL_F32 && out_w.is_contiguous()) {   // the row norm inside the projection
+    Tensor y = out ? *out : call.empty({batch, OO}, x.scalar_type());
+    const sl::SkinnyArgs s{mptr(ws), C, ptr(norm_w), norm_eps, sl::step_partials(mptr(ws), batch, heads, P), 8 * heads, ptr(out_w),
+                           ptr(out_b), ptr(residual), mptr(y), (int)batch, (int)K, (int)OO, sl::LINEAR_NONE, io};
+    check(sl::skinny_linear(s, st), "skinny_linear");
+    return {y, b_next, ws};
+  }
+  Tensor normed = call.empty({batch, C}, x.scalar_type());
+  check(sl::mixer_step_norm(mptr(ws), ptr(norm_w), norm_eps, mptr(normed), batch, heads, P, io, st), "mixer_step");
+  return {linear_rows(call, normed, Norm{}, out_w, out_b, sl::LINEAR_NONE, residual, out), b_next, ws};
+}
+
+// x (batch, d_model) -> x + out_proj(act(in_proj(norm(x)))); kind 0: GELU, 1: SwiGLU
+Tensor ffn_token(const Tensor& x, const Tensor& norm_w, float eps, const Tensor& w1, const OptT& b1, const Tensor& w2,
+                 const OptT& b2, int kind) {
+  Call call(x, norm_w, w1, b1, w2, b2);
+  const Tensor hidden = linear_rows(call, x, Norm{norm_w, eps}, w1, b1, kind == 1 ? sl::LINEAR_SWIGLU : sl::LINEAR_GELU, {}, {});
+  return linear_rows(call, hidden, Norm{}, w2, b2, sl::LINEAR_NONE, x, {});
+}
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("scan_fwd", &scan_fwd);
+  m.def("scan_bwd", &scan_bwd);
+  m.def("scan_decode", &scan_decode);
+  m.def("scanprep_fwd", &scanprep_fwd);
+  m.def("scanprep_bwd", &scanprep_bwd);
+  m.def("tail_fwd", &tail_fwd);
+  m.def("tail_bwd", &tail_bwd);
+  m.def("rmsnorm_fwd", &rmsnorm_fwd);
+  m.def("rmsnorm_bwd", &rmsnorm_bwd);
+  m.def("ffn_act_fwd", &ffn_act_fwd);
+  m.def("ffn_act_bwd", &ffn_act_bwd);
+  m.def("mixer_token", &mixer_token);
+  m.def("ffn_token", &ffn_token);
+}

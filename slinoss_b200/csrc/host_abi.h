@@ -1,0 +1,57 @@
+// Entry points of the library that only the package's own host module calls (not part of the C ABI): the decode step
+// on strided operands and the small-batch linear layers around it.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "../../include/slinoss_b200.h"
+
+namespace sl {
+
+struct MixerStepArgs {
+  const void *gate, *value, *params, *bc;   // rows of the in_proj output, with their row strides (elements)
+  int64_t gate_stride, value_stride, params_stride, bc_stride;
+  const void *conv_weight, *conv_bias;
+  void* conv_state;
+  int d_conv;
+  const float *dt_bias, *alpha_bias, *theta_mod_bias, *theta_bias, *theta_sign;
+  const sl_scanprep_config* cfg;
+  const float* d_skip;
+  float* state;
+  const void* b_prev_in;
+  void* b_prev_out;   // may be b_prev_in when every head has its own group
+  void* u_prev;
+  void* workspace;    // receives the gated values (batch, heads * P) and their partial sums of squares
+  size_t workspace_bytes;
+  int batch, heads, groups, P, N, io_dtype;
+};
+
+size_t mixer_step_workspace(int batch, int heads, int P);
+// the partial sums of squares (batch, heads, 8) inside the workspace
+inline float* step_partials(void* workspace, int batch, int heads, int P) {
+  return reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + ((size_t)batch * heads * P * 4 + 255) / 256 * 256);
+}
+SL_API int mixer_step_launch(const MixerStepArgs& a, cudaStream_t st);
+SL_API int mixer_step_norm(const void* workspace, const void* norm_weight, float eps, void* normed, int batch, int heads,
+                           int P, int io_dtype, cudaStream_t st);
+
+// y (M, O) = act(norm(x) W^T + bias) (+ residual), 16-bit, M <= 64 rows.  norm: none, RMSNorm with weight, or RMSNorm
+// whose sums of squares are given as partials per row.
+enum { LINEAR_NONE = 0, LINEAR_GELU = 1, LINEAR_SWIGLU = 2 };
+struct SkinnyArgs {
+  const void* x;          // (M, K), row stride x_stride
+  int64_t x_stride;
+  const void* norm_weight;   // (K) or null
+  float norm_eps;
+  const float* partials;  // (M, n_partials) or null
+  int n_partials;
+  const void *weight, *bias;   // (O, K) dense [SwiGLU: (2 O, K), value rows then gate rows], bias or null
+  const void* residual;   // (M, O) dense or null
+  void* out;              // (M, O) dense
+  int M, K, O, act, io_dtype;
+};
+bool skinny_supported(int M, int K, int O, int io_dtype);
+SL_API int skinny_linear(const SkinnyArgs& a, cudaStream_t st);
+
+}  // namespace sl

@@ -237,19 +237,6 @@ namespace {
 inline int blocks_of(const ScanDims& d) { return d.N <= 64 ? 1 : 2; }
 inline int chunks_of(const ScanDims& d) { return (d.T + L - 1) / L; }
 
-// Kernel attributes stick to a device: set once per (kernel, device) instead of on every launch.
-template <typename F>
-int ensure_smem(F k, size_t bytes, std::atomic<unsigned long long>& done) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return SL_ERR_LAUNCH_FAILED;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (done.load(std::memory_order_relaxed) & bit) return SL_OK;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
-    return SL_ERR_LAUNCH_FAILED;
-  done.fetch_or(bit, std::memory_order_relaxed);
-  return SL_OK;
-}
-
 // Encoding a tensor map is a driver call and needs a current context, which a thread that has only been told its
 // device (an autograd worker, say) may not have yet: the runtime makes one current on the first cudaSetDevice.
 void ensure_context() {

@@ -13,7 +13,6 @@ from __future__ import annotations
 import torch
 
 from .layers.state import SLinOSSMixerState
-from .ops.mixer.projection import split_mixer_projection
 
 
 class MixerDecodeEngine:
@@ -37,8 +36,7 @@ class MixerDecodeEngine:
         kw = dict(device=self.device, dtype=self.dtype)
         self.x = torch.zeros((self.batch, mixer.d_model), **kw)
         self.y = torch.zeros((self.batch, mixer.d_model), **kw)
-        self._normed = torch.empty((self.batch, mixer.d_inner), **kw)
-        self._b_next = torch.empty_like(self.state.scan.b_prev)
+        self._b_prev = self.state.scan.b_prev    # (the step hands the new one on in a tensor of its own when heads share groups)
         self._workspace = _C.mixer_decode_workspace(self.batch, mixer.n_heads, mixer.d_head, self.device)
         self._graph = None
         if use_graph:
@@ -46,20 +44,11 @@ class MixerDecodeEngine:
 
     # one token over the static buffers (everything in place: the graph sees fixed addresses)
     def _token(self):
-        from . import _C
-        m, st = self.mixer, self.state
-        gate, value, params, bc = split_mixer_projection(
-            self.x, m.in_proj.weight, d_inner=m.d_inner, param_proj_dim=m.param_proj_dim)
-        sp = m.scanprep
-        biases = tuple(getattr(sp, k).detach().float() for k in
-                       ("dt_bias", "alpha_bias", "theta_mod_bias", "theta_bias", "theta_sign"))
-        _C.mixer_decode_step(
-            gate, value, params, bc.view(self.batch, m.bc_groups, 4, m.d_state), m.dw_weight.detach(),
-            m.dw_bias.detach(), st.conv, biases, _C.make_config(sp), m.d_skip.detach().float(),
-            m.out_norm.weight.detach(), m.out_norm.eps, st.scan.state, st.scan.b_prev, self._b_next,
-            st.scan.u_prev, self._workspace, heads=m.n_heads, P=m.d_head, normed=self._normed)
-        st.scan.b_prev.copy_(self._b_next)
-        torch.mm(self._normed, m.out_proj.weight.detach().t(), out=self.y)
+        st = self.state
+        self.mixer.decode_native(self.x, st, workspace=self._workspace, out=self.y)
+        if st.scan.b_prev is not self._b_prev:
+            self._b_prev.copy_(st.scan.b_prev)
+            st.scan.b_prev = self._b_prev
 
     def _capture(self):
         side = torch.cuda.Stream(self.device)

@@ -14,6 +14,7 @@ from typing import Protocol
 
 import torch
 
+from .. import _C
 from ..ops.scanprep import causal_conv_silu_b200, scanprep_b200
 from ..ops.v2x2ssd import v2x2ssd_cute, v2x2ssd_decode
 from .state import ScanState
@@ -134,12 +135,11 @@ class B200MixerDecodeBackend:
     def supports(self, owner, *, batch_size, device, dtype) -> bool:
         return device.type == "cuda" and dtype in (torch.float32, torch.bfloat16, torch.float16)
 
-    @torch.compiler.disable
+    @_C.opaque
     def fused_step(self, owner, gate, value_raw, params, bc, state, *, normed=None, workspace=None):
         """``gate, value_raw (batch, d_inner)`` (row-strided views are fine), ``params (batch, 3H)``,
         ``bc (batch, G*4*N)``; ``state`` is the mixer's decode state (conv window, float32 scan
         state, previous b and u), all of it updated in place.  Returns ``normed (batch, d_inner)``."""
-        from .. import _C
         batch = int(gate.shape[0])
         sp, scan = owner.scanprep, state.scan
         dev, dt = gate.device, gate.dtype

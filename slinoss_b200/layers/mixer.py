@@ -14,6 +14,7 @@ import math
 import torch
 from torch import nn
 
+from .. import _C
 from ..ops.mixer import mixer_tail, split_mixer_projection
 from ..ops.scanprep import conv_scanprep_b200
 from .backend import (B200CConv1dBackend, B200MixerDecodeBackend, B200ScanBackend,
@@ -22,6 +23,10 @@ from .backend import (B200CConv1dBackend, B200MixerDecodeBackend, B200ScanBacken
 from .norm import RMSNorm
 from .scanprep import SLinOSSScanPrep, _require
 from .state import ScanState, SLinOSSMixerState
+
+
+def _norm_eps(norm: nn.RMSNorm) -> float:
+    return norm.eps if norm.eps is not None else torch.finfo(norm.weight.dtype).eps
 
 
 class SLinOSSMixer(nn.Module):
@@ -205,8 +210,45 @@ class SLinOSSMixer(nn.Module):
                 and sc.b_prev.dtype == token.dtype and sc.u_prev.dtype == token.dtype
                 and sc.b_prev.is_contiguous() and sc.u_prev.is_contiguous())
 
+    def _native_decode_ready(self, token: torch.Tensor) -> bool:
+        """The native decode step reads the parameters itself: plain bias-free projections of the token's type, no
+        hooks to honour, the package's own decode backend, no autocast."""
+        w_in, out = self.in_proj._parameters["weight"], self.out_proj
+        w_out = out._parameters["weight"]
+        return (type(self.decode_backend) is B200MixerDecodeBackend and type(out) is nn.Linear
+                and not out._forward_hooks and not out._forward_pre_hooks and token.stride(1) == 1
+                and w_in.dtype == token.dtype and w_out.dtype == token.dtype and w_in.device == token.device
+                and w_in.is_contiguous() and not torch.is_autocast_enabled())
+
+    @_C.opaque
+    def decode_native(self, token: torch.Tensor, state: SLinOSSMixerState, *, pre_norm=None, residual=None,
+                      workspace=None, out=None) -> torch.Tensor:
+        """One token through the native host module: ``(residual +) mixer(norm(token))`` in three launches (two GEMMs
+        around the fused step) for small batches, with the state updated in place.  ``pre_norm``: an RMSNorm module
+        applied inside the first of them."""
+        sp, mine, scan, dt = self.scanprep, self._parameters, state.scan, token.dtype
+        p = sp._parameters
+        if workspace is None:
+            workspace = getattr(state, "_step_workspace", None)
+        y, b_next, used = _C.host().mixer_token(
+            token, None if pre_norm is None else pre_norm.weight,
+            0.0 if pre_norm is None else _norm_eps(pre_norm), self.in_proj._parameters["weight"],
+            _C.as_type(mine["dw_weight"], dt), _C.as_type(mine["dw_bias"], dt),
+            [_C.as_f32(t) for t in (p["dt_bias"], p["alpha_bias"], p["theta_mod_bias"], p["theta_bias"],
+                                    sp._buffers["theta_sign"])],
+            [getattr(sp, n) for n in _C.CONFIG_FIELDS], _C.as_f32(mine["d_skip"]),
+            _C.as_type(self.out_norm._parameters["weight"], dt), _norm_eps(self.out_norm),
+            self.out_proj._parameters["weight"], self.out_proj._parameters["bias"], state.conv, scan.state, scan.b_prev,
+            scan.u_prev, workspace, self.n_heads, self.bc_groups, self.d_head, self.d_state, residual, out)
+        scan.b_prev = b_next
+        if used is not workspace:
+            state._step_workspace = used
+        return y
+
     def _decode_token(self, token: torch.Tensor, state: SLinOSSMixerState) -> torch.Tensor:
         batch = int(token.shape[0])
+        if token.is_cuda and self._fused_decode_ready(state, token) and self._native_decode_ready(token):
+            return self.decode_native(token, state)
         gate, value_proj, params, bc = split_mixer_projection(
             token, self.in_proj.weight, d_inner=self.d_inner, param_proj_dim=self.param_proj_dim)
         if self._fused_decode_ready(state, token):

@@ -27,9 +27,11 @@ class _RMSNormFn(torch.autograd.Function):
                 d_w.to(weight.dtype) if ctx.needs_input_grad[1] else None, None)
 
 
-@torch.compiler.disable
+@_C.opaque
 def rmsnorm_rows(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
     """RMSNorm over the last axis on the CUDA row kernels (same type for rows and weight)."""
+    if not _C.grad_needed(x, weight):
+        return _C.rmsnorm_fwd(x.contiguous(), weight, float(eps))
     return _RMSNormFn.apply(x, weight, float(eps))
 
 

@@ -43,7 +43,8 @@ def split_mixer_projection(x: torch.Tensor, weight: torch.Tensor, *, d_inner: in
     p_end = gv_end + int(param_proj_dim)
     flat = x.reshape(-1, x.shape[-1])
     lead = x.shape[:-1]
-    if weight.is_contiguous() and flat.dtype == weight.dtype and not torch.is_autocast_enabled():
+    if weight.is_contiguous() and flat.dtype == weight.dtype and not torch.is_autocast_enabled() and \
+            torch.is_grad_enabled() and (flat.requires_grad or weight.requires_grad):
         gate_value, params, bc = _SplitProjectionFn.apply(flat, weight, gv_end, p_end)
     else:
         gate_value = torch.mm(flat, weight[:gv_end].t())

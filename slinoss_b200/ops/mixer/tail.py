@@ -27,15 +27,16 @@ def _dims(scan_output, gate):
     return batch, heads, T, P
 
 
+def _operands(scan_output, gate, skip_input, d_skip, norm_weight):
+    io = scan_output.dtype
+    return (_C.as_type(scan_output, io), gate if gate.dtype is io else gate.detach().to(io), _C.as_type(skip_input, io),
+            None if d_skip is None else _C.as_f32(d_skip), _C.as_type(norm_weight, io))
+
+
 class _GatedNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, scan_output, gate, skip_input, d_skip, norm_weight, eps):
-        io = scan_output.dtype
-        Y = scan_output.detach().contiguous()
-        g = gate.detach().to(io)
-        S = None if skip_input is None else skip_input.detach().to(io).contiguous()
-        ds = None if d_skip is None else d_skip.detach().to(torch.float32).contiguous()
-        w = norm_weight.detach().to(io).contiguous()
+        Y, g, S, ds, w = _operands(scan_output, gate, skip_input, d_skip, norm_weight)
         normed = _C.mixer_tail_fwd(Y, g, S, ds, w, eps)
         ctx.save_for_backward(Y, g, S, ds, w)
         ctx.eps = eps
@@ -53,7 +54,7 @@ class _GatedNormFn(torch.autograd.Function):
                 None if d_d_skip is None else d_d_skip.to(dsd), d_w.to(wd), None)
 
 
-@torch.compiler.disable
+@_C.opaque
 def mixer_gated_norm(scan_output, gate, norm_weight, eps, *, skip_input=None, d_skip=None):
     """Row-wise part of the tail -> ``(batch, T, heads*P)`` in scan_output's dtype."""
     _, heads, _, _ = _dims(scan_output, gate)
@@ -67,10 +68,12 @@ def mixer_gated_norm(scan_output, gate, norm_weight, eps, *, skip_input=None, d_
             raise ValueError(f"d_skip must be 1-D with length {heads}; got {tuple(d_skip.shape)}.")
     if eps is None:
         eps = float(torch.finfo(norm_weight.dtype).eps)
+    if not _C.grad_needed(scan_output, gate, skip_input, d_skip, norm_weight):
+        return _C.mixer_tail_fwd(*_operands(scan_output, gate, skip_input, d_skip, norm_weight), float(eps))
     return _GatedNormFn.apply(scan_output, gate, skip_input, d_skip, norm_weight, float(eps))
 
 
-@torch.compiler.disable
+@_C.opaque
 def mixer_tail(scan_output, gate, out_norm: nn.RMSNorm, out_proj: nn.Module, *, skip_input=None,
                d_skip=None):
     """Full tail including ``out_proj`` (same call as the reference's ``mixer_tail``)."""

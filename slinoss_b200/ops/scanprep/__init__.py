@@ -17,9 +17,14 @@ from ... import _C
 
 
 def _biases(owner):
-    f = lambda t: t.detach().to(torch.float32).contiguous()
-    return (f(owner.dt_bias), f(owner.alpha_bias), f(owner.theta_mod_bias), f(owner.theta_bias),
-            f(owner.theta_sign))
+    p = owner._parameters
+    return tuple(_C.as_f32(t) for t in (p["dt_bias"], p["alpha_bias"], p["theta_mod_bias"], p["theta_bias"],
+                                        owner._buffers["theta_sign"]))
+
+
+def _operands(value, params, bc, conv_weight, conv_bias, conv_state):
+    io = value.dtype
+    return tuple(_C.as_type(t, io) for t in (params, bc, conv_weight, conv_bias, conv_state))
 
 
 class _ConvScanPrepFn(torch.autograd.Function):
@@ -29,12 +34,7 @@ class _ConvScanPrepFn(torch.autograd.Function):
         heads, P = owner.n_heads, owner.d_head
         cfg = _C.make_config(owner)
         biases = _biases(owner)
-        io = value.dtype
-        c = lambda x: None if x is None else x.detach().to(io)
-        params_c, bc_c = c(params).contiguous(), c(bc).contiguous()
-        w_c = None if conv_weight is None else c(conv_weight).contiguous()
-        b_c = None if conv_bias is None else c(conv_bias).contiguous()
-        st_c = None if conv_state is None else c(conv_state).contiguous()
+        params_c, bc_c, w_c, b_c, st_c = _operands(value, params, bc, conv_weight, conv_bias, conv_state)
         value_d = value.detach()
         U, M, K, Bo, Co, nstate = _C.scanprep_conv_fwd(
             value_d, w_c, b_c, st_c, params_c, bc_c, biases, cfg, heads=heads, P=P,
@@ -79,19 +79,24 @@ class _ConvScanPrepFn(torch.autograd.Function):
                 g["d_theta_mod_bias"], g["d_theta_bias"], None, None)
 
 
-@torch.compiler.disable
+@_C.opaque
 def conv_scanprep_b200(owner, value, params, bc, *, conv_weight=None, conv_bias=None,
                        conv_state=None, want_state=False):
     """``owner`` is the SLinOSSScanPrep module (bounds, biases, head geometry).
 
     ``value (batch,T,heads*P)`` may be a column slice of the in_proj output (row
     strided).  Returns ``(U, M, K, B, C, next_conv_state)``."""
+    if not _C.grad_needed(value, params, bc, conv_weight, conv_bias, conv_state, *owner._parameters.values()):
+        params, bc, w, b, st = _operands(value, params, bc, conv_weight, conv_bias, conv_state)
+        out = _C.scanprep_conv_fwd(value, w, b, st, params, bc, _biases(owner), _C.make_config(owner),
+                                   heads=owner.n_heads, P=owner.d_head, want_state=want_state and w is not None)
+        return out if out[5] is not None else (*out[:5], value.new_empty((value.shape[0], owner.n_heads * owner.d_head, 0)))
     return _ConvScanPrepFn.apply(value, params, bc, conv_weight, conv_bias, conv_state,
                                  owner.dt_bias, owner.alpha_bias, owner.theta_mod_bias,
                                  owner.theta_bias, owner, want_state)
 
 
-@torch.compiler.disable
+@_C.opaque
 def scanprep_b200(owner, value, params, bc):
     """Scan preparation without the convolution.  Returns ``(U, M, K, B, C)``."""
     return conv_scanprep_b200(owner, value, params, bc)[:5]
@@ -128,7 +133,7 @@ class _ConvFn(torch.autograd.Function):
                 None)
 
 
-@torch.compiler.disable
+@_C.opaque
 def causal_conv_silu_b200(x, weight, bias, conv_state=None, *, want_state=True):
     """``SiLU(depthwise causal conv1d(x) + bias)`` for channel-last ``x (batch,T,C)``,
     ``weight (C,d_conv)``, optional left state ``(batch,C,d_conv-1)``.

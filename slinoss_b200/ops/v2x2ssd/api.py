@@ -19,12 +19,38 @@ def _require(cond: bool, message: str) -> None:
         raise ValueError(message)
 
 
+def _accept(U, M, K, B, C, initial_states, B_prev, U_prev):
+    """The dims of a call that meets the whole contract below, else None: the accepting path is one pass over the
+    shapes, and only a call that fails it pays for finding out why."""
+    if U.ndim != 4 or B.ndim != 4:
+        return None
+    batch, heads, T, P = U.shape
+    groups, D = B.shape[1], B.shape[3]
+    want = [(M, (batch, heads, T, 2)), (K, (batch, heads, T, 2, 2)), (B, (batch, groups, T, D)), (C, (batch, groups, T, D))]
+    if initial_states is not None:
+        want.append((initial_states, (batch, heads, P, D)))
+    if B_prev is not None and U_prev is not None:
+        want += [(B_prev, (batch, groups, D)), (U_prev, (batch, heads, P))]
+    elif B_prev is not None or U_prev is not None:
+        return None
+    device = U.device
+    if D % 2 or groups == 0 or heads % groups or not (U.is_contiguous() and U.is_floating_point()):
+        return None
+    for t, shape in want:
+        if t.shape != shape or t.device != device or not (t.is_contiguous() and t.is_floating_point()):
+            return None
+    return batch, heads, T, D // 2, P
+
+
 def validate_inputs(U, M, K, B, C, initial_states, B_prev, U_prev):
     """Shape / device / layout contract of the scan.  The conditions and the messages are the
     reference's (``_validate_inputs``, slinoss/ops/v2x2ssd/reference.py:152-234), since callers
     match on them; the checks are grouped here as: the five operands as a set, the per-operand
     rank table, cross-operand extents, then the optional carried tensors.
     Returns ``(batch, heads, T, N, P)``."""
+    dims = _accept(U, M, K, B, C, initial_states, B_prev, U_prev)
+    if dims is not None:
+        return dims
     operands = {"U": U, "M": M, "K": K, "B": B, "C": C}
     values = tuple(operands.values())
     _require(all(torch.is_floating_point(t) for t in values),
@@ -85,6 +111,9 @@ def validate_inputs(U, M, K, B, C, initial_states, B_prev, U_prev):
 def resolve_dtypes(input_dtypes, compute_dtype, output_dtype, default_output_dtype):
     """Compute / output dtype policy (reference.py:61-82); the CUDA kernels compute
     in float32 only (cute/api.py:91-95)."""
+    if compute_dtype is None and output_dtype is None and default_output_dtype in _IO_DTYPES and \
+            torch.float64 not in input_dtypes:
+        return torch.float32, default_output_dtype
     if compute_dtype is None:
         promoted = input_dtypes[0]
         for dt in input_dtypes[1:]:
@@ -120,9 +149,9 @@ def _io_dtype(U: torch.Tensor) -> torch.dtype:
 def _prep(U, M, K, B, C, initial_states, B_prev, U_prev):
     """Cast to what the C ABI takes: U/B/C/B_prev/U_prev in one io dtype, the rest float32."""
     io = _io_dtype(U)
-    cast = lambda x, dt: None if x is None else x.detach().to(dtype=dt).contiguous()
-    return (cast(U, io), cast(M, torch.float32), cast(K, torch.float32), cast(B, io), cast(C, io),
-            cast(initial_states, torch.float32), cast(B_prev, io), cast(U_prev, io))
+    cast, f32 = _C.as_type, torch.float32
+    return (cast(U, io), cast(M, f32), cast(K, f32), cast(B, io), cast(C, io), cast(initial_states, f32),
+            cast(B_prev, io), cast(U_prev, io))
 
 
 def assert_nonzero_transitions(M: torch.Tensor) -> None:
@@ -161,7 +190,8 @@ class _ScanFn(torch.autograd.Function):
         ctx.in_dtypes = [None if x is None else x.dtype
                          for x in (U, M, K, B, C, initial_states, B_prev, U_prev)]
         ctx.chunk_size, ctx.path, ctx.return_state = chunk_size, path, return_state
-        Y = Y.to(dtype=odtype)
+        if Y.dtype is not odtype:
+            Y = Y.to(dtype=odtype)
         if not return_state:
             return Y
         return (Y, final.to(dtype=odtype), B[:, :, -1, :].detach().to(dtype=odtype).contiguous(),
@@ -207,7 +237,7 @@ class _ScanFn(torch.autograd.Function):
         return (*res, None, None, None, None, None)
 
 
-@torch.compiler.disable
+@_C.opaque
 def v2x2ssd_cute(U, M, K, B, C, *, chunk_size, initial_states=None, B_prev=None, U_prev=None,
                  compute_dtype=None, output_dtype=None, return_state=False, path="auto",
                  save_chunk_states=True):
@@ -228,9 +258,7 @@ def v2x2ssd_cute(U, M, K, B, C, *, chunk_size, initial_states=None, B_prev=None,
         empty = _empty_outputs(batch, heads, int(B.shape[1]), P, 2 * N, U.device, odtype,
                                initial_states, B_prev, U_prev)
         return empty if return_state else empty[0]
-    needs_grad = torch.is_grad_enabled() and any(
-        t is not None and t.requires_grad for t in (U, M, K, B, C, initial_states, B_prev, U_prev))
-    if needs_grad:
+    if _C.grad_needed(U, M, K, B, C, initial_states, B_prev, U_prev):
         return _ScanFn.apply(U, M, K, B, C, initial_states, B_prev, U_prev, int(chunk_size),
                              odtype, bool(return_state), path, bool(save_chunk_states))
     args = _prep(U, M, K, B, C, initial_states, B_prev, U_prev)
@@ -244,7 +272,7 @@ def v2x2ssd_cute(U, M, K, B, C, *, chunk_size, initial_states=None, B_prev=None,
             U[:, :, -1, :].to(dtype=odtype).contiguous())
 
 
-@torch.compiler.disable
+@_C.opaque
 def v2x2ssd(U, M, K, B, C, *, chunk_size=64, initial_states=None, B_prev=None, U_prev=None,
             compute_dtype=None, output_dtype=None, path="auto"):
     """Same call and 4-tuple result as the reference's ``v2x2ssd``."""
@@ -253,7 +281,7 @@ def v2x2ssd(U, M, K, B, C, *, chunk_size=64, initial_states=None, B_prev=None, U
                         output_dtype=output_dtype, return_state=True, path=path)
 
 
-@torch.compiler.disable
+@_C.opaque
 def v2x2ssd_decode(U, M, K, B, C, *, state, B_prev=None, U_prev=None, output_dtype=None,
                    inplace=False):
     """One decode token.  ``U (batch,heads,P)``, ``M (batch,heads,2)``, ``K (batch,heads,2,2)``,
@@ -273,7 +301,7 @@ def v2x2ssd_decode(U, M, K, B, C, *, state, B_prev=None, U_prev=None, output_dty
         raise ValueError(f"state must be {(batch, heads, P, B.shape[-1])}. Got {tuple(state.shape)}.")
     io = _io_dtype(U)
     odtype = U.dtype if output_dtype is None else output_dtype
-    cast = lambda x, dt: None if x is None else x.to(dtype=dt).contiguous()
+    cast = _C.as_type
     if inplace and (state.dtype != torch.float32 or not state.is_contiguous()):
         raise ValueError("in-place decode needs a contiguous float32 state.")
     st = cast(state, torch.float32)
