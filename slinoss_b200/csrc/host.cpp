@@ -370,6 +370,95 @@ Tensor ffn_token(const Tensor& x, const Tensor& norm_w, float eps, const Tensor&
   const Tensor hidden = linear_rows(call, x, Norm{norm_w, eps}, w1, b1, kind == 1 ? sl::LINEAR_SWIGLU : sl::LINEAR_GELU, {}, {});
   return linear_rows(call, hidden, Norm{}, w2, b2, sl::LINEAR_NONE, x, {});
 }
+// ---- language-model training step --------------------------------------------------------------------------------------
+// per-row losses and log-sum-exps of logits (rows, V)
+std::tuple<Tensor, Tensor> ce_fwd(const Tensor& logits, const Tensor& target) {
+  Call call(logits, target);
+  const int64_t rows = logits.size(0), V = logits.size(1);
+  Tensor loss = call.empty({rows}, at::kFloat), lse = call.empty({rows}, at::kFloat);
+  check(sl::cross_entropy_fwd(ptr(logits), target.const_data_ptr<int64_t>(), mfptr(loss), mfptr(lse), rows, V,
+                              code_of(logits.scalar_type()), static_cast<cudaStream_t>(call.stream())),
+        "cross_entropy_fwd");
+  return {loss, lse};
+}
+Tensor ce_bwd(const Tensor& logits, const Tensor& target, const Tensor& lse, const Tensor& g, double scale) {
+  Call call(logits, target, lse, g);
+  const int64_t rows = logits.size(0), V = logits.size(1);
+  Tensor d = at::empty_like(logits);
+  check(sl::cross_entropy_bwd(ptr(logits), target.const_data_ptr<int64_t>(), fptr(lse), fptr(g), (float)scale, mptr(d), rows, V,
+                              code_of(logits.scalar_type()), static_cast<cudaStream_t>(call.stream())),
+        "cross_entropy_bwd");
+  return d;
+}
+Tensor embed_bwd(const Tensor& ids, const Tensor& d_out, int64_t V) {
+  Call call(ids, d_out);
+  const int64_t n = ids.numel(), C = d_out.size(-1);
+  auto [sorted, order] = at::sort(ids.reshape({-1}).to(at::kInt), c10::optional<bool>(true), 0, false);
+  const Tensor rows = d_out.contiguous();
+  Tensor dE = call.empty({V, C}, d_out.scalar_type());
+  check(sl::embedding_bwd(sorted.const_data_ptr<int>(), order.const_data_ptr<int64_t>(), ptr(rows), mptr(dE), n, V, C,
+                          code_of(d_out.scalar_type()), static_cast<cudaStream_t>(call.stream())),
+        "embedding_bwd");
+  return dE;
+}
+
+// {global norm, max(1, (norm + 1e-6) / clip)} of a list of tensors of up to three types
+Tensor grad_norm_scale(const std::vector<Tensor>& grads, double clip) {
+  if (grads.empty()) throw pybind11::value_error("no gradients.");
+  Call call(grads[0]);
+  for (const auto& g : grads) call.need(g);
+  const auto st = static_cast<cudaStream_t>(call.stream());
+  int64_t total = 0;
+  for (const auto& g : grads) total += sl::mt_chunks(g.numel());
+  Tensor partial = call.empty({std::max<int64_t>(total, 1)}, at::kFloat), out = call.empty({2}, at::kFloat);
+  int64_t at_chunk = 0;
+  for (int io : {SL_F32, SL_BF16, SL_F16}) {
+    sl::MtList1 list{};
+    unsigned chunks = 0;
+    auto flush = [&] {
+      if (!chunks) return;
+      check(sl::multi_sumsq(list, chunks, mfptr(partial) + at_chunk, io, st), "grad_norm");
+      at_chunk += chunks; chunks = 0; list.n = 0;
+    };
+    for (const auto& g : grads) {
+      if (code_of(g.scalar_type()) != io || g.numel() == 0) continue;
+      list.p[list.n] = ptr(g); list.len[list.n] = g.numel(); list.first[list.n] = chunks; ++list.n;
+      chunks += sl::mt_chunks(g.numel());
+      if (list.n == sl::MT_MAX) flush();
+    }
+    flush();
+  }
+  check(sl::norm_finish(fptr(partial), (int)at_chunk, (float)clip, mfptr(out), st), "grad_norm");
+  return out;
+}
+
+// one AdamW step over lists of parameters, gradients and moments (all dense and of one type per position)
+void adamw_step(const std::vector<Tensor>& ps, const std::vector<Tensor>& gs, const std::vector<Tensor>& ms,
+                const std::vector<Tensor>& vs, const Tensor& step, double lr, double beta1, double beta2, double eps,
+                double weight_decay, const OptT& grad_scale) {
+  Call call(step, grad_scale);
+  for (const auto& p : ps) call.need(p);
+  const auto st = static_cast<cudaStream_t>(call.stream());
+  const sl::AdamWArgs a{(float)lr, (float)beta1, (float)beta2, (float)eps, (float)weight_decay, fptr(step), fptr(grad_scale)};
+  for (int io : {SL_F32, SL_BF16, SL_F16}) {
+    sl::MtList4 list{};
+    unsigned chunks = 0;
+    auto flush = [&] {
+      if (chunks) check(sl::multi_adamw(list, chunks, a, io, st), "adamw");
+      chunks = 0; list.n = 0;
+    };
+    for (size_t i = 0; i < ps.size(); ++i) {
+      if (code_of(ps[i].scalar_type()) != io || ps[i].numel() == 0) continue;
+      const int n = list.n++;
+      list.p[n] = mptr(ps[i]); list.g[n] = mptr(gs[i]); list.m[n] = mptr(ms[i]); list.v[n] = mptr(vs[i]);
+      list.len[n] = ps[i].numel(); list.first[n] = chunks;
+      chunks += sl::mt_chunks(ps[i].numel());
+      if (list.n == sl::MT_MAX) flush();
+    }
+    flush();
+  }
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -384,6 +473,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("ffn_act_fwd", &ffn_act_fwd);
   m.def("ffn_act_bwd", &ffn_act_bwd);
+  m.def("ce_fwd", &ce_fwd);
+  m.def("ce_bwd", &ce_bwd);
+  m.def("embed_bwd", &embed_bwd);
+  m.def("grad_norm_scale", &grad_norm_scale);
+  m.def("adamw_step", &adamw_step);
   m.def("mixer_token", &mixer_token);
   m.def("ffn_token", &ffn_token);
 }

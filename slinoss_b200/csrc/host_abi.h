@@ -54,4 +54,22 @@ struct SkinnyArgs {
 bool skinny_supported(int M, int K, int O, int io_dtype);
 SL_API int skinny_linear(const SkinnyArgs& a, cudaStream_t st);
 
+// ---- language-model training step ------------------------------------------------------------------------------------
+SL_API int cross_entropy_fwd(const void* logits, const int64_t* target, float* loss, float* lse, int64_t rows, int V, int io,
+                             cudaStream_t st);
+SL_API int cross_entropy_bwd(const void* logits, const int64_t* target, const float* lse, const float* g, float scale, void* d,
+                             int64_t rows, int V, int io, cudaStream_t st);
+// ids sorted (stable) and the positions they came from -> dE (V, C)
+SL_API int embedding_bwd(const int* sorted, const int64_t* order, const void* d_out, void* dE, int n, int V, int C, int io,
+                         cudaStream_t st);
+// lists of tensors by value; first[i] = chunks of the tensors before i
+constexpr int MT_MAX = 72;
+struct MtList1 { const void* p[MT_MAX]; int64_t len[MT_MAX]; unsigned first[MT_MAX]; int n; };
+struct MtList4 { void *p[MT_MAX], *g[MT_MAX], *m[MT_MAX], *v[MT_MAX]; int64_t len[MT_MAX]; unsigned first[MT_MAX]; int n; };
+struct AdamWArgs { float lr, beta1, beta2, eps, weight_decay; const float *step, *grad_scale; };
+SL_API unsigned mt_chunks(int64_t len);
+SL_API int multi_sumsq(const MtList1& list, unsigned chunks, float* partial, int io, cudaStream_t st);
+SL_API int norm_finish(const float* partial, int n, float clip, float* out, cudaStream_t st);
+SL_API int multi_adamw(const MtList4& list, unsigned chunks, const AdamWArgs& a, int io, cudaStream_t st);
+
 }  // namespace sl

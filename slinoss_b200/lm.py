@@ -4,7 +4,8 @@ Token embedding -> ``SLinOSSStack`` -> tied output head, cross-entropy on shifte
 the reference's performance harness (scripts/perf/_training_model.py:204-252, minus its positional
 table: the configuration this package is benchmarked on feeds the stack with token embeddings
 only) and of its example (examples/blocks_lm.py:18-55).  The stack itself calls the CUDA kernels
-of this package; embedding, head and loss are library calls (torch).
+of this package; the loss, the embedding's gradient, the gradient norm
+and the optimizer run on its kernels as well; the lookup and the head are library calls (torch).
 """
 
 from __future__ import annotations
@@ -13,9 +14,60 @@ import torch
 from torch import nn
 from torch.nn import functional as F
 
-from . import shard
+from . import _C, optim, shard
 from .blocks import SLinOSSBlockConfig, SLinOSSMixerConfig, SLinOSSStack, SLinOSSStackConfig
 from .layers import SLinOSSMLPConfig
+
+
+class _CrossEntropyFn(torch.autograd.Function):
+    """Summed cross-entropy times ``scale`` on the row kernels: the logits are kept in their own type and read once
+    each way (the library route goes through four float32 tensors of their size)."""
+
+    @staticmethod
+    def forward(ctx, logits, targets, scale):
+        rows, lse = _C.host().ce_fwd(logits, targets)
+        ctx.save_for_backward(logits, targets, lse)
+        ctx.scale = scale
+        return rows.sum() * scale
+
+    @staticmethod
+    def backward(ctx, d_loss):
+        logits, targets, lse = ctx.saved_tensors
+        return _C.host().ce_bwd(logits, targets, lse, d_loss.to(torch.float32), ctx.scale), None, None
+
+
+class _EmbeddingFn(torch.autograd.Function):
+    """Lookup whose gradient is one kernel over the vocabulary rows (no memset, no scatter)."""
+
+    @staticmethod
+    def forward(ctx, ids, weight):
+        ctx.save_for_backward(ids)
+        ctx.rows = weight.shape[0]
+        return F.embedding(ids, weight)
+
+    @staticmethod
+    def backward(ctx, d_out):
+        (ids,) = ctx.saved_tensors
+        return None, _C.host().embed_bwd(ids, d_out, ctx.rows)
+
+
+@_C.opaque
+def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, *, reduction: str = "mean") -> torch.Tensor:
+    """``F.cross_entropy(logits.float(), targets)`` of ``logits (rows, vocab)``."""
+    if not logits.is_cuda or logits.dtype not in _C._DTYPE_CODE or logits.numel() == 0 or not logits.is_contiguous():
+        return F.cross_entropy(logits.float(), targets, reduction=reduction)
+    scale = 1.0 / logits.shape[0] if reduction == "mean" else 1.0
+    return _CrossEntropyFn.apply(logits, targets.contiguous(), scale)
+
+
+@_C.opaque
+def embed(ids: torch.Tensor, table: nn.Embedding) -> torch.Tensor:
+    w = table.weight
+    plain = type(table) is nn.Embedding and table.padding_idx is None and table.max_norm is None and not table.sparse \
+        and not table.scale_grad_by_freq and not table._forward_hooks and not table._forward_pre_hooks
+    if not (plain and w.is_cuda and w.dtype in _C._DTYPE_CODE and ids.dtype == torch.int64 and ids.numel() > 0):
+        return table(ids)
+    return _EmbeddingFn.apply(ids, w)
 
 
 def lm_stack_config(d_model: int = 2048, n_layers: int = 24, d_state: int = 64, d_head: int = 64,
@@ -57,7 +109,7 @@ class SLinOSSLM(nn.Module):
         return F.linear(self.hidden(ids), self.token_embed.weight)
 
     def hidden(self, ids: torch.Tensor, *, sequence_group=None) -> torch.Tensor:
-        x = self.token_embed(ids)
+        x = embed(ids, self.token_embed)
         return self.backbone(x) if sequence_group is None else self.backbone(x, sequence_group=sequence_group)
 
     def loss(self, ids: torch.Tensor, *, sequence_group=None) -> torch.Tensor:
@@ -72,7 +124,7 @@ class SLinOSSLM(nn.Module):
         if sequence_group is None:
             rows = self.hidden(ids)[:, :-1].reshape(-1, self.d_model)
             logits = F.linear(rows, self.token_embed.weight)
-            return F.cross_entropy(logits.float(), ids[:, 1:].reshape(-1))
+            return cross_entropy(logits, ids[:, 1:].reshape(-1))
         import torch.distributed as dist
         world, rank = dist.get_world_size(sequence_group), dist.get_rank(sequence_group)
         firsts = [torch.empty_like(ids[:, :1]) for _ in range(world)]
@@ -85,7 +137,7 @@ class SLinOSSLM(nn.Module):
         count = torch.tensor([targets.numel()], device=ids.device, dtype=torch.float64)
         dist.all_reduce(count, group=sequence_group)
         logits = F.linear(rows.reshape(-1, self.d_model), self.token_embed.weight)
-        return F.cross_entropy(logits.float(), targets.reshape(-1), reduction="sum") / count.item()
+        return cross_entropy(logits, targets.reshape(-1), reduction="sum") / count.item()
 
 
 def decay_groups(model: nn.Module, weight_decay: float):
@@ -112,8 +164,9 @@ class DataParallelTrainer:
         self.model, self.grad_clip = model, grad_clip
         self.sequence_parallel = bool(sequence_parallel)
         fused = self.fused = next(model.parameters()).is_cuda
-        self.opt = torch.optim.AdamW(decay_groups(model, weight_decay), lr=lr, betas=(0.9, 0.95),
-                                     fused=fused)
+        groups = decay_groups(model, weight_decay)
+        self.opt = optim.AdamW(groups, lr=lr, betas=(0.9, 0.95)) if fused else \
+            torch.optim.AdamW(groups, lr=lr, betas=(0.9, 0.95), fused=False)
         self.reducer = shard.GradBucketReducer(model.parameters(), bucket_bytes=bucket_bytes) \
             if reduce else None
 
@@ -147,9 +200,12 @@ class DataParallelTrainer:
         if not self.fused:
             torch.nn.utils.clip_grad_norm_(self.model.parameters(), self.grad_clip)
             return
+        # clip_grad_norm_'s coefficient is min(1, clip / (total + 1e-6)); grad_scale is its reciprocal
+        if len({g.device for g in grads}) == 1 and all(g.is_contiguous() and g.dtype in _C._DTYPE_CODE for g in grads):
+            self.last_grad_norm, self.opt.grad_scale = optim.grad_norm_and_scale(grads, self.grad_clip)
+            return
         norms = torch._foreach_norm(grads, 2.0)
         total = torch.linalg.vector_norm(torch.stack([n.float() for n in norms]), 2.0)
-        # clip_grad_norm_'s coefficient is min(1, clip / (total + 1e-6)); grad_scale is its reciprocal
         self.opt.grad_scale = torch.clamp((total + 1e-6) / self.grad_clip, min=1.0).reshape(())
         self.last_grad_norm = total
 

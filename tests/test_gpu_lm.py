@@ -64,3 +64,56 @@ def test_projection_backward_equals_autograd_of_the_three_gemms(dtype):
     for o, o2 in zip(outs, want):
         assert rel(o, o2) <= t
     assert rel(x.grad, x2.grad) <= t and rel(w.grad, w2.grad) <= t
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 1), (3, 7), (5, 256), (17, 4099), (9, 32000)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_cross_entropy_and_its_gradient_equal_torch(rows, vocab, dtype):
+    from slinoss_b200.lm import cross_entropy
+    torch.manual_seed(rows)
+    logits = (4 * torch.randn(rows, vocab, device=DEV)).to(dtype).requires_grad_()
+    targets = torch.randint(0, vocab, (rows,), device=DEV)
+    want_in = logits.detach().double().requires_grad_()
+    for reduction in ("mean", "sum"):
+        loss, want = cross_entropy(logits, targets, reduction=reduction), F.cross_entropy(want_in, targets, reduction=reduction)
+        (g,), (gw,) = torch.autograd.grad(loss * 3, logits), torch.autograd.grad(want * 3, want_in)
+        t = 1e-5 if dtype == torch.float32 else 1e-2
+        assert rel(loss, want) <= 1e-5 and (rel(g, gw) <= t or (g - gw).abs().max() < 1e-6)
+
+
+@pytest.mark.parametrize("n,vocab,width", [(1, 1, 8), (40, 7, 12), (300, 1000, 264), (513, 33, 2048)])
+def test_embedding_gradient_equals_torch(n, vocab, width):
+    from slinoss_b200.lm import embed
+    table = torch.nn.Embedding(vocab, width, device=DEV, dtype=torch.bfloat16)
+    ids = torch.randint(0, vocab, (n,), device=DEV)
+    d = torch.randn(n, width, device=DEV, dtype=torch.bfloat16)
+    (g,) = torch.autograd.grad(embed(ids, table), table.weight, d)
+    want = torch.zeros(vocab, width, device=DEV, dtype=torch.float64).index_add_(0, ids, d.double())
+    assert rel(g, want) <= 5e-3
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_adamw_equals_torch_also_after_loading_its_state_and_with_missing_gradients(dtype):
+    from slinoss_b200.optim import AdamW
+    torch.manual_seed(2)
+    shapes = [(1,), (7, 3), (64, 129), (8193,), (300, 256)] + [(5,)] * 70
+    a = [torch.nn.Parameter(torch.randn(s, device=DEV).to(dtype)) for s in shapes]
+    b = [torch.nn.Parameter(p.detach().clone()) for p in a]
+    groups = lambda ps: [{"params": ps[:3], "weight_decay": 0.05}, {"params": ps[3:], "weight_decay": 0.0}]
+    oa = AdamW(groups(a), lr=1e-2, betas=(0.9, 0.95))
+    ob = torch.optim.AdamW(groups(b), lr=1e-2, betas=(0.9, 0.95), fused=True)
+    for it in range(6):
+        for i, (p, q) in enumerate(zip(a, b)):
+            p.grad = None if (it == 3 and i % 2) else torch.randn_like(p)
+            q.grad = None if p.grad is None else p.grad.clone()
+        if it == 4:
+            state = oa.state_dict()
+            oa.load_state_dict(copy.deepcopy(ob.state_dict()))
+            ob.load_state_dict(copy.deepcopy(state))
+        oa.step()
+        ob.step()
+        for p, q in zip(a, b):
+            # (in bfloat16 a state may round the other way, which moves an element by a part of a step)
+            assert float((p - q).detach().abs().max()) <= (1e-5 if dtype == torch.float32 else 2e-2), (it, tuple(p.shape))
+            assert p.grad is None or torch.equal(p.grad, q.grad)
+            assert (p in oa.state) == (q in ob.state) and float(oa.state[p]["step"]) == float(ob.state[q]["step"])
