@@ -54,6 +54,40 @@ struct SkinnyArgs {
 bool skinny_supported(int M, int K, int O, int io_dtype);
 SL_API int skinny_linear(const SkinnyArgs& a, cudaStream_t st);
 
+// ---- scan preparation and mixer tail on strided rows ---------------------------------------------------------------------
+// Operands and results are rows of (batch * T) with a row stride each (columns of the in_proj output and of its
+// gradient); a null pointer skips its part, as in sl_scanprep_conv_fwd / _bwd.
+struct ScanPrepArgs {
+  const void* value; int64_t value_stride;
+  const void *conv_weight, *conv_bias, *conv_state_in;
+  void* conv_state_out;
+  int d_conv;
+  const void* params; int64_t params_stride;
+  const void* bc; int64_t bc_stride;
+  const float *dt_bias, *alpha_bias, *theta_mod_bias, *theta_bias, *theta_sign;
+  const sl_scanprep_config* cfg;
+  int64_t u_b, u_h, u_t;                    // strides of U (dU)
+  int batch, heads, groups, T, P, N, io_dtype;
+};
+struct ScanPrepOut { void* U; float *M, *K; void *B, *C; };
+struct ScanPrepGrads {
+  const void* dU; const float *dM, *dK; const void *dB, *dC;
+  void* d_value; int64_t d_value_stride;
+  float *d_conv_weight, *d_conv_bias;
+  void* d_conv_state;
+  void* d_params; int64_t d_params_stride;
+  void* d_bc; int64_t d_bc_stride;
+  float *d_dt_bias, *d_alpha_bias, *d_theta_mod_bias, *d_theta_bias;
+  const void* dY = nullptr;       // with skip: the gradient of U is dU + skip[head] * dY (dY laid out like dU)
+  const float* skip = nullptr;
+};
+SL_API int scanprep_fwd(const ScanPrepArgs& a, const ScanPrepOut& o, cudaStream_t st);
+SL_API int scanprep_bwd(const ScanPrepArgs& a, const ScanPrepGrads& g, cudaStream_t st);
+SL_API int mixer_tail_bwd(const void* Y, const void* gate, int64_t gate_stride, const void* skip, const float* d_skip,
+                          const void* norm_weight, float eps, const void* d_normed, void* dY, void* d_gate,
+                          int64_t d_gate_stride, void* d_skip_input, float* d_d_skip, float* d_norm_weight, int batch, int heads,
+                          int T, int P, int io_dtype, cudaStream_t st);
+
 // ---- language-model training step ------------------------------------------------------------------------------------
 SL_API int cross_entropy_fwd(const void* logits, const int64_t* target, float* loss, float* lse, int64_t rows, int V, int io,
                              cudaStream_t st);

@@ -9,6 +9,7 @@
 // heads*P channels; Y and U are read in their (batch, heads, T, P) layout and the
 // result is written channel-last, ready for the out_proj GEMM.
 #include "common.cuh"
+#include "host_abi.h"
 
 namespace sl {
 namespace {
@@ -35,7 +36,7 @@ struct TailParams {
   const float* d_skip;
   void *normed, *dY, *dgate, *dskip_in;
   float *d_d_skip, *d_w;
-  int64_t gs;
+  int64_t gs, dgs;   // row strides of gate and dgate
   float eps;
   int batch, H, T, P;
 };
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) tail_bwd_kernel(TailParams p) {
         const float g = to_f32(gate[(size_t)row * p.gs + c]);
         const float sg = sigmoid_f(g);
         const float dpre = dh * g * sg;
-        dgate[(size_t)row * C + c] = from_f32<T>(dh * pre * sg * (1.f + g * (1.f - sg)));
+        dgate[(size_t)row * p.dgs + c] = from_f32<T>(dh * pre * sg * (1.f + g * (1.f - sg)));
         dY[yi] = from_f32<T>(dpre);
         if (S) {
           if (dS) dS[yi] = from_f32<T>(dpre * p.d_skip[h]);
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) tail_bwd_vec_kernel(TailParams p
             if (S) { o_ds[k] = dpre * dsk[i]; dsk_acc[i] += dpre * sv[i][k]; }
           }
         }
-        store16<T>(dgate + (size_t)row * C + c, o_dg);
+        store16<T>(dgate + (size_t)row * p.dgs + c, o_dg);
         store16<T>(dY + yi, o_dy);
         if (S && dS) store16<T>(dS + yi, o_ds);
       }
@@ -376,7 +377,8 @@ __global__ void __launch_bounds__(TAIL_THREADS) tail_bwd_vec_kernel(TailParams p
 // The common width (heads * P <= 256 pieces of 16 bytes: one piece per thread) with fewer live registers,
 // so that three CTAs stay resident per SM: the row is kept as its four packed pieces and unpacked again
 // after the reduction (same operations, same roundings), both row sums travel in one reduction, and its
-// shared-memory slots alternate with the row so that one barrier per row is enough.
+// shared-memory slots alternate with the row so that one barrier per row is enough.  The CTA has just the warps the
+// row fills: with a fixed 256 threads a row of 1152 channels left 44 % of the lanes idle.
 template <typename T>
 __global__ void __launch_bounds__(TAIL_THREADS, 3) tail_bwd_row_kernel(TailParams p) {
   constexpr int V = Vec16<T>::N;
@@ -442,7 +444,8 @@ __global__ void __launch_bounds__(TAIL_THREADS, 3) tail_bwd_row_kernel(TailParam
     __syncthreads();
     ss = 0.f; dot = 0.f;
 #pragma unroll
-    for (int k = 0; k < TAIL_THREADS / 32; ++k) { const float2 v = s_red[par][k]; ss += v.x; dot += v.y; }
+    for (int k = 0; k < TAIL_THREADS / 32; ++k)
+      if (k < (int)(blockDim.x >> 5)) { const float2 v = s_red[par][k]; ss += v.x; dot += v.y; }
     const float rstd = rsqrtf(ss / (float)C + p.eps);
     const float coef = dot * rstd * rstd * rstd / (float)C;
     if (act) {
@@ -481,7 +484,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 3) tail_bwd_row_kernel(TailParam
           if (S) { o_ds[k] = dpre * dsk; dsk_acc += dpre * sv[k]; }
         }
       }
-      store16<T>(dgate + (size_t)row * C + c, o_dg);
+      store16<T>(dgate + (size_t)row * p.dgs + c, o_dg);
       store16<T>(dY + yi, o_dy);
       if (S && dS) store16<T>(dS + yi, o_ds);
     }
@@ -499,7 +502,7 @@ bool tail_vec_ok(const TailParams& p) {
   const long long C = (long long)p.H * p.P;
   auto al = [](const void* q) { return q == nullptr || aligned(q, 16); };
   return (long long)p.batch * p.T < (1ll << 31) && p.P % V == 0 && p.gs % V == 0 && C <= (long long)TAIL_VIT_MAX * TAIL_THREADS * V && al(p.Y) &&
-         al(p.gate) && al(p.skip) && al(p.w) && al(p.dn) && al(p.normed) && al(p.dY) && al(p.dgate) &&
+         al(p.gate) && al(p.skip) && al(p.w) && al(p.dn) && al(p.normed) && al(p.dY) && al(p.dgate) && p.dgs % V == 0 &&
          al(p.dskip_in);
 }
 
@@ -531,7 +534,11 @@ extern "C" int sl_mixer_tail_fwd(const void* Y, const void* gate, int64_t gate_r
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   SL_DISPATCH_DTYPE(io_dtype, Tt, {
     if (tail_vec_ok<Tt>(p)) {
-      if ((long long)heads * P <= TAIL_THREADS * Vec16<Tt>::N) tail_fwd_vec_kernel<Tt, 1><<<grid, TAIL_THREADS, 0, st>>>(p);
+      const int pieces = heads * P / Vec16<Tt>::N, threads = (pieces + 31) / 32 * 32;
+      if (pieces <= TAIL_THREADS) {   // one piece per thread, just the warps a row fills
+        const long long fit = 148ll * (8 * TAIL_THREADS / threads);
+        tail_fwd_vec_kernel<Tt, 1><<<(unsigned)(rows < fit ? rows : fit), threads, 0, st>>>(p);
+      }
       else tail_fwd_vec_kernel<Tt, 2><<<grid, TAIL_THREADS, 0, st>>>(p);
     } else tail_fwd_kernel<Tt><<<grid, TAIL_THREADS, 0, st>>>(p);
   });
@@ -539,30 +546,42 @@ extern "C" int sl_mixer_tail_fwd(const void* Y, const void* gate, int64_t gate_r
   return launch_status();
 }
 
-extern "C" int sl_mixer_tail_bwd(const void* Y, const void* gate, int64_t gate_row_stride,
-                                 const void* skip, const float* d_skip, const void* norm_weight,
-                                 float eps, const void* d_normed, void* dY, void* d_gate,
-                                 void* d_skip_input, float* d_d_skip, float* d_norm_weight,
-                                 int batch, int heads, int T, int P, int io_dtype, void* stream) {
-  using namespace sl;
+namespace sl {
+int mixer_tail_bwd(const void* Y, const void* gate, int64_t gate_stride, const void* skip, const float* d_skip,
+                   const void* norm_weight, float eps, const void* d_normed, void* dY, void* d_gate, int64_t d_gate_stride,
+                   void* d_skip_input, float* d_d_skip, float* d_norm_weight, int batch, int heads, int T, int P, int io_dtype,
+                   cudaStream_t st) {
   if (int e = tail_check(Y, gate, skip, d_skip, norm_weight, batch, heads, T, P, io_dtype)) return e;
   if (!d_normed || !dY || !d_gate || !d_norm_weight) return SL_ERR_NULL_POINTER;
   TailParams p{};
   p.Y = Y; p.gate = gate; p.skip = skip; p.w = norm_weight; p.d_skip = d_skip; p.dn = d_normed;
   p.dY = dY; p.dgate = d_gate; p.dskip_in = d_skip_input; p.d_d_skip = d_d_skip;
-  p.d_w = d_norm_weight; p.gs = gate_row_stride; p.eps = eps;
+  p.d_w = d_norm_weight; p.gs = gate_stride; p.dgs = d_gate_stride; p.eps = eps;
   p.batch = batch; p.H = heads; p.T = T; p.P = P;
   const long long rows = (long long)batch * T;
   const unsigned grid = (unsigned)(rows < 148 * 2 ? rows : 148 * 2);   // two resident CTAs per SM
-  const unsigned grid3 = (unsigned)(rows < 148 * 3 ? rows : 148 * 3);  // three for the one-piece kernel
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const size_t smem = (size_t)heads * sizeof(float);
   SL_DISPATCH_DTYPE(io_dtype, Tt, {
+    const int pieces = heads * P / Vec16<Tt>::N;
     if (tail_vec_ok<Tt>(p)) {
-      if ((long long)heads * P <= TAIL_THREADS * Vec16<Tt>::N) tail_bwd_row_kernel<Tt><<<grid3, TAIL_THREADS, 0, st>>>(p);
-      else tail_bwd_vec_kernel<Tt, 2><<<grid, TAIL_THREADS, 0, st>>>(p);
+      if (pieces <= TAIL_THREADS) {   // one piece per thread; 24 warps per SM stay resident
+        const int threads = (pieces + 31) / 32 * 32;
+        const long long fit = 148ll * (24 * 32 / threads);
+        tail_bwd_row_kernel<Tt><<<(unsigned)(rows < fit ? rows : fit), threads, 0, st>>>(p);
+      } else tail_bwd_vec_kernel<Tt, 2><<<grid, TAIL_THREADS, 0, st>>>(p);
     } else tail_bwd_kernel<Tt><<<grid, TAIL_THREADS, smem, st>>>(p);
   });
   note_launches(1);
   return launch_status();
+}
+}  // namespace sl
+
+extern "C" int sl_mixer_tail_bwd(const void* Y, const void* gate, int64_t gate_row_stride,
+                                 const void* skip, const float* d_skip, const void* norm_weight,
+                                 float eps, const void* d_normed, void* dY, void* d_gate,
+                                 void* d_skip_input, float* d_d_skip, float* d_norm_weight,
+                                 int batch, int heads, int T, int P, int io_dtype, void* stream) {
+  return sl::mixer_tail_bwd(Y, gate, gate_row_stride, skip, d_skip, norm_weight, eps, d_normed, dY, d_gate,
+                            (int64_t)heads * P, d_skip_input, d_d_skip, d_norm_weight, batch, heads, T, P, io_dtype,
+                            reinterpret_cast<cudaStream_t>(stream));
 }

@@ -20,6 +20,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "host_abi.h"
 
 namespace sl {
 namespace {
@@ -105,6 +106,9 @@ struct ValueBwdParams {
   ValueParams f;
   const void* dU;
   void *dx, *dstate;
+  int64_t dxs;                  // row stride of dx
+  const void* dY;               // optional, laid out like dU: the gradient of U is dU + skip[head] * dY
+  const float* skip;
   float *dw, *dbias;
 };
 
@@ -128,10 +132,11 @@ __global__ void __launch_bounds__(256) value_bwd_kernel(ValueBwdParams q) {
   const int h = c / p.P, pp = c - h * p.P;
   const int t1 = min(t0 + CONV_TT, p.T);
   auto dy_at = [&](int t) -> float {
-    return to_f32(dU[(size_t)b * p.usb + (size_t)h * p.ush + (size_t)t * p.ust + pp]);
+    const size_t i = (size_t)b * p.usb + (size_t)h * p.ush + (size_t)t * p.ust + pp;
+    return to_f32(dU[i]) + (q.dY ? q.skip[h] * to_f32(reinterpret_cast<const T*>(q.dY)[i]) : 0.f);
   };
   if (!p.w) {
-    for (int t = t0; t < t1; ++t) dx[((size_t)b * p.T + t) * p.C + c] = from_f32<T>(dy_at(t));
+    for (int t = t0; t < t1; ++t) dx[((size_t)b * p.T + t) * q.dxs + c] = from_f32<T>(dy_at(t));
     return;
   }
   const T* w = reinterpret_cast<const T*>(p.w);
@@ -168,7 +173,7 @@ __global__ void __launch_bounds__(256) value_bwd_kernel(ValueBwdParams q) {
     // dx[t] = sum_k wj[k] * da[t + 3 - k], complete for t = s - 3
     const int t = s - 3;
     const float g = wj[3] * da[0] + wj[2] * da[1] + wj[1] * da[2] + wj[0] * da[3];
-    if (t >= t0 && t < t1) dx[((size_t)b * p.T + t) * p.C + c] = from_f32<T>(g);
+    if (t >= t0 && t < t1) dx[((size_t)b * p.T + t) * q.dxs + c] = from_f32<T>(g);
     else if (t < 0 && t0 == 0 && q.dstate && t >= -(W - 1))
       reinterpret_cast<T*>(q.dstate)[((size_t)b * p.C + c) * (W - 1) + (W - 1 + t)] = from_f32<T>(g);
   }
@@ -317,7 +322,7 @@ __global__ void __launch_bounds__(256, 3) value_fwd_vec_kernel(ValueParams p) {
   }
 }
 
-template <typename T>
+template <typename T, bool SKIP>
 __global__ void __launch_bounds__(256, 2) value_bwd_vec_kernel(ValueBwdParams q) {
   const ValueParams& p = q.f;
   __shared__ float s_acc[CONV_SUB][5][32 * CONV_V];   // dw (4 taps) and dbias partials per sub-tile
@@ -338,13 +343,25 @@ __global__ void __launch_bounds__(256, 2) value_bwd_vec_kernel(ValueBwdParams q)
     const T* dU = reinterpret_cast<const T*>(q.dU);
     T* dx = reinterpret_cast<T*>(q.dx);
     const int h = c / p.P, pp = c - h * p.P;
-    const T* dUb = dU + (size_t)b * p.usb + (size_t)h * p.ush + pp;
+    const size_t ub = (size_t)b * p.usb + (size_t)h * p.ush + pp;
+    const T* dUb = dU + ub;
+    const T* dYb = SKIP ? reinterpret_cast<const T*>(q.dY) + ub : nullptr;
+    const float skip = SKIP ? q.skip[h] : 0.f;
+    auto load_gy = [&](int t, float (&v)[CONV_V]) {
+      load4<T>(dUb + (size_t)t * p.ust, v);
+      if constexpr (SKIP) {
+        float y[CONV_V];
+        load4<T>(dYb + (size_t)t * p.ust, y);
+#pragma unroll
+        for (int k = 0; k < CONV_V; ++k) v[k] = fmaf(skip, y[k], v[k]);
+      }
+    };
     const int t1 = min(t0 + CONV_TT, p.T);
     if (!p.w) {
       for (int t = t0; t < t1; ++t) {
         float v[CONV_V];
-        load4<T>(dUb + (size_t)t * p.ust, v);
-        store4<T>(dx + ((size_t)b * p.T + t) * p.C + c, v);
+        load_gy(t, v);
+        store4<T>(dx + ((size_t)b * p.T + t) * q.dxs + c, v);
       }
     } else {
       const T* w = reinterpret_cast<const T*>(p.w);
@@ -411,7 +428,7 @@ __global__ void __launch_bounds__(256, 2) value_bwd_vec_kernel(ValueBwdParams q)
           g[k] = wj[3][k] * da[0][k] + wj[2][k] * da[1][k] + wj[1][k] * da[2][k] + wj[0][k] * da[3][k];
         }
         const int t = s - 3;
-        if (t >= t0 && t < t1) store4<T>(dx + ((size_t)b * p.T + t) * p.C + c, g);
+        if (t >= t0 && t < t1) store4<T>(dx + ((size_t)b * p.T + t) * q.dxs + c, g);
         else if (t < 0 && t0 == 0 && q.dstate && t >= -(W - 1)) {
 #pragma unroll
           for (int k = 0; k < CONV_V; ++k)
@@ -426,11 +443,12 @@ __global__ void __launch_bounds__(256, 2) value_bwd_vec_kernel(ValueBwdParams q)
 #pragma unroll 1
         for (int sb = s_begin; sb < s_end; sb += SB) {
           using Raw = typename std::conditional<sizeof(T) == 4, uint4, uint2>::type;   // 4 channels
-          Raw xr[SB], gr[SB];
+          Raw xr[SB], gr[SB], yr[SKIP ? SB : 1];
 #pragma unroll
           for (int i = 0; i < SB; ++i) {
             xr[i] = *reinterpret_cast<const Raw*>(x + ((size_t)b * p.T + sb + i) * p.xs + c);
             gr[i] = *reinterpret_cast<const Raw*>(dUb + (size_t)(sb + i) * p.ust);
+            if constexpr (SKIP) yr[i] = *reinterpret_cast<const Raw*>(dYb + (size_t)(sb + i) * p.ust);
           }
 #pragma unroll
           for (int i = 0; i < SB; ++i) {
@@ -439,6 +457,11 @@ __global__ void __launch_bounds__(256, 2) value_bwd_vec_kernel(ValueBwdParams q)
             const T* eg = reinterpret_cast<const T*>(&gr[i]);
 #pragma unroll
             for (int k = 0; k < CONV_V; ++k) { xin[k] = to_f32(ex[k]); gy[k] = to_f32(eg[k]); }
+            if constexpr (SKIP) {
+              const T* ey = reinterpret_cast<const T*>(&yr[i]);
+#pragma unroll
+              for (int k = 0; k < CONV_V; ++k) gy[k] = fmaf(skip, to_f32(ey[k]), gy[k]);
+            }
             step(sb + i, true, xin, gy);
           }
         }
@@ -448,7 +471,7 @@ __global__ void __launch_bounds__(256, 2) value_bwd_vec_kernel(ValueBwdParams q)
           const bool in = s < p.T;
           if (in) {
             load4<T>(x + ((size_t)b * p.T + s) * p.xs + c, xin);
-            load4<T>(dUb + (size_t)s * p.ust, gy);
+            load_gy(s, gy);
           }
           step(s, in, xin, gy);
         }
@@ -487,7 +510,7 @@ inline bool value_vec_ok(const ValueParams& p, const void* a, const void* b, int
 
 template <typename T>
 __global__ void __launch_bounds__(256) bc_fwd_kernel(const T* __restrict__ bc, T* __restrict__ Bo,
-                                                     T* __restrict__ Co, int batch, int Tn,
+                                                     T* __restrict__ Co, int64_t bcs, int batch, int Tn,
                                                      int G, int N, float eps) {
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -495,7 +518,7 @@ __global__ void __launch_bounds__(256) bc_fwd_kernel(const T* __restrict__ bc, T
   const int g = (int)(row % G);
   const long long bt = row / G;
   const int t = (int)(bt % Tn), b = (int)(bt / Tn);
-  const T* src = bc + (size_t)row * 4 * N;
+  const T* src = bc + (size_t)bt * bcs + (size_t)g * 4 * N;
   T* outs[2] = {Bo + (((size_t)b * G + g) * Tn + t) * 2 * N, Co + (((size_t)b * G + g) * Tn + t) * 2 * N};
 #pragma unroll
   for (int which = 0; which < 2; ++which) {
@@ -523,16 +546,16 @@ template <typename T>
 __global__ void __launch_bounds__(256) bc_bwd_kernel(const T* __restrict__ bc,
                                                      const T* __restrict__ dBo,
                                                      const T* __restrict__ dCo,
-                                                     T* __restrict__ dbc, int batch, int Tn,
-                                                     int G, int N, float eps) {
+                                                     T* __restrict__ dbc, int64_t bcs, int64_t dbcs, int batch,
+                                                     int Tn, int G, int N, float eps) {
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= (long long)batch * Tn * G) return;
   const int g = (int)(row % G);
   const long long bt = row / G;
   const int t = (int)(bt % Tn), b = (int)(bt / Tn);
-  const T* src = bc + (size_t)row * 4 * N;
-  T* dst = dbc + (size_t)row * 4 * N;
+  const T* src = bc + (size_t)bt * bcs + (size_t)g * 4 * N;
+  T* dst = dbc + (size_t)bt * dbcs + (size_t)g * 4 * N;
   const T* gs[2] = {dBo + (((size_t)b * G + g) * Tn + t) * 2 * N, dCo + (((size_t)b * G + g) * Tn + t) * 2 * N};
 #pragma unroll
   for (int which = 0; which < 2; ++which) {
@@ -567,10 +590,12 @@ __global__ void __launch_bounds__(256) bc_bwd_kernel(const T* __restrict__ bc,
   }
 }
 
-// ---- vector path of the B / C kernels (N % 4 == 0, N <= 64) ----------------------------------------
-// One warp per (batch, token, group) record of 4 rows x N: lanes 0-15 produce B, lanes 16-31 C;
+// ---- vector path of the B / C kernels (N % 4 == 0, N <= 128) ---------------------------------------
+// One warp per (batch, token, group) record of 4 rows x N: lanes 0-15 produce B, lanes 16-31 C (N <= 64), or
+// two neighbouring warps, one for B and one for C (WIDE, N <= 128: the one-element-per-lane kernels above took
+// 53 us for 1021 tokens x 32 groups x 128);
 // a lane owns 4 consecutive n: two 8-byte loads (amplitude and phase logits), one 16-byte store of
-// 4 complex values.  The mean over n is a shuffle reduction inside the 16-lane half.  With 16-bit
+// 4 complex values.  The mean over n is a shuffle reduction inside the lanes of B or C.  With 16-bit
 // io the transcendental functions are the fast intrinsics (their error is far below the output's
 // rounding); float32 io keeps the precise ones.
 template <bool FAST> __device__ __forceinline__ float softplus_v(float x) {
@@ -611,9 +636,9 @@ template <typename T> __device__ __forceinline__ void store8(T* p, const float (
       *reinterpret_cast<float4*>(p + 4 * h) = make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
   }
 }
-__device__ __forceinline__ float half_warp_sum(float v) {   // over the 16 lanes of a half-warp
+template <bool WIDE> __device__ __forceinline__ float part_sum(float v) {   // over the 16 (WIDE: 32) lanes of B or C
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = WIDE ? 16 : 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
@@ -623,16 +648,17 @@ constexpr int BC_GCH = 8;   // groups one warp walks: grid = (tokens / 8, groups
 // index is divided at run time.  The next record's logits are requested before the current one is
 // evaluated.  (The kernels are bound by instruction issue and the XU pipe - five to six MUFU operations per
 // complex pair - not by DRAM.)
-template <typename T>
+template <typename T, bool WIDE>
 __global__ void __launch_bounds__(256) bc_fwd_vec_kernel(const T* __restrict__ bc, T* __restrict__ Bo,
-                                                         T* __restrict__ Co, int Tn, int G, int N, float eps) {
+                                                         T* __restrict__ Co, int64_t bcs, int Tn, int G, int N, float eps) {
   constexpr bool FAST = sizeof(T) == 2;
-  const int lane = threadIdx.x & 31, which = lane >> 4, n0 = 4 * (lane & 15);
-  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), b = blockIdx.z;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int which = WIDE ? warp & 1 : lane >> 4, n0 = 4 * (WIDE ? lane : lane & 15);
+  const int t = WIDE ? blockIdx.x * 4 + (warp >> 1) : blockIdx.x * 8 + warp, b = blockIdx.z;
   const int g0 = blockIdx.y * BC_GCH, g1 = min(G, g0 + BC_GCH);
   if (t >= Tn) return;
   const bool act = n0 < N;
-  const T* src = bc + (((size_t)b * Tn + t) * G + g0) * 4 * N + (size_t)(2 * which) * N + n0;
+  const T* src = bc + ((size_t)b * Tn + t) * bcs + (size_t)(4 * g0 + 2 * which) * N + n0;
   T* dst = (which ? Co : Bo) + (((size_t)b * G + g0) * Tn + t) * 2 * N + 2 * n0;
   const size_t dstep = (size_t)Tn * 2 * N;
   const float inv_n = 1.f / (float)N;
@@ -648,7 +674,7 @@ __global__ void __launch_bounds__(256) bc_fwd_vec_kernel(const T* __restrict__ b
       amp[i] = act ? softplus_v<FAST>(amp[i]) : 0.f;
       ss += amp[i] * amp[i];
     }
-    ss = half_warp_sum(ss);
+    ss = part_sum<WIDE>(ss);
     if (act) {
       const float inv = rsqrtf(fmaxf(ss * inv_n, eps));
       float o[8];
@@ -667,20 +693,22 @@ __global__ void __launch_bounds__(256) bc_fwd_vec_kernel(const T* __restrict__ b
   }
 }
 
-template <typename T>
+template <typename T, bool WIDE>
 __global__ void __launch_bounds__(256) bc_bwd_vec_kernel(const T* __restrict__ bc,
                                                          const T* __restrict__ dBo,
                                                          const T* __restrict__ dCo,
-                                                         T* __restrict__ dbc, int Tn, int G, int N, float eps) {
+                                                         T* __restrict__ dbc, int64_t bcs, int64_t dbcs, int Tn, int G,
+                                                         int N, float eps) {
   constexpr bool FAST = sizeof(T) == 2;
-  const int lane = threadIdx.x & 31, which = lane >> 4, n0 = 4 * (lane & 15);
-  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), b = blockIdx.z;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int which = WIDE ? warp & 1 : lane >> 4, n0 = 4 * (WIDE ? lane : lane & 15);
+  const int t = WIDE ? blockIdx.x * 4 + (warp >> 1) : blockIdx.x * 8 + warp, b = blockIdx.z;
   const int g0 = blockIdx.y * BC_GCH, g1 = min(G, g0 + BC_GCH);
   if (t >= Tn) return;
   const bool act = n0 < N;
-  const size_t in_off = (((size_t)b * Tn + t) * G + g0) * 4 * N + (size_t)(2 * which) * N + n0;
-  const T* src = bc + in_off;
-  T* dst = dbc + in_off;
+  const size_t in_off = (size_t)(4 * g0 + 2 * which) * N + n0;
+  const T* src = bc + ((size_t)b * Tn + t) * bcs + in_off;
+  T* dst = dbc + ((size_t)b * Tn + t) * dbcs + in_off;
   const T* grad = (which ? dCo : dBo) + (((size_t)b * G + g0) * Tn + t) * 2 * N + 2 * n0;
   const size_t gstep = (size_t)Tn * 2 * N;
   const float inv_n = 1.f / (float)N;
@@ -704,7 +732,7 @@ __global__ void __launch_bounds__(256) bc_bwd_vec_kernel(const T* __restrict__ b
       ss += a[i] * a[i];
       gsum += a[i] * (cs[i] * gr[2 * i] + sn[i] * gr[2 * i + 1]);
     }
-    ss = half_warp_sum(ss); gsum = half_warp_sum(gsum);
+    ss = part_sum<WIDE>(ss); gsum = part_sum<WIDE>(gsum);
     if (act) {
       const float ms = ss * inv_n;
       const float inv = rsqrtf(fmaxf(ms, eps));
@@ -729,9 +757,12 @@ __global__ void __launch_bounds__(256) bc_bwd_vec_kernel(const T* __restrict__ b
   }
 }
 
-inline bool bc_vec_ok(int batch, int groups, int N, const void* a, const void* b, const void* c, const void* d) {
-  return batch <= 65535 && (groups + BC_GCH - 1) / BC_GCH <= 65535 && N % 4 == 0 && N <= 64 && aligned(a, 16) &&
-         aligned(b, 16) && aligned(c, 16) && (d == nullptr || aligned(d, 16));
+// (the logits and their gradients are read and written 4 at a time: 8 bytes of 16-bit values)
+inline bool bc_vec_ok(int batch, int groups, int N, const void* a, const void* b, const void* c, const void* d, int64_t bcs,
+                      int64_t dbcs, int io) {
+  const size_t in = io == SL_F32 ? 16 : 8;
+  return batch <= 65535 && (groups + BC_GCH - 1) / BC_GCH <= 65535 && N % 4 == 0 && N <= 128 && aligned(a, in) &&
+         aligned(b, 16) && aligned(c, 16) && (d == nullptr || aligned(d, in)) && bcs % 4 == 0 && dbcs % 4 == 0;
 }
 
 // (the coefficient arithmetic - zc, CoeffOut, wrap_angle_f, coeff_eval - lives in scanprep_math.cuh)
@@ -742,6 +773,7 @@ struct CoeffParams {
   float *M, *K;
   const float *dM, *dK;
   void* dparams;
+  int64_t ps, dps;              // row strides of params and dparams
   float *d_dt_bias, *d_alpha_bias, *d_theta_mod_bias, *d_theta_bias;
   int batch, T, H;
 };
@@ -751,7 +783,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) coeff_fwd_kernel(CoeffParams p) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x, h = blockIdx.y, b = blockIdx.z;
   if (t >= p.T) return;
-  const T* pr = reinterpret_cast<const T*>(p.params) + ((size_t)b * p.T + t) * 3 * p.H + 3 * h;
+  const T* pr = reinterpret_cast<const T*>(p.params) + ((size_t)b * p.T + t) * p.ps + 3 * h;
   const CoeffOut o = coeff_eval<false>(to_f32(pr[0]) + p.dt_bias[h], to_f32(pr[1]) + p.alpha_bias[h],
                                 to_f32(pr[2]) + p.theta_mod_bias[h], p.theta_bias[h],
                                 p.theta_sign[h], p.cfg);
@@ -768,7 +800,7 @@ __global__ void __launch_bounds__(128) coeff_bwd_kernel(CoeffParams p) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x, h = blockIdx.y, b = blockIdx.z;
   float g0 = 0.f, g1 = 0.f, g2 = 0.f, gx = 0.f;
   if (t < p.T) {
-    const T* pr = reinterpret_cast<const T*>(p.params) + ((size_t)b * p.T + t) * 3 * p.H + 3 * h;
+    const T* pr = reinterpret_cast<const T*>(p.params) + ((size_t)b * p.T + t) * p.ps + 3 * h;
     const CoeffOut o = coeff_eval(to_f32(pr[0]) + p.dt_bias[h], to_f32(pr[1]) + p.alpha_bias[h],
                                   to_f32(pr[2]) + p.theta_mod_bias[h], p.theta_bias[h],
                                   p.theta_sign[h], p.cfg);
@@ -793,7 +825,7 @@ __global__ void __launch_bounds__(128) coeff_bwd_kernel(CoeffParams p) {
     g1 = (float)((double)(p.cfg.alpha_max - p.cfg.alpha_min) * o.dsg_al * g_alpha);
     g2 = (float)((double)p.cfg.theta_mod_scale * (1.0 - o.tanh2) * g_x);
     gx = (float)g_x;
-    T* dp = reinterpret_cast<T*>(p.dparams) + ((size_t)b * p.T + t) * 3 * p.H + 3 * h;
+    T* dp = reinterpret_cast<T*>(p.dparams) + ((size_t)b * p.T + t) * p.dps + 3 * h;
     dp[0] = from_f32<T>(g0); dp[1] = from_f32<T>(g1); dp[2] = from_f32<T>(g2);
   }
   g0 = warp_sum(g0); g1 = warp_sum(g1); g2 = warp_sum(g2); gx = warp_sum(gx);
@@ -881,6 +913,132 @@ struct PartFork {
 };
 
 }  // namespace
+
+int scanprep_fwd(const ScanPrepArgs& a, const ScanPrepOut& o, cudaStream_t st) {
+  if (int e = check_common(a.batch, a.heads, a.groups, a.T, a.P, a.N, a.io_dtype, a.conv_weight ? a.d_conv : 1)) return e;
+  if (a.value && !o.U) return SL_ERR_NULL_POINTER;
+  if (a.bc && (!o.B || !o.C || !a.cfg)) return SL_ERR_NULL_POINTER;
+  if (a.params) {
+    if (!o.M || !o.K || !a.cfg || !a.dt_bias || !a.alpha_bias || !a.theta_mod_bias || !a.theta_bias || !a.theta_sign)
+      return SL_ERR_NULL_POINTER;
+    if (!aligned(o.M, 8) || !aligned(o.K, 16)) return SL_ERR_BAD_ALIGNMENT;
+  }
+  const int batch = a.batch, T = a.T, heads = a.heads, groups = a.groups, N = a.N;
+  PartFork fork(st, (a.value != nullptr) + (a.bc != nullptr) + (a.params != nullptr), (long long)batch * T);
+  if (a.value) {
+    ValueParams p{};
+    p.x = a.value; p.w = a.conv_weight; p.bias = a.conv_bias; p.state_in = a.conv_state_in;
+    p.state_out = a.conv_state_out; p.U = o.U; p.xs = a.value_stride;
+    p.usb = a.u_b; p.ush = a.u_h; p.ust = a.u_t;
+    p.batch = batch; p.T = T; p.C = heads * a.P; p.P = a.P; p.W = a.conv_weight ? a.d_conv : 1;
+    const int vf = CONV_V;   // 4 channels per thread (8- or 16-byte pieces)
+    if (value_vec_ok(p, nullptr, nullptr, vf)) {
+      dim3 grid((p.C + 32 * vf - 1) / (32 * vf), (T + CONV_SUB * CONV_TT - 1) / (CONV_SUB * CONV_TT), batch);
+      SL_DISPATCH_DTYPE(a.io_dtype, Tt, { value_fwd_vec_kernel<Tt, CONV_V><<<grid, 256, 0, fork.v>>>(p); });
+    } else {
+      dim3 grid((p.C + 255) / 256, (T + CONV_TT - 1) / CONV_TT, batch);
+      SL_DISPATCH_DTYPE(a.io_dtype, Tt, { value_fwd_kernel<Tt><<<grid, 256, 0, fork.v>>>(p); });
+    }
+    note_launches(1);
+  }
+  if (a.bc) {
+    const long long rows = (long long)batch * T * groups;
+    const bool wide = N > 64;
+    const dim3 vgrid((T + (wide ? 3 : 7)) / (wide ? 4 : 8), (groups + BC_GCH - 1) / BC_GCH, batch);
+    const float eps = a.cfg->eps;
+    SL_DISPATCH_DTYPE(a.io_dtype, Tt, {
+      const Tt* bc = reinterpret_cast<const Tt*>(a.bc);
+      Tt *Bo = reinterpret_cast<Tt*>(o.B), *Co = reinterpret_cast<Tt*>(o.C);
+      if (!bc_vec_ok(batch, groups, N, bc, Bo, Co, nullptr, a.bc_stride, 0, a.io_dtype))
+        bc_fwd_kernel<Tt><<<(unsigned)((rows + 7) / 8), 256, 0, fork.b>>>(bc, Bo, Co, a.bc_stride, batch, T, groups, N, eps);
+      else if (wide)
+        bc_fwd_vec_kernel<Tt, true><<<vgrid, 256, 0, fork.b>>>(bc, Bo, Co, a.bc_stride, T, groups, N, eps);
+      else
+        bc_fwd_vec_kernel<Tt, false><<<vgrid, 256, 0, fork.b>>>(bc, Bo, Co, a.bc_stride, T, groups, N, eps);
+    });
+    note_launches(1);
+  }
+  if (a.params) {
+    CoeffParams p{};
+    p.params = a.params; p.ps = a.params_stride; p.dt_bias = a.dt_bias; p.alpha_bias = a.alpha_bias;
+    p.theta_mod_bias = a.theta_mod_bias; p.theta_bias = a.theta_bias; p.theta_sign = a.theta_sign;
+    p.cfg = *a.cfg; p.M = o.M; p.K = o.K; p.batch = batch; p.T = T; p.H = heads;
+    dim3 grid((T + 127) / 128, heads, batch);
+    SL_DISPATCH_DTYPE(a.io_dtype, Tt, { coeff_fwd_kernel<Tt><<<grid, 128, 0, fork.c>>>(p); });
+    note_launches(1);
+  }
+  fork.join();
+  return launch_status();
+}
+
+int scanprep_bwd(const ScanPrepArgs& a, const ScanPrepGrads& g, cudaStream_t st) {
+  if (int e = check_common(a.batch, a.heads, a.groups, a.T, a.P, a.N, a.io_dtype, a.conv_weight ? a.d_conv : 1)) return e;
+  if (g.dU && (!g.d_value || !a.value || (a.conv_weight && !g.d_conv_weight) || (g.dY && !g.skip))) return SL_ERR_NULL_POINTER;
+  if (g.dB && (!g.dC || !a.bc || !g.d_bc || !a.cfg)) return SL_ERR_NULL_POINTER;
+  if (g.dM) {
+    if (!g.dK || !a.params || !g.d_params || !a.cfg || !a.dt_bias || !a.alpha_bias || !a.theta_mod_bias || !a.theta_bias ||
+        !a.theta_sign)
+      return SL_ERR_NULL_POINTER;
+    if (!aligned(g.dM, 8) || !aligned(g.dK, 16)) return SL_ERR_BAD_ALIGNMENT;
+  }
+  const int batch = a.batch, T = a.T, heads = a.heads, groups = a.groups, N = a.N;
+  PartFork fork(st, (g.dU != nullptr) + (g.dB != nullptr) + (g.dM != nullptr), (long long)batch * T);
+  if (g.dU) {
+    ValueBwdParams q{};
+    ValueParams& p = q.f;
+    p.x = a.value; p.w = a.conv_weight; p.bias = a.conv_bias; p.state_in = a.conv_state_in;
+    p.xs = a.value_stride; p.usb = a.u_b; p.ush = a.u_h; p.ust = a.u_t;
+    p.batch = batch; p.T = T; p.C = heads * a.P; p.P = a.P; p.W = a.conv_weight ? a.d_conv : 1;
+    q.dU = g.dU; q.dx = g.d_value; q.dxs = g.d_value_stride; q.dstate = g.d_conv_state; q.dw = g.d_conv_weight;
+    q.dbias = g.d_conv_bias; q.dY = g.dY; q.skip = g.skip;
+    ValueParams pv = p;
+    pv.U = const_cast<void*>(g.dU);
+    if (value_vec_ok(pv, g.d_value, nullptr) && g.d_value_stride % CONV_V == 0 && aligned(g.dY, 16)) {
+      dim3 grid((p.C + 32 * CONV_V - 1) / (32 * CONV_V), (T + CONV_SUB * CONV_TT - 1) / (CONV_SUB * CONV_TT), batch);
+      SL_DISPATCH_DTYPE(a.io_dtype, Tt, {
+        if (g.dY) value_bwd_vec_kernel<Tt, true><<<grid, 256, 0, fork.v>>>(q);
+        else value_bwd_vec_kernel<Tt, false><<<grid, 256, 0, fork.v>>>(q);
+      });
+    } else {
+      dim3 grid((p.C + 255) / 256, (T + CONV_TT - 1) / CONV_TT, batch);
+      SL_DISPATCH_DTYPE(a.io_dtype, Tt, { value_bwd_kernel<Tt><<<grid, 256, 0, fork.v>>>(q); });
+    }
+    note_launches(1);
+  }
+  if (g.dB) {
+    const long long rows = (long long)batch * T * groups;
+    const bool wide = N > 64;
+    const dim3 vgrid((T + (wide ? 3 : 7)) / (wide ? 4 : 8), (groups + BC_GCH - 1) / BC_GCH, batch);
+    const float eps = a.cfg->eps;
+    SL_DISPATCH_DTYPE(a.io_dtype, Tt, {
+      const Tt *bc = reinterpret_cast<const Tt*>(a.bc), *dB = reinterpret_cast<const Tt*>(g.dB);
+      const Tt* dC = reinterpret_cast<const Tt*>(g.dC);
+      Tt* dbc = reinterpret_cast<Tt*>(g.d_bc);
+      if (!bc_vec_ok(batch, groups, N, bc, dB, dC, dbc, a.bc_stride, g.d_bc_stride, a.io_dtype))
+        bc_bwd_kernel<Tt><<<(unsigned)((rows + 7) / 8), 256, 0, fork.b>>>(bc, dB, dC, dbc, a.bc_stride, g.d_bc_stride, batch, T,
+                                                                          groups, N, eps);
+      else if (wide)
+        bc_bwd_vec_kernel<Tt, true><<<vgrid, 256, 0, fork.b>>>(bc, dB, dC, dbc, a.bc_stride, g.d_bc_stride, T, groups, N, eps);
+      else
+        bc_bwd_vec_kernel<Tt, false><<<vgrid, 256, 0, fork.b>>>(bc, dB, dC, dbc, a.bc_stride, g.d_bc_stride, T, groups, N, eps);
+    });
+    note_launches(1);
+  }
+  if (g.dM) {
+    CoeffParams p{};
+    p.params = a.params; p.ps = a.params_stride; p.dt_bias = a.dt_bias; p.alpha_bias = a.alpha_bias;
+    p.theta_mod_bias = a.theta_mod_bias; p.theta_bias = a.theta_bias; p.theta_sign = a.theta_sign;
+    p.cfg = *a.cfg; p.dM = g.dM; p.dK = g.dK; p.dparams = g.d_params; p.dps = g.d_params_stride; p.d_dt_bias = g.d_dt_bias;
+    p.d_alpha_bias = g.d_alpha_bias; p.d_theta_mod_bias = g.d_theta_mod_bias;
+    p.d_theta_bias = g.d_theta_bias; p.batch = batch; p.T = T; p.H = heads;
+    dim3 grid((T + 127) / 128, heads, batch);
+    SL_DISPATCH_DTYPE(a.io_dtype, Tt, { coeff_bwd_kernel<Tt><<<grid, 128, 0, fork.c>>>(p); });
+    note_launches(1);
+  }
+  fork.join();
+  return launch_status();
+}
+
 }  // namespace sl
 
 extern "C" int sl_scanprep_conv_fwd(const void* value, int64_t value_row_stride,
@@ -893,58 +1051,11 @@ extern "C" int sl_scanprep_conv_fwd(const void* value, int64_t value_row_stride,
                                     int64_t u_stride_h, int64_t u_stride_t, float* M, float* K,
                                     void* Bo, void* Co, int batch, int heads, int groups, int T,
                                     int P, int N, int io_dtype, void* stream) {
-  using namespace sl;
-  if (int e = check_common(batch, heads, groups, T, P, N, io_dtype, conv_weight ? d_conv : 1)) return e;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (value && !U) return SL_ERR_NULL_POINTER;
-  if (bc && (!Bo || !Co || !cfg)) return SL_ERR_NULL_POINTER;
-  if (params) {
-    if (!M || !K || !cfg || !dt_bias || !alpha_bias || !theta_mod_bias || !theta_bias || !theta_sign)
-      return SL_ERR_NULL_POINTER;
-    if (!aligned(M, 8) || !aligned(K, 16)) return SL_ERR_BAD_ALIGNMENT;
-  }
-  PartFork fork(st, (value != nullptr) + (bc != nullptr) + (params != nullptr), (long long)batch * T);
-  if (value) {
-    ValueParams p{};
-    p.x = value; p.w = conv_weight; p.bias = conv_bias; p.state_in = conv_state_in;
-    p.state_out = conv_state_out; p.U = U; p.xs = value_row_stride;
-    p.usb = u_stride_b; p.ush = u_stride_h; p.ust = u_stride_t;
-    p.batch = batch; p.T = T; p.C = heads * P; p.P = P; p.W = conv_weight ? d_conv : 1;
-    const int vf = CONV_V;   // 4 channels per thread (8- or 16-byte pieces)
-    if (value_vec_ok(p, nullptr, nullptr, vf)) {
-      dim3 grid((p.C + 32 * vf - 1) / (32 * vf), (T + CONV_SUB * CONV_TT - 1) / (CONV_SUB * CONV_TT), batch);
-      SL_DISPATCH_DTYPE(io_dtype, Tt, { value_fwd_vec_kernel<Tt, CONV_V><<<grid, 256, 0, fork.v>>>(p); });
-    } else {
-      dim3 grid((p.C + 255) / 256, (T + CONV_TT - 1) / CONV_TT, batch);
-      SL_DISPATCH_DTYPE(io_dtype, Tt, { value_fwd_kernel<Tt><<<grid, 256, 0, fork.v>>>(p); });
-    }
-    note_launches(1);
-  }
-  if (bc) {
-    const long long rows = (long long)batch * T * groups;
-    const unsigned blocks = (unsigned)((rows + 7) / 8);
-    const dim3 vgrid((T + 7) / 8, (groups + BC_GCH - 1) / BC_GCH, batch);
-    SL_DISPATCH_DTYPE(io_dtype, Tt, {
-      if (bc_vec_ok(batch, groups, N, bc, Bo, Co, nullptr))
-        bc_fwd_vec_kernel<Tt><<<vgrid, 256, 0, fork.b>>>(reinterpret_cast<const Tt*>(bc), reinterpret_cast<Tt*>(Bo),
-                                                     reinterpret_cast<Tt*>(Co), T, groups, N, cfg->eps);
-      else
-        bc_fwd_kernel<Tt><<<blocks, 256, 0, fork.b>>>(reinterpret_cast<const Tt*>(bc), reinterpret_cast<Tt*>(Bo),
-                                                  reinterpret_cast<Tt*>(Co), batch, T, groups, N, cfg->eps);
-    });
-    note_launches(1);
-  }
-  if (params) {
-    CoeffParams p{};
-    p.params = params; p.dt_bias = dt_bias; p.alpha_bias = alpha_bias;
-    p.theta_mod_bias = theta_mod_bias; p.theta_bias = theta_bias; p.theta_sign = theta_sign;
-    p.cfg = *cfg; p.M = M; p.K = K; p.batch = batch; p.T = T; p.H = heads;
-    dim3 grid((T + 127) / 128, heads, batch);
-    SL_DISPATCH_DTYPE(io_dtype, Tt, { coeff_fwd_kernel<Tt><<<grid, 128, 0, fork.c>>>(p); });
-    note_launches(1);
-  }
-  fork.join();
-  return launch_status();
+  const sl::ScanPrepArgs a{value, value_row_stride, conv_weight, conv_bias, conv_state_in, conv_state_out, d_conv,
+                           params, 3 * (int64_t)heads, bc, 4 * (int64_t)groups * N, dt_bias, alpha_bias, theta_mod_bias,
+                           theta_bias, theta_sign, cfg, u_stride_b, u_stride_h, u_stride_t, batch, heads, groups, T, P, N,
+                           io_dtype};
+  return sl::scanprep_fwd(a, sl::ScanPrepOut{U, M, K, Bo, Co}, reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int sl_scanprep_conv_bwd(
@@ -957,64 +1068,11 @@ extern "C" int sl_scanprep_conv_bwd(
     float* d_conv_bias, void* d_conv_state, void* d_params, void* d_bc, float* d_dt_bias,
     float* d_alpha_bias, float* d_theta_mod_bias, float* d_theta_bias, int batch, int heads,
     int groups, int T, int P, int N, int io_dtype, void* stream) {
-  using namespace sl;
-  if (int e = check_common(batch, heads, groups, T, P, N, io_dtype, conv_weight ? d_conv : 1)) return e;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (dU && (!d_value || !value || (conv_weight && !d_conv_weight))) return SL_ERR_NULL_POINTER;
-  if (dBo && (!dCo || !bc || !d_bc || !cfg)) return SL_ERR_NULL_POINTER;
-  if (dM) {
-    if (!dK || !params || !d_params || !cfg || !dt_bias || !alpha_bias || !theta_mod_bias ||
-        !theta_bias || !theta_sign)
-      return SL_ERR_NULL_POINTER;
-    if (!aligned(dM, 8) || !aligned(dK, 16)) return SL_ERR_BAD_ALIGNMENT;
-  }
-  PartFork fork(st, (dU != nullptr) + (dBo != nullptr) + (dM != nullptr), (long long)batch * T);
-  if (dU) {
-    ValueBwdParams q{};
-    ValueParams& p = q.f;
-    p.x = value; p.w = conv_weight; p.bias = conv_bias; p.state_in = conv_state_in;
-    p.xs = value_row_stride; p.usb = u_stride_b; p.ush = u_stride_h; p.ust = u_stride_t;
-    p.batch = batch; p.T = T; p.C = heads * P; p.P = P; p.W = conv_weight ? d_conv : 1;
-    q.dU = dU; q.dx = d_value; q.dstate = d_conv_state; q.dw = d_conv_weight; q.dbias = d_conv_bias;
-    ValueParams pv = p;
-    pv.U = const_cast<void*>(dU);
-    if (value_vec_ok(pv, d_value, nullptr)) {
-      dim3 grid((p.C + 32 * CONV_V - 1) / (32 * CONV_V), (T + CONV_SUB * CONV_TT - 1) / (CONV_SUB * CONV_TT), batch);
-      SL_DISPATCH_DTYPE(io_dtype, Tt, { value_bwd_vec_kernel<Tt><<<grid, 256, 0, fork.v>>>(q); });
-    } else {
-      dim3 grid((p.C + 255) / 256, (T + CONV_TT - 1) / CONV_TT, batch);
-      SL_DISPATCH_DTYPE(io_dtype, Tt, { value_bwd_kernel<Tt><<<grid, 256, 0, fork.v>>>(q); });
-    }
-    note_launches(1);
-  }
-  if (dBo) {
-    const long long rows = (long long)batch * T * groups;
-    const unsigned blocks = (unsigned)((rows + 7) / 8);
-    const dim3 vgrid((T + 7) / 8, (groups + BC_GCH - 1) / BC_GCH, batch);
-    SL_DISPATCH_DTYPE(io_dtype, Tt, {
-      if (bc_vec_ok(batch, groups, N, bc, dBo, dCo, d_bc))
-        bc_bwd_vec_kernel<Tt><<<vgrid, 256, 0, fork.b>>>(reinterpret_cast<const Tt*>(bc),
-                                                     reinterpret_cast<const Tt*>(dBo),
-                                                     reinterpret_cast<const Tt*>(dCo), reinterpret_cast<Tt*>(d_bc),
-                                                     T, groups, N, cfg->eps);
-      else
-        bc_bwd_kernel<Tt><<<blocks, 256, 0, fork.b>>>(reinterpret_cast<const Tt*>(bc), reinterpret_cast<const Tt*>(dBo),
-                                                  reinterpret_cast<const Tt*>(dCo), reinterpret_cast<Tt*>(d_bc),
-                                                  batch, T, groups, N, cfg->eps);
-    });
-    note_launches(1);
-  }
-  if (dM) {
-    CoeffParams p{};
-    p.params = params; p.dt_bias = dt_bias; p.alpha_bias = alpha_bias;
-    p.theta_mod_bias = theta_mod_bias; p.theta_bias = theta_bias; p.theta_sign = theta_sign;
-    p.cfg = *cfg; p.dM = dM; p.dK = dK; p.dparams = d_params; p.d_dt_bias = d_dt_bias;
-    p.d_alpha_bias = d_alpha_bias; p.d_theta_mod_bias = d_theta_mod_bias;
-    p.d_theta_bias = d_theta_bias; p.batch = batch; p.T = T; p.H = heads;
-    dim3 grid((T + 127) / 128, heads, batch);
-    SL_DISPATCH_DTYPE(io_dtype, Tt, { coeff_bwd_kernel<Tt><<<grid, 128, 0, fork.c>>>(p); });
-    note_launches(1);
-  }
-  fork.join();
-  return launch_status();
+  const int64_t params_row = 3 * (int64_t)heads, bc_row = 4 * (int64_t)groups * N;
+  const sl::ScanPrepArgs a{value, value_row_stride, conv_weight, conv_bias, conv_state_in, nullptr, d_conv, params, params_row,
+                           bc, bc_row, dt_bias, alpha_bias, theta_mod_bias, theta_bias, theta_sign, cfg, u_stride_b, u_stride_h,
+                           u_stride_t, batch, heads, groups, T, P, N, io_dtype};
+  const sl::ScanPrepGrads g{dU, dM, dK, dBo, dCo, d_value, (int64_t)heads * P, d_conv_weight, d_conv_bias, d_conv_state, d_params,
+                            params_row, d_bc, bc_row, d_dt_bias, d_alpha_bias, d_theta_mod_bias, d_theta_bias};
+  return sl::scanprep_bwd(a, g, reinterpret_cast<cudaStream_t>(stream));
 }
