@@ -370,6 +370,219 @@ Tensor ffn_token(const Tensor& x, const Tensor& norm_w, float eps, const Tensor&
   const Tensor hidden = linear_rows(call, x, Norm{norm_w, eps}, w1, b1, kind == 1 ? sl::LINEAR_SWIGLU : sl::LINEAR_GELU, {}, {});
   return linear_rows(call, hidden, Norm{}, w2, b2, sl::LINEAR_NONE, x, {});
 }
+// ---- the whole mixer over a sequence ------------------------------------------------------------------------------------
+// in_proj writes one buffer of rows [gate C | value C | params 3H | bc 4GN]; the kernels read their columns through the row
+// stride, and the backward writes the four gradients into a buffer of the same layout, so each direction of in_proj is one
+// GEMM and nothing is gathered in between.  Where 3H is not a multiple of 8 the bc columns start at the next one (the vector
+// kernels want 16-byte rows) and in_proj is two GEMMs.
+struct MixerShape {
+  int64_t batch, T, heads, groups, P, N, chunk, path;
+  int64_t C() const { return heads * P; }
+  int64_t rows() const { return batch * T; }
+  int64_t front() const { return 2 * C() + 3 * heads; }                // columns before bc in the weight
+  int64_t bc0() const { return (front() + 7) / 8 * 8; }               // ... and in the buffer
+  int64_t bcn() const { return 4 * groups * N; }
+  int64_t pitch() const { return (bc0() + bcn() + 7) / 8 * 8; }
+  bool whole() const { return bc0() == front(); }
+};
+struct MixerWeights {
+  Tensor in_w, dw_w, dw_b, d_skip, norm_w, out_w;
+  std::array<Tensor, 5> bias;
+  sl_scanprep_config cfg;
+  float eps;
+};
+Tensor as_typed(const Tensor& t, at::ScalarType type) { return t.to(type).contiguous(); }
+uint8_t* column(const Tensor& rows, int64_t c) { return static_cast<uint8_t*>(rows.data_ptr()) + c * rows.element_size(); }
+
+sl::ScanPrepArgs scanprep_args(const MixerShape& s, const MixerWeights& w, const Tensor& proj, const void* conv_in, void* conv_out) {
+  const ULayout lay = u_layout(true, s.heads, s.T, s.P);
+  return sl::ScanPrepArgs{column(proj, s.C()), s.pitch(), ptr(w.dw_w), ptr(w.dw_b), conv_in, conv_out, (int)w.dw_w.size(1),
+                          column(proj, 2 * s.C()), s.pitch(), column(proj, s.bc0()), s.pitch(), fptr(w.bias[0]), fptr(w.bias[1]),
+                          fptr(w.bias[2]), fptr(w.bias[3]), fptr(w.bias[4]), &w.cfg, lay.b, lay.h, lay.t, (int)s.batch,
+                          (int)s.heads, (int)s.groups, (int)s.T, (int)s.P, (int)s.N, code_of(proj.scalar_type())};
+}
+
+struct MixerRun {
+  Tensor proj, U, M, K, B, C, Y, normed, out;
+  OptT states, final_state, conv;
+};
+MixerRun mixer_run(const MixerShape& s, const MixerWeights& w, const Tensor& x, const OptT& conv_in, const OptT& z0, const OptT& Bp,
+                   const OptT& Up, bool save_states, bool want_state) {
+  Call call(x, w.in_w, w.dw_w, w.dw_b, w.d_skip, w.norm_w, w.out_w, conv_in, z0, Bp, Up);
+  for (const auto& t : w.bias) call.need(t);
+  const auto type = x.scalar_type();
+  const auto st = static_cast<cudaStream_t>(call.stream());
+  MixerRun r;
+  r.proj = call.empty({s.rows(), s.pitch()}, type);
+  if (s.whole()) {
+    Tensor all = r.proj.narrow(1, 0, w.in_w.size(0));
+    at::mm_out(all, x, w.in_w.t());
+  } else {
+    Tensor front = r.proj.narrow(1, 0, s.front()), bc = r.proj.narrow(1, s.bc0(), s.bcn());
+    at::mm_out(front, x, w.in_w.narrow(0, 0, s.front()).t());
+    at::mm_out(bc, x, w.in_w.narrow(0, s.front(), s.bcn()).t());
+  }
+  r.U = call.empty({s.batch, s.heads, s.T, s.P}, type);
+  r.M = call.empty({s.batch, s.heads, s.T, 2}, at::kFloat);
+  r.K = call.empty({s.batch, s.heads, s.T, 2, 2}, at::kFloat);
+  r.B = call.empty({s.batch, s.groups, s.T, 2 * s.N}, type);
+  r.C = at::empty_like(r.B);
+  if (want_state) r.conv = call.empty({s.batch, s.C(), w.dw_w.size(1) - 1}, type);
+  check(sl::scanprep_fwd(scanprep_args(s, w, r.proj, ptr(conv_in), mptr(r.conv)),
+                         sl::ScanPrepOut{mptr(r.U), mfptr(r.M), mfptr(r.K), mptr(r.B), mptr(r.C)}, st),
+        "sl_scanprep_conv_fwd");
+  std::tie(r.Y, r.final_state, r.states) =
+      scan_fwd(r.U, r.M, r.K, r.B, r.C, z0, Bp, Up, s.chunk, code_of(type), want_state, s.path, save_states);
+  r.normed = call.empty({s.rows(), s.C()}, type);
+  check(sl_mixer_tail_fwd(ptr(r.Y), ptr(r.proj), s.pitch(), ptr(r.U), fptr(w.d_skip), ptr(w.norm_w), w.eps, mptr(r.normed), s.batch,
+                          s.heads, s.T, s.P, code_of(type), st),
+        "sl_mixer_tail_fwd");
+  r.out = at::mm(r.normed, w.out_w.t());
+  return r;
+}
+
+MixerWeights mixer_weights(at::ScalarType type, const Tensor& in_w, const Tensor& dw_w, const Tensor& dw_b,
+                           const std::array<Tensor, 5>& bias, const Config& cfg, const Tensor& d_skip, const Tensor& norm_w,
+                           double eps, const Tensor& out_w) {
+  MixerWeights w{in_w, as_typed(dw_w, type), as_typed(dw_b, type), as_typed(d_skip, at::kFloat), as_typed(norm_w, type), out_w,
+                 {}, config_of(cfg), (float)eps};
+  for (size_t i = 0; i < 5; ++i) w.bias[i] = as_typed(bias[i], at::kFloat);
+  return w;
+}
+
+using Variables = torch::autograd::variable_list;
+struct MixerFn : torch::autograd::Function<MixerFn> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& in_w, const Tensor& dw_w,
+                        const Tensor& dw_b, const Tensor& dt_bias, const Tensor& alpha_bias, const Tensor& theta_mod_bias,
+                        const Tensor& theta_bias, const Tensor& d_skip, const Tensor& norm_w, const Tensor& out_w,
+                        const Tensor& theta_sign, std::vector<double> reals, std::vector<int64_t> dims) {
+    const MixerShape s = shape_of(dims);
+    const Tensor flat = x.reshape({s.rows(), x.size(-1)});
+    const MixerWeights w = weights_of(flat.scalar_type(), in_w, dw_w, dw_b, {dt_bias, alpha_bias, theta_mod_bias, theta_bias, theta_sign},
+                                      reals, d_skip, norm_w, out_w);
+    const MixerRun r = mixer_run(s, w, flat, {}, {}, {}, {}, true, false);
+    ctx->save_for_backward({flat, in_w, w.dw_w, w.dw_b, w.bias[0], w.bias[1], w.bias[2], w.bias[3], w.d_skip, w.norm_w, out_w,
+                            w.bias[4], r.proj, r.U, r.M, r.K, r.B, r.C, r.Y, r.normed, r.states ? *r.states : Tensor(),
+                            r.states ? *r.final_state : Tensor()});
+    for (const Tensor& t : {dw_w, dw_b, dt_bias, alpha_bias, theta_mod_bias, theta_bias, d_skip, norm_w})
+      dims.push_back((int64_t)t.scalar_type());
+    auto shape = x.sizes().vec();
+    ctx->saved_data["reals"] = reals;
+    ctx->saved_data["dims"] = dims;
+    ctx->saved_data["x"] = shape;
+    shape.back() = out_w.size(0);
+    return r.out.view(shape);
+  }
+
+  static Variables backward(torch::autograd::AutogradContext* ctx, Variables grads) {
+    const auto v = ctx->get_saved_variables();
+    const auto reals = ctx->saved_data["reals"].toDoubleVector();
+    const auto dims = ctx->saved_data["dims"].toIntVector();
+    const MixerShape s = shape_of(dims);
+    const Tensor &x = v[0], &in_w = v[1], &out_w = v[10], &proj = v[12], &U = v[13], &Y = v[18], &normed = v[19];
+    const MixerWeights w = weights_of(x.scalar_type(), in_w, v[2], v[3], {v[4], v[5], v[6], v[7], v[11]}, reals, v[8], v[9], out_w);
+    OptT states, final_state;
+    if (v[20].defined()) { states = v[20]; final_state = v[21]; }
+    Call call(x, grads[0]);
+    const auto type = x.scalar_type();
+    const auto st = static_cast<cudaStream_t>(call.stream());
+    Variables g(14);
+    const Tensor dout = grads[0].reshape({s.rows(), grads[0].size(-1)});
+    if (ctx->needs_input_grad(10)) g[10] = at::mm(dout.t(), normed);
+    Tensor dn = at::mm(dout, out_w);
+    // float32 accumulators of the small parameters: slices of one zeroed buffer, 16-byte aligned in every type
+    const int64_t W = w.dw_w.size(1), C = s.C(), H = s.heads;
+    const std::array<int64_t, 8> len{C * W, C, C, H, H, H, H, H};
+    std::array<int64_t, 9> at_{};
+    for (int i = 0; i < 8; ++i) at_[i + 1] = at_[i] + (len[i] + 7) / 8 * 8;
+    const Tensor acc = call.zeros({at_[8]}, at::kFloat);
+    auto slice = [&](int i) { return acc.narrow(0, at_[i], len[i]); };
+    float* const a = mfptr(acc);
+    Tensor d_proj = at::empty_like(proj), dY = at::empty_like(Y);
+    check(sl::mixer_tail_bwd(ptr(Y), ptr(proj), s.pitch(), ptr(U), fptr(w.d_skip), ptr(w.norm_w), w.eps, ptr(dn), mptr(dY),
+                             mptr(d_proj), s.pitch(), nullptr, a + at_[3], a + at_[2], s.batch, H, s.T, s.P, code_of(type), st),
+          "sl_mixer_tail_bwd");
+    dn.reset();
+    {
+      const auto [dU, dM, dK, dB, dC, dz, dbp, dup] =
+          scan_bwd(U, v[14], v[15], v[16], v[17], {}, {}, {}, states, final_state, dY, {}, s.chunk, s.path);
+      sl::ScanPrepGrads sg{ptr(dU), fptr(dM), fptr(dK), ptr(dB), ptr(dC), column(d_proj, C), s.pitch(), a + at_[0], a + at_[1],
+                           nullptr, column(d_proj, 2 * C), s.pitch(), column(d_proj, s.bc0()), s.pitch(), a + at_[4], a + at_[5],
+                           a + at_[6], a + at_[7]};
+      sg.dY = ptr(dY);   // the skip connection's share of dU is added where dU is read
+      sg.skip = fptr(w.d_skip);
+      check(sl::scanprep_bwd(scanprep_args(s, w, proj, nullptr, nullptr), sg, st), "sl_scanprep_conv_bwd");
+    }
+    auto type_at = [&](int i) { return static_cast<at::ScalarType>(dims[8 + i]); };   // dw_w dw_b dt alpha theta_mod theta d_skip norm
+    const auto t0 = type_at(0);
+    if (t0 == type_at(1) && t0 == type_at(7)) {   // one conversion for the three
+      const Tensor low = acc.narrow(0, 0, at_[3]).to(t0);
+      g[2] = low.narrow(0, at_[0], len[0]).view({C, W});
+      g[3] = low.narrow(0, at_[1], len[1]);
+      g[9] = low.narrow(0, at_[2], len[2]);
+    } else {
+      g[2] = slice(0).view({C, W}).to(t0);
+      g[3] = slice(1).to(type_at(1));
+      g[9] = slice(2).to(type_at(7));
+    }
+    g[8] = slice(3).to(type_at(6));
+    for (int i = 0; i < 4; ++i) g[4 + i] = slice(4 + i).to(type_at(2 + i));
+    const Tensor front = d_proj.narrow(1, 0, s.whole() ? in_w.size(0) : s.front());
+    const Tensor bc = s.whole() ? Tensor() : d_proj.narrow(1, s.bc0(), s.bcn());
+    if (ctx->needs_input_grad(0)) {
+      Tensor dx;
+      if (s.whole()) dx = at::mm(front, in_w);
+      else dx = at::mm(front, in_w.narrow(0, 0, s.front())).addmm_(bc, in_w.narrow(0, s.front(), s.bcn()));
+      g[0] = dx.view(ctx->saved_data["x"].toIntVector());
+    }
+    if (ctx->needs_input_grad(1)) {
+      if (s.whole()) g[1] = at::mm(front.t(), x);
+      else {
+        g[1] = at::empty_like(in_w);
+        Tensor top = g[1].narrow(0, 0, s.front()), bottom = g[1].narrow(0, s.front(), s.bcn());
+        at::mm_out(top, front.t(), x);
+        at::mm_out(bottom, bc.t(), x);
+      }
+    }
+    return g;
+  }
+
+  static MixerShape shape_of(const std::vector<int64_t>& d) { return MixerShape{d[0], d[1], d[2], d[3], d[4], d[5], d[6], d[7]}; }
+  static MixerWeights weights_of(at::ScalarType type, const Tensor& in_w, const Tensor& dw_w, const Tensor& dw_b,
+                                 const std::array<Tensor, 5>& bias, const std::vector<double>& reals, const Tensor& d_skip,
+                                 const Tensor& norm_w, const Tensor& out_w) {
+    Config c;
+    for (size_t i = 0; i < c.size(); ++i) c[i] = (float)reals[i];
+    return mixer_weights(type, in_w, dw_w, dw_b, bias, c, d_skip, norm_w, reals[c.size()], out_w);
+  }
+};
+
+// parameters: in_w dw_w dw_b dt_bias alpha_bias theta_mod_bias theta_bias d_skip norm_w out_w theta_sign; reals: the ten
+// configuration values and the norm's epsilon; dims: heads groups P N chunk path
+std::vector<int64_t> mixer_dims(const Tensor& x, const std::vector<int64_t>& dims) {
+  std::vector<int64_t> d{x.size(0), x.size(1)};
+  d.insert(d.end(), dims.begin(), dims.end());
+  return d;
+}
+Tensor mixer_train(const Tensor& x, const std::vector<Tensor>& p, const std::vector<double>& reals, const std::vector<int64_t>& dims) {
+  return MixerFn::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], p[9], p[10], reals, mixer_dims(x, dims));
+}
+// without gradients: out, and on request the streaming state (conv, scan state, last B, last U)
+std::tuple<Tensor, OptT, OptT, OptT, OptT> mixer_infer(const Tensor& x, const std::vector<Tensor>& p, const std::vector<double>& reals,
+                                                       const std::vector<int64_t>& dims_in, const OptT& conv, const OptT& z0,
+                                                       const OptT& Bp, const OptT& Up, bool want_state) {
+  const auto dims = mixer_dims(x, dims_in);
+  const MixerShape s = MixerFn::shape_of(dims);
+  const auto type = x.scalar_type();
+  const MixerWeights w = MixerFn::weights_of(type, p[0], p[1], p[2], {p[3], p[4], p[5], p[6], p[10]}, reals, p[7], p[8], p[9]);
+  auto cast = [](const OptT& t, at::ScalarType ty) { return t ? OptT(as_typed(*t, ty)) : OptT(); };
+  MixerRun r = mixer_run(s, w, x.reshape({s.rows(), x.size(-1)}), cast(conv, type), cast(z0, at::kFloat), cast(Bp, type),
+                         cast(Up, type), false, want_state);
+  Tensor out = r.out.view({s.batch, s.T, r.out.size(1)});
+  if (!want_state) return {out, {}, {}, {}, {}};
+  return {out, r.conv, r.final_state->to(type), r.B.select(2, s.T - 1).contiguous(), r.U.select(2, s.T - 1).contiguous()};
+}
+
 // ---- language-model training step --------------------------------------------------------------------------------------
 // per-row losses and log-sum-exps of logits (rows, V)
 std::tuple<Tensor, Tensor> ce_fwd(const Tensor& logits, const Tensor& target) {
@@ -478,6 +691,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embed_bwd", &embed_bwd);
   m.def("grad_norm_scale", &grad_norm_scale);
   m.def("adamw_step", &adamw_step);
+  m.def("mixer_train", &mixer_train);
+  m.def("mixer_infer", &mixer_infer);
   m.def("mixer_token", &mixer_token);
   m.def("ffn_token", &ffn_token);
 }

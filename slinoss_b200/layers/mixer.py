@@ -147,6 +147,10 @@ class SLinOSSMixer(nn.Module):
             empty = x.new_empty((batch, 0, self.d_model))
             nxt = SLinOSSMixerState() if state is None else state
             return (empty, nxt) if return_state else empty
+        if x.is_cuda and self._native_forward_ready(x, state):
+            parameters = self._native_parameters()
+            if not _C.grad_needed(x, *parameters) or (state is None and not return_state):
+                return self._forward_native(x, parameters, state, return_state)
         gate, value_proj, params, bc_flat = split_mixer_projection(
             x, self.in_proj.weight, d_inner=self.d_inner, param_proj_dim=self.param_proj_dim)
         bc = bc_flat.view(batch, T, self.bc_groups, self.scanprep.bc_param_rows, self.d_state)
@@ -161,6 +165,42 @@ class SLinOSSMixer(nn.Module):
         if scan_state is None:
             return out
         return out, SLinOSSMixerState(conv=conv_state, scan=scan_state)
+
+    def _native_forward_ready(self, x: torch.Tensor, state: SLinOSSMixerState | None) -> bool:
+        """The whole mixer in the host module: the package's own backends on every stage, bias-free projections of x's
+        type, and either no state or a complete one."""
+        w_in, out, backend, dt = self.in_proj.weight, self.out_proj, self.scan_backend, x.dtype
+        if not (dt in (torch.bfloat16, torch.float16, torch.float32) and w_in.dtype == dt and w_in.device == x.device
+                and x.numel() > 0 and type(out) is nn.Linear and out.bias is None and out.weight.dtype == dt
+                and out.weight.shape[1] == self.d_inner and self.out_norm.weight is not None
+                and type(backend) is B200ScanBackend and backend.compute_dtype in (None, torch.float32)
+                and self._fused_frontend() and w_in.is_contiguous() and not torch.is_autocast_enabled()):
+            return False
+        if state is None:
+            return True
+        batch, scan, D = x.shape[0], state.scan, 2 * self.d_state
+        want = ((state.conv, (batch, self.d_inner, self.d_conv - 1)), (scan.state, (batch, self.n_heads, self.d_head, D)),
+                (scan.b_prev, (batch, self.bc_groups, D)), (scan.u_prev, (batch, self.n_heads, self.d_head)))
+        return all(t is not None and t.shape == shape and t.device == x.device and t.is_floating_point()
+                   and t.is_contiguous() and not t.requires_grad for t, shape in want)
+
+    def _native_parameters(self) -> list:
+        sp = self.scanprep
+        return [self.in_proj.weight, self.dw_weight, self.dw_bias, sp.dt_bias, sp.alpha_bias, sp.theta_mod_bias, sp.theta_bias,
+                self.d_skip, self.out_norm.weight, self.out_proj.weight, sp.theta_sign]
+
+    @_C.opaque
+    def _forward_native(self, x: torch.Tensor, parameters: list, state: SLinOSSMixerState | None, return_state: bool):
+        host, sp, backend = _C.host(), self.scanprep, self.scan_backend
+        reals = [*(getattr(sp, n) for n in _C.CONFIG_FIELDS), _norm_eps(self.out_norm)]
+        dims = [self.n_heads, self.bc_groups, self.d_head, self.d_state, int(self.chunk_size), _C._PATHS[backend.path]]
+        if _C.grad_needed(x, *parameters):
+            return host.mixer_train(x, parameters, reals, dims)
+        carried = (None,) * 4 if state is None else (state.conv, state.scan.state, state.scan.b_prev, state.scan.u_prev)
+        out, conv, final, b_last, u_last = host.mixer_infer(x, parameters, reals, dims, *carried, return_state)
+        if not return_state:
+            return out
+        return out, SLinOSSMixerState(conv=conv, scan=ScanState(state=final, b_prev=b_last, u_prev=u_last))
 
     def _forward_sequence_parallel(self, x: torch.Tensor, group):
         from ..ops.v2x2ssd.sequence_parallel import previous_rank_value, v2x2ssd_sequence_parallel
