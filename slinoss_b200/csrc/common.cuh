@@ -100,9 +100,59 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// (__fdividef: 2 ulp, and 0 for a denominator beyond 2^126, which is the right limit here)
-__device__ __forceinline__ float silu_f(float x) { return __fdividef(x, 1.f + __expf(-x)); }
-__device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+// ---- packed float32 pairs (two independent lanes per instruction) ---------------------------
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 mk2(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ f2 dup2(float v) { return mk2(v, v); }
+__device__ __forceinline__ float2 un2(f2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// 2^x, log2(x) and 1/x on the special-function unit
+__device__ __forceinline__ float ex2f(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float lg2f(float x) {
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rcpf(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// (1 ulp for the reciprocal, and 0 for a denominator beyond 2^126, which is the right limit here)
+__device__ __forceinline__ float sigmoid_f(float x) { return rcpf(1.f + ex2f(-1.4426950408889634f * x)); }
+__device__ __forceinline__ float silu_f(float x) { return x * sigmoid_f(x); }
+__device__ __forceinline__ f2 sigmoid2(f2 x) {
+  const float2 e = un2(mul2(x, dup2(-1.4426950408889634f)));
+  const float2 d = un2(add2(mk2(ex2f(e.x), ex2f(e.y)), dup2(1.f)));
+  return mk2(rcpf(d.x), rcpf(d.y));
+}
 
 // 16-bit rows take the one-instruction tanh (relative error 2^-11, below the rounding of the output);
 // float32 rows the precise one.

@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(256) value_bwd_kernel(ValueBwdParams q) {
 // pointers; anything else takes the one-channel-per-thread kernels above.
 constexpr int CONV_V = 4;
 constexpr int CONV_SUB = 8;   // token sub-tiles per CTA
+constexpr int CONV_SB = 4;    // tokens of a batch
 
 template <typename T>
 __device__ __forceinline__ void load_xv(const ValueParams& p, const T* x, const T* st, int b, int t, int c,
@@ -201,294 +202,246 @@ __device__ __forceinline__ void load_xv(const ValueParams& p, const T* x, const 
     v[k] = (st && j >= 0) ? to_f32(st[((size_t)b * p.C + c + k) * (p.W - 1) + j]) : 0.f;
 }
 
-template <typename T, int V> __device__ __forceinline__ void loadv(const T* p, float (&v)[V]) {
-  if constexpr (V == 4) load4<T>(p, v); else load16<T>(p, v);
+// 4 channels as two packed pairs, and the memory piece they come in
+template <typename T> using Raw4 = typename std::conditional<sizeof(T) == 4, uint4, uint2>::type;
+template <typename T> __device__ __forceinline__ void unpack4(const Raw4<T>& r, f2 (&v)[2]) {
+  if constexpr (sizeof(T) == 4) {
+    v[0] = mk2(__uint_as_float(r.x), __uint_as_float(r.y));
+    v[1] = mk2(__uint_as_float(r.z), __uint_as_float(r.w));
+  } else {
+    const float2 a = unpack_pair<T>(r.x), b = unpack_pair<T>(r.y);
+    v[0] = mk2(a.x, a.y); v[1] = mk2(b.x, b.y);
+  }
 }
-template <typename T, int V> __device__ __forceinline__ void storev(T* p, const float (&v)[V]) {
-  if constexpr (V == 4) store4<T>(p, v); else store16<T>(p, v);
+template <typename T> __device__ __forceinline__ void store4(T* p, const f2 (&v)[2]) {
+  const float2 a = un2(v[0]), b = un2(v[1]);
+  const float q[4] = {a.x, a.y, b.x, b.y};
+  store4<T>(p, q);
 }
 
-// Forward (instantiated with V = CONV_V channels per thread).
-template <typename T, int V>
-__global__ void __launch_bounds__(256, 3) value_fwd_vec_kernel(ValueParams p) {
-  const int c = (blockIdx.x * 32 + (threadIdx.x & 31)) * V;
-  const int t0 = (blockIdx.y * CONV_SUB + (threadIdx.x >> 5)) * CONV_TT, b = blockIdx.z;
+// The taps, right-aligned in a window of 4, the bias, and the 3 inputs before token t0 (those that no tap reads as zeros) of
+// the channels c .. c + 3.
+template <typename T>
+__device__ __forceinline__ void conv_setup(const ValueParams& p, int b, int t0, int c, f2 (&w2)[4][2], f2 (&bias2)[2],
+                                           f2 (&win)[3][2]) {
+  const T *w = reinterpret_cast<const T*>(p.w), *x = reinterpret_cast<const T*>(p.x), *st = reinterpret_cast<const T*>(p.state_in);
+  float wj[4][CONV_V], bias[CONV_V] = {0.f, 0.f, 0.f, 0.f}, h[CONV_V];
+  if (p.W == 4 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
+    // the taps of the 4 channels are 16 contiguous values; bias is one 4-wide piece
+#pragma unroll
+    for (int k = 0; k < CONV_V; ++k) {
+      float q[4];
+      load4<T>(w + (size_t)(c + k) * 4, q);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) wj[j][k] = q[j];
+    }
+    if (p.bias) load4<T>(reinterpret_cast<const T*>(p.bias) + c, bias);
+  } else {
+#pragma unroll
+    for (int k = 0; k < CONV_V; ++k) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) wj[j][k] = (j >= 4 - p.W) ? to_f32(w[(size_t)(c + k) * p.W + (j - (4 - p.W))]) : 0.f;
+      if (p.bias) bias[k] = to_f32(reinterpret_cast<const T*>(p.bias)[c + k]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w2[j][i] = mk2(wj[j][2 * i], wj[j][2 * i + 1]);
+    bias2[i] = mk2(bias[2 * i], bias[2 * i + 1]);
+  }
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    win[r][0] = win[r][1] = 0;
+    if (3 - r > p.W - 1) continue;
+    load_xv<T>(p, x, st, b, t0 - 3 + r, c, h);
+    win[r][0] = mk2(h[0], h[1]); win[r][1] = mk2(h[2], h[3]);
+  }
+}
+
+// Forward.  Each batch of 4 tokens is requested one batch ahead of its use: the loads of a batch alone (3 KB per warp and
+// latency, as the walk alternated between waiting and computing) left two thirds of the bandwidth idle.
+template <typename T>
+__global__ void __launch_bounds__(256, 3) value_fwd_vec_kernel(ValueParams p, int tile) {
+  const int c = (blockIdx.x * 32 + (threadIdx.x & 31)) * CONV_V;
+  const int t0 = (blockIdx.y * CONV_SUB + (threadIdx.x >> 5)) * tile, b = blockIdx.z;
   if (c >= p.C || t0 >= p.T) return;
-  const T* x = reinterpret_cast<const T*>(p.x);
-  const T* st = reinterpret_cast<const T*>(p.state_in);
-  T* U = reinterpret_cast<T*>(p.U);
-  const int h = c / p.P, pp = c - h * p.P;
-  T* Ub = U + (size_t)b * p.usb + (size_t)h * p.ush + pp;
-  const T* xb = x + (size_t)b * p.T * p.xs + c;
-  const int t1 = min(t0 + CONV_TT, p.T);
+  const int h = c / p.P, pp = c - h * p.P, t1 = min(t0 + tile, p.T);
+  T* Ub = reinterpret_cast<T*>(p.U) + (size_t)b * p.usb + (size_t)h * p.ush + pp;
+  const T* xb = reinterpret_cast<const T*>(p.x) + (size_t)b * p.T * p.xs + c;
+  Raw4<T> nx[CONV_SB];
+  auto fetch = [&](int s) {
+#pragma unroll
+    for (int i = 0; i < CONV_SB; ++i)
+      if (s + i < p.T) nx[i] = *reinterpret_cast<const Raw4<T>*>(xb + (size_t)(s + i) * p.xs);
+  };
+  fetch(t0);
   if (!p.w) {
-    for (int t = t0; t < t1; ++t) {
-      float v[V];
-      loadv<T, V>(xb + (size_t)t * p.xs, v);
-      storev<T, V>(Ub + (size_t)t * p.ust, v);
+    for (int s = t0; s < t1; s += CONV_SB) {
+      Raw4<T> cx[CONV_SB];
+#pragma unroll
+      for (int i = 0; i < CONV_SB; ++i) cx[i] = nx[i];
+      if (s + CONV_SB < t1) fetch(s + CONV_SB);
+#pragma unroll
+      for (int i = 0; i < CONV_SB; ++i)
+        if (s + i < t1) *reinterpret_cast<Raw4<T>*>(Ub + (size_t)(s + i) * p.ust) = cx[i];
     }
     return;
   }
-  const T* w = reinterpret_cast<const T*>(p.w);
-  float wj[4][V], win[4][V], bias[V];
-  auto x_at = [&](int t, int k) -> float {   // scalar access for the halo (t may be negative)
-    if (t >= 0) return to_f32(xb[(size_t)t * p.xs + k]);
-    const int j = p.W - 1 + t;
-    return (st && j >= 0) ? to_f32(st[((size_t)b * p.C + c + k) * (p.W - 1) + j]) : 0.f;
-  };
-  if (p.W == 4 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 &&
-      (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
-    // taps of V channels are 4 V contiguous values; bias and the three halo rows are one piece each
-    float wf[4 * V];
-#pragma unroll
-    for (int i = 0; i < 4 * V / Vec16<T>::N; ++i) {
-      float q[Vec16<T>::N];
-      load16<T>(w + (size_t)c * 4 + i * Vec16<T>::N, q);
-#pragma unroll
-      for (int e = 0; e < Vec16<T>::N; ++e) wf[i * Vec16<T>::N + e] = q[e];
-    }
-#pragma unroll
-    for (int k = 0; k < V; ++k) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) wj[j][k] = wf[4 * k + j];
-      bias[k] = 0.f; win[0][k] = 0.f;
-    }
-    if (p.bias) loadv<T, V>(reinterpret_cast<const T*>(p.bias) + c, bias);
-#pragma unroll
-    for (int q = 1; q < 4; ++q) {
-      const int t = t0 - 4 + q;
-      if (t >= 0) loadv<T, V>(xb + (size_t)t * p.xs, win[q]);
-      else {
-#pragma unroll
-        for (int k = 0; k < V; ++k) win[q][k] = x_at(t, k);
-      }
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < V; ++k) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)   // right-aligned taps; static indices keep wj in registers
-        wj[j][k] = (j >= 4 - p.W) ? to_f32(w[(size_t)(c + k) * p.W + (j - (4 - p.W))]) : 0.f;
-      bias[k] = p.bias ? to_f32(reinterpret_cast<const T*>(p.bias)[c + k]) : 0.f;
-      win[0][k] = 0.f;
-#pragma unroll
-      for (int q = 1; q < 4; ++q) win[q][k] = (4 - q <= p.W - 1) ? x_at(t0 - 4 + q, k) : 0.f;
-    }
-  }
-  auto step = [&](int t, const float (&xin)[V]) {
-    float o[V];
-#pragma unroll
-    for (int k = 0; k < V; ++k) {
-      win[0][k] = win[1][k]; win[1][k] = win[2][k]; win[2][k] = win[3][k]; win[3][k] = xin[k];
-      const float a = bias[k] + wj[0][k] * win[0][k] + wj[1][k] * win[1][k] + wj[2][k] * win[2][k] +
-                      wj[3][k] * win[3][k];
-      o[k] = silu_f(a);
-    }
-    storev<T, V>(Ub + (size_t)t * p.ust, o);
-  };
-  if (t1 - t0 == CONV_TT) {
-    // full tile: batches of 8 tokens whose loads are all issued (unconditionally) before the first
-    // store of the batch - the compiler cannot move loads of x over stores to U by itself
-    constexpr int TB = 8;
-    using Raw = typename std::conditional<V * sizeof(T) == 16, uint4, uint2>::type;
+  f2 w[4][2], bias[2], win[3][2];
+  conv_setup<T>(p, b, t0, c, w, bias, win);
 #pragma unroll 1
-    for (int tb = t0; tb < t1; tb += TB) {
-      Raw raw[TB];
+  for (int s = t0; s < t1; s += CONV_SB) {
+    Raw4<T> cx[CONV_SB];
 #pragma unroll
-      for (int i = 0; i < TB; ++i) raw[i] = *reinterpret_cast<const Raw*>(xb + (size_t)(tb + i) * p.xs);
+    for (int i = 0; i < CONV_SB; ++i) cx[i] = nx[i];
+    if (s + CONV_SB < t1) fetch(s + CONV_SB);
 #pragma unroll
-      for (int i = 0; i < TB; ++i) {
-        float xin[V];
-        const T* e = reinterpret_cast<const T*>(&raw[i]);
+    for (int i = 0; i < CONV_SB; ++i) {
+      f2 x[2], o[2];
+      unpack4<T>(cx[i], x);
 #pragma unroll
-        for (int k = 0; k < V; ++k) xin[k] = to_f32(e[k]);
-        step(tb + i, xin);
+      for (int k = 0; k < 2; ++k) {
+        const f2 a = fma2(w[3][k], x[k], fma2(w[2][k], win[2][k], fma2(w[1][k], win[1][k], fma2(w[0][k], win[0][k], bias[k]))));
+        o[k] = mul2(a, sigmoid2(a));
+        win[0][k] = win[1][k]; win[1][k] = win[2][k]; win[2][k] = x[k];
       }
-    }
-  } else {
-    for (int t = t0; t < t1; ++t) {
-      float xin[V];
-      loadv<T, V>(xb + (size_t)t * p.xs, xin);
-      step(t, xin);
+      if (s + i < t1) store4<T>(Ub + (size_t)(s + i) * p.ust, o);
     }
   }
   if (p.state_out && t1 == p.T) {
     T* so = reinterpret_cast<T*>(p.state_out);
     for (int j = 0; j < p.W - 1; ++j) {
+      float v[CONV_V];
+      load_xv<T>(p, reinterpret_cast<const T*>(p.x), reinterpret_cast<const T*>(p.state_in), b, p.T - (p.W - 1) + j, c, v);
 #pragma unroll
-      for (int k = 0; k < V; ++k)
-        so[((size_t)b * p.C + c + k) * (p.W - 1) + j] = from_f32<T>(x_at(p.T - (p.W - 1) + j, k));
+      for (int k = 0; k < CONV_V; ++k) so[((size_t)b * p.C + c + k) * (p.W - 1) + j] = from_f32<T>(v[k]);
     }
   }
 }
 
+// Backward.  Bound by the instructions per channel and token (about 20 in packed pairs; 53 before) and by the latency of a
+// batch, which is requested one batch ahead.  A tile of n tokens walks n + 3 steps: the last three only complete dx.
+// (8, 2048) tokens of 2048 channels: 103 -> 71 us; (1, 1021), where the ragged last tile used to walk token by token: 42 -> 17
+// (forward 23 -> 10).
 template <typename T, bool SKIP>
-__global__ void __launch_bounds__(256, 2) value_bwd_vec_kernel(ValueBwdParams q) {
+__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 2 : 1) value_bwd_vec_kernel(ValueBwdParams q, int tile) {
   const ValueParams& p = q.f;
-  __shared__ float s_acc[CONV_SUB][5][32 * CONV_V];   // dw (4 taps) and dbias partials per sub-tile
+  constexpr int ROW = 32 * CONV_V + 8;              // 8 floats of padding: the sums below read 4 rows side by side
+  __shared__ float s_acc[CONV_SUB][5][ROW];         // dw (4 taps) and dbias partials per sub-tile
   const int lane = threadIdx.x & 31, sub = threadIdx.x >> 5;
   const int c = (blockIdx.x * 32 + lane) * CONV_V;
-  const int t0 = (blockIdx.y * CONV_SUB + sub) * CONV_TT, b = blockIdx.z;
-  const bool live = c < p.C && t0 < p.T;
-  float dwacc[4][CONV_V], dbacc[CONV_V];
+  const int t0 = (blockIdx.y * CONV_SUB + sub) * tile, b = blockIdx.z, t1 = min(t0 + tile, p.T);
+  f2 dw[4][2], db[2];
 #pragma unroll
-  for (int k = 0; k < CONV_V; ++k) {
-    dbacc[k] = 0.f;
+  for (int k = 0; k < 2; ++k) {
+    db[k] = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) dwacc[j][k] = 0.f;
+    for (int j = 0; j < 4; ++j) dw[j][k] = 0;
   }
-  if (live) {
-    const T* x = reinterpret_cast<const T*>(p.x);
-    const T* st = reinterpret_cast<const T*>(p.state_in);
-    const T* dU = reinterpret_cast<const T*>(q.dU);
-    T* dx = reinterpret_cast<T*>(q.dx);
+  if (c < p.C && t0 < p.T) {
     const int h = c / p.P, pp = c - h * p.P;
     const size_t ub = (size_t)b * p.usb + (size_t)h * p.ush + pp;
-    const T* dUb = dU + ub;
+    const T* xb = reinterpret_cast<const T*>(p.x) + (size_t)b * p.T * p.xs + c;
+    const T* dUb = reinterpret_cast<const T*>(q.dU) + ub;
     const T* dYb = SKIP ? reinterpret_cast<const T*>(q.dY) + ub : nullptr;
-    const float skip = SKIP ? q.skip[h] : 0.f;
-    auto load_gy = [&](int t, float (&v)[CONV_V]) {
-      load4<T>(dUb + (size_t)t * p.ust, v);
-      if constexpr (SKIP) {
-        float y[CONV_V];
-        load4<T>(dYb + (size_t)t * p.ust, y);
+    T* dxb = reinterpret_cast<T*>(q.dx) + (size_t)b * p.T * q.dxs + c;
+    const f2 skip = SKIP ? dup2(q.skip[h]) : 0;
+    Raw4<T> nx[CONV_SB], ng[CONV_SB], ny[SKIP ? CONV_SB : 1];
+    auto fetch = [&](int s) {      // tokens past the end count as zeros
 #pragma unroll
-        for (int k = 0; k < CONV_V; ++k) v[k] = fmaf(skip, y[k], v[k]);
+      for (int i = 0; i < CONV_SB; ++i) {
+        nx[i] = ng[i] = Raw4<T>{};
+        if constexpr (SKIP) ny[i] = Raw4<T>{};
+        if (s + i >= p.T) continue;
+        nx[i] = *reinterpret_cast<const Raw4<T>*>(xb + (size_t)(s + i) * p.xs);
+        ng[i] = *reinterpret_cast<const Raw4<T>*>(dUb + (size_t)(s + i) * p.ust);
+        if constexpr (SKIP) ny[i] = *reinterpret_cast<const Raw4<T>*>(dYb + (size_t)(s + i) * p.ust);
       }
     };
-    const int t1 = min(t0 + CONV_TT, p.T);
+    auto gradient = [&](const Raw4<T>& g, const Raw4<T>& y, f2 (&v)[2]) {
+      unpack4<T>(g, v);
+      if constexpr (SKIP) {
+        f2 yv[2];
+        unpack4<T>(y, yv);
+        v[0] = fma2(skip, yv[0], v[0]); v[1] = fma2(skip, yv[1], v[1]);
+      }
+    };
+    fetch(t0);
     if (!p.w) {
-      for (int t = t0; t < t1; ++t) {
-        float v[CONV_V];
-        load_gy(t, v);
-        store4<T>(dx + ((size_t)b * p.T + t) * q.dxs + c, v);
+      for (int s = t0; s < t1; s += CONV_SB) {
+        f2 v[CONV_SB][2];
+#pragma unroll
+        for (int i = 0; i < CONV_SB; ++i) gradient(ng[i], ny[SKIP ? i : 0], v[i]);
+        if (s + CONV_SB < t1) fetch(s + CONV_SB);
+#pragma unroll
+        for (int i = 0; i < CONV_SB; ++i)
+          if (s + i < t1) store4<T>(dxb + (size_t)(s + i) * q.dxs, v[i]);
       }
     } else {
-      const T* w = reinterpret_cast<const T*>(p.w);
       const int W = p.W;
-      float wj[4][CONV_V], win[4][CONV_V], da[4][CONV_V], bias[CONV_V];
-      const int s_begin = t0;   // the first tile also owns the gradient of the carried conv state
+      f2 w[4][2], bias[2], win[3][2], da[3][2];
+      conv_setup<T>(p, b, t0, c, w, bias, win);
 #pragma unroll
-      for (int k = 0; k < CONV_V; ++k) {
+      for (int k = 0; k < 2; ++k) da[0][k] = da[1][k] = da[2][k] = 0;
+      // da of token s; dx[s-3] is complete at step s.  ``mine``: the token's weight / bias contribution is counted here
+      auto step = [&](int s, auto mine, const f2 (&x)[2], const f2 (&gy)[2]) {
+        f2 g[2];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) da[j][k] = 0.f;
-        win[0][k] = 0.f; bias[k] = 0.f;
-      }
-      if (W == 4 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
-        // the taps of the 4 channels are 16 contiguous values; bias is one 4-wide piece
-#pragma unroll
-        for (int k = 0; k < CONV_V; ++k) {
-          float q4[4];
-          load4<T>(w + (size_t)(c + k) * 4, q4);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) wj[j][k] = q4[j];
-        }
-        if (p.bias) load4<T>(reinterpret_cast<const T*>(p.bias) + c, bias);
-      } else {
-#pragma unroll
-        for (int k = 0; k < CONV_V; ++k) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            wj[j][k] = (j >= 4 - W) ? to_f32(w[(size_t)(c + k) * W + (j - (4 - W))]) : 0.f;
-          bias[k] = p.bias ? to_f32(reinterpret_cast<const T*>(p.bias)[c + k]) : 0.f;
-        }
-      }
-#pragma unroll
-      for (int r = 1; r < 4; ++r) {
-        if (4 - r <= W - 1) load_xv<T>(p, x, st, b, s_begin - 4 + r, c, win[r]);
-        else {
-#pragma unroll
-          for (int k = 0; k < CONV_V; ++k) win[r][k] = 0.f;
-        }
-      }
-      // s runs over the tokens whose da is formed; dx[s-3] is complete at step s
-      const int s_end = min(t1 + 3, p.T + 3);
-      auto step = [&](int s, bool in, const float (&xin)[CONV_V], const float (&gy)[CONV_V]) {
-        float g[CONV_V];
-        const bool mine = s < t1;   // each token's weight / bias contribution is counted once
-#pragma unroll
-        for (int k = 0; k < CONV_V; ++k) {
-          win[0][k] = win[1][k]; win[1][k] = win[2][k]; win[2][k] = win[3][k];
-          da[0][k] = da[1][k]; da[1][k] = da[2][k]; da[2][k] = da[3][k];
-          float d = 0.f;
-          if (in) {
-            win[3][k] = xin[k];
-            const float a = bias[k] + wj[0][k] * win[0][k] + wj[1][k] * win[1][k] + wj[2][k] * win[2][k] +
-                            wj[3][k] * win[3][k];
-            d = gy[k] * dsilu_f(a);
-            if (mine) {
-              dwacc[0][k] += d * win[0][k]; dwacc[1][k] += d * win[1][k];
-              dwacc[2][k] += d * win[2][k]; dwacc[3][k] += d * win[3][k];
-              dbacc[k] += d;
-            }
-          } else {
-            win[3][k] = 0.f;
+        for (int k = 0; k < 2; ++k) {
+          const f2 a = fma2(w[3][k], x[k], fma2(w[2][k], win[2][k], fma2(w[1][k], win[1][k], fma2(w[0][k], win[0][k], bias[k]))));
+          const f2 sg = sigmoid2(a), one = dup2(1.f);
+          const f2 d = mul2(gy[k], mul2(sg, fma2(a, fma2(sg, dup2(-1.f), one), one)));
+          if constexpr (decltype(mine)::value) {
+            dw[0][k] = fma2(d, win[0][k], dw[0][k]); dw[1][k] = fma2(d, win[1][k], dw[1][k]);
+            dw[2][k] = fma2(d, win[2][k], dw[2][k]); dw[3][k] = fma2(d, x[k], dw[3][k]);
+            db[k] = add2(db[k], d);
           }
-          da[3][k] = d;
-          g[k] = wj[3][k] * da[0][k] + wj[2][k] * da[1][k] + wj[1][k] * da[2][k] + wj[0][k] * da[3][k];
+          g[k] = fma2(w[0][k], d, fma2(w[1][k], da[2][k], fma2(w[2][k], da[1][k], mul2(w[3][k], da[0][k]))));
+          win[0][k] = win[1][k]; win[1][k] = win[2][k]; win[2][k] = x[k];
+          da[0][k] = da[1][k]; da[1][k] = da[2][k]; da[2][k] = d;
         }
         const int t = s - 3;
-        if (t >= t0 && t < t1) store4<T>(dx + ((size_t)b * p.T + t) * q.dxs + c, g);
-        else if (t < 0 && t0 == 0 && q.dstate && t >= -(W - 1)) {
+        if (t >= t0) {
+          if (t < t1) store4<T>(dxb + (size_t)t * q.dxs, g);
+        } else if (q.dstate && t < 0 && t >= -(W - 1)) {   // the first tile also owns the gradient of the carried conv state
+          const float2 lo = un2(g[0]), hi = un2(g[1]);
+          const float v[4] = {lo.x, lo.y, hi.x, hi.y};
 #pragma unroll
           for (int k = 0; k < CONV_V; ++k)
-            reinterpret_cast<T*>(q.dstate)[((size_t)b * p.C + c + k) * (W - 1) + (W - 1 + t)] = from_f32<T>(g[k]);
+            reinterpret_cast<T*>(q.dstate)[((size_t)b * p.C + c + k) * (W - 1) + (W - 1 + t)] = from_f32<T>(v[k]);
         }
       };
-      if (s_end - s_begin == CONV_TT + 3 && s_end <= p.T) {
-        // full tile with its look-ahead inside the sequence: 35 steps as 5 batches of 7 whose loads
-        // are all issued (unconditionally) before the first store of the batch
-        constexpr int SB = 7;
-        static_assert((CONV_TT + 3) % SB == 0, "batching of the backward walk");
+      auto batch = [&](int s, auto mine, bool more) {
+        constexpr int n = decltype(mine)::value ? CONV_SB : 3;
+        Raw4<T> cx[n], cg[n], cy[SKIP ? n : 1];
+#pragma unroll
+        for (int i = 0; i < n; ++i) { cx[i] = nx[i]; cg[i] = ng[i]; if constexpr (SKIP) cy[i] = ny[i]; }
+        if (more) fetch(s + CONV_SB);
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+          f2 x[2], gy[2];
+          unpack4<T>(cx[i], x);
+          gradient(cg[i], cy[SKIP ? i : 0], gy);
+          step(s + i, mine, x, gy);
+        }
+      };
+      int s = t0;
 #pragma unroll 1
-        for (int sb = s_begin; sb < s_end; sb += SB) {
-          using Raw = typename std::conditional<sizeof(T) == 4, uint4, uint2>::type;   // 4 channels
-          Raw xr[SB], gr[SB], yr[SKIP ? SB : 1];
-#pragma unroll
-          for (int i = 0; i < SB; ++i) {
-            xr[i] = *reinterpret_cast<const Raw*>(x + ((size_t)b * p.T + sb + i) * p.xs + c);
-            gr[i] = *reinterpret_cast<const Raw*>(dUb + (size_t)(sb + i) * p.ust);
-            if constexpr (SKIP) yr[i] = *reinterpret_cast<const Raw*>(dYb + (size_t)(sb + i) * p.ust);
-          }
-#pragma unroll
-          for (int i = 0; i < SB; ++i) {
-            float xin[CONV_V], gy[CONV_V];
-            const T* ex = reinterpret_cast<const T*>(&xr[i]);
-            const T* eg = reinterpret_cast<const T*>(&gr[i]);
-#pragma unroll
-            for (int k = 0; k < CONV_V; ++k) { xin[k] = to_f32(ex[k]); gy[k] = to_f32(eg[k]); }
-            if constexpr (SKIP) {
-              const T* ey = reinterpret_cast<const T*>(&yr[i]);
-#pragma unroll
-              for (int k = 0; k < CONV_V; ++k) gy[k] = fmaf(skip, to_f32(ey[k]), gy[k]);
-            }
-            step(sb + i, true, xin, gy);
-          }
-        }
-      } else {
-        for (int s = s_begin; s < s_end; ++s) {
-          float xin[CONV_V], gy[CONV_V];
-          const bool in = s < p.T;
-          if (in) {
-            load4<T>(x + ((size_t)b * p.T + s) * p.xs + c, xin);
-            load_gy(s, gy);
-          }
-          step(s, in, xin, gy);
-        }
-      }
+      for (; s < t1; s += CONV_SB) batch(s, std::true_type{}, true);
+      batch(s, std::false_type{}, false);
     }
   }
   if (!p.w) return;
 #pragma unroll
-  for (int k = 0; k < CONV_V; ++k) {
+  for (int k = 0; k < 2; ++k) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) s_acc[sub][j][lane * CONV_V + k] = dwacc[j][k];
-    s_acc[sub][4][lane * CONV_V + k] = dbacc[k];
+    for (int j = 0; j < 5; ++j) *reinterpret_cast<f2*>(&s_acc[sub][j][lane * CONV_V + 2 * k]) = j < 4 ? dw[j & 3][k] : db[k];
   }
   __syncthreads();
-  // 5 x 128 sums of CONV_SUB partials; one atomic per (channel, tap) per CTA
+  // 5 x 128 sums of CONV_SUB partials; one atomic per (channel, tap) per CTA, the taps of a channel side by side
   for (int i = threadIdx.x; i < 5 * 32 * CONV_V; i += blockDim.x) {
-    const int j = i / (32 * CONV_V), cc = i - j * (32 * CONV_V);
+    const int j = i < 4 * 32 * CONV_V ? i & 3 : 4, cc = j < 4 ? i >> 2 : i - 4 * 32 * CONV_V;
     const int ch = blockIdx.x * 32 * CONV_V + cc;
     if (ch >= p.C) continue;
     float v = 0.f;
@@ -499,8 +452,17 @@ __global__ void __launch_bounds__(256, 2) value_bwd_vec_kernel(ValueBwdParams q)
   }
 }
 
-inline bool value_vec_ok(const ValueParams& p, const void* a, const void* b, int V = CONV_V) {
-  const int align = 16;
+// Tokens per warp: 32 (the walk restarts at a tile with 3 tokens of its neighbour), shorter while that leaves fewer than two
+// CTAs per SM - a warp walks its tile at one load latency per 4 tokens, 18 us for 32 of them.
+inline int conv_tile(int T, int C, int batch) {
+  int tile = 32;
+  const long long columns = (long long)batch * ((C + 32 * CONV_V - 1) / (32 * CONV_V));
+  while (tile > 8 && columns * ((T + CONV_SUB * tile - 1) / (CONV_SUB * tile)) < 2 * 148) tile /= 2;
+  return tile;
+}
+
+inline bool value_vec_ok(const ValueParams& p, const void* a, const void* b) {
+  constexpr int align = 16, V = CONV_V;
   return p.P % V == 0 && p.C % V == 0 && p.xs % V == 0 && p.usb % V == 0 &&
          p.ush % V == 0 && p.ust % V == 0 && aligned(p.x, align) && aligned(p.U, align) &&
          (a == nullptr || aligned(a, align)) && (b == nullptr || aligned(b, align));
@@ -931,10 +893,10 @@ int scanprep_fwd(const ScanPrepArgs& a, const ScanPrepOut& o, cudaStream_t st) {
     p.state_out = a.conv_state_out; p.U = o.U; p.xs = a.value_stride;
     p.usb = a.u_b; p.ush = a.u_h; p.ust = a.u_t;
     p.batch = batch; p.T = T; p.C = heads * a.P; p.P = a.P; p.W = a.conv_weight ? a.d_conv : 1;
-    const int vf = CONV_V;   // 4 channels per thread (8- or 16-byte pieces)
-    if (value_vec_ok(p, nullptr, nullptr, vf)) {
-      dim3 grid((p.C + 32 * vf - 1) / (32 * vf), (T + CONV_SUB * CONV_TT - 1) / (CONV_SUB * CONV_TT), batch);
-      SL_DISPATCH_DTYPE(a.io_dtype, Tt, { value_fwd_vec_kernel<Tt, CONV_V><<<grid, 256, 0, fork.v>>>(p); });
+    if (value_vec_ok(p, nullptr, nullptr)) {
+      const int tile = conv_tile(T, p.C, batch);
+      dim3 grid((p.C + 32 * CONV_V - 1) / (32 * CONV_V), (T + CONV_SUB * tile - 1) / (CONV_SUB * tile), batch);
+      SL_DISPATCH_DTYPE(a.io_dtype, Tt, { value_fwd_vec_kernel<Tt><<<grid, 256, 0, fork.v>>>(p, tile); });
     } else {
       dim3 grid((p.C + 255) / 256, (T + CONV_TT - 1) / CONV_TT, batch);
       SL_DISPATCH_DTYPE(a.io_dtype, Tt, { value_fwd_kernel<Tt><<<grid, 256, 0, fork.v>>>(p); });
@@ -994,10 +956,11 @@ int scanprep_bwd(const ScanPrepArgs& a, const ScanPrepGrads& g, cudaStream_t st)
     ValueParams pv = p;
     pv.U = const_cast<void*>(g.dU);
     if (value_vec_ok(pv, g.d_value, nullptr) && g.d_value_stride % CONV_V == 0 && aligned(g.dY, 16)) {
-      dim3 grid((p.C + 32 * CONV_V - 1) / (32 * CONV_V), (T + CONV_SUB * CONV_TT - 1) / (CONV_SUB * CONV_TT), batch);
+      const int tile = conv_tile(T, p.C, batch);
+      dim3 grid((p.C + 32 * CONV_V - 1) / (32 * CONV_V), (T + CONV_SUB * tile - 1) / (CONV_SUB * tile), batch);
       SL_DISPATCH_DTYPE(a.io_dtype, Tt, {
-        if (g.dY) value_bwd_vec_kernel<Tt, true><<<grid, 256, 0, fork.v>>>(q);
-        else value_bwd_vec_kernel<Tt, false><<<grid, 256, 0, fork.v>>>(q);
+        if (g.dY) value_bwd_vec_kernel<Tt, true><<<grid, 256, 0, fork.v>>>(q, tile);
+        else value_bwd_vec_kernel<Tt, false><<<grid, 256, 0, fork.v>>>(q, tile);
       });
     } else {
       dim3 grid((p.C + 255) / 256, (T + CONV_TT - 1) / CONV_TT, batch);
