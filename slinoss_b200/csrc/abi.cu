@@ -99,9 +99,9 @@ extern "C" size_t sl_workspace_bytes(int kind, int batch, int heads, int groups,
   if (batch < 1 || heads < 1 || groups < 1 || T < 1 || P < 1 || N < 1) return 0;
   switch (kind) {
     case SL_WS_SCAN_FWD:
-      return use_tc(path, d, io_dtype) ? scan_tc_fwd_workspace(d) : 0;
+      return use_tc(path, d, io_dtype) ? scan_tc_fwd_workspace(d) : scan_simt_fwd_workspace(d);
     case SL_WS_SCAN_BWD:
-      return use_tc(path, d, io_dtype) ? scan_tc_bwd_workspace(d) : scan_simt_bwd_workspace(d);
+      return use_tc(path, d, io_dtype) ? scan_tc_bwd_workspace(d) : scan_simt_bwd_split_workspace(d);
     case SL_WS_SCAN_STATES:
       return use_tc(path, d, io_dtype) ? scan_tc_states_bytes(d) : 0;
     default:
@@ -128,7 +128,7 @@ extern "C" int sl_v2x2ssd_fwd(const void* U, const float* M, const float* K, con
                        final_state ? chunk_states : nullptr, d, io_dtype, y_dtype, workspace,
                        workspace_bytes, st);
   return scan_simt_fwd(U, M, K, B, C, initial_states, B_prev, U_prev, Y, final_state, d,
-                       io_dtype, y_dtype, st);
+                       io_dtype, y_dtype, workspace, workspace_bytes, st);
 }
 
 extern "C" int sl_v2x2ssd_bwd(const void* U, const float* M, const float* K, const void* B,

@@ -223,8 +223,10 @@ struct ScanDims {
 
 int scan_simt_fwd(const void* U, const float* M, const float* K, const void* B, const void* C,
                   const float* z0, const void* Bprev, const void* Uprev, void* Y, float* zfinal,
-                  const ScanDims& d, int io_dtype, int y_dtype, cudaStream_t st);
+                  const ScanDims& d, int io_dtype, int y_dtype, void* ws, size_t ws_bytes, cudaStream_t st);
+size_t scan_simt_fwd_workspace(const ScanDims& d);
 size_t scan_simt_bwd_workspace(const ScanDims& d);
+size_t scan_simt_bwd_split_workspace(const ScanDims& d);
 int scan_simt_bwd(const void* U, const float* M, const float* K, const void* B, const void* C,
                   const float* z0, const void* Bprev, const void* Uprev, const void* dY,
                   const float* dfinal, void* dU, float* dM, float* dK, void* dB, void* dC,
