@@ -26,7 +26,7 @@
 // The walk over T is serial, so a problem with few (batch, head) streams is split in time: a first launch runs every
 // segment but the last from a zero state and keeps only where it ends and the product of its transitions; each CTA of the
 // sweeps then folds the segments before its own into its start state (all in float32, the products in float64).  B the same,
-// from the other end.  (2, 4, 256, P 64, N 32) forward + backward: 620 -> FIGURE us with 16 segments.
+// from the other end.  (2, 4, 256, P 64, N 32) forward + backward: 629 -> 74 us with 16 segments.
 #include <algorithm>
 
 #include "common.cuh"
@@ -92,18 +92,22 @@ template <int NC> struct Tile { f2 re[4][NC / 2], im[4][NC / 2]; };
 // src (P, 2N) of one (batch, head): the thread's piece, zeros outside
 template <int NC>
 __device__ __forceinline__ void load_tile(Tile<NC>& z, const float* src, const Place<NC>& o, int row0, int P, int N) {
+  const bool whole = (N & 1) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;   // 2 columns as one 16-byte piece
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
     for (int i = 0; i < NC / 2; ++i) {
       const int n = 2 * (o.pair + i), row = row0 + r;
-      float v[4] = {0.f, 0.f, 0.f, 0.f};
-      if (src && row < P) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (src && row < P && n < N) {
         const float* q = src + (size_t)row * 2 * N + 2 * n;
-        if (n < N) { v[0] = q[0]; v[1] = q[1]; }
-        if (n + 1 < N) { v[2] = q[2]; v[3] = q[3]; }
+        if (whole) v = *reinterpret_cast<const float4*>(q);
+        else {
+          v.x = q[0]; v.y = q[1];
+          if (n + 1 < N) { v.z = q[2]; v.w = q[3]; }
+        }
       }
-      z.re[r][i] = mk2(v[0], v[2]); z.im[r][i] = mk2(v[1], v[3]);
+      z.re[r][i] = mk2(v.x, v.z); z.im[r][i] = mk2(v.y, v.w);
     }
 }
 template <int NC>
@@ -138,13 +142,21 @@ template <int NC, bool CONJ>
 __device__ __forceinline__ void fold_tile(Tile<NC>& z, const SweepParams& p, const float* loc, const float* prod, int bh, int from,
                                           int step, int count, const Place<NC>& o, int row0) {
   const size_t bhs = (size_t)p.batch * p.heads;
-  Tile<NC> next;
-  if (count > 0) load_tile<NC>(next, loc + (from * bhs + bh) * p.P * 2 * p.N, o, row0, p.P, p.N);
-  for (int k = 0, q = from; k < count; ++k, q += step) {
-    const Tile<NC> add = next;
-    const float2 m = *reinterpret_cast<const float2*>(prod + 2 * (q * bhs + bh));
-    if (k + 1 < count) load_tile<NC>(next, loc + ((q + step) * bhs + bh) * p.P * 2 * p.N, o, row0, p.P, p.N);
-    advance_tile<NC, CONJ>(z, m.x, m.y, add);
+  constexpr int DEPTH = 8 / NC;   // segments of a batch of loads
+#pragma unroll 1
+  for (int k = 0; k < count; k += DEPTH) {
+    Tile<NC> add[DEPTH];
+    float2 m[DEPTH];
+#pragma unroll
+    for (int i = 0; i < DEPTH; ++i) {
+      if (k + i >= count) continue;
+      const size_t at = (from + step * (k + i)) * bhs + bh;
+      m[i] = *reinterpret_cast<const float2*>(prod + 2 * at);
+      load_tile<NC>(add[i], loc + at * p.P * 2 * p.N, o, row0, p.P, p.N);
+    }
+#pragma unroll
+    for (int i = 0; i < DEPTH; ++i)
+      if (k + i < count) advance_tile<NC, CONJ>(z, m[i].x, m[i].y, add[i]);
   }
 }
 // Product of the transitions [t0, t1) (1 past the end of the sequence), by one warp, to dst.
@@ -189,6 +201,28 @@ struct Stream {
   }
 };
 
+// A (rows, cols) array by the CTA, a warp per row: U rows are loaded, then stored, so that they cost one latency.
+template <int U, typename V, typename Load, typename Store>
+__device__ __forceinline__ void staged(int rows, int cols, Load load, Store store) {
+  const int nw = blockDim.x >> 5;
+#pragma unroll 1
+  for (int c = threadIdx.x & 31; c < cols; c += 32)
+#pragma unroll 1
+    for (int r = threadIdx.x >> 5; r < rows; r += U * nw) {
+      V v[U];
+#pragma unroll
+      for (int i = 0; i < U; ++i)
+        if (r + i * nw < rows) v[i] = load(r + i * nw, c);
+#pragma unroll
+      for (int i = 0; i < U; ++i)
+        if (r + i * nw < rows) store(r + i * nw, c, v[i]);
+    }
+}
+template <typename F> __device__ __forceinline__ void each_row(int rows, int cols, F f) {
+  for (int r = threadIdx.x >> 5; r < rows; r += blockDim.x >> 5)
+    for (int c = threadIdx.x & 31; c < cols; c += 32) f(r, c);
+}
+
 // A token's columns in shared memory: pair (n, n+1) as re re im im
 __device__ __forceinline__ int pair_slot(int n) { return 4 * (n >> 1) + (n & 1); }
 
@@ -197,46 +231,44 @@ template <typename TIn, typename TY>
 __device__ __forceinline__ void stage_columns(const SweepParams& p, const Stream<TIn, TY>& x, int t0, int nb, int Npad, float* s_bp,
                                               float* s_bc, float* s_c) {
   const int D = 2 * p.N, D2 = 2 * Npad;
-  for (int idx = threadIdx.x; idx < nb * Npad; idx += blockDim.x) {
-    const int tt = idx / Npad, n = idx - tt * Npad, t = t0 + tt;
-    cf bt = {0.f, 0.f}, bpv = {0.f, 0.f}, ct = {0.f, 0.f};
+  struct Piece { cf bt, bpv, ct; float4 k4; };
+  staged<2, Piece>(nb, Npad, [&](int tt, int n) {
+    const int t = t0 + tt;
+    Piece v{};
     if (n < p.N) {
-      if (s_bc) bt = load_c(x.B + (size_t)t * D, n);
-      if (s_c) ct = load_c(x.C + (size_t)t * D, n);
+      if (s_bc) v.bt = load_c(x.B + (size_t)t * D, n);
+      if (s_c) v.ct = load_c(x.C + (size_t)t * D, n);
       if (s_bp) {
-        if (t > 0) bpv = load_c(x.B + (size_t)(t - 1) * D, n);
-        else if (x.Bp) bpv = load_c(x.Bp, n);
+        if (t > 0) v.bpv = load_c(x.B + (size_t)(t - 1) * D, n);
+        else if (x.Bp) v.bpv = load_c(x.Bp, n);
       }
     }
+    if (s_bp || s_bc) v.k4 = *reinterpret_cast<const float4*>(x.K + (size_t)t * 4);
+    return v;
+  }, [&](int tt, int n, const Piece& v) {
     const int o = tt * D2 + pair_slot(n);
-    if (s_bp || s_bc) {
-      const float4 k4 = *reinterpret_cast<const float4*>(x.K + (size_t)t * 4);
-      const cf bp = cmul({k4.x, k4.y}, bpv), bc = cmul({k4.z, k4.w}, bt);
-      if (s_bp) { s_bp[o] = bp.re; s_bp[o + 2] = bp.im; }
-      if (s_bc) { s_bc[o] = bc.re; s_bc[o + 2] = bc.im; }
-    }
-    if (s_c) { s_c[o] = ct.re; s_c[o + 2] = ct.im; }
-  }
+    const cf bp = cmul({v.k4.x, v.k4.y}, v.bpv), bc = cmul({v.k4.z, v.k4.w}, v.bt);
+    if (s_bp) { s_bp[o] = bp.re; s_bp[o + 2] = bp.im; }
+    if (s_bc) { s_bc[o] = bc.re; s_bc[o + 2] = bc.im; }
+    if (s_c) { s_c[o] = v.ct.re; s_c[o + 2] = v.ct.im; }
+  });
 }
 // u of the tokens t0 - 1 .. t0 + nb - 1
 template <typename TIn, typename TY>
 __device__ __forceinline__ void stage_u(const SweepParams& p, const Stream<TIn, TY>& x, int t0, int nb, int PT, float* s_u) {
-  for (int idx = threadIdx.x; idx < (nb + 1) * PT; idx += blockDim.x) {
-    const int tt = idx / PT, pp = idx - tt * PT, t = t0 + tt - 1, pr = x.row0 + pp;
-    float v = 0.f;
-    if (pr < p.P) {
-      if (t >= 0) v = to_f32(x.U[(size_t)t * p.P + pr]);
-      else if (x.Up) v = to_f32(x.Up[pr]);
-    }
-    s_u[idx] = v;
-  }
+  staged<3, float>(nb + 1, PT, [&](int tt, int pp) {
+    const int t = t0 + tt - 1, pr = x.row0 + pp;
+    if (pr >= p.P) return 0.f;
+    if (t >= 0) return to_f32(x.U[(size_t)t * p.P + pr]);
+    return x.Up ? to_f32(x.Up[pr]) : 0.f;
+  }, [&](int tt, int pp, float v) { s_u[tt * PT + pp] = v; });
 }
 template <typename TIn, typename TY>
 __device__ __forceinline__ void stage_dy(const SweepParams& p, const Stream<TIn, TY>& x, int t0, int nb, int PT, float* s_dy) {
-  for (int idx = threadIdx.x; idx < nb * PT; idx += blockDim.x) {
-    const int tt = idx / PT, pp = idx - tt * PT, pr = x.row0 + pp;
-    s_dy[idx] = (pr < p.P && x.dY) ? to_f32(x.dY[(size_t)(t0 + tt) * p.P + pr]) : 0.f;
-  }
+  staged<2, float>(nb, PT, [&](int tt, int pp) {
+    const int pr = x.row0 + pp;
+    return (pr < p.P && x.dY) ? to_f32(x.dY[(size_t)(t0 + tt) * p.P + pr]) : 0.f;
+  }, [&](int tt, int pp, float v) { s_dy[tt * PT + pp] = v; });
 }
 // m of the tokens t0 + off ... (1 past the end of the sequence)
 __device__ __forceinline__ void stage_m(const float* M, int t0, int nb, int T, float* s_m) {
@@ -305,6 +337,7 @@ __device__ __forceinline__ void forward_sweep(const SweepParams& p, int pt, int 
 
     f2 up[4], u[4];
     rows4(s_u + o.pl, up);
+#pragma unroll 1
     for (int tt = 0; tt < nb; ++tt) {
       const f2 mr = dup2(s_m[2 * tt]), mi = dup2(s_m[2 * tt + 1]), mn = dup2(-s_m[2 * tt + 1]);
       rows4(s_u + (tt + 1) * PT + o.pl, u);
@@ -342,24 +375,24 @@ __device__ __forceinline__ void forward_sweep(const SweepParams& p, int pt, int 
 
     if (MODE == 0) {
       TY* Yb = reinterpret_cast<TY*>(p.Y) + (size_t)x.bh * p.T * P;
-      for (int idx = threadIdx.x; idx < nb * PT; idx += blockDim.x) {
-        const int tt = idx / PT, pp = idx - tt * PT, pr = x.row0 + pp;
+      each_row(nb, PT, [&](int tt, int pp) {
+        const int pr = x.row0 + pp;
         if (pr < P) {
           float s = 0.f;
           for (int k = 0; k < NS; ++k) s += s_part[(tt * NS + k) * PT + pp];
           Yb[(size_t)(t0 + tt) * P + pr] = from_f32<TY>(s);
         }
-      }
+      });
     }
     if (MODE == 1) {
       float* dcb = p.dc_head + (size_t)x.bh * p.T * D;
-      for (int idx = threadIdx.x; idx < nb * D; idx += blockDim.x) {
-        const int tt = idx / D, col = idx - tt * D, slot = pair_slot(col >> 1) + 2 * (col & 1);
+      each_row(nb, D, [&](int tt, int col) {
+        const int slot = pair_slot(col >> 1) + 2 * (col & 1);
         float s = 0.f;
         for (int k = 0; k < PW; ++k) s += s_part[(tt * PW + k) * D2 + slot];
         float* dst = dcb + (size_t)(t0 + tt) * D + col;
         if (p.ptiles > 1) atomicAdd(dst, s); else *dst = s;
-      }
+      });
     }
     // the staging of the next block only rewrites arrays last read before the
     // second barrier; s_part is next written after the first barrier of that block.
@@ -457,6 +490,7 @@ __device__ __forceinline__ void reverse_sweep(const SweepParams& p, int pt, int 
     stage_m(x.M, t0 + 1, nb, p.T, s_mn);
     __syncthreads();
 
+#pragma unroll 1
     for (int tt = nb - 1; tt >= 0; --tt) {
       const f2 mr = dup2(s_mn[2 * tt]), mi = dup2(s_mn[2 * tt + 1]), mn = dup2(-s_mn[2 * tt + 1]);
       f2 dy[4];
@@ -496,8 +530,8 @@ __device__ __forceinline__ void reverse_sweep(const SweepParams& p, int pt, int 
     __syncthreads();
     if (STATES) continue;
 
-    for (int idx = threadIdx.x; idx < nb * D; idx += blockDim.x) {
-      const int tt = idx / D, col = idx - tt * D, slot = pair_slot(col >> 1) + 2 * (col & 1);
+    each_row(nb, D, [&](int tt, int col) {
+      const int slot = pair_slot(col >> 1) + 2 * (col & 1);
       float sc = 0.f, sp = 0.f;
       for (int k = 0; k < PW; ++k) {
         sc += s_pc[(tt * PW + k) * D2 + slot];
@@ -506,10 +540,10 @@ __device__ __forceinline__ void reverse_sweep(const SweepParams& p, int pt, int 
       const size_t q = ((size_t)x.bh * p.T + t0 + tt) * D + col;
       if (p.ptiles > 1) { atomicAdd(p.dbc_head + q, sc); atomicAdd(p.dbp_head + q, sp); }
       else { p.dbc_head[q] = sc; p.dbp_head[q] = sp; }
-    }
+    });
     TIn* dUb = reinterpret_cast<TIn*>(p.dU) + (size_t)x.bh * p.T * P;
-    for (int idx = threadIdx.x; idx < nb * PT; idx += blockDim.x) {
-      const int tt = idx / PT, pp = idx - tt * PT, pr = x.row0 + pp;
+    each_row(nb, PT, [&](int tt, int pp) {
+      const int pr = x.row0 + pp;
       float s = tt == nb - 1 ? s_carry[par * PT + pp] : 0.f;
       for (int k = 0; k < NS; ++k) s += s_duc[(tt * NS + k) * PT + pp];
       if (tt < nb - 1)
@@ -520,7 +554,7 @@ __device__ __forceinline__ void reverse_sweep(const SweepParams& p, int pt, int 
         for (int k = 0; k < NS; ++k) c += s_dup[k * PT + pp];
         s_carry[(par ^ 1) * PT + pp] = c;
       }
-    }
+    });
     // the next block's staging rewrites arrays last read before the second barrier; s_pc, s_pp, s_duc, s_dup and the
     // other half of s_carry are next written or read after its first barrier.
   }
@@ -715,7 +749,7 @@ struct SimtConfig {
 };
 
 // Segments of T.  Per token a CTA takes as long alone on its SM as with others up to 16 warps; a split adds a pre-pass (half
-// the work of a sweep), its launch (worth about 40 tokens) and a fold of 3 tokens per segment passed.  Sequences up to 64 tokens stay whole.
+// the work of a sweep), its launch (worth about 30 tokens) and a fold of one per segment passed.  Sequences up to 64 tokens stay whole.
 void plan_segments(const ScanDims& d, SimtConfig& c) {
   c.nseg = 1; c.seg_len = d.T;
   if (d.T <= 64) return;
@@ -724,7 +758,7 @@ void plan_segments(const ScanDims& d, SimtConfig& c) {
   for (int n = 2; n <= 64; ++n) {
     const int len = ((d.T + n - 1) / n + c.TB - 1) / c.TB * c.TB, segs = (d.T + len - 1) / len;
     if (segs < 2) break;
-    const double cost = 1.5 * len * std::max(1.0, ctas * segs / slots) + 40 + 3.0 * segs;
+    const double cost = 1.5 * len * std::max(1.0, ctas * segs / slots) + 30 + segs;
     if (cost < 0.9 * best || (cost < best && c.nseg > 1)) { best = cost; c.nseg = segs; c.seg_len = len; }
   }
 }
