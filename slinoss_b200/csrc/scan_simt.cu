@@ -748,12 +748,12 @@ struct SimtConfig {
   size_t smem_fwd, smem_rev;
 };
 
-// Segments of T.  Per token a CTA takes as long alone on its SM as with others up to 16 warps; a split adds a pre-pass (half
+// Segments of T.  Per token a CTA takes as long alone on its SM as with others up to 8 warps; a split adds a pre-pass (half
 // the work of a sweep), its launch (worth about 30 tokens) and a fold of one per segment passed.  Sequences up to 64 tokens stay whole.
 void plan_segments(const ScanDims& d, SimtConfig& c) {
   c.nseg = 1; c.seg_len = d.T;
   if (d.T <= 64) return;
-  const double ctas = (double)d.batch * d.heads * c.ptiles, slots = 148.0 * std::max(1, 512 / c.threads);
+  const double ctas = (double)d.batch * d.heads * c.ptiles, slots = 148.0 * std::max(1, 256 / c.threads);
   double best = d.T * std::max(1.0, ctas / slots);
   for (int n = 2; n <= 64; ++n) {
     const int len = ((d.T + n - 1) / n + c.TB - 1) / c.TB * c.TB, segs = (d.T + len - 1) / len;
