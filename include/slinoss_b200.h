@@ -57,8 +57,8 @@ enum {
   SL_PATH_AUTO = 0, /* tensor-core path when the shape allows, else SIMT */
   SL_PATH_SIMT = 1, /* exact float32 sequential recurrence (any dtype in)     */
   SL_PATH_TC = 2    /* tcgen05/TMEM chunked path: bf16 / fp16 operands, P = 64, N = 64 or 128
-                       (N = 128 runs as two passes over the column blocks of B and C and needs the
-                       SL_WS_SCAN_FWD workspace in the forward pass too)       */
+                       (auto takes every N <= 128 that is a multiple of 4); without the SL_WS_SCAN_FWD workspace
+                       of a problem the forward pass is refused                 */
 };
 
 /* workspace kinds for sl_workspace_bytes */
@@ -301,8 +301,8 @@ SL_API int sl_mixer_tail_bwd(const void* Y, const void* gate, int64_t gate_row_s
  *          read one while one of them writes the other)
  *   u_prev (batch, heads, P) : io_dtype, the previous token's u, UPDATED IN PLACE
  *   normed (batch, heads*P) : io_dtype, dense - the input of out_proj
- *   workspace: sl_mixer_decode_step_workspace_bytes(batch, heads, P) bytes that are ZERO before the
- *          first call; every call leaves them zero again (calls on one workspace must not overlap).
+ *   workspace: sl_mixer_decode_step_workspace_bytes(batch, heads, P) bytes of scratch
+ *          (calls on one workspace must not overlap).
  */
 SL_API size_t sl_mixer_decode_step_workspace_bytes(int batch, int heads, int P);
 SL_API int sl_mixer_decode_step(const void* gate, int64_t gate_row_stride, const void* value,
