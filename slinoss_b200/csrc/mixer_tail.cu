@@ -374,10 +374,27 @@ __global__ void __launch_bounds__(TAIL_THREADS) tail_bwd_vec_kernel(TailParams p
   }
 }
 
-// The common width (heads * P <= 256 pieces of 16 bytes: one piece per thread) with fewer live registers,
-// so that three CTAs stay resident per SM: the row is kept as its four packed pieces and unpacked again
-// after the reduction (same operations, same roundings), both row sums travel in one reduction, and its
-// shared-memory slots alternate with the row so that one barrier per row is enough.  The CTA has just the warps the
+// Pair k of a 16-byte piece, and a pair put (rounded) into it.
+template <typename T> __device__ __forceinline__ f2 pair_of(const uint4& r, int k) {
+  const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+  if constexpr (sizeof(T) == 2) {
+    const float2 q = unpack_pair<T>(w[k]);
+    return mk2(q.x, q.y);
+  } else {
+    return mk2(__uint_as_float(w[2 * k]), __uint_as_float(w[2 * k + 1]));
+  }
+}
+template <typename T> __device__ __forceinline__ void put_pair(uint32_t (&w)[4], int k, f2 v) {
+  const float2 q = un2(v);
+  if constexpr (sizeof(T) == 2) w[k] = pack_pair<T>(q.x, q.y);
+  else { w[2 * k] = __float_as_uint(q.x); w[2 * k + 1] = __float_as_uint(q.y); }
+}
+__device__ __forceinline__ uint4 piece(const uint32_t (&w)[4]) { return make_uint4(w[0], w[1], w[2], w[3]); }
+
+// The common width (heads * P <= 256 pieces of 16 bytes: one piece per thread) with fewer live registers, so that three
+// CTAs stay resident per SM: between the two halves of a row its pieces stay packed, among them ``pre`` and ``hid``, which are
+// rounded to the io type anyway; both row sums travel in one reduction, and its shared-memory slots alternate with the row so
+// that one barrier per row is enough.  Was bound by instruction issue: 92 per channel, about 30 in packed pairs (16384 x 2048: 124 -> 110 us).  The CTA has just the warps the
 // row fills: with a fixed 256 threads a row of 1152 channels left 44 % of the lanes idle.
 template <typename T>
 __global__ void __launch_bounds__(TAIL_THREADS, 3) tail_bwd_row_kernel(TailParams p) {
@@ -398,9 +415,9 @@ __global__ void __launch_bounds__(TAIL_THREADS, 3) tail_bwd_row_kernel(TailParam
   const float dsk = (act && S) ? p.d_skip[hh] : 0.f;
   uint4 wraw = make_uint4(0, 0, 0, 0);
   if (act) wraw = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.w) + c);
-  float dw_acc[V], dsk_acc = 0.f;
+  f2 dw_acc[V / 2], dsk_acc = 0;
 #pragma unroll
-  for (int k = 0; k < V; ++k) dw_acc[k] = 0.f;
+  for (int k = 0; k < V / 2; ++k) dw_acc[k] = 0;
   const unsigned rows = (unsigned)p.batch * (unsigned)p.T;   // < 2^31, checked by the launcher
   const size_t head_off = (size_t)hh * p.T * p.P + pp, batch_step = (size_t)p.H * p.T * p.P;
   uint4 nY = make_uint4(0, 0, 0, 0), nG = nY, nS = nY, nD = nY;
@@ -419,25 +436,20 @@ __global__ void __launch_bounds__(TAIL_THREADS, 3) tail_bwd_row_kernel(TailParam
     const uint4 cY = nY, cG = nG, cS = nS, cD = nD;
     if (row + gridDim.x < rows) fetch(row + gridDim.x);
     float ss = 0.f, dot = 0.f;
+    uint32_t pre[4] = {cY.x, cY.y, cY.z, cY.w}, hid[4] = {0, 0, 0, 0};
     if (act) {
-      float pre[V], g[V], dnv[V], wv[V];
-      unpack16<T>(cY, pre); unpack16<T>(cG, g); unpack16<T>(cD, dnv); unpack16<T>(wraw, wv);
-      if (S) {
-        float sv[V];
-        unpack16<T>(cS, sv);
+      f2 ss2 = 0, dot2 = 0;
 #pragma unroll
-        for (int k = 0; k < V; k += 2) {
-          pre[k] += sv[k] * dsk; pre[k + 1] += sv[k + 1] * dsk;
-          round_pair<T>(pre[k], pre[k + 1]);
-        }
+      for (int k = 0; k < V / 2; ++k) {
+        const f2 g = pair_of<T>(cG, k);
+        if (S) put_pair<T>(pre, k, fma2(pair_of<T>(cS, k), dup2(dsk), pair_of<T>(cY, k)));
+        put_pair<T>(hid, k, mul2(pair_of<T>(piece(pre), k), mul2(g, sigmoid2(g))));
+        const f2 h = pair_of<T>(piece(hid), k);
+        ss2 = fma2(h, h, ss2);
+        dot2 = fma2(h, mul2(pair_of<T>(cD, k), pair_of<T>(wraw, k)), dot2);
       }
-#pragma unroll
-      for (int k = 0; k < V; k += 2) {
-        float h0 = pre[k] * silu_f(g[k]), h1 = pre[k + 1] * silu_f(g[k + 1]);
-        round_pair<T>(h0, h1);
-        ss += h0 * h0 + h1 * h1;
-        dot += h0 * dnv[k] * wv[k] + h1 * dnv[k + 1] * wv[k + 1];
-      }
+      const float2 a = un2(ss2), d = un2(dot2);
+      ss = a.x + a.y; dot = d.x + d.y;
     }
     ss = warp_sum(ss); dot = warp_sum(dot);
     if (lane == 0) s_red[par][warp] = make_float2(ss, dot);
@@ -451,42 +463,24 @@ __global__ void __launch_bounds__(TAIL_THREADS, 3) tail_bwd_row_kernel(TailParam
     if (act) {
       const unsigned b = row / (unsigned)p.T, t = row - b * (unsigned)p.T;
       const size_t yi = b * batch_step + head_off + (size_t)t * p.P;
-      float pre[V], g[V], dnv[V], wv[V], sv[V];
-      unpack16<T>(cY, pre); unpack16<T>(cG, g); unpack16<T>(cD, dnv); unpack16<T>(wraw, wv);
-      if (S) {
-        unpack16<T>(cS, sv);
+      const f2 r2 = dup2(rstd), c2 = dup2(-coef);
+      uint32_t o_dy[4], o_dg[4], o_ds[4];
 #pragma unroll
-        for (int k = 0; k < V; k += 2) {
-          pre[k] += sv[k] * dsk; pre[k + 1] += sv[k + 1] * dsk;
-          round_pair<T>(pre[k], pre[k + 1]);
+      for (int k = 0; k < V / 2; ++k) {
+        const f2 h = pair_of<T>(piece(hid), k), dnk = pair_of<T>(cD, k), g = pair_of<T>(cG, k), sg = sigmoid2(g);
+        dw_acc[k] = fma2(dnk, mul2(h, r2), dw_acc[k]);
+        const f2 dh = fma2(mul2(dnk, pair_of<T>(wraw, k)), r2, mul2(h, c2));
+        const f2 silu = mul2(g, sg), dpre = mul2(dh, silu);
+        put_pair<T>(o_dg, k, mul2(mul2(dh, pair_of<T>(piece(pre), k)), fma2(silu, fma2(sg, dup2(-1.f), dup2(1.f)), sg)));
+        put_pair<T>(o_dy, k, dpre);
+        if (S) {
+          dsk_acc = fma2(dpre, pair_of<T>(cS, k), dsk_acc);
+          if (dS) put_pair<T>(o_ds, k, mul2(dpre, dup2(dsk)));
         }
       }
-      float o_dy[V], o_dg[V], o_ds[V];
-#pragma unroll
-      for (int k2 = 0; k2 < V; k2 += 2) {
-        float sgv[2], hidv[2];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          sgv[q] = sigmoid_f(g[k2 + q]);
-          hidv[q] = pre[k2 + q] * silu_f(g[k2 + q]);
-        }
-        round_pair<T>(hidv[0], hidv[1]);
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int k = k2 + q;
-          const float gg = g[k], sg = sgv[q], hid = hidv[q];
-          dw_acc[k] += dnv[k] * hid * rstd;
-          const float dh = rstd * dnv[k] * wv[k] - hid * coef;
-          const float dpre = dh * gg * sg;
-          o_dg[k] = dh * pre[k] * sg * (1.f + gg * (1.f - sg));
-          o_dy[k] = dpre;
-          o_ds[k] = 0.f;
-          if (S) { o_ds[k] = dpre * dsk; dsk_acc += dpre * sv[k]; }
-        }
-      }
-      store16<T>(dgate + (size_t)row * p.dgs + c, o_dg);
-      store16<T>(dY + yi, o_dy);
-      if (S && dS) store16<T>(dS + yi, o_ds);
+      *reinterpret_cast<uint4*>(dgate + (size_t)row * p.dgs + c) = piece(o_dg);
+      *reinterpret_cast<uint4*>(dY + yi) = piece(o_dy);
+      if (S && dS) *reinterpret_cast<uint4*>(dS + yi) = piece(o_ds);
     }
   }
   // One atomic of the CTA per 4 weights and per head: adds to one 32-byte sector are serial in L2, and with one per thread
@@ -494,20 +488,27 @@ __global__ void __launch_bounds__(TAIL_THREADS, 3) tail_bwd_row_kernel(TailParam
   if (act) {
     if ((reinterpret_cast<uintptr_t>(p.d_w) & 15) == 0) {
 #pragma unroll
-      for (int k = 0; k < V; k += 4)
-        atomicAdd(reinterpret_cast<float4*>(p.d_w + c + k), make_float4(dw_acc[k], dw_acc[k + 1], dw_acc[k + 2], dw_acc[k + 3]));
+      for (int k = 0; k < V; k += 4) {
+        const float2 a = un2(dw_acc[k / 2]), b = un2(dw_acc[k / 2 + 1]);
+        atomicAdd(reinterpret_cast<float4*>(p.d_w + c + k), make_float4(a.x, a.y, b.x, b.y));
+      }
     } else {
 #pragma unroll
-      for (int k = 0; k < V; ++k) atomicAdd(p.d_w + c + k, dw_acc[k]);
+      for (int k = 0; k < V / 2; ++k) {
+        const float2 a = un2(dw_acc[k]);
+        atomicAdd(p.d_w + c + 2 * k, a.x); atomicAdd(p.d_w + c + 2 * k + 1, a.y);
+      }
     }
   }
   if (S && p.d_d_skip) {
     const int per_head = p.P / V;   // threads of one head
+    const float2 both = un2(dsk_acc);
+    float sum = both.x + both.y;
     if (per_head <= 32 && (per_head & (per_head - 1)) == 0) {   // whole warps, or an aligned share of one
-      for (int o = per_head >> 1; o; o >>= 1) dsk_acc += __shfl_xor_sync(0xffffffffu, dsk_acc, o);
-      if (act && (threadIdx.x & (per_head - 1)) == 0) atomicAdd(p.d_d_skip + hh, dsk_acc);
+      for (int o = per_head >> 1; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (act && (threadIdx.x & (per_head - 1)) == 0) atomicAdd(p.d_d_skip + hh, sum);
     } else if (act) {
-      atomicAdd(p.d_d_skip + hh, dsk_acc);
+      atomicAdd(p.d_d_skip + hh, sum);
     }
   }
 }
@@ -581,7 +582,7 @@ int mixer_tail_bwd(const void* Y, const void* gate, int64_t gate_stride, const v
     const int pieces = heads * P / Vec16<Tt>::N;
     if (tail_vec_ok<Tt>(p)) {
       // one piece per thread; 24 warps per SM stay resident.  16384 rows of 2048 channels: 153 us with an atomic per thread
-      // for the sums over rows, 130 with one per head and four weights; 8192 rows of 1152: 80 and 44
+      // for the sums over rows, 130 with one per head and four weights
       if (pieces <= TAIL_THREADS) {
         const int threads = (pieces + 31) / 32 * 32;
         const long long fit = 148ll * (24 * 32 / threads);

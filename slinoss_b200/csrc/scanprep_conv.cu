@@ -560,10 +560,6 @@ __global__ void __launch_bounds__(256) bc_bwd_kernel(const T* __restrict__ bc,
 // 4 complex values.  The mean over n is a shuffle reduction inside the lanes of B or C.  With 16-bit
 // io the transcendental functions are the fast intrinsics (their error is far below the output's
 // rounding); float32 io keeps the precise ones.
-template <bool FAST> __device__ __forceinline__ float softplus_v(float x) {
-  if (FAST) return fmaxf(x, 0.f) + __logf(1.f + __expf(-fabsf(x)));
-  return softplus_f(x);
-}
 template <bool FAST> __device__ __forceinline__ float tanh_v(float x) {
   if (FAST) {   // one MUFU op, relative error 2^-11: below the rounding of 16-bit outputs
     float y;
@@ -572,22 +568,9 @@ template <bool FAST> __device__ __forceinline__ float tanh_v(float x) {
   }
   return tanhf(x);
 }
-template <bool FAST> __device__ __forceinline__ float sigmoid_v(float x) {
-  if (FAST) return 0.5f * tanh_v<true>(0.5f * x) + 0.5f;
-  return sigmoid_f(x);
-}
 template <bool FAST> __device__ __forceinline__ void sincos_v(float x, float* s, float* c) {
   if (FAST) __sincosf(x, s, c);   // |x| <= pi here
   else sincosf(x, s, c);
-}
-template <typename T> __device__ __forceinline__ void load8(const T* p, float (&v)[8]) {
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    float q[4];
-    load4<T>(p + 4 * h, q);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[4 * h + i] = q[i];
-  }
 }
 template <typename T> __device__ __forceinline__ void store8(T* p, const float (&v)[8]) {
   if constexpr (sizeof(T) == 2) {
@@ -606,10 +589,55 @@ template <bool WIDE> __device__ __forceinline__ float part_sum(float v) {   // o
 
 constexpr int BC_GCH = 8;   // groups one warp walks: grid = (tokens / 8, groups / BC_GCH, batch)
 
+// Pairs of the maps above.  (The 16-bit forms spell out the special-function steps: __expf and __logf also rescale denormal
+// operands, which do not occur here - 3 instructions each.)
+template <bool FAST> __device__ __forceinline__ f2 softplus2(f2 x) {
+  const float2 v = un2(x);
+  if constexpr (!FAST) return mk2(softplus_f(v.x), softplus_f(v.y));
+  const f2 e = mk2(ex2f(-1.4426950408889634f * fabsf(v.x)), ex2f(-1.4426950408889634f * fabsf(v.y)));
+  const float2 d = un2(add2(e, dup2(1.f)));
+  return fma2(mk2(lg2f(d.x), lg2f(d.y)), dup2(0.6931471805599453f), mk2(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f)));
+}
+template <bool FAST> __device__ __forceinline__ f2 tanh2(f2 x) {
+  const float2 v = un2(x);
+  return mk2(tanh_v<FAST>(v.x), tanh_v<FAST>(v.y));
+}
+template <bool FAST> __device__ __forceinline__ f2 sigmoid_pair(f2 x) {
+  if constexpr (FAST) return fma2(tanh2<true>(mul2(x, dup2(0.5f))), dup2(0.5f), dup2(0.5f));
+  const float2 v = un2(x);
+  return mk2(sigmoid_f(v.x), sigmoid_f(v.y));
+}
+template <bool FAST> __device__ __forceinline__ void sincos2(f2 x, f2* s, f2* c) {
+  const float2 v = un2(x);
+  float2 a, b;
+  sincos_v<FAST>(v.x, &a.x, &b.x); sincos_v<FAST>(v.y, &a.y, &b.y);
+  *s = mk2(a.x, a.y); *c = mk2(b.x, b.y);
+}
+// 4 complex values (re, im interleaved) as two pairs of real and two of imaginary parts, and their memory pieces
+template <typename T> struct Raw8 { Raw4<T> lo, hi; };
+template <typename T> __device__ __forceinline__ Raw8<T> load_raw8(const T* p) {
+  if constexpr (sizeof(T) == 2) {
+    const uint4 q = *reinterpret_cast<const uint4*>(p);
+    return {make_uint2(q.x, q.y), make_uint2(q.z, q.w)};
+  } else {
+    return {*reinterpret_cast<const uint4*>(p), *reinterpret_cast<const uint4*>(p + 4)};
+  }
+}
+template <typename T> __device__ __forceinline__ void split8(const Raw8<T>& r, f2 (&re)[2], f2 (&im)[2]) {
+  f2 q[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    unpack4<T>(h ? r.hi : r.lo, q);
+    const float2 a = un2(q[0]), b = un2(q[1]);
+    re[h] = mk2(a.x, b.x); im[h] = mk2(a.y, b.y);
+  }
+}
+
 // One warp per (batch, token, run of up to BC_GCH groups); the grid carries batch and the run, so no
 // index is divided at run time.  The next record's logits are requested before the current one is
-// evaluated.  (The kernels are bound by instruction issue and the XU pipe - five to six MUFU operations per
-// complex pair - not by DRAM.)
+// evaluated.  Bound by the special-function unit (five operations per complex pair, 74 us of it in 16384 tokens x 32 groups x
+// N = 64 against 83 of DRAM) once the rest is in
+// packed pairs: 115 -> 96 us, the backward 197 -> 154 (DRAM 125).
 template <typename T, bool WIDE>
 __global__ void __launch_bounds__(256) bc_fwd_vec_kernel(const T* __restrict__ bc, T* __restrict__ Bo,
                                                          T* __restrict__ Co, int64_t bcs, int Tn, int G, int N, float eps) {
@@ -624,34 +652,36 @@ __global__ void __launch_bounds__(256) bc_fwd_vec_kernel(const T* __restrict__ b
   T* dst = (which ? Co : Bo) + (((size_t)b * G + g0) * Tn + t) * 2 * N + 2 * n0;
   const size_t dstep = (size_t)Tn * 2 * N;
   const float inv_n = 1.f / (float)N;
-  float amp[4] = {0.f, 0.f, 0.f, 0.f}, ph[4] = {0.f, 0.f, 0.f, 0.f};
-  if (act) { load4<T>(src, amp); load4<T>(src + N, ph); }
+  Raw4<T> na{}, np{};
+  auto fetch = [&] {
+    if (!act) return;
+    na = *reinterpret_cast<const Raw4<T>*>(src);
+    np = *reinterpret_cast<const Raw4<T>*>(src + N);
+  };
+  fetch();
+#pragma unroll 2
   for (int g = g0; g < g1; ++g) {
-    float namp[4] = {0.f, 0.f, 0.f, 0.f}, nph[4] = {0.f, 0.f, 0.f, 0.f};
+    f2 amp[2], ph[2];
+    unpack4<T>(na, amp); unpack4<T>(np, ph);
     src += 4 * N;
-    if (act && g + 1 < g1) { load4<T>(src, namp); load4<T>(src + N, nph); }
-    float ss = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      amp[i] = act ? softplus_v<FAST>(amp[i]) : 0.f;
-      ss += amp[i] * amp[i];
-    }
-    ss = part_sum<WIDE>(ss);
+    if (g + 1 < g1) fetch();
+    amp[0] = softplus2<FAST>(amp[0]); amp[1] = softplus2<FAST>(amp[1]);
+    const float2 sq = un2(fma2(amp[0], amp[0], mul2(amp[1], amp[1])));
+    const float ss = part_sum<WIDE>(act ? sq.x + sq.y : 0.f);
     if (act) {
-      const float inv = rsqrtf(fmaxf(ss * inv_n, eps));
+      const f2 inv = dup2(rsqrtf(fmaxf(ss * inv_n, eps)));
       float o[8];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float sn, cs;
-        sincos_v<FAST>(3.14159265358979323846f * tanh_v<FAST>(ph[i]), &sn, &cs);
-        const float a = amp[i] * inv;
-        o[2 * i] = a * cs; o[2 * i + 1] = a * sn;
+      for (int i = 0; i < 2; ++i) {
+        f2 sn, cs;
+        sincos2<FAST>(mul2(tanh2<FAST>(ph[i]), dup2(3.14159265358979323846f)), &sn, &cs);
+        const f2 a = mul2(amp[i], inv);
+        const float2 re = un2(mul2(a, cs)), im = un2(mul2(a, sn));
+        o[4 * i] = re.x; o[4 * i + 1] = im.x; o[4 * i + 2] = re.y; o[4 * i + 3] = im.y;
       }
       store8<T>(dst, o);
     }
     dst += dstep;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { amp[i] = namp[i]; ph[i] = nph[i]; }
   }
 }
 
@@ -674,48 +704,47 @@ __global__ void __launch_bounds__(256) bc_bwd_vec_kernel(const T* __restrict__ b
   const T* grad = (which ? dCo : dBo) + (((size_t)b * G + g0) * Tn + t) * 2 * N + 2 * n0;
   const size_t gstep = (size_t)Tn * 2 * N;
   const float inv_n = 1.f / (float)N;
-  float xa[4] = {0.f, 0.f, 0.f, 0.f}, xp[4] = {0.f, 0.f, 0.f, 0.f}, gr[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) gr[i] = 0.f;
-  if (act) { load4<T>(src, xa); load4<T>(src + N, xp); load8<T>(grad, gr); }
+  Raw4<T> na{}, np{};
+  Raw8<T> ng{};
+  auto fetch = [&] {
+    if (!act) return;
+    na = *reinterpret_cast<const Raw4<T>*>(src);
+    np = *reinterpret_cast<const Raw4<T>*>(src + N);
+    ng = load_raw8<T>(grad);
+  };
+  fetch();
+#pragma unroll 2
   for (int g = g0; g < g1; ++g) {
-    float nxa[4] = {0.f, 0.f, 0.f, 0.f}, nxp[4] = {0.f, 0.f, 0.f, 0.f}, ngr[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) ngr[i] = 0.f;
+    f2 xa[2], xp[2], gre[2], gim[2], a[2], th[2], sn[2], cs[2], dot[2];
+    unpack4<T>(na, xa); unpack4<T>(np, xp);
+    split8<T>(ng, gre, gim);
     src += 4 * N; grad += gstep;
-    if (act && g + 1 < g1) { load4<T>(src, nxa); load4<T>(src + N, nxp); load8<T>(grad, ngr); }
-    float a[4], th[4], sn[4], cs[4];
-    float ss = 0.f, gsum = 0.f;
+    if (g + 1 < g1) fetch();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      a[i] = act ? softplus_v<FAST>(xa[i]) : 0.f;
-      th[i] = tanh_v<FAST>(xp[i]);
-      sincos_v<FAST>(3.14159265358979323846f * th[i], &sn[i], &cs[i]);
-      ss += a[i] * a[i];
-      gsum += a[i] * (cs[i] * gr[2 * i] + sn[i] * gr[2 * i + 1]);
+    for (int i = 0; i < 2; ++i) {
+      a[i] = softplus2<FAST>(xa[i]);
+      th[i] = tanh2<FAST>(xp[i]);
+      sincos2<FAST>(mul2(th[i], dup2(3.14159265358979323846f)), &sn[i], &cs[i]);
+      dot[i] = fma2(sn[i], gim[i], mul2(cs[i], gre[i]));
     }
-    ss = part_sum<WIDE>(ss); gsum = part_sum<WIDE>(gsum);
+    const float2 sq = un2(fma2(a[0], a[0], mul2(a[1], a[1]))), gs = un2(fma2(a[0], dot[0], mul2(a[1], dot[1])));
+    const float ss = part_sum<WIDE>(act ? sq.x + sq.y : 0.f), gsum = part_sum<WIDE>(act ? gs.x + gs.y : 0.f);
     if (act) {
-      const float ms = ss * inv_n;
-      const float inv = rsqrtf(fmaxf(ms, eps));
-      const float g_ms = ms > eps ? -0.5f * inv * inv * inv * gsum : 0.f;
-      float da[4], dp[4];
+      const float ms = ss * inv_n, inv = rsqrtf(fmaxf(ms, eps));
+      const f2 inv2 = dup2(inv), g_ms = dup2(ms > eps ? -inv * inv * inv * gsum * inv_n : 0.f);
+      f2 da[2], dp[2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float gre = gr[2 * i], gim = gr[2 * i + 1];
-        const float g_amp = inv * (cs[i] * gre + sn[i] * gim) + g_ms * 2.f * a[i] * inv_n;
-        const float g_ph = a[i] * inv * (cs[i] * gim - sn[i] * gre);
-        da[i] = g_amp * sigmoid_v<FAST>(xa[i]);
-        dp[i] = g_ph * 3.14159265358979323846f * (1.f - th[i] * th[i]);
+      for (int i = 0; i < 2; ++i) {
+        const f2 g_amp = fma2(inv2, dot[i], mul2(g_ms, a[i]));
+        da[i] = mul2(g_amp, sigmoid_pair<FAST>(xa[i]));
+        const f2 cross = fma2(cs[i], gim[i], mul2(mul2(sn[i], gre[i]), dup2(-1.f)));
+        const f2 slope = fma2(mul2(th[i], th[i]), dup2(-3.14159265358979323846f), dup2(3.14159265358979323846f));
+        dp[i] = mul2(mul2(mul2(a[i], inv2), cross), slope);
       }
       store4<T>(dst, da);
       store4<T>(dst + N, dp);
     }
     dst += 4 * N;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { xa[i] = nxa[i]; xp[i] = nxp[i]; }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) gr[i] = ngr[i];
   }
 }
 
