@@ -14,7 +14,7 @@ from torch import nn
 
 from .. import _C
 from ..layers import RMSNorm, SLinOSSMixer
-from ..layers.mixer import _norm_eps
+from ..layers.mixer import _norm_eps, planned_step
 from ..layers.mlp import SLinOSSMLP
 from ..ops.block import ffn_residual, ffn_residual_supported, residual_add
 from .config import SLinOSSBlockConfig
@@ -110,14 +110,42 @@ class SLinOSSBlock(nn.Module):
             out = self._ffn_residual(out)
         return (out, nxt) if return_state else out
 
+    def _make_token_plan(self):
+        mixer, ffn, norm = self.mixer, self.ffn, self.mixer_norm
+        kids = self._modules
+        if type(norm) is not RMSNorm or norm.weight is None:
+            return None
+        held = [(kids if n in kids else self.__dict__, n) for n in ("mixer", "mixer_norm", "ffn", "ffn_norm")]
+        same = [(d, n, d[n]) for d, n in held]
+        same.append((norm._parameters, "weight", norm.weight))
+        empty = [mixer._forward_hooks, mixer._forward_pre_hooks, norm._forward_hooks, norm._forward_pre_hooks]
+        branch, ffn_eps, kind = [norm.weight], 0.0, 0
+        if ffn is not None:
+            fnorm = self.ffn_norm
+            if not (type(ffn) is SLinOSSMLP and type(fnorm) is RMSNorm and fnorm.weight is not None
+                    and type(ffn.in_proj) is nn.Linear and type(ffn.out_proj) is nn.Linear):
+                return None
+            same += [(ffn._modules, n, ffn._modules[n]) for n in ("in_proj", "out_proj")]
+            same += [(ffn.__dict__, "kind", ffn.kind), (fnorm._parameters, "weight", fnorm.weight)]
+            for layer in (ffn.in_proj, ffn.out_proj):
+                same += [(layer._parameters, n, layer._parameters[n]) for n in ("weight", "bias")]
+            for m in (ffn, fnorm, ffn.in_proj, ffn.out_proj):
+                empty += [m._forward_hooks, m._forward_pre_hooks]
+            branch += [fnorm.weight, ffn.in_proj.weight, ffn.in_proj.bias, ffn.out_proj.weight, ffn.out_proj.bias]
+            ffn_eps, kind = _norm_eps(fnorm), _C.FFN_KINDS[ffn.kind]
+        return mixer._make_token_plan(branch, (same, empty), _norm_eps(norm), ffn_eps, kind)
+
     def _native_step(self, token, state, inplace):
-        """The whole step in five launches (see ``SLinOSSMixer.decode_native``), or None when something asks for the
+        """The whole step in five launches (a native plan, or ``SLinOSSMixer.decode_native``), or None when something asks for the
         composed path: gradients, another norm, dropout, autocast, hooks, an injected backend, a partial state."""
         mixer = self.mixer
         if torch.is_grad_enabled() or state is None or not token.is_cuda or (inplace is not None and not inplace) or \
                 (self.residual_dropout > 0.0 and self.training) or type(mixer) is not SLinOSSMixer:
             return None
         norm, ms = self.mixer_norm, state.mixer
+        out = planned_step(self, token, ms, self._make_token_plan)
+        if out is not None:
+            return out, SLinOSSBlockState(mixer=ms)
         if not (_plain_rmsnorm(norm, token) and mixer._fused_decode_ready(ms, token)
                 and mixer._native_decode_ready(token)) or mixer._forward_hooks or mixer._forward_pre_hooks:
             return None

@@ -3,6 +3,7 @@
 // A launch from Python cost 15 to 30 us of interpreter time (argument conversion of up to 40 ctypes arguments, device
 // guard, stream lookup, output allocation); the same work takes 2 to 4 us here.  Every function allocates its outputs
 // and scratch with torch, launches on torch's current stream and turns status codes into exceptions.
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -10,6 +11,8 @@
 
 #include "../../include/slinoss_b200.h"
 #include "host_abi.h"
+
+namespace py = pybind11;
 
 namespace {
 
@@ -370,6 +373,105 @@ Tensor ffn_token(const Tensor& x, const Tensor& norm_w, float eps, const Tensor&
   const Tensor hidden = linear_rows(call, x, Norm{norm_w, eps}, w1, b1, kind == 1 ? sl::LINEAR_SWIGLU : sl::LINEAR_GELU, {}, {});
   return linear_rows(call, hidden, Norm{}, w2, b2, sl::LINEAR_NONE, x, {});
 }
+// One token of a mixer, or of a whole block, without Python per launch.  A plan holds the parameters of one module (the
+// tensors themselves, so data that moves or changes type is seen) and a list of guards: dictionary entries that must still be
+// the objects they were, and dictionaries that must still be empty (hooks, overrides).  Checking the guards costs 2 us, what
+// they replace - attribute lookups, conversions of 30 arguments, checks of every tensor - cost 25 us per block.
+class TokenPlan {
+ public:
+  // params: in_w dw_w dw_b dt alpha theta_mod theta theta_sign d_skip norm_w out_w out_b; branch: pre_norm [ffn_norm w1 b1 w2 b2]
+  TokenPlan(std::vector<py::tuple> same, std::vector<py::dict> empty, std::vector<OptT> params, std::vector<OptT> branch,
+            std::vector<double> eps, const Config& cfg, std::array<int64_t, 5> dims, int ffn_kind)
+      : same_(std::move(same)), empty_(std::move(empty)), p_(std::move(params)), b_(std::move(branch)), eps_(std::move(eps)),
+        cfg_(config_of(cfg)), heads_(dims[0]), groups_(dims[1]), P_(dims[2]), N_(dims[3]), d_conv_(dims[4]), ffn_kind_(ffn_kind) {
+    if (p_.size() != 12 || (b_.size() != 0 && b_.size() != 1 && b_.size() != 6) || eps_.size() != 3)
+      throw pybind11::value_error("bad plan.");
+  }
+
+  bool valid() const {
+    for (const auto& g : same_)
+      if (PyDict_GetItem(PyTuple_GET_ITEM(g.ptr(), 0), PyTuple_GET_ITEM(g.ptr(), 1)) != PyTuple_GET_ITEM(g.ptr(), 2)) return false;
+    for (const auto& d : empty_)
+      if (PyDict_Size(d.ptr()) != 0) return false;
+    return true;
+  }
+
+  // None where the call is not the plain one; else (out, next b_prev, workspace)
+  py::object step(const Tensor& x, const OptT& conv, const OptT& state, const OptT& b_prev, const OptT& u_prev,
+                  const OptT& workspace) const {
+    if (at::GradMode::is_enabled() || at::autocast::is_autocast_enabled(at::kCUDA) || !x.is_cuda() || x.dim() != 2) return py::none();
+    const auto type = x.scalar_type();
+    const int64_t M = x.size(0), D = x.size(1), C = heads_ * P_;
+    if ((type != at::kBFloat16 && type != at::kHalf) || M < 1 || M > 64 || x.stride(1) != 1 || x.stride(0) % 8 != 0) return py::none();
+    auto is = [&](const OptT& t, at::ScalarType ty, at::IntArrayRef shape) {
+      return t && t->scalar_type() == ty && t->device() == x.device() && t->is_contiguous() && t->sizes() == shape;
+    };
+    const int64_t O = 2 * C + 3 * heads_ + 4 * groups_ * N_;
+    bool ok = is(p_[0], type, {O, D}) && is(p_[1], type, {C, d_conv_}) && is(p_[2], type, {C}) && is(p_[9], type, {C}) &&
+              is(p_[10], type, {D, C}) && (!p_[11] || is(p_[11], type, {D})) && is(p_[8], at::kFloat, {heads_});
+    for (int i = 3; i < 8; ++i) ok = ok && is(p_[i], at::kFloat, {heads_});
+    ok = ok && is(conv, type, {M, C, d_conv_ - 1}) && is(state, at::kFloat, {M, heads_, P_, 2 * N_}) &&
+         is(b_prev, type, {M, groups_, 2 * N_}) && is(u_prev, type, {M, heads_, P_});
+    const bool block = !b_.empty(), ffn = b_.size() == 6;
+    int64_t F = 0;
+    if (block) ok = ok && is(b_[0], type, {D});
+    if (ok && ffn) {
+      F = b_[4] ? b_[4]->size(1) : 0;
+      const int64_t wide = ffn_kind_ == 1 ? 2 * F : F;
+      ok = is(b_[1], type, {D}) && is(b_[2], type, {wide, D}) && (!b_[3] || is(b_[3], type, {wide})) && is(b_[4], type, {D, F}) &&
+           (!b_[5] || is(b_[5], type, {D}));
+    }
+    const int io = code_of(type);
+    ok = ok && sl::skinny_supported(M, D, O, io) && sl::skinny_supported(M, C, D, io) && (!ffn || sl::skinny_supported(M, F, D, io));
+    if (!ok) return py::none();
+
+    Call call(x);
+    const auto st = static_cast<cudaStream_t>(call.stream());
+    // scratch: the step's own, the projection, the residual stream between the branches, the hidden row
+    const int64_t e = 2;
+    auto up = [](int64_t n) { return (n + 255) / 256 * 256; };
+    const int64_t n_step = up(sl_mixer_decode_step_workspace_bytes(M, heads_, P_)), n_proj = up(M * O * e), n_mid = up(M * D * e);
+    const int64_t need = n_step + n_proj + n_mid + up(M * F * e);
+    const Tensor ws = workspace && workspace->numel() >= need && workspace->device() == x.device() ? *workspace : call.bytes(need);
+    auto* const base = static_cast<uint8_t*>(ws.data_ptr());
+    void *const proj = base + n_step, *const mid = base + n_step + n_proj, *const hidden = base + n_step + n_proj + n_mid;
+    const Tensor out = call.empty({M, D}, type);
+    const Tensor b_next = groups_ == heads_ ? *b_prev : at::empty_like(*b_prev);
+
+    const sl::SkinnyArgs in{ptr(x), x.stride(0), block ? ptr(b_[0]) : nullptr, (float)eps_[0], nullptr, 0, ptr(p_[0]), nullptr, nullptr,
+                            proj, (int)M, (int)D, (int)O, sl::LINEAR_NONE, io};
+    check(sl::skinny_linear(in, st), "skinny_linear");
+    const auto* row = static_cast<const uint8_t*>(proj);
+    const sl::MixerStepArgs a{row, row + C * e, row + 2 * C * e, row + (2 * C + 3 * heads_) * e, O, O, O, O, ptr(p_[1]), ptr(p_[2]),
+                              mptr(conv), (int)d_conv_, fptr(p_[3]), fptr(p_[4]), fptr(p_[5]), fptr(p_[6]), fptr(p_[7]), &cfg_,
+                              fptr(p_[8]), mfptr(state), ptr(b_prev), mptr(b_next), mptr(u_prev), base, (size_t)n_step, (int)M,
+                              (int)heads_, (int)groups_, (int)P_, (int)N_, io};
+    check(sl::mixer_step_launch(a, st), "mixer_step");
+    const Tensor rows = block && x.stride(0) != D ? x.contiguous() : x;
+    const sl::SkinnyArgs o{base, C, ptr(p_[9]), (float)eps_[1], sl::step_partials(base, M, heads_, P_), (int)(8 * heads_), ptr(p_[10]),
+                           ptr(p_[11]), block ? ptr(rows) : nullptr, ffn ? mid : mptr(out), (int)M, (int)C, (int)D, sl::LINEAR_NONE, io};
+    check(sl::skinny_linear(o, st), "skinny_linear");
+    if (ffn) {
+      const sl::SkinnyArgs f1{mid, D, ptr(b_[1]), (float)eps_[2], nullptr, 0, ptr(b_[2]), ptr(b_[3]), nullptr, hidden, (int)M, (int)D,
+                              (int)F, ffn_kind_ == 1 ? sl::LINEAR_SWIGLU : sl::LINEAR_GELU, io};
+      check(sl::skinny_linear(f1, st), "skinny_linear");
+      const sl::SkinnyArgs f2{hidden, F, nullptr, 0.f, nullptr, 0, ptr(b_[4]), ptr(b_[5]), mid, mptr(out), (int)M, (int)F, (int)D,
+                              sl::LINEAR_NONE, io};
+      check(sl::skinny_linear(f2, st), "skinny_linear");
+    }
+    return py::make_tuple(out, b_next, ws);
+  }
+
+ private:
+  std::vector<py::tuple> same_;    // (dict, key, value)
+  std::vector<py::dict> empty_;
+  std::vector<OptT> p_, b_;
+  std::vector<double> eps_;        // pre-norm, mixer norm, FFN norm
+  sl_scanprep_config cfg_;
+  int64_t heads_, groups_, P_, N_, d_conv_;
+  int ffn_kind_;
+};
+
 // ---- the whole mixer over a sequence ------------------------------------------------------------------------------------
 // in_proj writes one buffer of rows [gate C | value C | params 3H | bc 4GN]; the kernels read their columns through the row
 // stride, and the backward writes the four gradients into a buffer of the same layout, so each direction of in_proj is one
@@ -688,4 +790,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("mixer_infer", &mixer_infer);
   m.def("mixer_token", &mixer_token);
   m.def("ffn_token", &ffn_token);
+  // (a copied or unpickled module makes a plan of its own)
+  py::class_<TokenPlan>(m, "TokenPlan")
+      .def(py::init<std::vector<py::tuple>, std::vector<py::dict>, std::vector<OptT>, std::vector<OptT>, std::vector<double>,
+                    const Config&, std::array<int64_t, 5>, int>())
+      .def("valid", &TokenPlan::valid)
+      .def("step", &TokenPlan::step)
+      .def("__deepcopy__", [](const TokenPlan&, py::dict) { return py::none(); })
+      .def("__reduce__", [](const TokenPlan&) { return py::make_tuple(py::type::of(py::none()), py::tuple()); });
 }

@@ -51,7 +51,7 @@ struct SkinnyArgs {
   void* out;              // (M, O) dense
   int M, K, O, act, io_dtype;
 };
-bool skinny_supported(int M, int K, int O, int io_dtype);
+SL_API bool skinny_supported(int M, int K, int O, int io_dtype);
 SL_API int skinny_linear(const SkinnyArgs& a, cudaStream_t st);
 
 // ---- scan preparation and mixer tail on strided rows ---------------------------------------------------------------------

@@ -29,6 +29,24 @@ def _norm_eps(norm: nn.RMSNorm) -> float:
     return norm.eps if norm.eps is not None else torch.finfo(norm.weight.dtype).eps
 
 
+@_C.opaque
+def planned_step(module: nn.Module, token: torch.Tensor, state: SLinOSSMixerState, make):
+    """One token through the module's native plan (made by ``make`` and kept while its guards hold), ``state`` updated in
+    place; None where the call needs the composed path."""
+    plan = module.__dict__.get("_token_plan")
+    if plan is None or not plan.valid():
+        plan = make()
+        if plan is None:
+            return None
+        module.__dict__["_token_plan"] = plan
+    scan = state.scan
+    done = plan.step(token, state.conv, scan.state, scan.b_prev, scan.u_prev, state.__dict__.get("_plan_workspace"))
+    if done is None:
+        return None
+    out, scan.b_prev, state._plan_workspace = done
+    return out
+
+
 class SLinOSSMixer(nn.Module):
     def __init__(self, d_model: int, *, d_state: int = 128, expand: float = 2, d_head: int = 64,
                  d_conv: int = 4, chunk_size: int = 64, bc_groups: int | None = None,
@@ -221,6 +239,10 @@ class SLinOSSMixer(nn.Module):
              inplace: bool | None = None):
         """One decode token.  ``x (batch, d_model)`` or ``(batch, 1, d_model)``."""
         squeeze = x.ndim == 2
+        if squeeze and state is not None and inplace is not False and x.is_cuda and x.shape[1] == self.d_model:
+            y = planned_step(self, x, state, self._make_token_plan)
+            if y is not None:
+                return y, state
         if squeeze:
             x = x.unsqueeze(1)
         _require(x.ndim == 3 and x.shape[1] == 1 and x.shape[-1] == self.d_model,
@@ -259,6 +281,40 @@ class SLinOSSMixer(nn.Module):
                 and not out._forward_hooks and not out._forward_pre_hooks and token.stride(1) == 1
                 and w_in.dtype == token.dtype and w_out.dtype == token.dtype and w_in.device == token.device
                 and w_in.is_contiguous() and not torch.is_autocast_enabled())
+
+    def _plan_guards(self):
+        """What a native token plan of this module relies on: (dictionary, key, object) entries, and dictionaries that
+        stay empty."""
+        sp, out = self.scanprep, self.out_proj
+        mine, kids = self.__dict__, self._modules
+        same = [(kids, n, kids[n]) for n in ("scanprep", "in_proj", "out_norm", "out_proj")]
+        same += [(mine, "decode_backend", self.decode_backend)]
+        for m, names in ((self, ("dw_weight", "dw_bias", "d_skip")), (self.in_proj, ("weight",)), (out, ("weight", "bias")),
+                         (self.out_norm, ("weight",)), (sp, ("dt_bias", "alpha_bias", "theta_mod_bias", "theta_bias"))):
+            same += [(m._parameters, n, m._parameters[n]) for n in names]
+        same.append((sp._buffers, "theta_sign", sp._buffers["theta_sign"]))
+        same += [(sp.__dict__, n, sp.__dict__[n]) for n in _C.CONFIG_FIELDS]
+        empty = [self.decode_backend.__dict__, out._forward_hooks, out._forward_pre_hooks]
+        return same, empty
+
+    def _make_token_plan(self, branch=(), guards=((), ()), pre_eps=0.0, ffn_eps=0.0, ffn_kind=0):
+        """``branch``: the norm in front of the mixer (the residual is then added), and the FFN branch behind it.  None if
+        a stage is not the package's own."""
+        out, sp = self.out_proj, self.scanprep
+        if not (type(self.decode_backend) is B200MixerDecodeBackend and type(out) is nn.Linear and self.d_conv <= 4
+                and self.out_norm.weight is not None and not self.decode_backend.__dict__
+                and all(n in sp.__dict__ for n in _C.CONFIG_FIELDS)):
+            return None
+        same, empty = self._plan_guards()
+        if any(len(d) for d in (*empty, *guards[1])):
+            return None
+        p, mine = sp._parameters, self._parameters
+        params = [self.in_proj.weight, mine["dw_weight"], mine["dw_bias"], p["dt_bias"], p["alpha_bias"],
+                  p["theta_mod_bias"], p["theta_bias"], sp._buffers["theta_sign"], mine["d_skip"], self.out_norm.weight,
+                  out.weight, out.bias]
+        return _C.host().TokenPlan([*same, *guards[0]], [*empty, *guards[1]], params, list(branch),
+                                   [pre_eps, _norm_eps(self.out_norm), ffn_eps], [getattr(sp, n) for n in _C.CONFIG_FIELDS],
+                                   [self.n_heads, self.bc_groups, self.d_head, self.d_state, self.d_conv], ffn_kind)
 
     @_C.opaque
     def decode_native(self, token: torch.Tensor, state: SLinOSSMixerState, *, pre_norm=None, residual=None,

@@ -1,6 +1,9 @@
 """The native decode step of a block (small-batch linear kernels, pipelined state update) against the composed path:
 library GEMMs, row kernels, and conv, scan preparation, decode and tail as launches of their own."""
 
+import copy
+import pickle
+
 import pytest
 import torch
 
@@ -60,3 +63,49 @@ def test_a_decode_token_is_bit_reproducible():
                 y, state = blk.step(x, state)
             runs.append((y, state.mixer.scan.state))
     assert all(torch.equal(a, b) for a, b in zip(*runs))
+
+
+def test_a_token_plan_notices_what_it_relies_on():
+    """A replaced or converted parameter, a hook, a swapped child and a copied module all take effect at the next token."""
+    blk = _block(128, 64, None, "gelu", True, torch.bfloat16)
+    x = torch.randn(3, 128, device=DEV, dtype=torch.bfloat16)
+
+    def token(b):
+        with torch.no_grad():
+            return b.step(x, b.init_decode_state(3))[0]
+
+    first = token(blk)
+    assert torch.equal(token(blk), first) and "_token_plan" in blk.__dict__
+    assert torch.equal(token(copy.deepcopy(blk)), first) and torch.equal(token(pickle.loads(pickle.dumps(blk))), first)
+    weight = blk.mixer.out_proj.weight
+    blk.mixer.out_proj.weight = torch.nn.Parameter(torch.zeros_like(weight))
+    assert not torch.equal(token(blk), first)
+    blk.mixer.out_proj.weight = weight
+    assert torch.equal(token(blk), first)
+    calls = []
+    handle = blk.ffn.register_forward_hook(lambda *a: calls.append(1))
+    assert rel(token(blk), first) <= 2e-2 and calls
+    handle.remove()
+    ffn, blk.ffn = blk.ffn, _block(128, 64, None, "gelu", True, torch.bfloat16).ffn
+    with torch.no_grad():
+        blk.ffn.out_proj.bias.add_(1.0)
+    assert (token(blk).float() - first.float()).abs().min() > 0.5
+    blk.ffn = ffn
+    blk.to(torch.float16)
+    x = x.to(torch.float16)
+    assert rel(token(blk), first) <= 2e-2
+
+
+@pytest.mark.parametrize("batch", [1, 5, 64, 65])
+def test_mixer_token_by_plan_equals_the_composed_token(batch, monkeypatch):
+    torch.manual_seed(2)
+    mixer = sb.SLinOSSMixer(192, d_state=64, d_head=64, bc_groups=2, device=DEV, dtype=torch.bfloat16)
+    x = torch.randn(3, batch, 192, device=DEV, dtype=torch.bfloat16)
+    with torch.no_grad():
+        a, b = mixer.init_decode_state(batch), mixer.init_decode_state(batch)
+        got = [mixer.step(t, a)[0] for t in x]
+        monkeypatch.setattr(type(mixer), "_make_token_plan", lambda *a, **k: None)
+        mixer.__dict__.pop("_token_plan", None)
+        want = [mixer.step(t, b)[0] for t in x]
+    assert rel(torch.stack(got), torch.stack(want)) <= 2e-2 and rel(a.scan.state, b.scan.state) <= 2e-2
+    assert rel(a.scan.b_prev, b.scan.b_prev) <= 2e-2 and rel(a.conv, b.conv) <= 2e-2
