@@ -367,9 +367,14 @@ def rmsnorm_fwd(x, weight, eps):
     return host().rmsnorm_fwd(x, weight, eps)
 
 
-def rmsnorm_bwd(x, weight, eps, d_out):
-    """Returns ``(d_x, d_weight float32)``."""
-    return host().rmsnorm_bwd(x, weight, eps, d_out)
+def rmsnorm_bwd(x, weight, eps, d_out, *, extra=None, as_rows_type=False):
+    """Returns ``(d_x (+ extra), d_weight float32)``, the latter in x's type with ``as_rows_type``."""
+    return host().rmsnorm_bwd(x, weight, eps, d_out, extra, as_rows_type)
+
+
+def column_sum(x):
+    """Sum over all but the last axis in float32, rounded once to x's type."""
+    return host().column_sum(x)
 
 
 def ffn_activation_fwd(projected, kind: str):

@@ -4,6 +4,7 @@
 // kernels of slinoss/ops/block/cute/norm.py:85,173 and activation.py:78,153.  The two GEMMs stay library
 // calls in the caller.  All four kernels are HBM-bound: 16-byte accesses, one pass over their rows.
 #include "common.cuh"
+#include "host_abi.h"
 
 namespace sl {
 namespace {
@@ -61,7 +62,8 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ 
 template <typename T, int MAXP>
 __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w,
                                                           const T* __restrict__ dy, T* __restrict__ dx,
-                                                          float* __restrict__ dw, long long rows, int C, float eps) {
+                                                          float* __restrict__ dw, double* __restrict__ dw64,
+                                                          const T* __restrict__ extra, long long rows, int C, float eps) {
   constexpr int V = Vec16<T>::N;
   extern __shared__ __align__(16) unsigned char s_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -112,6 +114,12 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_kernel(const T* __restrict
         }
 #pragma unroll
         for (int k = 0; k < V; ++k) o[k] = rstd * (gv[k] * wv[k] - xv[k] * coef);
+        if (extra) {
+          float ev[V];
+          load16<T>(extra + row * C + pc * V, ev);
+#pragma unroll
+          for (int k = 0; k < V; ++k) o[k] += ev[k];
+        }
         store16<T>(dx + row * C + pc * V, o);
       }
     }
@@ -120,7 +128,59 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_kernel(const T* __restrict
   for (int c = threadIdx.x; c < C; c += blockDim.x) {
     float v = 0.f;
     for (int q = 0; q < nw; ++q) v += s_dw[(size_t)q * C + c];
-    atomicAdd(dw + c, v);
+    if (dw64) atomicAdd(dw64 + c, (double)v);   // the order of these adds is lost in the rounding to the result's type
+    else atomicAdd(dw + c, v);
+  }
+}
+
+// Column sums of a (rows, C) matrix, in an order that does not depend on the schedule: each CTA sums a run of rows of 32 V
+// columns (a warp per row, 16 bytes a lane) to a row of float32 partials, the second kernel sums those.
+template <typename T>
+__global__ void __launch_bounds__(256) column_partials_kernel(const T* __restrict__ x, float* __restrict__ partial, long long rows,
+                                                              int C, int run) {
+  constexpr int V = Vec16<T>::N;
+  __shared__ float s_sum[8][32 * V + 4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = blockIdx.x * 32 * V, c = c0 + lane * V;
+  const long long r0 = (long long)blockIdx.y * run, r1 = min(rows, r0 + run);
+  float acc[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) acc[k] = 0.f;
+  if (c < C) {
+#pragma unroll 4
+    for (long long r = r0 + warp; r < r1; r += 8) {
+      float v[V];
+      load16<T>(x + r * C + c, v);
+#pragma unroll
+      for (int k = 0; k < V; ++k) acc[k] += v[k];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < V; ++k) s_sum[warp][lane * V + k] = acc[k];
+  __syncthreads();
+  for (int i = threadIdx.x; i < 32 * V && c0 + i < C; i += blockDim.x) {
+    float v = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v += s_sum[q][i];
+    partial[(size_t)blockIdx.y * C + c0 + i] = v;
+  }
+}
+// out[c] = sum of n partial rows: 32 columns per CTA, 8 warps share the rows
+template <typename T>
+__global__ void __launch_bounds__(256) sum_partials_kernel(const float* __restrict__ partial, T* __restrict__ out, int n, int C) {
+  __shared__ float s_sum[8][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+  float v = 0.f;
+  if (c < C) {
+#pragma unroll 8
+    for (int r = warp; r < n; r += 8) v += partial[(size_t)r * C + c];
+  }
+  s_sum[warp][lane] = v;
+  __syncthreads();
+  if (warp == 0 && c < C) {
+    v = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v += s_sum[q][lane];
+    out[c] = from_f32<T>(v);
   }
 }
 
@@ -216,13 +276,13 @@ extern "C" int sl_rmsnorm_fwd(const void* x, const void* weight, float eps, void
   return launch_status();
 }
 
-extern "C" int sl_rmsnorm_bwd(const void* x, const void* weight, float eps, const void* d_out, void* d_x,
-                              float* d_weight, long long rows, int C, int io_dtype, void* stream) {
-  using namespace sl;
-  if (!x || !weight || !d_out || !d_x || !d_weight) return SL_ERR_NULL_POINTER;
+namespace sl {
+// d_weight: float32 accumulators, or float64 ones (weight64); extra (or null) is added to d_x
+int rmsnorm_bwd(const void* x, const void* weight, float eps, const void* d_out, const void* extra, void* d_x, float* d_weight,
+                double* weight64, long long rows, int C, int io_dtype, cudaStream_t st) {
+  if (!x || !weight || !d_out || !d_x || !(d_weight || weight64)) return SL_ERR_NULL_POINTER;
   if (!dtype_ok(io_dtype)) return SL_ERR_UNSUPPORTED;
-  if (!rows_ok(rows, C, io_dtype, x, d_x) || !aligned(weight, 16) || !aligned(d_out, 16)) return SL_ERR_BAD_SHAPE;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (!rows_ok(rows, C, io_dtype, x, d_x) || !aligned(weight, 16) || !aligned(d_out, 16) || !aligned(extra, 16)) return SL_ERR_BAD_SHAPE;
   const long long want = (rows + 7) / 8;
   const bool narrow = C / (io_dtype == SL_F32 ? 4 : 8) <= 32 * RMS_MAXP_NARROW;
   const long long cap = narrow ? 148 * 4 : 148 * 2;   // CTAs that walk the rows: all resident at once
@@ -235,10 +295,40 @@ extern "C" int sl_rmsnorm_bwd(const void* x, const void* weight, float eps, cons
       return SL_ERR_LAUNCH_FAILED;
     kern<<<grid, 256, smem, st>>>(
         reinterpret_cast<const T*>(x), reinterpret_cast<const T*>(weight), reinterpret_cast<const T*>(d_out),
-        reinterpret_cast<T*>(d_x), d_weight, rows, C, eps);
+        reinterpret_cast<T*>(d_x), d_weight, weight64, reinterpret_cast<const T*>(extra), rows, C, eps);
   });
   note_launches(1);
   return launch_status();
+}
+
+// runs of rows: 8 at least per warp, and about two CTAs per SM
+static int column_runs(long long rows, int C, int io) {
+  const int cols = (C + 32 * (io == SL_F32 ? 4 : 8) - 1) / (32 * (io == SL_F32 ? 4 : 8));
+  const long long most = (rows + 63) / 64, want = (296 + cols - 1) / cols;
+  return (int)(most < want ? most : want);
+}
+size_t column_sum_partials(long long rows, int C, int io_dtype) { return (size_t)column_runs(rows, C, io_dtype) * C; }
+int column_sum(const void* x, void* out, float* partial, long long rows, int C, int io_dtype, cudaStream_t st) {
+  if (!x || !out || !partial) return SL_ERR_NULL_POINTER;
+  const int V = io_dtype == SL_F32 ? 4 : 8, runs = column_runs(rows, C, io_dtype);
+  if (rows < 1 || C < 1 || C % V || !aligned(x, 16)) return SL_ERR_BAD_SHAPE;
+  const int run = (int)((rows + runs - 1) / runs);
+  SL_DISPATCH_DTYPE(io_dtype, T, {
+    column_partials_kernel<T><<<dim3((C + 32 * V - 1) / (32 * V), runs), 256, 0, st>>>(reinterpret_cast<const T*>(x), partial, rows, C, run);
+  });
+  note_launches(1);
+  SL_DISPATCH_DTYPE(io_dtype, T, {
+    sum_partials_kernel<T><<<(C + 31) / 32, 256, 0, st>>>(partial, reinterpret_cast<T*>(out), runs, C);
+  });
+  note_launches(1);
+  return launch_status();
+}
+}  // namespace sl
+
+extern "C" int sl_rmsnorm_bwd(const void* x, const void* weight, float eps, const void* d_out, void* d_x,
+                              float* d_weight, long long rows, int C, int io_dtype, void* stream) {
+  return sl::rmsnorm_bwd(x, weight, eps, d_out, nullptr, d_x, d_weight, nullptr, rows, C, io_dtype,
+                         reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int sl_ffn_activation_fwd(const void* projected, void* hidden, long long rows, int hidden_dim,

@@ -272,13 +272,24 @@ Tensor rmsnorm_fwd(const Tensor& x, const Tensor& w, float eps) {
   check(sl_rmsnorm_fwd(ptr(x), ptr(w), eps, mptr(out), x.numel() / C, C, code_of(x.scalar_type()), call.stream()), "sl_rmsnorm_fwd");
   return out;
 }
-std::tuple<Tensor, Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, float eps, const Tensor& dy) {
-  Call call(x, w, dy);
+// ``extra`` is added to dx
+std::tuple<Tensor, Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, float eps, const Tensor& dy, const OptT& extra, bool as_rows_type) {
+  Call call(x, w, dy, extra);
   const int64_t C = x.size(-1);
-  Tensor dx = at::empty_like(x), dw = call.zeros({C}, at::kFloat);
-  check(sl_rmsnorm_bwd(ptr(x), ptr(w), eps, ptr(dy), mptr(dx), mfptr(dw), x.numel() / C, C, code_of(x.scalar_type()), call.stream()),
+  Tensor dx = at::empty_like(x), dw = call.zeros({C}, at::kDouble);
+  check(sl::rmsnorm_bwd(ptr(x), ptr(w), eps, ptr(dy), ptr(extra), mptr(dx), nullptr, dw.data_ptr<double>(), x.numel() / C, C,
+                        code_of(x.scalar_type()), static_cast<cudaStream_t>(call.stream())),
         "sl_rmsnorm_bwd");
-  return {dx, dw};
+  return {dx, dw.to(as_rows_type ? x.scalar_type() : at::kFloat)};
+}
+Tensor column_sum(const Tensor& x) {
+  Call call(x);
+  const int64_t C = x.size(-1), rows = x.numel() / C;
+  const int io = code_of(x.scalar_type());
+  Tensor out = call.empty({C}, x.scalar_type());
+  const Tensor partial = call.empty({(int64_t)sl::column_sum_partials(rows, C, io)}, at::kFloat);
+  check(sl::column_sum(ptr(x), mptr(out), mfptr(partial), rows, C, io, static_cast<cudaStream_t>(call.stream())), "column_sum");
+  return out;
 }
 Tensor ffn_act_fwd(const Tensor& proj, int kind) {
   Call call(proj);
@@ -779,6 +790,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("tail_bwd", &tail_bwd);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
+  m.def("column_sum", &column_sum);
   m.def("ffn_act_fwd", &ffn_act_fwd);
   m.def("ffn_act_bwd", &ffn_act_bwd);
   m.def("ce_fwd", &ce_fwd);

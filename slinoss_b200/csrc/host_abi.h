@@ -88,6 +88,14 @@ SL_API int mixer_tail_bwd(const void* Y, const void* gate, int64_t gate_stride, 
                           int64_t d_gate_stride, void* d_skip_input, float* d_d_skip, float* d_norm_weight, int batch, int heads,
                           int T, int P, int io_dtype, cudaStream_t st);
 
+// ---- row kernels whose sums over rows do not depend on the schedule -----------------------------------------------------
+// d_weight float32 or weight64 (sums that rounding to a shorter type makes independent of their order): added to; extra
+// (rows, C) or null is added to d_x
+SL_API int rmsnorm_bwd(const void* x, const void* weight, float eps, const void* d_out, const void* extra, void* d_x, float* d_weight,
+                       double* weight64, long long rows, int C, int io_dtype, cudaStream_t st);
+SL_API size_t column_sum_partials(long long rows, int C, int io_dtype);
+SL_API int column_sum(const void* x, void* out, float* partial, long long rows, int C, int io_dtype, cudaStream_t st);
+
 // ---- language-model training step ------------------------------------------------------------------------------------
 SL_API int cross_entropy_fwd(const void* logits, const int64_t* target, float* loss, float* lse, int64_t rows, int V, int io,
                              cudaStream_t st);

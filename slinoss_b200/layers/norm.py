@@ -22,7 +22,7 @@ class _RMSNormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d_out):
         x, weight = ctx.saved_tensors
-        d_x, d_w = _C.rmsnorm_bwd(x, weight, ctx.eps, d_out.contiguous())
+        d_x, d_w = _C.rmsnorm_bwd(x, weight, ctx.eps, d_out.contiguous(), as_rows_type=True)
         return (d_x if ctx.needs_input_grad[0] else None,
                 d_w.to(weight.dtype) if ctx.needs_input_grad[1] else None, None)
 
