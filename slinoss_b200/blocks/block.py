@@ -55,6 +55,14 @@ def _ffn_token(x, norm, ffn):
                                _C.FFN_KINDS[ffn.kind])
 
 
+@_C.opaque
+def _ffn_train(x, norm, ffn):
+    """``x + ffn(norm(x))`` as one autograd node."""
+    w1, w2 = ffn.in_proj._parameters, ffn.out_proj._parameters
+    return _C.host().ffn_train(x, norm.weight, w1["weight"], w1["bias"], w2["weight"], w2["bias"], _norm_eps(norm),
+                               _C.FFN_KINDS[ffn.kind])
+
+
 class SLinOSSBlock(nn.Module):
     def __init__(self, config: SLinOSSBlockConfig, *, device=None, dtype=None) -> None:
         super().__init__()
@@ -87,8 +95,22 @@ class SLinOSSBlock(nn.Module):
     def _add(self, residual, branch):
         return residual_add(residual, branch, self.residual_in_fp32)
 
+    def _native_training_ready(self, x) -> bool:
+        """The mixer branch with its norm and residual as one node: gradients wanted, one 16-bit type, no dropout, no hooks."""
+        mixer = self.mixer
+        return (x.is_cuda and torch.is_grad_enabled() and (self.residual_dropout <= 0.0 or not self.training)
+                and type(mixer) is SLinOSSMixer and not mixer._forward_hooks and not mixer._forward_pre_hooks
+                and not mixer._backward_hooks and not mixer._backward_pre_hooks and _plain_rmsnorm(self.mixer_norm, x)
+                and mixer._native_forward_ready(x, None))
+
     def _ffn_residual(self, x):
         no_drop = self.residual_dropout <= 0.0 or not self.training
+        ffn, norm = self.ffn, self.ffn_norm
+        if no_drop and self.ffn_remat == "none" and x.is_cuda and torch.is_grad_enabled() and type(ffn) is SLinOSSMLP \
+                and not (ffn._forward_hooks or ffn._forward_pre_hooks or ffn._backward_hooks or ffn._backward_pre_hooks) \
+                and _plain_rmsnorm(norm, x) and _plain_linear(ffn.in_proj, x) and _plain_linear(ffn.out_proj, x) \
+                and ffn_residual_supported(x, norm, ffn):
+            return _ffn_train(x, norm, ffn)
         if no_drop and self.ffn_remat != "none" and ffn_residual_supported(x, self.ffn_norm, self.ffn):
             return ffn_residual(x, self.ffn_norm, self.ffn, residual_in_fp32=self.residual_in_fp32,
                                 remat=self.ffn_remat)
@@ -98,6 +120,9 @@ class SLinOSSBlock(nn.Module):
                 context=None, sequence_group=None):
         if x.ndim != 3 or x.shape[-1] != self.d_model:
             raise ValueError(f"Expected x shape (batch, T, {self.d_model}), got {tuple(x.shape)}.")
+        if state is None and not return_state and sequence_group is None and self._native_training_ready(x):
+            out = self.mixer._forward_native(x, self.mixer._native_parameters(), None, False, pre_norm=self.mixer_norm)
+            return out if self.ffn is None else self._ffn_residual(out)
         extra = {} if sequence_group is None else {"sequence_group": sequence_group}
         mixed = self.mixer(apply_norm(self.mixer_norm, x),
                            state=None if state is None else state.mixer, return_state=return_state, **extra)

@@ -63,15 +63,17 @@ template <typename T, int MAXP>
 __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w,
                                                           const T* __restrict__ dy, T* __restrict__ dx,
                                                           float* __restrict__ dw, double* __restrict__ dw64,
-                                                          const T* __restrict__ extra, long long rows, int C, float eps) {
+                                                          const T* __restrict__ extra, double* __restrict__ extra_sum,
+                                                          long long rows, int C, float eps) {
   constexpr int V = Vec16<T>::N;
   extern __shared__ __align__(16) unsigned char s_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   float* s_dw = reinterpret_cast<float*>(s_raw);                        // [nw][C]
-  uint4* s_w = reinterpret_cast<uint4*>(s_raw + (size_t)nw * C * sizeof(float));   // [C / V]
+  const int kept = extra_sum ? 2 * nw : nw;                             // rows of sums: dw, then those of extra
+  uint4* s_w = reinterpret_cast<uint4*>(s_raw + (size_t)kept * C * sizeof(float));   // [C / V]
   float* my_dw = s_dw + (size_t)warp * C;
   const int pieces = C / V;
-  for (int c = threadIdx.x; c < nw * C; c += blockDim.x) s_dw[c] = 0.f;
+  for (int c = threadIdx.x; c < kept * C; c += blockDim.x) s_dw[c] = 0.f;
   for (int c = threadIdx.x; c < pieces; c += blockDim.x) s_w[c] = reinterpret_cast<const uint4*>(w)[c];
   __syncthreads();
   for (long long row = (long long)blockIdx.x * nw + warp; row < rows; row += (long long)gridDim.x * nw) {
@@ -119,6 +121,11 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_kernel(const T* __restrict
           load16<T>(extra + row * C + pc * V, ev);
 #pragma unroll
           for (int k = 0; k < V; ++k) o[k] += ev[k];
+          if (extra_sum) {
+            float* es = my_dw + (size_t)nw * C + pc * V;
+#pragma unroll
+            for (int k = 0; k < V; ++k) es[k] += ev[k];
+          }
         }
         store16<T>(dx + row * C + pc * V, o);
       }
@@ -130,6 +137,11 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_kernel(const T* __restrict
     for (int q = 0; q < nw; ++q) v += s_dw[(size_t)q * C + c];
     if (dw64) atomicAdd(dw64 + c, (double)v);   // the order of these adds is lost in the rounding to the result's type
     else atomicAdd(dw + c, v);
+    if (extra_sum) {
+      v = 0.f;
+      for (int q = nw; q < 2 * nw; ++q) v += s_dw[(size_t)q * C + c];
+      atomicAdd(extra_sum + c, (double)v);
+    }
   }
 }
 
@@ -247,6 +259,61 @@ __global__ void __launch_bounds__(256) ffn_act_bwd_kernel(const T* __restrict__ 
   }
 }
 
+// The activation's backward with the column sums of its result (the bias gradient of the projection): a CTA walks a run of rows
+// of 32 V columns, a warp per row, and adds its float32 sums to float64 accumulators once.  The elementwise kernel above followed by a
+// pass for the sums reads the result again (8192 x 2304: 24 + 15 us, now 24).
+template <typename T>
+__global__ void __launch_bounds__(256) ffn_act_bwd_sum_kernel(const T* __restrict__ proj, const T* __restrict__ dhid,
+                                                              T* __restrict__ dproj, double* __restrict__ sums, long long rows,
+                                                              int H, int kind, int run) {
+  constexpr int V = Vec16<T>::N;
+  __shared__ float s_sum[8][32 * V + 4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = blockIdx.x * 32 * V, c = c0 + lane * V;
+  const long long r0 = (long long)blockIdx.y * run, r1 = min(rows, r0 + run);
+  const size_t pitch = (size_t)(kind ? 2 : 1) * H;
+  float acc[V], acg[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) acc[k] = acg[k] = 0.f;
+  if (c < H) {
+#pragma unroll 2
+    for (long long r = r0 + warp; r < r1; r += 8) {
+      float a[V], d[V], o[V];
+      load16<T>(dhid + r * H + c, d);
+      load16<T>(proj + r * pitch + c, a);
+      if (kind == 0) {
+#pragma unroll
+        for (int k = 0; k < V; ++k) o[k] = d[k] * dgelu_tanh_f<sizeof(T) == 2>(a[k]);
+      } else {
+        float g[V], og[V];
+        load16<T>(proj + r * pitch + H + c, g);
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          const float sg = sigmoid_f(g[k]);
+          o[k] = d[k] * g[k] * sg;
+          og[k] = d[k] * a[k] * (sg + g[k] * sg * (1.f - sg));
+          acg[k] += og[k];
+        }
+        store16<T>(dproj + r * pitch + H + c, og);
+      }
+#pragma unroll
+      for (int k = 0; k < V; ++k) acc[k] += o[k];
+      store16<T>(dproj + r * pitch + c, o);
+    }
+  }
+  for (int part = 0; part <= kind; ++part) {
+#pragma unroll
+    for (int k = 0; k < V; ++k) s_sum[warp][lane * V + k] = part ? acg[k] : acc[k];
+    __syncthreads();
+    for (int i = threadIdx.x; i < 32 * V && c0 + i < H; i += blockDim.x) {
+      float v = 0.f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v += s_sum[q][i];
+      atomicAdd(sums + (size_t)part * H + c0 + i, (double)v);
+    }
+    __syncthreads();
+  }
+}
+
 constexpr int RMS_MAXP_NARROW = 2;   // rows up to 512 (256) channels keep the registers low
 constexpr int RMS_MAXP = 8;   // 16-byte pieces per lane: rows up to 8 * 32 * (4 or 8) channels
 
@@ -277,9 +344,11 @@ extern "C" int sl_rmsnorm_fwd(const void* x, const void* weight, float eps, void
 }
 
 namespace sl {
-// d_weight: float32 accumulators, or float64 ones (weight64); extra (or null) is added to d_x
+// d_weight: float32 accumulators, or float64 ones (weight64); extra (or null) is added to d_x, its column sums to extra_sum
+// (or null; up to 1024 columns, where the second row of sums per warp still leaves three CTAs per SM)
+bool rmsnorm_bwd_sums_extra(int C) { return C <= 1024; }
 int rmsnorm_bwd(const void* x, const void* weight, float eps, const void* d_out, const void* extra, void* d_x, float* d_weight,
-                double* weight64, long long rows, int C, int io_dtype, cudaStream_t st) {
+                double* weight64, double* extra_sum, long long rows, int C, int io_dtype, cudaStream_t st) {
   if (!x || !weight || !d_out || !d_x || !(d_weight || weight64)) return SL_ERR_NULL_POINTER;
   if (!dtype_ok(io_dtype)) return SL_ERR_UNSUPPORTED;
   if (!rows_ok(rows, C, io_dtype, x, d_x) || !aligned(weight, 16) || !aligned(d_out, 16) || !aligned(extra, 16)) return SL_ERR_BAD_SHAPE;
@@ -287,7 +356,8 @@ int rmsnorm_bwd(const void* x, const void* weight, float eps, const void* d_out,
   const bool narrow = C / (io_dtype == SL_F32 ? 4 : 8) <= 32 * RMS_MAXP_NARROW;
   const long long cap = narrow ? 148 * 4 : 148 * 2;   // CTAs that walk the rows: all resident at once
   const unsigned grid = (unsigned)(want < cap ? want : cap);
-  const size_t smem = (size_t)8 * C * sizeof(float) + (size_t)C * dtype_size(io_dtype);   // 8 warps' dw rows + w
+  if (extra_sum && (!extra || !rmsnorm_bwd_sums_extra(C))) return SL_ERR_UNSUPPORTED;
+  const size_t smem = (size_t)(extra_sum ? 16 : 8) * C * sizeof(float) + (size_t)C * dtype_size(io_dtype);   // 8 warps' rows + w
   SL_DISPATCH_DTYPE(io_dtype, T, {
     auto kern = narrow ? rmsnorm_bwd_kernel<T, RMS_MAXP_NARROW> : rmsnorm_bwd_kernel<T, RMS_MAXP>;
     if (smem > 48 * 1024 &&
@@ -295,17 +365,30 @@ int rmsnorm_bwd(const void* x, const void* weight, float eps, const void* d_out,
       return SL_ERR_LAUNCH_FAILED;
     kern<<<grid, 256, smem, st>>>(
         reinterpret_cast<const T*>(x), reinterpret_cast<const T*>(weight), reinterpret_cast<const T*>(d_out),
-        reinterpret_cast<T*>(d_x), d_weight, weight64, reinterpret_cast<const T*>(extra), rows, C, eps);
+        reinterpret_cast<T*>(d_x), d_weight, weight64, reinterpret_cast<const T*>(extra), extra_sum, rows, C, eps);
   });
   note_launches(1);
   return launch_status();
 }
 
-// runs of rows: 8 at least per warp, and about two CTAs per SM
+// runs of rows: 8 at least per warp, and about four CTAs per SM
 static int column_runs(long long rows, int C, int io) {
   const int cols = (C + 32 * (io == SL_F32 ? 4 : 8) - 1) / (32 * (io == SL_F32 ? 4 : 8));
-  const long long most = (rows + 63) / 64, want = (296 + cols - 1) / cols;
+  const long long most = (rows + 63) / 64, want = (592 + cols - 1) / cols;
   return (int)(most < want ? most : want);
+}
+int ffn_act_bwd_sum(const void* projected, const void* d_hidden, void* d_projected, double* sums, long long rows, int H, int kind,
+                    int io_dtype, cudaStream_t st) {
+  const int V = io_dtype == SL_F32 ? 4 : 8, runs = column_runs(rows, H, io_dtype);
+  if (rows < 1 || H < V || H % V || !aligned(projected, 16) || !aligned(d_hidden, 16) || !aligned(d_projected, 16)) return SL_ERR_BAD_SHAPE;
+  const int run = (int)((rows + runs - 1) / runs);
+  SL_DISPATCH_DTYPE(io_dtype, T, {
+    ffn_act_bwd_sum_kernel<T><<<dim3((H + 32 * V - 1) / (32 * V), runs), 256, 0, st>>>(
+        reinterpret_cast<const T*>(projected), reinterpret_cast<const T*>(d_hidden), reinterpret_cast<T*>(d_projected), sums, rows, H,
+        kind, run);
+  });
+  note_launches(1);
+  return launch_status();
 }
 size_t column_sum_partials(long long rows, int C, int io_dtype) { return (size_t)column_runs(rows, C, io_dtype) * C; }
 int column_sum(const void* x, void* out, float* partial, long long rows, int C, int io_dtype, cudaStream_t st) {
@@ -327,7 +410,7 @@ int column_sum(const void* x, void* out, float* partial, long long rows, int C, 
 
 extern "C" int sl_rmsnorm_bwd(const void* x, const void* weight, float eps, const void* d_out, void* d_x,
                               float* d_weight, long long rows, int C, int io_dtype, void* stream) {
-  return sl::rmsnorm_bwd(x, weight, eps, d_out, nullptr, d_x, d_weight, nullptr, rows, C, io_dtype,
+  return sl::rmsnorm_bwd(x, weight, eps, d_out, nullptr, d_x, d_weight, nullptr, nullptr, rows, C, io_dtype,
                          reinterpret_cast<cudaStream_t>(stream));
 }
 

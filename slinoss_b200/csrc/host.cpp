@@ -277,7 +277,7 @@ std::tuple<Tensor, Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, float e
   Call call(x, w, dy, extra);
   const int64_t C = x.size(-1);
   Tensor dx = at::empty_like(x), dw = call.zeros({C}, at::kDouble);
-  check(sl::rmsnorm_bwd(ptr(x), ptr(w), eps, ptr(dy), ptr(extra), mptr(dx), nullptr, dw.data_ptr<double>(), x.numel() / C, C,
+  check(sl::rmsnorm_bwd(ptr(x), ptr(w), eps, ptr(dy), ptr(extra), mptr(dx), nullptr, dw.data_ptr<double>(), nullptr, x.numel() / C, C,
                         code_of(x.scalar_type()), static_cast<cudaStream_t>(call.stream())),
         "sl_rmsnorm_bwd");
   return {dx, dw.to(as_rows_type ? x.scalar_type() : at::kFloat)};
@@ -521,7 +521,7 @@ struct MixerRun {
   OptT states, final_state, conv;
 };
 MixerRun mixer_run(const MixerShape& s, const MixerWeights& w, const Tensor& x, const OptT& conv_in, const OptT& z0, const OptT& Bp,
-                   const OptT& Up, bool save_states, bool want_state) {
+                   const OptT& Up, bool save_states, bool want_state, const OptT& residual = {}) {
   Call call(x, w.in_w, w.dw_w, w.dw_b, w.d_skip, w.norm_w, w.out_w, conv_in, z0, Bp, Up);
   for (const auto& t : w.bias) call.need(t);
   const auto type = x.scalar_type();
@@ -550,7 +550,7 @@ MixerRun mixer_run(const MixerShape& s, const MixerWeights& w, const Tensor& x, 
   check(sl_mixer_tail_fwd(ptr(r.Y), ptr(r.proj), s.pitch(), ptr(r.U), fptr(w.d_skip), ptr(w.norm_w), w.eps, mptr(r.normed), s.batch,
                           s.heads, s.T, s.P, code_of(type), st),
         "sl_mixer_tail_fwd");
-  r.out = at::mm(r.normed, w.out_w.t());
+  r.out = residual ? at::addmm(*residual, r.normed, w.out_w.t()) : at::mm(r.normed, w.out_w.t());
   return r;
 }
 
@@ -568,15 +568,17 @@ struct MixerFn : torch::autograd::Function<MixerFn> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& in_w, const Tensor& dw_w,
                         const Tensor& dw_b, const Tensor& dt_bias, const Tensor& alpha_bias, const Tensor& theta_mod_bias,
                         const Tensor& theta_bias, const Tensor& d_skip, const Tensor& norm_w, const Tensor& out_w,
-                        const Tensor& theta_sign, std::vector<double> reals, std::vector<int64_t> dims) {
+                        const Tensor& theta_sign, std::vector<double> reals, std::vector<int64_t> dims, const OptT& pre_w) {
     const MixerShape s = shape_of(dims);
-    const Tensor flat = x.reshape({s.rows(), x.size(-1)});
+    const bool block = pre_w.has_value();   // x + mixer(norm(x)) instead of mixer(x)
+    const Tensor stream = x.reshape({s.rows(), x.size(-1)}).contiguous();
+    const Tensor flat = block ? rmsnorm_fwd(stream, *pre_w, (float)reals[11]) : stream;
     const MixerWeights w = weights_of(flat.scalar_type(), in_w, dw_w, dw_b, {dt_bias, alpha_bias, theta_mod_bias, theta_bias, theta_sign},
                                       reals, d_skip, norm_w, out_w);
-    const MixerRun r = mixer_run(s, w, flat, {}, {}, {}, {}, true, false);
+    const MixerRun r = mixer_run(s, w, flat, {}, {}, {}, {}, true, false, block ? OptT(stream) : OptT());
     ctx->save_for_backward({flat, s.whole() ? in_w : r.in_w, w.dw_w, w.dw_b, w.bias[0], w.bias[1], w.bias[2], w.bias[3], w.d_skip, w.norm_w, out_w,
                             w.bias[4], r.proj, r.U, r.M, r.K, r.B, r.C, r.Y, r.normed, r.states ? *r.states : Tensor(),
-                            r.states ? *r.final_state : Tensor()});
+                            r.states ? *r.final_state : Tensor(), block ? stream : Tensor(), block ? *pre_w : Tensor()});
     for (const Tensor& t : {dw_w, dw_b, dt_bias, alpha_bias, theta_mod_bias, theta_bias, d_skip, norm_w})
       dims.push_back((int64_t)t.scalar_type());
     auto shape = x.sizes().vec();
@@ -599,7 +601,7 @@ struct MixerFn : torch::autograd::Function<MixerFn> {
     Call call(x, grads[0]);
     const auto type = x.scalar_type();
     const auto st = static_cast<cudaStream_t>(call.stream());
-    Variables g(14);
+    Variables g(15);
     const Tensor dout = grads[0].reshape({s.rows(), grads[0].size(-1)});
     if (ctx->needs_input_grad(10)) g[10] = at::mm(dout.t(), normed);
     Tensor dn = at::mm(dout, out_w);
@@ -645,7 +647,10 @@ struct MixerFn : torch::autograd::Function<MixerFn> {
       for (const auto& [from, to] : {std::pair<int64_t, int64_t>{s.front(), s.bc0()}, {end, s.pitch()}})
         if (to > from) C10_CUDA_CHECK(cudaMemset2DAsync(column(d_proj, from), s.pitch() * e, 0, (to - from) * e, s.rows(), st));
     }
-    if (ctx->needs_input_grad(0)) g[0] = at::mm(d_proj, in_w).view(ctx->saved_data["x"].toIntVector());
+    const bool block = v[22].defined();
+    if (ctx->needs_input_grad(0) || block) g[0] = at::mm(d_proj, in_w);
+    if (block) std::tie(g[0], g[14]) = rmsnorm_bwd(v[22], v[23], (float)reals[11], g[0], dout.contiguous(), true);
+    if (g[0].defined()) g[0] = g[0].view(ctx->saved_data["x"].toIntVector());
     if (ctx->needs_input_grad(1)) {
       g[1] = at::mm(d_proj.t(), x);
       if (!s.whole()) g[1] = at::cat({g[1].narrow(0, 0, s.front()), g[1].narrow(0, s.bc0(), s.bcn())});
@@ -663,15 +668,16 @@ struct MixerFn : torch::autograd::Function<MixerFn> {
   }
 };
 
-// parameters: in_w dw_w dw_b dt_bias alpha_bias theta_mod_bias theta_bias d_skip norm_w out_w theta_sign; reals: the ten
-// configuration values and the norm's epsilon; dims: heads groups P N chunk path
+// parameters: in_w dw_w dw_b dt_bias alpha_bias theta_mod_bias theta_bias d_skip norm_w out_w theta_sign [norm in front of the
+// mixer]; reals: the ten configuration values, the norm's epsilon, and that of the norm in front; dims: heads groups P N chunk path
 std::vector<int64_t> mixer_dims(const Tensor& x, const std::vector<int64_t>& dims) {
   std::vector<int64_t> d{x.size(0), x.size(1)};
   d.insert(d.end(), dims.begin(), dims.end());
   return d;
 }
 Tensor mixer_train(const Tensor& x, const std::vector<Tensor>& p, const std::vector<double>& reals, const std::vector<int64_t>& dims) {
-  return MixerFn::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], p[9], p[10], reals, mixer_dims(x, dims));
+  return MixerFn::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], p[9], p[10], reals, mixer_dims(x, dims),
+                        p.size() > 11 ? OptT(p[11]) : OptT());
 }
 // without gradients: out, and on request the streaming state (conv, scan state, last B, last U)
 std::tuple<Tensor, OptT, OptT, OptT, OptT> mixer_infer(const Tensor& x, const std::vector<Tensor>& p, const std::vector<double>& reals,
@@ -687,6 +693,66 @@ std::tuple<Tensor, OptT, OptT, OptT, OptT> mixer_infer(const Tensor& x, const st
   Tensor out = r.out.view({s.batch, s.T, r.out.size(1)});
   if (!want_state) return {out, {}, {}, {}, {}};
   return {out, r.conv, r.final_state->to(type), r.B.select(2, s.T - 1).contiguous(), r.U.select(2, s.T - 1).contiguous()};
+}
+
+// ---- FFN branch of a block in training: x + W2 act(W1 norm(x) + b1) + b2 ----------------------------------------------------
+// One node; the residual gradient is added where the norm's is written, and the bias gradients are column sums.
+struct FFNFn : torch::autograd::Function<FFNFn> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& norm_w, const Tensor& w1, const Tensor& w2,
+                        double eps, int64_t kind, const OptT& b1, const OptT& b2) {
+    const Tensor rows = x.reshape({-1, x.size(-1)}).contiguous();
+    const Tensor normed = rmsnorm_fwd(rows, norm_w, (float)eps), projected = at::linear(normed, w1, b1);
+    const Tensor hidden = ffn_act_fwd(projected, (int)kind);
+    const Tensor out = b2 ? rows + at::linear(hidden, w2, b2) : at::addmm(rows, hidden, w2.t());
+    ctx->save_for_backward({rows, norm_w, w1, w2, normed, projected, hidden});
+    ctx->saved_data["eps"] = eps;
+    ctx->saved_data["kind"] = kind;
+    ctx->saved_data["b1"] = b1.has_value();
+    ctx->saved_data["b2"] = b2.has_value();
+    ctx->saved_data["x"] = x.sizes().vec();
+    return out.view(x.sizes());
+  }
+  static Variables backward(torch::autograd::AutogradContext* ctx, Variables grads) {
+    const auto v = ctx->get_saved_variables();
+    const Tensor &rows = v[0], &norm_w = v[1], &w1 = v[2], &w2 = v[3], &normed = v[4], &projected = v[5], &hidden = v[6];
+    const bool b1 = ctx->saved_data["b1"].toBool(), b2 = ctx->saved_data["b2"].toBool();
+    const int64_t D = rows.size(1), W = projected.size(1), n = rows.size(0);
+    const int kind = (int)ctx->saved_data["kind"].toInt(), io = code_of(rows.scalar_type());
+    Variables g(8);
+    const Tensor dout = grads[0].reshape({n, D}).contiguous();
+    Call call(rows, dout);
+    const auto st = static_cast<cudaStream_t>(call.stream());
+    // float64 sums over the rows: norm weight, both biases
+    const Tensor sums = call.zeros({2 * D + W}, at::kDouble);
+    double* const acc = sums.data_ptr<double>();
+    const bool fused_b2 = b2 && sl::rmsnorm_bwd_sums_extra(D);
+    g[3] = at::mm(dout.t(), hidden);
+    const Tensor d_hid = at::mm(dout, w2);
+    Tensor d_proj;
+    if (b1) {
+      d_proj = at::empty_like(projected);
+      check(sl::ffn_act_bwd_sum(ptr(projected), ptr(d_hid), mptr(d_proj), acc + 2 * D, n, hidden.size(1), kind, io, st),
+            "sl_ffn_activation_bwd");
+    } else {
+      d_proj = ffn_act_bwd(projected, d_hid, kind);
+    }
+    g[2] = at::mm(d_proj.t(), normed);
+    const Tensor dn = at::mm(d_proj, w1);
+    g[0] = at::empty_like(rows);
+    check(sl::rmsnorm_bwd(ptr(rows), ptr(norm_w), (float)ctx->saved_data["eps"].toDouble(), ptr(dn), ptr(dout), mptr(g[0]), nullptr, acc,
+                          fused_b2 ? acc + D : nullptr, n, D, io, st),
+          "sl_rmsnorm_bwd");
+    g[0] = g[0].view(ctx->saved_data["x"].toIntVector());
+    const Tensor low = sums.to(rows.scalar_type());
+    g[1] = low.narrow(0, 0, D);
+    if (b1) g[6] = low.narrow(0, 2 * D, W);
+    if (b2) g[7] = fused_b2 ? low.narrow(0, D, D) : column_sum(dout);
+    return g;
+  }
+};
+Tensor ffn_train(const Tensor& x, const Tensor& norm_w, const Tensor& w1, const OptT& b1, const Tensor& w2, const OptT& b2, double eps,
+                 int64_t kind) {
+  return FFNFn::apply(x, norm_w, w1, w2, eps, kind, b1, b2);
 }
 
 // ---- language-model training step --------------------------------------------------------------------------------------
@@ -800,6 +866,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("adamw_step", &adamw_step);
   m.def("mixer_train", &mixer_train);
   m.def("mixer_infer", &mixer_infer);
+  m.def("ffn_train", &ffn_train);
   m.def("mixer_token", &mixer_token);
   m.def("ffn_token", &ffn_token);
   // (a copied or unpickled module makes a plan of its own)

@@ -208,10 +208,14 @@ class SLinOSSMixer(nn.Module):
                 self.d_skip, self.out_norm.weight, self.out_proj.weight, sp.theta_sign]
 
     @_C.opaque
-    def _forward_native(self, x: torch.Tensor, parameters: list, state: SLinOSSMixerState | None, return_state: bool):
+    def _forward_native(self, x: torch.Tensor, parameters: list, state: SLinOSSMixerState | None, return_state: bool, *,
+                        pre_norm: nn.RMSNorm | None = None):
+        """``pre_norm`` (training only): ``x + mixer(pre_norm(x))`` as one node."""
         host, sp, backend = _C.host(), self.scanprep, self.scan_backend
         reals = [*(getattr(sp, n) for n in _C.CONFIG_FIELDS), _norm_eps(self.out_norm)]
         dims = [self.n_heads, self.bc_groups, self.d_head, self.d_state, int(self.chunk_size), _C._PATHS[backend.path]]
+        if pre_norm is not None:
+            return host.mixer_train(x, [*parameters, pre_norm.weight], [*reals, _norm_eps(pre_norm)], dims)
         if _C.grad_needed(x, *parameters):
             return host.mixer_train(x, parameters, reals, dims)
         carried = (None,) * 4 if state is None else (state.conv, state.scan.state, state.scan.b_prev, state.scan.u_prev)

@@ -192,3 +192,39 @@ def test_mlp_module_runs_its_activation_on_the_row_kernel(kind):
     assert rel(out, out64) <= 1e-5 and rel(x.grad, x64.grad) <= 1e-5
     for (n, p), q in zip(mlp.named_parameters(), m64.parameters()):
         assert rel(p.grad, q.grad) <= 1e-5, n
+
+
+@pytest.mark.parametrize("rows, C", [(1, 8), (63, 16), (64, 264), (65, 576), (700, 2304), (20000, 8), (8192, 256)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_column_sum(rows, C, dtype):
+    x = torch.randn(rows, C, device="cuda").to(dtype)
+    want = x.double().sum(0)
+    err = (_C.column_sum(x).double() - want).abs().max() / want.abs().max()
+    assert err <= {torch.float32: 1e-5, torch.bfloat16: 4e-3, torch.float16: 6e-4}[dtype]
+
+
+@pytest.mark.parametrize("kind, bias, C, T", [("gelu", True, 128, 37), ("swiglu", False, 256, 130), ("gelu", False, 72, 1)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_training_nodes_of_a_block_equal_the_composed_block(kind, bias, C, T, dtype, monkeypatch):
+    torch.manual_seed(4)
+    cfg = sb.SLinOSSBlockConfig(d_model=C, mixer=sb.SLinOSSMixerConfig(d_state=64, d_head=64, expand=2.0),
+                                ffn=sb.SLinOSSMLPConfig(kind=kind, expand=2.0, multiple_of=8, bias=bias))
+    blk = sb.SLinOSSBlock(cfg, device="cuda", dtype=dtype)
+    x, dy = torch.randn(2, T, C, device="cuda", dtype=dtype), torch.randn(2, T, C, device="cuda", dtype=dtype)
+
+    def run():
+        blk.zero_grad(set_to_none=True)
+        xi = x.clone().requires_grad_()
+        y = blk(xi)
+        y.backward(dy)
+        return {"y": y.detach(), "x": xi.grad, **{n: p.grad for n, p in blk.named_parameters()}}
+
+    got = run()
+    monkeypatch.setattr(type(blk), "_native_training_ready", lambda self, x: False)
+    blk.ffn_remat = "plain"    # neither the one-node branch nor a rematerialising schedule
+    monkeypatch.setattr("slinoss_b200.blocks.block.ffn_residual_supported", lambda *a: False)
+    want = run()
+    for name, ref in want.items():
+        assert got[name].shape == ref.shape and got[name].dtype == ref.dtype
+        err = (got[name].float() - ref.float()).abs().max() / ref.float().abs().max().clamp_min(1e-6)
+        assert err <= 3e-2, (name, err)
