@@ -169,7 +169,25 @@ template <bool FAST> __device__ __forceinline__ float gelu_tanh_f(float x) {
   return 0.5f * x * (1.f + tanh_io<FAST>(u));
 }
 
+// ---- chains of launches ----------------------------------------------------------
+// A kernel launched as dependent may start while its predecessor in the stream still runs; it does what needs nothing of the
+// predecessor (its weights) and then waits for the end of that grid.  Every kernel that such a launch may follow releases it at its start.
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- host side -----------------------------------------------------------------
+template <typename K, typename A, typename... As>
+inline int launch_chained(K kernel, unsigned grid, unsigned block, size_t smem, cudaStream_t st, bool dependent, const A& a,
+                          const As&... as) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cfg.attrs = &attr; cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, a, as...) == cudaSuccess ? SL_OK : SL_ERR_LAUNCH_FAILED;
+}
+
 inline size_t dtype_size(int dt) { return dt == SL_F32 ? 4 : 2; }
 inline bool dtype_ok(int dt) { return dt == SL_F32 || dt == SL_BF16 || dt == SL_F16; }
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }

@@ -315,14 +315,18 @@ Tensor ffn_act_bwd(const Tensor& proj, const Tensor& dhid, int kind) {
 // row kernel of the norm.
 struct Norm { OptT weight; float eps = 0.f; };
 
+bool small_batch(const Tensor& x, const Tensor& W) {
+  return x.size(0) <= 64 && x.size(1) % 8 == 0 && x.size(1) <= 4096 && x.scalar_type() != at::kFloat && W.is_contiguous() &&
+         x.stride(1) == 1 && x.stride(0) % 8 == 0;
+}
 Tensor linear_rows(const Call& call, const Tensor& x, const Norm& norm, const Tensor& W, const OptT& bias, int act,
-                   const OptT& residual, const OptT& out_in) {
+                   const OptT& residual, const OptT& out_in, bool dependent = false) {
   const int64_t M = x.size(0), K = x.size(1), O = act == sl::LINEAR_SWIGLU ? W.size(0) / 2 : W.size(0);
   const int io = code_of(x.scalar_type());
-  if (M <= 64 && K % 8 == 0 && K <= 4096 && io != SL_F32 && W.is_contiguous() && x.stride(1) == 1 && x.stride(0) % 8 == 0) {
+  if (small_batch(x, W)) {
     Tensor out = out_in ? *out_in : call.empty({M, O}, x.scalar_type());
     const sl::SkinnyArgs a{ptr(x), x.stride(0), ptr(norm.weight), norm.eps, nullptr, 0, ptr(W), ptr(bias), ptr(residual),
-                           mptr(out), (int)M, (int)K, (int)O, act, io};
+                           mptr(out), (int)M, (int)K, (int)O, act, io, dependent};
     check(sl::skinny_linear(a, static_cast<cudaStream_t>(call.stream())), "skinny_linear");
     return out;
   }
@@ -350,6 +354,7 @@ std::tuple<Tensor, Tensor, Tensor> mixer_token(const Tensor& x, const OptT& pre_
   for (const auto& t : biases) call.need(t);
   const int64_t batch = x.size(0), C = (int64_t)heads * P, O = in_w.size(0);
   const int io = code_of(x.scalar_type());
+  const bool chained = small_batch(x, in_w);   // the step may start behind our own in_proj kernel
   const Tensor proj = linear_rows(call, x, Norm{pre_norm, pre_eps}, in_w, {}, sl::LINEAR_NONE, {}, {});
   const size_t ws_bytes = sl_mixer_decode_step_workspace_bytes(batch, heads, P);
   Tensor ws = workspace && (size_t)workspace->numel() >= ws_bytes ? *workspace : call.bytes(ws_bytes);
@@ -361,14 +366,14 @@ std::tuple<Tensor, Tensor, Tensor> mixer_token(const Tensor& x, const OptT& pre_
   const sl::MixerStepArgs a{base, base + C * e, base + 2 * C * e, base + (2 * C + 3 * heads) * e, O, O, O, O, ptr(dw_w), ptr(dw_b),
                             mptr(conv), (int)dw_w.size(1), bs.p[0], bs.p[1], bs.p[2], bs.p[3], bs.p[4], &c, fptr(d_skip),
                             mfptr(state), ptr(b_prev), mptr(b_next), mptr(u_prev), mptr(ws), (size_t)ws.numel(), (int)batch, heads,
-                            groups, P, N, io};
+                            groups, P, N, io, chained};
   const auto st = static_cast<cudaStream_t>(call.stream());
   check(sl::mixer_step_launch(a, st), "mixer_step");
   const int64_t K = C, OO = out_w.size(0);
   if (batch <= 64 && K % 8 == 0 && K <= 4096 && io != SL_F32 && out_w.is_contiguous()) {   // the row norm inside the projection
     Tensor y = out ? *out : call.empty({batch, OO}, x.scalar_type());
     const sl::SkinnyArgs s{mptr(ws), C, ptr(norm_w), norm_eps, sl::step_partials(mptr(ws), batch, heads, P), 8 * heads, ptr(out_w),
-                           ptr(out_b), ptr(residual), mptr(y), (int)batch, (int)K, (int)OO, sl::LINEAR_NONE, io};
+                           ptr(out_b), ptr(residual), mptr(y), (int)batch, (int)K, (int)OO, sl::LINEAR_NONE, io, true};
     check(sl::skinny_linear(s, st), "skinny_linear");
     return {y, b_next, ws};
   }
@@ -382,7 +387,7 @@ Tensor ffn_token(const Tensor& x, const Tensor& norm_w, float eps, const Tensor&
                  const OptT& b2, int kind) {
   Call call(x, norm_w, w1, b1, w2, b2);
   const Tensor hidden = linear_rows(call, x, Norm{norm_w, eps}, w1, b1, kind == 1 ? sl::LINEAR_SWIGLU : sl::LINEAR_GELU, {}, {});
-  return linear_rows(call, hidden, Norm{}, w2, b2, sl::LINEAR_NONE, x, {});
+  return linear_rows(call, hidden, Norm{}, w2, b2, sl::LINEAR_NONE, x, {}, small_batch(x, w1));
 }
 // One token of a mixer, or of a whole block, without Python per launch.  A plan holds the parameters of one module (the
 // tensors themselves, so data that moves or changes type is seen) and a list of guards: dictionary entries that must still be
@@ -449,6 +454,7 @@ class TokenPlan {
     const Tensor out = call.empty({M, D}, type);
     const Tensor b_next = groups_ == heads_ ? *b_prev : at::empty_like(*b_prev);
 
+    const Tensor rows = block && x.stride(0) != D ? x.contiguous() : x;   // (before the chain: it may launch a copy)
     const sl::SkinnyArgs in{ptr(x), x.stride(0), block ? ptr(b_[0]) : nullptr, (float)eps_[0], nullptr, 0, ptr(p_[0]), nullptr, nullptr,
                             proj, (int)M, (int)D, (int)O, sl::LINEAR_NONE, io};
     check(sl::skinny_linear(in, st), "skinny_linear");
@@ -456,18 +462,17 @@ class TokenPlan {
     const sl::MixerStepArgs a{row, row + C * e, row + 2 * C * e, row + (2 * C + 3 * heads_) * e, O, O, O, O, ptr(p_[1]), ptr(p_[2]),
                               mptr(conv), (int)d_conv_, fptr(p_[3]), fptr(p_[4]), fptr(p_[5]), fptr(p_[6]), fptr(p_[7]), &cfg_,
                               fptr(p_[8]), mfptr(state), ptr(b_prev), mptr(b_next), mptr(u_prev), base, (size_t)n_step, (int)M,
-                              (int)heads_, (int)groups_, (int)P_, (int)N_, io};
+                              (int)heads_, (int)groups_, (int)P_, (int)N_, io, true};
     check(sl::mixer_step_launch(a, st), "mixer_step");
-    const Tensor rows = block && x.stride(0) != D ? x.contiguous() : x;
     const sl::SkinnyArgs o{base, C, ptr(p_[9]), (float)eps_[1], sl::step_partials(base, M, heads_, P_), (int)(8 * heads_), ptr(p_[10]),
-                           ptr(p_[11]), block ? ptr(rows) : nullptr, ffn ? mid : mptr(out), (int)M, (int)C, (int)D, sl::LINEAR_NONE, io};
+                           ptr(p_[11]), block ? ptr(rows) : nullptr, ffn ? mid : mptr(out), (int)M, (int)C, (int)D, sl::LINEAR_NONE, io, true};
     check(sl::skinny_linear(o, st), "skinny_linear");
     if (ffn) {
       const sl::SkinnyArgs f1{mid, D, ptr(b_[1]), (float)eps_[2], nullptr, 0, ptr(b_[2]), ptr(b_[3]), nullptr, hidden, (int)M, (int)D,
-                              (int)F, ffn_kind_ == 1 ? sl::LINEAR_SWIGLU : sl::LINEAR_GELU, io};
+                              (int)F, ffn_kind_ == 1 ? sl::LINEAR_SWIGLU : sl::LINEAR_GELU, io, true};
       check(sl::skinny_linear(f1, st), "skinny_linear");
       const sl::SkinnyArgs f2{hidden, F, nullptr, 0.f, nullptr, 0, ptr(b_[4]), ptr(b_[5]), mid, mptr(out), (int)M, (int)F, (int)D,
-                              sl::LINEAR_NONE, io};
+                              sl::LINEAR_NONE, io, true};
       check(sl::skinny_linear(f2, st), "skinny_linear");
     }
     return py::make_tuple(out, b_next, ws);

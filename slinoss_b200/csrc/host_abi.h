@@ -25,6 +25,7 @@ struct MixerStepArgs {
   void* workspace;    // receives the gated values (batch, heads * P) and their partial sums of squares
   size_t workspace_bytes;
   int batch, heads, groups, P, N, io_dtype;
+  bool dependent = false;   // launched right behind a kernel of this library that wrote the rows
 };
 
 size_t mixer_step_workspace(int batch, int heads, int P);
@@ -50,6 +51,7 @@ struct SkinnyArgs {
   const void* residual;   // (M, O) dense or null
   void* out;              // (M, O) dense
   int M, K, O, act, io_dtype;
+  bool dependent = false;   // launched right behind a kernel of this library that wrote x (and no parameter)
 };
 SL_API bool skinny_supported(int M, int K, int O, int io_dtype);
 SL_API int skinny_linear(const SkinnyArgs& a, cudaStream_t st);

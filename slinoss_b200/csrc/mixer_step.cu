@@ -324,6 +324,7 @@ __global__ void __launch_bounds__(STEP_THREADS, KQ == 1 ? 2 : 1) mixer_step_pipe
     fence_barrier_init();
     s_abort = 0;
   }
+  grid_release();
   __syncthreads();
   auto wait = [&](uint64_t* bar, uint32_t parity, int code) {   // a converged warp; bounded
     bool ok = mbar_try_wait(bar, parity);
@@ -437,6 +438,7 @@ __global__ void __launch_bounds__(STEP_THREADS, KQ == 1 ? 2 : 1) mixer_step_pipe
     }
   } else {
     // ---- preparation warps, one (batch, head) ahead: 8, 9 conv | 10 b and taps | 11 c | 12 coefficients ---------------
+    grid_wait();   // the state tiles are already on their way
     const int pw = w - STEP_WARPS;
     bool live = true;
     for (int j = 0; j < n; ++j) {
@@ -575,12 +577,13 @@ int mixer_step_device_status(bool reset) {
 
 namespace {
 template <typename T, int KQ>
-int launch_step_pipe(const StepParams& p, int tasks, cudaStream_t st) {
+int launch_step_pipe(const StepParams& p, int tasks, bool dependent, cudaStream_t st) {
   auto k = mixer_step_pipe_kernel<T, KQ>;
   static std::atomic<unsigned long long> done{0};
   if (int e = ensure_smem(k, StepSmem<KQ>::BYTES, done)) return e;
   const int resident = 148 * (KQ == 1 ? 2 : 1);   // persistent: as many CTAs as fit, tasks dealt out round robin
-  k<<<tasks < resident ? tasks : resident, STEP_THREADS, StepSmem<KQ>::BYTES, st>>>(p, tasks);
+  if (int e = launch_chained(k, (unsigned)(tasks < resident ? tasks : resident), STEP_THREADS, StepSmem<KQ>::BYTES, st, dependent, p, tasks))
+    return e;
   return SL_OK;
 }
 }  // namespace
@@ -610,7 +613,7 @@ int mixer_step_launch(const MixerStepArgs& a, cudaStream_t st) {
   // (batch, head).
   if (a.P == 64 && (a.N == 64 || a.N == 128)) {
     int rc = SL_OK;
-    SL_DISPATCH_DTYPE(a.io_dtype, T, { rc = a.N == 64 ? launch_step_pipe<T, 1>(p, tasks, st) : launch_step_pipe<T, 2>(p, tasks, st); });
+    SL_DISPATCH_DTYPE(a.io_dtype, T, { rc = a.N == 64 ? launch_step_pipe<T, 1>(p, tasks, a.dependent, st) : launch_step_pipe<T, 2>(p, tasks, a.dependent, st); });
     if (rc != SL_OK) return rc;
   } else {
     const size_t smem = ((size_t)4 * 2 * a.N + 3 * (size_t)a.P) * sizeof(float);

@@ -54,6 +54,7 @@ __global__ void __launch_bounds__(512) skinny_linear_kernel(SkinnyArgs p) {
   const T* W = reinterpret_cast<const T*>(p.weight);
   const T* X = reinterpret_cast<const T*>(p.x);
 
+  grid_release();
   // ---- request this warp's run of W ---------------------------------------------------------------------------
   uint4 wv[NT][STEPS];
   const int k0 = w * KRUN + 8 * t;
@@ -67,6 +68,7 @@ __global__ void __launch_bounds__(512) skinny_linear_kernel(SkinnyArgs p) {
       if (row_ok && k0 + 32 * s < p.K) wv[j][s] = __ldg(reinterpret_cast<const uint4*>(W + (size_t)r * p.K + k0 + 32 * s));
     }
   }
+  grid_wait();
   // ---- row scales of the norm, while W is on its way ------------------------------------------------------------
   const bool norm = p.norm_weight != nullptr;
   if (norm) {
@@ -164,8 +166,7 @@ int launch_skinny(const SkinnyArgs& a, cudaStream_t st) {
     if (int e = ensure_smem(k, 16 * 16 * MT * 8 * NT * sizeof(float), done)) return e;
   }
   const int rows = 8 * (SWIGLU ? NT / 2 : NT);
-  k<<<(a.O + rows - 1) / rows, 32 * warps, smem, st>>>(a);
-  return SL_OK;
+  return launch_chained(k, (unsigned)((a.O + rows - 1) / rows), (unsigned)(32 * warps), smem, st, a.dependent, a);
 }
 template <typename T>
 int launch_skinny_m(const SkinnyArgs& a, cudaStream_t st) {
