@@ -160,6 +160,13 @@ class SLinOSSBlock(nn.Module):
             ffn_eps, kind = _norm_eps(fnorm), _C.FFN_KINDS[ffn.kind]
         return mixer._make_token_plan(branch, (same, empty), _norm_eps(norm), ffn_eps, kind)
 
+    def planned_step(self, token, state, inplace, chained: bool = False):
+        """The step through the block's native plan, or None (see ``layers.mixer.planned_step``)."""
+        if state is None or not token.is_cuda or (inplace is not None and not inplace) or type(self.mixer) is not SLinOSSMixer \
+                or (self.residual_dropout > 0.0 and self.training):
+            return None
+        return planned_step(self, token, state.mixer, self._make_token_plan, chained)
+
     def _native_step(self, token, state, inplace):
         """The whole step in five launches (a native plan, or ``SLinOSSMixer.decode_native``), or None when something asks for the
         composed path: gradients, another norm, dropout, autocast, hooks, an injected backend, a partial state."""
@@ -168,7 +175,7 @@ class SLinOSSBlock(nn.Module):
                 (self.residual_dropout > 0.0 and self.training) or type(mixer) is not SLinOSSMixer:
             return None
         norm, ms = self.mixer_norm, state.mixer
-        out = planned_step(self, token, ms, self._make_token_plan)
+        out = self.planned_step(token, state, inplace)
         if out is not None:
             return out, SLinOSSBlockState(mixer=ms)
         if not (_plain_rmsnorm(norm, token) and mixer._fused_decode_ready(ms, token)

@@ -412,9 +412,10 @@ class TokenPlan {
     return true;
   }
 
-  // None where the call is not the plain one; else (out, next b_prev, workspace)
+  // None where the call is not the plain one; else (out, next b_prev, workspace).  dependent: x is the result of a plan's
+  // step that was the last thing launched on this stream.
   py::object step(const Tensor& x, const OptT& conv, const OptT& state, const OptT& b_prev, const OptT& u_prev,
-                  const OptT& workspace) const {
+                  const OptT& workspace, bool dependent) const {
     if (at::GradMode::is_enabled() || at::autocast::is_autocast_enabled(at::kCUDA) || !x.is_cuda() || x.dim() != 2) return py::none();
     const auto type = x.scalar_type();
     const int64_t M = x.size(0), D = x.size(1), C = heads_ * P_;
@@ -456,7 +457,7 @@ class TokenPlan {
 
     const Tensor rows = block && x.stride(0) != D ? x.contiguous() : x;   // (before the chain: it may launch a copy)
     const sl::SkinnyArgs in{ptr(x), x.stride(0), block ? ptr(b_[0]) : nullptr, (float)eps_[0], nullptr, 0, ptr(p_[0]), nullptr, nullptr,
-                            proj, (int)M, (int)D, (int)O, sl::LINEAR_NONE, io};
+                            proj, (int)M, (int)D, (int)O, sl::LINEAR_NONE, io, dependent};
     check(sl::skinny_linear(in, st), "skinny_linear");
     const auto* row = static_cast<const uint8_t*>(proj);
     const sl::MixerStepArgs a{row, row + C * e, row + 2 * C * e, row + (2 * C + 3 * heads_) * e, O, O, O, O, ptr(p_[1]), ptr(p_[2]),

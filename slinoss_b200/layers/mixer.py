@@ -30,9 +30,9 @@ def _norm_eps(norm: nn.RMSNorm) -> float:
 
 
 @_C.opaque
-def planned_step(module: nn.Module, token: torch.Tensor, state: SLinOSSMixerState, make):
+def planned_step(module: nn.Module, token: torch.Tensor, state: SLinOSSMixerState, make, chained: bool = False):
     """One token through the module's native plan (made by ``make`` and kept while its guards hold), ``state`` updated in
-    place; None where the call needs the composed path."""
+    place; None where the call needs the composed path.  ``chained``: ``token`` is what another planned step has just returned."""
     plan = module.__dict__.get("_token_plan")
     if plan is None or not plan.valid():
         plan = make()
@@ -40,7 +40,8 @@ def planned_step(module: nn.Module, token: torch.Tensor, state: SLinOSSMixerStat
             return None
         module.__dict__["_token_plan"] = plan
     scan = state.scan
-    done = plan.step(token, state.conv, scan.state, scan.b_prev, scan.u_prev, state.__dict__.get("_plan_workspace"))
+    done = plan.step(token, state.conv, scan.state, scan.b_prev, scan.u_prev, state.__dict__.get("_plan_workspace"),
+                     chained)
     if done is None:
         return None
     out, scan.b_prev, state._plan_workspace = done

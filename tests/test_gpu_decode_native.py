@@ -109,3 +109,28 @@ def test_mixer_token_by_plan_equals_the_composed_token(batch, monkeypatch):
         want = [mixer.step(t, b)[0] for t in x]
     assert rel(torch.stack(got), torch.stack(want)) <= 2e-2 and rel(a.scan.state, b.scan.state) <= 2e-2
     assert rel(a.scan.b_prev, b.scan.b_prev) <= 2e-2 and rel(a.conv, b.conv) <= 2e-2
+
+
+@pytest.mark.parametrize("batch, d_model, dtype", [(1, 256, torch.bfloat16), (17, 512, torch.float16), (64, 264, torch.bfloat16)])
+def test_a_stack_token_through_chained_plans_equals_the_composed_token(batch, d_model, dtype, monkeypatch):
+    torch.manual_seed(5)
+    blk = sb.SLinOSSBlockConfig(d_model=d_model, mixer=sb.SLinOSSMixerConfig(d_state=64, d_head=64, expand=1.0),
+                                ffn=sb.SLinOSSMLPConfig(kind="swiglu", expand=2.0, multiple_of=8))
+    stack = sb.SLinOSSStack(sb.SLinOSSStackConfig.uniform(blk, n_layers=4), device=DEV, dtype=dtype).eval()
+    x = torch.randn(5, batch, d_model, device=DEV, dtype=dtype)
+
+    def tokens():
+        with torch.no_grad():
+            state = stack.init_decode_state(batch)
+            out = []
+            for t in x:
+                y, state = stack.step(t, state)
+                out.append(y)
+        return torch.stack(out)
+
+    got = tokens()
+    assert torch.equal(got, tokens())
+    monkeypatch.setattr(sb.SLinOSSBlock, "_make_token_plan", lambda self: None)
+    for b in stack.blocks:
+        b.__dict__.pop("_token_plan", None)
+    assert rel(got, tokens()) <= 2e-2
