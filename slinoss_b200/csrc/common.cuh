@@ -177,13 +177,13 @@ __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;
 
 // ---- host side -----------------------------------------------------------------
 template <typename K, typename A, typename... As>
-inline int launch_chained(K kernel, unsigned grid, unsigned block, size_t smem, cudaStream_t st, bool dependent, const A& a,
+inline int launch_chained(K kernel, dim3 grid, unsigned block, size_t smem, cudaStream_t st, bool dependent, const A& a,
                           const As&... as) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cfg.gridDim = grid; cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cfg.attrs = &attr; cfg.numAttrs = dependent ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, a, as...) == cudaSuccess ? SL_OK : SL_ERR_LAUNCH_FAILED;
 }

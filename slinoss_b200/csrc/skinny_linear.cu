@@ -55,7 +55,6 @@ __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyA
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
   const int g = lane >> 2, t = lane & 3, o0 = blockIdx.x * 8 * OT;
   const T* W = reinterpret_cast<const T*>(p.weight);
-  const T* X = reinterpret_cast<const T*>(p.x);
 
   grid_release();
   // ---- request this warp's run of W ---------------------------------------------------------------------------
@@ -72,12 +71,17 @@ __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyA
     }
   }
   grid_wait();
+  // this CTA's rows
+  const int mb = blockIdx.y * 16 * MT, M = min(p.M - mb, 16 * MT);
+  const T* X = reinterpret_cast<const T*>(p.x) + (size_t)mb * p.x_stride;
+  const float* partials = p.partials ? p.partials + (size_t)mb * p.n_partials : nullptr;
+  const T *bias = reinterpret_cast<const T*>(p.bias), *residual = reinterpret_cast<const T*>(p.residual);
+  if (residual) residual += (size_t)mb * p.O;
   // ---- row scales of the norm, while W is on its way ------------------------------------------------------------
   const bool norm = p.norm_weight != nullptr;
   // the first output of this thread: its residual and bias are requested ahead of the product
   const int m0 = tid / (8 * OT), c0 = tid % (8 * OT);
-  const bool out0 = tid < p.M * 8 * OT && o0 + c0 < p.O;
-  const T *bias = reinterpret_cast<const T*>(p.bias), *residual = reinterpret_cast<const T*>(p.residual);
+  const bool out0 = tid < M * 8 * OT && o0 + c0 < p.O;
   const float res0 = out0 && residual ? to_f32(residual[(size_t)m0 * p.O + o0 + c0]) : 0.f;
   const float bias0 = out0 && bias ? to_f32(bias[o0 + c0]) : 0.f;
   uint4 xk[KEEP ? STEPS : 1][KEEP ? MT : 1][2];
@@ -90,10 +94,10 @@ __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyA
 #pragma unroll
       for (int i = 0; i < 2 * MT; ++i) {
         xk[s][i / 2][i % 2] = make_uint4(0u, 0u, 0u, 0u);
-        if (8 * i + g < p.M && k0 + 32 * s < p.K)
+        if (8 * i + g < M && k0 + 32 * s < p.K)
           xk[s][i / 2][i % 2] = *reinterpret_cast<const uint4*>(X + (size_t)(8 * i + g) * p.x_stride + k0 + 32 * s);
       }
-    if (!p.partials) {
+    if (!partials) {
 #pragma unroll
       for (int s = 0; s < STEPS; ++s)
 #pragma unroll
@@ -111,11 +115,11 @@ __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyA
       }
     }
   }
-  if (norm && !(KEEP && !p.partials)) {
-    for (int m = w; m < p.M; m += nw) {
+  if (norm && !(KEEP && !partials)) {
+    for (int m = w; m < M; m += nw) {
       float ss = 0.f;
-      if (p.partials) {
-        for (int k = lane; k < p.n_partials; k += 32) ss += p.partials[(size_t)m * p.n_partials + k];
+      if (partials) {
+        for (int k = lane; k < p.n_partials; k += 32) ss += partials[(size_t)m * p.n_partials + k];
       } else {
         for (int k = 8 * lane; k < p.K; k += 256) {
           float v[8];
@@ -141,8 +145,8 @@ __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyA
 #pragma unroll
   for (int i = 0; i < 2 * MT; ++i) {
     rs[i] = 0.f;
-    if (!norm || g + 8 * i >= p.M) continue;
-    if (KEEP && !p.partials) {
+    if (!norm || g + 8 * i >= M) continue;
+    if (KEEP && !partials) {
       float ss = 0.f;
       for (int q = 0; q < nw; ++q) ss += s_ss[q][8 * i + g];
       rs[i] = rsqrtf(ss / (float)p.K + p.norm_eps);
@@ -163,7 +167,7 @@ __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyA
       for (int hh = 0; hh < 2; ++hh) {
         const int m = 16 * i + 8 * hh + g;
         xa[hh] = make_uint4(0u, 0u, 0u, 0u);
-        if (m < p.M && k < p.K) {
+        if (m < M && k < p.K) {
           if constexpr (KEEP) xa[hh] = xk[s][i][hh];
           else xa[hh] = *reinterpret_cast<const uint4*>(X + (size_t)m * p.x_stride + k);
           if (norm) xa[hh] = scale_pieces<T>(xa[hh], rs[2 * i + hh], nwv);
@@ -189,7 +193,7 @@ __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyA
         *reinterpret_cast<float2*>(mine + (16 * i + 8 * hh + g) * PITCH + 8 * j + 2 * t) =
             make_float2(acc[i][j][2 * hh], acc[i][j][2 * hh + 1]);
   __syncthreads();
-  for (int idx = tid; idx < p.M * 8 * OT; idx += blockDim.x) {
+  for (int idx = tid; idx < M * 8 * OT; idx += blockDim.x) {
     const int m = idx / (8 * OT), c = idx % (8 * OT), o = o0 + c;
     if (o >= p.O) continue;
     float v = 0.f, gate = 0.f;
@@ -202,7 +206,7 @@ __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyA
     if (SWIGLU) v = v * silu_f(round_io<T>(gate));
     else if (p.act == LINEAR_GELU) v = gelu_tanh_f<true>(v);
     if (residual) v = round_io<T>(v) + (idx == tid ? res0 : to_f32(residual[(size_t)m * p.O + o]));
-    reinterpret_cast<T*>(p.out)[(size_t)m * p.O + o] = from_f32<T>(v);
+    reinterpret_cast<T*>(p.out)[(size_t)(mb + m) * p.O + o] = from_f32<T>(v);
   }
 }
 
@@ -216,23 +220,22 @@ int launch_skinny_as(const SkinnyArgs& a, cudaStream_t st) {
     if (int e = ensure_smem(k, 16 * 16 * MT * 8 * NT * sizeof(float), done)) return e;
   }
   const int rows = 8 * (SWIGLU ? NT / 2 : NT);
-  return launch_chained(k, (unsigned)((a.O + rows - 1) / rows), (unsigned)(32 * warps), smem, st, a.dependent, a);
+  return launch_chained(k, dim3((a.O + rows - 1) / rows, (a.M + 16 * MT - 1) / (16 * MT)), (unsigned)(32 * warps), smem, st, a.dependent, a);
 }
 template <typename T, int MT, int NT, bool SWIGLU>
 int launch_skinny(const SkinnyArgs& a, cudaStream_t st) {
-  if constexpr (MT <= 2) {
-    if (a.norm_weight && a.K <= 8 * KRUN) return launch_skinny_as<T, MT, NT, SWIGLU, true>(a, st);
-  }
+  if (a.norm_weight && a.K <= 8 * KRUN) return launch_skinny_as<T, MT, NT, SWIGLU, true>(a, st);
   return launch_skinny_as<T, MT, NT, SWIGLU, false>(a, st);
 }
 template <typename T>
 int launch_skinny_m(const SkinnyArgs& a, cudaStream_t st) {
-  // one 8-row tile of W per warp keeps the most CTAs for the smallest batches; from 17 rows of x on two tiles share
-  // every x fragment, which is then read as often as W
+  // One 16-row tile of x and one 8-row tile of W per warp give the most CTAs and the shortest chain.  A CTA then reads 48 K
+  // bytes, and with many rows of a large layer that traffic takes longer than the chain (width 1024: 348 against 358 us per token
+  // of four blocks at 32 rows, 588 against 523 at 64; width 512: 284 against 346 at 64).
   const bool sw = a.act == LINEAR_SWIGLU;
-  if (a.M <= 16) return sw ? launch_skinny<T, 1, 2, true>(a, st) : launch_skinny<T, 1, 1, false>(a, st);
-  if (a.M <= 32) return sw ? launch_skinny<T, 2, 2, true>(a, st) : launch_skinny<T, 2, 2, false>(a, st);
-  return sw ? launch_skinny<T, 4, 2, true>(a, st) : launch_skinny<T, 4, 2, false>(a, st);
+  if (a.M <= 16 || (long long)a.M * a.K * a.O <= 120000000)
+    return sw ? launch_skinny<T, 1, 2, true>(a, st) : launch_skinny<T, 1, 1, false>(a, st);
+  return sw ? launch_skinny<T, 2, 2, true>(a, st) : launch_skinny<T, 2, 2, false>(a, st);
 }
 
 }  // namespace
