@@ -28,8 +28,7 @@ template <> __device__ __forceinline__ __half from_f32<__half>(float v) {
   return __float2half_rn(v);
 }
 
-// Pairs: packed conversions (one F2FP instruction on the ALU pipe) instead of two scalar ones,
-// which run on the much narrower XU pipe.
+// Pairs: one packed conversion instead of two scalar ones.
 template <typename T> __device__ __forceinline__ uint32_t pack_pair(float a, float b);
 template <> __device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);

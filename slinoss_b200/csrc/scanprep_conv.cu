@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(256) bc_bwd_kernel(const T* __restrict__ bc,
 // io the transcendental functions are the fast intrinsics (their error is far below the output's
 // rounding); float32 io keeps the precise ones.
 template <bool FAST> __device__ __forceinline__ float tanh_v(float x) {
-  if (FAST) {   // one MUFU op, relative error 2^-11: below the rounding of 16-bit outputs
+  if (FAST) {   // PTX tanh.approx, relative error 2^-11: below the rounding of 16-bit outputs
     float y;
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
@@ -589,8 +589,8 @@ template <bool WIDE> __device__ __forceinline__ float part_sum(float v) {   // o
 
 constexpr int BC_GCH = 8;   // groups one warp walks: grid = (tokens / 8, groups / BC_GCH, batch)
 
-// Pairs of the maps above.  (The 16-bit forms spell out the special-function steps: __expf and __logf also rescale denormal
-// operands, which do not occur here - 3 instructions each.)
+// Pairs of the maps above.  The 16-bit forms are softplus x = max(x, 0) + ln(1 + e^-|x|) with e^x = 2^(x log2 e) and
+// ln x = ln 2 log2 x on the PTX instructions ex2.approx and lg2.approx.
 template <bool FAST> __device__ __forceinline__ f2 softplus2(f2 x) {
   const float2 v = un2(x);
   if constexpr (!FAST) return mk2(softplus_f(v.x), softplus_f(v.y));
