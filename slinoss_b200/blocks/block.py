@@ -48,14 +48,6 @@ def _plain_linear(layer, x) -> bool:
 
 
 @_C.opaque
-def _ffn_token(x, norm, ffn):
-    """``x + ffn(norm(x))`` for the rows of one token: two launches for small batches."""
-    w1, w2 = ffn.in_proj._parameters, ffn.out_proj._parameters
-    return _C.host().ffn_token(x, norm.weight, _norm_eps(norm), w1["weight"], w1["bias"], w2["weight"], w2["bias"],
-                               _C.FFN_KINDS[ffn.kind])
-
-
-@_C.opaque
 def _ffn_train(x, norm, ffn):
     """``x + ffn(norm(x))`` as one autograd node."""
     w1, w2 = ffn.in_proj._parameters, ffn.out_proj._parameters
@@ -160,36 +152,15 @@ class SLinOSSBlock(nn.Module):
             ffn_eps, kind = _norm_eps(fnorm), _C.FFN_KINDS[ffn.kind]
         return mixer._make_token_plan(branch, (same, empty), _norm_eps(norm), ffn_eps, kind)
 
-    def planned_step(self, token, state, inplace, chained: bool = False):
-        """The step through the block's native plan, or None (see ``layers.mixer.planned_step``)."""
-        if state is None or not token.is_cuda or (inplace is not None and not inplace) or type(self.mixer) is not SLinOSSMixer \
-                or (self.residual_dropout > 0.0 and self.training):
-            return None
-        return planned_step(self, token, state.mixer, self._make_token_plan, chained)
-
     def _native_step(self, token, state, inplace):
-        """The whole step in five launches (a native plan, or ``SLinOSSMixer.decode_native``), or None when something asks for the
-        composed path: gradients, another norm, dropout, autocast, hooks, an injected backend, a partial state."""
-        mixer = self.mixer
+        """The whole step through the block's native plan (the composed path's products and kernels as one call), or None when
+        something asks for the composed path: gradients, another norm, dropout, autocast, hooks, an injected backend, a
+        partial state."""
         if torch.is_grad_enabled() or state is None or not token.is_cuda or (inplace is not None and not inplace) or \
-                (self.residual_dropout > 0.0 and self.training) or type(mixer) is not SLinOSSMixer:
+                (self.residual_dropout > 0.0 and self.training) or type(self.mixer) is not SLinOSSMixer:
             return None
-        norm, ms = self.mixer_norm, state.mixer
-        out = self.planned_step(token, state, inplace)
-        if out is not None:
-            return out, SLinOSSBlockState(mixer=ms)
-        if not (_plain_rmsnorm(norm, token) and mixer._fused_decode_ready(ms, token)
-                and mixer._native_decode_ready(token)) or mixer._forward_hooks or mixer._forward_pre_hooks:
-            return None
-        ffn = self.ffn
-        if ffn is not None and not (_plain_rmsnorm(self.ffn_norm, token) and type(ffn) is SLinOSSMLP
-                                    and not ffn._forward_hooks and not ffn._forward_pre_hooks
-                                    and _plain_linear(ffn.in_proj, token) and _plain_linear(ffn.out_proj, token)):
-            return None
-        out = mixer.decode_native(token, ms, pre_norm=norm, residual=token)
-        if ffn is not None:
-            out = _ffn_token(out, self.ffn_norm, ffn)
-        return out, SLinOSSBlockState(mixer=ms)
+        out = planned_step(self, token, state.mixer, self._make_token_plan)
+        return None if out is None else (out, SLinOSSBlockState(mixer=state.mixer))
 
     def step(self, x, state: SLinOSSBlockState | None = None, *, inplace=None, context=None):
         token = x
@@ -203,8 +174,11 @@ class SLinOSSBlock(nn.Module):
         done = self._native_step(token, state, inplace)
         if done is not None:
             return done if x.ndim == 2 else (done[0].unsqueeze(1), done[1])
-        mixed, mixer_state = self.mixer.step(apply_norm(self.mixer_norm, token),
-                                             None if state is None else state.mixer, inplace=inplace)
+        normed, carried, mixer = apply_norm(self.mixer_norm, token), None if state is None else state.mixer, self.mixer
+        if type(mixer) is SLinOSSMixer and "step" not in mixer.__dict__:
+            mixed, mixer_state = mixer._step(normed, carried, inplace, True)
+        else:
+            mixed, mixer_state = mixer.step(normed, carried, inplace=inplace)
         out = self._add(token, self._drop(mixed.to(dtype=token.dtype)))
         if self.ffn is not None:
             out = self._ffn_residual(out)

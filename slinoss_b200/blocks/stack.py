@@ -10,7 +10,7 @@ from torch import nn
 
 from .block import SLinOSSBlock, apply_norm, make_norm
 from .config import SLinOSSStackConfig
-from .state import SLinOSSBlockState, SLinOSSStackState
+from .state import SLinOSSStackState
 
 
 class SLinOSSStack(nn.Module):
@@ -82,15 +82,10 @@ class SLinOSSStack(nn.Module):
         if hidden.ndim != 2 or hidden.shape[-1] != self.d_model:
             raise ValueError(f"Expected hidden shape (batch, {self.d_model}), got {tuple(hidden.shape)}.")
         self._check_state(state)
-        layers, chained = [], False
+        layers = []
         for i, block in enumerate(self.blocks):
-            carried = None if state is None else state.layers[i]
-            out = block.planned_step(hidden, carried, inplace, chained) if type(block) is SLinOSSBlock else None
-            chained = out is not None
-            if chained:
-                hidden, nxt = out, SLinOSSBlockState(mixer=carried.mixer)
-            else:
-                hidden, nxt = block.step(hidden, carried, inplace=inplace, context=context)
+            hidden, nxt = block.step(hidden, None if state is None else state.layers[i],
+                                     inplace=inplace, context=context)
             layers.append(nxt)
         hidden = self._final(hidden).to(dtype=x.dtype)
         if x.ndim == 3:

@@ -64,6 +64,8 @@ const float* fptr(const OptT& t) { return t ? static_cast<const float*>(t->data_
 float* mfptr(const Tensor& t) { return static_cast<float*>(t.data_ptr()); }
 float* mfptr(const OptT& t) { return t ? static_cast<float*>(t->data_ptr()) : nullptr; }
 
+uint8_t* column(const Tensor& rows, int64_t c) { return static_cast<uint8_t*>(rows.data_ptr()) + c * rows.element_size(); }
+
 using Config = std::array<float, 10>;
 sl_scanprep_config config_of(const Config& c) {
   return sl_scanprep_config{c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], c[8], c[9]};
@@ -310,52 +312,42 @@ Tensor ffn_act_bwd(const Tensor& proj, const Tensor& dhid, int kind) {
   return dproj;
 }
 
-// ---- decode: one token of a mixer, and of an FFN branch ---------------------------------------------------------------
-// y = W x' (+ residual), x' = x or its RMSNorm: the small-batch kernel where it applies, else the library GEMM behind the
-// row kernel of the norm.
-struct Norm { OptT weight; float eps = 0.f; };
-
+// ---- decode: one token of a mixer ------------------------------------------------------------------------------------
+// y = W x: the small-batch kernel where it applies, else the library GEMM.
 bool small_batch(const Tensor& x, const Tensor& W) {
   return x.size(0) <= 64 && x.size(1) % 8 == 0 && x.size(1) <= 4096 && x.scalar_type() != at::kFloat && W.is_contiguous() &&
          x.stride(1) == 1 && x.stride(0) % 8 == 0;
 }
-Tensor linear_rows(const Call& call, const Tensor& x, const Norm& norm, const Tensor& W, const OptT& bias, int act,
-                   const OptT& residual, const OptT& out_in, bool dependent = false) {
-  const int64_t M = x.size(0), K = x.size(1), O = act == sl::LINEAR_SWIGLU ? W.size(0) / 2 : W.size(0);
-  const int io = code_of(x.scalar_type());
+Tensor linear_rows(const Call& call, const Tensor& x, const Tensor& W, const OptT& bias, const OptT& out_in) {
+  const int64_t M = x.size(0), K = x.size(1), O = W.size(0);
   if (small_batch(x, W)) {
     Tensor out = out_in ? *out_in : call.empty({M, O}, x.scalar_type());
-    const sl::SkinnyArgs a{ptr(x), x.stride(0), ptr(norm.weight), norm.eps, nullptr, 0, ptr(W), ptr(bias), ptr(residual),
-                           mptr(out), (int)M, (int)K, (int)O, act, io, dependent};
+    const sl::SkinnyArgs a{ptr(x), x.stride(0), nullptr, 0.f, nullptr, 0, ptr(W), ptr(bias), mptr(out), (int)M, (int)K, (int)O,
+                           code_of(x.scalar_type())};
     check(sl::skinny_linear(a, static_cast<cudaStream_t>(call.stream())), "skinny_linear");
     return out;
   }
-  const Tensor in = norm.weight ? rmsnorm_fwd(x.contiguous(), *norm.weight, norm.eps) : x;
-  Tensor y;
-  if (bias) y = at::linear(in, W, *bias);
-  else if (out_in && act == sl::LINEAR_NONE && !residual) { y = *out_in; at::mm_out(y, in, W.t()); return y; }
-  else y = at::mm(in, W.t());
-  if (act != sl::LINEAR_NONE) y = ffn_act_fwd(y, act == sl::LINEAR_SWIGLU ? 1 : 0);
-  if (residual) y = *residual + y;
+  if (out_in && !bias) { Tensor y = *out_in; at::mm_out(y, x, W.t()); return y; }
+  const Tensor y = at::linear(x, W, bias);
   if (out_in) { out_in->copy_(y); return *out_in; }
   return y;
 }
 
-// One token between the residual stream and itself: x (batch, d_model) -> (residual +) mixer(norm(x)).  conv, state and
-// u_prev are updated in place; the new b_prev goes to b_prev itself when every head has its own group, else to a tensor of
-// its own (the heads of a group read the old one at different times).
-std::tuple<Tensor, Tensor, Tensor> mixer_token(const Tensor& x, const OptT& pre_norm, float pre_eps, const Tensor& in_w,
-                                               const Tensor& dw_w, const Tensor& dw_b, const std::vector<Tensor>& biases,
-                                               const Config& cfg, const Tensor& d_skip, const Tensor& norm_w, float norm_eps,
-                                               const Tensor& out_w, const OptT& out_b, const Tensor& conv, const Tensor& state,
-                                               const Tensor& b_prev, const Tensor& u_prev, const OptT& workspace, int heads,
-                                               int groups, int P, int N, const OptT& residual, const OptT& out) {
-  Call call(x, pre_norm, in_w, dw_w, dw_b, d_skip, norm_w, out_w, out_b, conv, state, b_prev, u_prev, workspace, residual, out);
+// One token x (batch, d_model) -> mixer(x).  conv, state and u_prev are updated in place; the new b_prev goes to b_prev
+// itself when every head has its own group, else to a tensor of its own (the heads of a group read the old one at different
+// times).
+std::tuple<Tensor, Tensor, Tensor> mixer_token(const Tensor& x, const Tensor& in_w, const Tensor& dw_w, const Tensor& dw_b,
+                                               const std::vector<Tensor>& biases, const Config& cfg, const Tensor& d_skip,
+                                               const Tensor& norm_w, float norm_eps, const Tensor& out_w, const OptT& out_b,
+                                               const Tensor& conv, const Tensor& state, const Tensor& b_prev,
+                                               const Tensor& u_prev, const OptT& workspace, int heads, int groups, int P, int N,
+                                               const OptT& out) {
+  Call call(x, in_w, dw_w, dw_b, d_skip, norm_w, out_w, out_b, conv, state, b_prev, u_prev, workspace, out);
   for (const auto& t : biases) call.need(t);
   const int64_t batch = x.size(0), C = (int64_t)heads * P, O = in_w.size(0);
   const int io = code_of(x.scalar_type());
   const bool chained = small_batch(x, in_w);   // the step may start behind our own in_proj kernel
-  const Tensor proj = linear_rows(call, x, Norm{pre_norm, pre_eps}, in_w, {}, sl::LINEAR_NONE, {}, {});
+  const Tensor proj = linear_rows(call, x, in_w, {}, {});
   const size_t ws_bytes = sl_mixer_decode_step_workspace_bytes(batch, heads, P);
   Tensor ws = workspace && (size_t)workspace->numel() >= ws_bytes ? *workspace : call.bytes(ws_bytes);
   Tensor b_next = groups == heads ? b_prev : at::empty_like(b_prev);
@@ -373,22 +365,15 @@ std::tuple<Tensor, Tensor, Tensor> mixer_token(const Tensor& x, const OptT& pre_
   if (batch <= 64 && K % 8 == 0 && K <= 4096 && io != SL_F32 && out_w.is_contiguous()) {   // the row norm inside the projection
     Tensor y = out ? *out : call.empty({batch, OO}, x.scalar_type());
     const sl::SkinnyArgs s{mptr(ws), C, ptr(norm_w), norm_eps, sl::step_partials(mptr(ws), batch, heads, P), 8 * heads, ptr(out_w),
-                           ptr(out_b), ptr(residual), mptr(y), (int)batch, (int)K, (int)OO, sl::LINEAR_NONE, io, true};
+                           ptr(out_b), mptr(y), (int)batch, (int)K, (int)OO, io, true};
     check(sl::skinny_linear(s, st), "skinny_linear");
     return {y, b_next, ws};
   }
   Tensor normed = call.empty({batch, C}, x.scalar_type());
   check(sl::mixer_step_norm(mptr(ws), ptr(norm_w), norm_eps, mptr(normed), batch, heads, P, io, st), "mixer_step");
-  return {linear_rows(call, normed, Norm{}, out_w, out_b, sl::LINEAR_NONE, residual, out), b_next, ws};
+  return {linear_rows(call, normed, out_w, out_b, out), b_next, ws};
 }
 
-// x (batch, d_model) -> x + out_proj(act(in_proj(norm(x)))); kind 0: GELU, 1: SwiGLU
-Tensor ffn_token(const Tensor& x, const Tensor& norm_w, float eps, const Tensor& w1, const OptT& b1, const Tensor& w2,
-                 const OptT& b2, int kind) {
-  Call call(x, norm_w, w1, b1, w2, b2);
-  const Tensor hidden = linear_rows(call, x, Norm{norm_w, eps}, w1, b1, kind == 1 ? sl::LINEAR_SWIGLU : sl::LINEAR_GELU, {}, {});
-  return linear_rows(call, hidden, Norm{}, w2, b2, sl::LINEAR_NONE, x, {}, small_batch(x, w1));
-}
 // One token of a mixer, or of a whole block, without Python per launch.  A plan holds the parameters of one module (the
 // tensors themselves, so data that moves or changes type is seen) and a list of guards: dictionary entries that must still be
 // the objects they were, and dictionaries that must still be empty (hooks, overrides).  Checking the guards costs 2 us, what
@@ -412,14 +397,13 @@ class TokenPlan {
     return true;
   }
 
-  // None where the call is not the plain one; else (out, next b_prev, workspace).  dependent: x is the result of a plan's
-  // step that was the last thing launched on this stream.
+  // None where the call is not the plain one; else (out, next b_prev, workspace).
   py::object step(const Tensor& x, const OptT& conv, const OptT& state, const OptT& b_prev, const OptT& u_prev,
-                  const OptT& workspace, bool dependent) const {
+                  const OptT& workspace) const {
     if (at::GradMode::is_enabled() || at::autocast::is_autocast_enabled(at::kCUDA) || !x.is_cuda() || x.dim() != 2) return py::none();
     const auto type = x.scalar_type();
     const int64_t M = x.size(0), D = x.size(1), C = heads_ * P_;
-    if ((type != at::kBFloat16 && type != at::kHalf) || M < 1 || M > 64 || x.stride(1) != 1 || x.stride(0) % 8 != 0) return py::none();
+    if ((type != at::kBFloat16 && type != at::kHalf) || M < 1) return py::none();
     auto is = [&](const OptT& t, at::ScalarType ty, at::IntArrayRef shape) {
       return t && t->scalar_type() == ty && t->device() == x.device() && t->is_contiguous() && t->sizes() == shape;
     };
@@ -430,51 +414,63 @@ class TokenPlan {
     ok = ok && is(conv, type, {M, C, d_conv_ - 1}) && is(state, at::kFloat, {M, heads_, P_, 2 * N_}) &&
          is(b_prev, type, {M, groups_, 2 * N_}) && is(u_prev, type, {M, heads_, P_});
     const bool block = !b_.empty(), ffn = b_.size() == 6;
-    int64_t F = 0;
-    if (block) ok = ok && is(b_[0], type, {D});
+    if (block) ok = ok && is(b_[0], type, {D}) && D % 8 == 0 && D <= 2048;   // (what the row kernel of the norm takes)
     if (ok && ffn) {
-      F = b_[4] ? b_[4]->size(1) : 0;
-      const int64_t wide = ffn_kind_ == 1 ? 2 * F : F;
+      const int64_t F = b_[4] ? b_[4]->size(1) : 0, wide = ffn_kind_ == 1 ? 2 * F : F;
       ok = is(b_[1], type, {D}) && is(b_[2], type, {wide, D}) && (!b_[3] || is(b_[3], type, {wide})) && is(b_[4], type, {D, F}) &&
-           (!b_[5] || is(b_[5], type, {D}));
+           (!b_[5] || is(b_[5], type, {D})) && F % 8 == 0;
     }
     const int io = code_of(type);
-    ok = ok && sl::skinny_supported(M, D, O, io) && sl::skinny_supported(M, C, D, io) && (!ffn || sl::skinny_supported(M, F, D, io));
+    if (!block) ok = ok && x.stride(1) == 1 && x.stride(0) % 8 == 0 && sl::skinny_supported(M, D, O, io) && sl::skinny_supported(M, C, D, io);
     if (!ok) return py::none();
 
     Call call(x);
     const auto st = static_cast<cudaStream_t>(call.stream());
-    // scratch: the step's own, the projection, the residual stream between the branches, the hidden row
-    const int64_t e = 2;
+    const Tensor b_next = groups_ == heads_ ? *b_prev : at::empty_like(*b_prev);
     auto up = [](int64_t n) { return (n + 255) / 256 * 256; };
-    const int64_t n_step = up(sl_mixer_decode_step_workspace_bytes(M, heads_, P_)), n_proj = up(M * O * e), n_mid = up(M * D * e);
-    const int64_t need = n_step + n_proj + n_mid + up(M * F * e);
+    const int64_t n_step = up(sl_mixer_decode_step_workspace_bytes(M, heads_, P_)), need = n_step + (block ? 0 : up(M * O * 2));
     const Tensor ws = workspace && workspace->numel() >= need && workspace->device() == x.device() ? *workspace : call.bytes(need);
     auto* const base = static_cast<uint8_t*>(ws.data_ptr());
-    void *const proj = base + n_step, *const mid = base + n_step + n_proj, *const hidden = base + n_step + n_proj + n_mid;
-    const Tensor out = call.empty({M, D}, type);
-    const Tensor b_next = groups_ == heads_ ? *b_prev : at::empty_like(*b_prev);
-
-    const Tensor rows = block && x.stride(0) != D ? x.contiguous() : x;   // (before the chain: it may launch a copy)
-    const sl::SkinnyArgs in{ptr(x), x.stride(0), block ? ptr(b_[0]) : nullptr, (float)eps_[0], nullptr, 0, ptr(p_[0]), nullptr, nullptr,
-                            proj, (int)M, (int)D, (int)O, sl::LINEAR_NONE, io, dependent};
-    check(sl::skinny_linear(in, st), "skinny_linear");
-    const auto* row = static_cast<const uint8_t*>(proj);
-    const sl::MixerStepArgs a{row, row + C * e, row + 2 * C * e, row + (2 * C + 3 * heads_) * e, O, O, O, O, ptr(p_[1]), ptr(p_[2]),
-                              mptr(conv), (int)d_conv_, fptr(p_[3]), fptr(p_[4]), fptr(p_[5]), fptr(p_[6]), fptr(p_[7]), &cfg_,
-                              fptr(p_[8]), mfptr(state), ptr(b_prev), mptr(b_next), mptr(u_prev), base, (size_t)n_step, (int)M,
-                              (int)heads_, (int)groups_, (int)P_, (int)N_, io, true};
-    check(sl::mixer_step_launch(a, st), "mixer_step");
-    const sl::SkinnyArgs o{base, C, ptr(p_[9]), (float)eps_[1], sl::step_partials(base, M, heads_, P_), (int)(8 * heads_), ptr(p_[10]),
-                           ptr(p_[11]), block ? ptr(rows) : nullptr, ffn ? mid : mptr(out), (int)M, (int)C, (int)D, sl::LINEAR_NONE, io, true};
-    check(sl::skinny_linear(o, st), "skinny_linear");
+    // rows of the in_proj output -> gated values and their partial sums of squares in the workspace
+    auto mixer_step = [&](const void* gate, const void* value, const void* params, const void* bc, int64_t gv, int64_t ps, int64_t bs,
+                          bool dependent) {
+      const sl::MixerStepArgs a{gate, value, params, bc, gv, gv, ps, bs, ptr(p_[1]), ptr(p_[2]), mptr(conv), (int)d_conv_, fptr(p_[3]),
+                                fptr(p_[4]), fptr(p_[5]), fptr(p_[6]), fptr(p_[7]), &cfg_, fptr(p_[8]), mfptr(state), ptr(b_prev),
+                                mptr(b_next), mptr(u_prev), base, (size_t)n_step, (int)M, (int)heads_, (int)groups_, (int)P_, (int)N_,
+                                io, dependent};
+      check(sl::mixer_step_launch(a, st), "mixer_step");
+    };
+    if (!block) {   // in_proj, step, and out_proj with the row norm inside, each behind the kernel before it
+      const Tensor out = call.empty({M, D}, type);
+      uint8_t* const row = base + n_step;
+      const sl::SkinnyArgs in{ptr(x), x.stride(0), nullptr, 0.f, nullptr, 0, ptr(p_[0]), nullptr, row, (int)M, (int)D, (int)O, io};
+      check(sl::skinny_linear(in, st), "skinny_linear");
+      mixer_step(row, row + C * 2, row + 2 * C * 2, row + (2 * C + 3 * heads_) * 2, O, O, O, true);
+      const sl::SkinnyArgs o{base, C, ptr(p_[9]), (float)eps_[1], sl::step_partials(base, M, heads_, P_), (int)(8 * heads_), ptr(p_[10]),
+                             ptr(p_[11]), mptr(out), (int)M, (int)C, (int)D, io, true};
+      check(sl::skinny_linear(o, st), "skinny_linear");
+      return py::make_tuple(out, b_next, ws);
+    }
+    // A block: the library's products at the shapes and in the order of the composed path.  Any other order of their sums moves
+    // last bits, which residual stream, norms and B/C phases carry on from block to block: six blocks of width 1024 end up 1.6 % from
+    // the composed token (the small-batch kernel, or one product for the three parts of in_proj).
+    at::AutoDispatchBelowAutograd below;
+    const Tensor rows = x.contiguous(), normed = rmsnorm_fwd(rows, *b_[0], (float)eps_[0]);
+    auto product = [](const Tensor& a, const Tensor& W, int64_t row, int64_t n) {   // a (rows row .. row + n of W)^T
+      return at::mm(a, W.as_strided({W.size(1), n}, {1, W.size(1)}, W.storage_offset() + row * W.size(1)));
+    };
+    auto linear = [&](const Tensor& a, const Tensor& W, const OptT& bias) {
+      return bias ? at::linear(a, W, bias) : product(a, W, 0, W.size(0));
+    };
+    const Tensor gv = product(normed, *p_[0], 0, 2 * C), params = product(normed, *p_[0], 2 * C, 3 * heads_),
+                 bc = product(normed, *p_[0], 2 * C + 3 * heads_, 4 * groups_ * N_);
+    mixer_step(gv.data_ptr(), column(gv, C), params.data_ptr(), bc.data_ptr(), 2 * C, 3 * heads_, 4 * groups_ * N_, false);
+    const Tensor hid = call.empty({M, C}, type);
+    check(sl::mixer_step_norm(base, ptr(p_[9]), (float)eps_[1], mptr(hid), M, heads_, P_, io, st), "mixer_step");
+    Tensor out = rows + linear(hid, *p_[10], p_[11]);
     if (ffn) {
-      const sl::SkinnyArgs f1{mid, D, ptr(b_[1]), (float)eps_[2], nullptr, 0, ptr(b_[2]), ptr(b_[3]), nullptr, hidden, (int)M, (int)D,
-                              (int)F, ffn_kind_ == 1 ? sl::LINEAR_SWIGLU : sl::LINEAR_GELU, io, true};
-      check(sl::skinny_linear(f1, st), "skinny_linear");
-      const sl::SkinnyArgs f2{hidden, F, nullptr, 0.f, nullptr, 0, ptr(b_[4]), ptr(b_[5]), mid, mptr(out), (int)M, (int)F, (int)D,
-                              sl::LINEAR_NONE, io, true};
-      check(sl::skinny_linear(f2, st), "skinny_linear");
+      const Tensor wide = linear(rmsnorm_fwd(out, *b_[1], (float)eps_[2]), *b_[2], b_[3]);
+      out = out + linear(ffn_act_fwd(wide, ffn_kind_), *b_[4], b_[5]);
     }
     return py::make_tuple(out, b_next, ws);
   }
@@ -512,7 +508,6 @@ struct MixerWeights {
   float eps;
 };
 Tensor as_typed(const Tensor& t, at::ScalarType type) { return t.to(type).contiguous(); }
-uint8_t* column(const Tensor& rows, int64_t c) { return static_cast<uint8_t*>(rows.data_ptr()) + c * rows.element_size(); }
 
 sl::ScanPrepArgs scanprep_args(const MixerShape& s, const MixerWeights& w, const Tensor& proj, const void* conv_in, void* conv_out) {
   const ULayout lay = u_layout(true, s.heads, s.T, s.P);
@@ -874,7 +869,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("mixer_infer", &mixer_infer);
   m.def("ffn_train", &ffn_train);
   m.def("mixer_token", &mixer_token);
-  m.def("ffn_token", &ffn_token);
   // (a copied or unpickled module makes a plan of its own)
   py::class_<TokenPlan>(m, "TokenPlan")
       .def(py::init<std::vector<py::tuple>, std::vector<py::dict>, std::vector<OptT>, std::vector<OptT>, std::vector<double>,

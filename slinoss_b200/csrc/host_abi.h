@@ -37,20 +37,18 @@ SL_API int mixer_step_launch(const MixerStepArgs& a, cudaStream_t st);
 SL_API int mixer_step_norm(const void* workspace, const void* norm_weight, float eps, void* normed, int batch, int heads,
                            int P, int io_dtype, cudaStream_t st);
 
-// y (M, O) = act(norm(x) W^T + bias) (+ residual), 16-bit, M <= 64 rows.  norm: none, RMSNorm with weight, or RMSNorm
-// whose sums of squares are given as partials per row.
-enum { LINEAR_NONE = 0, LINEAR_GELU = 1, LINEAR_SWIGLU = 2 };
+// y (M, O) = norm(x) W^T + bias, 16-bit, M <= 64 rows.  norm: none, or RMSNorm whose sums of squares are given as partials
+// per row.
 struct SkinnyArgs {
   const void* x;          // (M, K), row stride x_stride
   int64_t x_stride;
   const void* norm_weight;   // (K) or null
   float norm_eps;
-  const float* partials;  // (M, n_partials) or null
+  const float* partials;  // (M, n_partials), with norm_weight
   int n_partials;
-  const void *weight, *bias;   // (O, K) dense [SwiGLU: (2 O, K), value rows then gate rows], bias or null
-  const void* residual;   // (M, O) dense or null
+  const void *weight, *bias;   // (O, K) dense, bias (O) or null
   void* out;              // (M, O) dense
-  int M, K, O, act, io_dtype;
+  int M, K, O, io_dtype;
   bool dependent = false;   // launched right behind a kernel of this library that wrote x (and no parameter)
 };
 SL_API bool skinny_supported(int M, int K, int O, int io_dtype);

@@ -1,16 +1,13 @@
-// Linear layers of a decode token: y (M, O) = act(norm(x) W^T + bias) (+ residual) for M <= 64 rows of 16-bit values.
+// Linear layers of a mixer's decode token: y (M, O) = norm(x) W^T + bias for M <= 64 rows of 16-bit values.
 //
-// Bound by reading W once (O K 2 bytes); at these sizes also by launches, so what surrounds the product - RMSNorm of
-// the input, bias, activation, residual - happens inside.  A library GEMM pads M to its tile and took 4 to 6 us for
-// each of the five products of a block; the norms, the activation and the residual were launches of their own.
+// Bound by reading W once (O K 2 bytes); at these sizes also by launches, so the row norm in front of the output projection
+// is applied as x is read (its sums of squares come with x).  A library GEMM pads M to its tile and took 4 to 6 us.
 //
 // A CTA owns 8 NT output rows; its warps split K in runs of 256.  W is the (n = 8) operand of mma.sync m16n8k16: a
 // lane reads 16 consecutive bytes of one row of W (four lanes cover 64 bytes) and uses them for two k-steps under a
 // permutation of k that the x fragments share.  All loads of a run are requested before anything else is done, so a
 // warp has 4 KB NT in flight; x comes through L1, where all CTAs of an SM find it.  The warps' partial products meet
 // in shared memory.  mma.sync, not tcgen05: the tensor pipe idles either way and fragments stay in registers.
-#include <atomic>
-
 #include "common.cuh"
 #include "host_abi.h"
 
@@ -29,7 +26,6 @@ template <> __device__ __forceinline__ void mma16816<__half>(float (&d)[4], cons
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <typename T> __device__ __forceinline__ float round_io(float v) { return to_f32(from_f32<T>(v)); }
 template <typename T> __device__ __forceinline__ uint4 scale_pieces(uint4 x, float s, uint4 w) {   // round(x s w)
   float xv[8], wv[8];
   unpack16<T>(x, xv);
@@ -42,18 +38,15 @@ template <typename T> __device__ __forceinline__ uint4 scale_pieces(uint4 x, flo
 }
 
 constexpr int KRUN = 256;                 // k values of a warp
-// MT: 16-row tiles of x; NT: 8-row tiles of W per warp (SwiGLU: NT / 2 of values and as many of gates).
-// KEEP (with a norm, up to 8 warps and 32 rows): the warp's fragments of x stay in registers, so that x is read once and its
-// sums of squares come from there; a pass of its own over x put a load and a reduction per row and warp in front of the
-// product (width 512, 8 rows: 7.1 -> 5.4 us per kernel).
-template <typename T, int MT, int NT, bool SWIGLU, bool KEEP>
+// MT: 16-row tiles of x; NT: 8-row tiles of W per warp.
+// KEEP (with the norm, up to 8 warps): the warp's fragments of x are requested ahead of the row scales that they wait for.
+template <typename T, int MT, int NT, bool KEEP>
 __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyArgs p) {
   constexpr int STEPS = KRUN / 32;
-  constexpr int OT = SWIGLU ? NT / 2 : NT;            // output tiles of the CTA
   extern __shared__ __align__(16) float s_acc[];      // [warps][16 MT][8 NT]
-  __shared__ float s_rstd[64], s_ss[KEEP ? 8 : 1][16 * MT];
+  __shared__ float s_rstd[16 * MT];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
-  const int g = lane >> 2, t = lane & 3, o0 = blockIdx.x * 8 * OT;
+  const int g = lane >> 2, t = lane & 3, o0 = blockIdx.x * 8 * NT;
   const T* W = reinterpret_cast<const T*>(p.weight);
 
   grid_release();
@@ -62,33 +55,24 @@ __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyA
   const int k0 = w * KRUN + 8 * t;
 #pragma unroll
   for (int j = 0; j < NT; ++j) {
-    const int r = (SWIGLU && j >= OT ? p.O + o0 + 8 * (j - OT) : o0 + 8 * j) + g;
-    const bool row_ok = o0 + 8 * (SWIGLU && j >= OT ? j - OT : j) + g < p.O;
+    const int r = o0 + 8 * j + g;
 #pragma unroll
     for (int s = 0; s < STEPS; ++s) {
       wv[j][s] = make_uint4(0u, 0u, 0u, 0u);
-      if (row_ok && k0 + 32 * s < p.K) wv[j][s] = __ldg(reinterpret_cast<const uint4*>(W + (size_t)r * p.K + k0 + 32 * s));
+      if (r < p.O && k0 + 32 * s < p.K) wv[j][s] = __ldg(reinterpret_cast<const uint4*>(W + (size_t)r * p.K + k0 + 32 * s));
     }
   }
   grid_wait();
   // this CTA's rows
   const int mb = blockIdx.y * 16 * MT, M = min(p.M - mb, 16 * MT);
   const T* X = reinterpret_cast<const T*>(p.x) + (size_t)mb * p.x_stride;
-  const float* partials = p.partials ? p.partials + (size_t)mb * p.n_partials : nullptr;
-  const T *bias = reinterpret_cast<const T*>(p.bias), *residual = reinterpret_cast<const T*>(p.residual);
-  if (residual) residual += (size_t)mb * p.O;
-  // ---- row scales of the norm, while W is on its way ------------------------------------------------------------
+  const T* bias = reinterpret_cast<const T*>(p.bias);
   const bool norm = p.norm_weight != nullptr;
-  // the first output of this thread: its residual and bias are requested ahead of the product
-  const int m0 = tid / (8 * OT), c0 = tid % (8 * OT);
-  const bool out0 = tid < M * 8 * OT && o0 + c0 < p.O;
-  const float res0 = out0 && residual ? to_f32(residual[(size_t)m0 * p.O + o0 + c0]) : 0.f;
-  const float bias0 = out0 && bias ? to_f32(bias[o0 + c0]) : 0.f;
+  // the bias of this thread's first output is requested ahead of the product
+  const int c0 = tid % (8 * NT);
+  const float bias0 = bias && tid < M * 8 * NT && o0 + c0 < p.O ? to_f32(bias[o0 + c0]) : 0.f;
   uint4 xk[KEEP ? STEPS : 1][KEEP ? MT : 1][2];
   if constexpr (KEEP) {
-    float sq[2 * MT];
-#pragma unroll
-    for (int i = 0; i < 2 * MT; ++i) sq[i] = 0.f;
 #pragma unroll
     for (int s = 0; s < STEPS; ++s)
 #pragma unroll
@@ -97,42 +81,17 @@ __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyA
         if (8 * i + g < M && k0 + 32 * s < p.K)
           xk[s][i / 2][i % 2] = *reinterpret_cast<const uint4*>(X + (size_t)(8 * i + g) * p.x_stride + k0 + 32 * s);
       }
-    if (!partials) {
-#pragma unroll
-      for (int s = 0; s < STEPS; ++s)
-#pragma unroll
-        for (int i = 0; i < 2 * MT; ++i) {
-          float v[8];
-          unpack16<T>(xk[s][i / 2][i % 2], v);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) sq[i] += v[q] * v[q];
-        }
-#pragma unroll
-      for (int i = 0; i < 2 * MT; ++i) {
-        sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], 1);
-        sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], 2);
-        if (t == 0) s_ss[w][8 * i + g] = sq[i];
-      }
-    }
   }
-  if (norm && !(KEEP && !partials)) {
+  // ---- row scales of the norm, while W is on its way ------------------------------------------------------------
+  if (norm) {
     for (int m = w; m < M; m += nw) {
       float ss = 0.f;
-      if (partials) {
-        for (int k = lane; k < p.n_partials; k += 32) ss += partials[(size_t)m * p.n_partials + k];
-      } else {
-        for (int k = 8 * lane; k < p.K; k += 256) {
-          float v[8];
-          load16<T>(X + (size_t)m * p.x_stride + k, v);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) ss += v[q] * v[q];
-        }
-      }
+      for (int k = lane; k < p.n_partials; k += 32) ss += p.partials[(size_t)(mb + m) * p.n_partials + k];
       ss = warp_sum(ss);
       if (lane == 0) s_rstd[m] = rsqrtf(ss / (float)p.K + p.norm_eps);
     }
+    __syncthreads();
   }
-  if (norm) __syncthreads();
   // ---- products ---------------------------------------------------------------------------------------------------
   float acc[MT][NT][4];
 #pragma unroll
@@ -143,17 +102,7 @@ __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyA
       for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
   float rs[2 * MT];
 #pragma unroll
-  for (int i = 0; i < 2 * MT; ++i) {
-    rs[i] = 0.f;
-    if (!norm || g + 8 * i >= M) continue;
-    if (KEEP && !partials) {
-      float ss = 0.f;
-      for (int q = 0; q < nw; ++q) ss += s_ss[q][8 * i + g];
-      rs[i] = rsqrtf(ss / (float)p.K + p.norm_eps);
-    } else {
-      rs[i] = s_rstd[g + 8 * i];
-    }
-  }
+  for (int i = 0; i < 2 * MT; ++i) rs[i] = norm && g + 8 * i < M ? s_rstd[g + 8 * i] : 0.f;
 #pragma unroll
   for (int s = 0; s < STEPS; ++s) {
     const int k = k0 + 32 * s;
@@ -193,49 +142,35 @@ __global__ void __launch_bounds__(KEEP ? 256 : 512) skinny_linear_kernel(SkinnyA
         *reinterpret_cast<float2*>(mine + (16 * i + 8 * hh + g) * PITCH + 8 * j + 2 * t) =
             make_float2(acc[i][j][2 * hh], acc[i][j][2 * hh + 1]);
   __syncthreads();
-  for (int idx = tid; idx < M * 8 * OT; idx += blockDim.x) {
-    const int m = idx / (8 * OT), c = idx % (8 * OT), o = o0 + c;
+  for (int idx = tid; idx < M * PITCH; idx += blockDim.x) {
+    const int m = idx / PITCH, c = idx % PITCH, o = o0 + c;
     if (o >= p.O) continue;
-    float v = 0.f, gate = 0.f;
-    for (int q = 0; q < nw; ++q) {
-      v += s_acc[((size_t)q * 16 * MT + m) * PITCH + c];
-      if (SWIGLU) gate += s_acc[((size_t)q * 16 * MT + m) * PITCH + 8 * OT + c];
-    }
-    if (bias) { v += idx == tid ? bias0 : to_f32(bias[o]); if (SWIGLU) gate += to_f32(bias[p.O + o]); }
-    v = round_io<T>(v);
-    if (SWIGLU) v = v * silu_f(round_io<T>(gate));
-    else if (p.act == LINEAR_GELU) v = gelu_tanh_f<true>(v);
-    if (residual) v = round_io<T>(v) + (idx == tid ? res0 : to_f32(residual[(size_t)m * p.O + o]));
+    float v = 0.f;
+    for (int q = 0; q < nw; ++q) v += s_acc[((size_t)q * 16 * MT + m) * PITCH + c];
+    if (bias) v += idx == tid ? bias0 : to_f32(bias[o]);
     reinterpret_cast<T*>(p.out)[(size_t)(mb + m) * p.O + o] = from_f32<T>(v);
   }
 }
 
-template <typename T, int MT, int NT, bool SWIGLU, bool KEEP>
+template <typename T, int MT, int NT, bool KEEP>
 int launch_skinny_as(const SkinnyArgs& a, cudaStream_t st) {
-  auto k = skinny_linear_kernel<T, MT, NT, SWIGLU, KEEP>;
   const int warps = (a.K + KRUN - 1) / KRUN;
-  const size_t smem = (size_t)warps * 16 * MT * 8 * NT * sizeof(float);
-  static std::atomic<unsigned long long> done{0};
-  if (smem > 48 * 1024) {
-    if (int e = ensure_smem(k, 16 * 16 * MT * 8 * NT * sizeof(float), done)) return e;
-  }
-  const int rows = 8 * (SWIGLU ? NT / 2 : NT);
-  return launch_chained(k, dim3((a.O + rows - 1) / rows, (a.M + 16 * MT - 1) / (16 * MT)), (unsigned)(32 * warps), smem, st, a.dependent, a);
+  const size_t smem = (size_t)warps * 16 * MT * 8 * NT * sizeof(float);   // at most 16 warps x 32 rows x 16 columns: 32 KB
+  return launch_chained(skinny_linear_kernel<T, MT, NT, KEEP>, dim3((a.O + 8 * NT - 1) / (8 * NT), (a.M + 16 * MT - 1) / (16 * MT)),
+                        (unsigned)(32 * warps), smem, st, a.dependent, a);
 }
-template <typename T, int MT, int NT, bool SWIGLU>
+template <typename T, int MT, int NT>
 int launch_skinny(const SkinnyArgs& a, cudaStream_t st) {
-  if (a.norm_weight && a.K <= 8 * KRUN) return launch_skinny_as<T, MT, NT, SWIGLU, true>(a, st);
-  return launch_skinny_as<T, MT, NT, SWIGLU, false>(a, st);
+  if (a.norm_weight && a.K <= 8 * KRUN) return launch_skinny_as<T, MT, NT, true>(a, st);
+  return launch_skinny_as<T, MT, NT, false>(a, st);
 }
 template <typename T>
 int launch_skinny_m(const SkinnyArgs& a, cudaStream_t st) {
   // One 16-row tile of x and one 8-row tile of W per warp give the most CTAs and the shortest chain.  A CTA then reads 48 K
   // bytes, and with many rows of a large layer that traffic takes longer than the chain (width 1024: 348 against 358 us per token
   // of four blocks at 32 rows, 588 against 523 at 64; width 512: 284 against 346 at 64).
-  const bool sw = a.act == LINEAR_SWIGLU;
-  if (a.M <= 16 || (long long)a.M * a.K * a.O <= 120000000)
-    return sw ? launch_skinny<T, 1, 2, true>(a, st) : launch_skinny<T, 1, 1, false>(a, st);
-  return sw ? launch_skinny<T, 2, 2, true>(a, st) : launch_skinny<T, 2, 2, false>(a, st);
+  if (a.M <= 16 || (long long)a.M * a.K * a.O <= 120000000) return launch_skinny<T, 1, 1>(a, st);
+  return launch_skinny<T, 2, 2>(a, st);
 }
 
 }  // namespace
@@ -246,7 +181,7 @@ bool skinny_supported(int M, int K, int O, int io_dtype) {
 
 int skinny_linear(const SkinnyArgs& a, cudaStream_t st) {
   if (!skinny_supported(a.M, a.K, a.O, a.io_dtype)) return SL_ERR_UNSUPPORTED;
-  if (!a.x || !a.weight || !a.out) return SL_ERR_NULL_POINTER;
+  if (!a.x || !a.weight || !a.out || (a.norm_weight && !a.partials)) return SL_ERR_NULL_POINTER;
   if (!aligned(a.x, 16) || a.x_stride % 8 || !aligned(a.weight, 16) || (a.norm_weight && !aligned(a.norm_weight, 16)))
     return SL_ERR_BAD_ALIGNMENT;
   const int rc = a.io_dtype == SL_BF16 ? launch_skinny_m<__nv_bfloat16>(a, st) : launch_skinny_m<__half>(a, st);

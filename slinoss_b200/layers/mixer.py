@@ -30,9 +30,9 @@ def _norm_eps(norm: nn.RMSNorm) -> float:
 
 
 @_C.opaque
-def planned_step(module: nn.Module, token: torch.Tensor, state: SLinOSSMixerState, make, chained: bool = False):
+def planned_step(module: nn.Module, token: torch.Tensor, state: SLinOSSMixerState, make):
     """One token through the module's native plan (made by ``make`` and kept while its guards hold), ``state`` updated in
-    place; None where the call needs the composed path.  ``chained``: ``token`` is what another planned step has just returned."""
+    place; None where the call needs the composed path."""
     plan = module.__dict__.get("_token_plan")
     if plan is None or not plan.valid():
         plan = make()
@@ -40,8 +40,7 @@ def planned_step(module: nn.Module, token: torch.Tensor, state: SLinOSSMixerStat
             return None
         module.__dict__["_token_plan"] = plan
     scan = state.scan
-    done = plan.step(token, state.conv, scan.state, scan.b_prev, scan.u_prev, state.__dict__.get("_plan_workspace"),
-                     chained)
+    done = plan.step(token, state.conv, scan.state, scan.b_prev, scan.u_prev, state.__dict__.get("_plan_workspace"))
     if done is None:
         return None
     out, scan.b_prev, state._plan_workspace = done
@@ -243,8 +242,13 @@ class SLinOSSMixer(nn.Module):
     def step(self, x: torch.Tensor, state: SLinOSSMixerState | None = None, *,
              inplace: bool | None = None):
         """One decode token.  ``x (batch, d_model)`` or ``(batch, 1, d_model)``."""
+        return self._step(x, state, inplace, False)
+
+    def _step(self, x, state, inplace, library: bool):
+        """``library``: the projections on the library, as in a whole sequence.  A block asks for them: whatever order
+        of sums another product has, the blocks behind it carry the difference on and multiply it."""
         squeeze = x.ndim == 2
-        if squeeze and state is not None and inplace is not False and x.is_cuda and x.shape[1] == self.d_model:
+        if squeeze and not library and state is not None and inplace is not False and x.is_cuda and x.shape[1] == self.d_model:
             y = planned_step(self, x, state, self._make_token_plan)
             if y is not None:
                 return y, state
@@ -262,7 +266,7 @@ class SLinOSSMixer(nn.Module):
             batch = int(token.shape[0])
             nxt = (self.init_decode_state(batch, device=token.device, dtype=token.dtype)
                    if state is None else (state if inplace else state.clone()))
-            y = self._decode_token(token, nxt).unsqueeze(1)
+            y = self._decode_token(token, nxt, library).unsqueeze(1)
         return (y[:, 0, :], nxt) if squeeze else (y, nxt)
 
     def _fused_decode_ready(self, state: SLinOSSMixerState, token: torch.Tensor) -> bool:
@@ -322,33 +326,30 @@ class SLinOSSMixer(nn.Module):
                                    [self.n_heads, self.bc_groups, self.d_head, self.d_state, self.d_conv], ffn_kind)
 
     @_C.opaque
-    def decode_native(self, token: torch.Tensor, state: SLinOSSMixerState, *, pre_norm=None, residual=None,
-                      workspace=None, out=None) -> torch.Tensor:
-        """One token through the native host module: ``(residual +) mixer(norm(token))`` in three launches (two GEMMs
-        around the fused step) for small batches, with the state updated in place.  ``pre_norm``: an RMSNorm module
-        applied inside the first of them."""
+    def decode_native(self, token: torch.Tensor, state: SLinOSSMixerState, *, workspace=None, out=None) -> torch.Tensor:
+        """One token through the native host module: in_proj, the fused step and out_proj as three launches for small
+        batches, two library GEMMs around the step for others, with the state updated in place."""
         sp, mine, scan, dt = self.scanprep, self._parameters, state.scan, token.dtype
         p = sp._parameters
         if workspace is None:
             workspace = getattr(state, "_step_workspace", None)
         y, b_next, used = _C.host().mixer_token(
-            token, None if pre_norm is None else pre_norm.weight,
-            0.0 if pre_norm is None else _norm_eps(pre_norm), self.in_proj._parameters["weight"],
+            token, self.in_proj._parameters["weight"],
             _C.as_type(mine["dw_weight"], dt), _C.as_type(mine["dw_bias"], dt),
             [_C.as_f32(t) for t in (p["dt_bias"], p["alpha_bias"], p["theta_mod_bias"], p["theta_bias"],
                                     sp._buffers["theta_sign"])],
             [getattr(sp, n) for n in _C.CONFIG_FIELDS], _C.as_f32(mine["d_skip"]),
             _C.as_type(self.out_norm._parameters["weight"], dt), _norm_eps(self.out_norm),
             self.out_proj._parameters["weight"], self.out_proj._parameters["bias"], state.conv, scan.state, scan.b_prev,
-            scan.u_prev, workspace, self.n_heads, self.bc_groups, self.d_head, self.d_state, residual, out)
+            scan.u_prev, workspace, self.n_heads, self.bc_groups, self.d_head, self.d_state, out)
         scan.b_prev = b_next
         if used is not workspace:
             state._step_workspace = used
         return y
 
-    def _decode_token(self, token: torch.Tensor, state: SLinOSSMixerState) -> torch.Tensor:
+    def _decode_token(self, token: torch.Tensor, state: SLinOSSMixerState, library: bool = False) -> torch.Tensor:
         batch = int(token.shape[0])
-        if token.is_cuda and self._fused_decode_ready(state, token) and self._native_decode_ready(token):
+        if not library and token.is_cuda and self._fused_decode_ready(state, token) and self._native_decode_ready(token):
             return self.decode_native(token, state)
         gate, value_proj, params, bc = split_mixer_projection(
             token, self.in_proj.weight, d_inner=self.d_inner, param_proj_dim=self.param_proj_dim)

@@ -1,5 +1,6 @@
-"""The native decode step of a block (small-batch linear kernels, pipelined state update) against the composed path:
-library GEMMs, row kernels, and conv, scan preparation, decode and tail as launches of their own."""
+"""The native decode step of a block (library products and row kernels as one call) and of a mixer (small-batch linear
+kernels, pipelined state update) against the composed path: library GEMMs, row kernels, and conv, scan preparation, decode
+and tail as launches of their own."""
 
 import copy
 import pickle
@@ -111,26 +112,47 @@ def test_mixer_token_by_plan_equals_the_composed_token(batch, monkeypatch):
     assert rel(a.scan.b_prev, b.scan.b_prev) <= 2e-2 and rel(a.conv, b.conv) <= 2e-2
 
 
-@pytest.mark.parametrize("batch, d_model, dtype", [(1, 256, torch.bfloat16), (17, 512, torch.float16), (64, 264, torch.bfloat16)])
-def test_a_stack_token_through_chained_plans_equals_the_composed_token(batch, d_model, dtype, monkeypatch):
+# a deep stack multiplies whatever a product's order of sums moves (1.6 % after one token at the last size), so the plan has
+# to have the composed path's products, bit for bit
+@pytest.mark.parametrize("batch, d_model, dtype, layers, state, groups, kind, tokens", [
+    (1, 256, torch.bfloat16, 4, 64, None, "swiglu", 5), (17, 512, torch.float16, 4, 64, None, "swiglu", 5),
+    (64, 264, torch.bfloat16, 4, 64, None, "swiglu", 5), (65, 128, torch.bfloat16, 3, 32, 1, "gelu", 3),
+    (8, 1024, torch.bfloat16, 6, 128, 1, "swiglu", 20)])
+def test_a_stack_token_through_plans_equals_the_composed_token(batch, d_model, dtype, layers, state, groups, kind, tokens, monkeypatch):
     torch.manual_seed(5)
-    blk = sb.SLinOSSBlockConfig(d_model=d_model, mixer=sb.SLinOSSMixerConfig(d_state=64, d_head=64, expand=1.0),
-                                ffn=sb.SLinOSSMLPConfig(kind="swiglu", expand=2.0, multiple_of=8))
-    stack = sb.SLinOSSStack(sb.SLinOSSStackConfig.uniform(blk, n_layers=4), device=DEV, dtype=dtype).eval()
-    x = torch.randn(5, batch, d_model, device=DEV, dtype=dtype)
+    blk = sb.SLinOSSBlockConfig(d_model=d_model, mixer=sb.SLinOSSMixerConfig(d_state=state, d_head=64, expand=1.0, bc_groups=groups),
+                                ffn=sb.SLinOSSMLPConfig(kind=kind, expand=2.0, multiple_of=8, bias=kind == "gelu"))
+    stack = sb.SLinOSSStack(sb.SLinOSSStackConfig.uniform(blk, n_layers=layers), device=DEV, dtype=dtype).eval()
+    x = torch.randn(tokens, batch, d_model, device=DEV, dtype=dtype)
 
-    def tokens():
+    def run(step):
         with torch.no_grad():
             state = stack.init_decode_state(batch)
             out = []
             for t in x:
-                y, state = stack.step(t, state)
+                y, state = step(t, state)
                 out.append(y)
-        return torch.stack(out)
+        return [torch.stack(out)] + [t for layer in state.layers for t in (layer.mixer.conv, layer.mixer.scan.state,
+                                                                          layer.mixer.scan.b_prev, layer.mixer.scan.u_prev)]
 
-    got = tokens()
-    assert torch.equal(got, tokens())
+    def composed(t, state):    # every product a library call on the weight's own rows
+        for b, layer in zip(stack.blocks, state.layers):
+            m, carried = b.mixer, layer.mixer
+            normed, w = b.mixer_norm(t), m.in_proj.weight
+            gate_value, params, bc = (torch.mm(normed, part.t()) for part in w.split(
+                [2 * m.d_inner, m.param_proj_dim, m.bc_proj_dim]))
+            rows = m.decode_backend.fused_step(m, gate_value[:, :m.d_inner], gate_value[:, m.d_inner:], params, bc, carried)
+            t = t + m.out_proj(rows)
+            t = t + b.ffn(b.ffn_norm(t))
+        return stack.final_norm(t), state
+
+    got = run(stack.step)
+    assert all("_token_plan" in b.__dict__ for b in stack.blocks)
+    want = run(composed)
     monkeypatch.setattr(sb.SLinOSSBlock, "_make_token_plan", lambda self: None)
     for b in stack.blocks:
         b.__dict__.pop("_token_plan", None)
-    assert rel(got, tokens()) <= 2e-2
+    plain = run(stack.step)
+    assert all("_token_plan" not in b.mixer.__dict__ for b in stack.blocks)
+    for a, b, c in zip(got, want, plain):
+        assert a.shape == b.shape and torch.equal(a, b) and torch.equal(a, c)
