@@ -54,11 +54,11 @@ enum { SL_F32 = 0, SL_BF16 = 1, SL_F16 = 2 };
 
 /* kernel family selector for the scan */
 enum {
-  SL_PATH_AUTO = 0, /* tensor-core path when the shape allows, else SIMT */
+  SL_PATH_AUTO = 0, /* tensor-core path when type and sizes allow it, else SIMT */
   SL_PATH_SIMT = 1, /* exact float32 sequential recurrence (any dtype in)     */
-  SL_PATH_TC = 2    /* tcgen05/TMEM chunked path: bf16 / fp16 operands, P = 64, N = 64 or 128
-                       (auto takes every N <= 128 that is a multiple of 4); without the SL_WS_SCAN_FWD workspace
-                       of a problem the forward pass is refused                 */
+  SL_PATH_TC = 2    /* tcgen05/TMEM chunked path: bf16 / fp16 operands, P = 64, N = 64 or 128 (other
+                       sizes are refused here and take SIMT under auto); without the SL_WS_SCAN_FWD
+                       workspace of a problem the forward pass is refused          */
 };
 
 /* workspace kinds for sl_workspace_bytes */

@@ -44,11 +44,6 @@ int check_scan(const void* U, const float* M, const float* K, const void* B, con
   return SL_OK;
 }
 
-// SL_PATH_TC asks for the widths the kernels hold without padding; SL_PATH_AUTO also pads narrower ones to them
-bool tc_on_request(const ScanDims& d, int io_dtype) {
-  return (d.N == 64 || d.N == 128) && scan_tc_supported(d, io_dtype);
-}
-
 bool use_tc(int path, const ScanDims& d, int io_dtype) {
   if (path == SL_PATH_SIMT) return false;
   return scan_tc_supported(d, io_dtype);
@@ -122,7 +117,7 @@ extern "C" int sl_v2x2ssd_fwd(const void* U, const float* M, const float* K, con
   if (!dtype_ok(y_dtype)) return SL_ERR_UNSUPPORTED;
   if (!aligned(Y, 16) || (chunk_states && !aligned(chunk_states, 16))) return SL_ERR_BAD_ALIGNMENT;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (path == SL_PATH_TC && !tc_on_request(d, io_dtype)) return SL_ERR_UNSUPPORTED;
+  if (path == SL_PATH_TC && !scan_tc_supported(d, io_dtype)) return SL_ERR_UNSUPPORTED;
   if (use_tc(path, d, io_dtype))
     return scan_tc_fwd(U, M, K, B, C, initial_states, B_prev, U_prev, Y, final_state,
                        final_state ? chunk_states : nullptr, d, io_dtype, y_dtype, workspace,
@@ -149,7 +144,7 @@ extern "C" int sl_v2x2ssd_bwd(const void* U, const float* M, const float* K, con
     return SL_ERR_BAD_ALIGNMENT;
   if (!dtype_ok(dy_dtype)) return SL_ERR_UNSUPPORTED;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (path == SL_PATH_TC && !tc_on_request(d, io_dtype)) return SL_ERR_UNSUPPORTED;
+  if (path == SL_PATH_TC && !scan_tc_supported(d, io_dtype)) return SL_ERR_UNSUPPORTED;
   if (use_tc(path, d, io_dtype))
     return scan_tc_bwd(U, M, K, B, C, initial_states, B_prev, U_prev,
                        final_state ? chunk_states : nullptr, chunk_states ? final_state : nullptr, dY,

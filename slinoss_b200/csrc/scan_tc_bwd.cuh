@@ -148,11 +148,7 @@ __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __g
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const size_t o = ((size_t)bh * 64 + row) * D + 2 * (osc0 + 2 * e);
-        float4 g = make_float4(0.f, 0.f, 0.f, 0.f), z = g;
-        if (osc0 + 2 * e < p.N) {
-          g = *reinterpret_cast<const float4*>(p.dfinal + o);
-          z = *reinterpret_cast<const float4*>(p.zfinal + o);
-        }
+        const float4 g = *reinterpret_cast<const float4*>(p.dfinal + o), z = *reinterpret_cast<const float4*>(p.zfinal + o);
         ar += g.x * z.x + g.y * z.y + g.z * z.z + g.w * z.w;   // d_final * conj(z_final)
         ai += g.y * z.x - g.x * z.y + g.w * z.z - g.z * z.w;
         dza[e] = mk2(g.x, g.z); dzb[e] = mk2(-g.y, -g.w);
@@ -377,16 +373,14 @@ __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __g
           umma(tmem + 384, desc_adv(mDYO, 2048 * k), desc_adv(mQ, 2048 * k), ID_MM128, k > 0);
         umma_commit(&bar_mma[4]);   // dZ
         // (4) output tiles: the workers overwrite dead operand tiles of this stage in place (C with dB,
-        // B with dC, dY with dU) and signal; one TMA store per tile writes full 128-byte rows.  With N <= 32 the
-        // second tile of dB / dC lies outside the tensors.
-        const bool second = 2 * p.N > 128 * blk + 64;
+        // B with dC, dY with dU) and signal; one TMA store per tile writes full 128-byte rows.
         if (!mbar_wait(&bar_st[0], it & 1, wl)) { report_timeout(17); s_abort = 1; break; }
         tma_store_3d(&p.tmdB, tC, 128 * blk, t0, bh);
-        if (second) tma_store_3d(&p.tmdB, tC + TILE, 128 * blk + 64, t0, bh);
+        tma_store_3d(&p.tmdB, tC + TILE, 128 * blk + 64, t0, bh);
         tma_store_commit();
         if (!mbar_wait(&bar_st[1], it & 1, wl)) { report_timeout(18); s_abort = 1; break; }
         tma_store_3d(&p.tmdC, tB, 128 * blk, t0, bh);
-        if (second) tma_store_3d(&p.tmdC, tB + TILE, 128 * blk + 64, t0, bh);
+        tma_store_3d(&p.tmdC, tB + TILE, 128 * blk + 64, t0, bh);
         tma_store_commit();
         if (!mbar_wait(&bar_st[2], it & 1, wl)) { report_timeout(19); s_abort = 1; break; }
         tma_store_3d(&p.tmdU[blk], tDY, 0, t0, bh);
@@ -705,12 +699,10 @@ __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __g
   if (ok && tid == 128 * NW) finish_anchor(n - 1);   // (of the segment before this one)
   if (ok && p.dinit && worker && c_lo == 0) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (osc0 + 2 * e < p.N) {
-        const float2 a = un2(dza[e]), c = un2(dzb[e]);
-        *reinterpret_cast<float4*>(p.dinit + ((size_t)bh * 64 + row) * D + 2 * (osc0 + 2 * e)) =
-            make_float4(a.x, -c.x, a.y, -c.y);
-      }
+    for (int e = 0; e < 4; ++e) {
+      const float2 a = un2(dza[e]), c = un2(dzb[e]);
+      *reinterpret_cast<float4*>(p.dinit + ((size_t)bh * 64 + row) * D + 2 * (osc0 + 2 * e)) = make_float4(a.x, -c.x, a.y, -c.y);
+    }
   }
   // Unwind: nothing of this CTA may still be in flight when shared memory and TMEM are released.  The
   // issue lane started every asynchronous operation (but for the loads of the first iteration), so it

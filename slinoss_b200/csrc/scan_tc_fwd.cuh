@@ -1,7 +1,7 @@
 // Forward kernel of the chunked scan on tcgen05 (included by scan_tc.cu inside its namespaces).
 //
 // One CTA walks the chunks of one segment of one (batch, head) stream.  NB = 64-column blocks of the state
-// dimension held by the CTA (1: N <= 64, 2: N <= 128); NWQ = warps per TMEM lane quadrant.  The CTA has 4 NWQ worker
+// dimension held by the CTA (N = 64 NB); NWQ = warps per TMEM lane quadrant.  The CTA has 4 NWQ worker
 // warps (4 lane quadrants x NWQ column groups), one scalar warp and one issue warp.
 //
 // MODE 0  full forward: Y, final state, optional 16-bit chunk-start states
@@ -46,7 +46,7 @@ struct alignas(64) TcFwdParams {
   void* states16;       // optional (NB, BH, nchunks, 64, 128) 16-bit: conjugated start state of every chunk
   float* seg;           // (BH, nseg, 64, 128 NB) float32: start states (from_seg) or, MODE 1 / 2 pre-pass, results
   float2* seg_pi;       // (BH, nseg): transition product of the segment (pre-pass)
-  int heads, groups, T, N, nchunks, cps, nseg, seg0;   // cps: chunks per segment; seg0: segment of blockIdx.y = 0
+  int heads, groups, T, nchunks, cps, nseg, seg0;   // cps: chunks per segment; seg0: segment of blockIdx.y = 0
   int from_seg;   // start states: 1 given in seg, 2 to be folded from the segments' contributions in seg
   int to_seg;     // pre-pass: leave this segment's contribution in seg
   long long wait_limit;  // SM clocks a wait of the main loop may take before the kernel gives up
@@ -85,7 +85,8 @@ __global__ void __launch_bounds__(128 * NWQ + 64, NWQ == 2 ? 2 : 1)
   const int bg = b * p.groups + h / (p.heads / p.groups);
   const int seg = p.seg0 + blockIdx.y;
   const int c0 = seg * p.cps, n = min(p.cps, p.nchunks - c0);   // this CTA's chunks: c0 .. c0 + n - 1
-  const int T = p.T, D = 2 * p.N;
+  const int T = p.T;
+  constexpr int D = 128 * NB;   // real columns of a state row
   const float* Mb = p.M + (size_t)bh * T * 2;
   const float* Kb = p.K + (size_t)bh * T * 4;
   const long long wl = p.wait_limit;
@@ -156,7 +157,6 @@ __global__ void __launch_bounds__(128 * NWQ + 64, NWQ == 2 ? 2 : 1)
 #pragma unroll
     for (int m = 0; m < ZB / 2; ++m) {
       const int nn = n_of(m);
-      if (nn >= p.N) continue;
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -566,7 +566,6 @@ __global__ void __launch_bounds__(128 * NWQ + 64, NWQ == 2 ? 2 : 1)
 #pragma unroll
       for (int m = 0; m < ZB / 2; ++m) {
         const int nn = n_of(m);
-        if (nn >= p.N) continue;
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           const float2 re = un2(zz[4 * m + hh]), im = un2(zz[4 * m + 2 + hh]);
@@ -593,29 +592,27 @@ __global__ void __launch_bounds__(256) scan_tc_combine_kernel(float* __restrict_
                                                               const TIn* __restrict__ Bprev,
                                                               const TIn* __restrict__ Uprev,
                                                               const float* __restrict__ M, const float* __restrict__ K,
-                                                              int heads, int groups, int T, int N, int nb, int nseg) {
+                                                              int heads, int groups, int T, int N, int nseg) {
   const int e = blockIdx.y * 256 + threadIdx.x, bh = blockIdx.x;
-  const int width = 64 * nb, row = e / width, n = e % width;
+  const int row = e / N, n = e % N;
   if (row >= 64) return;
   float zr = 0.f, zi = 0.f;
-  if (n < N) {
-    if (init) {
-      const float2 z = *reinterpret_cast<const float2*>(init + ((size_t)bh * 64 + row) * 2 * N + 2 * n);
-      zr = z.x; zi = z.y;
-    }
-    if (Bprev) {
-      const int bg = (bh / heads) * groups + (bh % heads) / (heads / groups);
-      float xr, xi;
-      pending_tap(M + (size_t)bh * T * 2, K + (size_t)bh * T * 4, xr, xi);
-      const float br = to_f32(Bprev[(size_t)bg * 2 * N + 2 * n]), bi = to_f32(Bprev[(size_t)bg * 2 * N + 2 * n + 1]);
-      const float u = to_f32(Uprev[(size_t)bh * 64 + row]);
-      zr += u * (xr * br - xi * bi);
-      zi += u * (xr * bi + xi * br);
-    }
+  if (init) {
+    const float2 z = *reinterpret_cast<const float2*>(init + ((size_t)bh * 64 + row) * 2 * N + 2 * n);
+    zr = z.x; zi = z.y;
+  }
+  if (Bprev) {
+    const int bg = (bh / heads) * groups + (bh % heads) / (heads / groups);
+    float xr, xi;
+    pending_tap(M + (size_t)bh * T * 2, K + (size_t)bh * T * 4, xr, xi);
+    const float br = to_f32(Bprev[(size_t)bg * 2 * N + 2 * n]), bi = to_f32(Bprev[(size_t)bg * 2 * N + 2 * n + 1]);
+    const float u = to_f32(Uprev[(size_t)bh * 64 + row]);
+    zr += u * (xr * br - xi * bi);
+    zi += u * (xr * bi + xi * br);
   }
   zi = -zi;
-  const size_t stride = (size_t)64 * 2 * width;
-  float* base = seg + (size_t)bh * nseg * stride + (size_t)row * 2 * width + (n >> 3) * 16 + (n & 7);
+  const size_t stride = (size_t)64 * 2 * N;
+  float* base = seg + (size_t)bh * nseg * stride + (size_t)row * 2 * N + (n >> 3) * 16 + (n & 7);
   const float2* pis = seg_pi + (size_t)bh * nseg;
   for (int k0 = 0; k0 < nseg; k0 += 8) {
     float fr[8], fi[8];

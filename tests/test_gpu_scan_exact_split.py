@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from oracle import scan_np
+from slinoss_b200 import _C
 from slinoss_b200.ops.v2x2ssd import v2x2ssd
 from slinoss_b200.synthetic import make_scan_case
 from tests.util import n64, rel
@@ -36,3 +37,32 @@ def test_split_float32_scan_matches_the_oracle(shape):
     want = scan_np.v2x2ssd_bwd(*args, n64(case.dY), d_final_state=None if d_final is None else n64(d_final), **kw)
     for name, grad in zip(leaves, grads):
         assert rel(grad, want[name]) <= 1e-5, (name, rel(grad, want[name]))
+
+
+# 16-bit operands of widths that the tensor-core kernels do not hold take the float32 sweeps: the operands are exact, so
+# float32 results keep the float32 bar and 16-bit ones add one rounding; a zero transition (a forgotten past) is computed
+# through, where the chunked kernels would divide by it
+@pytest.mark.parametrize("dtype, unit", [(torch.bfloat16, 2.0 ** -8), (torch.float16, 2.0 ** -11)])
+@pytest.mark.parametrize("N, groups, T", [(4, 2, 70), (32, 1, 257), (48, 2, 333), (60, 2, 64), (68, 1, 130), (124, 2, 200)])
+def test_16_bit_operands_of_other_widths_keep_float32_precision(N, groups, T, dtype, unit):
+    case = make_scan_case(1, 2, T, 64, N, groups=groups, dtype=dtype, seed=T + N, streaming=True, with_init=True)
+    zero = T // 3
+    case.M[:, 1, zero] = 0.0
+    c = case.to("cuda")
+    ops = (c.U, c.M, c.K, c.B, c.C, c.initial_states.float(), c.B_prev, c.U_prev)
+    Y, fin, states = _C.scan_fwd(*ops, chunk_size=64, y_dtype=torch.float32, want_final=True, save_states=True)
+    got = _C.scan_bwd(*ops, c.dY, None, chunk_size=64)
+    assert states is None
+    with pytest.raises(RuntimeError):
+        _C.scan_fwd(*ops, chunk_size=64, y_dtype=dtype, want_final=False, path="tc")
+    args = [n64(t) for t in case.tensors()]
+    kw = dict(initial_states=n64(case.initial_states), B_prev=n64(case.B_prev), U_prev=n64(case.U_prev))
+    wY, wfin, _, _ = scan_np.v2x2ssm(*args, **kw)
+    assert rel(Y, wY) <= 1e-5 and rel(fin, wfin) <= 1e-5
+    want = scan_np.v2x2ssd_bwd(*args, n64(case.dY), **kw)
+    want["M"][:, 1, zero] = 0.0    # (not defined by the formula S / conj(m) that the sweeps use)
+    for name, grad in zip(NAMES, got):
+        if name in ("initial_states", "M", "K"):
+            assert grad.dtype == torch.float32 and rel(grad, want[name]) <= 1e-5, (name, rel(grad, want[name]))
+        else:
+            assert grad.dtype == dtype and rel(grad, want[name]) <= unit + 1e-5, (name, rel(grad, want[name]))

@@ -1,6 +1,6 @@
-"""The tensor-core scan where it is split in time and where N is padded to the kernels' column blocks, against the
-oracle: segments of one and of several chunks, a last segment that is shorter, ragged last chunks, carried state
-and taps, grouped B/C, widths at the edges of the 64-column tiles."""
+"""16-bit scans against the oracle: the tensor-core kernels where they are split in time (segments of one and of several
+chunks, a last segment that is shorter, ragged last chunks, carried state and taps, grouped B/C), and widths around the
+64 and 128 columns that these hold, which take the float32 sweeps."""
 
 import pytest
 import torch
