@@ -132,8 +132,9 @@ class SLinOSSBlock(nn.Module):
         kids = self._modules
         if type(norm) is not RMSNorm or norm.weight is None:
             return None
-        held = [(kids if n in kids else self.__dict__, n) for n in ("mixer", "mixer_norm", "ffn", "ffn_norm")]
-        same = [(d, n, d[n]) for d, n in held]
+        # (None: this block's __dict__, which keeps the plan)
+        same = [(kids, n, kids[n]) if n in kids else (None, n, self.__dict__[n])
+                for n in ("mixer", "mixer_norm", "ffn", "ffn_norm")]
         same.append((norm._parameters, "weight", norm.weight))
         empty = [mixer._forward_hooks, mixer._forward_pre_hooks, norm._forward_hooks, norm._forward_pre_hooks]
         branch, ffn_eps, kind = [norm.weight], 0.0, 0

@@ -378,8 +378,13 @@ std::tuple<Tensor, Tensor, Tensor> mixer_token(const Tensor& x, const Tensor& in
 // tensors themselves, so data that moves or changes type is seen) and a list of guards: dictionary entries that must still be
 // the objects they were, and dictionaries that must still be empty (hooks, overrides).  Checking the guards costs 2 us, what
 // they replace - attribute lookups, conversions of 30 arguments, checks of every tensor - cost 25 us per block.
+//
+// The module keeps its plan in its own __dict__, so the plan does not hold that one: its entries are guards without a
+// dictionary, and valid() is given it.  What the plan does hold it shows to the garbage collector, for modules that lie on a
+// cycle of the program's own.
 class TokenPlan {
  public:
+  // same: (dict or None for the module's own, key, object);
   // params: in_w dw_w dw_b dt alpha theta_mod theta theta_sign d_skip norm_w out_w out_b; branch: pre_norm [ffn_norm w1 b1 w2 b2]
   TokenPlan(std::vector<py::tuple> same, std::vector<py::dict> empty, std::vector<OptT> params, std::vector<OptT> branch,
             std::vector<double> eps, const Config& cfg, std::array<int64_t, 5> dims, int ffn_kind)
@@ -389,18 +394,42 @@ class TokenPlan {
       throw pybind11::value_error("bad plan.");
   }
 
-  bool valid() const {
-    for (const auto& g : same_)
-      if (PyDict_GetItem(PyTuple_GET_ITEM(g.ptr(), 0), PyTuple_GET_ITEM(g.ptr(), 1)) != PyTuple_GET_ITEM(g.ptr(), 2)) return false;
+  bool valid(const py::dict& own) const {
+    if (cleared_) return false;
+    for (const auto& g : same_) {
+      PyObject* const d = PyTuple_GET_ITEM(g.ptr(), 0);
+      if (PyDict_GetItem(d == Py_None ? own.ptr() : d, PyTuple_GET_ITEM(g.ptr(), 1)) != PyTuple_GET_ITEM(g.ptr(), 2)) return false;
+    }
     for (const auto& d : empty_)
       if (PyDict_Size(d.ptr()) != 0) return false;
     return true;
   }
 
+  static void collectable(PyHeapTypeObject* heap) {
+    PyTypeObject* const type = &heap->ht_type;
+    type->tp_flags |= Py_TPFLAGS_HAVE_GC;
+    type->tp_traverse = [](PyObject* self, visitproc visit, void* arg) {
+      Py_VISIT(Py_TYPE(self));
+      if (const TokenPlan* const plan = of(self)) {
+        for (const auto& g : plan->same_) Py_VISIT(g.ptr());
+        for (const auto& d : plan->empty_) Py_VISIT(d.ptr());
+      }
+      return 0;
+    };
+    type->tp_clear = [](PyObject* self) {
+      if (TokenPlan* const plan = of(self)) {
+        plan->cleared_ = true;
+        plan->same_.clear(); plan->empty_.clear(); plan->p_.clear(); plan->b_.clear();
+      }
+      return 0;
+    };
+  }
+
   // None where the call is not the plain one; else (out, next b_prev, workspace).
   py::object step(const Tensor& x, const OptT& conv, const OptT& state, const OptT& b_prev, const OptT& u_prev,
                   const OptT& workspace) const {
-    if (at::GradMode::is_enabled() || at::autocast::is_autocast_enabled(at::kCUDA) || !x.is_cuda() || x.dim() != 2) return py::none();
+    if (cleared_ || at::GradMode::is_enabled() || at::autocast::is_autocast_enabled(at::kCUDA) || !x.is_cuda() || x.dim() != 2)
+      return py::none();
     const auto type = x.scalar_type();
     const int64_t M = x.size(0), D = x.size(1), C = heads_ * P_;
     if ((type != at::kBFloat16 && type != at::kHalf) || M < 1) return py::none();
@@ -476,13 +505,19 @@ class TokenPlan {
   }
 
  private:
-  std::vector<py::tuple> same_;    // (dict, key, value)
+  static TokenPlan* of(PyObject* self) {   // null while the constructor has not run
+    const auto held = reinterpret_cast<py::detail::instance*>(self)->get_value_and_holder();
+    return held.holder_constructed() ? static_cast<TokenPlan*>(held.value_ptr()) : nullptr;
+  }
+
+  std::vector<py::tuple> same_;
   std::vector<py::dict> empty_;
   std::vector<OptT> p_, b_;
   std::vector<double> eps_;        // pre-norm, mixer norm, FFN norm
   sl_scanprep_config cfg_;
   int64_t heads_, groups_, P_, N_, d_conv_;
   int ffn_kind_;
+  bool cleared_ = false;
 };
 
 // ---- the whole mixer over a sequence ------------------------------------------------------------------------------------
@@ -870,7 +905,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("ffn_train", &ffn_train);
   m.def("mixer_token", &mixer_token);
   // (a copied or unpickled module makes a plan of its own)
-  py::class_<TokenPlan>(m, "TokenPlan")
+  py::class_<TokenPlan>(m, "TokenPlan", py::custom_type_setup(&TokenPlan::collectable))
       .def(py::init<std::vector<py::tuple>, std::vector<py::dict>, std::vector<OptT>, std::vector<OptT>, std::vector<double>,
                     const Config&, std::array<int64_t, 5>, int>())
       .def("valid", &TokenPlan::valid)

@@ -34,7 +34,7 @@ def planned_step(module: nn.Module, token: torch.Tensor, state: SLinOSSMixerStat
     """One token through the module's native plan (made by ``make`` and kept while its guards hold), ``state`` updated in
     place; None where the call needs the composed path."""
     plan = module.__dict__.get("_token_plan")
-    if plan is None or not plan.valid():
+    if plan is None or not plan.valid(module.__dict__):
         plan = make()
         if plan is None:
             return None
@@ -291,11 +291,10 @@ class SLinOSSMixer(nn.Module):
                 and w_in.dtype == token.dtype and w_out.dtype == token.dtype and w_in.device == token.device
                 and w_in.is_contiguous() and not torch.is_autocast_enabled())
 
-    def _plan_guards(self):
+    def _plan_guards(self, mine):
         """What a native token plan of this module relies on: (dictionary, key, object) entries, and dictionaries that
-        stay empty."""
-        sp, out = self.scanprep, self.out_proj
-        mine, kids = self.__dict__, self._modules
+        stay empty.  ``mine``: this module's ``__dict__``, or None where the plan is kept in it."""
+        sp, out, kids = self.scanprep, self.out_proj, self._modules
         same = [(kids, n, kids[n]) for n in ("scanprep", "in_proj", "out_norm", "out_proj")]
         same += [(mine, "decode_backend", self.decode_backend)]
         for m, names in ((self, ("dw_weight", "dw_bias", "d_skip")), (self.in_proj, ("weight",)), (out, ("weight", "bias")),
@@ -314,7 +313,7 @@ class SLinOSSMixer(nn.Module):
                 and self.out_norm.weight is not None and not self.decode_backend.__dict__
                 and all(n in sp.__dict__ for n in _C.CONFIG_FIELDS)):
             return None
-        same, empty = self._plan_guards()
+        same, empty = self._plan_guards(self.__dict__ if branch else None)
         if any(len(d) for d in (*empty, *guards[1])):
             return None
         p, mine = sp._parameters, self._parameters
