@@ -130,25 +130,26 @@ class SLinOSSBlock(nn.Module):
     def _make_token_plan(self):
         mixer, ffn, norm = self.mixer, self.ffn, self.mixer_norm
         kids = self._modules
-        if type(norm) is not RMSNorm or norm.weight is None:
+        if type(norm) is not RMSNorm or norm.weight is None or norm.eps is None:
             return None
         # (None: this block's __dict__, which keeps the plan)
         same = [(kids, n, kids[n]) if n in kids else (None, n, self.__dict__[n])
                 for n in ("mixer", "mixer_norm", "ffn", "ffn_norm")]
-        same.append((norm._parameters, "weight", norm.weight))
+        same += [(norm._parameters, "weight", norm.weight), (norm.__dict__, "eps", norm.eps), (norm.__dict__, "forward")]
         empty = [mixer._forward_hooks, mixer._forward_pre_hooks, norm._forward_hooks, norm._forward_pre_hooks]
         branch, ffn_eps, kind = [norm.weight], 0.0, 0
         if ffn is not None:
             fnorm = self.ffn_norm
-            if not (type(ffn) is SLinOSSMLP and type(fnorm) is RMSNorm and fnorm.weight is not None
+            if not (type(ffn) is SLinOSSMLP and type(fnorm) is RMSNorm and fnorm.weight is not None and fnorm.eps is not None
                     and type(ffn.in_proj) is nn.Linear and type(ffn.out_proj) is nn.Linear):
                 return None
             same += [(ffn._modules, n, ffn._modules[n]) for n in ("in_proj", "out_proj")]
-            same += [(ffn.__dict__, "kind", ffn.kind), (fnorm._parameters, "weight", fnorm.weight)]
+            same += [(ffn.__dict__, "kind", ffn.kind), (fnorm._parameters, "weight", fnorm.weight), (fnorm.__dict__, "eps", fnorm.eps)]
             for layer in (ffn.in_proj, ffn.out_proj):
                 same += [(layer._parameters, n, layer._parameters[n]) for n in ("weight", "bias")]
             for m in (ffn, fnorm, ffn.in_proj, ffn.out_proj):
                 empty += [m._forward_hooks, m._forward_pre_hooks]
+                same.append((m.__dict__, "forward"))
             branch += [fnorm.weight, ffn.in_proj.weight, ffn.in_proj.bias, ffn.out_proj.weight, ffn.out_proj.bias]
             ffn_eps, kind = _norm_eps(fnorm), _C.FFN_KINDS[ffn.kind]
         return mixer._make_token_plan(branch, (same, empty), _norm_eps(norm), ffn_eps, kind)

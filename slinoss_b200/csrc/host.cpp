@@ -376,7 +376,7 @@ std::tuple<Tensor, Tensor, Tensor> mixer_token(const Tensor& x, const Tensor& in
 
 // One token of a mixer, or of a whole block, without Python per launch.  A plan holds the parameters of one module (the
 // tensors themselves, so data that moves or changes type is seen) and a list of guards: dictionary entries that must still be
-// the objects they were, and dictionaries that must still be empty (hooks, overrides).  Checking the guards costs 2 us, what
+// the objects they were or still be absent, and dictionaries that must still be empty (hooks).  Checking the guards costs 2 us, what
 // they replace - attribute lookups, conversions of 30 arguments, checks of every tensor - cost 25 us per block.
 //
 // The module keeps its plan in its own __dict__, so the plan does not hold that one: its entries are guards without a
@@ -384,7 +384,7 @@ std::tuple<Tensor, Tensor, Tensor> mixer_token(const Tensor& x, const Tensor& in
 // cycle of the program's own.
 class TokenPlan {
  public:
-  // same: (dict or None for the module's own, key, object);
+  // same: (dict or None for the module's own, key[, object]), without an object: no such entry;
   // params: in_w dw_w dw_b dt alpha theta_mod theta theta_sign d_skip norm_w out_w out_b; branch: pre_norm [ffn_norm w1 b1 w2 b2]
   TokenPlan(std::vector<py::tuple> same, std::vector<py::dict> empty, std::vector<OptT> params, std::vector<OptT> branch,
             std::vector<double> eps, const Config& cfg, std::array<int64_t, 5> dims, int ffn_kind)
@@ -398,7 +398,8 @@ class TokenPlan {
     if (cleared_) return false;
     for (const auto& g : same_) {
       PyObject* const d = PyTuple_GET_ITEM(g.ptr(), 0);
-      if (PyDict_GetItem(d == Py_None ? own.ptr() : d, PyTuple_GET_ITEM(g.ptr(), 1)) != PyTuple_GET_ITEM(g.ptr(), 2)) return false;
+      PyObject* const want = PyTuple_GET_SIZE(g.ptr()) == 3 ? PyTuple_GET_ITEM(g.ptr(), 2) : nullptr;
+      if (PyDict_GetItem(d == Py_None ? own.ptr() : d, PyTuple_GET_ITEM(g.ptr(), 1)) != want) return false;
     }
     for (const auto& d : empty_)
       if (PyDict_Size(d.ptr()) != 0) return false;

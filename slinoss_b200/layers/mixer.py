@@ -25,6 +25,9 @@ from .scanprep import SLinOSSScanPrep, _require
 from .state import ScanState, SLinOSSMixerState
 
 
+_GLOBAL_HOOKS = (torch.nn.modules.module._global_forward_hooks, torch.nn.modules.module._global_forward_pre_hooks)
+
+
 def _norm_eps(norm: nn.RMSNorm) -> float:
     return norm.eps if norm.eps is not None else torch.finfo(norm.weight.dtype).eps
 
@@ -292,17 +295,19 @@ class SLinOSSMixer(nn.Module):
                 and w_in.is_contiguous() and not torch.is_autocast_enabled())
 
     def _plan_guards(self, mine):
-        """What a native token plan of this module relies on: (dictionary, key, object) entries, and dictionaries that
-        stay empty.  ``mine``: this module's ``__dict__``, or None where the plan is kept in it."""
+        """What a native token plan of this module relies on: (dictionary, key, object) entries, (dictionary, key) without
+        an entry, and dictionaries that stay empty.  ``mine``: this module's ``__dict__``, or None where the plan is
+        kept in it."""
         sp, out, kids = self.scanprep, self.out_proj, self._modules
         same = [(kids, n, kids[n]) for n in ("scanprep", "in_proj", "out_norm", "out_proj")]
-        same += [(mine, "decode_backend", self.decode_backend)]
+        same += [(mine, "decode_backend", self.decode_backend), (self.out_norm.__dict__, "eps", self.out_norm.eps)]
+        same += [(out.__dict__, "forward"), (mine, "_decode_token")]   # what an instance may have replaced
         for m, names in ((self, ("dw_weight", "dw_bias", "d_skip")), (self.in_proj, ("weight",)), (out, ("weight", "bias")),
                          (self.out_norm, ("weight",)), (sp, ("dt_bias", "alpha_bias", "theta_mod_bias", "theta_bias"))):
             same += [(m._parameters, n, m._parameters[n]) for n in names]
         same.append((sp._buffers, "theta_sign", sp._buffers["theta_sign"]))
         same += [(sp.__dict__, n, sp.__dict__[n]) for n in _C.CONFIG_FIELDS]
-        empty = [self.decode_backend.__dict__, out._forward_hooks, out._forward_pre_hooks]
+        empty = [self.decode_backend.__dict__, out._forward_hooks, out._forward_pre_hooks, *_GLOBAL_HOOKS]
         return same, empty
 
     def _make_token_plan(self, branch=(), guards=((), ()), pre_eps=0.0, ffn_eps=0.0, ffn_kind=0):
@@ -311,10 +316,13 @@ class SLinOSSMixer(nn.Module):
         out, sp = self.out_proj, self.scanprep
         if not (type(self.decode_backend) is B200MixerDecodeBackend and type(out) is nn.Linear and self.d_conv <= 4
                 and self.out_norm.weight is not None and not self.decode_backend.__dict__
+                and self.out_norm.eps is not None    # (else it follows the weight's type, which no guard sees)
                 and all(n in sp.__dict__ for n in _C.CONFIG_FIELDS)):
             return None
         same, empty = self._plan_guards(self.__dict__ if branch else None)
-        if any(len(d) for d in (*empty, *guards[1])):
+        same += [(self.__dict__, "step")] if branch else []
+        if any(len(d) for d in (*empty, *guards[1])) or \
+                any(len(g) == 2 and g[1] in (self.__dict__ if g[0] is None else g[0]) for g in (*same, *guards[0])):
             return None
         p, mine = sp._parameters, self._parameters
         params = [self.in_proj.weight, mine["dw_weight"], mine["dw_bias"], p["dt_bias"], p["alpha_bias"],
