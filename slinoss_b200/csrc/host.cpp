@@ -313,14 +313,18 @@ Tensor ffn_act_bwd(const Tensor& proj, const Tensor& dhid, int kind) {
 }
 
 // ---- decode: one token of a mixer ------------------------------------------------------------------------------------
-// y = W x: the small-batch kernel where it applies, else the library GEMM.
-bool small_batch(const Tensor& x, const Tensor& W) {
-  return x.size(0) <= 64 && x.size(1) % 8 == 0 && x.size(1) <= 4096 && x.scalar_type() != at::kFloat && W.is_contiguous() &&
-         x.stride(1) == 1 && x.stride(0) % 8 == 0;
+// y = W x: the small-batch kernel where it applies, else the library GEMM, which also says what is wrong with operands that
+// do not fit together.
+bool small_batch(at::ScalarType type, int64_t rows, int64_t K, const Tensor& W, const OptT& bias) {
+  return rows <= 64 && K % 8 == 0 && K <= 4096 && type != at::kFloat && W.scalar_type() == type && W.dim() == 2 && W.size(1) == K &&
+         W.is_contiguous() && (!bias || (bias->scalar_type() == type && bias->is_contiguous() && bias->numel() == W.size(0)));
+}
+bool small_batch(const Tensor& x, const Tensor& W, const OptT& bias) {
+  return small_batch(x.scalar_type(), x.size(0), x.size(1), W, bias) && x.stride(1) == 1 && x.stride(0) % 8 == 0;
 }
 Tensor linear_rows(const Call& call, const Tensor& x, const Tensor& W, const OptT& bias, const OptT& out_in) {
   const int64_t M = x.size(0), K = x.size(1), O = W.size(0);
-  if (small_batch(x, W)) {
+  if (small_batch(x, W, bias)) {
     Tensor out = out_in ? *out_in : call.empty({M, O}, x.scalar_type());
     const sl::SkinnyArgs a{ptr(x), x.stride(0), nullptr, 0.f, nullptr, 0, ptr(W), ptr(bias), mptr(out), (int)M, (int)K, (int)O,
                            code_of(x.scalar_type())};
@@ -346,7 +350,10 @@ std::tuple<Tensor, Tensor, Tensor> mixer_token(const Tensor& x, const Tensor& in
   for (const auto& t : biases) call.need(t);
   const int64_t batch = x.size(0), C = (int64_t)heads * P, O = in_w.size(0);
   const int io = code_of(x.scalar_type());
-  const bool chained = small_batch(x, in_w);   // the step may start behind our own in_proj kernel
+  if (O != 2 * C + 3 * heads + 4 * (int64_t)groups * N) throw pybind11::value_error("in_proj does not fit the mixer's sizes.");
+  for (const Tensor& t : {conv, b_prev, u_prev})
+    if (t.scalar_type() != x.scalar_type()) throw pybind11::value_error("the decode state does not have the token's type.");
+  const bool chained = small_batch(x, in_w, {});   // the step may start behind our own in_proj kernel
   const Tensor proj = linear_rows(call, x, in_w, {}, {});
   const size_t ws_bytes = sl_mixer_decode_step_workspace_bytes(batch, heads, P);
   Tensor ws = workspace && (size_t)workspace->numel() >= ws_bytes ? *workspace : call.bytes(ws_bytes);
@@ -362,7 +369,7 @@ std::tuple<Tensor, Tensor, Tensor> mixer_token(const Tensor& x, const Tensor& in
   const auto st = static_cast<cudaStream_t>(call.stream());
   check(sl::mixer_step_launch(a, st), "mixer_step");
   const int64_t K = C, OO = out_w.size(0);
-  if (batch <= 64 && K % 8 == 0 && K <= 4096 && io != SL_F32 && out_w.is_contiguous()) {   // the row norm inside the projection
+  if (small_batch(x.scalar_type(), batch, K, out_w, out_b)) {   // the row norm inside the projection
     Tensor y = out ? *out : call.empty({batch, OO}, x.scalar_type());
     const sl::SkinnyArgs s{mptr(ws), C, ptr(norm_w), norm_eps, sl::step_partials(mptr(ws), batch, heads, P), 8 * heads, ptr(out_w),
                            ptr(out_b), mptr(y), (int)batch, (int)K, (int)OO, io, true};

@@ -156,3 +156,19 @@ def test_a_stack_token_through_plans_equals_the_composed_token(batch, d_model, d
     assert all("_token_plan" not in b.mixer.__dict__ for b in stack.blocks)
     for a, b, c in zip(got, want, plain):
         assert a.shape == b.shape and torch.equal(a, b) and torch.equal(a, c)
+
+
+# the projections of the engine's token: either weight of another type than the token, at batches of the small-batch kernel and
+# of the library
+@pytest.mark.parametrize("batch", [2, 64, 80])
+@pytest.mark.parametrize("weights, token", [(torch.bfloat16, torch.float16), (torch.float16, torch.bfloat16),
+                                            (torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32)])
+def test_the_engine_refuses_weights_of_another_type(batch, weights, token):
+    from slinoss_b200.engine import MixerDecodeEngine
+    mixer = sb.SLinOSSMixer(128, d_state=64, d_head=64, device=DEV, dtype=weights)
+    with pytest.raises(RuntimeError, match="dtype"):
+        MixerDecodeEngine(mixer, batch, dtype=token)
+    mixer.in_proj.to(token)
+    with pytest.raises(RuntimeError, match="dtype"):
+        MixerDecodeEngine(mixer, batch, dtype=token)
+    assert MixerDecodeEngine(mixer.to(token), batch, dtype=token).step(torch.zeros(batch, 128, device=DEV, dtype=token)).isfinite().all()
