@@ -800,21 +800,25 @@ Tensor ffn_train(const Tensor& x, const Tensor& norm_w, const Tensor& w1, const 
 }
 
 // ---- language-model training step --------------------------------------------------------------------------------------
-// per-row losses and log-sum-exps of logits (rows, V)
-std::tuple<Tensor, Tensor> ce_fwd(const Tensor& logits, const Tensor& target) {
+// loss, scale of the gradient and the log-sum-exps of the rows of logits (rows, V)
+std::tuple<Tensor, Tensor, Tensor> ce_fwd(const Tensor& logits, const Tensor& target, bool mean) {
   Call call(logits, target);
   const int64_t rows = logits.size(0), V = logits.size(1);
-  Tensor loss = call.empty({rows}, at::kFloat), lse = call.empty({rows}, at::kFloat);
+  const Tensor loss = call.empty({rows}, at::kFloat), lse = call.empty({rows}, at::kFloat);
+  const Tensor total = call.empty({}, at::kFloat), scale = call.empty({}, at::kFloat);
   check(sl::cross_entropy_fwd(ptr(logits), target.const_data_ptr<int64_t>(), mfptr(loss), mfptr(lse), rows, V,
                               code_of(logits.scalar_type()), static_cast<cudaStream_t>(call.stream())),
         "cross_entropy_fwd");
-  return {loss, lse};
+  check(sl::cross_entropy_finish(fptr(loss), target.const_data_ptr<int64_t>(), rows, mean, mfptr(total), mfptr(scale),
+                                 static_cast<cudaStream_t>(call.stream())),
+        "cross_entropy_fwd");
+  return {total, scale, lse};
 }
-Tensor ce_bwd(const Tensor& logits, const Tensor& target, const Tensor& lse, const Tensor& g, double scale) {
-  Call call(logits, target, lse, g);
+Tensor ce_bwd(const Tensor& logits, const Tensor& target, const Tensor& lse, const Tensor& g, const Tensor& scale) {
+  Call call(logits, target, lse, g, scale);
   const int64_t rows = logits.size(0), V = logits.size(1);
   Tensor d = at::empty_like(logits);
-  check(sl::cross_entropy_bwd(ptr(logits), target.const_data_ptr<int64_t>(), fptr(lse), fptr(g), (float)scale, mptr(d), rows, V,
+  check(sl::cross_entropy_bwd(ptr(logits), target.const_data_ptr<int64_t>(), fptr(lse), fptr(g), fptr(scale), mptr(d), rows, V,
                               code_of(logits.scalar_type()), static_cast<cudaStream_t>(call.stream())),
         "cross_entropy_bwd");
   return d;

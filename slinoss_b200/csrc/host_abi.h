@@ -103,7 +103,9 @@ SL_API int column_sum(const void* x, void* out, float* partial, long long rows, 
 // ---- language-model training step ------------------------------------------------------------------------------------
 SL_API int cross_entropy_fwd(const void* logits, const int64_t* target, float* loss, float* lse, int64_t rows, int V, int io,
                              cudaStream_t st);
-SL_API int cross_entropy_bwd(const void* logits, const int64_t* target, const float* lse, const float* g, float scale, void* d,
+SL_API int cross_entropy_finish(const float* loss, const int64_t* target, int64_t rows, bool mean, float* total, float* scale,
+                                cudaStream_t st);
+SL_API int cross_entropy_bwd(const void* logits, const int64_t* target, const float* lse, const float* g, const float* scale, void* d,
                              int64_t rows, int V, int io, cudaStream_t st);
 // ids sorted (stable) and the positions they came from -> dE (V, C)
 SL_API int embedding_bwd(const int* sorted, const int64_t* order, const void* d_out, void* dE, int n, int V, int C, int io,

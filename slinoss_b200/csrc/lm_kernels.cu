@@ -7,6 +7,8 @@
 namespace sl {
 namespace {
 
+constexpr int64_t CE_IGNORE = -100;   // the target that torch's cross-entropy leaves out by default
+
 template <bool PRECISE> __device__ __forceinline__ float exp_io(float x) { return PRECISE ? expf(x) : __expf(x); }
 
 // ---- cross-entropy -------------------------------------------------------------------------------------------------
@@ -50,22 +52,52 @@ __global__ void __launch_bounds__(512) ce_fwd_kernel(const T* __restrict__ logit
     const float l = mm + logf(tot);
     const int64_t t = target[row];
     lse[row] = l;
-    loss[row] = t >= 0 && t < V ? l - to_f32(x[t]) : NAN;
+    loss[row] = t >= 0 && t < V ? l - to_f32(x[t]) : t == CE_IGNORE ? 0.f : NAN;
   }
 }
 
-// d logits = (softmax - onehot) * g * scale, g a device scalar
+// total: the rows' losses summed in float64 times scale, the reciprocal of the number of rows that are not
+// ignored, or one
+__global__ void __launch_bounds__(1024) ce_finish_kernel(const float* __restrict__ loss, const int64_t* __restrict__ target,
+                                                         int64_t rows, bool mean, float* __restrict__ total,
+                                                         float* __restrict__ scale_out) {
+  __shared__ double s_sum[32];
+  __shared__ int s_n[32];
+  double sum = 0.0;
+  int n = 0;
+  for (int64_t i = threadIdx.x; i < rows; i += 1024) { sum += loss[i]; n += target[i] != CE_IGNORE; }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) { sum += __shfl_xor_sync(0xffffffffu, sum, o); n += __shfl_xor_sync(0xffffffffu, n, o); }
+  if ((threadIdx.x & 31) == 0) { s_sum[threadIdx.x >> 5] = sum; s_n[threadIdx.x >> 5] = n; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    sum = 0.0; n = 0;
+    for (int k = 0; k < 32; ++k) { sum += s_sum[k]; n += s_n[k]; }
+    const double scale = mean ? 1.0 / n : 1.0;
+    total[0] = (float)(sum * scale);    // (every row ignored: 0 / 0)
+    scale_out[0] = (float)scale;
+  }
+}
+
+// d logits = (softmax - onehot) * g * scale, both device scalars; zeros in ignored rows
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(512) ce_bwd_kernel(const T* __restrict__ logits, const int64_t* __restrict__ target,
-                                                     const float* __restrict__ lse, const float* __restrict__ g, float scale,
-                                                     T* __restrict__ d, int V) {
+                                                     const float* __restrict__ lse, const float* __restrict__ g,
+                                                     const float* __restrict__ scale, T* __restrict__ d, int V) {
   constexpr int W = VEC ? Vec16<T>::N : 1;
   constexpr bool PRECISE = sizeof(T) == 4;
   const size_t row = blockIdx.x;
   const T* x = logits + row * V;
   T* o = d + row * V;
-  const float l = lse[row], f = g[0] * scale;
-  const int t = (int)target[row];
+  const int64_t t = target[row];
+  if (t == CE_IGNORE) {
+    const float zero[W] = {};
+    for (int c = threadIdx.x; c < V / W; c += blockDim.x) {
+      if constexpr (VEC) store16<T>(o + (size_t)c * W, zero); else o[c] = from_f32<T>(0.f);
+    }
+    return;
+  }
+  const float l = lse[row], f = g[0] * scale[0];
 #pragma unroll 2
   for (int c = threadIdx.x; c < V / W; c += blockDim.x) {
     float v[W];
@@ -229,7 +261,13 @@ int cross_entropy_fwd(const void* logits, const int64_t* target, float* loss, fl
   note_launches(1);
   return launch_status();
 }
-int cross_entropy_bwd(const void* logits, const int64_t* target, const float* lse, const float* g, float scale, void* d,
+int cross_entropy_finish(const float* loss, const int64_t* target, int64_t rows, bool mean, float* total, float* scale,
+                         cudaStream_t st) {
+  ce_finish_kernel<<<1, 1024, 0, st>>>(loss, target, rows, mean, total, scale);
+  note_launches(1);
+  return launch_status();
+}
+int cross_entropy_bwd(const void* logits, const int64_t* target, const float* lse, const float* g, const float* scale, void* d,
                       int64_t rows, int V, int io, cudaStream_t st) {
   if (rows < 1 || V < 1) return SL_ERR_BAD_SHAPE;
   const int w = io == SL_F32 ? 4 : 8;

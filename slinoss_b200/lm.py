@@ -20,20 +20,19 @@ from .layers import SLinOSSMLPConfig
 
 
 class _CrossEntropyFn(torch.autograd.Function):
-    """Summed cross-entropy times ``scale`` on the row kernels: the logits are kept in their own type and read once
-    each way (the library route goes through four float32 tensors of their size)."""
+    """Cross-entropy on the row kernels: the logits are kept in their own type and read once each way (the library route
+    goes through four float32 tensors of their size)."""
 
     @staticmethod
-    def forward(ctx, logits, targets, scale):
-        rows, lse = _C.host().ce_fwd(logits, targets)
-        ctx.save_for_backward(logits, targets, lse)
-        ctx.scale = scale
-        return rows.sum() * scale
+    def forward(ctx, logits, targets, mean):
+        loss, scale, lse = _C.host().ce_fwd(logits, targets, mean)
+        ctx.save_for_backward(logits, targets, lse, scale)
+        return loss
 
     @staticmethod
     def backward(ctx, d_loss):
-        logits, targets, lse = ctx.saved_tensors
-        return _C.host().ce_bwd(logits, targets, lse, d_loss.to(torch.float32), ctx.scale), None, None
+        logits, targets, lse, scale = ctx.saved_tensors
+        return _C.host().ce_bwd(logits, targets, lse, d_loss.to(torch.float32), scale), None, None
 
 
 class _EmbeddingFn(torch.autograd.Function):
@@ -53,11 +52,12 @@ class _EmbeddingFn(torch.autograd.Function):
 
 @_C.opaque
 def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, *, reduction: str = "mean") -> torch.Tensor:
-    """``F.cross_entropy(logits.float(), targets)`` of ``logits (rows, vocab)``."""
-    if not logits.is_cuda or logits.dtype not in _C._DTYPE_CODE or logits.numel() == 0 or not logits.is_contiguous():
+    """``F.cross_entropy(logits.float(), targets)`` of ``logits (rows, vocab)``: targets of -100 are left out."""
+    if not logits.is_cuda or logits.dtype not in _C._DTYPE_CODE or logits.numel() == 0 or not logits.is_contiguous() \
+            or logits.ndim != 2 or targets.dtype != torch.int64 or targets.shape != logits.shape[:1] \
+            or reduction not in ("mean", "sum"):
         return F.cross_entropy(logits.float(), targets, reduction=reduction)
-    scale = 1.0 / logits.shape[0] if reduction == "mean" else 1.0
-    return _CrossEntropyFn.apply(logits, targets.contiguous(), scale)
+    return _CrossEntropyFn.apply(logits, targets.contiguous(), reduction == "mean")
 
 
 @_C.opaque

@@ -81,6 +81,27 @@ def test_cross_entropy_and_its_gradient_equal_torch(rows, vocab, dtype):
         assert rel(loss, want) <= 1e-5 and (rel(g, gw) <= t or (g - gw).abs().max() < 1e-6)
 
 
+@pytest.mark.parametrize("rows,vocab,ignored", [(1, 7, 1), (5, 256, 2), (1030, 33, 1029), (2, 4099, 0)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_cross_entropy_leaves_out_the_ignored_index(rows, vocab, ignored, dtype):
+    from slinoss_b200.lm import cross_entropy
+    torch.manual_seed(rows)
+    logits = (4 * torch.randn(rows, vocab, device=DEV)).to(dtype).requires_grad_()
+    targets = torch.randint(0, vocab, (rows,), device=DEV)
+    targets[torch.randperm(rows, device=DEV)[:ignored]] = -100
+    want_in = logits.detach().double().requires_grad_()
+    for reduction in ("mean", "sum", "none"):
+        loss, want = cross_entropy(logits, targets, reduction=reduction), F.cross_entropy(want_in, targets, reduction=reduction)
+        assert loss.shape == want.shape
+        if rows == ignored and reduction == "mean":
+            assert loss.isnan() and want.isnan()
+            continue
+        (g,), (gw,) = torch.autograd.grad(loss.sum(), logits), torch.autograd.grad(want.sum(), want_in)
+        t = 1e-5 if dtype == torch.float32 else 1e-2
+        assert rel(loss, want) <= 1e-5 and rel(g, gw) <= t
+        assert g[targets == -100].count_nonzero() == 0
+
+
 @pytest.mark.parametrize("n,vocab,width", [(1, 1, 8), (40, 7, 12), (300, 1000, 264), (513, 33, 2048)])
 def test_embedding_gradient_equals_torch(n, vocab, width):
     from slinoss_b200.lm import embed
