@@ -9,6 +9,8 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 
+#include <cmath>
+
 #include "../../include/slinoss_b200.h"
 #include "host_abi.h"
 
@@ -872,7 +874,8 @@ void adamw_step(const std::vector<Tensor>& ps, const std::vector<Tensor>& gs, co
   Call call(step, grad_scale);
   for (const auto& p : ps) call.need(p);
   const auto st = static_cast<cudaStream_t>(call.stream());
-  const sl::AdamWArgs a{(float)lr, (float)beta1, (float)beta2, (float)eps, (float)weight_decay, fptr(step), fptr(grad_scale)};
+  const sl::AdamWArgs a{(float)lr, (float)eps, (float)(1.0 - lr * weight_decay), (float)beta2, (float)(1.0 - beta1),
+                        (float)(1.0 - beta2), std::log(beta1), std::log(beta2), fptr(step), fptr(grad_scale)};
   for (int io : {SL_F32, SL_BF16, SL_F16}) {
     sl::MtList4 list{};
     unsigned chunks = 0;

@@ -114,7 +114,8 @@ SL_API int embedding_bwd(const int* sorted, const int64_t* order, const void* d_
 constexpr int MT_MAX = 72;
 struct MtList1 { const void* p[MT_MAX]; int64_t len[MT_MAX]; unsigned first[MT_MAX]; int n; };
 struct MtList4 { void *p[MT_MAX], *g[MT_MAX], *m[MT_MAX], *v[MT_MAX]; int64_t len[MT_MAX]; unsigned first[MT_MAX]; int n; };
-struct AdamWArgs { float lr, beta1, beta2, eps, weight_decay; const float *step, *grad_scale; };
+// what beta does not hold to float32 precision near one is formed in float64: 1 - beta, ln beta, 1 - lr * weight_decay
+struct AdamWArgs { float lr, eps, decay, beta2, one_minus_beta1, one_minus_beta2; double ln_beta1, ln_beta2; const float *step, *grad_scale; };
 SL_API unsigned mt_chunks(int64_t len);
 SL_API int multi_sumsq(const MtList1& list, unsigned chunks, float* partial, int io, cudaStream_t st);
 SL_API int norm_finish(const float* partial, int n, float clip, float* out, cudaStream_t st);

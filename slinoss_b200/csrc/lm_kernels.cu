@@ -209,13 +209,15 @@ __global__ void __launch_bounds__(256) adamw_kernel(MtList4 list, AdamWArgs a) {
   T* v = reinterpret_cast<T*>(list.v[ti]);
   const size_t base = (size_t)(blockIdx.x - list.first[ti]) * MT_CHUNK, end = min((size_t)list.len[ti], base + MT_CHUNK);
   const float step = a.step[0], gs = a.grad_scale ? a.grad_scale[0] : 1.f;
-  const float bc1 = 1.f - powf(a.beta1, step), bc2s = sqrtf(1.f - powf(a.beta2, step));
-  const float step_size = a.lr / bc1, decay = 1.f - a.lr * a.weight_decay;
+  // bias corrections 1 - beta^step = -(e^(step ln beta) - 1): the product in float64, so that they keep float32 precision
+  // for beta near one (1 - 0.999 in float32 is off by 5e-5)
+  const float bc1 = -expm1f((float)(step * a.ln_beta1)), bc2s = sqrtf(-expm1f((float)(step * a.ln_beta2)));
+  const float step_size = a.lr / bc1;
   auto update = [&](float& pv, float& gv, float& mv, float& vv) {
     gv = gs == 1.f ? gv : gv / gs;
-    pv *= decay;
-    mv += (1.f - a.beta1) * (gv - mv);
-    vv = a.beta2 * vv + (1.f - a.beta2) * gv * gv;
+    pv *= a.decay;
+    mv += a.one_minus_beta1 * (gv - mv);
+    vv = a.beta2 * vv + a.one_minus_beta2 * gv * gv;
     pv -= step_size * mv / (sqrtf(vv) / bc2s + a.eps);
   };
   const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(m) |

@@ -113,6 +113,25 @@ def test_embedding_gradient_equals_torch(n, vocab, width):
     assert rel(g, want) <= 5e-3
 
 
+@pytest.mark.parametrize("betas", [(0.9, 0.999), (0.9, 0.95), (0.0, 0.9999)])
+def test_adamw_keeps_float32_precision_for_betas_near_one(betas):
+    """From zero parameters a step is the update itself: a few float32 roundings (2^-24 each) from float64, in the states too."""
+    from slinoss_b200.optim import AdamW
+    torch.manual_seed(3)
+    p = torch.nn.Parameter(torch.zeros(4096, device=DEV))
+    q = torch.nn.Parameter(torch.zeros(4096, dtype=torch.float64))
+    kw = dict(lr=1e-3, betas=betas, eps=1e-8, weight_decay=0.05)
+    a, b = AdamW([p], **kw), torch.optim.AdamW([q], **kw)
+    for _ in range(4):
+        p.grad = torch.rand_like(p) + 0.5
+        q.grad = p.grad.double().cpu()
+        a.step()
+        b.step()
+        sa, sb = a.state[p], b.state[q]
+        for got, want in ((p, q), (sa["exp_avg"], sb["exp_avg"]), (sa["exp_avg_sq"], sb["exp_avg_sq"])):
+            assert float(((got.detach().double().cpu() - want.detach()) / want.detach()).abs().max()) <= 12 * 2.0 ** -24
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_adamw_equals_torch_also_after_loading_its_state_and_with_missing_gradients(dtype):
     from slinoss_b200.optim import AdamW
