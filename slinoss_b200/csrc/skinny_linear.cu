@@ -166,10 +166,13 @@ int launch_skinny(const SkinnyArgs& a, cudaStream_t st) {
 }
 template <typename T>
 int launch_skinny_m(const SkinnyArgs& a, cudaStream_t st) {
-  // One 16-row tile of x and one 8-row tile of W per warp give the most CTAs and the shortest chain.  A CTA then reads 48 K
-  // bytes, and with many rows of a large layer that traffic takes longer than the chain (width 1024: 348 against 358 us per token
-  // of four blocks at 32 rows, 588 against 523 at 64; width 512: 284 against 346 at 64).
-  if (a.M <= 16 || (long long)a.M * a.K * a.O <= 120000000) return launch_skinny<T, 1, 1>(a, st);
+  // One 16-row tile of x and one 8-row tile of W per warp give the most CTAs and the shortest chain; with 32 and 16 rows a CTA
+  // reads half as many bytes per product.  The line lies where the former no longer fit on the chip at once (64 registers per
+  // thread, 128 with the norm's fragments kept).  us, small against large tiles: in_proj 512 x 6192 at 48 rows 8.2 / 10.3 and
+  // at 64 12.2 / 10.3, 768 x 9288 at 17 rows 12.1 / 10.2, 1024 x 12384 at 64 29.9 / 24.5; out_proj 2048 x 1024 at 32 rows
+  // 10.7 / 12.3 and at 33 14.4 / 12.3, 1536 x 768 at 48 12.3 / 14.9 and at 64 19.4 / 15.0, 1024 x 512 at 64 10.3 / 14.3.
+  const int warps = (a.K + KRUN - 1) / KRUN, per_sm = (a.norm_weight && warps <= 8 ? 16 : 32) / warps;
+  if (a.M <= 16 || (long long)((a.O + 7) / 8) * ((a.M + 15) / 16) <= 148 * per_sm) return launch_skinny<T, 1, 1>(a, st);
   return launch_skinny<T, 2, 2>(a, st);
 }
 
