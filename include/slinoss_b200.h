@@ -58,7 +58,8 @@ enum {
   SL_PATH_SIMT = 1, /* exact float32 sequential recurrence (any dtype in)     */
   SL_PATH_TC = 2    /* tcgen05/TMEM chunked path: bf16 / fp16 operands, P = 64, N = 64 or 128 (other
                        sizes are refused here and take SIMT under auto); without the SL_WS_SCAN_FWD
-                       workspace of a problem the forward pass is refused          */
+                       workspace of a problem a forward pass with N = 64 walks every stream whole
+                       instead of in segments, one with N = 128 is refused              */
 };
 
 /* workspace kinds for sl_workspace_bytes */

@@ -409,8 +409,11 @@ int scan_tc_fwd(const void* U, const float* M, const float* K, const void* B, co
                 const float* z0, const void* Bprev, const void* Uprev, void* Y, float* zfinal,
                 void* states_out, const ScanDims& d, int io_dtype, int y_dtype, void* ws, size_t ws_bytes,
                 cudaStream_t st) {
-  const SegPlan plan = fwd_plan(d);
-  if (plan.nseg > 1 && (!ws || ws_bytes < seg_layout(d, plan.nseg).total)) return SL_ERR_WORKSPACE_TOO_SMALL;
+  SegPlan plan = fwd_plan(d);
+  if (!ws || ws_bytes < scan_tc_fwd_workspace(d)) {   // N = 64 has always run without: the streams are then walked whole
+    if (blocks_of(d) == 2) return SL_ERR_WORKSPACE_TOO_SMALL;
+    plan = {1, chunks_of(d)};
+  }
   return scan_tc_fwd_impl(U, M, K, B, C, z0, Bprev, Uprev, Y, zfinal, states_out, d, plan,
                           reinterpret_cast<uint8_t*>(ws), io_dtype, y_dtype, st);
 }

@@ -41,3 +41,18 @@ def test_split_and_padded_scan_matches_the_oracle(shape, dtype):
     want = scan_np.v2x2ssd_bwd(*args, n64(case.dY), d_final_state=None if d_final is None else n64(d_final), **kw)
     for name, grad in zip(leaves, grads):
         assert rel(grad, want[name]) <= 2e-2, (name, rel(grad, want[name]))
+
+
+@pytest.mark.parametrize("N", [64, 128])
+def test_forward_without_its_workspace_walks_whole_or_is_refused(N):
+    c = make_scan_case(1, 2, 1300, 64, N, dtype=torch.bfloat16, seed=N).to("cuda")
+    assert _C.workspace_bytes(_C.WS_SCAN_FWD, 1, 2, 2, 1300, 64, N, 64, torch.bfloat16) > 0
+    want, _ = _C.scan_fwd(c.U, c.M, c.K, c.B, c.C, None, None, None, chunk_size=64, y_dtype=torch.float32, want_final=False)
+    Y = torch.full_like(want, float("nan"))
+    status = _C.lib().sl_v2x2ssd_fwd(*[t.data_ptr() for t in (c.U, c.M, c.K, c.B, c.C)], None, None, None, Y.data_ptr(), None, None,
+                                     1, 2, 2, 1300, 64, N, 64, _C.SL_BF16, _C.SL_F32, _C.PATH_AUTO, None, 0,
+                                     torch.cuda.current_stream().cuda_stream)
+    if N == 128:
+        assert _C.lib().sl_status_string(status).decode() == "workspace missing or too small"
+    else:
+        assert status == 0 and rel(Y, want) <= 2e-2 and _C.device_status() == 0
