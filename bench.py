@@ -1,4 +1,4 @@
-"""Benchmark of the v2x2ssd scan forward+backward (BASELINE config 1) on B200.
+"""Benchmark of the v2x2ssd scan forward+backward on B200.
 
     python bench.py --gpus N --steps K --warmup W [--impl reference]
 
@@ -491,7 +491,7 @@ def main():
                     "note": "copy_only = the same host<->device bytes over the same streams without the op: "
                             "the host-link bound of this step on this box"},
             "gpu_launches": launches_timed,
-            "roofline": {"bound": "hbm", "kernel": "backward sweep (scan_tc_bwd_kernel + its scalar finish)",
+            "roofline": {"bound": "hbm", "kernel": "backward sweep (scan_tc_bwd_kernel + scan_tc_bwd_post_kernel)",
                          "achieved": bwd_gbs, "peak": peak, "unit": "GB/s", "frac": bwd_gbs / peak,
                          "traffic": traffic, "traffic_source": traffic_source,
                          "peak_source": peak_kind, "algorithmic_bytes": ab["bwd"], "ms": bwd_ms,

@@ -285,9 +285,8 @@ SL_API int sl_mixer_tail_bwd(const void* Y, const void* gate, int64_t gate_row_s
                       int heads, int T, int P, int io_dtype, void* stream);
 
 /*
- * One decode token of the whole mixer between in_proj and out_proj, in one launch: causal conv
- * update + bias + SiLU, scan preparation of the token, state update and read-out, skip, gate and
- * RMSNorm.  Replaces the per-token path of SLinOSSMixer.step: run_reference_decode_step
+ * One decode token of the whole mixer between in_proj and out_proj: causal conv update + bias + SiLU,
+ * scan preparation of the token, state update and read-out, skip and gate in one launch, and RMSNorm.  Replaces the per-token path of SLinOSSMixer.step: run_reference_decode_step
  * (slinoss/ops/mixer/step.py:201-258, 323-429; a chain of torch ops) and mixer_decode_step_cute
  * (slinoss/ops/v2x2ssd/cute/step.py:224-627; fused, but unreachable for mixers with d_skip).
  *   gate, value (batch, heads*P) : io_dtype, row strides in elements (column slices of the in_proj

@@ -321,15 +321,15 @@ def mixer_tail_bwd(Y, gate, skip, d_skip, norm_weight, eps, d_normed):
 # fused decode step of the mixer
 # ---------------------------------------------------------------------------------
 def mixer_decode_workspace(batch, heads, P, dev) -> torch.Tensor:
-    """The zero-initialised scratch ``mixer_decode_step`` needs (allocate once, reuse every token)."""
+    """Scratch for ``mixer_decode_step`` (allocate once, reuse every token; its content does not matter)."""
     n = lib().sl_mixer_decode_step_workspace_bytes(batch, heads, P)
-    return torch.zeros(n, dtype=torch.uint8, device=dev)
+    return torch.empty(n, dtype=torch.uint8, device=dev)
 
 
 def mixer_decode_step(gate, value, params, bc, conv_weight, conv_bias, conv_state, biases, cfg, d_skip,
                       norm_weight, eps, state, b_prev_in, b_prev_out, u_prev, workspace, *, heads, P,
                       normed=None):
-    """Launch ``sl_mixer_decode_step``.  ``gate`` and ``value`` are (batch, heads*P) views with a row
+    """Call ``sl_mixer_decode_step`` (the step and its row norm: two launches).  ``gate`` and ``value`` are (batch, heads*P) views with a row
     stride; ``conv_state``, ``state`` and ``u_prev`` are updated in place; ``b_prev_out`` receives this
     token's b.  Returns ``normed`` (batch, heads*P)."""
     dev = require_cuda(gate, value, params, bc, conv_weight, conv_bias, conv_state, d_skip, norm_weight, state,

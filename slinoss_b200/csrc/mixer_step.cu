@@ -1,4 +1,4 @@
-// One decode token of the whole mixer between in_proj and out_proj, in ONE launch:
+// One decode token of the whole mixer between in_proj and out_proj, in one launch up to the row norm:
 //
 //   causal conv update + bias + SiLU  ->  u          (per channel, carried conv window)
 //   scan preparation of the token     ->  m, kp, kc  (per head)   and  b, c  (per group)
@@ -8,7 +8,7 @@
 //
 // (what run_reference_decode_step evaluates with separate torch ops, slinoss/ops/mixer/step.py:201-258 and
 // 323-429, and what mixer_decode_step_cute fuses for d_skip-free mixers only,
-// slinoss/ops/v2x2ssd/cute/step.py:224-627; out_proj stays a library GEMM in the caller.)
+// slinoss/ops/v2x2ssd/cute/step.py:224-627; the projections are the caller's.)
 //
 // The RMSNorm needs the sum of squares over ALL heads of a batch row: the step kernels leave the gated values of the
 // row and eight partial sums of squares per head (plain stores, no atomics, so a token is bit-reproducible); whoever

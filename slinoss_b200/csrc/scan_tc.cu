@@ -23,8 +23,8 @@
 // applied to the 16-bit operands, decays to float32 accumulators.
 //
 // A stream is walked chunk by chunk by one CTA; streams that do not fill the chip are split into segments of
-// chunks: a cheap pre-pass over the segments (states only) and a combine kernel give every segment its start
-// state, and the segments then run side by side.  scan_tc_fwd.cuh and scan_tc_bwd.cuh describe the kernels and
+// chunks: a cheap pre-pass over the segments (states only) and a fold (in the sweeps, or a combine kernel for many
+// segments) give every segment its start state, and the segments then run side by side.  scan_tc_fwd.cuh and scan_tc_bwd.cuh describe the kernels and
 // the thread-to-data mappings; plan_segments() below holds the rule for the split.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -421,8 +421,8 @@ int scan_tc_fwd(const void* U, const float* M, const float* K, const void* B, co
 namespace {
 
 // Tensor-core backward: state pre-sweep (unless the forward saved its chunk states), adjoint pre-pass when the
-// sweep is split in time, reverse sweep, the boundary terms of carried B_prev / U_prev, scalar finish, the sum of
-// the column blocks' dU (N > 64) and, for grouped B/C, the reduction of dB / dC over the heads of a group.
+// sweep is split in time, reverse sweep, the boundary terms of carried B_prev / U_prev, and one launch for dM / dK from
+// the scalars, the sum of the column blocks' dU (N = 128) and, for grouped B/C, that of dB / dC over the heads of a group.
 template <typename TIn>
 int run_bwd(const void* U, const float* M, const float* K, const void* B, const void* C, const float* z0,
             const void* Bprev, const void* Uprev, const void* states_in, const float* zfinal_in, const void* dY,

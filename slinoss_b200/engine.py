@@ -1,9 +1,10 @@
 """CUDA-graph decode engine for ``SLinOSSMixer``: one captured graph per token.
 
-A decode token of the mixer is in_proj (library GEMM) -> ``sl_mixer_decode_step`` (one launch: conv
-update, scan preparation, state update, skip, gate, RMSNorm) -> out_proj (library GEMM).  Launching
-these three from Python costs more host time than the GPU needs at small batch; the engine captures
-them once over static buffers and replays the graph per token.  The reference has the same idea for
+A decode token of the mixer is in_proj, the step kernel (conv update, scan preparation, state update, skip,
+gate, partial sums for the row norm) and out_proj.  Up to 64 rows of a 16-bit type the projections are the
+small-batch kernels, the second with the row norm inside: three launches; else they are library GEMMs with
+a kernel for the norm in between.  Their launches cost more host time than the GPU needs at small batch; the engine
+captures them once over static buffers and replays the graph per token.  The reference has the same idea for
 its whole model (scripts/perf/_training_model.py:120-200); here it is part of the package because
 the fused step exists to be replayed.
 """

@@ -124,9 +124,9 @@ class B200MixerDecodeBackend:
     """Per-token decode on CUDA kernels (d_skip is supported, unlike the reference's fast path,
     slinoss/ops/mixer/step.py:107-122).
 
-    ``fused_step`` is the one-launch path ``SLinOSSMixer.step`` takes outside autograd: conv update,
-    scan preparation of the token, state update, skip, gate and RMSNorm in ``sl_mixer_decode_step``,
-    with the mixer state updated in place.  ``__call__`` is the Protocol entry
+    ``fused_step`` is the step between library projections: conv update, scan preparation of the token, state
+    update, skip and gate as one launch and the row norm as another (``sl_mixer_decode_step``), with the mixer state
+    updated in place.  ``__call__`` is the Protocol entry
     (slinoss/layers/backend.py:220-237): it takes the already convolved value and runs scan
     preparation, the decode kernel and the gated RMSNorm as separate launches."""
 

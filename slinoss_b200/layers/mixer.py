@@ -273,7 +273,7 @@ class SLinOSSMixer(nn.Module):
         return (y[:, 0, :], nxt) if squeeze else (y, nxt)
 
     def _fused_decode_ready(self, state: SLinOSSMixerState, token: torch.Tensor) -> bool:
-        """The one-launch decode step needs a complete in-place state in the kernel's layouts."""
+        """The fused decode step needs a complete in-place state in the kernel's layouts."""
         sc = state.scan
         return (getattr(self.decode_backend, "fused", False)
                 and self.decode_backend.supports(self, batch_size=int(token.shape[0]), device=token.device,

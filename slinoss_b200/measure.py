@@ -273,7 +273,7 @@ def measure_mixer(iters, dev, batch=8):
 
 def measure_mixer_step(iters, dev, batch=256, N=64):
     """One decode token of the whole mixer (d_model 1024, 32 heads x 64, N 64, conv width 4, bf16) at
-    the decode configuration's batch: in_proj, the one-launch fused step, out_proj.  Eager through
+    the decode configuration's batch: in_proj, the fused step, out_proj.  Eager through
     ``SLinOSSMixer.step`` and replayed from the CUDA-graph engine; the traffic that bounds it is the
     float32 state read and written once (2 x 268 MB at batch 256)."""
     import slinoss_b200 as sb
@@ -367,8 +367,8 @@ def measure_ffn_rows(iters, dev, rows=16384, C=2048, hidden=8192):
 
 
 def measure_scan_n128(iters, dev):
-    """The config-1 streams with 128 state columns (the mixer's default d_state): two passes over the
-    column blocks of B and C."""
+    """The config-1 streams with 128 state columns (the mixer's default d_state): two blocks of 64
+    columns, in one CTA forwards and as a grid dimension backwards."""
     from . import _C
     from .synthetic import make_scan_case
     c = make_scan_case(8, 16, 4096, 64, 128, dtype=torch.bfloat16, seed=0).to(dev)

@@ -228,7 +228,7 @@ TC_SHAPES = [
 ]
 
 
-@pytest.mark.parametrize("N", [64, 128])           # 128: two passes over the column blocks of B and C
+@pytest.mark.parametrize("N", [64, 128])           # 128: two column blocks of B and C
 @pytest.mark.parametrize("shape", TC_SHAPES)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_forward_tensor_core_path(shape, dtype, N):
