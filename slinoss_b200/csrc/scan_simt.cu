@@ -1,51 +1,78 @@
-// Exact float32 sequential v2x2ssd scan (forward and backward), SIMT.
+// Float32 v2x2ssd scan (forward and backward).
 //
-// This is the path taken for float32 inputs (parity to 1e-5 needs float32
-// products, which the tensor cores do not offer) and for shapes the tensor-core
-// path does not cover.  It evaluates the recurrence token by token exactly as the
-// sequential oracle does (reference: slinoss/ops/v2x2ssd/reference.py:815-840):
+// This is the path taken for float32 inputs (parity to 1e-5 needs float32 products, which one tensor-core product is not)
+// and for shapes the tensor-core path does not cover.  It evaluates the recurrence (reference:
+// slinoss/ops/v2x2ssd/reference.py:815-840)
 //
-//   z_t = m_t z_{t-1} + u_{t-1} (x) (kp_t b_{t-1}) + u_t (x) (kc_t b_t)
-//   y_t[p] = Re sum_n conj(c_t[n]) z_t[p,n]
+//   z_t = m_t z_{t-1} + u_{t-1} (x) (kp_t b_{t-1}) + u_t (x) (kc_t b_t),    y_t[p] = Re sum_n conj(c_t[n]) z_t[p,n]
 //
-// One CTA owns one (batch, head, 64-row slice of P, segment of T).  A warp owns 32 rows of P and 4 NC complex columns of
-// the state, a lane 4 rows of NC columns, kept in registers as packed pairs of columns for the whole segment.  With
-// 8 x 4 lanes on the tile both sums (over columns for y, over rows for the gradients of b and c) are mostly inside a lane:
-// 3 + 4 shuffles per token and warp, where a lane per row with all the columns needed 31 for every sum over rows.  Tokens
-// are staged TB at a time in shared memory, already multiplied by their taps.
+// as V_t = z_t - u_t (x) (kc_t b_t), the state before the token's own injection, which has ONE injection per token and
+// needs no division, so that an exactly zero transition is computed through:
 //
-// Backward = two more sweeps of the same shape (in one launch: they do not depend on one another) plus two small
-// finishing kernels:
-//   sweep A (forward in time)  recomputes z_t and emits dc_t[n] = sum_p dy_t[p] z_t[p,n]
-//   sweep B (backward in time) carries G_t = dy_t (x) c_t + conj(m_{t+1}) G_{t+1} and
-//           emits dbc_t = sum_p u_t G_t, dbp_t = sum_p u_{t-1} G_t, dU, d_initial
-//   finish  dK, dB, dC (group sums), and dM from the identity
-//           conj(m_t) dm_t = S_t,  S_t = S_{t+1} + <c_t,dc_t> - conj(kp_t)dkp_t - conj(kc_t)dkc_t,
-//           S_T = <d_final, z_final>   (no state history is needed for dM).
+//   V_{t+1} = m_{t+1} V_t + u_t (x) (h_t b_t),   h_t = m_{t+1} kc_t + kp_{t+1}   (m_T = 1, kp_T = 0: V_T is the final state)
+//   y_t     = Re <c_t, V_t> + u_t Re(conj(c_t) kc_t b_t)
+//
+// in chunks of L = 16 tokens.  With P(j, i) = m_{i+2} .. m_j (products of at most 16 float32 transitions) and V the state at
+// the chunk's first token:
+//
+//   y_j  = Re sum conj(c_j) a_j V + sum_{i<j} Re(P(j,i) h_i d(j,i)) u_i + Re(kc_j d(j,j)) u_j,  a_j = P(j,-1), d(j,i) = <c_j, b_i>
+//   V'   = a_L V + sum_i u_i (x) (P(L,i) h_i b_i)
+//
+// Two multiply-adds per (row, real column) and token for each of the two instead of eight and six for a walk token by token.
+// The adjoint (lambda_t of V_t) walks the chunks the other way with the same products; X(j,i) = <dy_j, u_i>:
+//
+//   A, forward in time: dC_j = a_j sum_p dy_j V + sum_{i<j} X(j,i) P(j,i) h_i b_i + X(j,j) kc_j b_j
+//   B, backward:        D_i = conj(P(L,i)) sum_p u_i lambda + sum_{j>i} X(j,i) conj(P(j,i)) c_j,
+//                       dB_i = conj(h_i) D_i + X(i,i) conj(kc_i) c_i,  dh_i = <b_i, D_i>  (-> dK),
+//                       dU_i = Re sum conj(P(L,i) h_i b_i) lambda + sum_{j>=i} S(j,i) dy_j,   S: the factors of u_i in y_j
+//   dM from S_t = S_{t+1} + <c_t, dC_t without its last term> - conj(h_t) dh_t,  conj(m_t) dm_t = S_t - conj(kp_t) dkp_t,
+//   S_T = <d_final, z_final>, in float64 by the finishing kernel (no state history is kept).
+//
+// The products run on the tensor cores as products of bfloat16 parts (mma.sync m16n8k16): a float32 is the sum of three, a
+// 16-bit operand of one or two, and the products of parts down to 2^-24 are kept (see products()), at 8 times the FMA rate.
+// One CTA owns one (batch, head, 64 rows of P, segment of T); a warp owns 16 complex columns x 64 rows of the state, in
+// registers as accumulators, which serve as the operand of the next chunk's products as they are (sums over the rows of P) or
+// through an 8 x 8 transposition in registers (over the columns).  The operands that belong to a warp's columns are made by
+// the warp itself from the raw rows, which arrive by cp.async one chunk ahead in their own type; only the sums over all
+// columns (Y, dU, d(j,i)) and the per-token scalars cross warps.  The chain of transition products is one warp's, one chunk
+// ahead.
+//
+// What bounds it now: issue and latency at 12 warps per SM (168 registers hold the state, its parts and the operands); 41 % of
+// the issue slots and 33 % of the tensor pipe are busy in the forward sweep.  Forward + backward, us, against sweeps token by
+// token on the FMA pipe: (16, 4, 2048, N 48 fp16) 2973 -> 663, (2, 4, 256, N 32 fp32) 61 -> 51.
+// Distance from float64 against those sweeps (2-norm, float32 operands, T 256 to 8192): Y 1.27e-7 -> 1.13e-7, dC 1.28e-7 ->
+// 1.17e-7, dU 1.13e-7 and dK 1.30e-7 both, dB 1.10e-7 -> 1.12e-7, d_initial 9.2e-8 -> 7.5e-8, dM a third nearer.
 //
 // The walk over T is serial, so a problem with few (batch, head) streams is split in time: a first launch runs every
-// segment but the last from a zero state and keeps only where it ends and the product of its transitions; each CTA of the
-// sweeps then folds the segments before its own into its start state (all in float32, the products in float64).  B the same,
-// from the other end.  (2, 4, 256, P 64, N 32) forward + backward: 629 -> 74 us with 16 segments.
+// segment but the last from a zero state and keeps only where it ends and the product of its transitions (in float64), a second
+// one combines them to the segments' start states.  The adjoint's the same, from the other end.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
 namespace sl {
 namespace {
 
+constexpr int L = 16;          // tokens of a chunk
+constexpr int ROWS = 64;       // rows of P of a CTA
+constexpr int TABW = 18;       // row pitch (complex) of the table of products
+
 struct SweepParams {
   const void *U, *B, *C, *Bprev, *Uprev, *dY;
   const float *M, *K, *z0, *dfinal;
   void* Y;
   float* zfinal;
-  float *dc_head, *dbc_head, *dbp_head;  // (batch, heads, T, 2N) float32
-  float* sT;                             // (batch, heads, 2)  <d_final, z_final>
-  void *dU, *dUprev;
+  float *dB_head, *dC_head, *dBprev_head;   // (batch, heads, T, 2N) float32 where heads or rows of P are still to be summed
+  float* sterm;                             // (batch, heads, T, 2)  <c_t, dC_t without the diagonal>
+  float* sT;                                // (batch, heads, 2)     <d_final, z_final>
+  float *dK, *dM;
+  void *dU, *dB, *dC, *dUprev, *dBprev;
   float* dinit;
-  float *zloc, *zprod, *gloc, *gprod;    // per segment: (batch, heads, P, 2N) end of the walk from zero, (batch, heads, 2)
+  float *zloc, *zprod, *gloc, *gprod;       // per segment: (batch, heads, P, 2N) end of the walk from zero, (batch, heads, 2)
   int batch, heads, groups, T, P, N;
-  int NS, PW, TB, ptiles, nseg, seg_len;
+  int W, ptiles, nseg, seg_len;             // W: warps, 16 complex columns each
+  int spread;                               // dB, dC, dB_prev go to the float32 buffers
 };
 
 // Sum over the lanes whose index differs in the bits HI .. LO (powers of two), scattering the values: a lane ends with LEN
@@ -54,121 +81,281 @@ template <int LEN, int HI, int LO>
 struct Scatter {
   static __device__ __forceinline__ void run(float* v, int lane) {
     if constexpr (HI >= LO) {
-      if constexpr (LEN > 1) {
-        constexpr int H = LEN / 2;
-        const bool up = (lane & HI) != 0;
+      constexpr int H = LEN / 2;
+      const bool up = (lane & HI) != 0;
 #pragma unroll
-        for (int i = 0; i < H; ++i) {
-          const float send = up ? v[i] : v[i + H], keep = up ? v[i + H] : v[i];
-          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, HI);
-        }
-        Scatter<H, HI / 2, LO>::run(v, lane);
-      } else {
-        v[0] += __shfl_xor_sync(0xffffffffu, v[0], HI);
-        Scatter<1, HI / 2, LO>::run(v, lane);
+      for (int i = 0; i < H; ++i) {
+        const float send = up ? v[i] : v[i + H], keep = up ? v[i + H] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, HI);
       }
+      Scatter<H, HI / 2, LO>::run(v, lane);
     }
   }
 };
 
+// row pitch in bytes of an array of rows in shared memory: an odd number of 16-byte pieces (no bank conflicts across rows)
+__host__ __device__ constexpr int row_pitch(int bytes) { return ((bytes + 15) / 16 | 1) * 16; }
+
+// ---- float32 as sums of bfloat16 ---------------------------------------------------------------------------------------
+// Parts that hold a type exactly (float32: 24 bits in three parts of 8).
+template <typename T> struct Parts { static constexpr int N = 3; };
+template <> struct Parts<__nv_bfloat16> { static constexpr int N = 1; };
+template <> struct Parts<__half> { static constexpr int N = 2; };
+// w[k] = part k of the pair v
+template <int NP>
+__device__ __forceinline__ void split(f2 v, uint32_t (&w)[NP]) {
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    const float2 x = un2(v);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x.x, x.y);
+    w[k] = *reinterpret_cast<const uint32_t*>(&h);
+    if (k + 1 < NP) v = fma2(mk2(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u)), dup2(-1.f), v);
+  }
+}
+template <bool FIRST>
+__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  if constexpr (FIRST)
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%10,%10,%10,%10};"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+  else asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// d = A B over 16 terms, smallest products first (those of parts whose weights together are below 2^-24 are left out).  The
+// tensor cores cut the bits of a sum off instead of rounding them: that is harmless for the small products, and the large
+// ones are added up here over 16 terms at most; longer sums go through rounded float32 additions.  Measured against float64
+// over normal operands: 4.8e-8 relative for 16 terms and 6.3e-8 for 64, where a chain of fmaf has 7.4e-8 and 1.5e-7.
+// NT independent tiles at a time, a product of each in turn: a tensor-core operation waits for the one before it on its sum.
+template <int NT, int NA, int NB, typename FA, typename FB>
+__device__ __forceinline__ void products(float (&d)[NT][4], FA a, FB b) {
+  constexpr int SUM = NA + NB - 2 < 2 ? NA + NB - 2 : 2, FIRST = SUM - (NB - 1) > 0 ? SUM - (NB - 1) : 0;
+#pragma unroll
+  for (int sum = SUM; sum >= 0; --sum)
+#pragma unroll
+    for (int i = 0; i < NA; ++i)
+      if (sum - i >= 0 && sum - i < NB)
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          if (sum == SUM && i == FIRST) mma<true>(d[t], a(t)[i], b(t)[sum - i][0], b(t)[sum - i][1]);
+          else mma<false>(d[t], a(t)[i], b(t)[sum - i][0], b(t)[sum - i][1]);
+        }
+}
+__device__ __forceinline__ uint32_t transposed(uint32_t w) {   // an 8 x 8 tile of pairs across the warp
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(w));
+  return r;
+}
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const uint8_t* row) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(row);
+  if constexpr (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+
+constexpr int TABF = 17 * TABW * 2 + 10 * L;                         // floats of one table
+constexpr int V_H = 17 * TABW * 2, V_KAPPA = V_H + 2 * L, V_KC = V_H + 4 * L, V_MNEXT = V_H + 6 * L, V_HLOW = V_H + 8 * L;
+
+enum Mode { FORWARD, SWEEP_A, STATES, SWEEP_B, ADJ_STATES };
+
+// Shared memory of a CTA.  Raw rows are in the tensors' types, two chunks of each but of rows that are converted first.
+struct Layout {
+  int pD, pU, pY, pP;                       // row pitches in bytes
+  int b, c, u, y, raw_end, up, yp, tab, part, dpart, red, sig, dd, bytes;
+  __host__ __device__ constexpr Layout(int W, int esz, int ysz, int nu, int ny, Mode mode)
+      : pD(row_pitch(32 * W * esz)), pU(row_pitch(ROWS * esz)), pY(row_pitch(ROWS * ysz)), pP(row_pitch(ROWS * 2)), b(0), c(0),
+        u(0), y(0), raw_end(0), up(0), yp(0), tab(0), part(0), dpart(0), red(0), sig(0), dd(0), bytes(0) {
+    const bool back = mode == SWEEP_A || mode == SWEEP_B, dy = back || mode == ADJ_STATES, cross = mode == FORWARD || mode == SWEEP_B;
+    int o = 0;
+    b = o; o += mode != ADJ_STATES ? 2 * L * pD : 0;
+    c = o; o += mode != STATES ? 2 * L * pD : 0;
+    u = o; o += mode != ADJ_STATES ? (nu > 1 ? 1 : 2) * L * pU : 0;
+    y = o; o += dy ? (ny > 1 ? 1 : 2) * L * pY : 0;
+    raw_end = o;
+    up = o; o += mode != ADJ_STATES && nu > 1 ? nu * L * pP : 0;   // rows of U and dY as bfloat16 parts
+    yp = o; o += dy && ny > 1 ? ny * L * pP : 0;
+    tab = o; o += 2 * TABF * 4;                                    // P(j, i); h, P(L,i) h, kc, m behind the token, rest of h
+    part = o; o += cross ? W * 8 * 32 * 16 : 0;                    // sums over a warp's columns, by fragment
+    dpart = o; o += cross ? W * 4 * 32 * 16 : 0;                   // <c_j, b_i> over a warp's columns, by fragment
+    red = o; o += back ? 2 * W * L * 8 : 0;                        // a warp's part of the per-token scalars, of two chunks
+    sig = o; o += back ? W * L * 4 : 0;                            // X(i,i), a copy for each warp
+    dd = o; o += mode == SWEEP_B ? 2 * L * 16 : 0;                 // X(i,i) conj(d(i,i)) and m behind the token, of two chunks
+    bytes = o;
+  }
+};
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Rows [0, nb) of cols elements, pitch elements apart in memory, into shared memory.  16-byte pieces where every row starts
+// on such a boundary and is a whole number of them, element by element where not.
 template <typename T>
-__device__ __forceinline__ cf load_c(const T* base, size_t cidx) {
+__device__ __forceinline__ void stage_rows(uint8_t* dst, int dst_pitch, const T* src, int nb, int cols, int pitch) {
+  const int bytes = cols * (int)sizeof(T);
+  if (((reinterpret_cast<uintptr_t>(src) | (uintptr_t)bytes | (uintptr_t)(pitch * (int)sizeof(T))) & 15) == 0) {
+    const int pieces = bytes >> 4;   // (at most 64, so the reciprocal is exact for the at most 1024 indexes)
+    const unsigned inv = 65536u / pieces + 1;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < nb * pieces; i += blockDim.x) {
+      const int r = (int)(((unsigned)i * inv) >> 16), k = i - r * pieces;
+      cp_async16(dst + r * dst_pitch + 16 * k, reinterpret_cast<const uint8_t*>(src + (size_t)r * pitch) + 16 * k);
+    }
+  } else {
+#pragma unroll 1
+    for (int r = threadIdx.x >> 5; r < nb; r += blockDim.x >> 5)
+#pragma unroll 1
+      for (int k = threadIdx.x & 31; k < cols; k += 32) reinterpret_cast<T*>(dst + r * dst_pitch)[k] = src[(size_t)r * pitch + k];
+  }
+}
+
+// columns 2q, 2q + 1 of a raw row as pairs of real and of imaginary parts
+template <typename T> __device__ __forceinline__ void raw_complex2(const uint8_t* row, int q, f2& re, f2& im) {
+  float2 a, b;
+  if constexpr (sizeof(T) == 2) {
+    const uint2 w = reinterpret_cast<const uint2*>(row)[q];
+    a = unpack_pair<T>(w.x); b = unpack_pair<T>(w.y);
+  } else {
+    const float4 w = reinterpret_cast<const float4*>(row)[q];
+    a = make_float2(w.x, w.y); b = make_float2(w.z, w.w);
+  }
+  re = mk2(a.x, b.x); im = mk2(a.y, b.y);
+}
+// column n of two successive raw rows, as pairs over the rows
+template <typename T> __device__ __forceinline__ void raw_tokens2(const uint8_t* row, int pitch, int n, f2& re, f2& im) {
+  float2 a, b;
+  if constexpr (sizeof(T) == 2) {
+    a = unpack_pair<T>(reinterpret_cast<const uint32_t*>(row)[n]);
+    b = unpack_pair<T>(reinterpret_cast<const uint32_t*>(row + pitch)[n]);
+  } else {
+    a = reinterpret_cast<const float2*>(row)[n];
+    b = reinterpret_cast<const float2*>(row + pitch)[n];
+  }
+  re = mk2(a.x, b.x); im = mk2(a.y, b.y);
+}
+template <typename T> __device__ __forceinline__ void raw_quad(const uint8_t* row, int q, f2 (&v)[2]) {   // elements 4q .. 4q + 3
+  if constexpr (sizeof(T) == 2) {
+    const uint2 w = reinterpret_cast<const uint2*>(row)[q];
+    const float2 a = unpack_pair<T>(w.x), b = unpack_pair<T>(w.y);
+    v[0] = mk2(a.x, a.y); v[1] = mk2(b.x, b.y);
+  } else {
+    const float4 w = reinterpret_cast<const float4*>(row)[q];
+    v[0] = mk2(w.x, w.y); v[1] = mk2(w.z, w.w);
+  }
+}
+__device__ __forceinline__ float hsum(f2 v) { const float2 q = un2(v); return q.x + q.y; }
+__device__ __forceinline__ f2 neg2(f2 v) { return mul2(v, dup2(-1.f)); }
+// (ar + i ai)(br + i bi) and its conjugated form conj(a) b, elementwise on pairs
+__device__ __forceinline__ void cmul2(f2 ar, f2 ai, f2 br, f2 bi, f2& re, f2& im) {
+  re = fma2(neg2(ai), bi, mul2(ar, br)); im = fma2(ai, br, mul2(ar, bi));
+}
+__device__ __forceinline__ void cmul2_conj_a(f2 ar, f2 ai, f2 br, f2 bi, f2& re, f2& im) {
+  re = fma2(ai, bi, mul2(ar, br)); im = fma2(neg2(ai), br, mul2(ar, bi));
+}
+// the latter added to re, im
+__device__ __forceinline__ void cmac2_conj_a(f2 ar, f2 ai, f2 br, f2 bi, f2& re, f2& im) {
+  re = fma2(ar, br, fma2(ai, bi, re)); im = fma2(ar, bi, fma2(neg2(ai), br, im));
+}
+__device__ __forceinline__ cf load_cf(const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return {v.x, v.y}; }
+__device__ __forceinline__ void store_cf(float* p, cf v) { *reinterpret_cast<float2*>(p) = make_float2(v.re, v.im); }
+// two successive complex numbers ``step`` floats apart as pairs
+__device__ __forceinline__ void load_cf2(const float* p, int step, f2& re, f2& im) {
+  const cf a = load_cf(p), b = load_cf(p + step);
+  re = mk2(a.re, b.re); im = mk2(a.im, b.im);
+}
+template <typename T> __device__ __forceinline__ cf load_c(const T* base, size_t cidx) {
   return {to_f32(base[2 * cidx]), to_f32(base[2 * cidx + 1])};
 }
+// two neighbouring elements of an array that may start anywhere; the second only if there is one
+template <typename T> __device__ __forceinline__ void store_two(T* dst, bool vec, float a, float b, bool second) {
+  if (vec && second) {
+    if constexpr (sizeof(T) == 2) *reinterpret_cast<uint32_t*>(dst) = pack_pair<T>(a, b);
+    else *reinterpret_cast<float2*>(dst) = make_float2(a, b);
+  } else {
+    dst[0] = from_f32<T>(a);
+    if (second) dst[1] = from_f32<T>(b);
+  }
+}
+__device__ __forceinline__ void put(float* dst, float v, bool add) {
+  if (add) atomicAdd(dst, v); else *dst = v;
+}
 
-// Where a thread sits: its warp's run of columns and rows, its 4 rows and NC columns (NC / 2 pairs).
-template <int NC>
+// Where a thread sits in its warp's 16 columns x 64 rows of the state, which are the accumulators of 16 x 8 products: 16
+// rows of 8 real and 8 imaginary parts.  Lane (g, q) holds column 8 grp + g of the warp's, rows 8 pt + 2q, + 1 of P.
 struct Place {
-  int lane, w, ns, pw, rg, cg, pl, pair;   // pl: first of the 4 rows inside the CTA tile; pair: first column pair
-  __device__ __forceinline__ Place(const SweepParams& p) {
+  int lane, w, g, q;
+  __device__ __forceinline__ Place() {
     lane = threadIdx.x & 31; w = threadIdx.x >> 5;
-    ns = w % p.NS; pw = w / p.NS; rg = lane >> 2; cg = lane & 3;
-    pl = pw * 32 + rg * 4; pair = (ns * 4 + cg) * (NC / 2);
+    g = lane >> 2; q = lane & 3;
   }
 };
-// 4 rows x NC / 2 pairs of columns, real and imaginary parts
-template <int NC> struct Tile { f2 re[4][NC / 2], im[4][NC / 2]; };
+struct Tile { f2 re[2][8], im[2][8]; };
 
-// src (P, 2N) of one (batch, head): the thread's piece, zeros outside
-template <int NC>
-__device__ __forceinline__ void load_tile(Tile<NC>& z, const float* src, const Place<NC>& o, int row0, int P, int N) {
-  const bool whole = (N & 1) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;   // 2 columns as one 16-byte piece
+// f(grp, pt, re pair, im pair) for the tile of src (P, 2N), zeros outside.  VEC: src is aligned to a complex number.
+template <bool VEC, typename F>
+__device__ __forceinline__ void read_tile(const float* src, const Place& o, int row0, int P, int N, F f) {
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+  for (int grp = 0; grp < 2; ++grp)
 #pragma unroll
-    for (int i = 0; i < NC / 2; ++i) {
-      const int n = 2 * (o.pair + i), row = row0 + r;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (src && row < P && n < N) {
-        const float* q = src + (size_t)row * 2 * N + 2 * n;
-        if (whole) v = *reinterpret_cast<const float4*>(q);
-        else {
-          v.x = q[0]; v.y = q[1];
-          if (n + 1 < N) { v.z = q[2]; v.w = q[3]; }
+    for (int pt = 0; pt < 8; ++pt) {
+      const int n = 16 * o.w + 8 * grp + o.g;
+      cf v[2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int row = row0 + 8 * pt + 2 * o.q + e;
+        const float* x = src + (size_t)row * 2 * N + 2 * n;
+        if (row < P && n < N) v[e] = VEC ? load_cf(x) : cf{x[0], x[1]};
+      }
+      f(grp, pt, mk2(v[0].re, v[1].re), mk2(v[0].im, v[1].im));
+    }
+}
+template <bool VEC>
+__device__ __forceinline__ void store_tile(const Tile& z, float* dst, const Place& o, int row0, int P, int N) {
+#pragma unroll
+  for (int grp = 0; grp < 2; ++grp)
+#pragma unroll
+    for (int pt = 0; pt < 8; ++pt) {
+      const int n = 16 * o.w + 8 * grp + o.g;
+      const float2 re = un2(z.re[grp][pt]), im = un2(z.im[grp][pt]);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int row = row0 + 8 * pt + 2 * o.q + e;
+        float* x = dst + (size_t)row * 2 * N + 2 * n;
+        if (row < P && n < N) {
+          const cf v = {e ? re.y : re.x, e ? im.y : im.x};
+          if (VEC) store_cf(x, v);
+          else { x[0] = v.re; x[1] = v.im; }
         }
       }
-      z.re[r][i] = mk2(v.x, v.z); z.im[r][i] = mk2(v.y, v.w);
     }
 }
-template <int NC>
-__device__ __forceinline__ void store_tile(const Tile<NC>& z, float* dst, const Place<NC>& o, int row0, int P, int N) {
+// z = m z (CONJ: conj(m) z)
+template <bool CONJ>
+__device__ __forceinline__ void scale_tile(Tile& z, cf m) {
+  const f2 r2 = dup2(m.re), i2 = dup2(CONJ ? -m.im : m.im), n2 = dup2(CONJ ? m.im : -m.im);
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+  for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int i = 0; i < NC / 2; ++i) {
-      const int n = 2 * (o.pair + i), row = row0 + r;
-      if (row >= P) continue;
-      const float2 re = un2(z.re[r][i]), im = un2(z.im[r][i]);
-      float* q = dst + (size_t)row * 2 * N + 2 * n;
-      if (n < N) { q[0] = re.x; q[1] = im.x; }
-      if (n + 1 < N) { q[2] = re.y; q[3] = im.y; }
-    }
-}
-// z = m z + add (CONJ: conj(m) z + add)
-template <int NC, bool CONJ>
-__device__ __forceinline__ void advance_tile(Tile<NC>& z, float mr, float mi, const Tile<NC>& add) {
-  const f2 r2 = dup2(mr), i2 = dup2(CONJ ? -mi : mi), n2 = dup2(CONJ ? mi : -mi);
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int i = 0; i < NC / 2; ++i) {
+    for (int i = 0; i < 8; ++i) {
       const f2 a = z.re[r][i], b = z.im[r][i];
-      z.re[r][i] = fma2(n2, b, fma2(r2, a, add.re[r][i]));
-      z.im[r][i] = fma2(i2, a, fma2(r2, b, add.im[r][i]));
+      z.re[r][i] = fma2(n2, b, mul2(r2, a));
+      z.im[r][i] = fma2(i2, a, mul2(r2, b));
     }
-}
-// Start state of a segment: the caller's state at that end of the sequence through the segments between, in walking order.
-template <int NC, bool CONJ>
-__device__ __forceinline__ void fold_tile(Tile<NC>& z, const SweepParams& p, const float* loc, const float* prod, int bh, int from,
-                                          int step, int count, const Place<NC>& o, int row0) {
-  const size_t bhs = (size_t)p.batch * p.heads;
-  constexpr int DEPTH = 8 / NC;   // segments of a batch of loads
-#pragma unroll 1
-  for (int k = 0; k < count; k += DEPTH) {
-    Tile<NC> add[DEPTH];
-    float2 m[DEPTH];
-#pragma unroll
-    for (int i = 0; i < DEPTH; ++i) {
-      if (k + i >= count) continue;
-      const size_t at = (from + step * (k + i)) * bhs + bh;
-      m[i] = *reinterpret_cast<const float2*>(prod + 2 * at);
-      load_tile<NC>(add[i], loc + at * p.P * 2 * p.N, o, row0, p.P, p.N);
-    }
-#pragma unroll
-    for (int i = 0; i < DEPTH; ++i)
-      if (k + i < count) advance_tile<NC, CONJ>(z, m[i].x, m[i].y, add[i]);
-  }
 }
 // Product of the transitions [t0, t1) (1 past the end of the sequence), by one warp, to dst.
 __device__ __forceinline__ void transition_product(const float* Mb, int t0, int t1, int T, float* dst) {
   const int lane = threadIdx.x & 31;
   double re = 1.0, im = 0.0;
+#pragma unroll 1
   for (int t = t0 + lane; t < t1; t += 32) {
     if (t >= T) continue;
     const double mr = Mb[2 * t], mi = Mb[2 * t + 1], r = re * mr - im * mi;
     im = re * mi + im * mr; re = r;
   }
-#pragma unroll
+#pragma unroll 1
   for (int o = 16; o > 0; o >>= 1) {
     const double orr = __shfl_xor_sync(0xffffffffu, re, o), oi = __shfl_xor_sync(0xffffffffu, im, o);
     const double r = re * orr - im * oi;
@@ -177,544 +364,828 @@ __device__ __forceinline__ void transition_product(const float* Mb, int t0, int 
   if (lane == 0) { dst[0] = (float)re; dst[1] = (float)im; }
 }
 
-// What every sweep reads of one (batch, head, slice of P).
-template <typename TIn, typename TY>
-struct Stream {
-  const TIn *U, *B, *C, *Bp, *Up;
-  const TY* dY;
-  const float *M, *K;
-  int bh, row0, seg, t_lo, t_hi;   // row0: first row of the CTA tile; [t_lo, t_hi): the segment
-  __device__ __forceinline__ Stream(const SweepParams& p, int pt, int segment) {
-    const int h = blockIdx.x, b = blockIdx.y, g = h / (p.heads / p.groups), D = 2 * p.N;
-    bh = b * p.heads + h;
-    const int bg = b * p.groups + g;
-    U = reinterpret_cast<const TIn*>(p.U) + (size_t)bh * p.T * p.P;
-    B = reinterpret_cast<const TIn*>(p.B) + (size_t)bg * p.T * D;
-    C = reinterpret_cast<const TIn*>(p.C) + (size_t)bg * p.T * D;
-    Bp = p.Bprev ? reinterpret_cast<const TIn*>(p.Bprev) + (size_t)bg * D : nullptr;
-    Up = p.Uprev ? reinterpret_cast<const TIn*>(p.Uprev) + (size_t)bh * p.P : nullptr;
-    dY = p.dY ? reinterpret_cast<const TY*>(p.dY) + (size_t)bh * p.T * p.P : nullptr;
-    M = p.M + (size_t)bh * p.T * 2;
-    K = p.K + (size_t)bh * p.T * 4;
-    row0 = pt * p.PW * 32; seg = segment;
-    t_lo = seg * p.seg_len; t_hi = min(p.T, t_lo + p.seg_len);
-  }
-};
-
-// A (rows, cols) array by the CTA, a warp per row: U rows are loaded, then stored, so that they cost one latency.
-template <int U, typename V, typename Load, typename Store>
-__device__ __forceinline__ void staged(int rows, int cols, Load load, Store store) {
-  const int nw = blockDim.x >> 5;
-#pragma unroll 1
-  for (int c = threadIdx.x & 31; c < cols; c += 32)
-#pragma unroll 1
-    for (int r = threadIdx.x >> 5; r < rows; r += U * nw) {
-      V v[U];
-#pragma unroll
-      for (int i = 0; i < U; ++i)
-        if (r + i * nw < rows) v[i] = load(r + i * nw, c);
-#pragma unroll
-      for (int i = 0; i < U; ++i)
-        if (r + i * nw < rows) store(r + i * nw, c, v[i]);
+// The products of one chunk, by one warp.  Lane l stands for the source token i = l - 1 (l = 0: the chunk's start state):
+// tab[j][l] = P(j, i), then per source h, P(nb, i) h, kc, the transition behind it and what float32 leaves of h.  In
+// float64, rounded once: an error of a product is common to all rows and columns of the state, so the sums over them do not
+// average it out as they do the roundings of a walk token by token (dU and dB came 10 to 15 % further from float64 with
+// float32 products).
+struct ChainIn { float2 m, kp, kc; };
+__device__ __forceinline__ ChainIn load_chain(const float* M, const float* K, int t0, int T, int lane) {
+  ChainIn in{make_float2(1.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+  const int t = t0 + lane;
+  if (lane <= L) {
+    if (t < T) {
+      in.m = *reinterpret_cast<const float2*>(M + 2 * (size_t)t);
+      in.kp = *reinterpret_cast<const float2*>(K + 4 * (size_t)t);
     }
-}
-template <typename F> __device__ __forceinline__ void each_row(int rows, int cols, F f) {
-  for (int r = threadIdx.x >> 5; r < rows; r += blockDim.x >> 5)
-    for (int c = threadIdx.x & 31; c < cols; c += 32) f(r, c);
-}
-
-// A token's columns in shared memory: pair (n, n+1) as re re im im
-__device__ __forceinline__ int pair_slot(int n) { return 4 * (n >> 1) + (n & 1); }
-
-// Stage tokens [t0, t0 + nb): the tapped b_{t-1} and b_t, c on request.
-template <typename TIn, typename TY>
-__device__ __forceinline__ void stage_columns(const SweepParams& p, const Stream<TIn, TY>& x, int t0, int nb, int Npad, float* s_bp,
-                                              float* s_bc, float* s_c) {
-  const int D = 2 * p.N, D2 = 2 * Npad;
-  struct Piece { cf bt, bpv, ct; float4 k4; };
-  staged<2, Piece>(nb, Npad, [&](int tt, int n) {
-    const int t = t0 + tt;
-    Piece v{};
-    if (n < p.N) {
-      if (s_bc) v.bt = load_c(x.B + (size_t)t * D, n);
-      if (s_c) v.ct = load_c(x.C + (size_t)t * D, n);
-      if (s_bp) {
-        if (t > 0) v.bpv = load_c(x.B + (size_t)(t - 1) * D, n);
-        else if (x.Bp) v.bpv = load_c(x.Bp, n);
-      }
-    }
-    if (s_bp || s_bc) v.k4 = *reinterpret_cast<const float4*>(x.K + (size_t)t * 4);
-    return v;
-  }, [&](int tt, int n, const Piece& v) {
-    const int o = tt * D2 + pair_slot(n);
-    const cf bp = cmul({v.k4.x, v.k4.y}, v.bpv), bc = cmul({v.k4.z, v.k4.w}, v.bt);
-    if (s_bp) { s_bp[o] = bp.re; s_bp[o + 2] = bp.im; }
-    if (s_bc) { s_bc[o] = bc.re; s_bc[o + 2] = bc.im; }
-    if (s_c) { s_c[o] = v.ct.re; s_c[o + 2] = v.ct.im; }
-  });
-}
-// u of the tokens t0 - 1 .. t0 + nb - 1
-template <typename TIn, typename TY>
-__device__ __forceinline__ void stage_u(const SweepParams& p, const Stream<TIn, TY>& x, int t0, int nb, int PT, float* s_u) {
-  staged<3, float>(nb + 1, PT, [&](int tt, int pp) {
-    const int t = t0 + tt - 1, pr = x.row0 + pp;
-    if (pr >= p.P) return 0.f;
-    if (t >= 0) return to_f32(x.U[(size_t)t * p.P + pr]);
-    return x.Up ? to_f32(x.Up[pr]) : 0.f;
-  }, [&](int tt, int pp, float v) { s_u[tt * PT + pp] = v; });
-}
-template <typename TIn, typename TY>
-__device__ __forceinline__ void stage_dy(const SweepParams& p, const Stream<TIn, TY>& x, int t0, int nb, int PT, float* s_dy) {
-  staged<2, float>(nb, PT, [&](int tt, int pp) {
-    const int pr = x.row0 + pp;
-    return (pr < p.P && x.dY) ? to_f32(x.dY[(size_t)(t0 + tt) * p.P + pr]) : 0.f;
-  }, [&](int tt, int pp, float v) { s_dy[tt * PT + pp] = v; });
-}
-// m of the tokens t0 + off ... (1 past the end of the sequence)
-__device__ __forceinline__ void stage_m(const float* M, int t0, int nb, int T, float* s_m) {
-  for (int idx = threadIdx.x; idx < nb; idx += blockDim.x) {
-    const int t = t0 + idx;
-    s_m[2 * idx] = t < T ? M[2 * (size_t)t] : 1.f;
-    s_m[2 * idx + 1] = t < T ? M[2 * (size_t)t + 1] : 0.f;
+    if (lane > 0 && t - 1 < T) in.kc = *reinterpret_cast<const float2*>(K + 4 * (size_t)(t - 1) + 2);
   }
+  return in;
 }
-
-__device__ __forceinline__ void rows4(const float* s, f2 (&v)[4]) {
-  const float4 q = *reinterpret_cast<const float4*>(s);
-  v[0] = dup2(q.x); v[1] = dup2(q.y); v[2] = dup2(q.z); v[3] = dup2(q.w);
+struct cd { double re, im; };
+__device__ __forceinline__ cd cmul(cd a, cd b) { return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
+__device__ __forceinline__ cf rounded(cd a) { return {(float)a.re, (float)a.im}; }
+__device__ __forceinline__ cd coefficient(const ChainIn& in) {   // h
+  const cd v = cmul(cd{in.m.x, in.m.y}, cd{in.kc.x, in.kc.y});
+  return {v.re + in.kp.x, v.im + in.kp.y};
 }
-__device__ __forceinline__ void pair_at(const float* s, int pair, f2& re, f2& im) {
-  const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(s + 4 * pair);
-  re = q.x; im = q.y;
-}
-__device__ __forceinline__ float hsum(f2 v) { const float2 q = un2(v); return q.x + q.y; }
-// sum over the rows of the warp of NC columns a lane: 2 NC values in smem order, scattered over the row lanes
-template <int NC>
-__device__ __forceinline__ void store_columns(const f2 (&re)[NC / 2], const f2 (&im)[NC / 2], int lane, int pair, float* dst) {
-  float v[2 * NC];
+// The whole table.  The chains of the first nine tokens and of the others run side by side in different lanes, and meet in
+// P(j, i) = P(9, i) P(j, 8): this warp's chain is what the others of its CTA wait for.
+__device__ __forceinline__ void chain(float* tab, const ChainIn& in, int nb, int lane) {
+  const bool hi = lane >= 9;
+  cd p = {1.0, 0.0}, end = {1.0, 0.0}, q[7];
+  if (lane == 0 || lane == 9) store_cf(tab + 2 * (lane * TABW + lane), {1.f, 0.f});
 #pragma unroll
-  for (int i = 0; i < NC / 2; ++i) {
-    const float2 a = un2(re[i]), b = un2(im[i]);
-    v[4 * i] = a.x; v[4 * i + 1] = a.y; v[4 * i + 2] = b.x; v[4 * i + 3] = b.y;
+  for (int s = 1; s <= 9; ++s) {
+    const int j = hi ? 9 + s : s;
+    const cd m = {__shfl_sync(0xffffffffu, in.m.x, j & 31), __shfl_sync(0xffffffffu, in.m.y, j & 31)};
+    if (lane < j && j <= L) p = cmul(p, m);
+    if (lane <= j && j <= L && lane <= L) store_cf(tab + 2 * (j * TABW + lane), rounded(p));
+    if (j == nb) end = p;
+    if (s <= 7) q[s - 1] = {__shfl_sync(0xffffffffu, p.re, 9), __shfl_sync(0xffffffffu, p.im, 9)};
   }
-  Scatter<2 * NC, 16, 4>::run(v, lane);
-  const int hi = (lane >> 4) & 1, mid = (lane >> 3) & 1, lo = (lane >> 2) & 1;
-  if constexpr (NC == 2) {   // 4 values over 8 lanes: two lanes hold each
-    if (!lo) dst[4 * pair + 2 * hi + mid] = v[0];
+#pragma unroll
+  for (int s = 1; s <= 7; ++s) {
+    const cd v = cmul(p, q[s - 1]);
+    if (!hi) {
+      store_cf(tab + 2 * ((9 + s) * TABW + lane), rounded(v));
+      if (9 + s == nb) end = v;
+    }
+  }
+  if (lane >= 1 && lane <= L) {
+    const int i = lane - 1;
+    const cd h = coefficient(in);
+    const cf hf = rounded(h);
+    store_cf(tab + V_H + 2 * i, hf);
+    store_cf(tab + V_HLOW + 2 * i, {(float)(h.re - hf.re), (float)(h.im - hf.im)});
+    store_cf(tab + V_KAPPA + 2 * i, rounded(cmul(end, h)));
+    store_cf(tab + V_KC + 2 * i, {in.kc.x, in.kc.y});
+    store_cf(tab + V_MNEXT + 2 * i, {in.m.x, in.m.y});
+  }
+}
+// What the pre-passes need of it: forward in time P(L, i) h_i (a chunk that is shorter ends in transitions of 1) and a_nb, the
+// adjoint's a_j; products over all later or all earlier lanes.
+template <bool ADJ>
+__device__ __forceinline__ void chain_ends(float* tab, const ChainIn& in, int nb, int lane) {
+  const bool own = lane >= 1 && lane <= L;
+  cd p = {own ? in.m.x : 1.0, own ? in.m.y : 0.0};
+#pragma unroll
+  for (int o = 1; o <= L; o <<= 1) {
+    const cd v = {ADJ ? __shfl_up_sync(0xffffffffu, p.re, o) : __shfl_down_sync(0xffffffffu, p.re, o),
+                  ADJ ? __shfl_up_sync(0xffffffffu, p.im, o) : __shfl_down_sync(0xffffffffu, p.im, o)};
+    if (ADJ ? lane >= o : lane + o < 32) p = cmul(p, v);
+  }
+  if (ADJ) {
+    if (lane <= L) store_cf(tab + 2 * lane * TABW, rounded(p));
   } else {
-    dst[4 * pair + 4 * hi + 2 * mid + lo] = v[0];
+    const cd end = {__shfl_down_sync(0xffffffffu, p.re, 1), __shfl_down_sync(0xffffffffu, p.im, 1)};   // over the lanes behind this one
+    if (own) store_cf(tab + V_KAPPA + 2 * (lane - 1), rounded(cmul(end, coefficient(in))));
+    if (lane == 0) store_cf(tab + 2 * nb * TABW, rounded(end));
   }
 }
 
-// MODE 0: forward (writes Y, final state).  1: backward sweep A (writes dc_head, sT).  2: only where the segment ends.
-template <typename TIn, typename TY, int NC, int MODE>
-__device__ __forceinline__ void forward_sweep(const SweepParams& p, int pt, int seg, float* smem) {
-  const Place<NC> o(p);
-  const int NS = p.NS, PW = p.PW, TB = p.TB, Npad = NS * 4 * NC, D2 = 2 * Npad, PT = PW * 32, D = 2 * p.N, N = p.N, P = p.P;
-  const Stream<TIn, TY> x(p, pt, seg);
-  float* s_bp = smem;
-  float* s_bc = s_bp + TB * D2;
-  float* s_c = s_bc + TB * D2;
-  float* s_u = s_c + TB * D2;             // (TB+1) x PT
-  float* s_m = s_u + (TB + 1) * PT;       // TB x 2
-  float* s_dy = s_m + 2 * TB;             // TB x PT       (MODE 1)
-  float* s_part = s_dy + TB * PT;         // MODE0: TB x NS x PT ; MODE1: TB x PW x D2
-  const int row0 = x.row0 + o.pl;
+// One walk of one segment.  FORWARD: Y and the final state.  SWEEP_A / SWEEP_B: the two sweeps of the backward.  STATES /
+// ADJ_STATES: only where the segment ends, from zero.
+template <typename TIn, typename TY, Mode MODE>
+__device__ __forceinline__ void walk(const SweepParams& p, int pt0, int seg, uint8_t* smem) {
+  constexpr bool REV = MODE == SWEEP_B || MODE == ADJ_STATES, BACK = MODE == SWEEP_A || MODE == SWEEP_B;
+  constexpr bool ONLY_STATES = MODE == STATES || MODE == ADJ_STATES;
+  constexpr bool USE_B = MODE != ADJ_STATES, USE_C = MODE != STATES, USE_DY = BACK || MODE == ADJ_STATES, USE_U = USE_B;
+  constexpr int NI = Parts<TIn>::N, NY = Parts<TY>::N;
+  const int W = p.W, N = p.N, P = p.P, T = p.T, D = 2 * N, NT = 32 * W;
+  const Layout lay(W, sizeof(TIn), sizeof(TY), NI, NY, MODE);
+  const Place o;
+  const int tid = threadIdx.x;
+  const int h = blockIdx.x, b = blockIdx.y, bh = b * p.heads + h, bg = b * p.groups + h / (p.heads / p.groups);
+  const int row0 = pt0 * ROWS, prows = min(ROWS, P - row0);
+  const TIn* U = reinterpret_cast<const TIn*>(p.U) + (size_t)bh * T * P + row0;
+  const TIn* B = reinterpret_cast<const TIn*>(p.B) + (size_t)bg * T * D;
+  const TIn* C = reinterpret_cast<const TIn*>(p.C) + (size_t)bg * T * D;
+  const TY* dY = p.dY ? reinterpret_cast<const TY*>(p.dY) + (size_t)bh * T * P + row0 : nullptr;
+  const float* M = p.M + (size_t)bh * T * 2;
+  const float* K = p.K + (size_t)bh * T * 4;
+  const int t_lo = seg * p.seg_len, t_hi = min(T, t_lo + p.seg_len), nchunks = (t_hi - t_lo + L - 1) / L;
+  float* tabs = reinterpret_cast<float*>(smem + lay.tab);
+  float4* part = reinterpret_cast<float4*>(smem + lay.part);
+  float4* dpart = reinterpret_cast<float4*>(smem + lay.dpart);
+  float* red = reinterpret_cast<float*>(smem + lay.red);
+  float* sig = reinterpret_cast<float*>(smem + lay.sig) + o.w * L;
+  float4* dd = reinterpret_cast<float4*>(smem + lay.dd);
+  auto first_of = [&](int c) { return t_lo + L * (REV ? nchunks - 1 - c : c); };   // first token of the walk's chunk c
+  auto raw = [&](int base, int pitch, int c, int j) { return smem + base + ((c & 1) * L + j) * pitch; };
 
-  Tile<NC> z;
-  load_tile<NC>(z, MODE != 2 && p.z0 ? p.z0 + (size_t)x.bh * P * D : nullptr, o, row0, P, N);
-  if (MODE != 2 && seg > 0) fold_tile<NC, false>(z, p, p.zloc, p.zprod, x.bh, 0, 1, seg, o, row0);
-  if (MODE == 2 && pt == 0 && o.w == 0)
-    transition_product(x.M, x.t_lo, x.t_hi, p.T, p.zprod + 2 * ((size_t)seg * p.batch * p.heads + x.bh));
-
-  for (int t0 = x.t_lo; t0 < x.t_hi; t0 += TB) {
-    const int nb = min(TB, x.t_hi - t0);
-    stage_columns(p, x, t0, nb, Npad, s_bp, s_bc, MODE == 0 ? s_c : nullptr);
-    stage_u(p, x, t0, nb, PT, s_u);
-    if (MODE == 1) stage_dy(p, x, t0, nb, PT, s_dy);
-    stage_m(x.M, t0, nb, p.T, s_m);
-    __syncthreads();
-
-    f2 up[4], u[4];
-    rows4(s_u + o.pl, up);
+  auto raw_u = [&](int c) { return smem + lay.u + (NI > 1 ? 0 : (c & 1) * L * lay.pU); };
+  auto raw_y = [&](int c) { return smem + lay.y + (NY > 1 ? 0 : (c & 1) * L * lay.pY); };
+  // tensors whose rows are converted are staged behind that, the others at the start of the chunk before
+  auto stage = [&](int c, bool converted) {
+    const int t0 = first_of(c), nb = min(L, t_hi - t0);
+    if (USE_U && converted == (NI > 1)) stage_rows<TIn>(raw_u(c), lay.pU, U + (size_t)t0 * P, nb, prows, P);
+    if (USE_DY && dY && converted == (NY > 1)) stage_rows<TY>(raw_y(c), lay.pY, dY + (size_t)t0 * P, nb, prows, P);
+    if (converted) return;
+    if (USE_B) stage_rows<TIn>(raw(lay.b, lay.pD, c, 0), lay.pD, B + (size_t)t0 * D, nb, D, D);
+    if (USE_C) stage_rows<TIn>(raw(lay.c, lay.pD, c, 0), lay.pD, C + (size_t)t0 * D, nb, D, D);
+  };
+  // rows of U or dY as bfloat16 parts; bfloat16 rows are their own
+  auto convert = [&](auto type, const uint8_t* rows, int pitch, int parts) {
+    using X = decltype(type);
+    constexpr int NP = Parts<X>::N;
 #pragma unroll 1
-    for (int tt = 0; tt < nb; ++tt) {
-      const f2 mr = dup2(s_m[2 * tt]), mi = dup2(s_m[2 * tt + 1]), mn = dup2(-s_m[2 * tt + 1]);
-      rows4(s_u + (tt + 1) * PT + o.pl, u);
-      f2 acc[4], sre[NC / 2], sim[NC / 2], dy[4];
-      if (MODE == 1) rows4(s_dy + tt * PT + o.pl, dy);
+    for (int i = tid; i < L * ROWS / 4; i += NT) {
+      f2 v[2];
+      raw_quad<X>(rows + (i >> 4) * pitch, i & 15, v);
+      uint32_t w0[NP], w1[NP];
+      split<NP>(v[0], w0); split<NP>(v[1], w1);
 #pragma unroll
-      for (int i = 0; i < NC / 2; ++i) {
-        f2 ar, ai, cr, ci, qr, qi;
-        pair_at(s_bp + tt * D2, o.pair + i, ar, ai);
-        pair_at(s_bc + tt * D2, o.pair + i, cr, ci);
-        if (MODE == 0) pair_at(s_c + tt * D2, o.pair + i, qr, qi);
+      for (int k = 0; k < NP; ++k)
+        *reinterpret_cast<uint2*>(smem + parts + (k * L + (i >> 4)) * lay.pP + 8 * (i & 15)) = make_uint2(w0[k], w1[k]);
+    }
+  };
+  auto u_rows = [&](int c, int k) -> const uint8_t* { return NI == 1 ? raw_u(c) : smem + lay.up + k * L * lay.pP; };
+  auto y_rows = [&](int c, int k) -> const uint8_t* { return NY == 1 ? raw_y(c) : smem + lay.yp + k * L * lay.pP; };
+  static_assert(row_pitch(ROWS * 2) == 144, "raw bfloat16 rows and parts have one pitch");
+  constexpr int PP = 144;
+  const int r_lo = ((o.lane & 7) + 8 * ((o.lane >> 3) & 1)) * PP + 16 * (o.lane >> 4);     // ldmatrix: 16 tokens first, then 16 rows of P
+  const int r_hi = ((o.lane & 7) + 8 * (o.lane >> 4)) * PP + 16 * ((o.lane >> 3) & 1);     // and the other way round
+
+  // Columns beyond N and rows beyond P stay zero for good.  (So do the tokens that a ragged chunk has not in a walk backwards,
+  // which begins with it; forward in time such tokens have h = 0, and their results are not stored.)
+#pragma unroll 1
+  for (int i = tid; i < lay.raw_end / 16; i += NT) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+  stage(0, false);
+  stage(0, true);
+  auto products_of = [&](int c, const ChainIn& in) {   // one warp
+    float* tab = tabs + (c & 1) * TABF;
+    const int nb = min(L, t_hi - first_of(c));
+    if constexpr (ONLY_STATES) chain_ends<REV>(tab, in, nb, o.lane);
+    else chain(tab, in, nb, o.lane);
+  };
+  if (o.w == 0) products_of(0, load_chain(M, K, first_of(0), T, o.lane));
+
+  // ---- start state -------------------------------------------------------------------------------------------------
+  Tile z;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const f2 a = z.re[r][i], b = z.im[r][i];
-          const f2 zr = fma2(u[r], cr, fma2(up[r], ar, fma2(mn, b, mul2(mr, a))));
-          const f2 zi = fma2(u[r], ci, fma2(up[r], ai, fma2(mi, a, mul2(mr, b))));
-          z.re[r][i] = zr; z.im[r][i] = zi;
-          if (MODE == 0) acc[r] = fma2(qi, zi, i == 0 ? mul2(qr, zr) : fma2(qr, zr, acc[r]));
-          if (MODE == 1) {
-            sre[i] = r == 0 ? mul2(dy[r], zr) : fma2(dy[r], zr, sre[i]);
-            sim[i] = r == 0 ? mul2(dy[r], zi) : fma2(dy[r], zi, sim[i]);
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) z.re[r][i] = z.im[r][i] = 0ull;
+  if (!ONLY_STATES) {
+    auto take = [&](int r, int i, f2 re, f2 im) { z.re[r][i] = re; z.im[r][i] = im; };
+    if (p.nseg > 1) {   // combined by the launch before
+      read_tile<true>((REV ? p.gloc : p.zloc) + ((size_t)seg * p.batch * p.heads + bh) * P * D, o, row0, P, N, take);
+    } else if (REV) {
+      if (p.dfinal) read_tile<false>(p.dfinal + (size_t)bh * P * D, o, row0, P, N, take);
+    } else {
+      if (p.z0) {
+        read_tile<false>(p.z0 + (size_t)bh * P * D, o, row0, P, N, take);
+        scale_tile<false>(z, load_cf(M));
+      }
+      if (p.Bprev) {   // the prev-tap of the first token
+        const TIn* Bp = reinterpret_cast<const TIn*>(p.Bprev) + (size_t)bg * D;
+        const TIn* Up = reinterpret_cast<const TIn*>(p.Uprev) + (size_t)bh * P + row0;
+        const cf kp = load_cf(K);
+#pragma unroll
+        for (int grp = 0; grp < 2; ++grp) {
+          const int n = 16 * o.w + 8 * grp + o.g;
+          const cf x = n < N ? cmul(kp, load_c(Bp, n)) : cf{0.f, 0.f};
+#pragma unroll
+          for (int pt = 0; pt < 8; ++pt) {
+            const int r = 8 * pt + 2 * o.q;
+            const f2 u = mk2(r < prows ? to_f32(Up[r]) : 0.f, r + 1 < prows ? to_f32(Up[r + 1]) : 0.f);
+            z.re[grp][pt] = fma2(u, dup2(x.re), z.re[grp][pt]);
+            z.im[grp][pt] = fma2(u, dup2(x.im), z.im[grp][pt]);
           }
         }
       }
-      if (MODE == 0) {
-        float v[4] = {hsum(acc[0]), hsum(acc[1]), hsum(acc[2]), hsum(acc[3])};
-        Scatter<4, 2, 1>::run(v, o.lane);   // lane now holds row ``lane`` of the warp
-        s_part[(tt * NS + o.ns) * PT + o.pw * 32 + o.lane] = v[0];
-      }
-      if (MODE == 1) store_columns<NC>(sre, sim, o.lane, o.pair, s_part + (tt * PW + o.pw) * D2);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) up[r] = u[r];
     }
-    __syncthreads();
-
-    if (MODE == 0) {
-      TY* Yb = reinterpret_cast<TY*>(p.Y) + (size_t)x.bh * p.T * P;
-      each_row(nb, PT, [&](int tt, int pp) {
-        const int pr = x.row0 + pp;
-        if (pr < P) {
-          float s = 0.f;
-          for (int k = 0; k < NS; ++k) s += s_part[(tt * NS + k) * PT + pp];
-          Yb[(size_t)(t0 + tt) * P + pr] = from_f32<TY>(s);
-        }
-      });
-    }
-    if (MODE == 1) {
-      float* dcb = p.dc_head + (size_t)x.bh * p.T * D;
-      each_row(nb, D, [&](int tt, int col) {
-        const int slot = pair_slot(col >> 1) + 2 * (col & 1);
-        float s = 0.f;
-        for (int k = 0; k < PW; ++k) s += s_part[(tt * PW + k) * D2 + slot];
-        float* dst = dcb + (size_t)(t0 + tt) * D + col;
-        if (p.ptiles > 1) atomicAdd(dst, s); else *dst = s;
-      });
-    }
-    // the staging of the next block only rewrites arrays last read before the
-    // second barrier; s_part is next written after the first barrier of that block.
+  } else if (pt0 == 0 && o.w == W - 1) {
+    transition_product(M, t_lo + 1, t_hi + 1, T, (REV ? p.gprod : p.zprod) + 2 * ((size_t)seg * p.batch * p.heads + bh));
   }
 
-  if (MODE == 2) store_tile<NC>(z, p.zloc + ((size_t)seg * p.batch * p.heads + x.bh) * P * D, o, row0, P, N);
-  if (MODE == 0 && p.zfinal && seg == p.nseg - 1) store_tile<NC>(z, p.zfinal + (size_t)x.bh * P * D, o, row0, P, N);
-  if (MODE == 1 && seg == p.nseg - 1) {
-    // S_T = sum d_final * conj(z_final)
-    Tile<NC> d;
-    load_tile<NC>(d, p.dfinal ? p.dfinal + (size_t)x.bh * P * D : nullptr, o, row0, P, N);
-    f2 sr2 = 0, si2 = 0;
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int i = 0; i < NC / 2; ++i) {
-        sr2 = fma2(d.re[r][i], z.re[r][i], fma2(d.im[r][i], z.im[r][i], sr2));
-        si2 = add2(si2, fma2(d.im[r][i], z.re[r][i], mul2(mul2(d.re[r][i], dup2(-1.f)), z.im[r][i])));
-      }
-    const float sr = warp_sum(hsum(sr2)), si = warp_sum(hsum(si2));
-    __syncthreads();
-    if (o.lane == 0) { s_part[2 * o.w] = sr; s_part[2 * o.w + 1] = si; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float ar = 0.f, ai = 0.f;
-      for (int k = 0; k < (int)(blockDim.x >> 5); ++k) { ar += s_part[2 * k]; ai += s_part[2 * k + 1]; }
-      float* dst = p.sT + (size_t)x.bh * 2;
-      if (p.ptiles > 1) { atomicAdd(dst, ar); atomicAdd(dst + 1, ai); }
-      else { dst[0] = ar; dst[1] = ai; }
-    }
-  }
-}
-
-// Backward sweep B: reverse in time.  STATES: only where the segment ends (at its first token).
-template <typename TIn, typename TY, int NC, bool STATES>
-__device__ __forceinline__ void reverse_sweep(const SweepParams& p, int pt, int seg, float* smem) {
-  const Place<NC> o(p);
-  const int NS = p.NS, PW = p.PW, TB = p.TB, Npad = NS * 4 * NC, D2 = 2 * Npad, PT = PW * 32, D = 2 * p.N, N = p.N, P = p.P;
-  const Stream<TIn, TY> x(p, pt, seg);
-  float* s_bp = smem;
-  float* s_bc = s_bp + TB * D2;
-  float* s_c = s_bc + TB * D2;
-  float* s_u = s_c + TB * D2;              // (TB+1) x PT
-  float* s_mn = s_u + (TB + 1) * PT;       // TB x 2 : m_{t+1}
-  float* s_dy = s_mn + 2 * TB;             // TB x PT
-  float* s_pc = s_dy + TB * PT;            // TB x PW x D2
-  float* s_pp = s_pc + TB * PW * D2;       // TB x PW x D2
-  float* s_duc = s_pp + TB * PW * D2;      // TB x NS x PT
-  float* s_dup = s_duc + TB * NS * PT;     // TB x NS x PT
-  float* s_carry = s_dup + TB * NS * PT;   // 2 x PT: what the token after a block adds to the block's last dU
-  const int row0 = x.row0 + o.pl, t_last = (x.t_hi - x.t_lo - 1) / TB * TB + x.t_lo;
-
-  Tile<NC> G;
-  load_tile<NC>(G, !STATES && p.dfinal ? p.dfinal + (size_t)x.bh * P * D : nullptr, o, row0, P, N);
-  if (!STATES && seg < p.nseg - 1)
-    fold_tile<NC, true>(G, p, p.gloc, p.gprod, x.bh, p.nseg - 1, -1, p.nseg - 1 - seg, o, row0);
-  if (STATES && pt == 0 && o.w == 0)
-    transition_product(x.M, x.t_lo + 1, x.t_hi + 1, p.T, p.gprod + 2 * ((size_t)seg * p.batch * p.heads + x.bh));
-
-  auto row_sums = [&](const f2 (&v)[4], float* dst) {   // over the lane's columns and the 4 column lanes
-    float q[4] = {hsum(v[0]), hsum(v[1]), hsum(v[2]), hsum(v[3])};
-    Scatter<4, 2, 1>::run(q, o.lane);
-    dst[o.ns * PT + o.pw * 32 + o.lane] = q[0];
-  };
-  auto u_dot = [&](const float* s_col, f2 (&acc)[4]) {   // sum over the lane's columns of col . G
-#pragma unroll
-    for (int i = 0; i < NC / 2; ++i) {
-      f2 cr, ci;
-      pair_at(s_col, o.pair + i, cr, ci);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[r] = fma2(ci, G.im[r][i], i == 0 ? mul2(cr, G.re[r][i]) : fma2(cr, G.re[r][i], acc[r]));
-    }
-  };
-  if (!STATES) {
-    for (int idx = threadIdx.x; idx < 2 * PT; idx += blockDim.x) s_carry[idx] = 0.f;
-    if (x.t_hi < p.T) {   // the token after the segment
-      stage_columns(p, x, x.t_hi, 1, Npad, s_bp, static_cast<float*>(nullptr), static_cast<float*>(nullptr));
-      __syncthreads();
-      f2 acc[4];
-      u_dot(s_bp, acc);
-      row_sums(acc, s_dup);
-      __syncthreads();
-      for (int pp = threadIdx.x; pp < PT; pp += blockDim.x)
-        for (int k = 0; k < NS; ++k) s_carry[pp] += s_dup[k * PT + pp];
-      __syncthreads();
-    }
-  }
-
-  int par = 0;
-  for (int t0 = t_last; t0 >= x.t_lo; t0 -= TB, par ^= 1) {
-    const int nb = min(TB, x.t_hi - t0);
-    stage_columns(p, x, t0, nb, Npad, STATES ? nullptr : s_bp, STATES ? nullptr : s_bc, s_c);
-    if (!STATES) stage_u(p, x, t0, nb, PT, s_u);
-    stage_dy(p, x, t0, nb, PT, s_dy);
-    stage_m(x.M, t0 + 1, nb, p.T, s_mn);
-    __syncthreads();
-
+  // per-token scalars of chunk c from the warps' parts; warp W - 1, after the barrier that follows the chunk
+  auto finish_scalars = [&](int c) {
+    const int t0 = first_of(c), nb = min(L, t_hi - t0), j = o.lane;
+    if (o.w != W - 1 || j >= nb) return;
+    float re = 0.f, im = 0.f;
 #pragma unroll 1
-    for (int tt = nb - 1; tt >= 0; --tt) {
-      const f2 mr = dup2(s_mn[2 * tt]), mi = dup2(s_mn[2 * tt + 1]), mn = dup2(-s_mn[2 * tt + 1]);
-      f2 dy[4];
-      rows4(s_dy + tt * PT + o.pl, dy);
-      // G = conj(m_{t+1}) G + dy * c_t
+    for (int k = 0; k < W; ++k) { const cf v = load_cf(red + 2 * (((c & 1) * W + k) * L + j)); re += v.re; im += v.im; }
+    const size_t t = (size_t)bh * T + t0 + j;
+    const bool add = p.ptiles > 1;
+    if (MODE == SWEEP_A) { put(p.sterm + 2 * t, re, add); put(p.sterm + 2 * t + 1, im, add); }
+    if (MODE == SWEEP_B) {
+      float* dkp = t0 + j + 1 < T ? p.dK + 4 * (t + 1) : p.dM + 2 * t;   // dkp of the next token; the last one's for finish_dm
+      put(dkp, re, add); put(dkp + 1, im, add);
+      const float4 sd = dd[(c & 1) * L + j];
+      const cf g = cmul_conj_a({sd.z, sd.w}, {re, im});
+      put(p.dK + 4 * t + 2, g.re + sd.x, add); put(p.dK + 4 * t + 3, g.im + sd.y, add);
+    }
+  };
+
+  for (int c = 0; c < nchunks; ++c) {
+    const int t0 = first_of(c), nb = min(L, t_hi - t0);
+    const float* tab = tabs + (c & 1) * TABF;
+    cp_async_wait();
+    __syncthreads();
+    if (BACK && c > 0) finish_scalars(c - 1);
+    ChainIn next{};
+    if (c + 1 < nchunks) {
+      stage(c + 1, false);
+      if (o.w == 0) next = load_chain(M, K, first_of(c + 1), T, o.lane);
+    }
+    if ((USE_U && NI > 1) || (USE_DY && NY > 1)) {
+      if (USE_U && NI > 1) convert(TIn{}, raw_u(c), lay.pU, lay.up);
+      if (USE_DY && NY > 1) convert(TY{}, raw_y(c), lay.pY, lay.yp);
+      __syncthreads();
+      if (c + 1 < nchunks) stage(c + 1, true);
+    }
+    // column 8 grp + g of the warp's at the tokens 8 tt + 2q, + 1, as pairs over the tokens
+    auto tokens_of = [&](int base, int grp, int tt, f2& re, f2& im) {
+      raw_tokens2<TIn>(raw(base, lay.pD, c, 8 * tt + 2 * o.q), lay.pD, 16 * o.w + 8 * grp + o.g, re, im);
+    };
+    // columns 8 grp + 2q, + 1 at token 8 tt + g, as pairs over the columns
+    auto columns_of = [&](int base, int grp, int tt, f2& re, f2& im) {
+      raw_complex2<TIn>(raw(base, lay.pD, c, 8 * tt + o.g), 8 * o.w + 4 * grp + o.q, re, im);
+    };
+
+    // ---- <c_j, b_i> over the warp's columns: rows j (SWEEP_B: i), columns i (j) ---------------------------------------
+    if (MODE == FORWARD || MODE == SWEEP_B) {
+      f2 re[2][2], im[2][2];   // [column tile][row half]
 #pragma unroll
-      for (int i = 0; i < NC / 2; ++i) {
-        f2 qr, qi;
-        pair_at(s_c + tt * D2, o.pair + i, qr, qi);
+      for (int k = 0; k < 4; ++k) re[k >> 1][k & 1] = im[k >> 1][k & 1] = 0ull;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const f2 a = G.re[r][i], b = G.im[r][i];
-          G.re[r][i] = fma2(dy[r], qr, fma2(mi, b, mul2(mr, a)));
-          G.im[r][i] = fma2(dy[r], qi, fma2(mn, a, mul2(mr, b)));
+      for (int grp = 0; grp < 2; ++grp) {
+        uint32_t a[NI][4];
+#pragma unroll
+        for (int tt = 0; tt < 2; ++tt) {
+          f2 r, i;
+          uint32_t wr[NI], wi[NI];
+          columns_of(MODE == FORWARD ? lay.c : lay.b, grp, tt, r, i);
+          split<NI>(r, wr); split<NI>(i, wi);
+#pragma unroll
+          for (int k = 0; k < NI; ++k) { a[k][tt] = wr[k]; a[k][2 + tt] = wi[k]; }
+        }
+        uint32_t x[4][NI][2];   // [column tile: re, im]
+#pragma unroll
+        for (int tt = 0; tt < 2; ++tt) {
+          f2 r, i;
+          uint32_t wr[NI], wi[NI];
+          columns_of(MODE == FORWARD ? lay.b : lay.c, grp, tt, r, i);
+          split<NI>(r, wr); split<NI>(i, wi);
+#pragma unroll
+          for (int k = 0; k < NI; ++k) {
+            x[2 * tt][k][0] = wr[k]; x[2 * tt][k][1] = wi[k];
+            // Im <c, b> = c_re b_im - c_im b_re
+            x[2 * tt + 1][k][0] = MODE == FORWARD ? wi[k] : wi[k] ^ 0x80008000u;
+            x[2 * tt + 1][k][1] = MODE == FORWARD ? wr[k] ^ 0x80008000u : wr[k];
+          }
+        }
+        float d[4][4];
+        products<4, NI, NI>(d, [&](int) { return &a[0]; }, [&](int t) { return &x[t][0]; });
+#pragma unroll
+        for (int tt = 0; tt < 2; ++tt) {
+          re[tt][0] = add2(re[tt][0], mk2(d[2 * tt][0], d[2 * tt][1])); re[tt][1] = add2(re[tt][1], mk2(d[2 * tt][2], d[2 * tt][3]));
+          im[tt][0] = add2(im[tt][0], mk2(d[2 * tt + 1][0], d[2 * tt + 1][1]));
+          im[tt][1] = add2(im[tt][1], mk2(d[2 * tt + 1][2], d[2 * tt + 1][3]));
         }
       }
-      if (STATES) continue;
-      f2 acc[4], w[4], sre[NC / 2], sim[NC / 2];
-      u_dot(s_bc + tt * D2, acc);
-      row_sums(acc, s_duc + tt * NS * PT);
-      u_dot(s_bp + tt * D2, acc);
-      row_sums(acc, s_dup + tt * NS * PT);
-      auto outer = [&](const float* s_row, float* dst) {
-        rows4(s_row, w);
 #pragma unroll
-        for (int i = 0; i < NC / 2; ++i)
-#pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            sre[i] = r == 0 ? mul2(w[r], G.re[r][i]) : fma2(w[r], G.re[r][i], sre[i]);
-            sim[i] = r == 0 ? mul2(w[r], G.im[r][i]) : fma2(w[r], G.im[r][i], sim[i]);
-          }
-        store_columns<NC>(sre, sim, o.lane, o.pair, dst);
-      };
-      outer(s_u + (tt + 1) * PT + o.pl, s_pc + (tt * PW + o.pw) * D2);
-      outer(s_u + tt * PT + o.pl, s_pp + (tt * PW + o.pw) * D2);
+      for (int tt = 0; tt < 2; ++tt) {
+        const float2 r0 = un2(re[tt][0]), r1 = un2(re[tt][1]), i0 = un2(im[tt][0]), i1 = un2(im[tt][1]);
+        dpart[(o.w * 4 + 2 * tt) * 32 + o.lane] = make_float4(r0.x, r0.y, r1.x, r1.y);
+        dpart[(o.w * 4 + 2 * tt + 1) * 32 + o.lane] = make_float4(i0.x, i0.y, i1.x, i1.y);
+      }
     }
-    __syncthreads();
-    if (STATES) continue;
 
-    each_row(nb, D, [&](int tt, int col) {
-      const int slot = pair_slot(col >> 1) + 2 * (col & 1);
-      float sc = 0.f, sp = 0.f;
-      for (int k = 0; k < PW; ++k) {
-        sc += s_pc[(tt * PW + k) * D2 + slot];
-        sp += s_pp[(tt * PW + k) * D2 + slot];
+    // ---- products with the state at the chunk's start -----------------------------------------------------------------
+    f2 hre[2][2], him[2][2];   // SWEEP_A, SWEEP_B: sum over the rows of P of dy_j (u_i) times the state, [grp][token tile]
+    if (!ONLY_STATES) {
+      constexpr bool CROSS = MODE != SWEEP_A;
+      uint32_t op[2][3][4];    // FORWARD: conj(a_j) c_j, SWEEP_B: P(L,i) h_i b_i; rows tokens
+      if (CROSS) {
+#pragma unroll
+        for (int tt = 0; tt < 2; ++tt) {
+          const cf s = load_cf(MODE == FORWARD ? tab + 2 * (8 * tt + o.g) * TABW : tab + V_KAPPA + 2 * (8 * tt + o.g));
+#pragma unroll
+          for (int grp = 0; grp < 2; ++grp) {
+            f2 r, i, xr, xi;
+            uint32_t wr[3], wi[3];
+            columns_of(MODE == FORWARD ? lay.c : lay.b, grp, tt, r, i);
+            if (MODE == FORWARD) cmul2_conj_a(dup2(s.re), dup2(s.im), r, i, xr, xi);
+            else cmul2(dup2(s.re), dup2(s.im), r, i, xr, xi);
+            split<3>(xr, wr); split<3>(xi, wi);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) { op[grp][k][tt] = wr[k]; op[grp][k][2 + tt] = wi[k]; }
+          }
+        }
       }
-      const size_t q = ((size_t)x.bh * p.T + t0 + tt) * D + col;
-      if (p.ptiles > 1) { atomicAdd(p.dbc_head + q, sc); atomicAdd(p.dbp_head + q, sp); }
-      else { p.dbc_head[q] = sc; p.dbp_head[q] = sp; }
-    });
-    TIn* dUb = reinterpret_cast<TIn*>(p.dU) + (size_t)x.bh * p.T * P;
-    each_row(nb, PT, [&](int tt, int pp) {
-      const int pr = x.row0 + pp;
-      float s = tt == nb - 1 ? s_carry[par * PT + pp] : 0.f;
-      for (int k = 0; k < NS; ++k) s += s_duc[(tt * NS + k) * PT + pp];
-      if (tt < nb - 1)
-        for (int k = 0; k < NS; ++k) s += s_dup[((tt + 1) * NS + k) * PT + pp];
-      if (pr < P) dUb[(size_t)(t0 + tt) * P + pr] = from_f32<TIn>(s);
-      if (tt == 0) {
-        float c = 0.f;
-        for (int k = 0; k < NS; ++k) c += s_dup[k * PT + pp];
-        s_carry[(par ^ 1) * PT + pp] = c;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) hre[k >> 1][k & 1] = him[k >> 1][k & 1] = 0ull;
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {   // 16 rows of P at a time
+        constexpr int NR = MODE == SWEEP_A ? NY : NI;
+        uint32_t rows[2][NR][2];      // [token tile]
+        if (BACK)
+#pragma unroll
+          for (int k = 0; k < NR; ++k) {
+            uint32_t r[4];
+            ldmatrix4<false>(r, (MODE == SWEEP_A ? y_rows(c, k) : u_rows(c, k)) + r_hi + 32 * s);
+            rows[0][k][0] = r[0]; rows[0][k][1] = r[1]; rows[1][k][0] = r[2]; rows[1][k][1] = r[3];
+          }
+        f2 y0[2], y1[2];              // FORWARD, SWEEP_B: [pt]: tokens g and 8 + g
+        uint32_t a[2][3][4];
+#pragma unroll
+        for (int grp = 0; grp < 2; ++grp)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            uint32_t wr[3], wi[3];
+            split<3>(z.re[grp][2 * s + k], wr); split<3>(z.im[grp][2 * s + k], wi);
+#pragma unroll
+            for (int x = 0; x < 3; ++x) { a[grp][x][2 * k] = wr[x]; a[grp][x][2 * k + 1] = wi[x]; }
+          }
+        if (BACK) {
+          float d[4][4];   // [grp, token tile]
+          products<4, 3, NR>(d, [&](int t) { return &a[t >> 1][0]; }, [&](int t) { return &rows[t & 1][0]; });
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            hre[t >> 1][t & 1] = add2(hre[t >> 1][t & 1], mk2(d[t][0], d[t][1]));
+            him[t >> 1][t & 1] = add2(him[t >> 1][t & 1], mk2(d[t][2], d[t][3]));
+          }
+        }
+        if (CROSS) {
+          uint32_t x[4][3][2];   // [grp, pt]
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+              x[t][e][0] = transposed(a[t >> 1][e][2 * (t & 1)]); x[t][e][1] = transposed(a[t >> 1][e][2 * (t & 1) + 1]);
+            }
+          float d[4][4];
+          products<4, 3, 3>(d, [&](int t) { return &op[t >> 1][0]; }, [&](int t) { return &x[t][0]; });
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            y0[k] = add2(mk2(d[k][0], d[k][1]), mk2(d[2 + k][0], d[2 + k][1]));
+            y1[k] = add2(mk2(d[k][2], d[k][3]), mk2(d[2 + k][2], d[2 + k][3]));
+          }
+        }
+        if (CROSS)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const float2 v0 = un2(y0[k]), v1 = un2(y1[k]);
+            part[(o.w * 8 + 2 * s + k) * 32 + o.lane] = make_float4(v0.x, v0.y, v1.x, v1.y);
+          }
       }
-    });
-    // the next block's staging rewrites arrays last read before the second barrier; s_pc, s_pp, s_duc, s_dup and the
-    // other half of s_carry are next written or read after its first barrier.
+    }
+
+    // ---- SWEEP_A, SWEEP_B: the chunk's own part, dC / dB and the scalars -----------------------------------------------
+    if (BACK) {
+      // X(j,i) = <dy_j, u_i>: rows j, columns i in SWEEP_A, the other way round in SWEEP_B
+      constexpr int NA = MODE == SWEEP_A ? NY : NI, NB = MODE == SWEEP_A ? NI : NY;
+      f2 x[2][2];   // [column tile][row half]
+      x[0][0] = x[0][1] = x[1][0] = x[1][1] = 0ull;
+#pragma unroll
+      for (int s = 0; s < 4; s += 2) {
+        uint32_t a[2][NA][4], r[4][NB][2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+#pragma unroll
+          for (int k = 0; k < NA; ++k) ldmatrix4<false>(a[e][k], (MODE == SWEEP_A ? y_rows(c, k) : u_rows(c, k)) + r_lo + 32 * (s + e));
+#pragma unroll
+          for (int k = 0; k < NB; ++k) {
+            uint32_t v[4];
+            ldmatrix4<false>(v, (MODE == SWEEP_A ? u_rows(c, k) : y_rows(c, k)) + r_hi + 32 * (s + e));
+            r[2 * e][k][0] = v[0]; r[2 * e][k][1] = v[1]; r[2 * e + 1][k][0] = v[2]; r[2 * e + 1][k][1] = v[3];
+          }
+        }
+        float d[4][4];   // [rows of P, column tile]
+        products<4, NA, NB>(d, [&](int t) { return &a[t >> 1][0]; }, [&](int t) { return &r[t][0]; });
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          x[t][0] = add2(x[t][0], add2(mk2(d[t][0], d[t][1]), mk2(d[2 + t][0], d[2 + t][1])));
+          x[t][1] = add2(x[t][1], add2(mk2(d[t][2], d[t][3]), mk2(d[2 + t][2], d[2 + t][3])));
+        }
+      }
+      if (o.q == (o.g >> 1)) {   // the diagonal
+        const float2 v0 = un2(x[0][0]), v1 = un2(x[1][1]);
+        sig[o.g] = (o.g & 1) ? v0.y : v0.x;
+        sig[8 + o.g] = (o.g & 1) ? v1.y : v1.x;
+      }
+      __syncwarp();
+      // times the coefficients, below the diagonal: A  P(j,i) h_i,  B  conj(P(j,i)); columns of the product below
+      uint32_t x3[4][3][2];   // [real, imaginary; token tile]
+#pragma unroll
+      for (int tt = 0; tt < 2; ++tt)
+#pragma unroll
+        for (int it = 0; it < 2; ++it) {
+          const int own = 8 * tt + o.g, src = 8 * it + 2 * o.q;   // A: j = own, i = src; B: i = own, j = src
+          f2 pr, pi, gr, gi;
+          if (MODE == SWEEP_A) {
+            f2 hr, hi;
+            load_cf2(tab + 2 * (own * TABW + src + 1), 2, pr, pi);
+            load_cf2(tab + V_H + 2 * src, 2, hr, hi);
+            cmul2(pr, pi, hr, hi, gr, gi);
+          } else {
+            load_cf2(tab + 2 * (src * TABW + own + 1), 2 * TABW, gr, pi);
+            gi = neg2(pi);
+          }
+          const float2 vr = un2(mul2(x[it][tt], gr)), vi = un2(mul2(x[it][tt], gi));
+          const bool m0 = MODE == SWEEP_A ? src < own : src > own, m1 = MODE == SWEEP_A ? src + 1 < own : src + 1 > own;
+          uint32_t wr[3], wi[3];
+          split<3>(mk2(m0 ? vr.x : 0.f, m1 ? vr.y : 0.f), wr);
+          split<3>(mk2(m0 ? vi.x : 0.f, m1 ? vi.y : 0.f), wi);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) { x3[tt][k][it] = wr[k]; x3[2 + tt][k][it] = wi[k]; }
+        }
+      const int other = MODE == SWEEP_A ? lay.b : lay.c, self = MODE == SWEEP_A ? lay.c : lay.b;
+      f2 sre[2], sim[2];   // <c_j, .>, <b_i, .> over the lane's columns, [token tile]
+      sre[0] = sre[1] = sim[0] = sim[1] = 0ull;
+#pragma unroll
+      for (int grp = 0; grp < 2; ++grp) {
+        uint32_t a[2][NI][4];   // (re | im) and (-im | re)
+        f2 ore[2], oim[2];
+#pragma unroll
+        for (int tt = 0; tt < 2; ++tt) {
+          uint32_t wr[NI], wi[NI];
+          tokens_of(other, grp, tt, ore[tt], oim[tt]);
+          split<NI>(ore[tt], wr); split<NI>(oim[tt], wi);
+#pragma unroll
+          for (int k = 0; k < NI; ++k) {
+            a[0][k][2 * tt] = wr[k]; a[0][k][2 * tt + 1] = wi[k];
+            a[1][k][2 * tt] = wi[k] ^ 0x80008000u; a[1][k][2 * tt + 1] = wr[k];
+          }
+        }
+        float d[4][4];   // [times the real, the imaginary factors; token tile]
+        products<4, NI, 3>(d, [&](int t) { return &a[t >> 1][0]; }, [&](int t) { return &x3[t][0]; });
+#pragma unroll
+        for (int tt = 0; tt < 2; ++tt) {
+          const int t = 8 * tt + 2 * o.q;
+          f2 er, ei, vr, vi, nr, ni;
+          f2 pr = add2(mk2(d[tt][0], d[tt][1]), mk2(d[2 + tt][0], d[2 + tt][1]));
+          f2 pi = add2(mk2(d[tt][2], d[tt][3]), mk2(d[2 + tt][2], d[2 + tt][3]));
+          if (MODE == SWEEP_A) {   // a_j times the sum
+            load_cf2(tab + 2 * t * TABW, 2 * TABW, er, ei);
+            cmul2(er, ei, hre[grp][tt], him[grp][tt], vr, vi);
+          } else {                 // conj(P(L,i)) times the sum
+            load_cf2(tab + 2 * (nb * TABW + t + 1), 2, er, ei);
+            cmul2_conj_a(er, ei, hre[grp][tt], him[grp][tt], vr, vi);
+          }
+          vr = add2(vr, pr); vi = add2(vi, pi);
+          f2 sr, si, kr, ki;
+          tokens_of(self, grp, tt, sr, si);
+          // A: <.., c>: c conj(v); B: conj(b) v
+          sre[tt] = fma2(si, vi, fma2(sr, vr, sre[tt]));
+          sim[tt] = MODE == SWEEP_A ? fma2(neg2(sr), vi, fma2(si, vr, sim[tt])) : fma2(neg2(si), vr, fma2(sr, vi, sim[tt]));
+          load_cf2(tab + V_KC + 2 * t, 2, kr, ki);
+          const f2 sg = *reinterpret_cast<const f2*>(sig + t);
+          if (MODE == SWEEP_A) {   // + X(j,j) kc_j b_j
+            cmul2(mul2(sg, kr), mul2(sg, ki), ore[tt], oim[tt], nr, ni);
+            nr = add2(nr, vr); ni = add2(ni, vi);
+          } else {                 // conj(h_i) D_i + X(i,i) conj(kc_i) c_i
+            f2 hr, hi;
+            load_cf2(tab + V_HLOW + 2 * t, 2, hr, hi);
+            cmul2_conj_a(hr, hi, vr, vi, nr, ni);
+            cmac2_conj_a(mul2(sg, kr), mul2(sg, ki), ore[tt], oim[tt], nr, ni);
+            load_cf2(tab + V_H + 2 * t, 2, hr, hi);
+            cmac2_conj_a(hr, hi, vr, vi, nr, ni);
+          }
+          const float2 o_re = un2(nr), o_im = un2(ni);
+          const int n = 16 * o.w + 8 * grp + o.g;
+#pragma unroll
+          for (int e1 = 0; e1 < 2; ++e1) {
+            if (n >= N || t + e1 >= nb) continue;
+            const float v_re = e1 ? o_re.y : o_re.x, v_im = e1 ? o_im.y : o_im.x;
+            if (p.spread) {
+              float* dst = (MODE == SWEEP_A ? p.dC_head : p.dB_head) + ((size_t)bh * T + t0 + t + e1) * D + 2 * n;
+              put(dst, v_re, p.ptiles > 1); put(dst + 1, v_im, p.ptiles > 1);
+            } else {
+              TIn* dst = reinterpret_cast<TIn*>(MODE == SWEEP_A ? p.dC : p.dB) + ((size_t)bg * T + t0 + t + e1) * D + 2 * n;
+              store_two(dst, (reinterpret_cast<uintptr_t>(dst) & (2 * sizeof(TIn) - 1)) == 0, v_re, v_im, true);
+            }
+          }
+        }
+      }
+      float v[8];   // [token tile][re, im][token]
+#pragma unroll
+      for (int tt = 0; tt < 2; ++tt) {
+        const float2 r = un2(sre[tt]), i = un2(sim[tt]);
+        v[4 * tt] = r.x; v[4 * tt + 1] = r.y; v[4 * tt + 2] = i.x; v[4 * tt + 3] = i.y;
+      }
+      Scatter<8, 16, 4>::run(v, o.lane);
+      red[2 * (((c & 1) * W + o.w) * L + 8 * ((o.lane >> 4) & 1) + 2 * o.q + ((o.lane >> 2) & 1)) + ((o.lane >> 3) & 1)] = v[0];
+    }
+
+    // ---- the state behind the chunk --------------------------------------------------------------------------------------
+    {
+      constexpr int NR = REV ? NY : NI;
+      uint32_t op[2][3][4];   // columns of P(L,i) h_i b_i or of conj(a_j) c_j, k = token
+#pragma unroll
+      for (int tt = 0; tt < 2; ++tt) {
+        const int t = 8 * tt + 2 * o.q;
+        f2 er, ei;
+        if (REV) load_cf2(tab + 2 * t * TABW, 2 * TABW, er, ei);
+        else load_cf2(tab + V_KAPPA + 2 * t, 2, er, ei);
+#pragma unroll
+        for (int grp = 0; grp < 2; ++grp) {
+          f2 r, i, xr, xi;
+          uint32_t wr[3], wi[3];
+          tokens_of(REV ? lay.c : lay.b, grp, tt, r, i);
+          if (REV) cmul2_conj_a(er, ei, r, i, xr, xi);
+          else cmul2(er, ei, r, i, xr, xi);
+          split<3>(xr, wr); split<3>(xi, wi);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) { op[grp][k][2 * tt] = wr[k]; op[grp][k][2 * tt + 1] = wi[k]; }
+        }
+      }
+      const cf m = load_cf(tab + 2 * nb * TABW);
+      const f2 r2 = dup2(m.re), i2 = dup2(REV ? -m.im : m.im), n2 = dup2(REV ? m.im : -m.im);
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        uint32_t rows[2][NR][2];   // [pt]
+#pragma unroll
+        for (int k = 0; k < NR; ++k) {
+          uint32_t r[4];
+          ldmatrix4<true>(r, (REV ? y_rows(c, k) : u_rows(c, k)) + r_lo + 32 * s);
+          rows[0][k][0] = r[0]; rows[0][k][1] = r[1]; rows[1][k][0] = r[2]; rows[1][k][1] = r[3];
+        }
+        float d[4][4];   // [grp, pt]
+        products<4, 3, NR>(d, [&](int t) { return &op[t >> 1][0]; }, [&](int t) { return &rows[t & 1][0]; });
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const int grp = t >> 1, k = t & 1;
+          const f2 zr = z.re[grp][2 * s + k], zi = z.im[grp][2 * s + k];
+          z.re[grp][2 * s + k] = fma2(n2, zi, fma2(r2, zr, mk2(d[t][0], d[t][1])));
+          z.im[grp][2 * s + k] = fma2(i2, zr, fma2(r2, zi, mk2(d[t][2], d[t][3])));
+        }
+      }
+    }
+    if (c + 1 < nchunks && o.w == 0) products_of(c + 1, next);
+    if (MODE != FORWARD && MODE != SWEEP_B) continue;
+    __syncthreads();
+
+    // ---- y or dU: the warps' sums, and the chunk's own part S u (S^T dy) ---------------------------------------------------
+    {
+      using TO = typename std::conditional<MODE == FORWARD, TY, TIn>::type;
+      constexpr int NR = MODE == FORWARD ? NI : NY;
+      TO* out = reinterpret_cast<TO*>(MODE == FORWARD ? p.Y : p.dU) + ((size_t)bh * T + t0) * P + row0;
+      const bool vec = (P & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & (2 * sizeof(TO) - 1)) == 0;
+      uint32_t a[3][4];
+#pragma unroll
+      for (int it = 0; it < 2; ++it) {
+        float4 dr = dpart[2 * it * 32 + o.lane], di = dpart[(2 * it + 1) * 32 + o.lane];
+#pragma unroll 1
+        for (int k = 1; k < W; ++k) {
+          const float4 r = dpart[(k * 4 + 2 * it) * 32 + o.lane], i = dpart[(k * 4 + 2 * it + 1) * 32 + o.lane];
+          dr.x += r.x; dr.y += r.y; dr.z += r.z; dr.w += r.w;
+          di.x += i.x; di.y += i.y; di.z += i.z; di.w += i.w;
+        }
+#pragma unroll
+        for (int tt = 0; tt < 2; ++tt) {
+          const int own = 8 * tt + o.g, src = 8 * it + 2 * o.q;   // FORWARD: j = own, i = src; SWEEP_B: i = own, j = src
+          const f2 vr = tt ? mk2(dr.z, dr.w) : mk2(dr.x, dr.y), vi = tt ? mk2(di.z, di.w) : mk2(di.x, di.y);
+          f2 pr, pi, hr, hi, gr, gi;
+          if (MODE == FORWARD) {
+            load_cf2(tab + 2 * (own * TABW + src + 1), 2, pr, pi);
+            load_cf2(tab + V_H + 2 * src, 2, hr, hi);
+          } else {
+            load_cf2(tab + 2 * (src * TABW + own + 1), 2 * TABW, pr, pi);
+            const cf h1 = load_cf(tab + V_H + 2 * own);
+            hr = dup2(h1.re); hi = dup2(h1.im);
+          }
+          cmul2(pr, pi, hr, hi, gr, gi);
+          const cf kc = load_cf(tab + V_KC + 2 * own);
+          const float2 s = un2(fma2(neg2(gi), vi, mul2(gr, vr))), v_r = un2(vr), v_i = un2(vi);
+          const float g0 = kc.re * v_r.x - kc.im * v_i.x, g1 = kc.re * v_r.y - kc.im * v_i.y;
+          const bool m0 = MODE == FORWARD ? src < own : src > own, m1 = MODE == FORWARD ? src + 1 < own : src + 1 > own;
+          uint32_t wd[3];
+          split<3>(mk2(src == own ? g0 : m0 ? s.x : 0.f, src + 1 == own ? g1 : m1 ? s.y : 0.f), wd);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) a[k][2 * it + tt] = wd[k];
+          if (MODE == SWEEP_B && o.w == 0 && it == tt && o.q == (o.g >> 1)) {
+            const cf mn = load_cf(tab + V_MNEXT + 2 * own);
+            dd[(c & 1) * L + own] = make_float4(sig[own] * ((o.g & 1) ? v_r.y : v_r.x), -sig[own] * ((o.g & 1) ? v_i.y : v_i.x), mn.re, mn.im);
+          }
+        }
+      }
+#pragma unroll 1
+      for (int pt = o.w; pt < 8; pt += W) {
+        uint32_t rows[NR][2];
+#pragma unroll
+        for (int k = 0; k < NR; ++k) {
+          uint32_t r[4];   // (the second pair of tiles is not used)
+          ldmatrix4<true>(r, (MODE == FORWARD ? u_rows(c, k) : y_rows(c, k)) + ((o.lane & 15) * PP) + 16 * pt);
+          rows[k][0] = r[0]; rows[k][1] = r[1];
+        }
+        float d[1][4];
+        products<1, 3, NR>(d, [&](int) { return &a[0]; }, [&](int) { return &rows[0]; });
+        float4 v = part[pt * 32 + o.lane];
+#pragma unroll 1
+        for (int k = 1; k < W; ++k) {
+          const float4 x = part[(k * 8 + pt) * 32 + o.lane];
+          v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+        }
+        const int pp = 8 * pt + 2 * o.q;
+        if (pp < prows) {
+          if (o.g < nb) store_two(out + (size_t)o.g * P + pp, vec, v.x + d[0][0], v.y + d[0][1], pp + 1 < prows);
+          if (8 + o.g < nb) store_two(out + (size_t)(8 + o.g) * P + pp, vec, v.z + d[0][2], v.w + d[0][3], pp + 1 < prows);
+        }
+      }
+    }
   }
-  if (STATES) {
-    store_tile<NC>(G, p.gloc + ((size_t)seg * p.batch * p.heads + x.bh) * P * D, o, row0, P, N);
+
+  if (ONLY_STATES) {
+    store_tile<true>(z, (REV ? p.gloc : p.zloc) + ((size_t)seg * p.batch * p.heads + bh) * P * D, o, row0, P, N);
     return;
   }
-  if (seg > 0) return;
+  if (MODE == FORWARD && p.zfinal && seg == p.nseg - 1) store_tile<false>(z, p.zfinal + (size_t)bh * P * D, o, row0, P, N);
+  if (!BACK) return;
   __syncthreads();
-  if (p.dUprev) {
-    TIn* dUp = reinterpret_cast<TIn*>(p.dUprev) + (size_t)x.bh * P;
-    for (int pp = threadIdx.x; pp < PT; pp += blockDim.x)
-      if (x.row0 + pp < P) dUp[x.row0 + pp] = from_f32<TIn>(s_carry[par * PT + pp]);
+  finish_scalars(nchunks - 1);
+  float* scratch = reinterpret_cast<float*>(smem);   // (the raw rows are done with)
+  if (MODE == SWEEP_A && seg == p.nseg - 1) {   // S_T = sum d_final conj(z_final)
+    f2 sr = 0ull, si = 0ull;
+    if (p.dfinal)
+      read_tile<false>(p.dfinal + (size_t)bh * P * D, o, row0, P, N, [&](int r, int i, f2 re, f2 im) {
+        sr = fma2(im, z.im[r][i], fma2(re, z.re[r][i], sr));
+        si = fma2(neg2(re), z.im[r][i], fma2(im, z.re[r][i], si));
+      });
+    const float re = warp_sum(hsum(sr)), im = warp_sum(hsum(si));
+    if (o.lane == 0) { scratch[2 * o.w] = re; scratch[2 * o.w + 1] = im; }
+    __syncthreads();
+    if (tid == 0) {
+      float a = 0.f, d = 0.f;
+      for (int k = 0; k < W; ++k) { a += scratch[2 * k]; d += scratch[2 * k + 1]; }
+      put(p.sT + 2 * (size_t)bh, a, p.ptiles > 1); put(p.sT + 2 * (size_t)bh + 1, d, p.ptiles > 1);
+    }
   }
-  if (p.dinit) {
-    Tile<NC> zero{};
-    advance_tile<NC, true>(G, x.M[0], x.M[1], zero);
-    store_tile<NC>(G, p.dinit + (size_t)x.bh * P * D, o, row0, P, N);
+  if (MODE == SWEEP_B && seg == 0) {   // z = lambda_0: the start state and the prev-tap of the first token
+    if (p.Bprev) {
+      const TIn* Bp = reinterpret_cast<const TIn*>(p.Bprev) + (size_t)bg * D;
+      const TIn* Up = reinterpret_cast<const TIn*>(p.Uprev) + (size_t)bh * P + row0;
+      const cf kp = load_cf(K);
+      float* s_du = scratch + 2 * W;   // [W][64]: Re sum conj(kp b_prev) lambda over a warp's columns
+      cf dkp = {0.f, 0.f}, x[2];
+#pragma unroll
+      for (int grp = 0; grp < 2; ++grp) {   // sum over the rows of u_prev lambda, per column
+        const int n = 16 * o.w + 8 * grp + o.g;
+        f2 sr = 0ull, si = 0ull;
+#pragma unroll
+        for (int pt = 0; pt < 8; ++pt) {
+          const int r = 8 * pt + 2 * o.q;
+          const f2 u = mk2(r < prows ? to_f32(Up[r]) : 0.f, r + 1 < prows ? to_f32(Up[r + 1]) : 0.f);
+          sr = fma2(u, z.re[grp][pt], sr); si = fma2(u, z.im[grp][pt], si);
+        }
+        float re = hsum(sr), im = hsum(si);
+        re += __shfl_xor_sync(0xffffffffu, re, 1); im += __shfl_xor_sync(0xffffffffu, im, 1);
+        re += __shfl_xor_sync(0xffffffffu, re, 2); im += __shfl_xor_sync(0xffffffffu, im, 2);
+        const cf bp = n < N ? load_c(Bp, n) : cf{0.f, 0.f};
+        x[grp] = cmul(kp, bp);
+        if (o.q == 0 && n < N) {
+          const cf g = cmul_conj_a(kp, {re, im});
+          dkp = cadd(dkp, cmul_conj_a(bp, {re, im}));
+          if (p.dBprev) {
+            if (p.spread) {
+              float* dst = p.dBprev_head + (size_t)bh * D + 2 * n;
+              put(dst, g.re, p.ptiles > 1); put(dst + 1, g.im, p.ptiles > 1);
+            } else {
+              TIn* dst = reinterpret_cast<TIn*>(p.dBprev) + (size_t)bg * D + 2 * n;
+              dst[0] = from_f32<TIn>(g.re); dst[1] = from_f32<TIn>(g.im);
+            }
+          }
+        }
+      }
+      const float re = warp_sum(dkp.re), im = warp_sum(dkp.im);
+      if (o.lane == 0) { scratch[2 * o.w] = re; scratch[2 * o.w + 1] = im; }
+#pragma unroll
+      for (int pt = 0; pt < 8; ++pt) {
+        f2 v = 0ull;
+#pragma unroll
+        for (int grp = 0; grp < 2; ++grp) v = fma2(dup2(x[grp].im), z.im[grp][pt], fma2(dup2(x[grp].re), z.re[grp][pt], v));
+        float2 s = un2(v);
+#pragma unroll
+        for (int m = 4; m < 32; m <<= 1) { s.x += __shfl_xor_sync(0xffffffffu, s.x, m); s.y += __shfl_xor_sync(0xffffffffu, s.y, m); }
+        if (o.g == 0) { s_du[o.w * ROWS + 8 * pt + 2 * o.q] = s.x; s_du[o.w * ROWS + 8 * pt + 2 * o.q + 1] = s.y; }
+      }
+      __syncthreads();
+      if (p.dUprev)
+        for (int r = tid; r < prows; r += NT) {
+          float s = 0.f;
+          for (int k = 0; k < W; ++k) s += s_du[k * ROWS + r];
+          reinterpret_cast<TIn*>(p.dUprev)[(size_t)bh * P + row0 + r] = from_f32<TIn>(s);
+        }
+    }
+    if (tid == 0) {
+      cf dkp = {0.f, 0.f};
+      if (p.Bprev)
+        for (int k = 0; k < W; ++k) dkp = cadd(dkp, load_cf(scratch + 2 * k));
+      put(p.dK + (size_t)bh * T * 4, dkp.re, p.ptiles > 1); put(p.dK + (size_t)bh * T * 4 + 1, dkp.im, p.ptiles > 1);
+    }
+    if (p.dinit) {
+      scale_tile<true>(z, load_cf(M));
+      store_tile<false>(z, p.dinit + (size_t)bh * P * D, o, row0, P, N);
+    }
   }
 }
 
 // grid (heads, batch, ptiles x segments [x the two sweeps])
-template <typename TIn, typename TY, int NC>
-__global__ void __launch_bounds__(128 * NC) sweep_fwd_kernel(SweepParams p) {
-  extern __shared__ __align__(16) float smem[];
-  forward_sweep<TIn, TY, NC, 0>(p, blockIdx.z % p.ptiles, blockIdx.z / p.ptiles, smem);
+template <typename TIn, typename TY>
+__global__ void __maxnreg__(168) sweep_fwd_kernel(SweepParams p) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  walk<TIn, TY, FORWARD>(p, blockIdx.z % p.ptiles, blockIdx.z / p.ptiles, smem);
 }
-template <typename TIn, typename TY, int NC>
-__global__ void __launch_bounds__(128 * NC) sweep_bwd_kernel(SweepParams p) {
-  extern __shared__ __align__(16) float smem[];
+template <typename TIn, typename TY>
+__global__ void __maxnreg__(168) sweep_bwd_kernel(SweepParams p) {
+  extern __shared__ __align__(16) uint8_t smem[];
   const int pt = blockIdx.z % p.ptiles, seg = blockIdx.z / p.ptiles;   // the longer sweep first
-  if (seg < p.nseg) reverse_sweep<TIn, TY, NC, false>(p, pt, seg, smem);
-  else forward_sweep<TIn, TY, NC, 1>(p, pt, seg - p.nseg, smem);
+  if (seg < p.nseg) walk<TIn, TY, SWEEP_B>(p, pt, seg, smem);
+  else walk<TIn, TY, SWEEP_A>(p, pt, seg - p.nseg, smem);
 }
 // where each segment ends from zero: forward segments 0 .. nseg - 2, and for the backward also reverse segments 1 .. nseg - 1
-template <typename TIn, typename TY, int NC>
-__global__ void __launch_bounds__(128 * NC) segment_kernel(SweepParams p) {
-  extern __shared__ __align__(16) float smem[];
+template <typename TIn, typename TY>
+__global__ void __maxnreg__(168) segment_kernel(SweepParams p) {
+  extern __shared__ __align__(16) uint8_t smem[];
   const int pt = blockIdx.z % p.ptiles, seg = blockIdx.z / p.ptiles;
-  if (seg < p.nseg - 1) forward_sweep<TIn, TY, NC, 2>(p, pt, seg, smem);
-  else reverse_sweep<TIn, TY, NC, true>(p, pt, seg - (p.nseg - 2), smem);
+  if (seg < p.nseg - 1) walk<TIn, TY, STATES>(p, pt, seg, smem);
+  else walk<TIn, TY, ADJ_STATES>(p, pt, seg - (p.nseg - 2), smem);
 }
 
-// One warp per (batch, group, t): dK and the dM scan terms per head, dB / dC summed
-// over the heads of the group.
+// From where the segments end from zero to where they start: the caller's state at that end of the sequence through the
+// segments between, in walking order and in place (all in float32).  A thread per (row, column) of the state, 8 segments'
+// loads at a time; blockIdx.z 0: the walk forward in time, 1: the adjoint's.  (Folded by every CTA of the sweeps for itself
+// this was a chain of up to nseg round trips to L2 in front of each: at (2, 4, 256, N 32) 48 of the forward sweep's 50 us.)
+template <typename TIn>
+__global__ void __launch_bounds__(256) combine_kernel(SweepParams p) {
+  const int e = blockIdx.y * 256 + threadIdx.x, bh = blockIdx.x, N = p.N, D = 2 * N, nseg = p.nseg;
+  if (e >= p.P * N) return;
+  const bool rev = blockIdx.z != 0;
+  const size_t bhs = (size_t)p.batch * p.heads, size = (size_t)p.P * D;
+  float* loc = (rev ? p.gloc : p.zloc) + bh * size + 2 * (size_t)e;
+  const float* prod = (rev ? p.gprod : p.zprod) + 2 * (size_t)bh;
+  const float* init = rev ? p.dfinal : p.z0;
+  cf z = {0.f, 0.f};
+  if (init) z = {init[bh * size + 2 * (size_t)e], init[bh * size + 2 * (size_t)e + 1]};
+  if (!rev) {
+    z = cmul(load_cf(p.M + (size_t)bh * p.T * 2), z);
+    if (p.Bprev) {   // the prev-tap of the first token
+      const int row = e / N, n = e % N, bg = bh / p.heads * p.groups + bh % p.heads / (p.heads / p.groups);
+      const cf x = cmul(load_cf(p.K + (size_t)bh * p.T * 4), load_c(reinterpret_cast<const TIn*>(p.Bprev) + (size_t)bg * D, n));
+      const float u = to_f32(reinterpret_cast<const TIn*>(p.Uprev)[(size_t)bh * p.P + row]);
+      z = {z.re + u * x.re, z.im + u * x.im};
+    }
+  }
+  for (int k0 = 0; k0 < nseg; k0 += 8) {
+    cf f[8], m[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      f[k] = m[k] = {0.f, 0.f};
+      if (k0 + k < nseg - 1) {   // (nothing starts behind the last segment of the walk)
+        const size_t at = (size_t)(rev ? nseg - 1 - (k0 + k) : k0 + k) * bhs;
+        f[k] = load_cf(loc + at * size); m[k] = load_cf(prod + 2 * at);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (k0 + k >= nseg) break;
+      store_cf(loc + (size_t)(rev ? nseg - 1 - (k0 + k) : k0 + k) * bhs * size, z);
+      z = cadd(rev ? cmul_conj_a(m[k], z) : cmul(m[k], z), f[k]);
+    }
+  }
+}
+
+// What follows the sweeps, in one launch: dM per (batch, head), and where heads or slices of P were still apart, dB, dC
+// and dB_prev from their float32 parts.
+constexpr int FINISH = 1024;   // threads
 struct FinishParams {
-  const void *B, *C, *Bprev;
-  const float *K, *dc_head, *dbc_head, *dbp_head;
-  float *dK, *sterm;
+  const float *M, *K, *dK, *sterm, *sT, *dB_head, *dC_head, *dBprev_head;
+  float* dM;
   void *dB, *dC, *dBprev;
-  int batch, heads, groups, T, N;
+  int BH, heads, groups, T, N, spread;
 };
 
-template <typename TIn>
-__global__ void __launch_bounds__(256) bwd_finish_kernel(FinishParams p) {
-  constexpr int MAXN = 4;  // N <= 128
-  const int lane = threadIdx.x & 31;
-  const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const long long rows = (long long)p.batch * p.groups * p.T;
-  if (row >= rows) return;
-  const int t = (int)(row % p.T);
-  const int bg = (int)(row / p.T);
-  const int g = bg % p.groups, b = bg / p.groups;
-  const int hpg = p.heads / p.groups, N = p.N, D = 2 * N, T = p.T;
-  const TIn* Bb = reinterpret_cast<const TIn*>(p.B) + ((size_t)bg * T) * D;
-  const TIn* Cb = reinterpret_cast<const TIn*>(p.C) + ((size_t)bg * T) * D;
-  const TIn* Bp = p.Bprev ? reinterpret_cast<const TIn*>(p.Bprev) + (size_t)bg * D : nullptr;
-
-  cf bt[MAXN], bprev[MAXN], ct[MAXN], db[MAXN], dc[MAXN], dbp0[MAXN];
-#pragma unroll
-  for (int i = 0; i < MAXN; ++i) {
-    const int n = lane + 32 * i;
-    bt[i] = bprev[i] = ct[i] = db[i] = dc[i] = dbp0[i] = {0.f, 0.f};
-    if (n < N) {
-      bt[i] = load_c(Bb + (size_t)t * D, n);
-      ct[i] = load_c(Cb + (size_t)t * D, n);
-      if (t > 0) bprev[i] = load_c(Bb + (size_t)(t - 1) * D, n);
-      else if (Bp) bprev[i] = load_c(Bp, n);
-    }
-  }
-  for (int hh = 0; hh < hpg; ++hh) {
-    const int h = g * hpg + hh;
-    const size_t bh = (size_t)b * p.heads + h;
-    const float* Kt = p.K + (bh * T + t) * 4;
-    const cf kp = {Kt[0], Kt[1]}, kc = {Kt[2], Kt[3]};
-    cf kpn = {0.f, 0.f};
-    if (t + 1 < T) kpn = {Kt[4], Kt[5]};
-    const float* dch = p.dc_head + (bh * T + t) * D;
-    const float* dbch = p.dbc_head + (bh * T + t) * D;
-    const float* dbph = p.dbp_head + (bh * T + t) * D;
-    float kcr = 0.f, kci = 0.f, kpr = 0.f, kpi = 0.f, sr = 0.f, si = 0.f;
-#pragma unroll
-    for (int i = 0; i < MAXN; ++i) {
-      const int n = lane + 32 * i;
-      if (n < N) {
-        const cf vdc = {dch[2 * n], dch[2 * n + 1]};
-        const cf vbc = {dbch[2 * n], dbch[2 * n + 1]};
-        const cf vbp = {dbph[2 * n], dbph[2 * n + 1]};
-        // dkc += dbc * conj(b_t); dkp += dbp * conj(b_{t-1}); s += c_t * conj(dc_t)
-        kcr += vbc.re * bt[i].re + vbc.im * bt[i].im;
-        kci += vbc.im * bt[i].re - vbc.re * bt[i].im;
-        kpr += vbp.re * bprev[i].re + vbp.im * bprev[i].im;
-        kpi += vbp.im * bprev[i].re - vbp.re * bprev[i].im;
-        sr += ct[i].re * vdc.re + ct[i].im * vdc.im;
-        si += ct[i].im * vdc.re - ct[i].re * vdc.im;
-        db[i] = cadd(db[i], cmul_conj_a(kc, vbc));
-        if (t + 1 < T) {
-          const cf vbpn = {dbph[D + 2 * n], dbph[D + 2 * n + 1]};
-          db[i] = cadd(db[i], cmul_conj_a(kpn, vbpn));
-        }
-        dc[i] = cadd(dc[i], vdc);
-        if (t == 0) dbp0[i] = cadd(dbp0[i], cmul_conj_a(kp, vbp));
-      }
-    }
-    kcr = warp_sum(kcr); kci = warp_sum(kci); kpr = warp_sum(kpr); kpi = warp_sum(kpi);
-    sr = warp_sum(sr); si = warp_sum(si);
-    if (lane == 0) {
-      float* dKt = p.dK + (bh * T + t) * 4;
-      dKt[0] = kpr; dKt[1] = kpi; dKt[2] = kcr; dKt[3] = kci;
-      // s_t = <c,dc> - conj(kp) dkp - conj(kc) dkc
-      const cf a = cmul_conj_a(kp, {kpr, kpi}), c2 = cmul_conj_a(kc, {kcr, kci});
-      float* st = p.sterm + (bh * T + t) * 2;
-      st[0] = sr - a.re - c2.re;
-      st[1] = si - a.im - c2.im;
-    }
-  }
-  TIn* dBo = reinterpret_cast<TIn*>(p.dB) + ((size_t)bg * T + t) * D;
-  TIn* dCo = reinterpret_cast<TIn*>(p.dC) + ((size_t)bg * T + t) * D;
-#pragma unroll
-  for (int i = 0; i < MAXN; ++i) {
-    const int n = lane + 32 * i;
-    if (n < N) {
-      dBo[2 * n] = from_f32<TIn>(db[i].re); dBo[2 * n + 1] = from_f32<TIn>(db[i].im);
-      dCo[2 * n] = from_f32<TIn>(dc[i].re); dCo[2 * n + 1] = from_f32<TIn>(dc[i].im);
-      if (t == 0 && p.dBprev) {
-        TIn* o = reinterpret_cast<TIn*>(p.dBprev) + (size_t)bg * D;
-        o[2 * n] = from_f32<TIn>(dbp0[i].re); o[2 * n + 1] = from_f32<TIn>(dbp0[i].im);
-      }
-    }
-  }
-}
-
-// One CTA per (batch, head): S_t = S_T + sum_{s >= t} sterm_s ; dM_t = S_t / conj(m_t).
-__global__ void __launch_bounds__(256) bwd_dm_scan_kernel(const float* __restrict__ sterm,
-                                                          const float* __restrict__ sT,
-                                                          const float* __restrict__ M,
-                                                          float* __restrict__ dM, int T) {
-  __shared__ double s_wr[8], s_wi[8];
-  __shared__ double s_carry[2];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+// One CTA per (batch, head): S_t = S_T + sum_{s >= t} (sterm_s - conj(h_s) dh_s), dM_t = (S_t - conj(kp_t) dkp_t) / conj(m_t).
+// 1024 tokens at a time: the turns are serial (256 at a time took 20 us over 4096 tokens).
+__device__ void finish_dm(const FinishParams& p) {
+  __shared__ double s_wr[FINISH / 32], s_wi[FINISH / 32];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, T = p.T;
   const size_t bh = blockIdx.x;
-  const float* st = sterm + bh * T * 2;
-  const float* Mb = M + bh * T * 2;
-  float* dMb = dM + bh * T * 2;
-  if (tid == 0) { s_carry[0] = sT[bh * 2]; s_carry[1] = sT[bh * 2 + 1]; }
-  __syncthreads();
-  for (int hi = T; hi > 0; hi -= 256) {
+  const float *st = p.sterm + bh * T * 2, *M = p.M + bh * T * 2, *K = p.K + bh * T * 4, *dK = p.dK + bh * T * 4;
+  float* dM = p.dM + bh * T * 2;
+  double carry_r = p.sT[bh * 2], carry_i = p.sT[bh * 2 + 1];
+  for (int hi = T; hi > 0; hi -= FINISH) {
     const int t = hi - 1 - tid;  // thread 0 owns the latest token of the tile
     double vr = 0.0, vi = 0.0;
-    if (t >= 0) { vr = st[2 * t]; vi = st[2 * t + 1]; }
+    cf m = {0.f, 0.f}, kd = {0.f, 0.f};
+    if (t >= 0) {
+      cf mn = {1.f, 0.f}, kpn = {0.f, 0.f}, dh;
+      m = load_cf(M + 2 * (size_t)t);
+      kd = cmul_conj_a(load_cf(K + 4 * (size_t)t), {dK[4 * (size_t)t], dK[4 * (size_t)t + 1]});   // conj(kp) dkp
+      const cf kc = load_cf(K + 4 * (size_t)t + 2);
+      if (t + 1 < T) {
+        mn = load_cf(M + 2 * (size_t)t + 2); kpn = load_cf(K + 4 * (size_t)t + 4);
+        dh = {dK[4 * (size_t)t + 4], dK[4 * (size_t)t + 5]};
+      } else {
+        dh = {dM[2 * (size_t)t], dM[2 * (size_t)t + 1]};   // (left there by the sweep: the last token has no next one)
+      }
+      const cf r = cmul_conj_a(cadd(cmul(mn, kc), kpn), dh);
+      vr = (double)st[2 * t] - r.re; vi = (double)st[2 * t + 1] - r.im;
+    }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const double ar = __shfl_up_sync(0xffffffffu, vr, o), ai = __shfl_up_sync(0xffffffffu, vi, o);
@@ -722,65 +1193,88 @@ __global__ void __launch_bounds__(256) bwd_dm_scan_kernel(const float* __restric
     }
     if (lane == 31) { s_wr[w] = vr; s_wi[w] = vi; }
     __syncthreads();
-    double offr = s_carry[0], offi = s_carry[1];
-    for (int k = 0; k < w; ++k) { offr += s_wr[k]; offi += s_wi[k]; }
-    vr += offr; vi += offi;
+    vr += carry_r; vi += carry_i;
+    for (int k = 0; k < FINISH / 32; ++k) {
+      if (k < w) { vr += s_wr[k]; vi += s_wi[k]; }
+      carry_r += s_wr[k]; carry_i += s_wi[k];
+    }
     if (t >= 0) {
-      const float mr = Mb[2 * t], mi = Mb[2 * t + 1];
-      const float den = mr * mr + mi * mi;
+      const float den = m.re * m.re + m.im * m.im;
       // S / conj(m) = S * m / |m|^2
       float outr = 0.f, outi = 0.f;
       if (den > 0.f) {
-        outr = (float)((vr * mr - vi * mi) / den);
-        outi = (float)((vr * mi + vi * mr) / den);
+        const double sr = vr - kd.re, si = vi - kd.im, inv = 1.0 / (double)den;
+        outr = (float)((sr * m.re - si * m.im) * inv);
+        outi = (float)((sr * m.im + si * m.re) * inv);
       }
-      dMb[2 * t] = outr; dMb[2 * t + 1] = outi;
+      dM[2 * t] = outr; dM[2 * t + 1] = outi;
     }
-    __syncthreads();
-    if (tid == 255) { s_carry[0] = vr; s_carry[1] = vi; }
     __syncthreads();
   }
 }
+// a thread per complex column of a row of dB / dC
+template <typename TIn>
+__device__ __forceinline__ void finish_columns(const FinishParams& p, unsigned block) {
+  const int hpg = p.heads / p.groups, N = p.N, D = 2 * N;
+  const size_t i = (size_t)block * FINISH + threadIdx.x, rows = (size_t)(p.BH / p.heads) * p.groups * p.T;
+  if (i >= rows * N) return;
+  const size_t row = i / N, n = i % N, bg = row / p.T, t = row % p.T;
+  const size_t bh0 = bg / p.groups * p.heads + bg % p.groups * hpg;
+  auto sum_heads = [&](const float* src, size_t stride, void* out, size_t at) {
+    cf v = {0.f, 0.f};
+    for (int h = 0; h < hpg; ++h) v = cadd(v, {src[h * stride], src[h * stride + 1]});
+    TIn* dst = reinterpret_cast<TIn*>(out) + at;
+    dst[0] = from_f32<TIn>(v.re); dst[1] = from_f32<TIn>(v.im);
+  };
+  sum_heads(p.dB_head + (bh0 * p.T + t) * D + 2 * n, (size_t)p.T * D, p.dB, row * D + 2 * n);
+  sum_heads(p.dC_head + (bh0 * p.T + t) * D + 2 * n, (size_t)p.T * D, p.dC, row * D + 2 * n);
+  if (t == 0 && p.dBprev) sum_heads(p.dBprev_head + bh0 * D + 2 * n, D, p.dBprev, bg * D + 2 * n);
+}
+template <typename TIn>
+__global__ void __launch_bounds__(FINISH) bwd_finish_kernel(FinishParams p) {
+  if (blockIdx.x < (unsigned)p.BH) finish_dm(p);
+  else finish_columns<TIn>(p, blockIdx.x - p.BH);
+}
 
-constexpr size_t SIMT_SMEM_MAX = 200 * 1024;
 struct SimtConfig {
-  int NC, NS, PW, ptiles, TB, threads, nseg, seg_len;
-  size_t smem_fwd, smem_rev;
+  int W, ptiles, nseg, seg_len;
 };
 
-// Segments of T.  Per token a CTA takes as long alone on its SM as with others up to 8 warps; a split adds a pre-pass (half
-// the work of a sweep), its launch (worth about 30 tokens) and a fold of one per segment passed.  Sequences up to 64 tokens stay whole.
+template <typename TIn, typename TY>
+size_t smem_of(int W, Mode mode) { return (size_t)Layout(W, sizeof(TIn), sizeof(TY), Parts<TIn>::N, Parts<TY>::N, mode).bytes; }
+
+// Segments of T.  The model counts the time of the most loaded SM in chunks of a full one: it holds ``fit`` CTAs at a time
+// (168 registers a thread and shared memory) and is slowed by latency when it holds fewer; measured per chunk of the forward
+// sweep with N = 48: 4.6, 5.9, 7.3 and 8.2 us for 1 to 4 CTAs.  A split adds a pre-pass (0.37 of a chunk per chunk), two launches
+// (1 chunk) and the combination's traffic.  Sequences up to 64 tokens stay whole.  Forward + backward by segments, us:
+// (16, 4, 2048, N 48 fp16) 1: 1650, 4: 831, 9: 647, 16: 669, 32: 698; (16, 32, 1024, N 32 bf16) 1: 1301, 4: 1359, 16: 1509;
+// (2, 4, 256, N 32 fp32) 1: 242, 4: 98, 16: 48.
 void plan_segments(const ScanDims& d, SimtConfig& c) {
   c.nseg = 1; c.seg_len = d.T;
   if (d.T <= 64) return;
-  const double ctas = (double)d.batch * d.heads * c.ptiles, slots = 148.0 * std::max(1, 256 / c.threads);
-  double best = d.T * std::max(1.0, ctas / slots);
-  for (int n = 2; n <= 64; ++n) {
-    const int len = ((d.T + n - 1) / n + c.TB - 1) / c.TB * c.TB, segs = (d.T + len - 1) / len;
+  const int fit = c.W == 1 ? 5 : c.W <= 3 ? 4 : c.W == 4 ? 2 : 1;
+  const long long ctas = (long long)d.batch * d.heads * c.ptiles;
+  auto load = [&](long long n) {
+    const long long q = (n + 147) / 148;
+    return (double)(q / fit) + (q % fit ? 0.42 + 0.58 * (double)(q % fit) / fit : 0.0);
+  };
+  double best = (d.T + L - 1) / L * load(ctas);
+  for (int n = 2, last = 0; n <= 64 && last != 1; ++n) {
+    const int chunks = ((d.T + n - 1) / n + L - 1) / L, len = chunks * L, segs = (d.T + len - 1) / len;
     if (segs < 2) break;
-    const double cost = 1.5 * len * std::max(1.0, ctas * segs / slots) + 30 + segs;
-    if (cost < 0.9 * best || (cost < best && c.nseg > 1)) { best = cost; c.nseg = segs; c.seg_len = len; }
+    if (chunks == last) continue;
+    last = chunks;
+    const double cost = chunks * (load(ctas * segs) + 0.37 * load(ctas * (segs - 1))) + 1.0 + 3e-4 * (double)(ctas * segs * c.W);
+    if (cost < 0.97 * best) { best = cost; c.nseg = segs; c.seg_len = len; }
   }
 }
 
 bool make_config(const ScanDims& d, SimtConfig& c) {
   if (d.N < 1 || d.N > 128 || d.P < 1) return false;
-  c.NC = d.N <= 32 ? 2 : 4;
-  c.NS = (d.N + 4 * c.NC - 1) / (4 * c.NC);
-  c.PW = d.P > 32 ? 2 : 1;
-  const int PT = 32 * c.PW;
-  c.ptiles = (d.P + PT - 1) / PT;
-  c.threads = 32 * c.NS * c.PW;
-  const int D2 = 2 * c.NS * 4 * c.NC;
-  for (c.TB = 16; c.TB >= 4; c.TB /= 2) {
-    const size_t TB = c.TB;
-    const size_t part_fwd = TB * (size_t)std::max(c.NS * PT, c.PW * D2);
-    c.smem_fwd = 4 * (3 * TB * D2 + (TB + 1) * PT + 2 * TB + TB * PT + part_fwd);
-    c.smem_rev = 4 * (3 * TB * D2 + (TB + 1) * PT + 2 * TB + TB * PT + 2 * TB * c.PW * D2 +
-                      2 * TB * c.NS * PT + 2 * PT);
-    if (c.smem_rev <= SIMT_SMEM_MAX) { plan_segments(d, c); return true; }
-  }
-  return false;
+  c.W = (d.N + 15) / 16;
+  c.ptiles = (d.P + ROWS - 1) / ROWS;
+  plan_segments(d, c);
+  return true;
 }
 
 SweepParams base_params(const void* U, const float* M, const float* K, const void* B,
@@ -789,7 +1283,7 @@ SweepParams base_params(const void* U, const float* M, const float* K, const voi
   SweepParams p{};
   p.U = U; p.B = B; p.C = C; p.Bprev = Bprev; p.Uprev = Uprev; p.M = M; p.K = K; p.z0 = z0;
   p.batch = d.batch; p.heads = d.heads; p.groups = d.groups; p.T = d.T; p.P = d.P; p.N = d.N;
-  p.NS = c.NS; p.PW = c.PW; p.TB = c.TB; p.ptiles = c.ptiles; p.nseg = c.nseg; p.seg_len = c.seg_len;
+  p.W = c.W; p.ptiles = c.ptiles; p.nseg = c.nseg; p.seg_len = c.seg_len;
   return p;
 }
 
@@ -804,20 +1298,23 @@ void segment_scratch(const ScanDims& d, const SimtConfig& c, float* at, float** 
   *prod = at + (size_t)c.nseg * d.batch * d.heads * d.P * 2 * d.N;
 }
 
-template <typename TIn, typename TY, int NC>
+constexpr size_t SIMT_SMEM_MAX = 200 * 1024;
+static_assert(Layout(8, 4, 4, 3, 3, SWEEP_B).bytes <= (int)SIMT_SMEM_MAX, "the widest state fits");
+
+template <typename TIn, typename TY>
 int launch_sweeps(const SweepParams& p, const SimtConfig& c, bool bwd, cudaStream_t st) {
-  auto pre = segment_kernel<TIn, TY, NC>;
-  auto k = bwd ? sweep_bwd_kernel<TIn, TY, NC> : sweep_fwd_kernel<TIn, TY, NC>;
-  const size_t smem = bwd ? c.smem_rev : c.smem_fwd;
+  auto pre = segment_kernel<TIn, TY>;
+  auto k = bwd ? sweep_bwd_kernel<TIn, TY> : sweep_fwd_kernel<TIn, TY>;
   static std::atomic<unsigned long long> done[3];
   if (int e = ensure_smem(k, SIMT_SMEM_MAX, done[bwd])) return e;
   if (int e = c.nseg > 1 ? ensure_smem(pre, SIMT_SMEM_MAX, done[2]) : SL_OK) return e;
   const unsigned dirs = bwd ? 2 : 1;
   if (c.nseg > 1) {
-    pre<<<dim3(p.heads, p.batch, dirs * (c.nseg - 1) * c.ptiles), c.threads, c.smem_fwd, st>>>(p);
-    note_launches(1);
+    pre<<<dim3(p.heads, p.batch, dirs * (c.nseg - 1) * c.ptiles), 32 * c.W, std::max(smem_of<TIn, TY>(c.W, STATES), smem_of<TIn, TY>(c.W, ADJ_STATES)), st>>>(p);
+    combine_kernel<TIn><<<dim3((unsigned)p.batch * p.heads, (unsigned)(p.P * p.N + 255) / 256, dirs), 256, 0, st>>>(p);
+    note_launches(2);
   }
-  k<<<dim3(p.heads, p.batch, dirs * c.nseg * c.ptiles), c.threads, smem, st>>>(p);
+  k<<<dim3(p.heads, p.batch, dirs * c.nseg * c.ptiles), 32 * c.W, bwd ? smem_of<TIn, TY>(c.W, SWEEP_B) : smem_of<TIn, TY>(c.W, FORWARD), st>>>(p);
   note_launches(1);
   return launch_status();
 }
@@ -845,14 +1342,12 @@ int scan_simt_fwd(const void* U, const float* M, const float* K, const void* B, 
   p.Y = Y; p.zfinal = zfinal;
   segment_scratch(d, c, reinterpret_cast<float*>(ws), &p.zloc, &p.zprod);
   int rc = SL_ERR_UNSUPPORTED;
-  SL_DISPATCH_DTYPE(io_dtype, TIn, SL_DISPATCH_DTYPE(y_dtype, TY, {
-    rc = c.NC == 2 ? launch_sweeps<TIn, TY, 2>(p, c, false, st) : launch_sweeps<TIn, TY, 4>(p, c, false, st);
-  }));
+  SL_DISPATCH_DTYPE(io_dtype, TIn, SL_DISPATCH_DTYPE(y_dtype, TY, { rc = launch_sweeps<TIn, TY>(p, c, false, st); }));
   return rc;
 }
 
-// workspace layout: dc_head | dbc_head | dbp_head (each batch*heads*T*2N floats) |
-//                   sterm (batch*heads*T*2) | sT (batch*heads*2) | the segments of the two sweeps
+// workspace layout: sterm (batch*heads*T*2) | sT (batch*heads*2) | where heads or slices of P are summed by the last launch:
+//                   dB | dC (each batch*heads*T*2N floats) | dB_prev (batch*heads*2N) | the segments of the two sweeps
 size_t scan_simt_bwd_workspace(const ScanDims& d) {
   const size_t bht = (size_t)d.batch * d.heads * d.T;
   return round_up(4 * (3 * bht * 2 * d.N + bht * 2 + (size_t)d.batch * d.heads * 2), 256);
@@ -873,35 +1368,33 @@ int scan_simt_bwd(const void* U, const float* M, const float* K, const void* B, 
   const size_t need = scan_simt_bwd_workspace(d);
   if (!ws || ws_bytes < need) return SL_ERR_WORKSPACE_TOO_SMALL;
   if (ws_bytes < need + 8 * segment_floats(d, c) || !aligned(ws, 16)) { c.nseg = 1; c.seg_len = d.T; }
-  const size_t bht = (size_t)d.batch * d.heads * d.T, D = 2 * (size_t)d.N;
-  float* dc_head = reinterpret_cast<float*>(ws);
-  float* dbc_head = dc_head + bht * D;
-  float* dbp_head = dbc_head + bht * D;
-  float* sterm = dbp_head + bht * D;
-  float* sT = sterm + bht * 2;
-  if (c.ptiles > 1) {  // partial sums of the P tiles are accumulated atomically
-    if (cudaMemsetAsync(ws, 0, need, st) != cudaSuccess) return SL_ERR_LAUNCH_FAILED;
-  }
+  const size_t bh = (size_t)d.batch * d.heads, bht = bh * d.T, D = 2 * (size_t)d.N;
   SweepParams p = base_params(U, M, K, B, C, z0, Bprev, Uprev, d, c);
-  p.dY = dY; p.dfinal = dfinal; p.dc_head = dc_head; p.dbc_head = dbc_head;
-  p.dbp_head = dbp_head; p.sT = sT; p.dU = dU; p.dUprev = dUprev; p.dinit = dinit;
+  p.dY = dY; p.dfinal = dfinal;
+  p.sterm = reinterpret_cast<float*>(ws);
+  p.sT = p.sterm + bht * 2;
+  p.dB_head = p.sT + bh * 2; p.dC_head = p.dB_head + bht * D; p.dBprev_head = p.dC_head + bht * D;
+  p.spread = d.groups != d.heads || c.ptiles > 1;
+  p.dU = dU; p.dB = dB; p.dC = dC; p.dK = dK; p.dM = dM; p.dUprev = dUprev; p.dBprev = dBprev; p.dinit = dinit;
+  if (c.ptiles > 1) {  // partial sums of the P tiles are accumulated atomically
+    if (cudaMemsetAsync(ws, 0, need, st) != cudaSuccess || cudaMemsetAsync(dK, 0, bht * 16, st) != cudaSuccess ||
+        cudaMemsetAsync(dM, 0, bht * 8, st) != cudaSuccess)
+      return SL_ERR_LAUNCH_FAILED;
+  }
   float* segments = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws) + need);
   segment_scratch(d, c, segments, &p.zloc, &p.zprod);
   segment_scratch(d, c, segments + segment_floats(d, c), &p.gloc, &p.gprod);
   int rc = SL_ERR_UNSUPPORTED;
-  SL_DISPATCH_DTYPE(io_dtype, TIn, SL_DISPATCH_DTYPE(dy_dtype, TY, {
-    rc = c.NC == 2 ? launch_sweeps<TIn, TY, 2>(p, c, true, st) : launch_sweeps<TIn, TY, 4>(p, c, true, st);
-  }));
+  SL_DISPATCH_DTYPE(io_dtype, TIn, SL_DISPATCH_DTYPE(dy_dtype, TY, { rc = launch_sweeps<TIn, TY>(p, c, true, st); }));
   if (rc != SL_OK) return rc;
   FinishParams f{};
-  f.B = B; f.C = C; f.Bprev = Bprev; f.K = K; f.dc_head = dc_head; f.dbc_head = dbc_head;
-  f.dbp_head = dbp_head; f.dK = dK; f.sterm = sterm; f.dB = dB; f.dC = dC; f.dBprev = dBprev;
-  f.batch = d.batch; f.heads = d.heads; f.groups = d.groups; f.T = d.T; f.N = d.N;
-  const long long rows = (long long)d.batch * d.groups * d.T;
-  const unsigned blocks = (unsigned)((rows + 7) / 8);
-  SL_DISPATCH_DTYPE(io_dtype, TIn, { bwd_finish_kernel<TIn><<<blocks, 256, 0, st>>>(f); });
-  bwd_dm_scan_kernel<<<d.batch * d.heads, 256, 0, st>>>(sterm, sT, M, dM, d.T);
-  note_launches(2);
+  f.M = M; f.K = K; f.dK = dK; f.sterm = p.sterm; f.sT = p.sT; f.dB_head = p.dB_head; f.dC_head = p.dC_head;
+  f.dBprev_head = p.dBprev_head; f.dM = dM; f.dB = dB; f.dC = dC; f.dBprev = Bprev ? dBprev : nullptr;
+  f.BH = (int)bh; f.heads = d.heads; f.groups = d.groups; f.T = d.T; f.N = d.N;
+  const size_t columns = p.spread ? (size_t)d.batch * d.groups * d.T * d.N : 0;
+  const unsigned blocks = (unsigned)(bh + (columns + FINISH - 1) / FINISH);
+  SL_DISPATCH_DTYPE(io_dtype, TIn, { bwd_finish_kernel<TIn><<<blocks, FINISH, 0, st>>>(f); });
+  note_launches(1);
   return launch_status();
 }
 

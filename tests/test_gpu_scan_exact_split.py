@@ -66,3 +66,32 @@ def test_16_bit_operands_of_other_widths_keep_float32_precision(N, groups, T, dt
             assert grad.dtype == torch.float32 and rel(grad, want[name]) <= 1e-5, (name, rel(grad, want[name]))
         else:
             assert grad.dtype == dtype and rel(grad, want[name]) <= unit + 1e-5, (name, rel(grad, want[name]))
+
+
+# Edges of the chunks of 16 tokens, of the warps of 16 columns, of the slices of 64 rows and of the 16-byte pieces in which
+# rows are staged, each operand type beside each type of dY (the products are of one, two or three bfloat16 parts of it).
+# Operands are exact in every case, and sums of 24-bit products err by 2^-24 of their terms: the float32 bar holds.
+@pytest.mark.parametrize("dtype, dy_dtype", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16),
+                                             (torch.bfloat16, torch.float32), (torch.float16, torch.bfloat16),
+                                             (torch.float16, torch.float16), (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("b, h, g, T, P, N", [(1, 2, 1, 1, 64, 16), (2, 1, 1, 15, 1, 17), (1, 2, 2, 16, 63, 15),
+                                              (1, 1, 1, 17, 65, 48), (1, 3, 1, 33, 130, 31), (1, 2, 2, 97, 64, 128),
+                                              (1, 1, 1, 1500, 9, 1), (1, 1, 1, 1041, 64, 65)])
+def test_chunks_of_bfloat16_parts_at_their_edges(b, h, g, T, P, N, dtype, dy_dtype):
+    case = make_scan_case(b, h, T, P, N, groups=g, dtype=dtype, seed=T + 3 * N, streaming=True, with_init=True)
+    gen = torch.Generator().manual_seed(T)
+    dY = torch.randn(b, h, T, P, generator=gen).to(dy_dtype)
+    d_final = torch.randn(b, h, P, 2 * N, generator=gen)
+    c = case.to("cuda")
+    ops = (c.U, c.M, c.K, c.B, c.C, c.initial_states.float(), c.B_prev, c.U_prev)
+    Y, fin = _C.scan_fwd(*ops, chunk_size=64, y_dtype=torch.float32, want_final=True, path="simt")
+    got = _C.scan_bwd(*ops, dY.cuda(), d_final.cuda(), chunk_size=64, path="simt")
+    args = [n64(t) for t in case.tensors()]
+    kw = dict(initial_states=n64(case.initial_states), B_prev=n64(case.B_prev), U_prev=n64(case.U_prev))
+    wY, wfin, _, _ = scan_np.v2x2ssm(*args, **kw)
+    assert rel(Y, wY) <= 1e-5 and rel(fin, wfin) <= 1e-5
+    want = scan_np.v2x2ssd_bwd(*args, n64(dY), d_final_state=n64(d_final), **kw)
+    unit = {torch.float32: 0.0, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]   # one rounding of the result
+    for name, grad in zip(NAMES, got):
+        bar = 1e-5 + (unit if grad.dtype == dtype else 0.0)
+        assert rel(grad, want[name]) <= bar, (name, rel(grad, want[name]))
