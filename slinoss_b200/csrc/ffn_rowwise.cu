@@ -3,17 +3,44 @@
 // is kept), as the reference does: block_ffn_residual, slinoss/ops/block/training.py:193-354, with the
 // kernels of slinoss/ops/block/cute/norm.py:85,173 and activation.py:78,153.  The two GEMMs stay library
 // calls in the caller.  All four kernels are HBM-bound: 16-byte accesses, one pass over their rows.
+#include <type_traits>
+
 #include "common.cuh"
 #include "host_abi.h"
 
 namespace sl {
 namespace {
 
+// a + b, added in float32 and rounded once, without the saturation of from_f32: bit for bit torch's sum of two such tensors
+template <typename T>
+__device__ __forceinline__ uint4 plain_sum(const uint4& a, const uint4& b) {
+  float x[Vec16<T>::N], y[Vec16<T>::N];
+  unpack16<T>(a, x); unpack16<T>(b, y);
+#pragma unroll
+  for (int k = 0; k < Vec16<T>::N; ++k) x[k] += y[k];
+  if constexpr (std::is_same<T, __half>::value) {
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const __half2 h = __floats2half2_rn(x[2 * k], x[2 * k + 1]);
+      w[k] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+  } else {
+    uint4 r;
+    store16<T>(reinterpret_cast<T*>(&r), x);
+    return r;
+  }
+}
+
 // out = x * rsqrt(mean(x^2) + eps) * w.  One warp per row; the row stays packed in registers (16-byte
 // pieces, MAXP per lane), so it is read once.
+// add: x is first replaced by x + add rounded to its type (the sum of two tensors as torch forms it: a token's residual),
+// which is kept in sum; without out that is all.
 template <typename T, int MAXP>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w,
-                                                          T* __restrict__ out, long long rows, int C, float eps) {
+                                                          T* __restrict__ out, long long rows, int C, float eps,
+                                                          const T* __restrict__ add, T* __restrict__ sum) {
   constexpr int V = Vec16<T>::N;
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -26,6 +53,17 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ 
   for (int i = 0; i < MAXP; ++i) {
     const int pc = lane + 32 * i;
     if (pc < pieces) raw[i] = xr[pc];
+  }
+  if (add) {
+#pragma unroll
+    for (int i = 0; i < MAXP; ++i) {
+      const int pc = lane + 32 * i;
+      if (pc < pieces) {
+        raw[i] = plain_sum<T>(raw[i], reinterpret_cast<const uint4*>(add + row * C)[pc]);
+        reinterpret_cast<uint4*>(sum + row * C)[pc] = raw[i];
+      }
+    }
+    if (!out) return;
   }
 #pragma unroll
   for (int i = 0; i < MAXP; ++i) {
@@ -329,21 +367,26 @@ extern "C" int sl_rmsnorm_fwd(const void* x, const void* weight, float eps, void
                               int io_dtype, void* stream) {
   using namespace sl;
   if (!x || !weight || !out) return SL_ERR_NULL_POINTER;
+  return rmsnorm_fwd_sum(x, nullptr, nullptr, weight, eps, out, rows, C, io_dtype, reinterpret_cast<cudaStream_t>(stream));
+}
+
+namespace sl {
+// sum = x + add (both null: x itself), out = norm(sum) * weight or null
+int rmsnorm_fwd_sum(const void* x, const void* add, void* sum, const void* weight, float eps, void* out, long long rows, int C,
+                    int io_dtype, cudaStream_t st) {
+  if (!x || (!add) != (!sum) || (!out && !add) || (out && !weight)) return SL_ERR_NULL_POINTER;
   if (!dtype_ok(io_dtype)) return SL_ERR_UNSUPPORTED;
-  if (!rows_ok(rows, C, io_dtype, x, out) || !aligned(weight, 16)) return SL_ERR_BAD_SHAPE;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (!rows_ok(rows, C, io_dtype, x, out) || !aligned(weight, 16) || !aligned(add, 16) || !aligned(sum, 16)) return SL_ERR_BAD_SHAPE;
   const unsigned grid = (unsigned)((rows + 7) / 8);
   const bool narrow = C / (io_dtype == SL_F32 ? 4 : 8) <= 32 * RMS_MAXP_NARROW;
   SL_DISPATCH_DTYPE(io_dtype, T, {
     auto kern = narrow ? rmsnorm_fwd_kernel<T, RMS_MAXP_NARROW> : rmsnorm_fwd_kernel<T, RMS_MAXP>;
     kern<<<grid, 256, 0, st>>>(reinterpret_cast<const T*>(x), reinterpret_cast<const T*>(weight),
-                               reinterpret_cast<T*>(out), rows, C, eps);
+                               reinterpret_cast<T*>(out), rows, C, eps, reinterpret_cast<const T*>(add), reinterpret_cast<T*>(sum));
   });
   note_launches(1);
   return launch_status();
 }
-
-namespace sl {
 // d_weight: float32 accumulators, or float64 ones (weight64); extra (or null) is added to d_x, its column sums to extra_sum
 // (or null; up to 1024 columns, where the second row of sums per warp still leaves three CTAs per SM)
 bool rmsnorm_bwd_sums_extra(int C) { return C <= 1024; }

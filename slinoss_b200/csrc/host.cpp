@@ -5,6 +5,9 @@
 // and scratch with torch, launches on torch's current stream and turns status codes into exceptions.
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/ops/as_strided_native.h>
+#include <ATen/ops/mm_cuda_dispatch.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
@@ -490,26 +493,62 @@ class TokenPlan {
       check(sl::skinny_linear(o, st), "skinny_linear");
       return py::make_tuple(out, b_next, ws);
     }
-    // A block: the library's products at the shapes and in the order of the composed path.  Any other order of their sums moves
-    // last bits, which residual stream, norms and B/C phases carry on from block to block: six blocks of width 1024 end up 1.6 % from
-    // the composed token (the small-batch kernel, or one product for the three parts of in_proj).
+    // A block: the bits of the library's products at the shapes of the composed path.  Any other order of their sums moves last
+    // bits, which residual stream, norms and B/C phases carry on from block to block: six blocks of width 1024 end up 1.6 % from the
+    // composed token.  token_linear adds in the library's order, with residual and activation inside; what it does not take (more than
+    // 64 rows, widths that are no multiple of 8) goes to the library, there without a dispatch.  A token of four blocks of width 512
+    // at batch 8 is bound by the host: 398 us with 24 library products and 29 other launches, 184 with 8 launches a block (172 of them on the device).
     at::AutoDispatchBelowAutograd below;
-    const Tensor rows = x.contiguous(), normed = rmsnorm_fwd(rows, *b_[0], (float)eps_[0]);
+    auto fresh = [&](int64_t cols) { return at::detail::empty_cuda({M, cols}, type, x.device(), c10::nullopt); };
+    auto norm = [&](const Tensor& a, const Tensor& w, double eps) {
+      Tensor out = fresh(D);
+      check(sl_rmsnorm_fwd(ptr(a), ptr(w), (float)eps, mptr(out), M, D, io, st), "sl_rmsnorm_fwd");
+      return out;
+    };
+    const Tensor rows = x.contiguous(), normed = norm(rows, *b_[0], eps_[0]);
     auto product = [](const Tensor& a, const Tensor& W, int64_t row, int64_t n) {   // a (rows row .. row + n of W)^T
-      return at::mm(a, W.as_strided({W.size(1), n}, {1, W.size(1)}, W.storage_offset() + row * W.size(1)));
+      return at::cuda::mm(a, at::native::as_strided_tensorimpl(W, {W.size(1), n}, {1, W.size(1)}, W.storage_offset() + row * W.size(1)));
+    };
+    // own kernel with what follows the product inside; false where it is left to the library
+    auto fused = [&](const Tensor& a, const Tensor& W, int64_t row, int64_t n, const OptT& bias, std::initializer_list<const Tensor*> out,
+                     const Tensor* residual = nullptr, int act = -1) {
+      sl::TokenLinearArgs t{ptr(a), static_cast<const uint8_t*>(W.data_ptr()) + row * W.size(1) * 2, ptr(bias), {}, {},
+                            residual ? ptr(*residual) : nullptr, (int)M, (int)W.size(1), (int)n, io, act == 0, act == 1};
+      int i = 0;
+      for (const Tensor* o : out) { t.out[i] = mptr(*o); t.width[i++] = (int)o->size(1); }
+      if (!sl::token_linear_supported(t)) return false;
+      check(sl::token_linear(t, st), "token_linear");
+      return true;
     };
     auto linear = [&](const Tensor& a, const Tensor& W, const OptT& bias) {
       return bias ? at::linear(a, W, bias) : product(a, W, 0, W.size(0));
     };
-    const Tensor gv = product(normed, *p_[0], 0, 2 * C), params = product(normed, *p_[0], 2 * C, 3 * heads_),
-                 bc = product(normed, *p_[0], 2 * C + 3 * heads_, 4 * groups_ * N_);
-    mixer_step(gv.data_ptr(), column(gv, C), params.data_ptr(), bc.data_ptr(), 2 * C, 3 * heads_, 4 * groups_ * N_, false);
-    const Tensor hid = call.empty({M, C}, type);
+    // residual + linear
+    auto onto = [&](const Tensor& residual, const Tensor& a, const Tensor& W, const OptT& bias) {
+      Tensor out = fresh(D);
+      if (fused(a, W, 0, D, bias, {&out}, &residual)) return out;
+      const Tensor branch = linear(a, W, bias);
+      check(sl::rmsnorm_fwd_sum(ptr(residual), ptr(branch), mptr(out), nullptr, 0.f, nullptr, M, D, io, st), "sl_rmsnorm_fwd");
+      return out;
+    };
+    const int64_t n_gv = 2 * C, n_par = 3 * heads_, n_bc = 4 * groups_ * N_;
+    Tensor gv = fresh(n_gv), params = fresh(n_par), bc = fresh(n_bc);
+    if (!fused(normed, *p_[0], 0, O, {}, {&gv, &params, &bc})) {
+      if (!fused(normed, *p_[0], 0, n_gv, {}, {&gv})) gv = product(normed, *p_[0], 0, n_gv);
+      if (!fused(normed, *p_[0], n_gv, n_par, {}, {&params})) params = product(normed, *p_[0], n_gv, n_par);
+      if (!fused(normed, *p_[0], n_gv + n_par, n_bc, {}, {&bc})) bc = product(normed, *p_[0], n_gv + n_par, n_bc);
+    }
+    mixer_step(gv.data_ptr(), column(gv, C), params.data_ptr(), bc.data_ptr(), n_gv, n_par, n_bc, false);
+    const Tensor hid = fresh(C);
     check(sl::mixer_step_norm(base, ptr(p_[9]), (float)eps_[1], mptr(hid), M, heads_, P_, io, st), "mixer_step");
-    Tensor out = rows + linear(hid, *p_[10], p_[11]);
+    Tensor out = onto(rows, hid, *p_[10], p_[11]);
     if (ffn) {
-      const Tensor wide = linear(rmsnorm_fwd(out, *b_[1], (float)eps_[2]), *b_[2], b_[3]);
-      out = out + linear(ffn_act_fwd(wide, ffn_kind_), *b_[4], b_[5]);
+      const Tensor in = norm(out, *b_[1], eps_[2]), act = fresh(b_[4]->size(1));
+      if (!fused(in, *b_[2], 0, b_[2]->size(0), b_[3], {&act}, nullptr, ffn_kind_)) {
+        const Tensor wide = linear(in, *b_[2], b_[3]);
+        check(sl_ffn_activation_fwd(ptr(wide), mptr(act), M, act.size(1), ffn_kind_, io, st), "sl_ffn_activation_fwd");
+      }
+      out = onto(out, act, *b_[4], b_[5]);
     }
     return py::make_tuple(out, b_next, ws);
   }

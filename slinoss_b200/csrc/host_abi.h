@@ -54,6 +54,19 @@ struct SkinnyArgs {
 SL_API bool skinny_supported(int M, int K, int O, int io_dtype);
 SL_API int skinny_linear(const SkinnyArgs& a, cudaStream_t st);
 
+// One linear layer of a block's token, with the bits of the library's product and of what follows it (token_linear.cu):
+// x (M, K) dense, weight (O, K) dense, M <= 64.
+struct TokenLinearArgs {
+  const void *x, *weight, *bias;   // bias (O) or null
+  void* out[3];                    // dense (M, width[i]) each, the columns in turn; swiglu: one of O / 2
+  int width[3];
+  const void* residual;            // (M, O) or null: added to the rounded product
+  int M, K, O, io_dtype;
+  bool gelu, swiglu;               // activation of the rounded product; swiglu: value rows, then gate rows
+};
+SL_API bool token_linear_supported(const TokenLinearArgs& a);
+SL_API int token_linear(const TokenLinearArgs& a, cudaStream_t st);
+
 // ---- scan preparation and mixer tail on strided rows ---------------------------------------------------------------------
 // Operands and results are rows of (batch * T) with a row stride each (columns of the in_proj output and of its
 // gradient); a null pointer skips its part, as in sl_scanprep_conv_fwd / _bwd.
@@ -92,6 +105,8 @@ SL_API int mixer_tail_bwd(const void* Y, const void* gate, int64_t gate_stride, 
 // d_weight float32 or weight64 (sums that rounding to a shorter type makes independent of their order): added to; extra
 // (rows, C) or null is added to d_x, and its column sums to extra_sum (or null) where rmsnorm_bwd_sums_extra
 SL_API bool rmsnorm_bwd_sums_extra(int C);
+SL_API int rmsnorm_fwd_sum(const void* x, const void* add, void* sum, const void* weight, float eps, void* out, long long rows, int C,
+                           int io_dtype, cudaStream_t st);
 SL_API int rmsnorm_bwd(const void* x, const void* weight, float eps, const void* d_out, const void* extra, void* d_x, float* d_weight,
                        double* weight64, double* extra_sum, long long rows, int C, int io_dtype, cudaStream_t st);
 // sl_ffn_activation_bwd that also adds the column sums of its result to sums (one or two times H)

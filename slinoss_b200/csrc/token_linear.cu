@@ -1,0 +1,213 @@
+// The linear layers of a block's decode token: y = act(x W^T + bias) or residual + x W^T + bias, M <= 64 rows of 16-bit values,
+// with the very bits of the library's product and of the row kernels behind it.
+//
+// A block's token has to keep the bits of the composed path (any other order of sums grows from block to block).  For outputs
+// of a multiple of 8 columns the library adds the products of 16 values of k at a time, in turn, on one float32 accumulator,
+// whatever its tile (560 shapes of 1 to 64 rows, k from 64 to 4096, either type, with and without bias; widths that are no
+// multiple of 8 take others and stay with it).  So does a warp here, with mma.sync m16n8k16; the order inside a step of 16
+// does not matter, which lets a lane read 8 consecutive bytes of a row for its four values.
+//
+// What bounds it: the launch.  A library product costs the host 7 to 9 us and a launch of its own for each part of in_proj, the
+// residual and the activation; here it is 2 to 3 us with all of them inside.  On the device: latency of one trip to memory
+// (all of a warp's rows of W are requested at the start, x two pieces ahead) and the chain of K / 16 steps on one accumulator.
+#include "common.cuh"
+#include "host_abi.h"
+
+namespace sl {
+namespace {
+
+template <typename T> __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
+template <> __device__ __forceinline__ void mma16816<__nv_bfloat16>(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <> __device__ __forceinline__ void mma16816<__half>(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// rounded as the library and torch's sums round (no saturation)
+template <typename T> __device__ __forceinline__ float rounded(float v);
+template <> __device__ __forceinline__ float rounded<__nv_bfloat16>(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+template <> __device__ __forceinline__ float rounded<__half>(float v) { return __half2float(__float2half_rn(v)); }
+template <typename T> __device__ __forceinline__ uint32_t plain_pair(float a, float b);
+template <> __device__ __forceinline__ uint32_t plain_pair<__nv_bfloat16>(float a, float b) { return pack_pair<__nv_bfloat16>(a, b); }
+template <> __device__ __forceinline__ uint32_t plain_pair<__half>(float a, float b) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {   // the rest of the 16 is zeroed
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+constexpr int KC = 256;                       // k values of a piece of x
+constexpr int X_PITCH = 2 * KC + 32;          // rows 32 bytes off a multiple of 128: 8-byte reads of 4 rows x 32 bytes hit all banks
+__host__ __device__ constexpr int w_pitch(int K) { return (2 * K + 127) / 128 * 128 + 32; }
+
+// MT: 16-row tiles of x; NT: 8-row tiles of W per warp (2: value and gate of SwiGLU)
+template <typename T, int MT, int NT>
+__global__ void __launch_bounds__(128) token_linear_kernel(TokenLinearArgs p) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5, g = lane >> 2, t = lane & 3;
+  const int K = p.K, wp = w_pitch(K), half = p.O / NT, o0 = 8 * (blockIdx.x * nw + w);   // this warp's rows of W: o0 .. (+ half)
+  uint8_t* const s_x = smem;                                    // [2][16 MT][X_PITCH]
+  uint8_t* const s_w = smem + 2 * 16 * MT * X_PITCH + (size_t)w * NT * 8 * wp;
+  const T* W = reinterpret_cast<const T*>(p.weight);
+  grid_release();
+  // ---- request this warp's rows of W; k beyond K reads as zero up to the next step ---------------------------------
+  const int pieces = (K + 15) / 16 * 2;   // 16-byte pieces of a row
+  if (o0 < half)
+#pragma unroll 1
+    for (int r = 0; r < 8 * NT; ++r) {
+      const T* row = W + (size_t)((r >> 3) * half + o0 + (r & 7)) * K;
+      for (int c = lane; c < pieces; c += 32) cp_async16(s_w + r * wp + 16 * c, row + (8 * c < K ? 8 * c : 0), 8 * c < K ? 16 : 0);
+    }
+  cp_async_commit();
+  grid_wait();
+  // ---- x, two pieces of k ahead ------------------------------------------------------------------------------------
+  const int M = p.M, chunks = (K + KC - 1) / KC;
+  const T* X = reinterpret_cast<const T*>(p.x);
+  auto stage = [&](int c) {
+    if (c < chunks)
+      for (int i = tid; i < M * (KC / 8); i += blockDim.x) {
+        const int m = i / (KC / 8), k = c * KC + 8 * (i % (KC / 8));
+        cp_async16(s_x + ((c & 1) * 16 * MT + m) * X_PITCH + 16 * (i % (KC / 8)), X + (size_t)m * K + (k < K ? k : 0), k < K ? 16 : 0);
+      }
+    cp_async_commit();
+  };
+  stage(0);
+  stage(1);
+  float acc[MT][NT][4];
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
+  for (int c = 0; c < chunks; ++c) {
+    cp_async_wait<1>();
+    __syncthreads();
+    if (o0 < half) {
+      const uint8_t* xs = s_x + (c & 1) * 16 * MT * X_PITCH + 8 * t;
+      const uint8_t* ws = s_w + 2 * c * KC + 8 * t;
+      const int steps = min(KC, K - c * KC + 15) / 16;
+#pragma unroll 4
+      for (int s = 0; s < steps; ++s) {
+        uint2 b[NT];
+#pragma unroll
+        for (int j = 0; j < NT; ++j) b[j] = *reinterpret_cast<const uint2*>(ws + (8 * j + g) * wp + 32 * s);
+#pragma unroll
+        for (int i = 0; i < MT; ++i) {
+          const uint2 lo = *reinterpret_cast<const uint2*>(xs + (16 * i + g) * X_PITCH + 32 * s);
+          const uint2 hi = *reinterpret_cast<const uint2*>(xs + (16 * i + 8 + g) * X_PITCH + 32 * s);
+          const uint32_t a[4] = {lo.x, hi.x, lo.y, hi.y};   // (rows beyond M hold anything: they reach their own results only)
+#pragma unroll
+          for (int j = 0; j < NT; ++j) mma16816<T>(acc[i][j], a, b[j].x, b[j].y);
+        }
+      }
+    }
+    __syncthreads();
+    stage(c + 2);
+  }
+  if (o0 >= half) return;
+  // ---- epilogue: rounded as the product, then what follows it --------------------------------------------------------
+  T* out = reinterpret_cast<T*>(p.out[0]);
+  int width = p.width[0], col = o0;
+  if (NT == 1) {
+    if (col >= width) { col -= width; out = reinterpret_cast<T*>(p.out[1]); width = p.width[1]; }
+    if (col >= width && p.out[2]) { col -= width; out = reinterpret_cast<T*>(p.out[2]); width = p.width[2]; }
+  }
+  const T* bias = reinterpret_cast<const T*>(p.bias);
+  float bv[NT][2];
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) bv[j][e] = bias ? to_f32(bias[j * half + o0 + 2 * t + e]) : 0.f;
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      const int m = 16 * i + 8 * hh + g;
+      if (m >= M) continue;
+      float v[NT][2];
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          v[j][e] = acc[i][j][2 * hh + e];
+          if (bias) v[j][e] += bv[j][e];
+        }
+      const size_t at = (size_t)m * width + col + 2 * t;
+      uint32_t word;
+      if (NT == 2) {
+        word = pack_pair<T>(rounded<T>(v[0][0]) * silu_f(rounded<T>(v[NT - 1][0])), rounded<T>(v[0][1]) * silu_f(rounded<T>(v[NT - 1][1])));
+      } else if (p.gelu) {
+        word = pack_pair<T>(gelu_tanh_f<true>(rounded<T>(v[0][0])), gelu_tanh_f<true>(rounded<T>(v[0][1])));
+      } else if (p.residual) {
+        const float2 r = unpack_pair<T>(*reinterpret_cast<const uint32_t*>(reinterpret_cast<const T*>(p.residual) + at));
+        word = plain_pair<T>(r.x + rounded<T>(v[0][0]), r.y + rounded<T>(v[0][1]));
+      } else {
+        word = plain_pair<T>(v[0][0], v[0][1]);
+      }
+      *reinterpret_cast<uint32_t*>(out + at) = word;
+    }
+}
+
+// Warps of a CTA: one while their rows of W (8 a warp) still spread over the SMs, more when there are several for each.
+int warps_of(const TokenLinearArgs& a, size_t* smem) {
+  const int NT = a.swiglu ? 2 : 1, MT = (a.M + 15) / 16;
+  const int tiles = a.O / NT / 8;
+  int nw = tiles <= 2 * 148 ? 1 : tiles <= 8 * 148 ? 2 : 4;
+  for (;; nw /= 2) {
+    *smem = 2 * 16 * (size_t)MT * X_PITCH + (size_t)nw * NT * 8 * w_pitch(a.K);
+    if (nw == 0 || *smem <= 200 * 1024) return nw;
+  }
+}
+
+template <typename T, int MT, int NT>
+int launch_token_as(const TokenLinearArgs& a, int nw, size_t smem, cudaStream_t st) {
+  static std::atomic<unsigned long long> done{0};
+  if (int e = ensure_smem(token_linear_kernel<T, MT, NT>, 200 * 1024, done)) return e;
+  const int tiles = a.O / NT / 8;
+  return launch_chained(token_linear_kernel<T, MT, NT>, dim3((tiles + nw - 1) / nw), (unsigned)(32 * nw), smem, st, true, a);
+}
+template <typename T, int MT>
+int launch_token_m(const TokenLinearArgs& a, int nw, size_t smem, cudaStream_t st) {
+  return a.swiglu ? launch_token_as<T, MT, 2>(a, nw, smem, st) : launch_token_as<T, MT, 1>(a, nw, smem, st);
+}
+template <typename T>
+int launch_token(const TokenLinearArgs& a, int nw, size_t smem, cudaStream_t st) {
+  switch ((a.M + 15) / 16) {
+    case 1: return launch_token_m<T, 1>(a, nw, smem, st);
+    case 2: return launch_token_m<T, 2>(a, nw, smem, st);
+    case 3: return launch_token_m<T, 3>(a, nw, smem, st);
+    default: return launch_token_m<T, 4>(a, nw, smem, st);
+  }
+}
+
+}  // namespace
+
+// Widths that are no multiple of 8 are the library's (its kernels for them sum in another order).
+bool token_linear_supported(const TokenLinearArgs& a) {
+  size_t smem;
+  if (a.M < 1 || a.M > 64 || a.K < 8 || a.K % 8 || a.O < 8 || a.O % (a.swiglu ? 16 : 8) || (a.io_dtype != SL_BF16 && a.io_dtype != SL_F16))
+    return false;
+  for (int i = 0; i < 3; ++i)
+    if (a.width[i] % 8 || !aligned(a.out[i], 4)) return false;
+  return aligned(a.x, 16) && aligned(a.weight, 16) && aligned(a.residual, 4) && warps_of(a, &smem) > 0;
+}
+
+int token_linear(const TokenLinearArgs& a, cudaStream_t st) {
+  if (!a.x || !a.weight || !a.out[0]) return SL_ERR_NULL_POINTER;
+  if (!token_linear_supported(a)) return SL_ERR_UNSUPPORTED;
+  size_t smem;
+  const int nw = warps_of(a, &smem);
+  const int rc = a.io_dtype == SL_BF16 ? launch_token<__nv_bfloat16>(a, nw, smem, st) : launch_token<__half>(a, nw, smem, st);
+  if (rc != SL_OK) return rc;
+  note_launches(1);
+  return launch_status();
+}
+
+}  // namespace sl

@@ -208,3 +208,32 @@ def test_the_engine_refuses_weights_of_another_type(batch, weights, token):
     with pytest.raises(RuntimeError, match="dtype"):
         MixerDecodeEngine(mixer, batch, dtype=token)
     assert MixerDecodeEngine(mixer.to(token), batch, dtype=token).step(torch.zeros(batch, 128, device=DEV, dtype=token)).isfinite().all()
+
+
+# the sizes where a block's own products change: row tiles of 16, k tails of 8, biases, parts of in_proj whose width is no
+# multiple of 8 (3 heads of 18: that part stays the library's), layers too long for shared memory
+@pytest.mark.parametrize("batch, d_model, dtype, d_head, kind, bias, hidden", [
+    (1, 8, torch.bfloat16, 8, "gelu", False, 8), (16, 264, torch.float16, 64, "gelu", True, 520),
+    (32, 576, torch.bfloat16, 32, "swiglu", True, 1000), (33, 128, torch.float16, 64, "swiglu", False, 72),
+    (48, 1024, torch.bfloat16, 64, "gelu", False, 4096), (64, 192, torch.bfloat16, 64, "swiglu", False, 8192)])
+def test_token_products_have_the_librarys_bits(batch, d_model, dtype, d_head, kind, bias, hidden, monkeypatch):
+    torch.manual_seed(batch)
+    blk = sb.SLinOSSBlockConfig(d_model=d_model, mixer=sb.SLinOSSMixerConfig(d_state=64, d_head=d_head, expand=1.0),
+                                ffn=sb.SLinOSSMLPConfig(kind=kind, hidden_dim=hidden, multiple_of=8, bias=bias))
+    stack = sb.SLinOSSStack(sb.SLinOSSStackConfig.uniform(blk, n_layers=2), device=DEV, dtype=dtype).eval()
+    x = torch.randn(3, batch, d_model, device=DEV, dtype=dtype)
+
+    def run():
+        with torch.no_grad():
+            state, out = stack.init_decode_state(batch), []
+            for t in x:
+                y, state = stack.step(t, state)
+                out.append(y)
+        return torch.stack(out)
+
+    got = run()
+    planned = ["_token_plan" in b.__dict__ for b in stack.blocks]
+    monkeypatch.setattr(sb.SLinOSSBlock, "_make_token_plan", lambda self: None)
+    for b in stack.blocks:
+        b.__dict__.pop("_token_plan", None)
+    assert all(planned) and torch.equal(got, run())
