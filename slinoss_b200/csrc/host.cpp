@@ -497,7 +497,8 @@ class TokenPlan {
     // bits, which residual stream, norms and B/C phases carry on from block to block: six blocks of width 1024 end up 1.6 % from the
     // composed token.  token_linear adds in the library's order, with residual and activation inside; what it does not take (more than
     // 64 rows, widths that are no multiple of 8) goes to the library, there without a dispatch.  A token of four blocks of width 512
-    // at batch 8 is bound by the host: 398 us with 24 library products and 29 other launches, 184 with 8 launches a block (172 of them on the device).
+    // at batch 8 is bound by the host: 398 us with 24 library products and 29 other launches, 146 with 5 launches a block (the host needs 123; 8 launches, the norms by
+    // themselves: 184).
     at::AutoDispatchBelowAutograd below;
     auto fresh = [&](int64_t cols) { return at::detail::empty_cuda({M, cols}, type, x.device(), c10::nullopt); };
     auto norm = [&](const Tensor& a, const Tensor& w, double eps) {
@@ -505,17 +506,19 @@ class TokenPlan {
       check(sl_rmsnorm_fwd(ptr(a), ptr(w), (float)eps, mptr(out), M, D, io, st), "sl_rmsnorm_fwd");
       return out;
     };
-    const Tensor rows = x.contiguous(), normed = norm(rows, *b_[0], eps_[0]);
+    const Tensor rows = x.contiguous();
     auto product = [](const Tensor& a, const Tensor& W, int64_t row, int64_t n) {   // a (rows row .. row + n of W)^T
       return at::cuda::mm(a, at::native::as_strided_tensorimpl(W, {W.size(1), n}, {1, W.size(1)}, W.storage_offset() + row * W.size(1)));
     };
     // own kernel with what follows the product inside; false where it is left to the library
-    auto fused = [&](const Tensor& a, const Tensor& W, int64_t row, int64_t n, const OptT& bias, std::initializer_list<const Tensor*> out,
-                     const Tensor* residual = nullptr, int act = -1) {
-      sl::TokenLinearArgs t{ptr(a), static_cast<const uint8_t*>(W.data_ptr()) + row * W.size(1) * 2, ptr(bias), {}, {},
+    auto fused = [&](const void* a, const Tensor& W, int64_t row, int64_t n, const OptT& bias, std::initializer_list<const Tensor*> out,
+                     const Tensor* residual = nullptr, int act = -1, const Tensor* norm_w = nullptr, double eps = 0.0,
+                     const float* partials = nullptr) {
+      sl::TokenLinearArgs t{a, static_cast<const uint8_t*>(W.data_ptr()) + row * W.size(1) * 2, ptr(bias), {}, {},
                             residual ? ptr(*residual) : nullptr, (int)M, (int)W.size(1), (int)n, io, act == 0, act == 1};
       int i = 0;
       for (const Tensor* o : out) { t.out[i] = mptr(*o); t.width[i++] = (int)o->size(1); }
+      if (norm_w) { t.norm_weight = ptr(*norm_w); t.norm_eps = (float)eps; t.partials = partials; t.n_partials = (int)(8 * heads_); }
       if (!sl::token_linear_supported(t)) return false;
       check(sl::token_linear(t, st), "token_linear");
       return true;
@@ -526,27 +529,36 @@ class TokenPlan {
     // residual + linear
     auto onto = [&](const Tensor& residual, const Tensor& a, const Tensor& W, const OptT& bias) {
       Tensor out = fresh(D);
-      if (fused(a, W, 0, D, bias, {&out}, &residual)) return out;
+      if (fused(ptr(a), W, 0, D, bias, {&out}, &residual)) return out;
       const Tensor branch = linear(a, W, bias);
       check(sl::rmsnorm_fwd_sum(ptr(residual), ptr(branch), mptr(out), nullptr, 0.f, nullptr, M, D, io, st), "sl_rmsnorm_fwd");
       return out;
     };
     const int64_t n_gv = 2 * C, n_par = 3 * heads_, n_bc = 4 * groups_ * N_;
     Tensor gv = fresh(n_gv), params = fresh(n_par), bc = fresh(n_bc);
-    if (!fused(normed, *p_[0], 0, O, {}, {&gv, &params, &bc})) {
-      if (!fused(normed, *p_[0], 0, n_gv, {}, {&gv})) gv = product(normed, *p_[0], 0, n_gv);
-      if (!fused(normed, *p_[0], n_gv, n_par, {}, {&params})) params = product(normed, *p_[0], n_gv, n_par);
-      if (!fused(normed, *p_[0], n_gv + n_par, n_bc, {}, {&bc})) bc = product(normed, *p_[0], n_gv + n_par, n_bc);
+    if (!fused(ptr(rows), *p_[0], 0, O, {}, {&gv, &params, &bc}, nullptr, -1, &*b_[0], eps_[0])) {
+      const Tensor normed = norm(rows, *b_[0], eps_[0]);
+      if (!fused(ptr(normed), *p_[0], 0, O, {}, {&gv, &params, &bc})) {
+        if (!fused(ptr(normed), *p_[0], 0, n_gv, {}, {&gv})) gv = product(normed, *p_[0], 0, n_gv);
+        if (!fused(ptr(normed), *p_[0], n_gv, n_par, {}, {&params})) params = product(normed, *p_[0], n_gv, n_par);
+        if (!fused(ptr(normed), *p_[0], n_gv + n_par, n_bc, {}, {&bc})) bc = product(normed, *p_[0], n_gv + n_par, n_bc);
+      }
     }
     mixer_step(gv.data_ptr(), column(gv, C), params.data_ptr(), bc.data_ptr(), n_gv, n_par, n_bc, false);
-    const Tensor hid = fresh(C);
-    check(sl::mixer_step_norm(base, ptr(p_[9]), (float)eps_[1], mptr(hid), M, heads_, P_, io, st), "mixer_step");
-    Tensor out = onto(rows, hid, *p_[10], p_[11]);
+    Tensor out = fresh(D);
+    if (!fused(base, *p_[10], 0, D, p_[11], {&out}, &rows, -1, &*p_[9], eps_[1], sl::step_partials(base, M, heads_, P_))) {
+      const Tensor hid = fresh(C);
+      check(sl::mixer_step_norm(base, ptr(p_[9]), (float)eps_[1], mptr(hid), M, heads_, P_, io, st), "mixer_step");
+      out = onto(rows, hid, *p_[10], p_[11]);
+    }
     if (ffn) {
-      const Tensor in = norm(out, *b_[1], eps_[2]), act = fresh(b_[4]->size(1));
-      if (!fused(in, *b_[2], 0, b_[2]->size(0), b_[3], {&act}, nullptr, ffn_kind_)) {
-        const Tensor wide = linear(in, *b_[2], b_[3]);
-        check(sl_ffn_activation_fwd(ptr(wide), mptr(act), M, act.size(1), ffn_kind_, io, st), "sl_ffn_activation_fwd");
+      const Tensor act = fresh(b_[4]->size(1));
+      if (!fused(ptr(out), *b_[2], 0, b_[2]->size(0), b_[3], {&act}, nullptr, ffn_kind_, &*b_[1], eps_[2])) {
+        const Tensor in = norm(out, *b_[1], eps_[2]);
+        if (!fused(ptr(in), *b_[2], 0, b_[2]->size(0), b_[3], {&act}, nullptr, ffn_kind_)) {
+          const Tensor wide = linear(in, *b_[2], b_[3]);
+          check(sl_ffn_activation_fwd(ptr(wide), mptr(act), M, act.size(1), ffn_kind_, io, st), "sl_ffn_activation_fwd");
+        }
       }
       out = onto(out, act, *b_[4], b_[5]);
     }

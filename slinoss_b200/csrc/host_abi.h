@@ -63,6 +63,11 @@ struct TokenLinearArgs {
   const void* residual;            // (M, O) or null: added to the rounded product
   int M, K, O, io_dtype;
   bool gelu, swiglu;               // activation of the rounded product; swiglu: value rows, then gate rows
+  // of x first, M <= 16: RMSNorm with the bits of sl_rmsnorm_fwd, or with the partial sums of squares of mixer_step_norm
+  const void* norm_weight = nullptr;
+  float norm_eps = 0.f;
+  const float* partials = nullptr;
+  int n_partials = 0;
 };
 SL_API bool token_linear_supported(const TokenLinearArgs& a);
 SL_API int token_linear(const TokenLinearArgs& a, cudaStream_t st);

@@ -8,7 +8,7 @@
 // does not matter, which lets a lane read 8 consecutive bytes of a row for its four values.
 //
 // What bounds it: the launch.  A library product costs the host 7 to 9 us and a launch of its own for each part of in_proj, the
-// residual and the activation; here it is 2 to 3 us with all of them inside.  On the device: latency of one trip to memory
+// residual, the activation and the norm; here it is 2 to 3 us with all of them inside (norms: up to 16 rows).  On the device: latency of one trip to memory
 // (all of a warp's rows of W are requested at the start, x two pieces ahead) and the chain of K / 16 steps on one accumulator.
 #include "common.cuh"
 #include "host_abi.h"
@@ -48,14 +48,52 @@ constexpr int KC = 256;                       // k values of a piece of x
 constexpr int X_PITCH = 2 * KC + 32;          // rows 32 bytes off a multiple of 128: 8-byte reads of 4 rows x 32 bytes hit all banks
 __host__ __device__ constexpr int w_pitch(int K) { return (2 * K + 127) / 128 * 128 + 32; }
 
-// MT: 16-row tiles of x; NT: 8-row tiles of W per warp (2: value and gate of SwiGLU)
-template <typename T, int MT, int NT>
-__global__ void __launch_bounds__(128) token_linear_kernel(TokenLinearArgs p) {
+// The norm of the rows of x in shared memory, in place, a warp per row: the additions of rmsnorm_fwd_kernel (partials null) or of
+// step_norm_kernel in their order.  Every CTA does it for itself, with more warps than it has
+// rows of W for: at 16 rows at most that is shorter than a launch (with the 1 or 2 warps of the product it was longer).
+template <typename T>
+__device__ __forceinline__ void norm_rows(const TokenLinearArgs& p, uint8_t* s_x, int pitch) {
+  const int lane = threadIdx.x & 31, pieces = p.K / 8;
+  for (int m = threadIdx.x >> 5; m < p.M; m += blockDim.x >> 5) {
+    uint4* row = reinterpret_cast<uint4*>(s_x + m * pitch);
+    float ss = 0.f;
+    if (p.partials) {
+      const float* part = p.partials + (size_t)m * p.n_partials;
+      for (int v = 0; v < 8; ++v) {
+        float s = 0.f;
+        for (int k = 32 * v + lane; k < p.n_partials; k += 256) s += part[k];
+        ss += warp_sum(s);
+      }
+    } else {
+      for (int c = lane; c < pieces; c += 32) {
+        float v[8];
+        unpack16<T>(row[c], v);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ss += v[k] * v[k];
+      }
+      ss = warp_sum(ss);
+    }
+    const float rstd = rsqrtf(ss / (float)p.K + p.norm_eps);
+    for (int c = lane; c < pieces; c += 32) {
+      float v[8], wv[8];
+      unpack16<T>(row[c], v);
+      load16<T>(reinterpret_cast<const T*>(p.norm_weight) + 8 * c, wv);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = v[k] * rstd * wv[k];
+      store16<T>(reinterpret_cast<T*>(row + c), v);
+    }
+  }
+}
+
+// MT: 16-row tiles of x; NT: 8-row tiles of W per warp (2: value and gate of SwiGLU); NORM: x whole in shared memory
+template <typename T, int MT, int NT, bool NORM>
+__global__ void __launch_bounds__(NORM ? 256 : 128) token_linear_kernel(TokenLinearArgs p, int nw) {   // nw: warps with rows of W
   extern __shared__ __align__(16) uint8_t smem[];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5, g = lane >> 2, t = lane & 3;
-  const int K = p.K, wp = w_pitch(K), half = p.O / NT, o0 = 8 * (blockIdx.x * nw + w);   // this warp's rows of W: o0 .. (+ half)
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int K = p.K, wp = w_pitch(K), half = p.O / NT;
+  const int o0 = w < nw ? 8 * (blockIdx.x * nw + w) : half;   // this warp's rows of W: o0 .. (+ half)
   uint8_t* const s_x = smem;                                    // [2][16 MT][X_PITCH]
-  uint8_t* const s_w = smem + 2 * 16 * MT * X_PITCH + (size_t)w * NT * 8 * wp;
+  uint8_t* const s_w = smem + (NORM ? 16 * wp : 2 * 16 * MT * X_PITCH) + (size_t)w * NT * 8 * wp;
   const T* W = reinterpret_cast<const T*>(p.weight);
   grid_release();
   // ---- request this warp's rows of W; k beyond K reads as zero up to the next step ---------------------------------
@@ -79,20 +117,33 @@ __global__ void __launch_bounds__(128) token_linear_kernel(TokenLinearArgs p) {
       }
     cp_async_commit();
   };
-  stage(0);
-  stage(1);
+  if (NORM) {
+    for (int m = 0; m < M; ++m)
+      for (int c = tid; c < pieces; c += blockDim.x) cp_async16(s_x + m * wp + 16 * c, X + (size_t)m * K + (8 * c < K ? 8 * c : 0), 8 * c < K ? 16 : 0);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    norm_rows<T>(p, s_x, wp);
+    __syncthreads();
+  } else {
+    stage(0);
+    stage(1);
+  }
+  const int x_pitch = NORM ? wp : X_PITCH, turns = NORM ? 1 : chunks;
   float acc[MT][NT][4];
 #pragma unroll
   for (int i = 0; i < MT; ++i)
 #pragma unroll
     for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
-  for (int c = 0; c < chunks; ++c) {
-    cp_async_wait<1>();
-    __syncthreads();
+  for (int c = 0; c < turns; ++c) {
+    if (!NORM) {
+      cp_async_wait<1>();
+      __syncthreads();
+    }
     if (o0 < half) {
       const uint8_t* xs = s_x + (c & 1) * 16 * MT * X_PITCH + 8 * t;
       const uint8_t* ws = s_w + 2 * c * KC + 8 * t;
-      const int steps = min(KC, K - c * KC + 15) / 16;
+      const int steps = ((NORM ? K : min(KC, K - c * KC)) + 15) / 16;
 #pragma unroll 4
       for (int s = 0; s < steps; ++s) {
         uint2 b[NT];
@@ -100,16 +151,18 @@ __global__ void __launch_bounds__(128) token_linear_kernel(TokenLinearArgs p) {
         for (int j = 0; j < NT; ++j) b[j] = *reinterpret_cast<const uint2*>(ws + (8 * j + g) * wp + 32 * s);
 #pragma unroll
         for (int i = 0; i < MT; ++i) {
-          const uint2 lo = *reinterpret_cast<const uint2*>(xs + (16 * i + g) * X_PITCH + 32 * s);
-          const uint2 hi = *reinterpret_cast<const uint2*>(xs + (16 * i + 8 + g) * X_PITCH + 32 * s);
+          const uint2 lo = *reinterpret_cast<const uint2*>(xs + (16 * i + g) * x_pitch + 32 * s);
+          const uint2 hi = *reinterpret_cast<const uint2*>(xs + (16 * i + 8 + g) * x_pitch + 32 * s);
           const uint32_t a[4] = {lo.x, hi.x, lo.y, hi.y};   // (rows beyond M hold anything: they reach their own results only)
 #pragma unroll
           for (int j = 0; j < NT; ++j) mma16816<T>(acc[i][j], a, b[j].x, b[j].y);
         }
       }
     }
-    __syncthreads();
-    stage(c + 2);
+    if (!NORM) {
+      __syncthreads();
+      stage(c + 2);
+    }
   }
   if (o0 >= half) return;
   // ---- epilogue: rounded as the product, then what follows it --------------------------------------------------------
@@ -161,21 +214,23 @@ int warps_of(const TokenLinearArgs& a, size_t* smem) {
   const int tiles = a.O / NT / 8;
   int nw = tiles <= 2 * 148 ? 1 : tiles <= 8 * 148 ? 2 : 4;
   for (;; nw /= 2) {
-    *smem = 2 * 16 * (size_t)MT * X_PITCH + (size_t)nw * NT * 8 * w_pitch(a.K);
+    *smem = (a.norm_weight ? 16 * w_pitch(a.K) : 2 * 16 * (size_t)MT * X_PITCH) + (size_t)nw * NT * 8 * w_pitch(a.K);
     if (nw == 0 || *smem <= 200 * 1024) return nw;
   }
 }
 
-template <typename T, int MT, int NT>
+template <typename T, int MT, int NT, bool NORM>
 int launch_token_as(const TokenLinearArgs& a, int nw, size_t smem, cudaStream_t st) {
   static std::atomic<unsigned long long> done{0};
-  if (int e = ensure_smem(token_linear_kernel<T, MT, NT>, 200 * 1024, done)) return e;
+  if (int e = ensure_smem(token_linear_kernel<T, MT, NT, NORM>, 200 * 1024, done)) return e;
   const int tiles = a.O / NT / 8;
-  return launch_chained(token_linear_kernel<T, MT, NT>, dim3((tiles + nw - 1) / nw), (unsigned)(32 * nw), smem, st, true, a);
+  return launch_chained(token_linear_kernel<T, MT, NT, NORM>, dim3((tiles + nw - 1) / nw), (unsigned)(NORM ? 256 : 32 * nw), smem, st, true, a, nw);
 }
 template <typename T, int MT>
 int launch_token_m(const TokenLinearArgs& a, int nw, size_t smem, cudaStream_t st) {
-  return a.swiglu ? launch_token_as<T, MT, 2>(a, nw, smem, st) : launch_token_as<T, MT, 1>(a, nw, smem, st);
+  if constexpr (MT == 1)
+    if (a.norm_weight) return a.swiglu ? launch_token_as<T, 1, 2, true>(a, nw, smem, st) : launch_token_as<T, 1, 1, true>(a, nw, smem, st);
+  return a.swiglu ? launch_token_as<T, MT, 2, false>(a, nw, smem, st) : launch_token_as<T, MT, 1, false>(a, nw, smem, st);
 }
 template <typename T>
 int launch_token(const TokenLinearArgs& a, int nw, size_t smem, cudaStream_t st) {
@@ -196,6 +251,7 @@ bool token_linear_supported(const TokenLinearArgs& a) {
     return false;
   for (int i = 0; i < 3; ++i)
     if (a.width[i] % 8 || !aligned(a.out[i], 4)) return false;
+  if (a.norm_weight && (a.M > 16 || !aligned(a.norm_weight, 16) || (!a.partials && a.K > 2048))) return false;
   return aligned(a.x, 16) && aligned(a.weight, 16) && aligned(a.residual, 4) && warps_of(a, &smem) > 0;
 }
 
