@@ -252,30 +252,46 @@ void ensure_context() {
 // (``fixed`` chunk times).  The model below counts the chunk times of the most loaded SM: an SM with one
 // resident CTA takes 1 per chunk, one with two takes ``pair`` (2 when only one fits).
 constexpr int FOLD_SEGS = 8;
-struct SegPlan { int nseg, cps; };
+struct SegPlan { int nseg, cps, tail, whole; };   // tail, whole: see bwd_plan
 struct SegCost { double pair, pre, fixed; };
 constexpr int SMS = 148;
 inline double load_time(long long ctas, double chunks, double pair) {
   const long long per_sm = (ctas + SMS - 1) / SMS;
   return chunks * ((per_sm / 2) * pair + (per_sm & 1));
 }
-inline SegPlan plan_segments(long long streams, int nchunks, const SegCost& c) {
-  SegPlan best{1, nchunks};
+inline SegPlan plan_segments(long long streams, int nchunks, const SegCost& c, double* cost = nullptr) {
+  SegPlan best{1, nchunks, 0, 0};
   double t_best = load_time(streams, nchunks, c.pair);
   for (int s = 2; s <= nchunks && s * streams <= 4 * SMS; ++s) {
     const int cps = (nchunks + s - 1) / s, ns = (nchunks + cps - 1) / cps;
     if (ns != s) continue;
     const double t = load_time(streams * s, cps, c.pair) + c.pre * load_time(streams * (s - 1), cps, c.pair) + c.fixed;
-    if (t < 0.97 * t_best) { t_best = t; best = {s, cps}; }
+    if (t < 0.97 * t_best) { t_best = t; best = {s, cps, 0, 0}; }
   }
+  if (cost) *cost = t_best;
   return best;
 }
 inline SegPlan fwd_plan(const ScanDims& d) {
   return plan_segments((long long)d.batch * d.heads, chunks_of(d),
                        blocks_of(d) == 1 ? SegCost{1.6, 0.5, 4.5} : SegCost{2.0, 0.4, 3.0});
 }
+// The reverse sweep holds one CTA per SM, so its last round of CTAs leaves SMs idle (20 of 148 with 128 streams, 40 in the
+// second round of 256).  There the streams of that round give their last ``tail`` chunks to the idle SMs: these CTAs come
+// last in the grid and need nothing of the others, while the rest of a stream waits for the pre-pass over its tail only.
+// An idle SM takes ``fill`` tails one after the other, each with 0.7 of a chunk to start up, beside the nC - tail chunks of the
+// rest.  The pre-pass takes 0.25 of a chunk per chunk and 1.0 for its launch.  Sweep and pre-pass, us, whole against so split:
+// 128 streams x 64 chunks 297 / 280 (tail 7; 8: 297, 4: 291), 256 x 32 301 / 285 (7), 100 x 64 291 (in two equal segments) / 256
+// (16), 64 x 64 of two column blocks 297 / 285 (7).
 inline SegPlan bwd_plan(const ScanDims& d) {
-  return plan_segments((long long)d.batch * d.heads * blocks_of(d), chunks_of(d), SegCost{2.0, 0.25, 2.0});
+  const int nb = blocks_of(d), nC = chunks_of(d);
+  const long long streams = (long long)d.batch * d.heads, ctas = streams * nb;
+  double best;
+  const SegPlan plan = plan_segments(ctas, nC, SegCost{2.0, 0.25, 2.0}, &best);
+  const int rounds = (int)(ctas / SMS), over = (int)(ctas % SMS);
+  if (!over) return plan;
+  const int fill = (over + SMS - over - 1) / (SMS - over), tail = (int)((nC - 0.7 * fill) / (fill + 1));
+  if (tail < 1 || rounds * (double)nC + (nC - tail) + 0.25 * tail + 1.3 >= 0.98 * best) return plan;
+  return {2, nC - tail, tail, (int)((long long)rounds * SMS / nb)};
 }
 struct SegLayout { size_t seg, pi, total; };
 inline SegLayout seg_layout(const ScanDims& d, int nseg) {
@@ -412,7 +428,7 @@ int scan_tc_fwd(const void* U, const float* M, const float* K, const void* B, co
   SegPlan plan = fwd_plan(d);
   if (!ws || ws_bytes < scan_tc_fwd_workspace(d)) {   // N = 64 has always run without: the streams are then walked whole
     if (blocks_of(d) == 2) return SL_ERR_WORKSPACE_TOO_SMALL;
-    plan = {1, chunks_of(d)};
+    plan = {1, chunks_of(d), 0, 0};
   }
   return scan_tc_fwd_impl(U, M, K, B, C, z0, Bprev, Uprev, Y, zfinal, states_out, d, plan,
                           reinterpret_cast<uint8_t*>(ws), io_dtype, y_dtype, st);
@@ -461,6 +477,7 @@ int run_bwd(const void* U, const float* M, const float* K, const void* B, const 
   float* dstart = dinit ? dinit : (Bprev ? reinterpret_cast<float*>(w + lay.dstart) : nullptr);
   float2* dgb = Bprev ? reinterpret_cast<float2*>(w + lay.dgb) : nullptr;
   p.dinit = dstart; p.T = d.T; p.N = d.N; p.nchunks = nC; p.cps = plan.cps; p.nseg = plan.nseg;
+  p.tail = plan.tail; p.whole = plan.whole;
   p.heads = d.heads; p.groups = d.groups;
   p.wait_limit = wait_limit_clocks();
   if (plan.nseg > 1) {   // the adjoint at the end of every segment
@@ -469,9 +486,10 @@ int run_bwd(const void* U, const float* M, const float* K, const void* B, const 
     q.tmU = p.tmdY; q.tmB = p.tmC;
     q.M = M; q.K = K; q.heads = d.heads; q.groups = d.groups; q.T = d.T;
     q.nchunks = nC; q.cps = plan.cps; q.nseg = plan.nseg; q.wait_limit = p.wait_limit;
+    q.tail = plan.tail; q.bh0 = plan.whole;
     q.seg = reinterpret_cast<float*>(w + lay.segs + sl.seg);
     q.seg_pi = reinterpret_cast<float2*>(w + lay.segs + sl.pi);
-    if (int e = launch_prepass<TIn, 2>(q, (int)BH, nb, st)) return e;
+    if (int e = launch_prepass<TIn, 2>(q, (int)BH - plan.whole, nb, st)) return e;
     p.fold = plan.nseg <= FOLD_SEGS;
     if (!p.fold) {
       scan_tc_combine_kernel<TIn, true><<<dim3((unsigned)BH, 16u * nb), 256, 0, st>>>(
@@ -484,7 +502,7 @@ int run_bwd(const void* U, const float* M, const float* K, const void* B, const 
     auto k = scan_tc_bwd_kernel<TIn, 4>;
     static std::atomic<unsigned long long> done{0};
     if (int e = ensure_smem(k, B_SMEM_BYTES, done)) return e;
-    k<<<dim3((unsigned)BH, (unsigned)plan.nseg, (unsigned)nb), 576, B_SMEM_BYTES, st>>>(p);
+    k<<<dim3((unsigned)BH, (unsigned)nb, (unsigned)plan.nseg), 576, B_SMEM_BYTES, st>>>(p);
     note_launches(1);
     if (int e = launch_status()) return e;
   }

@@ -53,11 +53,12 @@ struct alignas(64) TcBwdParams {
   float2 *dg, *sterm, *dkcd, *anchor;   // per token / per chunk scalars (workspace), one set per column block
   float* dinit;          // (BH, 64, 2N) adjoint of the carried start state, or null
   int T, N, nchunks, cps, nseg;
+  int tail, whole;       // tail > 0: two segments, the last of ``tail`` chunks, for the streams from ``whole`` on; the others in one
   int heads, groups;     // B and C are shared by the heads of a group; dB / dC leave per head
   long long wait_limit;  // SM clocks a wait of the main loop may take before the kernel gives up
 };
 
-// grid (batch * heads, segments, column blocks).  NW = warps per TMEM lane quadrant.
+// grid (batch * heads, column blocks, segments).  NW = warps per TMEM lane quadrant.
 template <typename TIn, int NW>
 __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __grid_constant__ TcBwdParams p) {
   static_assert(NW == 4, "a thread owns 8 oscillators of a row: 16 worker warps");
@@ -83,10 +84,14 @@ __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __g
   constexpr int WC = 64 / NW, WB = WC / 8;   // columns / 8-column blocks per warp of a 64-wide accumulator
   const int d0 = cg * 16;                    // first column (inside the half) of this thread
   const uint32_t cell0 = sw128(row, 2 * cg), cell1 = sw128(row, 2 * cg + 1);   // its 32 bytes of a tile row
-  const int bh = blockIdx.x, seg = blockIdx.y, blk = blockIdx.z;
+  const int bh = blockIdx.x, blk = blockIdx.y, seg = blockIdx.z, nb = gridDim.y;
+  const int nseg = p.tail && bh < p.whole ? 1 : p.nseg;   // of this stream
+  if (seg >= nseg) return;
   const int bg = (bh / p.heads) * p.groups + (bh % p.heads) / (p.heads / p.groups);   // row of B and C
   const int T = p.T, nC = p.nchunks, D = 2 * p.N;
-  const int c_lo = seg * p.cps, n = min(p.cps, nC - c_lo);   // this CTA's chunks: c_lo + n - 1 down to c_lo
+  // this CTA's chunks: c_lo + n - 1 down to c_lo
+  const int c_lo = p.tail ? (seg ? nC - p.tail : 0) : seg * p.cps;
+  const int n = p.tail ? (nseg == 1 ? nC : seg ? p.tail : nC - p.tail) : min(p.cps, nC - c_lo);
   const int osc0 = 64 * blk + 32 * hf + 8 * cg;              // first of this thread's 8 oscillators
   const size_t set = (size_t)blk * gridDim.x + bh;           // row of the scalar workspaces
   const float* Mb = p.M + (size_t)bh * T * 2;
@@ -141,7 +146,7 @@ __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __g
   f2 dza[4], dzb[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) { dza[e] = 0ull; dzb[e] = 0ull; }
-  const bool last = seg == p.nseg - 1;
+  const bool last = seg == nseg - 1;
   if (worker && (last || p.fold)) {
     float ar = 0.f, ai = 0.f;
     if (p.dfinal) {
@@ -161,8 +166,8 @@ __global__ void __launch_bounds__(128 * NW + 64, 1) scan_tc_bwd_kernel(const __g
     }
   }
   if (worker && !last) {   // the adjoint at this segment's end: given, or folded from the later segments' contributions
-    const size_t stride = (size_t)64 * 128 * gridDim.z;
-    const float* src = p.seg + ((size_t)bh * p.nseg * 64 + row) * 128 * gridDim.z + 128 * blk + 64 * hf + d0;
+    const size_t stride = (size_t)64 * 128 * nb;
+    const float* src = p.seg + ((size_t)bh * p.nseg * 64 + row) * 128 * nb + 128 * blk + 64 * hf + d0;
     for (int s = p.fold ? p.nseg - 1 : seg; s >= (p.fold ? seg + 1 : seg); --s) {
       const float2 pi = p.fold ? p.seg_pi[(size_t)bh * p.nseg + s] : make_float2(0.f, 0.f);
       const f2 pr = dup2(pi.x), pim = dup2(pi.y), npim = dup2(-pi.y);

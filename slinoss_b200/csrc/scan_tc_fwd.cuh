@@ -47,6 +47,7 @@ struct alignas(64) TcFwdParams {
   float* seg;           // (BH, nseg, 64, 128 NB) float32: start states (from_seg) or, MODE 1 / 2 pre-pass, results
   float2* seg_pi;       // (BH, nseg): transition product of the segment (pre-pass)
   int heads, groups, T, nchunks, cps, nseg, seg0;   // cps: chunks per segment; seg0: segment of blockIdx.y = 0
+  int tail, bh0;   // MODE 2: the last segment's chunks where the others are longer (else 0); first stream of the grid
   int from_seg;   // start states: 1 given in seg, 2 to be folded from the segments' contributions in seg
   int to_seg;     // pre-pass: leave this segment's contribution in seg
   long long wait_limit;  // SM clocks a wait of the main loop may take before the kernel gives up
@@ -81,10 +82,10 @@ __global__ void __launch_bounds__(128 * NWQ + 64, NWQ == 2 ? 2 : 1)
   const int rowA = 16 * quad + (lane >> 2), rowB = rowA + 8, cq = lane & 3;   // epilogue identity
   const int rrow = (tid >> 2) & 63, rk = tid & 3, rgrp = tid >> 8;   // rotation identity
   const uint32_t lane_base = (uint32_t)(32 * quad) << 16;
-  const int bh = blockIdx.x, b = bh / p.heads, h = bh % p.heads;
+  const int bh = ADJ ? p.bh0 + blockIdx.x : blockIdx.x, b = bh / p.heads, h = bh % p.heads;
   const int bg = b * p.groups + h / (p.heads / p.groups);
   const int seg = p.seg0 + blockIdx.y;
-  const int c0 = seg * p.cps, n = min(p.cps, p.nchunks - c0);   // this CTA's chunks: c0 .. c0 + n - 1
+  const int c0 = ADJ && p.tail ? p.nchunks - p.tail : seg * p.cps, n = min(p.cps, p.nchunks - c0);   // this CTA's chunks: c0 .. c0 + n - 1
   const int T = p.T;
   constexpr int D = 128 * NB;   // real columns of a state row
   const float* Mb = p.M + (size_t)bh * T * 2;

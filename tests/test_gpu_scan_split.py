@@ -56,3 +56,23 @@ def test_forward_without_its_workspace_walks_whole_or_is_refused(N):
         assert _C.lib().sl_status_string(status).decode() == "workspace missing or too small"
     else:
         assert status == 0 and rel(Y, want) <= 2e-2 and _C.device_status() == 0
+
+
+# Reverse sweeps whose last round of CTAs gives the ends of its streams to idle SMs: no whole stream and some, a tail of one
+# chunk (ragged) and of several, two column blocks, grouped B/C, carried state and taps.  Against the float32 sweeps on the
+# same 16-bit operands, which are held to the oracle elsewhere: the bar of 16-bit scans.
+@pytest.mark.parametrize("b, h, g, T, N, carried, with_dfinal", [
+    (8, 16, 16, 2500, 64, False, True), (4, 32, 4, 2111, 64, True, True), (8, 32, 32, 2049, 64, False, False),
+    (4, 16, 16, 2305, 128, True, False), (10, 10, 10, 2177, 64, True, True)])
+def test_streams_that_give_their_end_to_idle_sms(b, h, g, T, N, carried, with_dfinal):
+    c = make_scan_case(b, h, T, 64, N, groups=g, dtype=torch.bfloat16, seed=T, streaming=carried, with_init=carried).to("cuda")
+    z0 = None if c.initial_states is None else c.initial_states.float()
+    ops = (c.U, c.M, c.K, c.B, c.C, z0, c.B_prev, c.U_prev)
+    d_final = torch.randn(b, h, 64, 2 * N, device="cuda", generator=torch.Generator("cuda").manual_seed(1)) if with_dfinal else None
+    got = _C.scan_bwd(*ops, c.dY, d_final, chunk_size=64)
+    want = _C.scan_bwd(*ops, c.dY, d_final, chunk_size=64, path="simt")
+    assert _C.device_status() == 0
+    for name, x, y in zip(NAMES, got, want):
+        assert (x is None) == (y is None)
+        if x is not None:
+            assert rel(x, y) <= 2e-2, (name, rel(x, y))
