@@ -213,6 +213,12 @@ def scan_fwd(U, M, K, B, C, z0, B_prev, U_prev, *, chunk_size, y_dtype, want_fin
     return out if save_states else out[:2]
 
 
+def scan_fwd_last(U, M, K, B, C, z0, B_prev, U_prev, *, chunk_size, path="auto"):
+    """The forward scan of 16-bit operands with what a caller carries on from, all in their type: ``(Y, final_state, B_last,
+    U_last)``.  None where the tensor-core path does not run."""
+    return host().scan_fwd_last(U, M, K, B, C, z0, B_prev, U_prev, chunk_size, _PATHS[path])
+
+
 def scan_bwd(U, M, K, B, C, z0, B_prev, U_prev, dY, d_final, *, chunk_size, path="auto",
              saved=None):
     """Launch ``sl_v2x2ssd_bwd``.  Returns ``(dU, dM, dK, dB, dC, d_initial, dB_prev,

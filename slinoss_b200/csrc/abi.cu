@@ -2,6 +2,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "host_abi.h"
 
 namespace sl {
 
@@ -18,7 +19,7 @@ size_t scan_tc_states_bytes(const ScanDims& d);
 int scan_tc_fwd(const void* U, const float* M, const float* K, const void* B, const void* C,
                 const float* z0, const void* Bprev, const void* Uprev, void* Y, float* zfinal,
                 void* states_out, const ScanDims& d, int io_dtype, int y_dtype, void* ws,
-                size_t ws_bytes, cudaStream_t st);
+                size_t ws_bytes, cudaStream_t st, const ScanLast* last = nullptr);
 int scan_tc_bwd(const void* U, const float* M, const float* K, const void* B, const void* C,
                 const float* z0, const void* Bprev, const void* Uprev, const void* states_in,
                 const float* zfinal_in, const void* dY,
@@ -50,6 +51,20 @@ bool use_tc(int path, const ScanDims& d, int io_dtype) {
 }
 
 }  // namespace
+}  // namespace sl
+
+namespace sl {
+int scan_fwd_last(const void* U, const float* M, const float* K, const void* B, const void* C, const float* initial_states,
+                  const void* B_prev, const void* U_prev, void* Y, const ScanLast& last, int batch, int heads, int groups, int T,
+                  int P, int N, int chunk, int io_dtype, int path, void* workspace, size_t workspace_bytes, void* stream) {
+  const ScanDims d{batch, heads, groups, T, P, N, chunk};
+  if (int e = check_scan(U, M, K, B, C, B_prev, U_prev, d, io_dtype)) return e;
+  if (!Y || !last.state || !last.B || !last.U) return SL_ERR_NULL_POINTER;
+  if (!aligned(Y, 16) || !aligned(last.state, 16) || !aligned(last.B, 16) || !aligned(last.U, 16)) return SL_ERR_BAD_ALIGNMENT;
+  if (!use_tc(path, d, io_dtype)) return SL_ERR_UNSUPPORTED;
+  return scan_tc_fwd(U, M, K, B, C, initial_states, B_prev, U_prev, Y, nullptr, nullptr, d, io_dtype, io_dtype, workspace,
+                     workspace_bytes, reinterpret_cast<cudaStream_t>(stream), &last);
+}
 }  // namespace sl
 
 extern "C" int sl_version(void) { return 100; }

@@ -98,6 +98,29 @@ std::tuple<Tensor, OptT, OptT> scan_fwd(const Tensor& U, const Tensor& M, const 
   return {Y, final_state, states};
 }
 
+// the same with the end state and the last rows of B and U, all in the type of the operands; nothing where the tensor-core path
+// does not run
+c10::optional<std::tuple<Tensor, Tensor, Tensor, Tensor>> scan_fwd_last(const Tensor& U, const Tensor& M, const Tensor& K,
+                                                                        const Tensor& B, const Tensor& C, const OptT& z0, const OptT& Bp,
+                                                                        const OptT& Up, int chunk, int path) {
+  Call call(U, M, K, B, C, z0, Bp, Up);
+  const int batch = U.size(0), heads = U.size(1), T = U.size(2), P = U.size(3), groups = B.size(1), N = B.size(3) / 2;
+  const auto type = U.scalar_type();
+  if ((type != at::kBFloat16 && type != at::kHalf) || P != 64 || (N != 64 && N != 128) || path == SL_PATH_SIMT) return {};
+  const int io = code_of(type);
+  Tensor Y = call.empty({batch, heads, T, P}, type), state = call.empty({batch, heads, P, 2 * N}, type);
+  Tensor B_last = call.empty({batch, groups, 2 * N}, type), U_last = call.empty({batch, heads, P}, type);
+  const size_t n = sl_workspace_bytes(SL_WS_SCAN_FWD, batch, heads, groups, T, P, N, chunk, io, path);
+  OptT ws;
+  if (n) ws = call.bytes(n);
+  const int rc = sl::scan_fwd_last(ptr(U), fptr(M), fptr(K), ptr(B), ptr(C), fptr(z0), ptr(Bp), ptr(Up), mptr(Y),
+                                   sl::ScanLast{mptr(state), mptr(B_last), mptr(U_last)}, batch, heads, groups, T, P, N, chunk, io, path,
+                                   mptr(ws), n, call.stream());
+  if (rc == SL_ERR_UNSUPPORTED) return {};
+  check(rc, "sl_v2x2ssd_fwd");
+  return std::make_tuple(Y, state, B_last, U_last);
+}
+
 std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, OptT, OptT, OptT> scan_bwd(
     const Tensor& U, const Tensor& M, const Tensor& K, const Tensor& B, const Tensor& C, const OptT& z0, const OptT& Bp,
     const OptT& Up, const OptT& states, const OptT& final_state, const OptT& dY, const OptT& dfinal, int chunk, int path) {
@@ -615,7 +638,7 @@ sl::ScanPrepArgs scanprep_args(const MixerShape& s, const MixerWeights& w, const
 
 struct MixerRun {
   Tensor in_w, proj, U, M, K, B, C, Y, normed, out;
-  OptT states, final_state, conv;
+  OptT states, final_state, conv, B_last, U_last;   // the last two, and the state, in x's type
 };
 MixerRun mixer_run(const MixerShape& s, const MixerWeights& w, const Tensor& x, const OptT& conv_in, const OptT& z0, const OptT& Bp,
                    const OptT& Up, bool save_states, bool want_state, const OptT& residual = {}) {
@@ -641,8 +664,18 @@ MixerRun mixer_run(const MixerShape& s, const MixerWeights& w, const Tensor& x, 
   check(sl::scanprep_fwd(scanprep_args(s, w, r.proj, ptr(conv_in), mptr(r.conv)),
                          sl::ScanPrepOut{mptr(r.U), mfptr(r.M), mfptr(r.K), mptr(r.B), mptr(r.C)}, st),
         "sl_scanprep_conv_fwd");
-  std::tie(r.Y, r.final_state, r.states) =
-      scan_fwd(r.U, r.M, r.K, r.B, r.C, z0, Bp, Up, s.chunk, code_of(type), want_state, s.path, save_states);
+  const auto last = want_state && !save_states ? scan_fwd_last(r.U, r.M, r.K, r.B, r.C, z0, Bp, Up, s.chunk, s.path) : c10::nullopt;
+  if (last) {
+    std::tie(r.Y, r.final_state, r.B_last, r.U_last) = *last;
+  } else {
+    std::tie(r.Y, r.final_state, r.states) =
+        scan_fwd(r.U, r.M, r.K, r.B, r.C, z0, Bp, Up, s.chunk, code_of(type), want_state, s.path, save_states);
+    if (want_state && !save_states) {
+      r.final_state = r.final_state->to(type);
+      r.B_last = r.B.select(2, s.T - 1).contiguous();
+      r.U_last = r.U.select(2, s.T - 1).contiguous();
+    }
+  }
   r.normed = call.empty({s.rows(), s.C()}, type);
   check(sl_mixer_tail_fwd(ptr(r.Y), ptr(r.proj), s.pitch(), ptr(r.U), fptr(w.d_skip), ptr(w.norm_w), w.eps, mptr(r.normed), s.batch,
                           s.heads, s.T, s.P, code_of(type), st),
@@ -789,7 +822,7 @@ std::tuple<Tensor, OptT, OptT, OptT, OptT> mixer_infer(const Tensor& x, const st
                          cast(Up, type), false, want_state);
   Tensor out = r.out.view({s.batch, s.T, r.out.size(1)});
   if (!want_state) return {out, {}, {}, {}, {}};
-  return {out, r.conv, r.final_state->to(type), r.B.select(2, s.T - 1).contiguous(), r.U.select(2, s.T - 1).contiguous()};
+  return {out, r.conv, r.final_state, r.B_last, r.U_last};
 }
 
 // ---- FFN branch of a block in training: x + W2 act(W1 norm(x) + b1) + b2 ----------------------------------------------------
@@ -950,6 +983,7 @@ void adamw_step(const std::vector<Tensor>& ps, const std::vector<Tensor>& gs, co
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("scan_fwd", &scan_fwd);
+  m.def("scan_fwd_last", &scan_fwd_last);
   m.def("scan_bwd", &scan_bwd);
   m.def("scan_decode", &scan_decode);
   m.def("scanprep_fwd", &scanprep_fwd);

@@ -9,6 +9,14 @@
 
 namespace sl {
 
+// sl_v2x2ssd_fwd on the tensor-core path for 16-bit operands, that also leaves what a caller carries on from (in the operands'
+// type): the end state (batch, heads, P, 2N), the last row of B (batch, groups, 2N) and of U (batch, heads, P).
+// SL_ERR_UNSUPPORTED where another path would run; nothing is launched then.
+struct ScanLast { void *state, *B, *U; };
+SL_API int scan_fwd_last(const void* U, const float* M, const float* K, const void* B, const void* C, const float* initial_states,
+                         const void* B_prev, const void* U_prev, void* Y, const ScanLast& last, int batch, int heads, int groups,
+                         int T, int P, int N, int chunk, int io_dtype, int path, void* workspace, size_t workspace_bytes, void* stream);
+
 struct MixerStepArgs {
   const void *gate, *value, *params, *bc;   // rows of the in_proj output, with their row strides (elements)
   int64_t gate_stride, value_stride, params_stride, bc_stride;

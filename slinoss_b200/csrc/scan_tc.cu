@@ -34,6 +34,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "host_abi.h"
 #include "tc_common.cuh"
 
 namespace sl {
@@ -356,7 +357,7 @@ int run_fwd(TcFwdParams& p, const ScanDims& d, int y_dtype, cudaStream_t st) {
 int scan_tc_fwd_impl(const void* U, const float* M, const float* K, const void* B, const void* C, const float* z0,
                      const void* Bprev, const void* Uprev, void* Y, float* zfinal, void* states16,
                      const ScanDims& d, const SegPlan& plan, uint8_t* seg_ws, int io_dtype, int y_dtype,
-                     cudaStream_t st) {
+                     cudaStream_t st, const ScanLast* last = nullptr) {
   TcFwdParams p{};
   ensure_context();
   const bool bf = io_dtype == SL_BF16;
@@ -366,6 +367,7 @@ int scan_tc_fwd_impl(const void* U, const float* M, const float* K, const void* 
     return SL_ERR_LAUNCH_FAILED;
   p.M = M; p.K = K; p.z0 = z0; p.Bprev = Bprev; p.Uprev = Uprev; p.Y = Y; p.zfinal = zfinal;
   p.states16 = states16;
+  if (last) { p.state_last = last->state; p.B_last = last->B; p.U_last = last->U; p.U = U; p.B = B; }
   p.heads = d.heads; p.groups = d.groups; p.T = d.T; p.nchunks = chunks_of(d);
   p.nseg = plan.nseg; p.cps = plan.cps;
   if (plan.nseg > 1) {
@@ -424,14 +426,14 @@ size_t scan_tc_states_bytes(const ScanDims& d) {   // two column blocks: one aft
 int scan_tc_fwd(const void* U, const float* M, const float* K, const void* B, const void* C,
                 const float* z0, const void* Bprev, const void* Uprev, void* Y, float* zfinal,
                 void* states_out, const ScanDims& d, int io_dtype, int y_dtype, void* ws, size_t ws_bytes,
-                cudaStream_t st) {
+                cudaStream_t st, const ScanLast* last) {
   SegPlan plan = fwd_plan(d);
   if (!ws || ws_bytes < scan_tc_fwd_workspace(d)) {   // N = 64 has always run without: the streams are then walked whole
     if (blocks_of(d) == 2) return SL_ERR_WORKSPACE_TOO_SMALL;
     plan = {1, chunks_of(d), 0, 0};
   }
   return scan_tc_fwd_impl(U, M, K, B, C, z0, Bprev, Uprev, Y, zfinal, states_out, d, plan,
-                          reinterpret_cast<uint8_t*>(ws), io_dtype, y_dtype, st);
+                          reinterpret_cast<uint8_t*>(ws), io_dtype, y_dtype, st, last);
 }
 
 namespace {

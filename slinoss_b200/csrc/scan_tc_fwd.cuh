@@ -43,6 +43,10 @@ struct alignas(64) TcFwdParams {
   const void* Uprev;
   void* Y;
   float* zfinal;        // (BH, 64, 2N) or null
+  // or null: what a caller carries on from, in the operands' type (their conversion and two row copies were launches of 2 to
+  // 2.6 us each behind a prompt of 121 us): the end state, and the last rows of B and U
+  void *state_last, *B_last, *U_last;
+  const void *U, *B;
   void* states16;       // optional (NB, BH, nchunks, 64, 128) 16-bit: conjugated start state of every chunk
   float* seg;           // (BH, nseg, 64, 128 NB) float32: start states (from_seg) or, MODE 1 / 2 pre-pass, results
   float2* seg_pi;       // (BH, nseg): transition product of the segment (pre-pass)
@@ -252,6 +256,13 @@ __global__ void __launch_bounds__(128 * NWQ + 64, NWQ == 2 ? 2 : 1)
       }
     }
     if (p.to_seg && lane == 0) p.seg_pi[(size_t)bh * p.nseg + seg] = make_float2(pr, pi);
+    if (FULL && p.state_last && seg == p.nseg - 1) {   // the last rows, in 16-byte pieces
+      if (lane < D / 8 && bh % (p.heads / p.groups) == 0)
+        reinterpret_cast<uint4*>(p.B_last)[(size_t)bg * (D / 8) + lane] =
+            reinterpret_cast<const uint4*>(p.B)[((size_t)bg * T + T - 1) * (D / 8) + lane];
+      if (lane < 8)
+        reinterpret_cast<uint4*>(p.U_last)[(size_t)bh * 8 + lane] = reinterpret_cast<const uint4*>(p.U)[((size_t)bh * T + T - 1) * 8 + lane];
+    }
   } else if (!worker) {
     // ---- issue warp (one lane): every TMA load and store and every MMA.  The workers never wait for it, only for
     // the commit barriers of the products they read.
@@ -563,15 +574,17 @@ __global__ void __launch_bounds__(128 * NWQ + 64, NWQ == 2 ? 2 : 1)
         *reinterpret_cast<float2*>(dst + (size_t)rowA * 128 * NB + 8 * j) = un2(zz[2 * j]);
         *reinterpret_cast<float2*>(dst + (size_t)rowB * 128 * NB + 8 * j) = un2(zz[2 * j + 1]);
       }
-    } else if (live && p.zfinal && seg == p.nseg - 1) {
+    } else if (live && (p.zfinal || (FULL && p.state_last)) && seg == p.nseg - 1) {
 #pragma unroll
       for (int m = 0; m < ZB / 2; ++m) {
         const int nn = n_of(m);
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           const float2 re = un2(zz[4 * m + hh]), im = un2(zz[4 * m + 2 + hh]);
-          *reinterpret_cast<float4*>(p.zfinal + ((size_t)bh * 64 + (hh ? rowB : rowA)) * D + 2 * nn) =
-              make_float4(re.x, -im.x, re.y, -im.y);
+          const size_t at = ((size_t)bh * 64 + (hh ? rowB : rowA)) * D + 2 * nn;
+          if (p.zfinal) *reinterpret_cast<float4*>(p.zfinal + at) = make_float4(re.x, -im.x, re.y, -im.y);
+          if (FULL && p.state_last)
+            *reinterpret_cast<uint2*>(reinterpret_cast<TIn*>(p.state_last) + at) = make_uint2(PK::pack(re.x, -im.x), PK::pack(re.y, -im.y));
         }
       }
     }

@@ -262,6 +262,10 @@ def v2x2ssd_cute(U, M, K, B, C, *, chunk_size, initial_states=None, B_prev=None,
         return _ScanFn.apply(U, M, K, B, C, initial_states, B_prev, U_prev, int(chunk_size),
                              odtype, bool(return_state), path, bool(save_chunk_states))
     args = _prep(U, M, K, B, C, initial_states, B_prev, U_prev)
+    if return_state and odtype is args[0].dtype:
+        last = _C.scan_fwd_last(*args, chunk_size=int(chunk_size), path=path)
+        if last is not None:
+            return last
     y_dtype = odtype if odtype in _IO_DTYPES else torch.float32
     Y, final = _C.scan_fwd(*args, chunk_size=int(chunk_size), y_dtype=y_dtype,
                            want_final=return_state, path=path)

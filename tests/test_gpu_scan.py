@@ -11,6 +11,7 @@ import pytest
 import torch
 
 from oracle import scan_np
+from slinoss_b200 import _C
 from slinoss_b200.ops.v2x2ssd import v2x2ssd, v2x2ssd_cute, v2x2ssd_decode
 from slinoss_b200.synthetic import make_scan_case
 from tests.util import n64, rel, tol
@@ -417,3 +418,17 @@ def test_tensor_core_path_at_small_transition_radius(dtype, lo, hi, bar_dm):
     for name, g in zip("UMKBC", grads):
         assert torch.isfinite(g).all(), name
         assert rel(g, want[name]) <= (bar_dm if name == "M" else 2e-2), (name, rel(g, want[name]))
+
+
+@pytest.mark.parametrize("b, h, g, T, N", [(1, 2, 1, 1, 64), (2, 4, 4, 64, 128), (1, 6, 2, 200, 64), (1, 16, 16, 1500, 64),
+                                           (10, 30, 5, 65, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_what_a_prompt_carries_on_from(b, h, g, T, N, dtype):
+    """The end state in the operands' type and the last rows of B and U, written by the forward kernel: the rows exactly, the
+    state exactly the rounding of the float32 one (whole and split streams, shared B/C)."""
+    c = make_scan_case(b, h, T, 64, N, groups=g, dtype=dtype, seed=T).to("cuda")
+    with torch.no_grad():
+        Y, state, B_last, U_last = v2x2ssd(c.U, c.M, c.K, c.B, c.C, chunk_size=64)
+    want_Y, want = _C.scan_fwd(c.U, c.M, c.K, c.B, c.C, None, None, None, chunk_size=64, y_dtype=dtype, want_final=True)
+    assert torch.equal(Y, want_Y) and torch.equal(state, want.to(dtype)) and state.dtype == dtype
+    assert torch.equal(B_last, c.B[:, :, -1]) and torch.equal(U_last, c.U[:, :, -1]) and B_last.is_contiguous()
