@@ -175,6 +175,9 @@ __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.la
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- host side -----------------------------------------------------------------
+// remembers the CUDA error behind the last SL_ERR_LAUNCH_FAILED (see sl_last_cuda_error)
+void note_cuda_error(int code);
+
 template <typename K, typename A, typename... As>
 inline int launch_chained(K kernel, dim3 grid, unsigned block, size_t smem, cudaStream_t st, bool dependent, const A& a,
                           const As&... as) {
@@ -184,7 +187,11 @@ inline int launch_chained(K kernel, dim3 grid, unsigned block, size_t smem, cuda
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid; cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cfg.attrs = &attr; cfg.numAttrs = dependent ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, a, as...) == cudaSuccess ? SL_OK : SL_ERR_LAUNCH_FAILED;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, as...);
+  if (e == cudaSuccess) return SL_OK;
+  cudaGetLastError();
+  note_cuda_error((int)e);
+  return SL_ERR_LAUNCH_FAILED;
 }
 
 inline size_t dtype_size(int dt) { return dt == SL_F32 ? 4 : 2; }
@@ -194,9 +201,6 @@ inline size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // process-wide count of kernels this library has launched (see sl_kernel_launches)
 void note_launches(int n);
-
-// remembers the CUDA error behind the last SL_ERR_LAUNCH_FAILED (see sl_last_cuda_error)
-void note_cuda_error(int code);
 
 inline int launch_status() {
   const cudaError_t e = cudaGetLastError();

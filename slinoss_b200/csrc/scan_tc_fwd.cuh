@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(128 * NWQ + 64, NWQ == 2 ? 2 : 1)
   const long long wl = p.wait_limit;
   auto chunk_of = [&](int i) { return ADJ ? c0 + n - 1 - i : c0 + i; };
 
+  if (!FULL) grid_release();   // (a pre-pass: what follows it may start up meanwhile)
   if (tid == 0) {
     mbar_init(&bar_u[0], 1); mbar_init(&bar_u[1], 1); mbar_init(&bar_bc[0], 1); mbar_init(&bar_bc[1], 1);
     for (int i = 0; i < 3; ++i) mbar_init(&bar_mma[i], 1);
@@ -179,6 +180,7 @@ __global__ void __launch_bounds__(128 * NWQ + 64, NWQ == 2 ? 2 : 1)
   }
   // start state of a later segment: given, or folded from the earlier segments' contributions
   if (worker && p.from_seg) {
+    grid_wait();
     const size_t stride = (size_t)64 * 128 * NB;
     const float* src = p.seg + (size_t)bh * p.nseg * stride + ZC * cg + 2 * cq;
     const bool fold = p.from_seg == 2;
@@ -609,6 +611,7 @@ __global__ void __launch_bounds__(256) scan_tc_combine_kernel(float* __restrict_
                                                               int heads, int groups, int T, int N, int nseg) {
   const int e = blockIdx.y * 256 + threadIdx.x, bh = blockIdx.x;
   const int row = e / N, n = e % N;
+  grid_release();
   if (row >= 64) return;
   float zr = 0.f, zi = 0.f;
   if (init) {
@@ -628,6 +631,7 @@ __global__ void __launch_bounds__(256) scan_tc_combine_kernel(float* __restrict_
   const size_t stride = (size_t)64 * 2 * N;
   float* base = seg + (size_t)bh * nseg * stride + (size_t)row * 2 * N + (n >> 3) * 16 + (n & 7);
   const float2* pis = seg_pi + (size_t)bh * nseg;
+  grid_wait();
   for (int k0 = 0; k0 < nseg; k0 += 8) {
     float fr[8], fi[8];
     float2 pi[8];
