@@ -3,6 +3,7 @@
 // is kept), as the reference does: block_ffn_residual, slinoss/ops/block/training.py:193-354, with the
 // kernels of slinoss/ops/block/cute/norm.py:85,173 and activation.py:78,153.  The two GEMMs stay library
 // calls in the caller.  All four kernels are HBM-bound: 16-byte accesses, one pass over their rows.
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -240,6 +241,92 @@ template <bool FAST> __device__ __forceinline__ float dgelu_tanh_f(float x) {
   return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * 0.7978845608028654f * (1.f + 3.f * 0.044715f * x * x);
 }
 
+// The same for rows of up to 3 pieces per lane: their sums over the rows stay in registers, the weight too.  In shared memory the sums cost a 32-byte read and write per piece and row, and the
+// general kernel's eight pieces were mostly predicated off: 8192 rows x 576 bf16 19.6 -> 12 us in a training step
+// (28 MB: 4.4; with the extra gradient and its sums 38 MB and 14.7 us).  What is left is one row's latency per turn and the atomics.
+template <typename T, int MAXP, bool SUM>
+__global__ void __launch_bounds__(512, 1) rmsnorm_bwd_narrow_kernel(const T* __restrict__ x, const T* __restrict__ w,
+                                                                 const T* __restrict__ dy, T* __restrict__ dx, float* __restrict__ dw,
+                                                                 double* __restrict__ dw64, const T* __restrict__ extra,
+                                                                 double* __restrict__ extra_sum, long long rows, int C, float eps) {
+  constexpr int V = Vec16<T>::N;
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  float* const s_sum = reinterpret_cast<float*>(s_raw);   // [warps][C]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, pieces = C / V;
+  uint4 wr[MAXP];
+  f2 sw[MAXP][V / 2], se[SUM ? MAXP : 1][V / 2];
+#pragma unroll
+  for (int i = 0; i < MAXP; ++i) {
+    wr[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (lane + 32 * i < pieces) wr[i] = reinterpret_cast<const uint4*>(w)[lane + 32 * i];
+#pragma unroll
+    for (int k = 0; k < V / 2; ++k) { sw[i][k] = 0ull; if (SUM) se[i][k] = 0ull; }
+  }
+  for (long long row = (long long)blockIdx.x * nw + warp; row < rows; row += (long long)gridDim.x * nw) {
+    uint4 xc[MAXP], gc[MAXP], ec[MAXP];
+#pragma unroll
+    for (int i = 0; i < MAXP; ++i) {
+      const int pc = lane + 32 * i;
+      xc[i] = gc[i] = ec[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (pc >= pieces) continue;
+      xc[i] = reinterpret_cast<const uint4*>(x + row * C)[pc];
+      gc[i] = reinterpret_cast<const uint4*>(dy + row * C)[pc];
+      if (extra) ec[i] = reinterpret_cast<const uint4*>(extra + row * C)[pc];
+    }
+    float ss = 0.f, dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < MAXP; ++i) {
+      float xv[V], gv[V], wv[V];
+      unpack16<T>(xc[i], xv); unpack16<T>(gc[i], gv); unpack16<T>(wr[i], wv);
+#pragma unroll
+      for (int k = 0; k < V; ++k) { ss += xv[k] * xv[k]; dot += gv[k] * wv[k] * xv[k]; }
+    }
+    ss = warp_sum(ss); dot = warp_sum(dot);
+    const float rstd = rsqrtf(ss / (float)C + eps);
+    const float coef = dot * rstd * rstd / (float)C;     // mean(g xhat) rstd
+    const f2 r2 = dup2(rstd), c2 = dup2(-coef);
+#pragma unroll
+    for (int i = 0; i < MAXP; ++i) {
+      float xv[V], gv[V], wv[V], ev[V], o[V];
+      unpack16<T>(xc[i], xv); unpack16<T>(gc[i], gv); unpack16<T>(wr[i], wv);
+      if (extra) unpack16<T>(ec[i], ev);
+#pragma unroll
+      for (int k = 0; k < V / 2; ++k) {
+        const f2 x2 = mk2(xv[2 * k], xv[2 * k + 1]), g2 = mk2(gv[2 * k], gv[2 * k + 1]), w2 = mk2(wv[2 * k], wv[2 * k + 1]);
+        sw[i][k] = fma2(g2, mul2(x2, r2), sw[i][k]);
+        f2 d = mul2(r2, fma2(x2, c2, mul2(g2, w2)));
+        if (extra) {
+          const f2 e2 = mk2(ev[2 * k], ev[2 * k + 1]);
+          d = add2(d, e2);
+          if (SUM) se[i][k] = add2(se[i][k], e2);
+        }
+        const float2 q = un2(d);
+        o[2 * k] = q.x; o[2 * k + 1] = q.y;
+      }
+      if (lane + 32 * i < pieces) store16<T>(dx + row * C + (lane + 32 * i) * V, o);
+    }
+  }
+#pragma unroll
+  for (int part = 0; part < (SUM ? 2 : 1); ++part) {
+#pragma unroll
+    for (int i = 0; i < MAXP; ++i)
+      if (lane + 32 * i < pieces)
+#pragma unroll
+        for (int k = 0; k < V / 2; ++k)
+          *reinterpret_cast<f2*>(s_sum + (size_t)warp * C + (lane + 32 * i) * V + 2 * k) = part ? se[SUM ? i : 0][k] : sw[i][k];
+    __syncthreads();
+    for (int c = threadIdx.x; c < C; c += blockDim.x) {
+      double v = 0.0;
+      for (int q = 0; q < nw; ++q) v += s_sum[(size_t)q * C + c];
+      if (part) atomicAdd(extra_sum + c, v);
+      else if (dw64) atomicAdd(dw64 + c, v);   // the order of these adds is lost in the rounding to the result's type
+      else atomicAdd(dw + c, (float)v);
+    }
+    __syncthreads();
+  }
+}
+
+
 // kind 0: hidden = gelu_tanh(projected) (same width).  kind 1 (SwiGLU): projected = [value | gate] of
 // width 2 H per row, hidden = value * silu(gate).  One 16-byte piece of the hidden row per thread.
 template <typename T>
@@ -396,13 +483,29 @@ int rmsnorm_bwd(const void* x, const void* weight, float eps, const void* d_out,
   if (!dtype_ok(io_dtype)) return SL_ERR_UNSUPPORTED;
   if (!rows_ok(rows, C, io_dtype, x, d_x) || !aligned(weight, 16) || !aligned(d_out, 16) || !aligned(extra, 16)) return SL_ERR_BAD_SHAPE;
   const long long want = (rows + 7) / 8;
-  const bool narrow = C / (io_dtype == SL_F32 ? 4 : 8) <= 32 * RMS_MAXP_NARROW;
-  const long long cap = narrow ? 148 * 4 : 148 * 2;   // CTAs that walk the rows: all resident at once
-  const unsigned grid = (unsigned)(want < cap ? want : cap);
+  const int lanes = (C / (io_dtype == SL_F32 ? 4 : 8) + 31) / 32;   // pieces per lane
   if (extra_sum && (!extra || !rmsnorm_bwd_sums_extra(C))) return SL_ERR_UNSUPPORTED;
+  if (lanes <= 3) {
+    const unsigned grid = (unsigned)std::min<long long>((rows + 15) / 16, 148);   // 16 warps each: half the atomics of 8
+    SL_DISPATCH_DTYPE(io_dtype, T, {
+      const T *tx = reinterpret_cast<const T*>(x), *tw = reinterpret_cast<const T*>(weight), *td = reinterpret_cast<const T*>(d_out);
+      const T* te = reinterpret_cast<const T*>(extra);
+      T* to = reinterpret_cast<T*>(d_x);
+      auto kern = extra_sum ? (lanes <= 2 ? rmsnorm_bwd_narrow_kernel<T, 2, true> : rmsnorm_bwd_narrow_kernel<T, 3, true>)
+                            : (lanes <= 2 ? rmsnorm_bwd_narrow_kernel<T, 2, false> : rmsnorm_bwd_narrow_kernel<T, 3, false>);
+      const size_t smem = (size_t)16 * C * sizeof(float);
+      if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return SL_ERR_LAUNCH_FAILED;
+      kern<<<grid, 512, smem, st>>>(tx, tw, td, to, d_weight, weight64, te, extra_sum, rows, C, eps);
+    });
+    note_launches(1);
+    return launch_status();
+  }
+  const long long cap = 148 * 2;   // CTAs that walk the rows: all resident at once
+  const unsigned grid = (unsigned)(want < cap ? want : cap);
   const size_t smem = (size_t)(extra_sum ? 16 : 8) * C * sizeof(float) + (size_t)C * dtype_size(io_dtype);   // 8 warps' rows + w
   SL_DISPATCH_DTYPE(io_dtype, T, {
-    auto kern = narrow ? rmsnorm_bwd_kernel<T, RMS_MAXP_NARROW> : rmsnorm_bwd_kernel<T, RMS_MAXP>;
+    auto kern = rmsnorm_bwd_kernel<T, RMS_MAXP>;
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return SL_ERR_LAUNCH_FAILED;
