@@ -216,6 +216,8 @@ def scan_fwd(U, M, K, B, C, z0, B_prev, U_prev, *, chunk_size, y_dtype, want_fin
 def scan_fwd_last(U, M, K, B, C, z0, B_prev, U_prev, *, chunk_size, path="auto"):
     """The forward scan of 16-bit operands with what a caller carries on from, all in their type: ``(Y, final_state, B_last,
     U_last)``.  None where the tensor-core path does not run."""
+    if U.dtype is torch.float32 or not U.is_cuda:
+        return None
     return host().scan_fwd_last(U, M, K, B, C, z0, B_prev, U_prev, chunk_size, _PATHS[path])
 
 
