@@ -214,7 +214,7 @@ class _ScanFn(torch.autograd.Function):
             if dY is not None:
                 if half and dY.dtype != U.dtype:
                     # a float32 output was asked of 16-bit operands: the tensor-core sweep takes dY as a 16-bit
-                    # operand like U, B and C (the exact sweeps would keep it in float32 at ~20x the time)
+                    # operand like U, B and C (the float32 sweeps would keep it at several times the time)
                     dY = dY.to(U.dtype)
                 elif dY.dtype not in _IO_DTYPES:
                     dY = dY.to(torch.float32)
@@ -233,7 +233,8 @@ class _ScanFn(torch.autograd.Function):
             out[0][:, :, -1, :].add_(dU_last.to(dtype=out[0].dtype))
         res = []
         for g, dt, need in zip(out, ctx.in_dtypes, ctx.needs_input_grad[:8]):
-            res.append(g.to(dtype=dt) if (g is not None and dt is not None and need) else None)
+            g = g if g is not None and dt is not None and need else None
+            res.append(g if g is None or g.dtype is dt else g.to(dtype=dt))
         return (*res, None, None, None, None, None)
 
 
