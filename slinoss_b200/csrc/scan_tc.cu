@@ -1,8 +1,8 @@
 // Chunked v2x2ssd scan on the 5th-generation tensor cores (tcgen05 + TMEM + TMA).
 //
 // Supported: P = 64, N = 64 or 128 (blocks of 64 oscillators, 128 real columns), bf16 or fp16 operands, float32 state.
-// Everything else takes the exact SIMT path.  (Narrower N would fit with zero columns and run 17 times faster than
-// there, fp16 forward + backward of 64 streams x 2048 tokens x N = 48: 174 against 2976 us; but the products round
+// Everything else takes the float32 path.  (Narrower N would fit with zero columns and run 4 times faster than
+// there, fp16 forward + backward of 64 streams x 2048 tokens x N = 48: 174 against 663 us; but the products round
 // their operands to 16 bits and need every |m| > 0, which the exact sweeps that these widths have always had do not.)
 //
 // Formulation (per (batch, head); chunk of L = 64 tokens, local index t, s).  The two
