@@ -516,12 +516,12 @@ class TokenPlan {
       check(sl::skinny_linear(o, st), "skinny_linear");
       return py::make_tuple(out, b_next, ws);
     }
-    // A block: the bits of the library's products at the shapes of the composed path.  Any other order of their sums moves last
-    // bits, which residual stream, norms and B/C phases carry on from block to block: six blocks of width 1024 end up 1.6 % from the
-    // composed token.  token_linear adds in the library's order, with residual and activation inside; what it does not take (more than
-    // 64 rows, widths that are no multiple of 8) goes to the library, there without a dispatch.  A token of four blocks of width 512
-    // at batch 8 is bound by the host: 398 us with 24 library products and 29 other launches, 146 with 5 launches a block (the host needs 123; 8 launches, the norms by
-    // themselves: 184).
+    // A block: five launches where token_linear takes its products, with norm, residual and activation inside; what it does not
+    // take (more than 64 rows, widths that are no multiple of 8) goes to the library.  The outputs have the bits of the composed
+    // path (tested): residual stream, norms and B/C phases carry a moved last bit on from block to block, up to 1.6 % after one token
+    // of six blocks of width 1024.  A token of four blocks of width 512 at batch 8: 398 us with 24 library products and 29 other
+    // launches, 184 with 8 launches a block (the norms by themselves), 146 with 5: the device's chain of launches bounds it now,
+    // the host needs 123 of it.
     at::AutoDispatchBelowAutograd below;
     auto fresh = [&](int64_t cols) { return at::detail::empty_cuda({M, cols}, type, x.device(), c10::nullopt); };
     auto norm = [&](const Tensor& a, const Tensor& w, double eps) {

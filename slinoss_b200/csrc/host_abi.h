@@ -62,8 +62,7 @@ struct SkinnyArgs {
 SL_API bool skinny_supported(int M, int K, int O, int io_dtype);
 SL_API int skinny_linear(const SkinnyArgs& a, cudaStream_t st);
 
-// One linear layer of a block's token, with the bits of the library's product and of what follows it (token_linear.cu):
-// x (M, K) dense, weight (O, K) dense, M <= 64.
+// One linear layer of a block's token and what follows it (token_linear.cu): x (M, K) dense, weight (O, K) dense, M <= 64.
 struct TokenLinearArgs {
   const void *x, *weight, *bias;   // bias (O) or null
   void* out[3];                    // dense (M, width[i]) each, the columns in turn; swiglu: one of O / 2

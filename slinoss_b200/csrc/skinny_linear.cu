@@ -1,7 +1,7 @@
 // Linear layers of a mixer's decode token: y (M, O) = norm(x) W^T + bias for M <= 64 rows of 16-bit values.
 //
 // Bound by reading W once (O K 2 bytes); at these sizes also by launches, so the row norm in front of the output projection
-// is applied as x is read (its sums of squares come with x).  A library GEMM pads M to its tile and took 4 to 6 us.
+// is applied as x is read (its sums of squares come with x).  A library GEMM took 4 to 6 us.
 //
 // A CTA owns 8 NT output rows; its warps split K in runs of 256.  W is the (n = 8) operand of mma.sync m16n8k16: a
 // lane reads 16 consecutive bytes of one row of W (four lanes cover 64 bytes) and uses them for two k-steps under a

@@ -1,15 +1,16 @@
-// The linear layers of a block's decode token: y = act(x W^T + bias) or residual + x W^T + bias, M <= 64 rows of 16-bit values,
-// with the very bits of the library's product and of the row kernels behind it.
+// The linear layers of a block's decode token: y = act(x W^T + bias) or residual + x W^T + bias, M <= 64 rows of 16-bit values.
 //
-// A block's token has to keep the bits of the composed path (any other order of sums grows from block to block).  For outputs
-// of a multiple of 8 columns the library adds the products of 16 values of k at a time, in turn, on one float32 accumulator,
-// whatever its tile (560 shapes of 1 to 64 rows, k from 64 to 4096, either type, with and without bias; widths that are no
-// multiple of 8 take others and stay with it).  So does a warp here, with mma.sync m16n8k16; the order inside a step of 16
-// does not matter, which lets a lane read 8 consecutive bytes of a row for its four values.
+// An output has one float32 accumulator, and k ascends in the steps of mma.sync m16n8k16: the plain order, the same for every
+// number of rows and every width, so a token does not depend on the batch that it comes in.  (A lane reads 8 consecutive bytes
+// of a row for its four values of a step: within a step the order of k is the instruction's own.)  Rounding points are those of
+// the composed path: the product is rounded to its type before residual, activation or norm.  The tests hold a block's token to
+// the composed path's bits, because a last bit moved here grows from block to block (1.6 % after one token of six blocks of
+// width 1024).  A tile is 8 columns, so widths that are no multiple of 8 are left to the library.
 //
 // What bounds it: the launch.  A library product costs the host 7 to 9 us and a launch of its own for each part of in_proj, the
-// residual, the activation and the norm; here it is 2 to 3 us with all of them inside (norms: up to 16 rows).  On the device: latency of one trip to memory
-// (all of a warp's rows of W are requested at the start, x two pieces ahead) and the chain of K / 16 steps on one accumulator.
+// residual, the activation and the norm; here it is 2 to 3 us with all of them inside (norms: up to 16 rows).  On the device:
+// latency of one trip to memory (all of a warp's rows of W are requested at the start, x two pieces ahead) and the chain of
+// K / 16 steps on one accumulator.
 #include "common.cuh"
 #include "host_abi.h"
 
@@ -27,7 +28,7 @@ template <> __device__ __forceinline__ void mma16816<__half>(float (&d)[4], cons
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// rounded as the library and torch's sums round (no saturation)
+// rounded as torch's sums round (no saturation)
 template <typename T> __device__ __forceinline__ float rounded(float v);
 template <> __device__ __forceinline__ float rounded<__nv_bfloat16>(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 template <> __device__ __forceinline__ float rounded<__half>(float v) { return __half2float(__float2half_rn(v)); }
@@ -244,7 +245,7 @@ int launch_token(const TokenLinearArgs& a, int nw, size_t smem, cudaStream_t st)
 
 }  // namespace
 
-// Widths that are no multiple of 8 are the library's (its kernels for them sum in another order).
+// Whole tiles of 8 columns, rows of W that start on 16 bytes.
 bool token_linear_supported(const TokenLinearArgs& a) {
   size_t smem;
   if (a.M < 1 || a.M > 64 || a.K < 8 || a.K % 8 || a.O < 8 || a.O % (a.swiglu ? 16 : 8) || (a.io_dtype != SL_BF16 && a.io_dtype != SL_F16))
