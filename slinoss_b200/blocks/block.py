@@ -154,17 +154,21 @@ class SLinOSSBlock(nn.Module):
             ffn_eps, kind = _norm_eps(fnorm), _C.FFN_KINDS[ffn.kind]
         return mixer._make_token_plan(branch, (same, empty), _norm_eps(norm), ffn_eps, kind)
 
-    def _native_step(self, token, state, inplace):
+    def _native_step(self, token, state, inplace, behind=False):
         """The whole step through the block's native plan (the composed path's products and kernels as one call), or None when
         something asks for the composed path: gradients, another norm, dropout, autocast, hooks, an injected backend, a
         partial state."""
         if torch.is_grad_enabled() or state is None or not token.is_cuda or (inplace is not None and not inplace) or \
                 (self.residual_dropout > 0.0 and self.training) or type(self.mixer) is not SLinOSSMixer:
             return None
-        out = planned_step(self, token, state.mixer, self._make_token_plan)
+        out = planned_step(self, token, state.mixer, self._make_token_plan, behind)
         return None if out is None else (out, SLinOSSBlockState(mixer=state.mixer))
 
     def step(self, x, state: SLinOSSBlockState | None = None, *, inplace=None, context=None):
+        return self._advance(x, state, inplace)[:2]
+
+    def _advance(self, x, state, inplace, behind=False):
+        """``step``, and whether its last kernel is the plan's own (``behind`` of a block right after this one)."""
         token = x
         if token.ndim == 3:
             if token.shape[1] != 1:
@@ -173,9 +177,9 @@ class SLinOSSBlock(nn.Module):
         if token.ndim != 2 or token.shape[-1] != self.d_model:
             raise ValueError(f"Expected x shape (batch, {self.d_model}) or "
                              f"(batch, 1, {self.d_model}), got {tuple(x.shape)}.")
-        done = self._native_step(token, state, inplace)
+        done = self._native_step(token, state, inplace, behind)
         if done is not None:
-            return done if x.ndim == 2 else (done[0].unsqueeze(1), done[1])
+            return done[0] if x.ndim == 2 else done[0].unsqueeze(1), done[1], True
         normed, carried, mixer = apply_norm(self.mixer_norm, token), None if state is None else state.mixer, self.mixer
         if type(mixer) is SLinOSSMixer and "step" not in mixer.__dict__:
             mixed, mixer_state = mixer._step(normed, carried, inplace, True)
@@ -186,7 +190,9 @@ class SLinOSSBlock(nn.Module):
             out = self._ffn_residual(out)
         if x.ndim == 3:
             out = out.unsqueeze(1)
-        return out, SLinOSSBlockState(mixer=mixer_state)
+        return out, SLinOSSBlockState(mixer=mixer_state), False
 
+
+PLAIN_STEP = SLinOSSBlock.step    # (a replaced method is called)
 
 __all__ = ["SLinOSSBlock", "apply_norm", "make_norm"]

@@ -8,7 +8,7 @@ import torch
 import torch.utils.checkpoint
 from torch import nn
 
-from .block import SLinOSSBlock, apply_norm, make_norm
+from .block import PLAIN_STEP, SLinOSSBlock, apply_norm, make_norm
 from .config import SLinOSSStackConfig
 from .state import SLinOSSStackState
 
@@ -82,10 +82,13 @@ class SLinOSSStack(nn.Module):
         if hidden.ndim != 2 or hidden.shape[-1] != self.d_model:
             raise ValueError(f"Expected hidden shape (batch, {self.d_model}), got {tuple(hidden.shape)}.")
         self._check_state(state)
-        layers = []
+        layers, behind = [], False
         for i, block in enumerate(self.blocks):
-            hidden, nxt = block.step(hidden, None if state is None else state.layers[i],
-                                     inplace=inplace, context=context)
+            carried = None if state is None else state.layers[i]
+            if type(block).step is PLAIN_STEP and "step" not in block.__dict__:
+                hidden, nxt, behind = block._advance(hidden, carried, inplace, behind)
+            else:
+                (hidden, nxt), behind = block.step(hidden, carried, inplace=inplace, context=context), False
             layers.append(nxt)
         hidden = self._final(hidden).to(dtype=x.dtype)
         if x.ndim == 3:

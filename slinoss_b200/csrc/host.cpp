@@ -461,9 +461,10 @@ class TokenPlan {
     };
   }
 
-  // None where the call is not the plain one; else (out, next b_prev, workspace).
+  // None where the call is not the plain one; else (out, next b_prev, workspace).  behind_own: nothing was queued since another
+  // plan's token left its last kernel on this stream.
   py::object step(const Tensor& x, const OptT& conv, const OptT& state, const OptT& b_prev, const OptT& u_prev,
-                  const OptT& workspace) const {
+                  const OptT& workspace, bool behind_own) const {
     if (cleared_ || at::GradMode::is_enabled() || at::autocast::is_autocast_enabled(at::kCUDA) || !x.is_cuda() || x.dim() != 2)
       return py::none();
     const auto type = x.scalar_type();
@@ -523,14 +524,21 @@ class TokenPlan {
     // launches, 184 with 8 launches a block (the norms by themselves), 146 with 5: the device's chain of launches bounds it now,
     // the host needs 123 of it.
     at::AutoDispatchBelowAutograd below;
+    // A product requests its rows of W while the kernel before it still runs, which is sound behind a kernel of this library only:
+    // those write no parameter, and start behind everything that was queued before the token.  What the program has queued in
+    // front of the token, and a library product in it, may write or still wait for a weight.  (Every block's first product an
+    // ordinary launch: 160 us instead of 148 for a token of four blocks of width 512.)
     auto fresh = [&](int64_t cols) { return at::detail::empty_cuda({M, cols}, type, x.device(), c10::nullopt); };
     auto norm = [&](const Tensor& a, const Tensor& w, double eps) {
       Tensor out = fresh(D);
       check(sl_rmsnorm_fwd(ptr(a), ptr(w), (float)eps, mptr(out), M, D, io, st), "sl_rmsnorm_fwd");
+      behind_own = true;
       return out;
     };
     const Tensor rows = x.contiguous();
-    auto product = [](const Tensor& a, const Tensor& W, int64_t row, int64_t n) {   // a (rows row .. row + n of W)^T
+    behind_own = behind_own && x.is_contiguous();
+    auto product = [&](const Tensor& a, const Tensor& W, int64_t row, int64_t n) {   // a (rows row .. row + n of W)^T
+      behind_own = false;
       return at::cuda::mm(a, at::native::as_strided_tensorimpl(W, {W.size(1), n}, {1, W.size(1)}, W.storage_offset() + row * W.size(1)));
     };
     // own kernel with what follows the product inside; false where it is left to the library
@@ -543,10 +551,12 @@ class TokenPlan {
       for (const Tensor* o : out) { t.out[i] = mptr(*o); t.width[i++] = (int)o->size(1); }
       if (norm_w) { t.norm_weight = ptr(*norm_w); t.norm_eps = (float)eps; t.partials = partials; t.n_partials = (int)(8 * heads_); }
       if (!sl::token_linear_supported(t)) return false;
+      t.dependent = behind_own;
       check(sl::token_linear(t, st), "token_linear");
-      return true;
+      return behind_own = true;
     };
     auto linear = [&](const Tensor& a, const Tensor& W, const OptT& bias) {
+      behind_own = false;
       return bias ? at::linear(a, W, bias) : product(a, W, 0, W.size(0));
     };
     // residual + linear
@@ -555,6 +565,7 @@ class TokenPlan {
       if (fused(ptr(a), W, 0, D, bias, {&out}, &residual)) return out;
       const Tensor branch = linear(a, W, bias);
       check(sl::rmsnorm_fwd_sum(ptr(residual), ptr(branch), mptr(out), nullptr, 0.f, nullptr, M, D, io, st), "sl_rmsnorm_fwd");
+      behind_own = true;
       return out;
     };
     const int64_t n_gv = 2 * C, n_par = 3 * heads_, n_bc = 4 * groups_ * N_;
@@ -568,6 +579,7 @@ class TokenPlan {
       }
     }
     mixer_step(gv.data_ptr(), column(gv, C), params.data_ptr(), bc.data_ptr(), n_gv, n_par, n_bc, false);
+    behind_own = true;
     Tensor out = fresh(D);
     if (!fused(base, *p_[10], 0, D, p_[11], {&out}, &rows, -1, &*p_[9], eps_[1], sl::step_partials(base, M, heads_, P_))) {
       const Tensor hid = fresh(C);

@@ -75,6 +75,7 @@ struct TokenLinearArgs {
   float norm_eps = 0.f;
   const float* partials = nullptr;
   int n_partials = 0;
+  bool dependent = false;          // launched right behind a kernel of this library (which writes no parameter)
 };
 SL_API bool token_linear_supported(const TokenLinearArgs& a);
 SL_API int token_linear(const TokenLinearArgs& a, cudaStream_t st);

@@ -225,7 +225,7 @@ int launch_token_as(const TokenLinearArgs& a, int nw, size_t smem, cudaStream_t 
   static std::atomic<unsigned long long> done{0};
   if (int e = ensure_smem(token_linear_kernel<T, MT, NT, NORM>, 200 * 1024, done)) return e;
   const int tiles = a.O / NT / 8;
-  return launch_chained(token_linear_kernel<T, MT, NT, NORM>, dim3((tiles + nw - 1) / nw), (unsigned)(NORM ? 256 : 32 * nw), smem, st, true, a, nw);
+  return launch_chained(token_linear_kernel<T, MT, NT, NORM>, dim3((tiles + nw - 1) / nw), (unsigned)(NORM ? 256 : 32 * nw), smem, st, a.dependent, a, nw);
 }
 template <typename T, int MT>
 int launch_token_m(const TokenLinearArgs& a, int nw, size_t smem, cudaStream_t st) {

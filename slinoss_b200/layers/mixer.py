@@ -33,9 +33,10 @@ def _norm_eps(norm: nn.RMSNorm) -> float:
 
 
 @_C.opaque
-def planned_step(module: nn.Module, token: torch.Tensor, state: SLinOSSMixerState, make):
+def planned_step(module: nn.Module, token: torch.Tensor, state: SLinOSSMixerState, make, behind: bool = False):
     """One token through the module's native plan (made by ``make`` and kept while its guards hold), ``state`` updated in
-    place; None where the call needs the composed path."""
+    place; None where the call needs the composed path.  ``behind``: the last thing queued on the stream is another plan's
+    token, which this one's first kernel may then overlap."""
     plan = module.__dict__.get("_token_plan")
     if plan is None or not plan.valid(module.__dict__):
         plan = make()
@@ -43,7 +44,8 @@ def planned_step(module: nn.Module, token: torch.Tensor, state: SLinOSSMixerStat
             return None
         module.__dict__["_token_plan"] = plan
     scan = state.scan
-    done = plan.step(token, state.conv, scan.state, scan.b_prev, scan.u_prev, state.__dict__.get("_plan_workspace"))
+    done = plan.step(token, state.conv, scan.state, scan.b_prev, scan.u_prev, state.__dict__.get("_plan_workspace"),
+                     behind)
     if done is None:
         return None
     out, scan.b_prev, state._plan_workspace = done

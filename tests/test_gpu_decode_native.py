@@ -3,6 +3,7 @@ kernels, pipelined state update) against the composed path: library GEMMs, row k
 and tail as launches of their own."""
 
 import copy
+import ctypes
 import pickle
 
 import pytest
@@ -237,3 +238,52 @@ def test_token_products_have_the_librarys_bits(batch, d_model, dtype, d_head, ki
     for b in stack.blocks:
         b.__dict__.pop("_token_plan", None)
     assert all(planned) and torch.equal(got, run())
+
+
+# widths whose products are all the kernel's own, and one with a part left to the library (3 heads of 9) behind 16-row norms
+@pytest.mark.parametrize("batch, d_model, by_block", [(4, 512, False), (24, 512, False), (24, 576, False), (4, 512, True)])
+def test_a_block_token_overlaps_only_kernels_of_this_library(batch, d_model, by_block):
+    """A product that requests its weight ahead of its predecessor's end follows one of this library's kernels: what the program
+    queued before the token, and a library product inside it, may write the weight or wait for it.  (Read from the edges of a
+    captured token behind an update of the first weight; by_block: in a loop of the program's own, of every block's.)"""
+    from cuda.bindings import driver
+
+    def ok(result):
+        assert result[0] == driver.CUresult.CUDA_SUCCESS, result[0]
+        return result[1:]
+
+    def name(node):
+        params, = ok(driver.cuGraphKernelNodeGetParams(node))
+        got = driver.cuFuncGetName(params.func) if int(params.func) else driver.cuKernelGetName(params.kern)
+        return ok(got)[0].decode()
+
+    cfg = sb.SLinOSSBlockConfig(d_model=d_model, mixer=sb.SLinOSSMixerConfig(d_state=64, d_head=64, expand=1.0),
+                                ffn=sb.SLinOSSMLPConfig(kind="gelu", expand=2.0, multiple_of=8))
+    stack = sb.SLinOSSStack(sb.SLinOSSStackConfig.uniform(cfg, n_layers=2), device=DEV, dtype=torch.bfloat16).eval()
+    x = torch.randn(batch, d_model, device=DEV, dtype=torch.bfloat16)
+
+    def token(state):
+        if not by_block:
+            stack.blocks[0].mixer.in_proj.weight.data.mul_(1.0)
+            return stack.step(x, state)
+        hidden = x
+        for block, carried in zip(stack.blocks, state.layers):
+            block.mixer.in_proj.weight.data.mul_(1.0)
+            hidden, _ = block.step(hidden, carried)
+
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.no_grad():
+        state = stack.init_decode_state(batch)
+        with torch.cuda.stream(side):
+            token(state)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            token(state)
+    raw, count = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
+    edges = ctypes.CDLL("libcuda.so.1").cuGraphGetEdges_v2     # (the binding's edge data does not outlive its call)
+    assert edges(raw, None, None, None, ctypes.byref(count)) == 0
+    sources, targets, data = (ctypes.c_void_p * count.value)(), (ctypes.c_void_p * count.value)(), (ctypes.c_uint8 * 8 * count.value)()
+    assert edges(raw, sources, targets, data, ctypes.byref(count)) == 0
+    programmatic = driver.CUgraphDependencyType.CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC.value
+    early = [name(driver.CUgraphNode(s)) for s, d in zip(sources, data) if d[2] == programmatic]    # (ports, then the type)
+    assert len(early) >= 6 and all(n.startswith("_ZN2sl") for n in early), early
