@@ -157,8 +157,9 @@ SL_API int sl_v2x2ssd_bwd(const void* U, const float* M, const float* K, const v
  * minus chunk / path / workspace.  The scratch is a fixed array of
  * SL_STATIC_SCRATCH_BYTES inside the library image, resident on every GPU that loads
  * the library until the process exits.  Limits and rules:
- *   - a problem needing more scratch (about batch*heads*T*(24*N+8) bytes) is refused
- *     with SL_ERR_STATIC_SCRATCH_EXCEEDED and nothing is launched;
+ *   - a problem with batch*heads*(T*(24*N+8) + 8) bytes above the array's is refused
+ *     with SL_ERR_STATIC_SCRATCH_EXCEEDED and nothing is launched (an upper bound of what
+ *     any problem of these sizes uses);
  *   - every call shares the array, so calls whose kernels can overlap on the GPU
  *     race: keep them on one stream or otherwise serialised;
  *   - the array keeps the previous call's contents; each call itself clears the

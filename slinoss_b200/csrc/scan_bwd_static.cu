@@ -10,7 +10,7 @@
 // Consequences the caller has to know:
 //  * the array (SL_STATIC_SCRATCH_BYTES) is resident on every GPU that loads the
 //    library, from load until the process exits;
-//  * problems whose scratch need exceeds it are refused with
+//  * problems above the bound that the header states by size are refused with
 //    SL_ERR_STATIC_SCRATCH_EXCEEDED - nothing is launched;
 //  * all calls share the one array: two calls whose kernels overlap on the GPU
 //    (different streams, different host threads) race on it.  Serialise them;
@@ -72,8 +72,9 @@ extern "C" int sl_v2x2ssd_bwd_static(const void* U, const float* M, const float*
   if (!aligned(M, 8) || !aligned(K, 16)) return SL_ERR_BAD_ALIGNMENT;
   const ScanDims d{batch, heads, groups, T, P, N, 64};
   if (!scan_simt_supported(d)) return SL_ERR_UNSUPPORTED;
-  const size_t need = scan_simt_bwd_workspace(d);
-  if (need > (size_t)SL_STATIC_SCRATCH_BYTES) return SL_ERR_STATIC_SCRATCH_EXCEEDED;
+  // The limit is a rule of the problem's size alone, at least what the sweeps use (equal to it for one token of shared B and C).
+  const size_t bh = (size_t)batch * heads;
+  if (round_up(bh * T * (24 * (size_t)N + 8) + 8 * bh, 256) > (size_t)SL_STATIC_SCRATCH_BYTES) return SL_ERR_STATIC_SCRATCH_EXCEEDED;
   void* scratch = nullptr;
   if (int e = scratch_address(&scratch)) return e;
   return scan_simt_bwd(U, M, K, B, C, initial_states, B_prev, U_prev, dY, d_final_state, dU, dM,

@@ -1402,11 +1402,14 @@ int scan_simt_fwd(const void* U, const float* M, const float* K, const void* B, 
   return rc;
 }
 
-// workspace layout: sterm (batch*heads*T*2) | sT (batch*heads*2) | where heads or slices of P are summed by the last launch:
-//                   dB | dC (each batch*heads*T*2N floats) | dB_prev (batch*heads*2N) | the segments of the two sweeps
+// heads or slices of P are summed by the last launch
+bool spread_of(const ScanDims& d) { return d.groups != d.heads || d.P > ROWS; }
+
+// workspace layout: sterm (batch*heads*T*2) | sT (batch*heads*2) | where spread: dB | dC (each batch*heads*T*2N floats) |
+//                   dB_prev (batch*heads*2N) | the segments of the two sweeps
 size_t scan_simt_bwd_workspace(const ScanDims& d) {
-  const size_t bht = (size_t)d.batch * d.heads * d.T;
-  return round_up(4 * (3 * bht * 2 * d.N + bht * 2 + (size_t)d.batch * d.heads * 2), 256);
+  const size_t bh = (size_t)d.batch * d.heads, bht = bh * d.T, D = 2 * (size_t)d.N;
+  return round_up(4 * (bht * 2 + bh * 2 + (spread_of(d) ? 2 * bht * D + bh * D : 0)), 256);
 }
 size_t scan_simt_bwd_split_workspace(const ScanDims& d) {
   SimtConfig c;
@@ -1430,7 +1433,7 @@ int scan_simt_bwd(const void* U, const float* M, const float* K, const void* B, 
   p.sterm = reinterpret_cast<float*>(ws);
   p.sT = p.sterm + bht * 2;
   p.dB_head = p.sT + bh * 2; p.dC_head = p.dB_head + bht * D; p.dBprev_head = p.dC_head + bht * D;
-  p.spread = d.groups != d.heads || c.ptiles > 1;
+  p.spread = spread_of(d);
   p.dU = dU; p.dB = dB; p.dC = dC; p.dK = dK; p.dM = dM; p.dUprev = dUprev; p.dBprev = dBprev; p.dinit = dinit;
   if (c.ptiles > 1) {  // partial sums of the P tiles are accumulated atomically
     if (cudaMemsetAsync(ws, 0, need, st) != cudaSuccess || cudaMemsetAsync(dK, 0, bht * 16, st) != cudaSuccess ||
