@@ -34,14 +34,19 @@ __device__ __forceinline__ uint4 plain_sum(const uint4& a, const uint4& b) {
   }
 }
 
+// out = a + b (a token's residual behind a product that is left to the library): 16 bytes a thread
+template <typename T>
+__global__ void __launch_bounds__(256) residual_sum_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b,
+                                                           uint4* __restrict__ out, long long pieces) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i < pieces) out[i] = plain_sum<T>(a[i], b[i]);
+}
+
 // out = x * rsqrt(mean(x^2) + eps) * w.  One warp per row; the row stays packed in registers (16-byte
 // pieces, MAXP per lane), so it is read once.
-// add: x is first replaced by x + add rounded to its type (the sum of two tensors as torch forms it: a token's residual),
-// which is kept in sum; without out that is all.
 template <typename T, int MAXP>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w,
-                                                          T* __restrict__ out, long long rows, int C, float eps,
-                                                          const T* __restrict__ add, T* __restrict__ sum) {
+                                                          T* __restrict__ out, long long rows, int C, float eps) {
   constexpr int V = Vec16<T>::N;
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -54,17 +59,6 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const T* __restrict__ 
   for (int i = 0; i < MAXP; ++i) {
     const int pc = lane + 32 * i;
     if (pc < pieces) raw[i] = xr[pc];
-  }
-  if (add) {
-#pragma unroll
-    for (int i = 0; i < MAXP; ++i) {
-      const int pc = lane + 32 * i;
-      if (pc < pieces) {
-        raw[i] = plain_sum<T>(raw[i], reinterpret_cast<const uint4*>(add + row * C)[pc]);
-        reinterpret_cast<uint4*>(sum + row * C)[pc] = raw[i];
-      }
-    }
-    if (!out) return;
   }
 #pragma unroll
   for (int i = 0; i < MAXP; ++i) {
@@ -241,9 +235,12 @@ template <bool FAST> __device__ __forceinline__ float dgelu_tanh_f(float x) {
   return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * 0.7978845608028654f * (1.f + 3.f * 0.044715f * x * x);
 }
 
-// The same for rows of up to 3 pieces per lane: their sums over the rows stay in registers, the weight too.  In shared memory the sums cost a 32-byte read and write per piece and row, and the
-// general kernel's eight pieces were mostly predicated off: 8192 rows x 576 bf16 19.6 -> 12 us in a training step
-// (28 MB: 4.4; with the extra gradient and its sums 38 MB and 14.7 us).  What is left is one row's latency per turn and the atomics.
+// The backward of rows of up to 3 pieces per lane (768 channels of 16-bit rows, 384 of float32): the weight, its gradient and the
+// sums of extra stay in registers.  In shared memory (rmsnorm_bwd_kernel) the sums cost a 32-byte read and write per piece and
+// row.  What is left is one row's latency per turn and the atomics.  us, bf16, in turn with the kernels of 2 and of 8 pieces that
+// these widths had, without / with extra and its sums: 256 rows x 128 4.2 -> 4.2 / 4.4 -> 4.3, 4096 x 256 12.4 -> 6.3 / 14.5 -> 6.4,
+// 8192 x 512 16.5 -> 8.4 / 22.8 -> 10.2, 8192 x 576 13.4 -> 10.5 / 22.8 -> 14.7, 16384 x 768 20.8 -> 14.9 / 43.5 -> 26.7; no
+// width from 128 to 768 at 256 to 16384 rows got slower, in any type.  With three pieces and the sums 200 bytes are spilled.
 template <typename T, int MAXP, bool SUM>
 __global__ void __launch_bounds__(512, 1) rmsnorm_bwd_narrow_kernel(const T* __restrict__ x, const T* __restrict__ w,
                                                                  const T* __restrict__ dy, T* __restrict__ dx, float* __restrict__ dw,
@@ -325,7 +322,6 @@ __global__ void __launch_bounds__(512, 1) rmsnorm_bwd_narrow_kernel(const T* __r
     __syncthreads();
   }
 }
-
 
 // kind 0: hidden = gelu_tanh(projected) (same width).  kind 1 (SwiGLU): projected = [value | gate] of
 // width 2 H per row, hidden = value * silu(gate).  One 16-byte piece of the hidden row per thread.
@@ -454,26 +450,35 @@ extern "C" int sl_rmsnorm_fwd(const void* x, const void* weight, float eps, void
                               int io_dtype, void* stream) {
   using namespace sl;
   if (!x || !weight || !out) return SL_ERR_NULL_POINTER;
-  return rmsnorm_fwd_sum(x, nullptr, nullptr, weight, eps, out, rows, C, io_dtype, reinterpret_cast<cudaStream_t>(stream));
-}
-
-namespace sl {
-// sum = x + add (both null: x itself), out = norm(sum) * weight or null
-int rmsnorm_fwd_sum(const void* x, const void* add, void* sum, const void* weight, float eps, void* out, long long rows, int C,
-                    int io_dtype, cudaStream_t st) {
-  if (!x || (!add) != (!sum) || (!out && !add) || (out && !weight)) return SL_ERR_NULL_POINTER;
   if (!dtype_ok(io_dtype)) return SL_ERR_UNSUPPORTED;
-  if (!rows_ok(rows, C, io_dtype, x, out) || !aligned(weight, 16) || !aligned(add, 16) || !aligned(sum, 16)) return SL_ERR_BAD_SHAPE;
+  if (!rows_ok(rows, C, io_dtype, x, out) || !aligned(weight, 16)) return SL_ERR_BAD_SHAPE;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const unsigned grid = (unsigned)((rows + 7) / 8);
   const bool narrow = C / (io_dtype == SL_F32 ? 4 : 8) <= 32 * RMS_MAXP_NARROW;
   SL_DISPATCH_DTYPE(io_dtype, T, {
     auto kern = narrow ? rmsnorm_fwd_kernel<T, RMS_MAXP_NARROW> : rmsnorm_fwd_kernel<T, RMS_MAXP>;
     kern<<<grid, 256, 0, st>>>(reinterpret_cast<const T*>(x), reinterpret_cast<const T*>(weight),
-                               reinterpret_cast<T*>(out), rows, C, eps, reinterpret_cast<const T*>(add), reinterpret_cast<T*>(sum));
+                               reinterpret_cast<T*>(out), rows, C, eps);
   });
   note_launches(1);
   return launch_status();
 }
+
+namespace sl {
+int residual_sum(const void* a, const void* b, void* out, long long n, int io_dtype, cudaStream_t st) {
+  if (!a || !b || !out) return SL_ERR_NULL_POINTER;
+  if (!dtype_ok(io_dtype)) return SL_ERR_UNSUPPORTED;
+  const int V = io_dtype == SL_F32 ? 4 : 8;
+  if (n < V || n % V || !aligned(a, 16) || !aligned(b, 16) || !aligned(out, 16)) return SL_ERR_BAD_SHAPE;
+  const long long pieces = n / V;
+  SL_DISPATCH_DTYPE(io_dtype, T, {
+    residual_sum_kernel<T><<<(unsigned)((pieces + 255) / 256), 256, 0, st>>>(
+        reinterpret_cast<const uint4*>(a), reinterpret_cast<const uint4*>(b), reinterpret_cast<uint4*>(out), pieces);
+  });
+  note_launches(1);
+  return launch_status();
+}
+
 // d_weight: float32 accumulators, or float64 ones (weight64); extra (or null) is added to d_x, its column sums to extra_sum
 // (or null; up to 1024 columns, where the second row of sums per warp still leaves three CTAs per SM)
 bool rmsnorm_bwd_sums_extra(int C) { return C <= 1024; }
@@ -493,9 +498,7 @@ int rmsnorm_bwd(const void* x, const void* weight, float eps, const void* d_out,
       T* to = reinterpret_cast<T*>(d_x);
       auto kern = extra_sum ? (lanes <= 2 ? rmsnorm_bwd_narrow_kernel<T, 2, true> : rmsnorm_bwd_narrow_kernel<T, 3, true>)
                             : (lanes <= 2 ? rmsnorm_bwd_narrow_kernel<T, 2, false> : rmsnorm_bwd_narrow_kernel<T, 3, false>);
-      const size_t smem = (size_t)16 * C * sizeof(float);
-      if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return SL_ERR_LAUNCH_FAILED;
+      const size_t smem = (size_t)16 * C * sizeof(float);   // (48 KB at most)
       kern<<<grid, 512, smem, st>>>(tx, tw, td, to, d_weight, weight64, te, extra_sum, rows, C, eps);
     });
     note_launches(1);

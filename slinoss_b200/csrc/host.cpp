@@ -564,7 +564,7 @@ class TokenPlan {
       Tensor out = fresh(D);
       if (fused(ptr(a), W, 0, D, bias, {&out}, &residual)) return out;
       const Tensor branch = linear(a, W, bias);
-      check(sl::rmsnorm_fwd_sum(ptr(residual), ptr(branch), mptr(out), nullptr, 0.f, nullptr, M, D, io, st), "sl_rmsnorm_fwd");
+      check(sl::residual_sum(ptr(residual), ptr(branch), mptr(out), M * D, io, st), "residual_sum");
       behind_own = true;
       return out;
     };

@@ -118,10 +118,10 @@ SL_API int mixer_tail_bwd(const void* Y, const void* gate, int64_t gate_stride, 
 // d_weight float32 or weight64 (sums that rounding to a shorter type makes independent of their order): added to; extra
 // (rows, C) or null is added to d_x, and its column sums to extra_sum (or null) where rmsnorm_bwd_sums_extra
 SL_API bool rmsnorm_bwd_sums_extra(int C);
-SL_API int rmsnorm_fwd_sum(const void* x, const void* add, void* sum, const void* weight, float eps, void* out, long long rows, int C,
-                           int io_dtype, cudaStream_t st);
 SL_API int rmsnorm_bwd(const void* x, const void* weight, float eps, const void* d_out, const void* extra, void* d_x, float* d_weight,
                        double* weight64, double* extra_sum, long long rows, int C, int io_dtype, cudaStream_t st);
+// out = a + b of n elements, rounded as torch rounds the sum of two such tensors
+SL_API int residual_sum(const void* a, const void* b, void* out, long long n, int io_dtype, cudaStream_t st);
 // sl_ffn_activation_bwd that also adds the column sums of its result to sums (one or two times H)
 SL_API int ffn_act_bwd_sum(const void* projected, const void* d_hidden, void* d_projected, double* sums, long long rows, int H, int kind,
                            int io_dtype, cudaStream_t st);
