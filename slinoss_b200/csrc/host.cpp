@@ -8,6 +8,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/as_strided_native.h>
 #include <ATen/ops/mm_cuda_dispatch.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
@@ -480,7 +481,8 @@ class TokenPlan {
     ok = ok && is(conv, type, {M, C, d_conv_ - 1}) && is(state, at::kFloat, {M, heads_, P_, 2 * N_}) &&
          is(b_prev, type, {M, groups_, 2 * N_}) && is(u_prev, type, {M, heads_, P_});
     const bool block = !b_.empty(), ffn = b_.size() == 6;
-    if (block) ok = ok && is(b_[0], type, {D}) && D % 8 == 0 && D <= 2048;   // (what the row kernel of the norm takes)
+    // (what the row kernel of the norm takes; a dispatch mode sees a block's products, which below pass the dispatcher by)
+    if (block) ok = ok && is(b_[0], type, {D}) && D % 8 == 0 && D <= 2048 && !c10::impl::TorchDispatchModeTLS::any_modes_set();
     if (ok && ffn) {
       const int64_t F = b_[4] ? b_[4]->size(1) : 0, wide = ffn_kind_ == 1 ? 2 * F : F;
       ok = is(b_[1], type, {D}) && is(b_[2], type, {wide, D}) && (!b_[3] || is(b_[3], type, {wide})) && is(b_[4], type, {D, F}) &&

@@ -287,3 +287,32 @@ def test_a_block_token_overlaps_only_kernels_of_this_library(batch, d_model, by_
     programmatic = driver.CUgraphDependencyType.CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC.value
     early = [name(driver.CUgraphNode(s)) for s, d in zip(sources, data) if d[2] == programmatic]    # (ports, then the type)
     assert len(early) >= 6 and all(n.startswith("_ZN2sl") for n in early), early
+
+
+def test_a_dispatch_mode_sees_the_products_of_a_block_token():
+    """The plan's products pass the dispatcher by, so under a mode that watches it a block takes the composed path, whose bits the
+    plan has."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Watch(TorchDispatchMode):
+        def __init__(self):
+            super().__init__()
+            self.seen = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.seen.append(func._schema.name)
+            return func(*args, **(kwargs or {}))
+
+    torch.manual_seed(1)
+    cfg = sb.SLinOSSBlockConfig(d_model=128, mixer=sb.SLinOSSMixerConfig(d_state=64, d_head=64, expand=1.0),
+                                ffn=sb.SLinOSSMLPConfig(kind="gelu", expand=2.0, multiple_of=8))
+    stack = sb.SLinOSSStack(sb.SLinOSSStackConfig.uniform(cfg, n_layers=2), device=DEV, dtype=torch.bfloat16).eval()
+    x = torch.randn(4, 128, device=DEV, dtype=torch.bfloat16)
+    watch = Watch()
+    with torch.no_grad():
+        want, _ = stack.step(x, stack.init_decode_state(4))
+        state = stack.init_decode_state(4)
+        with watch:
+            got, _ = stack.step(x, state)
+    products = [n for n in watch.seen if n in ("aten::mm", "aten::addmm", "aten::linear")]
+    assert len(products) >= 2 * 4 and torch.equal(got, want)
