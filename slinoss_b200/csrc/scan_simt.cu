@@ -196,9 +196,6 @@ struct Layout {
   }
 };
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Rows [0, nb) of cols elements, pitch elements apart in memory, into shared memory.  16-byte pieces where every row starts
