@@ -55,7 +55,9 @@ enum { SL_F32 = 0, SL_BF16 = 1, SL_F16 = 2 };
 /* kernel family selector for the scan */
 enum {
   SL_PATH_AUTO = 0, /* tensor-core path when type and sizes allow it, else SIMT */
-  SL_PATH_SIMT = 1, /* exact float32 sequential recurrence (any dtype in)     */
+  SL_PATH_SIMT = 1, /* float32 products and sums of any operand type, in chunks of 16 tokens; computes through
+                       zero transitions.  A value that is not finite reaches what depends on it and nothing
+                       else; an infinity may come out as NaN                            */
   SL_PATH_TC = 2    /* tcgen05/TMEM chunked path: bf16 / fp16 operands, P = 64, N = 64 or 128 (other
                        sizes are refused here and take SIMT under auto); without the SL_WS_SCAN_FWD
                        workspace of a problem a forward pass with N = 64 walks every stream whole
@@ -153,7 +155,7 @@ SL_API int sl_v2x2ssd_bwd(const void* U, const float* M, const float* K, const v
  * call cudaMalloc - the GPU already belongs to their own memory pool, their hot loop
  * bans allocator calls, or they are inside a stream capture.)
  *
- * Same arguments and results as sl_v2x2ssd_bwd on the exact float32 (SIMT) path,
+ * Same arguments and results as sl_v2x2ssd_bwd on the float32 path (SL_PATH_SIMT),
  * minus chunk / path / workspace.  The scratch is a fixed array of
  * SL_STATIC_SCRATCH_BYTES inside the library image, resident on every GPU that loads
  * the library until the process exits.  Limits and rules:

@@ -231,7 +231,7 @@ def scan_bwd(U, M, K, B, C, z0, B_prev, U_prev, dY, d_final, *, chunk_size, path
 
 
 def scan_bwd_static(U, M, K, B, C, z0, B_prev, U_prev, dY, d_final, outs):
-    """Launch ``sl_v2x2ssd_bwd_static``: the float32-exact backward with its scratch in the
+    """Launch ``sl_v2x2ssd_bwd_static``: the float32 backward with its scratch in the
     library's built-in array, for callers that may not allocate device memory.
 
     Nothing is allocated here either: ``outs`` is the tuple of caller-provided result

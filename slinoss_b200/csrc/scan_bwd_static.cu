@@ -4,7 +4,7 @@
 // that has already given the whole GPU to its own memory pool, a real-time loop that
 // forbids allocator calls on its hot path, or code running between
 // cudaStreamBeginCapture / EndCapture where cudaMalloc is illegal.  For them this
-// file offers the exact float32 (SIMT) backward of the scan with its scratch held in
+// file offers the float32 backward of the scan with its scratch held in
 // a fixed array that is part of the library image.
 //
 // Consequences the caller has to know:

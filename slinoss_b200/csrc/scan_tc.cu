@@ -3,7 +3,7 @@
 // Supported: P = 64, N = 64 or 128 (blocks of 64 oscillators, 128 real columns), bf16 or fp16 operands, float32 state.
 // Everything else takes the float32 path.  (Narrower N would fit with zero columns and run 4 times faster than
 // there, fp16 forward + backward of 64 streams x 2048 tokens x N = 48: 174 against 663 us; but the products round
-// their operands to 16 bits and need every |m| > 0, which the exact sweeps that these widths have always had do not.)
+// their operands to 16 bits and need every |m| > 0, which the float32 sweeps do not.)
 //
 // Formulation (per (batch, head); chunk of L = 64 tokens, local index t, s).  The two
 // taps are merged into one source coefficient with a one-token look-ahead,
@@ -537,7 +537,7 @@ int run_bwd(const void* U, const float* M, const float* K, const void* B, const 
 
 }  // namespace
 
-// A dY of another dtype than the operands (or none) takes the exact float32 sweeps.
+// A dY of another dtype than the operands (or none) takes the float32 sweeps.
 int scan_tc_bwd(const void* U, const float* M, const float* K, const void* B, const void* C,
                 const float* z0, const void* Bprev, const void* Uprev, const void* states_in,
                 const float* zfinal_in, const void* dY,

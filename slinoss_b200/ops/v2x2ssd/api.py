@@ -158,7 +158,7 @@ def assert_nonzero_transitions(M: torch.Tensor) -> None:
     """Raise the reference's error for an exact-zero transition (slinoss/ops/v2x2ssd/reference.py:509-517).
 
     ``|m_t| > 0`` is a precondition of the chunked (tensor-core) kernels: they form ``log|m|`` and, in the
-    merged-tap form, ``kp_{t+1} / m_{t+1}``; a zero transition yields NaN or Inf there (the exact path computes
+    merged-tap form, ``kp_{t+1} / m_{t+1}``; a zero transition yields NaN or Inf there (the float32 path computes
     a forward pass through it, with dM = 0 at that token).  The ops do not check it themselves, because the
     check synchronises the device (the reference's torch path does it on every call); call this where the
     transitions do not come from the scan preparation, whose radius is bounded below by ``r_min``."""
@@ -245,7 +245,7 @@ def v2x2ssd_cute(U, M, K, B, C, *, chunk_size, initial_states=None, B_prev=None,
     """GPU scan.  Returns ``Y`` or ``(Y, final_state, B_last, U_last)``.
 
     ``path`` selects the kernel family: "auto" (tensor cores when the shape and dtype
-    allow, else the exact float32 recurrence), "simt" or "tc".  ``save_chunk_states``
+    allow, else the float32 sweeps), "simt" (those) or "tc".  ``save_chunk_states``
     (training only) keeps the tensor-core path's 16-bit chunk-start states for the
     backward instead of recomputing them there; False saves only the inputs, like the
     reference."""
