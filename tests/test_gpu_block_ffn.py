@@ -228,3 +228,39 @@ def test_training_nodes_of_a_block_equal_the_composed_block(kind, bias, C, T, dt
         assert got[name].shape == ref.shape and got[name].dtype == ref.dtype
         err = (got[name].float() - ref.float()).abs().max() / ref.float().abs().max().clamp_min(1e-6)
         assert err <= 3e-2, (name, err)
+
+
+# rows of three 16-byte pieces a lane (513 to 768 channels of 16-bit types, 257 to 384 of float32), the last one partly empty and
+# full, over less than a row for each of the 148 x 16 warps, one for each, and several
+@pytest.mark.parametrize("dtype, C", [(torch.bfloat16, 520), (torch.bfloat16, 576), (torch.float16, 768), (torch.float32, 260),
+                                      (torch.float32, 384)])
+@pytest.mark.parametrize("rows", [5, 2368, 5000])
+@pytest.mark.parametrize("with_extra", [False, True])
+def test_rmsnorm_backward_of_rows_of_three_pieces(dtype, C, rows, with_extra):
+    torch.manual_seed(rows + C)
+    x, dy, extra = (torch.randn(rows, C, device=DEV).to(dtype) for _ in range(3))
+    w = (1 + 0.3 * torch.randn(C, device=DEV)).to(dtype)
+    x64, w64 = x.double().requires_grad_(), w.double().requires_grad_()
+    _rms64(x64, w64, 1e-5).backward(dy.double())
+    dx, dw = _C.rmsnorm_bwd(x, w, 1e-5, dy, extra=extra if with_extra else None)
+    assert rel(dx, x64.grad + extra.double() if with_extra else x64.grad) <= TOL[dtype]
+    assert rel(dw, w64.grad) <= 1e-5
+
+
+@pytest.mark.parametrize("dtype, C, rows", [(torch.bfloat16, 576, 70), (torch.bfloat16, 768, 4000), (torch.float16, 520, 2400),
+                                            (torch.bfloat16, 256, 3000), (torch.float16, 512, 2400)])
+def test_ffn_branch_sums_the_gradients_of_its_output_bias_beside_the_norms(dtype, C, rows):
+    blk = _block("gelu", True, dtype, d_model=C, remat="none")
+    x = torch.randn(1, rows, C, device=DEV).to(dtype)
+    dy = torch.randn_like(x)
+    xi = x.clone().requires_grad_()
+    blk._ffn_residual(xi).backward(dy)
+    blk64 = _block("gelu", True, dtype, d_model=C, remat="none").double()
+    x64 = x.double().requires_grad_()
+    blk64._ffn_residual(x64).backward(dy.double())
+    assert rel(xi.grad, x64.grad) <= TOL[dtype]
+    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert rel(blk.ffn.out_proj.bias.grad, dy.double().sum((0, 1))) <= unit     # one rounding of the sum
+    for name in ("ffn_norm.weight", "ffn.in_proj.bias"):    # sums over the rows of values that were rounded on the way
+        got, want = (dict(b.named_parameters())[name].grad for b in (blk, blk64))
+        assert rel(got, want) <= TOL[dtype], name
