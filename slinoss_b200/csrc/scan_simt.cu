@@ -40,8 +40,9 @@
 // What bounds it now: issue and latency at 12 warps per SM (168 registers hold the state, its parts and the operands); 41 % of
 // the issue slots and 33 % of the tensor pipe are busy in the forward sweep.  Forward + backward, us, against sweeps token by
 // token on the FMA pipe: (16, 4, 2048, N 48 fp16) 2973 -> 663, (2, 4, 256, N 32 fp32) 61 -> 51.
-// Distance from float64 against those sweeps (2-norm, float32 operands, T 256 to 8192): Y 1.27e-7 -> 1.13e-7, dC 1.28e-7 ->
-// 1.17e-7, dU 1.13e-7 and dK 1.30e-7 both, dB 1.10e-7 -> 1.12e-7, d_initial 9.2e-8 -> 7.5e-8, dM a third nearer.
+// Distance from float64 against those sweeps (2-norm, float32 operands, T 256 to 4096, by shape): Y 1.26..1.29e-7 -> 1.07..1.12e-7,
+// dU 1.13..1.15e-7 -> 1.07..1.12e-7, dB 1.08..1.09e-7 -> 1.01..1.02e-7, dC 1.25..1.26e-7 -> 1.05..1.06e-7, dK 1.27..1.32e-7 ->
+// 1.19..1.24e-7, dM a third nearer.
 //
 // The walk over T is serial, so a problem with few (batch, head) streams is split in time: a first launch runs every
 // segment but the last from a zero state and keeps only where it ends and the product of its transitions (in float64), a second
@@ -128,7 +129,11 @@ __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint3
 // ones are added up here over 16 terms at most; longer sums go through rounded float32 additions.  Measured against float64
 // over normal operands: 4.8e-8 relative for 16 terms and 6.3e-8 for 64, where a chain of fmaf has 7.4e-8 and 1.5e-7.
 // NT independent tiles at a time, a product of each in turn: a tensor-core operation waits for the one before it on its sum.
-template <int NT, int NA, int NB, typename FA, typename FB>
+// APART: the first parts' product, whose 16 terms of 16 bits are nearly exact, starts from zero too and the others' sum is added
+// to it by a rounded addition instead of being cut off under it.  Where a result is common to many others its error does not average
+// out: with the products over the rows of P (X) and with the state so, dB came from 1.11e-7 to 1.02e-7 of float64 and dU from 1.16e-7 to
+// 1.12e-7 (1.09e-7 and 1.15e-7 token by token), at 684 -> 686 us for (16, 4, 2048, N 48 fp16); all products so: 9.0e-8, 703 us.
+template <int NT, int NA, int NB, bool APART = false, typename FA, typename FB>
 __device__ __forceinline__ void products(float (&d)[NT][4], FA a, FB b) {
   constexpr int SUM = NA + NB - 2 < 2 ? NA + NB - 2 : 2, FIRST = SUM - (NB - 1) > 0 ? SUM - (NB - 1) : 0;
 #pragma unroll
@@ -138,8 +143,16 @@ __device__ __forceinline__ void products(float (&d)[NT][4], FA a, FB b) {
       if (sum - i >= 0 && sum - i < NB)
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-          if (sum == SUM && i == FIRST) mma<true>(d[t], a(t)[i], b(t)[sum - i][0], b(t)[sum - i][1]);
-          else mma<false>(d[t], a(t)[i], b(t)[sum - i][0], b(t)[sum - i][1]);
+          if (sum == SUM && i == FIRST) {
+            mma<true>(d[t], a(t)[i], b(t)[sum - i][0], b(t)[sum - i][1]);
+          } else if (APART && sum == 0) {
+            float e[4];
+            mma<true>(e, a(t)[0], b(t)[0][0], b(t)[0][1]);
+            const float2 u = un2(add2(mk2(e[0], e[1]), mk2(d[t][0], d[t][1]))), v = un2(add2(mk2(e[2], e[3]), mk2(d[t][2], d[t][3])));
+            d[t][0] = u.x; d[t][1] = u.y; d[t][2] = v.x; d[t][3] = v.y;
+          } else {
+            mma<false>(d[t], a(t)[i], b(t)[sum - i][0], b(t)[sum - i][1]);
+          }
         }
 }
 // ---- sums over the earlier (or later) tokens of a chunk ---------------------------------------------------------------
@@ -726,7 +739,7 @@ __device__ __forceinline__ void walk(const SweepParams& p, int pt0, int seg, uin
               x[t][e][0] = transposed(a[t >> 1][e][2 * (t & 1)]); x[t][e][1] = transposed(a[t >> 1][e][2 * (t & 1) + 1]);
             }
           float d[4][4];
-          products<4, 3, 3>(d, [&](int t) { return &op[t >> 1][0]; }, [&](int t) { return &x[t][0]; });
+          products<4, 3, 3, true>(d, [&](int t) { return &op[t >> 1][0]; }, [&](int t) { return &x[t][0]; });
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
             y0[k] = add2(mk2(d[k][0], d[k][1]), mk2(d[2 + k][0], d[2 + k][1]));
@@ -763,7 +776,7 @@ __device__ __forceinline__ void walk(const SweepParams& p, int pt0, int seg, uin
           }
         }
         float d[4][4];   // [rows of P, column tile]
-        products<4, NA, NB>(d, [&](int t) { return &a[t >> 1][0]; }, [&](int t) { return &r[t][0]; });
+        products<4, NA, NB, true>(d, [&](int t) { return &a[t >> 1][0]; }, [&](int t) { return &r[t][0]; });
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           x[t][0] = add2(x[t][0], add2(mk2(d[t][0], d[t][1]), mk2(d[2 + t][0], d[2 + t][1])));
