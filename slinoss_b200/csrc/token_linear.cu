@@ -11,6 +11,8 @@
 // residual, the activation and the norm; here it is 2 to 3 us with all of them inside (norms: up to 16 rows).  On the device:
 // latency of one trip to memory (all of a warp's rows of W are requested at the start, x two pieces ahead) and the chain of
 // K / 16 steps on one accumulator.
+#include <algorithm>
+
 #include "common.cuh"
 #include "host_abi.h"
 
@@ -31,6 +33,7 @@ template <> __device__ __forceinline__ uint32_t plain_pair<__half>(float a, floa
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+constexpr int CHAIN_MAX = 4096;               // see token_linear_supported
 constexpr int KC = 256;                       // k values of a piece of x
 constexpr int X_PITCH = 2 * KC + 32;          // rows 32 bytes off a multiple of 128: 8-byte reads of 4 rows x 32 bytes hit all banks
 __host__ __device__ constexpr int w_pitch(int K) { return (2 * K + 127) / 128 * 128 + 32; }
@@ -195,59 +198,73 @@ __global__ void __launch_bounds__(NORM ? 256 : 128) token_linear_kernel(TokenLin
     }
 }
 
-// Warps of a CTA: one while their rows of W (8 a warp) still spread over the SMs, more when there are several for each.
-int warps_of(const TokenLinearArgs& a, size_t* smem) {
-  const int NT = a.swiglu ? 2 : 1, MT = (a.M + 15) / 16;
-  const int tiles = a.O / NT / 8;
+// Warps with rows of W (8 a warp) of a CTA: one while they still spread over the SMs, more when there are several for each, or
+// (without a norm) where that saves a round of CTAs: 64 x 2048 by 4096 columns 29.6 us with two, 15.9 with four.
+struct Plan {
+  int nw, rounds;   // nw 0: does not fit
+  size_t smem;
+};
+Plan plan_of(const TokenLinearArgs& a) {
+  const int NT = a.swiglu ? 2 : 1, MT = (a.M + 15) / 16, tiles = a.O / NT / 8;
+  auto bytes = [&](int nw) {
+    return (a.norm_weight ? 16 * w_pitch(a.K) : 2 * 16 * (size_t)MT * X_PITCH) + (size_t)nw * NT * 8 * w_pitch(a.K);
+  };
+  auto rounds = [&](int nw) {   // (four CTAs on an SM at most: more would share its issue slots)
+    const int slots = 148 * std::max(1, std::min(4, (int)(227 * 1024 / (bytes(nw) + 1024))));
+    return ((tiles + nw - 1) / nw + slots - 1) / slots;
+  };
   int nw = tiles <= 2 * 148 ? 1 : tiles <= 8 * 148 ? 2 : 4;
-  for (;; nw /= 2) {
-    *smem = (a.norm_weight ? 16 * w_pitch(a.K) : 2 * 16 * (size_t)MT * X_PITCH) + (size_t)nw * NT * 8 * w_pitch(a.K);
-    if (nw == 0 || *smem <= 200 * 1024) return nw;
-  }
+  while (!a.norm_weight && nw < 4 && rounds(2 * nw) < rounds(nw)) nw *= 2;
+  while (nw > 0 && bytes(nw) > 200 * 1024) nw /= 2;
+  return nw ? Plan{nw, rounds(nw), bytes(nw)} : Plan{0, 0, 0};
 }
 
 template <typename T, int MT, int NT, bool NORM>
-int launch_token_as(const TokenLinearArgs& a, int nw, size_t smem, cudaStream_t st) {
+int launch_token_as(const TokenLinearArgs& a, const Plan& p, cudaStream_t st) {
   static std::atomic<unsigned long long> done{0};
   if (int e = ensure_smem(token_linear_kernel<T, MT, NT, NORM>, 200 * 1024, done)) return e;
   const int tiles = a.O / NT / 8;
-  return launch_chained(token_linear_kernel<T, MT, NT, NORM>, dim3((tiles + nw - 1) / nw), (unsigned)(NORM ? 256 : 32 * nw), smem, st, a.dependent, a, nw);
+  // (warps without rows of W help to stage x: 23 x 3840 by 960 columns was bound by one warp's copies)
+  return launch_chained(token_linear_kernel<T, MT, NT, NORM>, dim3((tiles + p.nw - 1) / p.nw), NORM ? 256u : 128u, p.smem, st, a.dependent, a, p.nw);
 }
 template <typename T, int MT>
-int launch_token_m(const TokenLinearArgs& a, int nw, size_t smem, cudaStream_t st) {
+int launch_token_m(const TokenLinearArgs& a, const Plan& p, cudaStream_t st) {
   if constexpr (MT == 1)
-    if (a.norm_weight) return a.swiglu ? launch_token_as<T, 1, 2, true>(a, nw, smem, st) : launch_token_as<T, 1, 1, true>(a, nw, smem, st);
-  return a.swiglu ? launch_token_as<T, MT, 2, false>(a, nw, smem, st) : launch_token_as<T, MT, 1, false>(a, nw, smem, st);
+    if (a.norm_weight) return a.swiglu ? launch_token_as<T, 1, 2, true>(a, p, st) : launch_token_as<T, 1, 1, true>(a, p, st);
+  return a.swiglu ? launch_token_as<T, MT, 2, false>(a, p, st) : launch_token_as<T, MT, 1, false>(a, p, st);
 }
 template <typename T>
-int launch_token(const TokenLinearArgs& a, int nw, size_t smem, cudaStream_t st) {
+int launch_token(const TokenLinearArgs& a, const Plan& p, cudaStream_t st) {
   switch ((a.M + 15) / 16) {
-    case 1: return launch_token_m<T, 1>(a, nw, smem, st);
-    case 2: return launch_token_m<T, 2>(a, nw, smem, st);
-    case 3: return launch_token_m<T, 3>(a, nw, smem, st);
-    default: return launch_token_m<T, 4>(a, nw, smem, st);
+    case 1: return launch_token_m<T, 1>(a, p, st);
+    case 2: return launch_token_m<T, 2>(a, p, st);
+    case 3: return launch_token_m<T, 3>(a, p, st);
+    default: return launch_token_m<T, 4>(a, p, st);
   }
 }
 
 }  // namespace
 
-// Whole tiles of 8 columns, rows of W that start on 16 bytes.
+// Whole tiles of 8 columns, rows of W that start on 16 bytes, and a chain that is not too long.  A warp takes 1.3 us and 1.7 ns for each
+// k of each of its 16 x 8 tiles, and CTAs that do not fit on the chip at once take turns: the library's product is 4 to 10 us on the
+// device with 5 to 7 more of host and of launches behind it, which is 4096 such k.  Device times, here / library: 32 x 1024 by 4096 columns 7.0 / 6.2,
+// by 16384 16.0 / 10.3; 32 x 4096 by 1024 18.6 / 10.3; 64 x 1024 by 2048 8.8 / 6.2, 64 x 2048 by 2048 16.0 / 8.0.
 bool token_linear_supported(const TokenLinearArgs& a) {
-  size_t smem;
   if (a.M < 1 || a.M > 64 || a.K < 8 || a.K % 8 || a.O < 8 || a.O % (a.swiglu ? 16 : 8) || (a.io_dtype != SL_BF16 && a.io_dtype != SL_F16))
     return false;
   for (int i = 0; i < 3; ++i)
     if (a.width[i] % 8 || !aligned(a.out[i], 4)) return false;
   if (a.norm_weight && (a.M > 16 || !aligned(a.norm_weight, 16) || (!a.partials && a.K > 2048))) return false;
-  return aligned(a.x, 16) && aligned(a.weight, 16) && aligned(a.residual, 4) && warps_of(a, &smem) > 0;
+  if (!aligned(a.x, 16) || !aligned(a.weight, 16) || !aligned(a.residual, 4)) return false;
+  const Plan p = plan_of(a);
+  return p.nw > 0 && (long long)p.rounds * a.K * ((a.M + 15) / 16) * (a.swiglu ? 2 : 1) <= CHAIN_MAX;
 }
 
 int token_linear(const TokenLinearArgs& a, cudaStream_t st) {
   if (!a.x || !a.weight || !a.out[0]) return SL_ERR_NULL_POINTER;
   if (!token_linear_supported(a)) return SL_ERR_UNSUPPORTED;
-  size_t smem;
-  const int nw = warps_of(a, &smem);
-  const int rc = a.io_dtype == SL_BF16 ? launch_token<__nv_bfloat16>(a, nw, smem, st) : launch_token<__half>(a, nw, smem, st);
+  const Plan p = plan_of(a);
+  const int rc = a.io_dtype == SL_BF16 ? launch_token<__nv_bfloat16>(a, p, st) : launch_token<__half>(a, p, st);
   if (rc != SL_OK) return rc;
   note_launches(1);
   return launch_status();
