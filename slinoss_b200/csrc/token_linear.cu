@@ -33,7 +33,6 @@ template <> __device__ __forceinline__ uint32_t plain_pair<__half>(float a, floa
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-constexpr int CHAIN_MAX = 4096;               // see token_linear_supported
 constexpr int KC = 256;                       // k values of a piece of x
 constexpr int X_PITCH = 2 * KC + 32;          // rows 32 bytes off a multiple of 128: 8-byte reads of 4 rows x 32 bytes hit all banks
 __host__ __device__ constexpr int w_pitch(int K) { return (2 * K + 127) / 128 * 128 + 32; }
@@ -245,10 +244,14 @@ int launch_token(const TokenLinearArgs& a, const Plan& p, cudaStream_t st) {
 
 }  // namespace
 
-// Whole tiles of 8 columns, rows of W that start on 16 bytes, and a chain that is not too long.  A warp takes 1.3 us and 1.7 ns for each
-// k of each of its 16 x 8 tiles, and CTAs that do not fit on the chip at once take turns: the library's product is 4 to 10 us on the
-// device with 5 to 7 more of host and of launches behind it, which is 4096 such k.  Device times, here / library: 32 x 1024 by 4096 columns 7.0 / 6.2,
-// by 16384 16.0 / 10.3; 32 x 4096 by 1024 18.6 / 10.3; 64 x 1024 by 2048 8.8 / 6.2, 64 x 2048 by 2048 16.0 / 8.0.
+// Whole tiles of 8 columns, rows of W that start on 16 bytes, and a chain that is not too long: a warp takes 1.3 us and 1.7 ns for
+// each k of each of its 16 x 8 tiles, and CTAs that do not fit on the chip at once take turns.  The library's product is 4 to 10 us on
+// the device, and 5 to 7 of host with what follows it as launches of their own.  Device times, here / library: 32 x 1024 by 4096
+// columns 7.0 / 6.2, by 16384 16.0 / 10.3; 32 x 4096 by 1024 18.6 / 10.3; 64 x 1024 by 2048 8.8 / 6.2, 64 x 2048 by 2048 16.0 / 8.0.
+// So 4096 such k where the norm is inside or the library would need more than a product (in_proj's three parts, the product in
+// front of a SwiGLU), 3072 up to 32 rows, 2048 beyond.  Two blocks, us, before this kernel / with one limit of 2048 / of 4096 / none: 24 rows of
+// width 960 (gelu, N 128) 216 / 207 / 229 / 228, 48 of 960 (swiglu, N 64) 202 / 201 / 221 / 255, 48 of 768 (swiglu, one group)
+// 199 / 187 / 145 / 172, 17 of 768 195 / 135 / 111 / 111, 1 of 1024 196 / 127 / 108 / 108.
 bool token_linear_supported(const TokenLinearArgs& a) {
   if (a.M < 1 || a.M > 64 || a.K < 8 || a.K % 8 || a.O < 8 || a.O % (a.swiglu ? 16 : 8) || (a.io_dtype != SL_BF16 && a.io_dtype != SL_F16))
     return false;
@@ -257,7 +260,8 @@ bool token_linear_supported(const TokenLinearArgs& a) {
   if (a.norm_weight && (a.M > 16 || !aligned(a.norm_weight, 16) || (!a.partials && a.K > 2048))) return false;
   if (!aligned(a.x, 16) || !aligned(a.weight, 16) || !aligned(a.residual, 4)) return false;
   const Plan p = plan_of(a);
-  return p.nw > 0 && (long long)p.rounds * a.K * ((a.M + 15) / 16) * (a.swiglu ? 2 : 1) <= CHAIN_MAX;
+  const int limit = a.M <= 16 || a.out[2] || a.swiglu ? 4096 : a.M <= 32 ? 3072 : 2048;
+  return p.nw > 0 && (long long)p.rounds * a.K * ((a.M + 15) / 16) * (a.swiglu ? 2 : 1) <= limit;
 }
 
 int token_linear(const TokenLinearArgs& a, cudaStream_t st) {

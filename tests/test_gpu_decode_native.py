@@ -212,14 +212,15 @@ def test_the_engine_refuses_weights_of_another_type(batch, weights, token):
 
 
 # the sizes where a block's own products change: row tiles of 16, k tails of 8, biases, parts of in_proj whose width is no
-# multiple of 8 (3 heads of 18: that part stays the library's), the longest layers that are the kernel's at 16 and at 64 rows and
-# the next longer ones (the library's, with the residual sum behind), layers too long for shared memory
+# multiple of 8 (3 heads of 18: that part stays the library's), the longest layers that are the kernel's at 16, 32 and 64 rows
+# and the next longer ones (the library's, with the residual sum behind), layers too long for shared memory
 @pytest.mark.parametrize("batch, d_model, dtype, d_head, kind, bias, hidden", [
     (1, 8, torch.bfloat16, 8, "gelu", False, 8), (16, 264, torch.float16, 64, "gelu", True, 520),
     (32, 576, torch.bfloat16, 32, "swiglu", True, 1000), (33, 128, torch.float16, 64, "swiglu", False, 72),
     (48, 1024, torch.bfloat16, 64, "gelu", False, 4096), (64, 192, torch.bfloat16, 64, "swiglu", False, 8192),
     (16, 192, torch.float16, 64, "gelu", False, 4096), (16, 192, torch.float16, 64, "gelu", True, 4104),
-    (64, 192, torch.bfloat16, 64, "gelu", True, 1024), (64, 192, torch.bfloat16, 64, "gelu", False, 1032),
+    (32, 192, torch.bfloat16, 64, "gelu", True, 1536), (32, 192, torch.bfloat16, 64, "gelu", False, 1544),
+    (64, 192, torch.bfloat16, 64, "gelu", True, 512), (64, 192, torch.bfloat16, 64, "gelu", False, 520),
     (3, 128, torch.bfloat16, 64, "swiglu", False, 12288)])
 def test_token_products_have_the_librarys_bits(batch, d_model, dtype, d_head, kind, bias, hidden, monkeypatch):
     torch.manual_seed(batch)
