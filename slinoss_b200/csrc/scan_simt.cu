@@ -37,9 +37,10 @@
 // columns (Y, dU, d(j,i)) and the per-token scalars cross warps.  The chain of transition products is one warp's, one chunk
 // ahead.
 //
-// What bounds it now: issue and latency at 12 warps per SM (168 registers hold the state, its parts and the operands); 41 % of
-// the issue slots and 33 % of the tensor pipe are busy in the forward sweep.  Forward + backward, us, against sweeps token by
-// token on the FMA pipe: (16, 4, 2048, N 48 fp16) 2973 -> 663, (2, 4, 256, N 32 fp32) 61 -> 51.
+// What bounds it now: issue and latency at 12 warps per SM: 168 registers hold the state, its parts and the operands, and the
+// backward spills 280 to 740 bytes beside them.  Forward + backward, us, against sweeps token by token on the FMA pipe: (16, 4, 2048,
+// N 48 fp16) 2973 -> 663, to which the looks for values that are not finite add 3 and the sums kept apart 2 (see below); (2, 4, 256,
+// N 32 fp32) 61 -> 51.
 // Distance from float64 against those sweeps (2-norm, float32 operands, T 256 to 4096, by shape): Y 1.26..1.29e-7 -> 1.07..1.12e-7,
 // dU 1.13..1.15e-7 -> 1.07..1.12e-7, dB 1.08..1.09e-7 -> 1.01..1.02e-7, dC 1.25..1.26e-7 -> 1.05..1.06e-7, dK 1.27..1.32e-7 ->
 // 1.19..1.24e-7, dM a third nearer.
